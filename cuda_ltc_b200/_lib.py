@@ -6,10 +6,13 @@ shared object is missing -- build it with ``python -m cuda_ltc_b200.build``.
 from __future__ import annotations
 
 import ctypes as C
+import importlib.machinery
+import importlib.util
 import os
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "libltc_attn.so")
+HOST_PATH = os.path.join(HERE, "_host.so")
 
 LTCA_F32, LTCA_BF16 = 0, 1
 MODE_AUTO, MODE_BF16, MODE_SPLIT, MODE_FP32 = 0, 1, 2, 3
@@ -122,3 +125,23 @@ def load() -> C.CDLL:
             fn.argtypes = args
         _lib = lib
     return _lib
+
+
+_host = None
+
+
+def load_host(error_class):
+    """Loads the native half of the torch front end (csrc/host_binding.cpp) once; failed calls raise ``error_class``."""
+    global _host
+    if _host is None:
+        load()
+        if not os.path.exists(HOST_PATH):
+            raise RuntimeError(f"{HOST_PATH} is missing: run python -m cuda_ltc_b200.build; there is no fallback path")
+        import torch                    # its libraries must be in the process
+        loader = importlib.machinery.ExtensionFileLoader("cuda_ltc_b200._host", HOST_PATH)
+        spec = importlib.util.spec_from_file_location("cuda_ltc_b200._host", HOST_PATH, loader=loader)
+        mod = importlib.util.module_from_spec(spec)
+        loader.exec_module(mod)
+        mod.set_error_classes(error_class, torch.OutOfMemoryError)
+        _host = mod
+    return _host

@@ -2,7 +2,8 @@
 
 torch is plumbing here: it owns device memory and streams.  Every function fills an
 ``ltca_attn_params`` block with raw pointers and strides and calls libltc_attn.so; nothing is
-computed in Python and nothing falls back to torch operators.
+computed in Python and nothing falls back to torch operators.  The calls of the hot path do that in
+native code (``csrc/host_binding.cpp``).
 
 Tensor convention: ``[batch, heads, seq, head_dim]`` views with ``head_dim`` contiguous (any
 batch/head/seq strides), float32 or bfloat16 -- e.g. ``x.view(B, S, H, D).transpose(1, 2)``
@@ -17,7 +18,7 @@ from typing import Optional, Tuple
 import torch
 
 from . import _lib
-from ._lib import AttnParams, Strides
+from ._lib import AttnParams, Strides, TsaParams
 
 
 class LtcaError(RuntimeError):
@@ -52,10 +53,11 @@ class Context:
         if rc != 0:
             raise LtcaError(rc, "ltca_ctx_create failed (is this an sm_100 GPU?)")
         self.handle = handle
-        self._ws = None
+        self._host = _lib.load_host(LtcaError).Host(handle.value, self.device)
 
     def close(self):
         if getattr(self, "handle", None):
+            self._host.close()
             self.lib.ltca_ctx_destroy(self.handle)
             self.handle = None
 
@@ -137,11 +139,7 @@ class Context:
 
     def workspace(self, nbytes: int) -> Optional[torch.Tensor]:
         """A cached scratch buffer of at least ``nbytes`` (grown on demand, 256-byte aligned)."""
-        if nbytes == 0:
-            return None
-        if self._ws is None or self._ws.numel() < nbytes:
-            self._ws = torch.empty(nbytes, dtype=torch.uint8, device=f"cuda:{self.device}")
-        return self._ws
+        return self._host.workspace(nbytes)
 
     # ---- parameter block -----------------------------------------------------------------
     def _params(self, q, k, v, o, lse, scale, causal, keep_mask, kv_len, score_clamp, mode) -> AttnParams:
@@ -167,66 +165,23 @@ class Context:
             p.kv_len = kv_len.data_ptr()
         return p
 
-    def _attach_workspace(self, p: AttnParams, backward: int, fixed: Optional[int] = None):
-        need = C.c_size_t(0)
-        if fixed is None:
-            self.lib.ltca_attn_workspace_bytes(C.byref(p), backward, C.byref(need))
-            n = need.value
-        else:
-            n = fixed
-        ws = self.workspace(n)
-        if ws is not None:
-            p.workspace, p.workspace_bytes = ws.data_ptr(), ws.numel()
-        return ws
-
     # ---- calls ---------------------------------------------------------------------------
     def attn_fwd(self, q, k, v, scale=None, causal=False, keep_mask=None, kv_len=None,
                  score_clamp=0.0, mode=_lib.MODE_AUTO, out=None, lse=None
                  ) -> Tuple[torch.Tensor, torch.Tensor]:
-        B, H, Sq, D = q.shape
-        scale = 1.0 / math.sqrt(D) if scale is None else scale
-        o = torch.empty((B, H, Sq, D), dtype=q.dtype, device=q.device) if out is None else out
-        lse = torch.empty((B, H, Sq), dtype=torch.float32, device=q.device) if lse is None else lse
-        p = self._params(q, k, v, o, lse, scale, causal, keep_mask, kv_len, score_clamp, mode)
-        ws = self._attach_workspace(p, 0)
-        self.check(self.lib.ltca_attn_fwd(self.handle, C.byref(p)))
-        del ws
-        return o, lse
+        return self._host.attn_fwd(q, k, v, scale, causal, keep_mask, kv_len, score_clamp, mode, out, lse)
 
     def attn_bwd(self, q, k, v, o, lse, dout, scale=None, causal=False, keep_mask=None,
                  kv_len=None, score_clamp=0.0, mode=_lib.MODE_AUTO, dq=None, dk=None, dv=None,
                  deterministic=False):
         """dq, dk, dv.  ``deterministic=True`` asks for bit-identical results from run to run (bf16 storage on the
         tensor pipe otherwise takes the fused kernel, whose dq can differ between runs by fp32 rounding)."""
-        D = q.shape[3]
-        scale = 1.0 / math.sqrt(D) if scale is None else scale
-        dq = torch.empty(q.shape, dtype=q.dtype, device=q.device) if dq is None else dq
-        dk = torch.empty(k.shape, dtype=k.dtype, device=k.device) if dk is None else dk
-        dv = torch.empty(v.shape, dtype=v.dtype, device=v.device) if dv is None else dv
-        p = self._params(q, k, v, o, lse, scale, causal, keep_mask, kv_len, score_clamp, mode)
-        p.bwd_deterministic = int(bool(deterministic))
-        p.dout, p.do_strides = dout.data_ptr(), _strides(dout)
-        p.dq, p.dq_strides = dq.data_ptr(), _strides(dq)
-        p.dk, p.dk_strides = dk.data_ptr(), _strides(dk)
-        p.dv, p.dv_strides = dv.data_ptr(), _strides(dv)
-        ws = self._attach_workspace(p, 1)
-        self.check(self.lib.ltca_attn_bwd(self.handle, C.byref(p)))
-        del ws
-        return dq, dk, dv
+        return self._host.attn_bwd(q, k, v, o, lse, dout, scale, causal, keep_mask, kv_len, score_clamp, mode, dq, dk, dv,
+                                   deterministic)
 
     def attn_decode(self, q, k, v, kv_len=None, scale=None, keep_mask=None, score_clamp=0.0,
                     out=None, lse=None):
-        B, H, Sq, D = q.shape
-        scale = 1.0 / math.sqrt(D) if scale is None else scale
-        o = torch.empty((B, H, 1, D), dtype=q.dtype, device=q.device) if out is None else out
-        lse = torch.empty((B, H, 1), dtype=torch.float32, device=q.device) if lse is None else lse
-        p = self._params(q, k, v, o, lse, scale, False, keep_mask, kv_len, score_clamp, _lib.MODE_FP32)
-        need = C.c_size_t(0)
-        self.lib.ltca_attn_decode_workspace_bytes(C.byref(p), C.byref(need))
-        ws = self._attach_workspace(p, 0, fixed=need.value)
-        self.check(self.lib.ltca_attn_decode(self.handle, C.byref(p)))
-        del ws
-        return o, lse
+        return self._host.attn_decode(q, k, v, kv_len, scale, keep_mask, score_clamp, out, lse)
 
     # ---- sequence sharding: fold one key/value shard's result into running accumulators ----
     def attn_merge(self, o_acc, lse_acc, o_blk, lse_blk, s0=0):
@@ -247,42 +202,20 @@ class Context:
                                                  B * H, S, s0, part.shape[2], D))
 
     # ---- TimeSelfAttention module --------------------------------------------------------
-    def _tsa_params(self, x, wq, wk, wv, wo, B, S, H, head_width, scale, causal, time_major,
-                    use_residual, use_layer_norm, gamma, beta, keep_mask, mode, biases=(None, None, None, None)):
-        from ._lib import TsaParams
-        E = x.shape[1]
+    def _tsa_sizes(self, x, wq, wk, wv, wo, B, S, H, head_width, mode, causal):
+        """The parameter block of a size query."""
+        E, HW = x.shape[1], H * head_width
         assert x.shape == (B * S, E) and x.dtype == torch.float32 and x.is_contiguous()
-        HW = H * head_width
         assert wq.shape == (E, HW) and wk.shape == (E, HW) and wv.shape == (E, HW) and wo.shape == (HW, E)
         p = TsaParams()
         p.B, p.S, p.E, p.H, p.head_width = B, S, E, H, head_width
-        p.causal, p.time_major = int(bool(causal)), int(bool(time_major))
-        p.use_residual, p.use_layer_norm, p.mode = int(bool(use_residual)), int(bool(use_layer_norm)), int(mode)
-        p.scale, p.score_clamp = float(scale), 0.0
-        p.x = x.data_ptr()
-        p.wq, p.wk, p.wv, p.wo = (w.data_ptr() for w in (wq, wk, wv, wo))
-        if gamma is not None:
-            p.ln_gamma, p.ln_beta = gamma.data_ptr(), beta.data_ptr()
-        if keep_mask is not None:
-            p.keep_mask = keep_mask.data_ptr()
-        for name, b in zip(("bq", "bk", "bv", "bo"), biases):
-            if b is not None:
-                assert b.dtype == torch.float32 and b.is_contiguous()
-                setattr(p, name, b.data_ptr())
+        p.causal, p.mode, p.scale = int(bool(causal)), int(mode), 1.0
         return p
-
-    def _tsa_workspace(self, p, which):
-        need = C.c_size_t(0)
-        self.check(self.lib.ltca_tsa_workspace_bytes(C.byref(p), which, C.byref(need)))
-        ws = self.workspace(need.value)
-        p.workspace, p.workspace_bytes = ws.data_ptr(), ws.numel()
-        return ws
 
     def tsa_saved_buffer(self, x, wq, wk, wv, wo, B, S, H, head_width, mode=_lib.MODE_AUTO, causal=False):
         """A buffer for the forward's intermediates: give it to ``tsa_fwd(saved=...)`` and then to
         ``tsa_bwd(saved=..., reuse_forward=True)`` to skip the backward's recomputation of the forward."""
-        p = self._tsa_params(x, wq, wk, wv, wo, B, S, H, head_width, 1.0, causal, False, False, False, None, None,
-                             None, mode, (None, None, None, None))
+        p = self._tsa_sizes(x, wq, wk, wv, wo, B, S, H, head_width, mode, causal)
         need = C.c_size_t(0)
         self.check(self.lib.ltca_tsa_saved_bytes(C.byref(p), C.byref(need)))
         return torch.empty(need.value, dtype=torch.uint8, device=x.device)
@@ -290,97 +223,43 @@ class Context:
     def tsa_weight_cache(self, x, wq, wk, wv, wo, B, S, H, head_width, mode=_lib.MODE_AUTO, causal=False):
         """A buffer for the reduced-precision copies of the weights (``ltca_tsa_params.weight_cache``): pass it as
         ``weight_cache=(buffer, False)`` to the first call and ``(buffer, True)`` while the weights stay unchanged."""
-        p = self._tsa_params(x, wq, wk, wv, wo, B, S, H, head_width, 1.0, causal, False, False, False, None, None,
-                             None, mode, (None, None, None, None))
+        p = self._tsa_sizes(x, wq, wk, wv, wo, B, S, H, head_width, mode, causal)
         need = C.c_size_t(0)
         self.check(self.lib.ltca_tsa_weight_cache_bytes(C.byref(p), C.byref(need)))
         return torch.empty(max(need.value, 1), dtype=torch.uint8, device=x.device)
-
-    @staticmethod
-    def _attach_weight_cache(p, weight_cache):
-        if weight_cache is not None:
-            buf, valid = weight_cache
-            p.weight_cache, p.weight_cache_bytes, p.weight_cache_valid = buf.data_ptr(), buf.numel(), int(valid)
 
     def tsa_fwd(self, x, wq, wk, wv, wo, B, S, H, head_width, scale=1.0, causal=False, time_major=True,
                 use_residual=True, use_layer_norm=True, gamma=None, beta=None, keep_mask=None,
                 mode=_lib.MODE_AUTO, bq=None, bk=None, bv=None, bo=None, saved=None, weight_cache=None):
         """out = LayerNorm(x + MHA(x)); x [B*S, E] fp32, weights as in ``ltca_tsa_params``."""
-        p = self._tsa_params(x, wq, wk, wv, wo, B, S, H, head_width, scale, causal, time_major,
-                             use_residual, use_layer_norm, gamma, beta, keep_mask, mode, (bq, bk, bv, bo))
-        self._attach_weight_cache(p, weight_cache)
-        if saved is not None:
-            p.saved, p.saved_bytes = saved.data_ptr(), saved.numel()
-        out = torch.empty_like(x)
-        p.out = out.data_ptr()
-        ws = self._tsa_workspace(p, 0)
-        self.check(self.lib.ltca_tsa_fwd(self.handle, C.byref(p)))
-        del ws
-        return out
+        return self._host.tsa_fwd(x, wq, wk, wv, wo, B, S, H, head_width, scale, causal, time_major, use_residual,
+                                  use_layer_norm, gamma, beta, keep_mask, mode, bq, bk, bv, bo, saved, weight_cache)
 
     def tsa_bwd(self, x, wq, wk, wv, wo, dy, B, S, H, head_width, scale=1.0, causal=False, time_major=True,
                 keep_mask=None, mode=_lib.MODE_AUTO, bq=None, bk=None, bv=None, saved=None, reuse_forward=False,
                 weight_cache=None):
         """(dx, dwq, dwk, dwv, dwo) of the module; LayerNorm and residual pass dy through."""
-        p = self._tsa_params(x, wq, wk, wv, wo, B, S, H, head_width, scale, causal, time_major,
-                             False, False, None, None, keep_mask, mode, (bq, bk, bv, None))
-        self._attach_weight_cache(p, weight_cache)
-        if saved is not None:
-            p.saved, p.saved_bytes, p.reuse_forward = saved.data_ptr(), saved.numel(), int(reuse_forward)
-        dx = torch.empty_like(x)
-        # the four weight gradients are views of one allocation, so a multi-GPU caller sums them over the
-        # ranks with a single collective on that allocation (shard.sum_weight_grads) without packing them
-        flat = torch.empty(sum(w.numel() for w in (wq, wk, wv, wo)), dtype=wq.dtype, device=wq.device)
-        dws, off = [], 0
-        for w in (wq, wk, wv, wo):
-            dws.append(flat[off:off + w.numel()].view(w.shape))
-            off += w.numel()
-        p.dy, p.dx = dy.data_ptr(), dx.data_ptr()
-        p.dwq, p.dwk, p.dwv, p.dwo = (w.data_ptr() for w in dws)
-        ws = self._tsa_workspace(p, 3)
-        self.check(self.lib.ltca_tsa_bwd(self.handle, C.byref(p)))
-        del ws
-        return (dx, *dws)
+        # the four weight gradients are views of one allocation (shard.sum_weight_grads sums it with one collective)
+        return self._host.tsa_bwd(x, wq, wk, wv, wo, B, S, H, head_width, scale, causal, time_major, False, False, None,
+                                  None, keep_mask, mode, bq, bk, bv, None, dy, saved, reuse_forward, weight_cache)
 
     def fa_fwd(self, x, wq, wk, wv, wo, B, S, H, head_dim, biases=(None, None, None, None), gamma=None, beta=None,
                use_layer_norm=True, use_residual=True, keep_mask=None, dropout_prob=0.0, dropout_seed=0,
                score_clamp=10.0, mode=_lib.MODE_AUTO):
         """The reference's FlashAttention module: out = dropout(x + Wo MHA(LayerNorm(x)) + bo); x [B*S, E]
         batch-major rows, scale 1/sqrt(head_dim), score clamp 10."""
-        p = self._tsa_params(x, wq, wk, wv, wo, B, S, H, head_dim, 1.0 / math.sqrt(head_dim), False, False,
-                             use_residual, use_layer_norm, gamma, beta, keep_mask, mode, biases)
-        p.pre_norm, p.score_clamp = 1, float(score_clamp)
-        p.dropout_prob, p.dropout_seed = float(dropout_prob), int(dropout_seed)
-        out = torch.empty_like(x)
-        p.out = out.data_ptr()
-        ws = self._tsa_workspace(p, 0)
-        self.check(self.lib.ltca_tsa_fwd(self.handle, C.byref(p)))
-        del ws
-        return out
+        return self._host.fa_fwd(x, wq, wk, wv, wo, B, S, H, head_dim, 1.0 / math.sqrt(head_dim), False, False,
+                                 use_residual, use_layer_norm, gamma, beta, keep_mask, mode, *biases, dropout_prob,
+                                 dropout_seed, score_clamp)
 
     def fa_bwd(self, x, wq, wk, wv, wo, dy, B, S, H, head_dim, biases=(None, None, None, None), gamma=None,
                beta=None, use_layer_norm=True, use_residual=True, keep_mask=None, dropout_prob=0.0,
                dropout_seed=0, score_clamp=10.0, mode=_lib.MODE_AUTO):
         """Backward of fa_fwd (an extension: the reference class has none).  Returns a dict with dx, dwq, dwk,
         dwv, dwo, dbq, dbk, dbv, dbo and, with LayerNorm, dgamma and dbeta."""
-        p = self._tsa_params(x, wq, wk, wv, wo, B, S, H, head_dim, 1.0 / math.sqrt(head_dim), False, False,
-                             use_residual, use_layer_norm, gamma, beta, keep_mask, mode, biases)
-        p.pre_norm, p.score_clamp = 1, float(score_clamp)
-        p.dropout_prob, p.dropout_seed = float(dropout_prob), int(dropout_seed)
-        E, HW = x.shape[1], H * head_dim
-        f32 = dict(dtype=torch.float32, device=x.device)
-        g = dict(dx=torch.empty_like(x), dwq=torch.empty_like(wq), dwk=torch.empty_like(wk),
-                 dwv=torch.empty_like(wv), dwo=torch.empty_like(wo), dbq=torch.empty(HW, **f32),
-                 dbk=torch.empty(HW, **f32), dbv=torch.empty(HW, **f32), dbo=torch.empty(E, **f32))
-        if use_layer_norm:
-            g["dgamma"], g["dbeta"] = torch.empty(E, **f32), torch.empty(E, **f32)
-        p.dy = dy.data_ptr()
-        for name, t in g.items():
-            setattr(p, name, t.data_ptr())
-        ws = self._tsa_workspace(p, 3)
-        self.check(self.lib.ltca_tsa_bwd(self.handle, C.byref(p)))
-        del ws
-        return g
+        return self._host.fa_bwd(x, wq, wk, wv, wo, B, S, H, head_dim, 1.0 / math.sqrt(head_dim), False, False,
+                                 use_residual, use_layer_norm, gamma, beta, keep_mask, mode, *biases, dropout_prob,
+                                 dropout_seed, score_clamp, dy)
 
     def uses_tensor_pipe(self, q, k, v, causal=False, mode=_lib.MODE_AUTO, backward=False) -> bool:
         o = q

@@ -1,8 +1,9 @@
-"""Builds libltc_attn.so (the C-ABI library) in-tree with nvcc for sm_100a.
+"""Builds libltc_attn.so (the C-ABI library) in-tree with nvcc for sm_100a, and _host.so, the native half of the
+torch front end, with g++ against torch's headers.
 
 Run as ``python -m cuda_ltc_b200.build`` or call :func:`build_library`.  Objects go to
-``cuda_ltc_b200/build/`` and the library to ``cuda_ltc_b200/libltc_attn.so``; a source file is
-recompiled only when it or one of the headers is newer than its object.
+``cuda_ltc_b200/build/``, the libraries to ``cuda_ltc_b200/``; a source file is recompiled only when it
+or one of the headers is newer than its object.
 """
 from __future__ import annotations
 
@@ -10,10 +11,13 @@ import concurrent.futures as cf
 import os
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "libltc_attn.so")
+HOST_SRC = os.path.join(CSRC, "host_binding.cpp")
+HOST_OUT = os.path.join(HERE, "_host.so")
 OBJ_DIR = os.path.join(HERE, "build")
 
 NVCC_FLAGS = [
@@ -43,6 +47,24 @@ def _compile(src: str, obj: str) -> str:
     return log
 
 
+def _build_host(force: bool = False) -> None:
+    """_host.so finds libltc_attn.so beside itself; torch's libraries are already in a process that imports it."""
+    header = os.path.join(HERE, "..", "include", "ltc_attn.h")
+    if not force and os.path.exists(HOST_OUT) and os.path.getmtime(HOST_OUT) >= max(
+            os.path.getmtime(HOST_SRC), os.path.getmtime(header)):
+        return
+    import torch
+    from torch.utils import cpp_extension
+    lib_dir = os.path.join(os.path.dirname(torch.__file__), "lib")
+    includes = [*cpp_extension.include_paths(), sysconfig.get_paths()["include"], "/usr/local/cuda/include"]
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           *(f"-isystem{p}" for p in includes), HOST_SRC, "-o", HOST_OUT, f"-L{HERE}", "-l:libltc_attn.so",
+           "-Wl,-rpath,$ORIGIN", f"-L{lib_dir}", "-ltorch_python", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError("g++ failed for host_binding.cpp:\n" + r.stdout + r.stderr)
+
+
 def build_library(force: bool = False, verbose: bool = False) -> str:
     os.makedirs(OBJ_DIR, exist_ok=True)
     hdr_m = _headers_mtime()
@@ -63,6 +85,7 @@ def build_library(force: bool = False, verbose: bool = False) -> str:
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError("link failed:\n" + r.stdout + r.stderr)
+    _build_host(force)
     return OUT
 
 
