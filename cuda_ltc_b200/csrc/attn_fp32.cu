@@ -1,23 +1,21 @@
 // fp32 attention: the exact arithmetic mode (fp32 FMA, accurate expf) and the path for every
 // shape the tensor-pipe kernels do not take (any head_dim up to 512, dense keep-masks, tiny
-// sequences).  Forward, backward (two passes, no atomics, bit-reproducible) and the
-// row-statistics helper shared with the tensor-pipe backward.
+// sequences).  Forward and backward (two passes, no atomics, bit-reproducible).
 //
 // Replaces flashAttentionKernel (reference src/ml/flash_attention.cu:18-272) on its own valid
 // domain (head_dim <= 16, one key tile) and extends it to a true online softmax for longer
-// sequences; the 16x16-thread tiling keeps one query row inside a half-warp so that row maxima
+// sequences; the score tiles keep one query row inside a half-warp so that row maxima
 // and row sums are half-warp shuffle reductions.
 #include <math.h>
 
 #include "host_common.h"
+#include "sm100_ptx.cuh"
 
 namespace ltca {
 
 namespace {
 
-constexpr int kTM = 64;     // query rows per CTA
-constexpr int kTN = 64;     // keys per step
-constexpr int kThreads = 256;
+constexpr float kNegInf = -INFINITY;
 
 __device__ __forceinline__ float ld_elem(const float* p) { return __ldg(p); }
 __device__ __forceinline__ float ld_elem(const __nv_bfloat16* p) { return __bfloat162float(*p); }
@@ -37,28 +35,76 @@ struct CoreArgs {
     float* delta;
     const float* keep_mask;
     const int32_t* kv_len;
+    const uint32_t* mask_bits;  // backward: the dense mask packed, [B, Sq, mask_nw]
+    int mask_nw;
+    int vec;            // every row starts on a 16-byte (fp32) or 8-byte (bf16) boundary and holds a multiple of 4 elements
 };
 
-// Loads rows [r0, r0+64) x [0, D) of a [.., seq, D] tensor into smem [64][ld], zero padded.
-template <typename T>
-__device__ __forceinline__ void load_tile(float* dst, int ld, const T* base, int64_t row_stride,
-                                          int r0, int rows_total, int D) {
-    for (int idx = threadIdx.x; idx < kTM * D; idx += kThreads) {
-        const int r = idx / D, d = idx - r * D;
-        const int gr = r0 + r;
-        dst[r * ld + d] = (gr < rows_total) ? ld_elem(base + (int64_t)gr * row_stride + d) : 0.f;
-    }
+// ---- packed fp32 pairs --------------------------------------------------------------------------
+// One instruction multiplies and adds two pairs of fp32 values, each half rounded as fmaf rounds it.  The products of
+// these kernels are bound by issue slots (loads, masks and exponentials share them with the multiply-adds), so halving
+// the number of multiply-add instructions is worth the second accumulator.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ f32x2 pair(float x, float y) {
+    f32x2 d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(x), "f"(y));
+    return d;
+}
+__device__ __forceinline__ float2 halves(f32x2 v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
 }
 
-__device__ __forceinline__ float half_warp_max(float v) {
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
+// 16-byte asynchronous copy global -> shared; nothing is read and zeros are written when `bytes` is 0.
+__device__ __forceinline__ void cp_async16(float* dst, const void* src, int bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ float half_warp_sum(float v) {
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+__device__ __forceinline__ float4 ld4(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
+__device__ __forceinline__ float4 ld4(const __nv_bfloat16* p) {
+    const uint2 u = __ldg(reinterpret_cast<const uint2*>(p));
+    const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x));
+    const float2 y = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
+    return make_float4(x.x, x.y, y.x, y.y);
+}
+// Four elements of a row from column d on; zeros beyond D.
+template <typename T>
+__device__ __forceinline__ float4 row4(const T* row, int d, int D, bool vec) {
+    if (vec) return d < D ? ld4(row + d) : make_float4(0.f, 0.f, 0.f, 0.f);
+    return make_float4(d < D ? ld_elem(row + d) : 0.f, d + 1 < D ? ld_elem(row + d + 1) : 0.f,
+                       d + 2 < D ? ld_elem(row + d + 2) : 0.f, d + 3 < D ? ld_elem(row + d + 3) : 0.f);
+}
+template <typename T>
+__device__ __forceinline__ void store4(T* row, int d, int D, float4 v, bool vec) {
+    if (vec) {
+        if (d >= D) return;
+        if constexpr (sizeof(T) == 4) {
+            *reinterpret_cast<float4*>(row + d) = v;
+        } else {
+            const __nv_bfloat162 x = __floats2bfloat162_rn(v.x, v.y), y = __floats2bfloat162_rn(v.z, v.w);
+            *reinterpret_cast<uint2*>(row + d) =
+                make_uint2(*reinterpret_cast<const uint32_t*>(&x), *reinterpret_cast<const uint32_t*>(&y));
+        }
+    } else {
+        if (d < D) st_elem(row + d, v.x);
+        if (d + 1 < D) st_elem(row + d + 1, v.y);
+        if (d + 2 < D) st_elem(row + d + 2, v.z);
+        if (d + 3 < D) st_elem(row + d + 3, v.w);
+    }
 }
 
 __device__ __forceinline__ bool key_visible(const CoreArgs& a, int b, int qi, int kj, int kvlen) {
@@ -70,131 +116,347 @@ __device__ __forceinline__ bool key_visible(const CoreArgs& a, int b, int qi, in
 }
 
 // ----------------------------------------------------------------------------------------------
-// forward
-// thread (ty, tx) of a 16x16 grid owns query rows ty + 16 i and key columns tx + 16 j (i, j < 4)
-// in the score step, and output columns tx + 16 c (c < DC) in the value step.
+// Score tiles of 64 (16 for calls with few rows) query rows x 64 keys for head_dim up to 128.
+//
+// A thread multiplies a block of 8 rows x 4 columns of a score tile, P (and dS) go through shared memory into the
+// accumulating products, whose threads hold 4 neighbouring columns of several rows.  Both read their operands as 16-byte
+// vectors along the contraction: a quarter of the shared-memory instructions of one word per operand, which is what
+// bounded these kernels before (1 read per 2 multiply-adds; now 12 per 128 and 8 per 64).  The sums run in the
+// same order as with one word per read, so tiles of both heights and every launch width give the same bits.
+// Measured at B16 H8 S250 D32 with a dense mask: forward 93 -> 48 us, backward 305 -> 174 us; at D64 without a mask, both
+// 640 -> 336 us; the smallest calls (tiles of 16 rows) 10.7 -> 4 us.  What bounds them now is the issue rate: half of the
+// instructions are multiply-adds, the rest masks, exponentials and reads, at 12 to 16 warps per SM (registers).
+// One (query or key) row per lane group with the other side's rows broadcast from shared memory was built as well:
+// fewer instructions, but a broadcast 16-byte read takes two wavefronts and the row state leaves two or three warps per
+// scheduler; the same times within 5 % (without the mask forward 41 against 44 us, backward 167 against 162).
 // ----------------------------------------------------------------------------------------------
-template <typename T, int DC>
-__global__ void __launch_bounds__(kThreads) attn_fwd_fp32_kernel(const CoreArgs a) {
-    extern __shared__ float sm[];
-    const int D = a.D;
-    const int ld = D + 1;
-    float* Qs = sm;
-    float* Ks = Qs + kTM * ld;
-    float* Vs = Ks + kTN * ld;
-    float* Ps = Vs + kTN * ld;          // [64][65]
+constexpr int kPad = 4;      // floats added to a shared row: neighbouring rows' 16-byte pieces lie in different banks
 
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const int q0 = blockIdx.x * kTM;
+// Rows [r0, r0 + ROWS) into shared [ROWS][DP + kPad]; see load_tile.
+template <int DP, int ROWS, int NT, typename T>
+__device__ __forceinline__ void load_padded(float* dst, const T* base, int64_t row_stride, int r0, int rows_total, int D, bool vec) {
+    constexpr int C4 = DP / 4, LD = DP + kPad;
+#pragma unroll
+    for (int e0 = 0; e0 < ROWS * C4; e0 += NT) {
+        const int e = e0 + threadIdx.x;
+        if (ROWS * C4 % NT != 0 && e >= ROWS * C4) break;
+        const int r = e / C4, c = (e % C4) * 4;
+        const bool in = r0 + r < rows_total && c < D;
+        const T* src = base + (int64_t)(r0 + r) * row_stride;
+        if constexpr (sizeof(T) == 4) {
+            if (vec) {
+                cp_async16(dst + r * LD + c, in ? src + c : base, in ? 16 : 0);
+                continue;
+            }
+        }
+        *reinterpret_cast<float4*>(dst + r * LD + c) = in ? row4(src, c, D, vec) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+}
+
+// Thread layout of the score products: NT threads as (NT / 16) x 16.  Thread (ty, tx) owns columns tx + 16 j and rows
+// row_of(ty) + (NT / 16) i; the two rows that a warp holds per i lie four apart, which puts their words in different banks.
+__device__ __forceinline__ int row_of(int ty) { return ((ty >> 1) & 3) + 4 * (ty & 1) + 8 * (ty >> 3); }
+
+// s[i][j] = A[row i] . B[col j] over DP features
+template <int DP, int NT, int RM, int CN>
+__device__ __forceinline__ void tile_dot(float (&s)[RM][CN], const float* A, const float* B, int row0, int tx) {
+    constexpr int LD = DP + kPad, RS = NT / 16;
+#pragma unroll
+    for (int i = 0; i < RM; ++i)
+#pragma unroll
+        for (int j = 0; j < CN; ++j) s[i][j] = 0.f;
+#pragma unroll 2
+    for (int d = 0; d < DP; d += 4) {
+        float4 b[CN];
+#pragma unroll
+        for (int j = 0; j < CN; ++j) b[j] = *reinterpret_cast<const float4*>(B + (tx + 16 * j) * LD + d);
+#pragma unroll
+        for (int i = 0; i < RM; ++i) {
+            const float4 x = *reinterpret_cast<const float4*>(A + (row0 + RS * i) * LD + d);
+#pragma unroll
+            for (int j = 0; j < CN; ++j) {
+                s[i][j] = fmaf(x.x, b[j].x, s[i][j]);
+                s[i][j] = fmaf(x.y, b[j].y, s[i][j]);
+                s[i][j] = fmaf(x.z, b[j].z, s[i][j]);
+                s[i][j] = fmaf(x.w, b[j].w, s[i][j]);
+            }
+        }
+    }
+}
+
+// Thread layout of the accumulating products: a [ROWS, DP] result, 4 columns (8 at DP = 128: two groups 64 apart) and
+// NR rows per thread.
+template <int DP, int ROWS, int NT>
+struct AccLayout {
+    static constexpr int TX = DP < 64 ? DP / 4 : 16;            // threads across the columns
+    static constexpr int CG = DP / (4 * TX);                    // column groups of 4 per thread
+    static constexpr int TY = NT / TX < ROWS ? NT / TX : ROWS;  // threads down the rows (the others idle)
+    static constexpr int NR = ROWS / TY;
+    int tx, ty;
+    bool active;
+    __device__ __forceinline__ AccLayout() {
+        tx = threadIdx.x % TX;
+        ty = threadIdx.x / TX;
+        active = ty < TY;
+    }
+};
+// acc[row][cols] += sum over j < n of A[row][j] * V[j][cols], j ascending; A has row pitch LA, n is a multiple of 4 (zeros
+// beyond).
+template <int DP, int ROWS, int NT>
+__device__ __forceinline__ void accumulate(f32x2 (&acc)[AccLayout<DP, ROWS, NT>::NR][2 * AccLayout<DP, ROWS, NT>::CG],
+                                           const AccLayout<DP, ROWS, NT>& L, const float* A, int LA, const float* V, int n) {
+    using Lt = AccLayout<DP, ROWS, NT>;
+    constexpr int LD = DP + kPad;
+#pragma unroll 2
+    for (int j = 0; j < n; j += 4) {
+        float4 x[Lt::NR];
+#pragma unroll
+        for (int i = 0; i < Lt::NR; ++i) x[i] = *reinterpret_cast<const float4*>(A + (L.ty + Lt::TY * i) * LA + j);
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+#pragma unroll
+            for (int c = 0; c < Lt::CG; ++c) {
+                const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(V + (j + e) * LD + 4 * L.tx + 64 * c);
+#pragma unroll
+                for (int i = 0; i < Lt::NR; ++i) {
+                    const float w = e == 0 ? x[i].x : e == 1 ? x[i].y : e == 2 ? x[i].z : x[i].w;
+                    const f32x2 ww = pair(w, w);
+                    acc[i][2 * c] = fma2(ww, v.x, acc[i][2 * c]);
+                    acc[i][2 * c + 1] = fma2(ww, v.y, acc[i][2 * c + 1]);
+                }
+            }
+    }
+}
+template <int NR>
+__device__ __forceinline__ void ld_row(float (&x)[NR], const float* p) {       // NR consecutive floats of a shared row
+    if constexpr (NR % 4 == 0) {
+#pragma unroll
+        for (int i = 0; i < NR; i += 4) {
+            const float4 v = *reinterpret_cast<const float4*>(p + i);
+            x[i] = v.x; x[i + 1] = v.y; x[i + 2] = v.z; x[i + 3] = v.w;
+        }
+    } else if constexpr (NR == 2) {
+        const float2 v = *reinterpret_cast<const float2*>(p);
+        x[0] = v.x; x[1] = v.y;
+    } else {
+        x[0] = *p;
+    }
+}
+
+// Dense mask as bits: word (row, i) holds keys 32 i .. 32 i + 31 of a query row.  Both passes and all heads read the same
+// mask; packed once it is 1/32 of the traffic and one load for 32 keys.  One warp per word, coalesced reads and a vote.
+__global__ void __launch_bounds__(256) attn_mask_bits_kernel(const float* __restrict__ mask, uint32_t* __restrict__ words, int64_t rows,
+                                                             int Sk, int nw) {
+    grid_launch_dependents();
+    grid_dependency_wait();
+    const int lane = threadIdx.x & 31;
+    for (int64_t w = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); w < rows * nw; w += (int64_t)gridDim.x * 8) {
+        const int64_t r = w / nw;
+        const int k = (int)(w % nw) * 32 + lane;
+        const bool keep = k < Sk && __ldg(mask + r * Sk + k) != 0.f;
+        const uint32_t bits = __ballot_sync(0xffffffffu, keep);
+        if (lane == 0) words[w] = bits;
+    }
+}
+
+// Visibility of the CN columns k + 16 j of a row whose last visible key (without the mask) is `last`: bit j.
+template <int CN>
+__device__ __forceinline__ uint32_t row_limit(int k, int last) {
+    uint32_t bits = 0;
+#pragma unroll
+    for (int j = 0; j < CN; ++j) bits |= (k + 16 * j <= last ? 1u : 0u) << j;
+    return bits;
+}
+// The same columns of a row of mask bits (`words`: 32 keys each, from the tile's first key on).
+template <int CN>
+__device__ __forceinline__ uint32_t row_mask(const uint32_t* words, int tx) {
+    uint32_t bits = 0;
+#pragma unroll
+    for (int j = 0; j < CN; ++j) bits |= (words[j / 2] >> (tx + 16 * (j % 2)) & 1u) << j;
+    return bits;
+}
+__device__ __forceinline__ float half_warp_max(float v) {
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+__device__ __forceinline__ float half_warp_sum(float v) {
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// ----------------------------------------------------------------------------------------------
+// forward: one CTA per TM query rows of a (batch, head) pair, 64 keys per step
+//
+// K arrives for the next step under the value product, V under the next scores; several CTAs per SM cover the rest.
+// ----------------------------------------------------------------------------------------------
+template <typename T, int DP, int TM, int NT, bool kMask>
+__global__ void __launch_bounds__(NT, TM < 64 ? 4 : DP <= 32 ? 4 : DP <= 64 ? 3 : 1) attn_fwd_fp32_kernel(const CoreArgs a) {
+    grid_launch_dependents();
+    grid_dependency_wait();
+    constexpr int KN = 64, LD = DP + kPad, LP = KN + kPad, RS = NT / 16, RM = TM / RS, CN = KN / 16;
+    using Lt = AccLayout<DP, TM, NT>;
+    extern __shared__ __align__(16) float sm[];
+    float* Qs = sm;
+    float* Ks = Qs + TM * LD;
+    float* Vs = Ks + KN * LD;
+    float* Ps = Vs + KN * LD;
+    float* row_scale = Ps + TM * LP;     // [TM]: what the accumulator is multiplied with (step), 1 / sum (end)
+    const bool vec = a.vec != 0;
+
+    const int tx = threadIdx.x & 15, row0 = row_of(threadIdx.x >> 4);
+    const int q0 = blockIdx.x * TM;
     const int h = blockIdx.y, b = blockIdx.z;
     int kvlen = a.Sk;
     if (a.kv_len) kvlen = min(max(a.kv_len[b], 0), a.Sk);
+    int k_end = kvlen;
+    if (a.causal) k_end = min(k_end, min(q0 + TM - 1, a.Sq - 1) + a.causal_off + 1);
 
     const T* qb = reinterpret_cast<const T*>(a.q) + b * a.qs.batch + h * a.qs.head;
     const T* kb = reinterpret_cast<const T*>(a.k) + b * a.ks.batch + h * a.ks.head;
     const T* vb = reinterpret_cast<const T*>(a.v) + b * a.vs.batch + h * a.vs.head;
+    load_padded<DP, TM, NT>(Qs, qb, a.qs.seq, q0, a.Sq, a.D, vec);
+    load_padded<DP, KN, NT>(Ks, kb, a.ks.seq, 0, a.Sk, a.D, vec);
+    cp_async_commit();
+    load_padded<DP, KN, NT>(Vs, vb, a.vs.seq, 0, a.Sk, a.D, vec);
+    cp_async_commit();
 
-    load_tile(Qs, ld, qb, a.qs.seq, q0, a.Sq, D);
-
-    float m_run[4], l_run[4], acc[4][DC];
+    // Dense mask of this thread's scores: bit CN i + j for row i, column j.  The next step's values are read in two
+    // halves, one under each product, and packed behind it.
+    constexpr int RH = RM / 2;
+    static_assert(RM * CN <= 32 && RM % 2 == 0, "one word");
+    const float* mask = kMask ? a.keep_mask + ((int64_t)b * a.Sq + q0 + row0) * a.Sk + tx : nullptr;
+    float mv[RH][CN];
+    auto mask_read = [&](int half, int k) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        m_run[i] = -INFINITY;
-        l_run[i] = 0.f;
+        for (int i = 0; i < RH; ++i)
 #pragma unroll
-        for (int c = 0; c < DC; ++c) acc[i][c] = 0.f;
+            for (int j = 0; j < CN; ++j) {
+                const int r = RS * (half * RH + i);
+                mv[i][j] = (q0 + row0 + r < a.Sq && k + tx + 16 * j < k_end) ? __ldg(mask + (int64_t)r * a.Sk + k + 16 * j) : 0.f;
+            }
+    };
+    auto mask_pack = [&](int half) {
+        uint32_t bits = 0;
+#pragma unroll
+        for (int i = 0; i < RH; ++i)
+#pragma unroll
+            for (int j = 0; j < CN; ++j) bits |= (mv[i][j] != 0.f ? 1u : 0u) << (CN * (half * RH + i) + j);
+        return bits;
+    };
+    uint32_t keep = ~0u;
+    if (kMask) {
+        mask_read(0, 0);
+        keep = mask_pack(0);
+        mask_read(1, 0);
+        keep |= mask_pack(1);
     }
 
-    int k_end = kvlen;
-    if (a.causal) k_end = min(k_end, min(q0 + kTM - 1, a.Sq - 1) + a.causal_off + 1);
-    for (int k0 = 0; k0 < k_end; k0 += kTN) {
-        __syncthreads();
-        load_tile(Ks, ld, kb, a.ks.seq, k0, a.Sk, D);
-        load_tile(Vs, ld, vb, a.vs.seq, k0, a.Sk, D);
-        __syncthreads();
+    const Lt L;
+    float m_run[RM], l_run[RM];
+    f32x2 acc[Lt::NR][2 * Lt::CG];
+#pragma unroll
+    for (int i = 0; i < RM; ++i) { m_run[i] = kNegInf; l_run[i] = 0.f; }
+#pragma unroll
+    for (int i = 0; i < Lt::NR; ++i)
+#pragma unroll
+        for (int c = 0; c < 2 * Lt::CG; ++c) acc[i][c] = 0ull;
 
-        float s[4][4];
+    for (int k0 = 0; k0 < k_end; k0 += KN) {
+        const bool more = k0 + KN < k_end;
+        uint32_t keep_next = 0;
+        if (kMask && more) mask_read(0, k0 + KN);
+        cp_async_wait<1>();
+        __syncthreads();
+        float s[RM][CN];
+        tile_dot<DP, NT, RM, CN>(s, Qs, Ks, row0, tx);
+        if (kMask && more) keep_next = mask_pack(0);
+        const bool all_visible = k0 + KN <= kvlen && !kMask && (!a.causal || k0 + KN - 1 <= q0 + a.causal_off);
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < RM; ++i) {
+            const int r = row0 + RS * i;
+            uint32_t visible = ~0u;
+            if (!all_visible) {
+                const int last = a.causal ? min(kvlen - 1, q0 + r + a.causal_off) : kvlen - 1;
+                visible = row_limit<CN>(k0 + tx, last);
+                if (kMask) visible &= keep >> (CN * i);
+            }
+            float mt = kNegInf;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
-        for (int d = 0; d < D; ++d) {
-            float qv[4], kv[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) qv[i] = Qs[(ty + 16 * i) * ld + d];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) kv[j] = Ks[(tx + 16 * j) * ld + d];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) s[i][j] = fmaf(qv[i], kv[j], s[i][j]);
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int qi = q0 + ty + 16 * i;
-            float mt = -INFINITY;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int kj = k0 + tx + 16 * j;
+            for (int j = 0; j < CN; ++j) {
                 float v = s[i][j] * a.scale;
                 if (a.use_clamp) v = fminf(v, a.clamp);
-                if (!key_visible(a, b, qi, kj, kvlen)) v = -INFINITY;
+                if (!(visible >> j & 1u)) v = kNegInf;
                 s[i][j] = v;
                 mt = fmaxf(mt, v);
             }
             mt = half_warp_max(mt);
             const float m_new = fmaxf(m_run[i], mt);
-            const float m_safe = (m_new == -INFINITY) ? 0.f : m_new;
-            const float corr = (m_run[i] == -INFINITY) ? 0.f : expf(m_run[i] - m_safe);
+            const float m_safe = (m_new == kNegInf) ? 0.f : m_new;
+            const float corr = (m_run[i] == kNegInf) ? 0.f : expf(m_run[i] - m_safe);
             float rs = 0.f;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
+            for (int j = 0; j < CN; ++j) {
                 const float p = expf(s[i][j] - m_safe);      // exp(-inf) = 0 for hidden keys
-                Ps[(ty + 16 * i) * (kTN + 1) + tx + 16 * j] = p;
+                Ps[r * LP + tx + 16 * j] = p;
                 rs += p;
             }
             rs = half_warp_sum(rs);
             l_run[i] = l_run[i] * corr + rs;
             m_run[i] = m_new;
-#pragma unroll
-            for (int c = 0; c < DC; ++c) acc[i][c] *= corr;
+            if (tx == 0) row_scale[r] = corr;
         }
+        if (kMask && more) mask_read(1, k0 + KN);
+        cp_async_wait<0>();
         __syncthreads();
-        for (int j = 0; j < kTN; ++j) {
-            float pv[4], vv[DC];
+        if (more) load_padded<DP, KN, NT>(Ks, kb, a.ks.seq, k0 + KN, a.Sk, a.D, vec);
+        cp_async_commit();
+        if (L.active) {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) pv[i] = Ps[(ty + 16 * i) * (kTN + 1) + j];
+            for (int i = 0; i < Lt::NR; ++i) {
+                const float corr = row_scale[L.ty + Lt::TY * i];
+                const f32x2 cc = pair(corr, corr);
 #pragma unroll
-            for (int c = 0; c < DC; ++c) {
-                const int d = tx + 16 * c;
-                vv[c] = (d < D) ? Vs[j * ld + d] : 0.f;
+                for (int c = 0; c < 2 * Lt::CG; ++c) acc[i][c] = mul2(acc[i][c], cc);
             }
+            accumulate<DP, TM, NT>(acc, L, Ps, LP, Vs, min(KN, (k_end - k0 + 3) & ~3));
+        }
+        if (kMask && more) keep = keep_next | mask_pack(1);
+        __syncthreads();
+        if (more) load_padded<DP, KN, NT>(Vs, vb, a.vs.seq, k0 + KN, a.Sk, a.D, vec);
+        cp_async_commit();
+    }
+    cp_async_wait<0>();
+
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int c = 0; c < DC; ++c) acc[i][c] = fmaf(pv[i], vv[c], acc[i][c]);
+    for (int i = 0; i < RM; ++i) {
+        const int r = row0 + RS * i, qi = q0 + r;
+        if (tx == 0) {
+            row_scale[r] = l_run[i] > 0.f ? 1.f / l_run[i] : 0.f;
+            if (a.lse && qi < a.Sq)
+                a.lse[((int64_t)b * a.H + h) * a.Sq + qi] = l_run[i] > 0.f ? m_run[i] + logf(l_run[i]) : kNegInf;
         }
     }
-
+    __syncthreads();
+    if (!L.active) return;
     T* ob = reinterpret_cast<T*>(a.o) + b * a.os.batch + h * a.os.head;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int qi = q0 + ty + 16 * i;
-        if (qi >= a.Sq) continue;
-        const float inv = l_run[i] > 0.f ? 1.f / l_run[i] : 0.f;
+    for (int i = 0; i < Lt::NR; ++i) {
+        const int r = L.ty + Lt::TY * i;
+        if (q0 + r >= a.Sq) continue;
+        const float inv = row_scale[r];
 #pragma unroll
-        for (int c = 0; c < DC; ++c) {
-            const int d = tx + 16 * c;
-            if (d < D) st_elem(ob + (int64_t)qi * a.os.seq + d, acc[i][c] * inv);
+        for (int c = 0; c < Lt::CG; ++c) {
+            const float2 x = halves(acc[i][2 * c]), y = halves(acc[i][2 * c + 1]);
+            store4(ob + (int64_t)(q0 + r) * a.os.seq, 4 * L.tx + 64 * c, a.D, make_float4(x.x * inv, x.y * inv, y.x * inv, y.y * inv),
+                   vec);
         }
-        if (a.lse && tx == 0)
-            a.lse[((int64_t)b * a.H + h) * a.Sq + qi] =
-                l_run[i] > 0.f ? m_run[i] + logf(l_run[i]) : -INFINITY;
     }
 }
 
 // ----------------------------------------------------------------------------------------------
-// backward helper: delta[b,h,i] = sum_d dO[i,d] * O[i,d]   (one warp per query row)
+// backward helper of the wide-head kernels: delta[b,h,i] = sum_d dO[i,d] * O[i,d]   (one warp per query row)
 // ----------------------------------------------------------------------------------------------
 template <typename T>
 __global__ void attn_bwd_delta_kernel(const CoreArgs a) {
@@ -216,21 +478,26 @@ __global__ void attn_bwd_delta_kernel(const CoreArgs a) {
 }
 
 // ----------------------------------------------------------------------------------------------
-// backward, pass 1: dQ.  One CTA per 64 query rows; loops over key tiles.
+// backward
 // ----------------------------------------------------------------------------------------------
-template <typename T, int DC>
-__global__ void __launch_bounds__(kThreads) attn_bwd_dq_fp32_kernel(const CoreArgs a) {
-    extern __shared__ float sm[];
-    const int D = a.D;
-    const int ld = D + 1;
+// pass 1: delta = rowsum(dO o O), left for pass 2, and dQ.  One CTA per TM query rows, KN keys per step.
+template <typename T, int DP, int TM, int KN, int NT, bool kMask>
+__global__ void __launch_bounds__(NT, NT == 128 ? 3 : 1) attn_bwd_dq_fp32_kernel(const CoreArgs a) {
+    grid_launch_dependents();
+    grid_dependency_wait();
+    constexpr int LD = DP + kPad, LP = KN + kPad, RS = NT / 16, RM = TM / RS, CN = KN / 16, NW = KN / 32;
+    using Lt = AccLayout<DP, TM, NT>;
+    extern __shared__ __align__(16) float sm[];
     float* Qs = sm;
-    float* Gs = Qs + kTM * ld;          // dO
-    float* Ks = Gs + kTM * ld;
-    float* Vs = Ks + kTN * ld;
-    float* Ss = Vs + kTN * ld;          // dS [64][65]
+    float* Gs = Qs + TM * LD;            // dO
+    float* Ks = Gs + TM * LD;
+    float* Vs = Ks + KN * LD;
+    float* Ss = Vs + KN * LD;            // dS
+    float* row_delta = Ss + TM * LP;
+    const bool vec = a.vec != 0;
 
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const int q0 = blockIdx.x * kTM;
+    const int tx = threadIdx.x & 15, row0 = row_of(threadIdx.x >> 4);
+    const int q0 = blockIdx.x * TM;
     const int h = blockIdx.y, b = blockIdx.z;
     int kvlen = a.Sk;
     if (a.kv_len) kvlen = min(max(a.kv_len[b], 0), a.Sk);
@@ -239,116 +506,131 @@ __global__ void __launch_bounds__(kThreads) attn_bwd_dq_fp32_kernel(const CoreAr
     const T* kb = reinterpret_cast<const T*>(a.k) + b * a.ks.batch + h * a.ks.head;
     const T* vb = reinterpret_cast<const T*>(a.v) + b * a.vs.batch + h * a.vs.head;
     const T* gb = reinterpret_cast<const T*>(a.dout) + b * a.dos.batch + h * a.dos.head;
-    load_tile(Qs, ld, qb, a.qs.seq, q0, a.Sq, D);
-    load_tile(Gs, ld, gb, a.dos.seq, q0, a.Sq, D);
+    const T* ob = reinterpret_cast<const T*>(a.o_in) + b * a.os.batch + h * a.os.head;
+    load_padded<DP, TM, NT>(Qs, qb, a.qs.seq, q0, a.Sq, a.D, vec);
+    load_padded<DP, TM, NT>(Gs, gb, a.dos.seq, q0, a.Sq, a.D, vec);
+    load_padded<DP, KN, NT>(Ks, kb, a.ks.seq, 0, a.Sk, a.D, vec);
+    load_padded<DP, KN, NT>(Vs, vb, a.vs.seq, 0, a.Sk, a.D, vec);
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncthreads();
 
-    float lse[4], dlt[4], acc[4][DC];
+    const int64_t stat0 = ((int64_t)b * a.H + h) * a.Sq;
+    // one warp per row, as the wide-head kernels form it
+    for (int r = threadIdx.x >> 5; r < TM; r += NT / 32) {
+        float d = 0.f;
+        if (q0 + r < a.Sq) {
+            const T* orow = ob + (int64_t)(q0 + r) * a.os.seq;
+            for (int c = threadIdx.x & 31; c < a.D; c += 32) d = fmaf(ld_elem(orow + c), Gs[r * LD + c], d);
+        }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int qi = q0 + ty + 16 * i;
-        const int64_t r = ((int64_t)b * a.H + h) * a.Sq + qi;
-        lse[i] = qi < a.Sq ? a.lse_in[r] : -INFINITY;
-        dlt[i] = qi < a.Sq ? a.delta[r] : 0.f;
-#pragma unroll
-        for (int c = 0; c < DC; ++c) acc[i][c] = 0.f;
+        for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+        if ((threadIdx.x & 31) == 0) {
+            row_delta[r] = d;
+            if (q0 + r < a.Sq) a.delta[stat0 + q0 + r] = d;
+        }
     }
+    __syncthreads();
+
+    const Lt L;
+    // A row without visible keys (lse = -inf) and rows beyond the tensor take lse = +inf: their probabilities are 0.
+    float lse[RM], dlt[RM];
+    f32x2 acc[Lt::NR][2 * Lt::CG];
+#pragma unroll
+    for (int i = 0; i < RM; ++i) {
+        const int r = row0 + RS * i;
+        const float l = q0 + r < a.Sq ? a.lse_in[stat0 + q0 + r] : kNegInf;
+        lse[i] = l == kNegInf ? INFINITY : l;
+        dlt[i] = row_delta[r];
+    }
+#pragma unroll
+    for (int i = 0; i < Lt::NR; ++i)
+#pragma unroll
+        for (int c = 0; c < 2 * Lt::CG; ++c) acc[i][c] = 0ull;
 
     int k_end = kvlen;
-    if (a.causal) k_end = min(k_end, min(q0 + kTM - 1, a.Sq - 1) + a.causal_off + 1);
-    for (int k0 = 0; k0 < k_end; k0 += kTN) {
-        __syncthreads();
-        load_tile(Ks, ld, kb, a.ks.seq, k0, a.Sk, D);
-        load_tile(Vs, ld, vb, a.vs.seq, k0, a.Sk, D);
-        __syncthreads();
-        float s[4][4], dp[4][4];
+    if (a.causal) k_end = min(k_end, min(q0 + TM - 1, a.Sq - 1) + a.causal_off + 1);
+    for (int k0 = 0; k0 < k_end; k0 += KN) {
+        if (k0 > 0) {
+            cp_async_wait<0>();
+            __syncthreads();
+        }
+        uint32_t words[RM][NW];
+        if (kMask) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+            for (int i = 0; i < RM; ++i)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) { s[i][j] = 0.f; dp[i][j] = 0.f; }
-        for (int d = 0; d < D; ++d) {
-            float qv[4], gv[4], kv[4], vv[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                qv[i] = Qs[(ty + 16 * i) * ld + d];
-                gv[i] = Gs[(ty + 16 * i) * ld + d];
-            }
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                kv[j] = Ks[(tx + 16 * j) * ld + d];
-                vv[j] = Vs[(tx + 16 * j) * ld + d];
-            }
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    s[i][j] = fmaf(qv[i], kv[j], s[i][j]);
-                    dp[i][j] = fmaf(gv[i], vv[j], dp[i][j]);
+                for (int w = 0; w < NW; ++w) {
+                    const int qi = q0 + row0 + RS * i, kw = k0 / 32 + w;
+                    words[i][w] = (qi < a.Sq && kw < a.mask_nw) ? a.mask_bits[((int64_t)b * a.Sq + qi) * a.mask_nw + kw] : 0u;
                 }
         }
+        float s[RM][CN], dp[RM][CN];
+        tile_dot<DP, NT, RM, CN>(s, Qs, Ks, row0, tx);
+        tile_dot<DP, NT, RM, CN>(dp, Gs, Vs, row0, tx);
+        const bool all_visible = k0 + KN <= kvlen && !kMask && (!a.causal || k0 + KN - 1 <= q0 + a.causal_off);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int qi = q0 + ty + 16 * i;
+        for (int i = 0; i < RM; ++i) {
+            const int r = row0 + RS * i;
+            uint32_t visible = ~0u;
+            if (!all_visible) {
+                const int last = a.causal ? min(kvlen - 1, q0 + r + a.causal_off) : kvlen - 1;
+                visible = row_limit<CN>(k0 + tx, last);
+                if (kMask) visible &= row_mask<CN>(words[i], tx);
+            }
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int kj = k0 + tx + 16 * j;
+            for (int j = 0; j < CN; ++j) {
                 float v = s[i][j] * a.scale;
-                bool clamped = false;
-                if (a.use_clamp && v >= a.clamp) { v = a.clamp; clamped = true; }
-                float ds = 0.f;
-                if (key_visible(a, b, qi, kj, kvlen) && lse[i] != -INFINITY) {
-                    const float p = expf(v - lse[i]);
-                    ds = clamped ? 0.f : p * (dp[i][j] - dlt[i]) * a.scale;
-                }
-                Ss[(ty + 16 * i) * (kTN + 1) + tx + 16 * j] = ds;
+                bool zero = !(visible >> j & 1u);
+                if (a.use_clamp && v >= a.clamp) { v = a.clamp; zero = true; }     // the gradient of a clamped score
+                const float p = expf(v - lse[i]);
+                Ss[r * LP + tx + 16 * j] = zero ? 0.f : p * (dp[i][j] - dlt[i]) * a.scale;
             }
         }
         __syncthreads();
-        for (int j = 0; j < kTN; ++j) {
-            float pv[4], kk[DC];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) pv[i] = Ss[(ty + 16 * i) * (kTN + 1) + j];
-#pragma unroll
-            for (int c = 0; c < DC; ++c) {
-                const int d = tx + 16 * c;
-                kk[c] = (d < D) ? Ks[j * ld + d] : 0.f;
-            }
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int c = 0; c < DC; ++c) acc[i][c] = fmaf(pv[i], kk[c], acc[i][c]);
-        }
+        const bool more = k0 + KN < k_end;
+        if (more) load_padded<DP, KN, NT>(Vs, vb, a.vs.seq, k0 + KN, a.Sk, a.D, vec);
+        cp_async_commit();
+        if (L.active) accumulate<DP, TM, NT>(acc, L, Ss, LP, Ks, min(KN, (k_end - k0 + 3) & ~3));   // columns beyond k_end are 0
+        __syncthreads();
+        if (more) load_padded<DP, KN, NT>(Ks, kb, a.ks.seq, k0 + KN, a.Sk, a.D, vec);
+        cp_async_commit();
     }
+    cp_async_wait<0>();
+    if (!L.active) return;
     T* dqb = reinterpret_cast<T*>(a.dq) + b * a.dqs.batch + h * a.dqs.head;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int qi = q0 + ty + 16 * i;
-        if (qi >= a.Sq) continue;
+    for (int i = 0; i < Lt::NR; ++i) {
+        const int r = L.ty + Lt::TY * i;
+        if (q0 + r >= a.Sq) continue;
 #pragma unroll
-        for (int c = 0; c < DC; ++c) {
-            const int d = tx + 16 * c;
-            if (d < D) st_elem(dqb + (int64_t)qi * a.dqs.seq + d, acc[i][c]);
+        for (int c = 0; c < Lt::CG; ++c) {
+            const float2 x = halves(acc[i][2 * c]), y = halves(acc[i][2 * c + 1]);
+            store4(dqb + (int64_t)(q0 + r) * a.dqs.seq, 4 * L.tx + 64 * c, a.D, make_float4(x.x, x.y, y.x, y.y), vec);
         }
     }
 }
 
-// ----------------------------------------------------------------------------------------------
-// backward, pass 2: dK and dV.  One CTA per 64 keys; loops over query tiles.
-// In the accumulation step thread (ty, tx) owns key rows ty + 16 i and feature columns tx + 16 c.
-// ----------------------------------------------------------------------------------------------
-template <typename T, int DC>
-__global__ void __launch_bounds__(kThreads) attn_bwd_dkv_fp32_kernel(const CoreArgs a) {
-    extern __shared__ float sm[];
-    const int D = a.D;
-    const int ld = D + 1;
-    float* Qs = sm;
-    float* Gs = Qs + kTM * ld;
-    float* Ks = Gs + kTM * ld;
-    float* Vs = Ks + kTN * ld;
-    float* Ps = Vs + kTN * ld;                  // P  [64 q][65]
-    float* Ss = Ps + kTM * (kTN + 1);           // dS [64 q][65]
+// pass 2: dK and dV.  One CTA per TK keys, QN query rows per step; a thread accumulates NR neighbouring keys.
+template <typename T, int DP, int TK, int QN, int NT, bool kMask>
+__global__ void __launch_bounds__(NT, TK < 64 ? 3 : DP <= 32 ? 3 : DP <= 64 ? 2 : 1) attn_bwd_dkv_fp32_kernel(const CoreArgs a) {
+    grid_launch_dependents();
+    grid_dependency_wait();
+    constexpr int LD = DP + kPad, LP = TK + kPad, RS = NT / 16, RM = QN / RS, CN = TK / 16, NW = (TK + 31) / 32;
+    using Lt = AccLayout<DP, TK, NT>;
+    extern __shared__ __align__(16) float sm[];
+    float* Ks = sm;
+    float* Vs = Ks + TK * LD;
+    float* Qs = Vs + TK * LD;
+    float* Gs = Qs + QN * LD;
+    float* Ps = Gs + QN * LD;            // P  [QN][LP]
+    float* Ss = Ps + QN * LP;            // dS [QN][LP]
+    float* row_lse = Ss + QN * LP;
+    float* row_delta = row_lse + QN;
+    const bool vec = a.vec != 0;
 
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const int k0 = blockIdx.x * kTN;
+    const int tx = threadIdx.x & 15, row0 = row_of(threadIdx.x >> 4);
+    const int k0 = blockIdx.x * TK;
     const int h = blockIdx.y, b = blockIdx.z;
     int kvlen = a.Sk;
     if (a.kv_len) kvlen = min(max(a.kv_len[b], 0), a.Sk);
@@ -357,109 +639,109 @@ __global__ void __launch_bounds__(kThreads) attn_bwd_dkv_fp32_kernel(const CoreA
     const T* kb = reinterpret_cast<const T*>(a.k) + b * a.ks.batch + h * a.ks.head;
     const T* vb = reinterpret_cast<const T*>(a.v) + b * a.vs.batch + h * a.vs.head;
     const T* gb = reinterpret_cast<const T*>(a.dout) + b * a.dos.batch + h * a.dos.head;
-    load_tile(Ks, ld, kb, a.ks.seq, k0, a.Sk, D);
-    load_tile(Vs, ld, vb, a.vs.seq, k0, a.Sk, D);
+    load_padded<DP, TK, NT>(Ks, kb, a.ks.seq, k0, a.Sk, a.D, vec);
+    load_padded<DP, TK, NT>(Vs, vb, a.vs.seq, k0, a.Sk, a.D, vec);
 
-    float acck[4][DC], accv[4][DC];
+    const Lt L;
+    f32x2 acck[Lt::NR][2 * Lt::CG], accv[Lt::NR][2 * Lt::CG];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < Lt::NR; ++i)
 #pragma unroll
-        for (int c = 0; c < DC; ++c) { acck[i][c] = 0.f; accv[i][c] = 0.f; }
+        for (int c = 0; c < 2 * Lt::CG; ++c) { acck[i][c] = 0ull; accv[i][c] = 0ull; }
 
+    const int64_t stat0 = ((int64_t)b * a.H + h) * a.Sq;
     // first query row that can see key k0 (causal): qi >= k0 - causal_off
     int q_begin = 0;
-    if (a.causal) q_begin = max(0, k0 - a.causal_off) / kTM * kTM;
+    if (a.causal) q_begin = max(0, k0 - a.causal_off) / QN * QN;
     const bool tile_live = k0 < kvlen;
-    for (int q0 = q_begin; q0 < a.Sq && tile_live; q0 += kTM) {
-        __syncthreads();
-        load_tile(Qs, ld, qb, a.qs.seq, q0, a.Sq, D);
-        load_tile(Gs, ld, gb, a.dos.seq, q0, a.Sq, D);
-        __syncthreads();
-        float s[4][4], dp[4][4];
+    for (int q0 = q_begin; q0 < a.Sq && tile_live; q0 += QN) {
+        load_padded<DP, QN, NT>(Qs, qb, a.qs.seq, q0, a.Sq, a.D, vec);
+        load_padded<DP, QN, NT>(Gs, gb, a.dos.seq, q0, a.Sq, a.D, vec);
+        cp_async_commit();
+        if (threadIdx.x < QN) {
+            // rows without visible keys and rows beyond the tensor: lse = +inf, probabilities 0
+            const int qi = q0 + threadIdx.x;
+            const float l = qi < a.Sq ? a.lse_in[stat0 + qi] : kNegInf;
+            row_lse[threadIdx.x] = l == kNegInf ? INFINITY : l;
+            row_delta[threadIdx.x] = qi < a.Sq ? a.delta[stat0 + qi] : 0.f;
+        }
+        uint32_t words[RM][NW];
+        if (kMask) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+            for (int i = 0; i < RM; ++i)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) { s[i][j] = 0.f; dp[i][j] = 0.f; }
-        for (int d = 0; d < D; ++d) {
-            float qv[4], gv[4], kv[4], vv[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                qv[i] = Qs[(ty + 16 * i) * ld + d];
-                gv[i] = Gs[(ty + 16 * i) * ld + d];
-            }
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                kv[j] = Ks[(tx + 16 * j) * ld + d];
-                vv[j] = Vs[(tx + 16 * j) * ld + d];
-            }
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    s[i][j] = fmaf(qv[i], kv[j], s[i][j]);
-                    dp[i][j] = fmaf(gv[i], vv[j], dp[i][j]);
+                for (int w = 0; w < NW; ++w) {
+                    const int qi = q0 + row0 + RS * i, kw = k0 / 32 + w;
+                    uint32_t x = (qi < a.Sq && kw < a.mask_nw) ? a.mask_bits[((int64_t)b * a.Sq + qi) * a.mask_nw + kw] : 0u;
+                    words[i][w] = TK < 32 ? x >> (k0 % 32) : x;
                 }
         }
+        cp_async_wait<0>();
+        __syncthreads();
+        float s[RM][CN], dp[RM][CN];
+        tile_dot<DP, NT, RM, CN>(s, Qs, Ks, row0, tx);
+        tile_dot<DP, NT, RM, CN>(dp, Gs, Vs, row0, tx);
+        const bool all_visible = k0 + TK <= kvlen && !kMask && (!a.causal || k0 + TK - 1 <= q0 + a.causal_off);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int qi = q0 + ty + 16 * i;
-            float lse = -INFINITY, dlt = 0.f;
-            if (qi < a.Sq) {
-                const int64_t r = ((int64_t)b * a.H + h) * a.Sq + qi;
-                lse = a.lse_in[r];
-                dlt = a.delta[r];
+        for (int i = 0; i < RM; ++i) {
+            const int r = row0 + RS * i;
+            const float lse = row_lse[r], dlt = row_delta[r];
+            uint32_t visible = ~0u;
+            if (!all_visible) {
+                const int last = a.causal ? min(kvlen - 1, q0 + r + a.causal_off) : kvlen - 1;
+                visible = row_limit<CN>(k0 + tx, last);
+                if (kMask) visible &= row_mask<CN>(words[i], tx);
             }
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int kj = k0 + tx + 16 * j;
+            for (int j = 0; j < CN; ++j) {
                 float v = s[i][j] * a.scale;
                 bool clamped = false;
                 if (a.use_clamp && v >= a.clamp) { v = a.clamp; clamped = true; }
-                float p = 0.f, ds = 0.f;
-                if (qi < a.Sq && key_visible(a, b, qi, kj, kvlen) && lse != -INFINITY) {
-                    p = expf(v - lse);
-                    ds = clamped ? 0.f : p * (dp[i][j] - dlt) * a.scale;
-                }
-                Ps[(ty + 16 * i) * (kTN + 1) + tx + 16 * j] = p;
-                Ss[(ty + 16 * i) * (kTN + 1) + tx + 16 * j] = ds;
+                float p = expf(v - lse);
+                if (!(visible >> j & 1u)) p = 0.f;
+                Ps[r * LP + tx + 16 * j] = p;
+                Ss[r * LP + tx + 16 * j] = clamped ? 0.f : p * (dp[i][j] - dlt) * a.scale;
             }
         }
         __syncthreads();
-        for (int r = 0; r < kTM; ++r) {
-            float pp[4], dd[4], gg[DC], qq[DC];
+        if (L.active) {
+            const int n = min(QN, a.Sq - q0);
+#pragma unroll 4
+            for (int r = 0; r < n; ++r) {
+                float pp[Lt::NR], dd[Lt::NR];
+                ld_row<Lt::NR>(pp, Ps + r * LP + Lt::NR * L.ty);
+                ld_row<Lt::NR>(dd, Ss + r * LP + Lt::NR * L.ty);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                pp[i] = Ps[r * (kTN + 1) + ty + 16 * i];
-                dd[i] = Ss[r * (kTN + 1) + ty + 16 * i];
-            }
+                for (int c = 0; c < Lt::CG; ++c) {
+                    const ulonglong2 g = *reinterpret_cast<const ulonglong2*>(Gs + r * LD + 4 * L.tx + 64 * c);
+                    const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(Qs + r * LD + 4 * L.tx + 64 * c);
 #pragma unroll
-            for (int c = 0; c < DC; ++c) {
-                const int d = tx + 16 * c;
-                gg[c] = (d < D) ? Gs[r * ld + d] : 0.f;
-                qq[c] = (d < D) ? Qs[r * ld + d] : 0.f;
-            }
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int c = 0; c < DC; ++c) {
-                    accv[i][c] = fmaf(pp[i], gg[c], accv[i][c]);
-                    acck[i][c] = fmaf(dd[i], qq[c], acck[i][c]);
+                    for (int i = 0; i < Lt::NR; ++i) {
+                        const f32x2 pw = pair(pp[i], pp[i]), dw = pair(dd[i], dd[i]);
+                        accv[i][2 * c] = fma2(pw, g.x, accv[i][2 * c]);
+                        accv[i][2 * c + 1] = fma2(pw, g.y, accv[i][2 * c + 1]);
+                        acck[i][2 * c] = fma2(dw, q.x, acck[i][2 * c]);
+                        acck[i][2 * c + 1] = fma2(dw, q.y, acck[i][2 * c + 1]);
+                    }
                 }
+            }
         }
+        __syncthreads();
     }
+    cp_async_wait<0>();
+    if (!L.active) return;
     T* dkb = reinterpret_cast<T*>(a.dk) + b * a.dks.batch + h * a.dks.head;
     T* dvb = reinterpret_cast<T*>(a.dv) + b * a.dvs.batch + h * a.dvs.head;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int kj = k0 + ty + 16 * i;
+    for (int i = 0; i < Lt::NR; ++i) {
+        const int kj = k0 + Lt::NR * L.ty + i;
         if (kj >= a.Sk) continue;
 #pragma unroll
-        for (int c = 0; c < DC; ++c) {
-            const int d = tx + 16 * c;
-            if (d < D) {
-                st_elem(dkb + (int64_t)kj * a.dks.seq + d, acck[i][c]);
-                st_elem(dvb + (int64_t)kj * a.dvs.seq + d, accv[i][c]);
-            }
+        for (int c = 0; c < Lt::CG; ++c) {
+            const float2 x = halves(acck[i][2 * c]), y = halves(acck[i][2 * c + 1]);
+            const float2 u = halves(accv[i][2 * c]), w = halves(accv[i][2 * c + 1]);
+            store4(dkb + (int64_t)kj * a.dks.seq, 4 * L.tx + 64 * c, a.D, make_float4(x.x, x.y, y.x, y.y), vec);
+            store4(dvb + (int64_t)kj * a.dvs.seq, 4 * L.tx + 64 * c, a.D, make_float4(u.x, u.y, w.x, w.y), vec);
         }
     }
 }
@@ -480,58 +762,78 @@ CoreArgs make_args(const ltca_attn_params* p) {
     a.lse = p->lse; a.lse_in = p->lse;
     a.keep_mask = p->keep_mask;
     a.kv_len = p->kv_len;
+    const int es = elem_size(p->dtype);
+    bool vec = p->D % 4 == 0;
+    auto rows = [&](const void* ptr, const ltca_strides& st) {
+        if (!ptr) return;
+        if ((reinterpret_cast<uintptr_t>(ptr) % (4 * es)) || (st.seq % 4) || (st.head % 4) || (st.batch % 4)) vec = false;
+    };
+    rows(a.q, a.qs); rows(a.k, a.ks); rows(a.v, a.vs); rows(a.o, a.os);
+    rows(a.dout, a.dos); rows(a.dq, a.dqs); rows(a.dk, a.dks); rows(a.dv, a.dvs);
+    a.vec = vec ? 1 : 0;
     return a;
 }
 
 template <typename K>
-int set_smem(ltca_ctx* ctx, K kern, size_t bytes) {
-    if (bytes > 48 * 1024)
-        LTCA_CUDA_OK(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)bytes));
+int set_smem(ltca_ctx* ctx, K kern, size_t bytes, SmemOptIn& once) {
+    if (bytes > 48 * 1024) LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(once, ctx->device, kern, (int)bytes));
     return LTCA_OK;
 }
 
-template <typename T, int DC>
+template <typename T, int DP, int TM, int NT, bool kMask>
 int run_fwd(ltca_ctx* ctx, const CoreArgs& a) {
-    const size_t smem = (size_t)(3 * kTM * (a.D + 1) + kTM * (kTN + 1)) * sizeof(float);
-    auto kern = attn_fwd_fp32_kernel<T, DC>;
-    int rc = set_smem(ctx, kern, smem);
+    static SmemOptIn once;
+    constexpr size_t smem = ((size_t)(TM + 128) * (DP + kPad) + TM * (64 + kPad) + TM) * sizeof(float);
+    int rc = set_smem(ctx, attn_fwd_fp32_kernel<T, DP, TM, NT, kMask>, smem, once);
     if (rc) return rc;
-    dim3 grid((a.Sq + kTM - 1) / kTM, a.H, a.B);
-    kern<<<grid, kThreads, smem, ctx->stream>>>(a);
-    LTCA_LAUNCH_OK(ctx, "attn_fwd_fp32_kernel");
+    dim3 grid((a.Sq + TM - 1) / TM, a.H, a.B);
+    LTCA_CUDA_OK(ctx, launch_dependent(attn_fwd_fp32_kernel<T, DP, TM, NT, kMask>, grid, dim3(NT), smem, ctx->stream, a));
     return LTCA_OK;
 }
 
-template <typename T, int DC>
-int run_bwd(ltca_ctx* ctx, const CoreArgs& a) {
-    {
-        const int wpb = 8;
-        const int64_t rows = (int64_t)a.B * a.H * a.Sq;
-        attn_bwd_delta_kernel<T><<<(unsigned)((rows + wpb - 1) / wpb), wpb * 32, 0, ctx->stream>>>(a);
-        LTCA_LAUNCH_OK(ctx, "attn_bwd_delta_kernel");
-    }
-    {
-        const size_t smem = (size_t)(4 * kTM * (a.D + 1) + kTM * (kTN + 1)) * sizeof(float);
-        auto kern = attn_bwd_dq_fp32_kernel<T, DC>;
-        int rc = set_smem(ctx, kern, smem);
-        if (rc) return rc;
-        dim3 grid((a.Sq + kTM - 1) / kTM, a.H, a.B);
-        kern<<<grid, kThreads, smem, ctx->stream>>>(a);
-        LTCA_LAUNCH_OK(ctx, "attn_bwd_dq_fp32_kernel");
-    }
-    {
-        const size_t smem = (size_t)(4 * kTM * (a.D + 1) + 2 * kTM * (kTN + 1)) * sizeof(float);
-        auto kern = attn_bwd_dkv_fp32_kernel<T, DC>;
-        int rc = set_smem(ctx, kern, smem);
-        if (rc) return rc;
-        dim3 grid((a.Sk + kTN - 1) / kTN, a.H, a.B);
-        kern<<<grid, kThreads, smem, ctx->stream>>>(a);
-        LTCA_LAUNCH_OK(ctx, "attn_bwd_dkv_fp32_kernel");
-    }
+template <typename T, int DP, int TM, int KN, int NT, bool kMask>
+int run_dq(ltca_ctx* ctx, const CoreArgs& a) {
+    static SmemOptIn once;
+    constexpr size_t smem = ((size_t)(2 * TM + 2 * KN) * (DP + kPad) + TM * (KN + kPad) + TM) * sizeof(float);
+    int rc = set_smem(ctx, attn_bwd_dq_fp32_kernel<T, DP, TM, KN, NT, kMask>, smem, once);
+    if (rc) return rc;
+    dim3 grid((a.Sq + TM - 1) / TM, a.H, a.B);
+    LTCA_CUDA_OK(ctx, launch_dependent(attn_bwd_dq_fp32_kernel<T, DP, TM, KN, NT, kMask>, grid, dim3(NT), smem, ctx->stream, a));
+    return LTCA_OK;
+}
+template <typename T, int DP, int TK, int QN, int NT, bool kMask>
+int run_dkv(ltca_ctx* ctx, const CoreArgs& a) {
+    static SmemOptIn once;
+    constexpr size_t smem = ((size_t)(2 * TK + 2 * QN) * (DP + kPad) + 2 * QN * (TK + kPad) + 2 * QN) * sizeof(float);
+    int rc = set_smem(ctx, attn_bwd_dkv_fp32_kernel<T, DP, TK, QN, NT, kMask>, smem, once);
+    if (rc) return rc;
+    dim3 grid((a.Sk + TK - 1) / TK, a.H, a.B);
+    LTCA_CUDA_OK(ctx, launch_dependent(attn_bwd_dkv_fp32_kernel<T, DP, TK, QN, NT, kMask>, grid, dim3(NT), smem, ctx->stream, a));
     return LTCA_OK;
 }
 
+// Tiles of 64 rows reuse what they load most; where they would leave SMs idle, tiles of 16 rows give four times the CTAs
+// and a quarter of the serial work.
+template <typename T, int DP, bool kMask>
+int run_rows(ltca_ctx* ctx, const CoreArgs& a, bool bwd) {
+    const int64_t bh = (int64_t)a.B * a.H;
+    auto fills = [&](int S) { return bh * ((S + 63) / 64) >= ctx->sm_device; };
+    constexpr int NT = DP > 64 ? 256 : 128;         // at DP = 128 eight columns per thread need the wider CTA
+    if (!bwd) return fills(a.Sq) ? run_fwd<T, DP, 64, NT, kMask>(ctx, a) : run_fwd<T, DP, 16, 128, kMask>(ctx, a);
+    int rc;
+    if ((rc = fills(a.Sq) ? run_dq<T, DP, 64, 64, NT, kMask>(ctx, a) : run_dq<T, DP, 16, 32, 128, kMask>(ctx, a))) return rc;
+    return fills(a.Sk) ? run_dkv<T, DP, 64, 64, NT, kMask>(ctx, a) : run_dkv<T, DP, 16, 32, 128, kMask>(ctx, a);
+}
+template <typename T, int DP>
+int run_rows(ltca_ctx* ctx, const CoreArgs& a, bool bwd) {
+    if (!a.keep_mask) return run_rows<T, DP, false>(ctx, a, bwd);
+    if (bwd) {
+        const int64_t rows = (int64_t)a.B * a.Sq, blocks = (rows * a.mask_nw + 7) / 8, most = 16ll * ctx->sm_device;
+        LTCA_CUDA_OK(ctx, launch_dependent(attn_mask_bits_kernel, dim3((unsigned)(blocks < most ? blocks : most)), dim3(256), 0,
+                                           ctx->stream, a.keep_mask, const_cast<uint32_t*>(a.mask_bits), rows, a.Sk, a.mask_nw));
+    }
+    return run_rows<T, DP, true>(ctx, a, bwd);
+}
 
 // ----------------------------------------------------------------------------------------------
 // Wide heads (128 < head_dim <= 512): the reference-compatible TimeSelfAttention gives every head
@@ -730,19 +1032,20 @@ int run_wide(ltca_ctx* ctx, const CoreArgs& a, bool bwd) {
 template <typename T>
 int dispatch(ltca_ctx* ctx, const CoreArgs& a, bool bwd) {
     if (a.D > 128) return run_wide<T>(ctx, a, bwd);
-    const int dc = (a.D + 15) / 16;
-#define LTCA_CASE(N) return bwd ? run_bwd<T, N>(ctx, a) : run_fwd<T, N>(ctx, a)
-    if (dc <= 1) LTCA_CASE(1);
-    if (dc <= 2) LTCA_CASE(2);
-    if (dc <= 4) LTCA_CASE(4);
-    LTCA_CASE(8);
-#undef LTCA_CASE
+    if (a.D <= 16) return run_rows<T, 16>(ctx, a, bwd);
+    if (a.D <= 32) return run_rows<T, 32>(ctx, a, bwd);
+    if (a.D <= 64) return run_rows<T, 64>(ctx, a, bwd);
+    return run_rows<T, 128>(ctx, a, bwd);
 }
 
 }  // namespace
 
+// delta, and the dense mask as bits (the kernels for head_dim up to 128)
+static size_t delta_bytes(const ltca_attn_params* p) { return align_up((size_t)p->B * p->H * p->Sq * sizeof(float), 256); }
 size_t attn_bwd_fp32_workspace(const ltca_attn_params* p) {
-    return align_up((size_t)p->B * p->H * p->Sq * sizeof(float), 256);
+    size_t n = delta_bytes(p);
+    if (p->keep_mask && p->D <= 128) n += align_up((size_t)p->B * p->Sq * ((p->Sk + 31) / 32) * 4, 256);
+    return n;
 }
 
 int launch_attn_fwd_fp32(ltca_ctx* ctx, const ltca_attn_params* p) {
@@ -760,6 +1063,8 @@ int launch_attn_bwd_fp32(ltca_ctx* ctx, const ltca_attn_params* p) {
                     attn_bwd_fp32_workspace(p));
     CoreArgs a = make_args(p);
     a.delta = reinterpret_cast<float*>(p->workspace);
+    a.mask_bits = reinterpret_cast<const uint32_t*>(reinterpret_cast<const char*>(p->workspace) + delta_bytes(p));
+    a.mask_nw = (p->Sk + 31) / 32;
     return p->dtype == LTCA_BF16 ? dispatch<__nv_bfloat16>(ctx, a, true) : dispatch<float>(ctx, a, true);
 }
 
