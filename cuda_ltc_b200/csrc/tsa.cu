@@ -20,6 +20,7 @@
 // Backward follows the reference:
 // the incoming gradient passes through LayerNorm and the residual unchanged
 // (src/ml/cudnn_time_self_attention.cu:291-299), dx = dQ Wq^T + dK Wk^T + dV Wv^T.
+#include "gemm_fp32.h"
 #include "gemm_sm100.h"
 #include "attn_wide.h"
 #include "host_common.h"
@@ -28,185 +29,6 @@
 namespace ltca {
 
 namespace {
-
-constexpr int kGT = 128;    // GEMM tile (M and N)
-constexpr int kGK = 16;     // GEMM K step
-constexpr int kGP = 4;      // row padding of the shared tiles (floats)
-
-// C[M,N] (+)= op(A) op(B) (+ bias[N]); row-major storage.
-//   ta == 0: A is [M,K] (lda = K-extent stride), ta == 1: A is stored [K,M].
-//   tb == 0: B is [K,N],                          tb == 1: B is stored [N,K].
-struct GemmArgs {
-    const float *A, *B, *bias;
-    float* C;
-    int M, N, K;
-    int lda, ldb, ldc;
-    int ta, tb, accumulate;
-    int kper;          // contraction extent one CTA covers (blockIdx.z selects the slice)
-    float* partial;    // [gridDim.z][M][N] slice results when the contraction is split, else null
-};
-
-// Exact-mode projection GEMM (fp32 FMA, the arithmetic of the reference's cublasSgemm with tensor cores
-// off, src/ml/flash_attention.cu:531-536): 128 x 128 tile per CTA, 16 x 16 threads with 8 x 8 outputs each
-// (two 4-wide groups 64 apart per dimension, so shared-memory reads are conflict-free float4 loads), the
-// next K slab is fetched from global memory into registers while the current one is multiplied.
-__global__ void __launch_bounds__(256) gemm_fp32_kernel(const GemmArgs g) {
-    __shared__ __align__(16) float As[kGK][kGT + kGP];
-    __shared__ __align__(16) float Bs[kGK][kGT + kGP];
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const int m0 = blockIdx.y * kGT, n0 = blockIdx.x * kGT;
-    const int kbeg = blockIdx.z * g.kper;
-    const int kend = min(g.K, kbeg + g.kper);
-    float acc[8][8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
-
-    // Each thread moves 8 elements of the A slab and 8 of the B slab.  With the contraction index
-    // contiguous in memory (ta == 0 / tb == 1) a thread takes elements (r, k..k+7) of one row half; with the
-    // M / N index contiguous (ta == 1 / tb == 0) it takes (k, c..c+7) of one K row.
-    float ra[8], rb[8];
-    auto fetch = [&](int k0) {
-        if (!g.ta) {
-            const int r = threadIdx.x >> 1, kk = (threadIdx.x & 1) * 8;
-            const int gm = m0 + r;
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                const int gk = k0 + kk + e;
-                ra[e] = (gm < g.M && gk < kend) ? __ldg(g.A + (int64_t)gm * g.lda + gk) : 0.f;
-            }
-        } else {
-            const int kk = threadIdx.x >> 4, c = (threadIdx.x & 15) * 8;
-            const int gk = k0 + kk;
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                const int gm = m0 + c + e;
-                ra[e] = (gm < g.M && gk < kend) ? __ldg(g.A + (int64_t)gk * g.lda + gm) : 0.f;
-            }
-        }
-        if (g.tb) {
-            const int r = threadIdx.x >> 1, kk = (threadIdx.x & 1) * 8;
-            const int gn = n0 + r;
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                const int gk = k0 + kk + e;
-                rb[e] = (gn < g.N && gk < kend) ? __ldg(g.B + (int64_t)gn * g.ldb + gk) : 0.f;
-            }
-        } else {
-            const int kk = threadIdx.x >> 4, c = (threadIdx.x & 15) * 8;
-            const int gk = k0 + kk;
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                const int gn = n0 + c + e;
-                rb[e] = (gn < g.N && gk < kend) ? __ldg(g.B + (int64_t)gk * g.ldb + gn) : 0.f;
-            }
-        }
-    };
-    auto stash = [&]() {
-        if (!g.ta) {
-            const int r = threadIdx.x >> 1, kk = (threadIdx.x & 1) * 8;
-#pragma unroll
-            for (int e = 0; e < 8; ++e) As[kk + e][r] = ra[e];
-        } else {
-            const int kk = threadIdx.x >> 4, c = (threadIdx.x & 15) * 8;
-#pragma unroll
-            for (int e = 0; e < 8; ++e) As[kk][c + e] = ra[e];
-        }
-        if (g.tb) {
-            const int r = threadIdx.x >> 1, kk = (threadIdx.x & 1) * 8;
-#pragma unroll
-            for (int e = 0; e < 8; ++e) Bs[kk + e][r] = rb[e];
-        } else {
-            const int kk = threadIdx.x >> 4, c = (threadIdx.x & 15) * 8;
-#pragma unroll
-            for (int e = 0; e < 8; ++e) Bs[kk][c + e] = rb[e];
-        }
-    };
-
-    fetch(kbeg);
-    for (int k0 = kbeg; k0 < kend; k0 += kGK) {
-        stash();
-        __syncthreads();
-        if (k0 + kGK < kend) fetch(k0 + kGK);
-#pragma unroll
-        for (int k = 0; k < kGK; ++k) {
-            const float4 a0 = *reinterpret_cast<const float4*>(&As[k][4 * ty]);
-            const float4 a1 = *reinterpret_cast<const float4*>(&As[k][64 + 4 * ty]);
-            const float4 b0 = *reinterpret_cast<const float4*>(&Bs[k][4 * tx]);
-            const float4 b1 = *reinterpret_cast<const float4*>(&Bs[k][64 + 4 * tx]);
-            const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-            const float b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-#pragma unroll
-                for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int gm = m0 + (i < 4 ? 4 * ty + i : 64 + 4 * ty + i - 4);
-        if (gm >= g.M) continue;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int gn = n0 + (j < 4 ? 4 * tx + j : 64 + 4 * tx + j - 4);
-            if (gn >= g.N) continue;
-            float v = acc[i][j];
-            if (g.partial) {
-                g.partial[((int64_t)blockIdx.z * g.M + gm) * g.N + gn] = v;
-                continue;
-            }
-            if (g.bias) v += g.bias[gn];
-            float* c = g.C + (int64_t)gm * g.ldc + gn;
-            *c = g.accumulate ? *c + v : v;
-        }
-    }
-}
-
-// C[m][n] = sum over slices, in slice order, of partial[z][m][n]: the second pass of a split contraction.
-__global__ void gemm_fp32_reduce_kernel(const float* __restrict__ partial, float* __restrict__ C, int M,
-                                        int N, int ldc, int slices) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (int64_t)M * N) return;
-    float v = 0.f;
-    for (int z = 0; z < slices; ++z) v += partial[(int64_t)z * M * N + i];
-    C[(i / N) * ldc + (i % N)] = v;
-}
-
-int gemm(ltca_ctx* ctx, const float* A, const float* B, const float* bias, float* C, int M, int N,
-         int K, int lda, int ldb, int ldc, int ta, int tb, int accumulate) {
-    GemmArgs g{A, B, bias, C, M, N, K, lda, ldb, ldc, ta, tb, accumulate, K, nullptr};
-    dim3 grid((N + kGT - 1) / kGT, (M + kGT - 1) / kGT);
-    gemm_fp32_kernel<<<grid, 256, 0, ctx->stream>>>(g);
-    LTCA_LAUNCH_OK(ctx, "gemm_fp32_kernel");
-    return LTCA_OK;
-}
-
-// A weight-gradient product (few output tiles, long contraction): the contraction is cut into slices, one
-// CTA per (tile, slice), and the slices are summed in a fixed order, so the result does not depend on
-// the launch.  `scratch` holds the slice results; with too little of it the product runs unsplit.
-int gemm_long_k(ltca_ctx* ctx, const float* A, const float* B, float* C, int M, int N, int K, int lda,
-                int ldb, int ldc, int ta, int tb, float* scratch, size_t scratch_bytes) {
-    const int tiles = ((N + kGT - 1) / kGT) * ((M + kGT - 1) / kGT);
-    int slices = (2 * ctx->sm_count + tiles - 1) / tiles;
-    const size_t one = (size_t)M * N * sizeof(float);
-    if ((size_t)slices * one > scratch_bytes) slices = (int)(scratch_bytes / one);
-    if (slices > K / (4 * kGK)) slices = K / (4 * kGK);
-    if (slices < 2) return gemm(ctx, A, B, nullptr, C, M, N, K, lda, ldb, ldc, ta, tb, 0);
-    int kper = (K + slices - 1) / slices;
-    kper = (kper + kGK - 1) / kGK * kGK;
-    slices = (K + kper - 1) / kper;
-    GemmArgs g{A, B, nullptr, C, M, N, K, lda, ldb, ldc, ta, tb, 0, kper, scratch};
-    dim3 grid((N + kGT - 1) / kGT, (M + kGT - 1) / kGT, slices);
-    gemm_fp32_kernel<<<grid, 256, 0, ctx->stream>>>(g);
-    LTCA_LAUNCH_OK(ctx, "gemm_fp32_kernel");
-    const int64_t n = (int64_t)M * N;
-    gemm_fp32_reduce_kernel<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(scratch, C, M, N, ldc,
-                                                                                  slices);
-    LTCA_LAUNCH_OK(ctx, "gemm_fp32_reduce_kernel");
-    return LTCA_OK;
-}
 
 // out[row] = LayerNorm(y[row] (+ x[row])) or just the sum / a copy; one warp per row.
 __global__ void residual_layer_norm_kernel(const float* __restrict__ y, const float* __restrict__ x,
@@ -292,6 +114,13 @@ __global__ void residual_layer_norm_kernel(const float* __restrict__ y, const fl
         outr[i] = (outr[i] - mean) * inv_std * (gamma ? gamma[i] : 1.f) + (beta ? beta[i] : 0.f);
 }
 
+int residual_layer_norm(ltca_ctx* ctx, const ltca_tsa_params* t, const float* y, int64_t rows) {
+    const int wpb = 8;
+    LTCA_CUDA_OK(ctx, launch_dependent(residual_layer_norm_kernel, dim3((unsigned)((rows + wpb - 1) / wpb)), dim3(wpb * 32),
+                                       0, ctx->stream, y, t->x, t->ln_gamma, t->ln_beta, t->out, rows, t->E,
+                                       t->use_residual, t->use_layer_norm, 1e-5f));
+    return LTCA_OK;
+}
 
 // ---- pieces of the FlashAttention form: dropout, LayerNorm backward, column sums -----------------
 
@@ -498,9 +327,10 @@ int forward_core(ltca_ctx* ctx, const ltca_tsa_params* t, const Plan& pl, char* 
     if (t->saved && t->reuse_forward) return LTCA_OK;
     const int rows = (int)pl.rows, E = t->E, HW = pl.HW;
     int rc;
-    if ((rc = gemm(ctx, t->x, t->wq, t->bq, fb->q, rows, HW, E, E, HW, HW, 0, 0, 0))) return rc;
-    if ((rc = gemm(ctx, t->x, t->wk, t->bk, fb->k, rows, HW, E, E, HW, HW, 0, 0, 0))) return rc;
-    if ((rc = gemm(ctx, t->x, t->wv, t->bv, fb->v, rows, HW, E, E, HW, HW, 0, 0, 0))) return rc;
+    const Gemm32Problem qkv[3] = {{t->x, t->wq, t->bq, fb->q, rows, HW, E, E, HW, HW},
+                                  {t->x, t->wk, t->bk, fb->k, rows, HW, E, E, HW, HW},
+                                  {t->x, t->wv, t->bv, fb->v, rows, HW, E, E, HW, HW}};
+    if ((rc = gemm_fp32(ctx, qkv, 3, 0, 0, false))) return rc;
     ltca_attn_params a;
     fill_attn(t, &a);
     a.q = fb->q; a.k = fb->k; a.v = fb->v; a.o = fb->ctx; a.lse = fb->lse;
@@ -791,12 +621,7 @@ int tensor_forward(ltca_ctx* ctx, const ltca_tsa_params* t) {
     gp.bias[0] = t->bo;
     gp.ldc = t->E;
     if ((rc = gemm_sm100(ctx, gp))) return rc;
-    const int wpb = 8;
-    LTCA_CUDA_OK(ctx, launch_dependent(residual_layer_norm_kernel, dim3((unsigned)((pl.rows + wpb - 1) / wpb)), dim3(wpb * 32),
-                                       0, ctx->stream, (const float*)y, t->x, t->ln_gamma, t->ln_beta, t->out, pl.rows, t->E,
-                                       t->use_residual, t->use_layer_norm, 1e-5f));
-    LTCA_LAUNCH_OK(ctx, "residual_layer_norm_kernel");
-    return LTCA_OK;
+    return residual_layer_norm(ctx, t, y, pl.rows);
 }
 
 int tensor_backward(ltca_ctx* ctx, const ltca_tsa_params* t, bool want_dx, bool want_dw, float* colsum_scratch) {
@@ -1107,14 +932,9 @@ int ltca_tsa_fwd(ltca_ctx* ctx, const ltca_tsa_params* t) {
     FwdBufs fb;
     if ((rc = forward_core(ctx, t, pl, w, &fb, pl.attn_fwd))) return rc;
     const int rows = (int)pl.rows;
-    if ((rc = gemm(ctx, fb.ctx, t->wo, t->bo, y, rows, t->E, pl.HW, pl.HW, t->E, t->E, 0, 0, 0)))
-        return rc;
-    const int wpb = 8;
-    residual_layer_norm_kernel<<<(unsigned)((pl.rows + wpb - 1) / wpb), wpb * 32, 0, ctx->stream>>>(
-        y, t->x, t->ln_gamma, t->ln_beta, t->out, pl.rows, t->E, t->use_residual, t->use_layer_norm,
-        1e-5f);
-    LTCA_LAUNCH_OK(ctx, "residual_layer_norm_kernel");
-    return LTCA_OK;
+    const Gemm32Problem proj = {fb.ctx, t->wo, t->bo, y, rows, t->E, pl.HW, pl.HW, t->E, t->E};
+    if ((rc = gemm_fp32(ctx, &proj, 1, 0, 0, false))) return rc;
+    return residual_layer_norm(ctx, t, y, pl.rows);
 }
 
 static int tsa_backward(ltca_ctx* ctx, const ltca_tsa_params* t, bool want_dx, bool want_dw) {
@@ -1150,7 +970,8 @@ static int tsa_backward(ltca_ctx* ctx, const ltca_tsa_params* t, bool want_dx, b
     if ((rc = forward_core(ctx, t, pl, w, &fb, pl.attn_fwd))) return rc;
     const int rows = (int)pl.rows, E = t->E, HW = pl.HW;
     // dctx = dy Wo^T
-    if ((rc = gemm(ctx, t->dy, t->wo, nullptr, dctx, rows, HW, E, E, E, HW, 0, 1, 0))) return rc;
+    const Gemm32Problem back = {t->dy, t->wo, nullptr, dctx, rows, HW, E, E, E, HW};
+    if ((rc = gemm_fp32(ctx, &back, 1, 0, 1, false))) return rc;
     ltca_attn_params a;
     fill_attn(t, &a);
     a.q = fb.q; a.k = fb.k; a.v = fb.v; a.o = fb.ctx; a.lse = fb.lse;
@@ -1166,18 +987,19 @@ static int tsa_backward(ltca_ctx* ctx, const ltca_tsa_params* t, bool want_dx, b
         if (t->dbo && (rc = column_sum(ctx, t->dy, E, pl.rows, E, t->dbo, colsum_scratch))) return rc;
     }
     if (want_dx) {
-        if ((rc = gemm(ctx, dq, t->wq, nullptr, t->dx, rows, E, HW, HW, HW, E, 0, 1, 0))) return rc;
-        if ((rc = gemm(ctx, dk, t->wk, nullptr, t->dx, rows, E, HW, HW, HW, E, 0, 1, 1))) return rc;
-        if ((rc = gemm(ctx, dv, t->wv, nullptr, t->dx, rows, E, HW, HW, HW, E, 0, 1, 1))) return rc;
+        const Gemm32Problem terms[3] = {{dq, t->wq, nullptr, t->dx, rows, E, HW, HW, HW, E},
+                                        {dk, t->wk, nullptr, t->dx, rows, E, HW, HW, HW, E},
+                                        {dv, t->wv, nullptr, t->dx, rows, E, HW, HW, HW, E}};
+        if ((rc = gemm_fp32(ctx, terms, 3, 0, 1, true))) return rc;
     }
     if (want_dw) {
         // dW = x^T dQ  ([E, rows] x [rows, HW]),  dWo = ctx^T dy  ([HW, rows] x [rows, E])
         // dctx is dead once the attention backward has run: it holds the contraction slices
-        if ((rc = gemm_long_k(ctx, t->x, dq, t->dwq, E, HW, rows, E, HW, HW, 1, 0, dctx, pl.buf))) return rc;
-        if ((rc = gemm_long_k(ctx, t->x, dk, t->dwk, E, HW, rows, E, HW, HW, 1, 0, dctx, pl.buf))) return rc;
-        if ((rc = gemm_long_k(ctx, t->x, dv, t->dwv, E, HW, rows, E, HW, HW, 1, 0, dctx, pl.buf))) return rc;
-        if ((rc = gemm_long_k(ctx, fb.ctx, t->dy, t->dwo, HW, E, rows, HW, E, E, 1, 0, dctx, pl.buf)))
-            return rc;
+        const Gemm32Problem dw[4] = {{t->x, dq, nullptr, t->dwq, E, HW, rows, E, HW, HW},
+                                     {t->x, dk, nullptr, t->dwk, E, HW, rows, E, HW, HW},
+                                     {t->x, dv, nullptr, t->dwv, E, HW, rows, E, HW, HW},
+                                     {fb.ctx, t->dy, nullptr, t->dwo, HW, E, rows, HW, E, E}};
+        if ((rc = gemm_fp32(ctx, dw, 4, 1, 0, false, dctx, pl.buf))) return rc;
     }
     return LTCA_OK;
 }
