@@ -474,36 +474,11 @@ __global__ void cvt_rows_bf16_vec_kernel(const float4* __restrict__ src, uint2* 
     }
 }
 
-// Several matrices of any sizes in ONE launch (the activations and the weights of a module call): the 16-byte
-// pieces of all of them form one index range that the grid strides over.
-constexpr int kMaxCvtMany = 6;
-struct CvtMany {
-    const float* src[kMaxCvtMany];
-    __nv_bfloat16* dst[kMaxCvtMany];
-    __nv_bfloat16* lo[kMaxCvtMany];         // second term bf16(x - bf16(x)), laid out like dst, or null
-    int64_t ld_src[kMaxCvtMany], ld_dst[kMaxCvtMany];
-    uint32_t cols4[kMaxCvtMany];
-    uint32_t start4[kMaxCvtMany + 1];       // first piece of matrix m; start4[n] = all pieces
-    int n;
-};
+// Several matrices of any sizes in ONE launch (the activations and the weights of a module call).
 __global__ void cvt_many_bf16_kernel(const __grid_constant__ CvtMany b) {
     grid_launch_dependents();
     grid_dependency_wait();
-    const uint32_t total = b.start4[b.n];
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
-        int m = 0;
-        while (m + 1 < b.n && i >= b.start4[m + 1]) ++m;
-        const uint32_t j = i - b.start4[m];
-        const uint32_t r = j / b.cols4[m], c4 = j - r * b.cols4[m];
-        const float4 v = __ldg(reinterpret_cast<const float4*>(b.src[m] + (int64_t)r * b.ld_src[m]) + c4);
-        const uint2 h = make_uint2(pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w));
-        reinterpret_cast<uint2*>(b.dst[m] + (int64_t)r * b.ld_dst[m])[c4] = h;
-        if (b.lo[m]) {
-            const uint2 l = make_uint2(pack_bf16x2(v.x - __uint_as_float(h.x << 16), v.y - __uint_as_float(h.x & 0xffff0000u)),
-                                       pack_bf16x2(v.z - __uint_as_float(h.y << 16), v.w - __uint_as_float(h.y & 0xffff0000u)));
-            reinterpret_cast<uint2*>(b.lo[m] + (int64_t)r * b.ld_dst[m])[c4] = l;
-        }
-    }
+    cvt_many_pieces(b, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 
 int make_operand_map(ltca_ctx* ctx, CUtensorMap* map, const GemmOperand& o, int mn_extent, int k_extent,
@@ -640,31 +615,32 @@ int convert_rows_bf16(ltca_ctx* ctx, const float* src, int64_t ld_src, void* dst
 }
 
 
+bool make_cvt_many(CvtMany* b, int n, const float* const* src, const int64_t* ld_src, void* const* dst, const int64_t* ld_dst,
+                   const int64_t* rows, const int* cols, void* const* lo) {
+    memset(b, 0, sizeof(*b));
+    uint64_t total = 0;
+    for (int i = 0; i < n; ++i) {
+        if (rows[i] < 1 || cols[i] < 1) continue;
+        if ((lo && lo[i] && (reinterpret_cast<uintptr_t>(lo[i]) & 7)) || (cols[i] & 3) || (ld_src[i] & 3) || (ld_dst[i] & 3) ||
+            (reinterpret_cast<uintptr_t>(src[i]) & 15) || (reinterpret_cast<uintptr_t>(dst[i]) & 7))
+            return false;
+        const int m = b->n++;
+        b->src[m] = src[i]; b->dst[m] = reinterpret_cast<__nv_bfloat16*>(dst[i]);
+        b->lo[m] = lo ? reinterpret_cast<__nv_bfloat16*>(lo[i]) : nullptr;
+        b->ld_src[m] = ld_src[i]; b->ld_dst[m] = ld_dst[i];
+        b->cols4[m] = (uint32_t)(cols[i] / 4);
+        b->start4[m] = (uint32_t)total;
+        total += (uint64_t)rows[i] * (uint64_t)(cols[i] / 4);
+    }
+    b->start4[b->n] = (uint32_t)total;
+    return total < (1ull << 31);
+}
+
 int convert_many_bf16(ltca_ctx* ctx, int n, const float* const* src, const int64_t* ld_src, void* const* dst,
                       const int64_t* ld_dst, const int64_t* rows, const int* cols, void* const* lo) {
     if (n < 1 || n > kMaxCvtMany) return fail(ctx, LTCA_ERR_INVALID, "convert_many_bf16 takes 1 to %d matrices", kMaxCvtMany);
     CvtMany b;
-    memset(&b, 0, sizeof(b));
-    b.n = 0;
-    uint64_t total = 0;
-    bool vec = true;
-    for (int i = 0; i < n; ++i) {
-        if (rows[i] < 1 || cols[i] < 1) continue;
-        if (lo && lo[i]) vec = vec && (reinterpret_cast<uintptr_t>(lo[i]) & 7) == 0;
-        if (!vec || (cols[i] & 3) || (ld_src[i] & 3) || (ld_dst[i] & 3) || (reinterpret_cast<uintptr_t>(src[i]) & 15) ||
-            (reinterpret_cast<uintptr_t>(dst[i]) & 7)) {
-            vec = false;
-            break;
-        }
-        const int m = b.n++;
-        b.src[m] = src[i]; b.dst[m] = reinterpret_cast<__nv_bfloat16*>(dst[i]);
-        b.lo[m] = lo ? reinterpret_cast<__nv_bfloat16*>(lo[i]) : nullptr;
-        b.ld_src[m] = ld_src[i]; b.ld_dst[m] = ld_dst[i];
-        b.cols4[m] = (uint32_t)(cols[i] / 4);
-        b.start4[m] = (uint32_t)total;
-        total += (uint64_t)rows[i] * (uint64_t)(cols[i] / 4);
-    }
-    if (!vec || total >= (1ull << 31)) {
+    if (!make_cvt_many(&b, n, src, ld_src, dst, ld_dst, rows, cols, lo)) {
         // odd shapes or alignments: one matrix at a time
         for (int i = 0; i < n; ++i) {
             int rc;
@@ -675,7 +651,7 @@ int convert_many_bf16(ltca_ctx* ctx, int n, const float* const* src, const int64
         return LTCA_OK;
     }
     if (b.n == 0) return LTCA_OK;
-    b.start4[b.n] = (uint32_t)total;
+    const uint32_t total = b.start4[b.n];
     const unsigned blocks = (unsigned)((total + 255) / 256 < 2368 ? (total + 255) / 256 : 2368);
     LTCA_CUDA_OK(ctx, launch_dependent(cvt_many_bf16_kernel, dim3(blocks), dim3(256), 0, ctx->stream, b));
     LTCA_LAUNCH_OK(ctx, "cvt_many_bf16_kernel");

@@ -2,6 +2,7 @@
 #pragma once
 
 #include "host_common.h"
+#include "sm100_ptx.cuh"
 
 namespace ltca {
 
@@ -40,9 +41,44 @@ size_t gemm_sm100_partial_bytes(int M, int N, int n_problems, int ksplit);
 // dst[r, c] = bf16(src[r, c]) for a [rows, cols] block with row pitches ld_src / ld_dst (elements).
 int convert_rows_bf16(ltca_ctx* ctx, const float* src, int64_t ld_src, void* dst, int64_t ld_dst, int64_t rows,
                       int cols);
+// Several matrices of any sizes whose 16-byte pieces form one index range: what one launch rounds to bf16.
+constexpr int kMaxCvtMany = 6;
+struct CvtMany {
+    const float* src[kMaxCvtMany];
+    __nv_bfloat16* dst[kMaxCvtMany];
+    __nv_bfloat16* lo[kMaxCvtMany];         // second term bf16(x - bf16(x)), laid out like dst, or null
+    int64_t ld_src[kMaxCvtMany], ld_dst[kMaxCvtMany];
+    uint32_t cols4[kMaxCvtMany];
+    uint32_t start4[kMaxCvtMany + 1];       // first piece of matrix m; start4[n] = all pieces
+    int n;
+};
+// Fills `b`; false when a matrix has rows that are no multiple of 16 bytes (those go one at a time).
+bool make_cvt_many(CvtMany* b, int n, const float* const* src, const int64_t* ld_src, void* const* dst, const int64_t* ld_dst,
+                   const int64_t* rows, const int* cols, void* const* lo);
 // The same for up to six matrices of any sizes in one launch (16-byte aligned rows; otherwise one launch each).
 // `lo` (or an entry of it) non-null: also the second term bf16(x - bf16(x)), laid out like the first.
 int convert_many_bf16(ltca_ctx* ctx, int n, const float* const* src, const int64_t* ld_src, void* const* dst,
                       const int64_t* ld_dst, const int64_t* rows, const int* cols, void* const* lo = nullptr);
+
+#ifdef __CUDACC__
+// Pieces i, i + step, ... of the range.
+__device__ __forceinline__ void cvt_many_pieces(const CvtMany& b, uint32_t i, uint32_t step) {
+    const uint32_t total = b.start4[b.n];
+    for (; i < total; i += step) {
+        int m = 0;
+        while (m + 1 < b.n && i >= b.start4[m + 1]) ++m;
+        const uint32_t j = i - b.start4[m];
+        const uint32_t r = j / b.cols4[m], c4 = j - r * b.cols4[m];
+        const float4 v = __ldg(reinterpret_cast<const float4*>(b.src[m] + (int64_t)r * b.ld_src[m]) + c4);
+        const uint2 h = make_uint2(pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w));
+        reinterpret_cast<uint2*>(b.dst[m] + (int64_t)r * b.ld_dst[m])[c4] = h;
+        if (b.lo[m]) {
+            const uint2 l = make_uint2(pack_bf16x2(v.x - __uint_as_float(h.x << 16), v.y - __uint_as_float(h.x & 0xffff0000u)),
+                                       pack_bf16x2(v.z - __uint_as_float(h.y << 16), v.w - __uint_as_float(h.y & 0xffff0000u)));
+            reinterpret_cast<uint2*>(b.lo[m] + (int64_t)r * b.ld_dst[m])[c4] = l;
+        }
+    }
+}
+#endif
 
 }  // namespace ltca

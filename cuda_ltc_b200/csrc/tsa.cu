@@ -30,23 +30,30 @@ namespace ltca {
 
 namespace {
 
-// out[row] = LayerNorm(y[row] (+ x[row])) or just the sum / a copy; one warp per row.
-__global__ void residual_layer_norm_kernel(const float* __restrict__ y, const float* __restrict__ x,
-                                           const float* __restrict__ gamma,
-                                           const float* __restrict__ beta, float* __restrict__ out,
-                                           int64_t rows, int E, int use_res, int use_ln, float eps) {
-    grid_launch_dependents();
-    grid_dependency_wait();
-    const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (row >= rows) return;
+// Where a row of results goes: fp32, bf16, or both; rows are `ld` elements apart in either.
+struct RowOut {
+    float* f32;
+    __nv_bfloat16* bf16;
+    int64_t ld_f32, ld_bf16;
+};
+__device__ __forceinline__ void put4(const RowOut& o, int64_t row, int c, float4 v) {
+    if (o.f32) *reinterpret_cast<float4*>(o.f32 + row * o.ld_f32 + c) = v;
+    if (o.bf16) *reinterpret_cast<uint2*>(o.bf16 + row * o.ld_bf16 + c) = make_uint2(pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w));
+}
+__device__ __forceinline__ void put1(const RowOut& o, int64_t row, int c, float v) {
+    if (o.f32) o.f32[row * o.ld_f32 + c] = v;
+    if (o.bf16) o.bf16[row * o.ld_bf16 + c] = __float2bfloat16_rn(v);
+}
+
+// One row by one warp: LayerNorm(y (+ x)), or just the sum / a copy.  `vec`: every row of every operand starts on a
+// 16-byte boundary and E is a multiple of 4.
+__device__ __forceinline__ void layer_norm_row(const float* __restrict__ y, const float* __restrict__ x,
+                                               const float* __restrict__ gamma, const float* __restrict__ beta, const RowOut& out,
+                                               int64_t row, int E, bool use_res, bool use_ln, float eps, bool vec) {
     const int lane = threadIdx.x & 31;
     const float* yr = y + row * E;
     const float* xr = x + row * E;
-    float* outr = out + row * E;
-    const uintptr_t align_bits = reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(x) |
-                                 reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(gamma) |
-                                 reinterpret_cast<uintptr_t>(beta);
-    if (use_ln && (E & 127) == 0 && E <= 1024 && (align_bits & 15) == 0) {
+    if (use_ln && vec && (E & 127) == 0 && E <= 1024) {
         // the row stays in registers: one read of y and x, one write of the result
         float4 v[8];
         const int n4 = E >> 7;                        // float4 per lane
@@ -87,31 +94,48 @@ __global__ void residual_layer_norm_kernel(const float* __restrict__ y, const fl
                 o4.y = (v[i].y - mean4) * inv4 * gm.y + bt.y;
                 o4.z = (v[i].z - mean4) * inv4 * gm.z + bt.z;
                 o4.w = (v[i].w - mean4) * inv4 * gm.w + bt.w;
-                reinterpret_cast<float4*>(outr)[lane + 32 * i] = o4;
+                put4(out, row, 4 * (lane + 32 * i), o4);
             }
         }
         return;
     }
-    float sum = 0.f;
-    for (int i = lane; i < E; i += 32) {
-        const float v = yr[i] + (use_res ? xr[i] : 0.f);
-        outr[i] = v;
-        sum += v;
+    auto value = [&](int i) { return yr[i] + (use_res ? xr[i] : 0.f); };
+    if (!use_ln) {
+        for (int i = lane; i < E; i += 32) put1(out, row, i, value(i));
+        return;
     }
-    if (!use_ln) return;
+    // any width: the lane's elements are formed again for each pass
+    float sum = 0.f;
+    for (int i = lane; i < E; i += 32) sum += value(i);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
     const float mean = sum / E;
     float var = 0.f;
     for (int i = lane; i < E; i += 32) {
-        const float d = outr[i] - mean;
+        const float d = value(i) - mean;
         var = fmaf(d, d, var);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) var += __shfl_xor_sync(0xffffffffu, var, o);
     const float inv_std = rsqrtf(var / E + eps);
     for (int i = lane; i < E; i += 32)
-        outr[i] = (outr[i] - mean) * inv_std * (gamma ? gamma[i] : 1.f) + (beta ? beta[i] : 0.f);
+        put1(out, row, i, fmaf((value(i) - mean) * inv_std, gamma ? gamma[i] : 1.f, beta ? beta[i] : 0.f));
+}
+__device__ __forceinline__ bool aligned16(const void* a, const void* b, const void* c, const void* d, const void* e) {
+    return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c) |
+             reinterpret_cast<uintptr_t>(d) | reinterpret_cast<uintptr_t>(e)) & 15) == 0;
+}
+
+__global__ void residual_layer_norm_kernel(const float* __restrict__ y, const float* __restrict__ x,
+                                           const float* __restrict__ gamma,
+                                           const float* __restrict__ beta, float* __restrict__ out,
+                                           int64_t rows, int E, int use_res, int use_ln, float eps) {
+    grid_launch_dependents();
+    grid_dependency_wait();
+    const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (row >= rows) return;
+    const RowOut o{out, nullptr, E, 0};
+    layer_norm_row(y, x, gamma, beta, o, row, E, use_res != 0, use_ln != 0, eps, aligned16(y, x, gamma, beta, out));
 }
 
 int residual_layer_norm(ltca_ctx* ctx, const ltca_tsa_params* t, const float* y, int64_t rows) {
@@ -134,22 +158,111 @@ __host__ __device__ inline float dropout_uniform(uint64_t seed, uint64_t idx) {
     return (float)(z >> 40) * (1.0f / 16777216.0f);
 }
 
-// dst[i] = keep(i) ? src[i] / (1 - p) : 0   (inverted dropout, reference src/ml/flash_attention.cu:380-399;
-// the reference draws from curand with a time-dependent offset, so only the distribution can match)
-__global__ void dropout_kernel(const float* __restrict__ src, float* __restrict__ dst, int64_t n, float p,
-                               uint64_t seed) {
+// Inverted dropout of element i (reference src/ml/flash_attention.cu:380-399; the reference draws from curand with a
+// time-dependent offset, so only the distribution can match).
+__device__ __forceinline__ float dropout(float v, int64_t i, float p, float scale, uint64_t seed) {
+    return dropout_uniform(seed, (uint64_t)i) >= p ? v * scale : 0.f;
+}
+
+// Everything the FlashAttention form does before its first product, in one launch whose blocks take one of three parts:
+// LayerNorm of the input rows, dropout of the incoming gradient, rounding of the weights to bf16.  As launches of their
+// own (with a separate rounding of the first two results) these were four of 12 kernels of a few microseconds.
+struct PrepareArgs {
+    const float *x, *gamma, *beta;      // rows [rows, E]; LayerNorm when use_ln, else a copy
+    RowOut xo;
+    const float* dy;                    // backward: gradient behind the dropout, [rows, E], or null
+    RowOut go;
+    int64_t rows;
+    int E, use_ln;
+    float eps, p;
+    uint64_t seed;
+    int row_blocks, dy_blocks;          // blocks of the first two parts
+    CvtMany w;                          // matrices to round
+};
+constexpr int kPrepareThreads = 256;
+__global__ void __launch_bounds__(kPrepareThreads) prenorm_prepare_kernel(const __grid_constant__ PrepareArgs a) {
+    grid_launch_dependents();
+    grid_dependency_wait();
+    int block = blockIdx.x;
+    if (block < a.row_blocks) {
+        const int64_t row = (int64_t)block * (kPrepareThreads / 32) + (threadIdx.x >> 5);
+        if (row >= a.rows) return;
+        const bool vec = aligned16(a.x, a.gamma, a.beta, a.xo.f32, a.xo.bf16);
+        layer_norm_row(a.x, a.x, a.gamma, a.beta, a.xo, row, a.E, false, a.use_ln != 0, a.eps, vec);
+        return;
+    }
+    block -= a.row_blocks;
+    if (block < a.dy_blocks) {
+        const float scale = 1.0f / (1.0f - a.p);
+        const int64_t n = a.rows * a.E, first = (int64_t)block * kPrepareThreads + threadIdx.x;
+        const int64_t step = (int64_t)a.dy_blocks * kPrepareThreads;
+        if ((a.E & 3) == 0 && (a.go.ld_bf16 & 3) == 0 && n < (1ll << 32) && aligned16(a.dy, a.go.f32, a.go.bf16, nullptr, nullptr)) {
+            const uint32_t e4 = (uint32_t)a.E / 4;
+            for (int64_t i = first; i < n / 4; i += step) {
+                const uint32_t row = (uint32_t)i / e4, c = ((uint32_t)i - row * e4) * 4;
+                float4 v = __ldg(reinterpret_cast<const float4*>(a.dy) + i);
+                if (a.p > 0.f) {
+                    v.x = dropout(v.x, 4 * i, a.p, scale, a.seed);
+                    v.y = dropout(v.y, 4 * i + 1, a.p, scale, a.seed);
+                    v.z = dropout(v.z, 4 * i + 2, a.p, scale, a.seed);
+                    v.w = dropout(v.w, 4 * i + 3, a.p, scale, a.seed);
+                }
+                put4(a.go, row, (int)c, v);
+            }
+            return;
+        }
+        for (int64_t i = first; i < n; i += step) {
+            const int64_t row = i / a.E;
+            const float v = a.p > 0.f ? dropout(a.dy[i], i, a.p, scale, a.seed) : a.dy[i];
+            put1(a.go, row, (int)(i - row * a.E), v);
+        }
+        return;
+    }
+    block -= a.dy_blocks;
+    cvt_many_pieces(a.w, (uint32_t)block * kPrepareThreads + threadIdx.x,
+                    (gridDim.x - a.row_blocks - a.dy_blocks) * kPrepareThreads);
+}
+
+// out = dropout(y (+ x)): the end of the FlashAttention form's forward.
+__global__ void __launch_bounds__(256) residual_dropout_kernel(const float* __restrict__ y, const float* __restrict__ x, float* __restrict__ out,
+                                                               int64_t n, int use_res, float p, uint64_t seed) {
+    grid_launch_dependents();
+    grid_dependency_wait();
     const float scale = 1.0f / (1.0f - p);
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        dst[i] = dropout_uniform(seed, (uint64_t)i) >= p ? src[i] * scale : 0.f;
+    const int64_t first = (int64_t)blockIdx.x * 256 + threadIdx.x, step = (int64_t)gridDim.x * 256;
+    if ((n & 3) == 0 && aligned16(y, x, out, nullptr, nullptr)) {
+        for (int64_t i = first; i < n / 4; i += step) {
+            float4 v = __ldg(reinterpret_cast<const float4*>(y) + i);
+            if (use_res) {
+                const float4 r = __ldg(reinterpret_cast<const float4*>(x) + i);
+                v.x += r.x; v.y += r.y; v.z += r.z; v.w += r.w;
+            }
+            if (p > 0.f) {
+                v.x = dropout(v.x, 4 * i, p, scale, seed);
+                v.y = dropout(v.y, 4 * i + 1, p, scale, seed);
+                v.z = dropout(v.z, 4 * i + 2, p, scale, seed);
+                v.w = dropout(v.w, 4 * i + 3, p, scale, seed);
+            }
+            reinterpret_cast<float4*>(out)[i] = v;
+        }
+        return;
+    }
+    for (int64_t i = first; i < n; i += step) {
+        float v = y[i];
+        if (use_res) v += x[i];
+        out[i] = p > 0.f ? dropout(v, i, p, scale, seed) : v;
+    }
 }
 
 // LayerNorm backward, one warp per row.  g = gradient at the LayerNorm output, x = its input.
 //   dx = inv_std * (g*gamma - mean(g*gamma) - xhat * mean(g*gamma*xhat))  (+ res[row] when res != null)
-// prod (optional) receives g * xhat, whose column sums are dgamma.
+// dx and prod are optional; prod receives g * xhat, whose column sums are dgamma.
 __global__ void layer_norm_bwd_kernel(const float* __restrict__ g, const float* __restrict__ x,
                                       const float* __restrict__ gamma, const float* __restrict__ res,
                                       float* __restrict__ dx, float* __restrict__ prod, int64_t rows, int E,
                                       float eps) {
+    grid_launch_dependents();
+    grid_dependency_wait();
     const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (row >= rows) return;
     const int lane = threadIdx.x & 31;
@@ -181,48 +294,111 @@ __global__ void layer_norm_bwd_kernel(const float* __restrict__ g, const float* 
     for (int i = lane; i < E; i += 32) {
         const float xh = (xr[i] - mean) * inv_std;
         const float gi = gr[i];
-        float v = inv_std * (gi * gamma[i] - m1 - xh * m2);
-        if (res) v += res[row * E + i];
-        if (prod) prod[row * E + i] = gi * xh;          // may alias g: each element is read before it is written
-        dx[row * E + i] = v;
+        if (dx) {
+            float v = inv_std * (gi * gamma[i] - m1 - xh * m2);
+            if (res) v += res[row * E + i];
+            dx[row * E + i] = v;
+        }
+        if (prod) prod[row * E + i] = gi * xh;
     }
 }
 
-// Column sums of a [rows, cols] matrix in two fixed-order stages (no atomics): kColChunks row chunks, then
-// the chunks.
-constexpr int kColChunks = 64;
+// Column sums of up to six [rows, cols] matrices in two fixed-order stages (no atomics): kColChunks row chunks, then
+// the chunks.  One launch per stage for all of them: each is a microsecond of reading behind two of launching.
+constexpr int kColChunks = 64, kMaxColJobs = 6;
+struct ColSum {
+    const void* src[kMaxColJobs];
+    float* dst[kMaxColJobs];
+    int64_t ld[kMaxColJobs];
+    int cols[kMaxColJobs], bf16[kMaxColJobs];
+    int64_t rows;
+    int n, max_cols;
+    float* partial;                     // [n][kColChunks][max_cols]
+    void add(const void* s, bool is_bf16, int64_t pitch, int c, float* d) {
+        if (!d) return;
+        src[n] = s; dst[n] = d; ld[n] = pitch; cols[n] = c; bf16[n] = is_bf16 ? 1 : 0;
+        if (c > max_cols) max_cols = c;
+        ++n;
+    }
+};
 __device__ __forceinline__ float ld_f(const float* p) { return *p; }
 __device__ __forceinline__ float ld_f(const __nv_bfloat16* p) { return __bfloat162float(*p); }
 template <typename T>
-__global__ void column_sum_partial_kernel(const T* __restrict__ src, int64_t ld, int64_t rows, int cols,
-                                          float* __restrict__ partial) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= cols) return;
-    const int64_t per = (rows + kColChunks - 1) / kColChunks;
-    const int64_t r0 = blockIdx.y * per, r1 = r0 + per < rows ? r0 + per : rows;
+__device__ __forceinline__ float column_chunk(const T* src, int64_t ld, int64_t r0, int64_t r1) {
     float acc = 0.f;
-    for (int64_t r = r0; r < r1; ++r) acc += ld_f(src + r * ld + c);
-    partial[(int64_t)blockIdx.y * cols + c] = acc;
+#pragma unroll 8
+    for (int64_t r = r0; r < r1; ++r) acc += ld_f(src + r * ld);
+    return acc;
 }
-__global__ void column_sum_final_kernel(const float* __restrict__ partial, int cols, float* __restrict__ dst) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= cols) return;
-    float acc = 0.f;
-    for (int k = 0; k < kColChunks; ++k) acc += partial[(int64_t)k * cols + c];
-    dst[c] = acc;
+__global__ void __launch_bounds__(128) column_sum_partial_kernel(const __grid_constant__ ColSum a) {
+    grid_launch_dependents();
+    grid_dependency_wait();
+    const int j = blockIdx.z, c = blockIdx.x * 128 + threadIdx.x;
+    if (c >= a.cols[j]) return;
+    const int64_t per = (a.rows + kColChunks - 1) / kColChunks;
+    const int64_t r0 = blockIdx.y * per, r1 = r0 + per < a.rows ? r0 + per : a.rows;
+    a.partial[((int64_t)j * kColChunks + blockIdx.y) * a.max_cols + c] =
+        a.bf16[j] ? column_chunk(static_cast<const __nv_bfloat16*>(a.src[j]) + c, a.ld[j], r0, r1)
+                  : column_chunk(static_cast<const float*>(a.src[j]) + c, a.ld[j], r0, r1);
 }
-template <typename T>
-int column_sum(ltca_ctx* ctx, const T* src, int64_t ld, int64_t rows, int cols, float* dst, float* scratch) {
-    dim3 grid((cols + 127) / 128, kColChunks);
-    column_sum_partial_kernel<T><<<grid, 128, 0, ctx->stream>>>(src, ld, rows, cols, scratch);
-    LTCA_LAUNCH_OK(ctx, "column_sum_partial_kernel");
-    column_sum_final_kernel<<<(cols + 127) / 128, 128, 0, ctx->stream>>>(scratch, cols, dst);
-    LTCA_LAUNCH_OK(ctx, "column_sum_final_kernel");
+__global__ void __launch_bounds__(128) column_sum_final_kernel(const __grid_constant__ ColSum a) {
+    grid_launch_dependents();
+    grid_dependency_wait();
+    const int j = blockIdx.y, c = blockIdx.x * 128 + threadIdx.x;
+    if (c >= a.cols[j]) return;
+    a.dst[j][c] = column_chunk(a.partial + (int64_t)j * kColChunks * a.max_cols + c, a.max_cols, 0, kColChunks);
+}
+int column_sums(ltca_ctx* ctx, ColSum a, int64_t rows, float* scratch) {
+    if (a.n == 0) return LTCA_OK;
+    a.rows = rows;
+    a.partial = scratch;
+    const unsigned bx = (unsigned)((a.max_cols + 127) / 128);
+    LTCA_CUDA_OK(ctx, launch_dependent(column_sum_partial_kernel, dim3(bx, kColChunks, a.n), dim3(128), 0, ctx->stream, a));
+    LTCA_CUDA_OK(ctx, launch_dependent(column_sum_final_kernel, dim3(bx, a.n), dim3(128), 0, ctx->stream, a));
     return LTCA_OK;
 }
 size_t colsum_scratch_bytes(const ltca_tsa_params* t) {
     const int hw = t->H * t->head_width;
-    return align_up((size_t)kColChunks * (hw > t->E ? hw : t->E) * sizeof(float), 256);
+    return align_up((size_t)kMaxColJobs * kColChunks * (hw > t->E ? hw : t->E) * sizeof(float), 256);
+}
+
+// `xo` receives LayerNorm(x) (or x), `go` the gradient behind the dropout (null outputs: no such part); w: matrices to round.
+int prenorm_prepare(ltca_ctx* ctx, const ltca_tsa_params* t, const RowOut& xo, const RowOut* go, const CvtMany* w) {
+    PrepareArgs a;
+    memset(&a, 0, sizeof(a));
+    a.x = t->x; a.gamma = t->ln_gamma; a.beta = t->ln_beta;
+    a.xo = xo;
+    a.rows = (int64_t)t->B * t->S;
+    a.E = t->E;
+    a.use_ln = t->use_layer_norm;
+    a.eps = 1e-5f;
+    if (!t->use_layer_norm) a.gamma = a.beta = nullptr;
+    if (xo.f32 || xo.bf16) a.row_blocks = (int)((a.rows + kPrepareThreads / 32 - 1) / (kPrepareThreads / 32));
+    const int sms = ctx->sm_count > 0 ? ctx->sm_count : kPlanSms;
+    if (go && (go->f32 || go->bf16)) {
+        a.dy = t->dy;
+        a.go = *go;
+        a.p = t->dropout_prob;
+        a.seed = t->dropout_seed;
+        const int64_t blocks = (a.rows * a.E + 4 * kPrepareThreads - 1) / (4 * kPrepareThreads);
+        a.dy_blocks = (int)(blocks < 8 * sms ? blocks : 8 * sms);
+    }
+    int w_blocks = 0;
+    if (w && w->n) {
+        a.w = *w;
+        const uint32_t blocks = (w->start4[w->n] + 2 * kPrepareThreads - 1) / (2 * kPrepareThreads);
+        w_blocks = blocks < 4u * sms ? (int)blocks : 4 * sms;
+    }
+    if (a.row_blocks + a.dy_blocks + w_blocks == 0) return LTCA_OK;
+    LTCA_CUDA_OK(ctx, launch_dependent(prenorm_prepare_kernel, dim3((unsigned)(a.row_blocks + a.dy_blocks + w_blocks)),
+                                       dim3(kPrepareThreads), 0, ctx->stream, a));
+    return LTCA_OK;
+}
+int prenorm_finish(ltca_ctx* ctx, const ltca_tsa_params* t, const float* y) {
+    const int64_t n = (int64_t)t->B * t->S * t->E, blocks = (n + 511) / 512;
+    LTCA_CUDA_OK(ctx, launch_dependent(residual_dropout_kernel, dim3((unsigned)(blocks < 2368 ? blocks : 2368)), dim3(256), 0, ctx->stream,
+                                       y, t->x, t->out, n, t->use_residual, t->dropout_prob, t->dropout_seed));
+    return LTCA_OK;
 }
 
 struct Plan {
@@ -474,8 +650,11 @@ void fill_wide(const ltca_tsa_params* t, const TBufs& tb, WideArgs* w) {
 // `also_src` / `also_dst`: one more [rows, E] fp32 matrix (the backward's dy) to be rounded to bf16 by the same launch
 // that rounds x and the weights; *also_done says whether that happened (not on the paths that convert otherwise
 // or not at all).
+// `outer`: the FlashAttention form around this module; its LayerNorm (of outer->x) and its dropout (of outer->dy, into
+// outer_g as fp32 and into also_dst) take the place of those conversions, in the same launch as the weights'.
 int tensor_forward_core(ltca_ctx* ctx, const ltca_tsa_params* t, const TPlan& pl, char* w, TBufs* tb, int which,
-                        const float* also_src = nullptr, void* also_dst = nullptr, bool* also_done = nullptr) {
+                        const float* also_src = nullptr, void* also_dst = nullptr, bool* also_done = nullptr,
+                        const ltca_tsa_params* outer = nullptr, float* outer_g = nullptr) {
     char* rest = w;
     const bool saved = t->saved != nullptr;
     if (saved) w = reinterpret_cast<char*>(t->saved);
@@ -533,13 +712,23 @@ int tensor_forward_core(ltca_ctx* ctx, const ltca_tsa_params* t, const TPlan& pl
         int64_t nrows[6] = {pl.rows, E, E, E, HW, pl.rows};
         int ncols[6] = {E, HW, HW, HW, E, E};
         int n = convert_weights ? 5 : 1;
-        if (also_src) {
+        if (outer) {
+            CvtMany wm;
+            const RowOut xo{nullptr, reinterpret_cast<__nv_bfloat16*>(tb->xb), 0, Ep};
+            const RowOut go{outer_g, reinterpret_cast<__nv_bfloat16*>(also_dst), E, Ep};
+            const bool one = make_cvt_many(&wm, n - 1, src + 1, ld_src + 1, dst + 1, ld_dst + 1, nrows + 1, ncols + 1, nullptr);
+            if (!one && n > 1 && (rc = convert_many_bf16(ctx, n - 1, src + 1, ld_src + 1, dst + 1, ld_dst + 1, nrows + 1, ncols + 1)))
+                return rc;
+            if ((rc = prenorm_prepare(ctx, outer, xo, also_src ? &go : nullptr, one ? &wm : nullptr))) return rc;
+            if (also_done) *also_done = true;
+            n = 0;
+        } else if (also_src) {
             src[n] = also_src; dst[n] = also_dst; lo[n] = nullptr;
             ld_src[n] = E; ld_dst[n] = Ep; nrows[n] = pl.rows; ncols[n] = E;
             ++n;
             if (also_done) *also_done = true;
         }
-        if ((rc = convert_many_bf16(ctx, n, src, ld_src, dst, ld_dst, nrows, ncols, lo))) return rc;
+        if (n && (rc = convert_many_bf16(ctx, n, src, ld_src, dst, ld_dst, nrows, ncols, lo))) return rc;
     }
     if (pl.wide) {
         const void* whi[2] = {tb->wq, tb->wk};
@@ -601,7 +790,8 @@ int tensor_forward_core(ltca_ctx* ctx, const ltca_tsa_params* t, const TPlan& pl
     return ltca_attn_fwd(ctx, &a);
 }
 
-int tensor_forward(ltca_ctx* ctx, const ltca_tsa_params* t) {
+// `outer` (or null): the FlashAttention form around this module, `fused`: its first steps are done in here.
+int tensor_forward(ltca_ctx* ctx, const ltca_tsa_params* t, const ltca_tsa_params* outer, bool fused) {
     TPlan pl;
     int rc;
     if ((rc = make_tplan(t, &pl, keeps_for_backward(t)))) return rc;
@@ -612,7 +802,7 @@ int tensor_forward(ltca_ctx* ctx, const ltca_tsa_params* t) {
     float* y = reinterpret_cast<float*>(w);
     w += pl.y;
     TBufs tb;
-    if ((rc = tensor_forward_core(ctx, t, pl, w, &tb, 0))) return rc;
+    if ((rc = tensor_forward_core(ctx, t, pl, w, &tb, 0, nullptr, nullptr, nullptr, fused ? outer : nullptr))) return rc;
     GemmProblem gp;
     gp.M = (int)pl.rows; gp.N = t->E; gp.K = pl.HW;
     gp.a[0] = GemmOperand{tb.ctx, pl.HW, 0};
@@ -621,10 +811,12 @@ int tensor_forward(ltca_ctx* ctx, const ltca_tsa_params* t) {
     gp.bias[0] = t->bo;
     gp.ldc = t->E;
     if ((rc = gemm_sm100(ctx, gp))) return rc;
-    return residual_layer_norm(ctx, t, y, pl.rows);
+    return outer ? prenorm_finish(ctx, outer, y) : residual_layer_norm(ctx, t, y, pl.rows);
 }
 
-int tensor_backward(ltca_ctx* ctx, const ltca_tsa_params* t, bool want_dx, bool want_dw, float* colsum_scratch) {
+// `sums` collects the bias gradients (column sums of buffers that stay as they are until the call ends).
+int tensor_backward(ltca_ctx* ctx, const ltca_tsa_params* t, bool want_dx, bool want_dw, ColSum* sums,
+                    const ltca_tsa_params* outer, float* outer_g) {
     TPlan pl;
     int rc;
     if ((rc = make_tplan(t, &pl, true))) return rc;
@@ -642,7 +834,7 @@ int tensor_backward(ltca_ctx* ctx, const ltca_tsa_params* t, bool want_dx, bool 
     // the forward is recomputed, as the reference's caller does before each backward
     // (src/ml/ml_liquid_net.cu:715-721)
     bool dy_done = false;
-    if ((rc = tensor_forward_core(ctx, t, pl, w, &tb, 1, t->dy, dyb, &dy_done))) return rc;
+    if ((rc = tensor_forward_core(ctx, t, pl, w, &tb, 1, t->dy, dyb, &dy_done, outer, outer_g))) return rc;
     const int rows = (int)pl.rows, E = t->E, HW = pl.HW, Ep = pl.Ep;
     if (!dy_done && (rc = convert_rows_bf16(ctx, t->dy, E, dyb, Ep, pl.rows, E))) return rc;
     {   // dctx = dy Wo^T : Wo is stored [HW, E] = [N, K]
@@ -672,11 +864,10 @@ int tensor_backward(ltca_ctx* ctx, const ltca_tsa_params* t, bool want_dx, bool 
     const void* grads[3] = {dq, dk, dv};
     if (want_dw) {
         // bias gradients (FlashAttention form): column sums of the projection outputs' gradients
-        float* db[3] = {t->dbq, t->dbk, t->dbv};
-        for (int i = 0; i < 3; ++i)
-            if (db[i] && (rc = column_sum(ctx, reinterpret_cast<const __nv_bfloat16*>(grads[i]), HW, pl.rows, HW, db[i],
-                                          colsum_scratch))) return rc;
-        if (t->dbo && (rc = column_sum(ctx, t->dy, E, pl.rows, E, t->dbo, colsum_scratch))) return rc;
+        sums->add(dq, true, HW, HW, t->dbq);
+        sums->add(dk, true, HW, HW, t->dbk);
+        sums->add(dv, true, HW, HW, t->dbv);
+        sums->add(t->dy, false, E, E, t->dbo);
     }
     if (want_dx) {
         // dx = dq Wq^T + dk Wk^T + dv Wv^T : each W is stored [E, HW] = [N, K]; one accumulator tile
@@ -816,7 +1007,16 @@ int ltca_tsa_workspace_bytes(const ltca_tsa_params* t, int which, size_t* bytes_
     return LTCA_OK;
 }
 
-static int tsa_backward(ltca_ctx* ctx, const ltca_tsa_params* t, bool want_dx, bool want_dw);
+static int tsa_forward(ltca_ctx* ctx, const ltca_tsa_params* t, const ltca_tsa_params* outer, bool fused);
+static int tsa_backward(ltca_ctx* ctx, const ltca_tsa_params* t, bool want_dx, bool want_dw, ColSum* sums,
+                        const ltca_tsa_params* outer, float* outer_g);
+
+// Whether the core of the module takes the raw rows and runs the first steps of the FlashAttention form itself: the
+// streaming tensor pipeline, whose operands are bf16.  (The exact pipeline and the written-out-score path, which keeps a
+// second term of x, read fp32 rows.)
+static bool fuses_prenorm(const ltca_tsa_params* c, bool backward) {
+    return use_tensor(c, backward) && !use_wide(c, backward);
+}
 
 // FlashAttention form, forward: LayerNorm on the input, the core module, residual with the raw input, dropout.
 static int prenorm_forward(ltca_ctx* ctx, const ltca_tsa_params* t) {
@@ -825,29 +1025,19 @@ static int prenorm_forward(ltca_ctx* ctx, const ltca_tsa_params* t) {
     if (rc) return rc;
     if (!t->workspace || t->workspace_bytes < need)
         return fail(ctx, LTCA_ERR_WORKSPACE, "forward needs %zu bytes of workspace", need);
-    const int64_t rows = (int64_t)t->B * t->S;
-    const int64_t n = rows * t->E;
     char* w = reinterpret_cast<char*>(t->workspace);
     float* xin = reinterpret_cast<float*>(w);
     w += act_bytes(t);
     ltca_tsa_params c = core_form(t);
-    if (t->use_layer_norm) {
-        const int wpb = 8;
-        residual_layer_norm_kernel<<<(unsigned)((rows + wpb - 1) / wpb), wpb * 32, 0, ctx->stream>>>(
-            t->x, t->x, t->ln_gamma, t->ln_beta, xin, rows, t->E, 0, 1, 1e-5f);
-        LTCA_LAUNCH_OK(ctx, "residual_layer_norm_kernel");
+    const bool fused = fuses_prenorm(&c, keeps_for_backward(&c));
+    if (!fused && t->use_layer_norm) {
+        const RowOut xo{xin, nullptr, t->E, 0};
+        if ((rc = prenorm_prepare(ctx, t, xo, nullptr, nullptr))) return rc;
         c.x = xin;
     }
     c.workspace = w;
     c.workspace_bytes = t->workspace_bytes - act_bytes(t);
-    if ((rc = ltca_tsa_fwd(ctx, &c))) return rc;
-    if (t->use_residual && (rc = ltca_add_tensors(ctx, t->out, t->x, t->out, (size_t)n))) return rc;
-    if (t->dropout_prob > 0.f) {
-        const unsigned blocks = (unsigned)((n + 255) / 256 < 2368 ? (n + 255) / 256 : 2368);
-        dropout_kernel<<<blocks, 256, 0, ctx->stream>>>(t->out, t->out, n, t->dropout_prob, t->dropout_seed);
-        LTCA_LAUNCH_OK(ctx, "dropout_kernel");
-    }
-    return LTCA_OK;
+    return tsa_forward(ctx, &c, t, fused);
 }
 
 // FlashAttention form, backward (an extension: the reference class has no backward pass).
@@ -866,21 +1056,14 @@ static int prenorm_backward(ltca_ctx* ctx, const ltca_tsa_params* t, bool want_d
     float* gbuf = reinterpret_cast<float*>(w);  w += act;
     float* dxin = reinterpret_cast<float*>(w);  w += act;
     float* colsum_scratch = reinterpret_cast<float*>(reinterpret_cast<char*>(t->workspace) + need - colsum_scratch_bytes(t));
-    const int wpb = 8;
-    const unsigned row_blocks = (unsigned)((rows + wpb - 1) / wpb);
     ltca_tsa_params c = core_form(t);
-    if (t->use_layer_norm) {
-        residual_layer_norm_kernel<<<row_blocks, wpb * 32, 0, ctx->stream>>>(
-            t->x, t->x, t->ln_gamma, t->ln_beta, xin, rows, t->E, 0, 1, 1e-5f);
-        LTCA_LAUNCH_OK(ctx, "residual_layer_norm_kernel");
-        c.x = xin;
-    }
-    const float* g = t->dy;                      // gradient behind the dropout
-    if (t->dropout_prob > 0.f) {
-        const unsigned blocks = (unsigned)((n + 255) / 256 < 2368 ? (n + 255) / 256 : 2368);
-        dropout_kernel<<<blocks, 256, 0, ctx->stream>>>(t->dy, gbuf, n, t->dropout_prob, t->dropout_seed);
-        LTCA_LAUNCH_OK(ctx, "dropout_kernel");
-        g = gbuf;
+    const bool fused = fuses_prenorm(&c, true);
+    const bool drops = t->dropout_prob > 0.f;
+    const float* g = drops ? gbuf : t->dy;       // gradient behind the dropout
+    if (!fused) {
+        const RowOut xo{t->use_layer_norm ? xin : nullptr, nullptr, t->E, 0}, go{drops ? gbuf : nullptr, nullptr, t->E, 0};
+        if ((rc = prenorm_prepare(ctx, t, xo, &go, nullptr))) return rc;
+        if (t->use_layer_norm) c.x = xin;
     }
     const bool want_ln_params = want_dw && t->use_layer_norm && (t->dgamma || t->dbeta);
     const bool need_dxin = want_dx || want_ln_params;
@@ -888,28 +1071,32 @@ static int prenorm_backward(ltca_ctx* ctx, const ltca_tsa_params* t, bool want_d
     c.dx = dxin;
     c.workspace = w;
     c.workspace_bytes = t->workspace_bytes - 3 * act;
-    if ((rc = tsa_backward(ctx, &c, need_dxin, want_dw))) return rc;
-    if (!need_dxin) return LTCA_OK;
-    if (!t->use_layer_norm) {
-        if (want_dx) {
-            if (t->use_residual) return ltca_add_tensors(ctx, dxin, g, t->dx, (size_t)n);
+    ColSum sums;
+    memset(&sums, 0, sizeof(sums));
+    if ((rc = tsa_backward(ctx, &c, need_dxin, want_dw, &sums, fused ? t : nullptr, drops ? gbuf : nullptr))) return rc;
+    if (need_dxin && !t->use_layer_norm) {
+        if (want_dx && t->use_residual) {
+            if ((rc = ltca_add_tensors(ctx, dxin, g, t->dx, (size_t)n))) return rc;
+        } else if (want_dx) {
             LTCA_CUDA_OK(ctx, cudaMemcpyAsync(t->dx, dxin, (size_t)n * sizeof(float), cudaMemcpyDeviceToDevice, ctx->stream));
         }
-        return LTCA_OK;
+    } else if (need_dxin) {
+        // LayerNorm(x) is no longer needed: its buffer takes dxin * xhat, whose column sums are dgamma
+        float* prod = (want_ln_params && t->dgamma) ? xin : nullptr;
+        const int wpb = 8;
+        LTCA_CUDA_OK(ctx, launch_dependent(layer_norm_bwd_kernel, dim3((unsigned)((rows + wpb - 1) / wpb)), dim3(wpb * 32), 0, ctx->stream,
+                                           (const float*)dxin, t->x, t->ln_gamma, (want_dx && t->use_residual) ? g : nullptr,
+                                           want_dx ? t->dx : nullptr, prod, rows, t->E, 1e-5f));
+        if (want_ln_params) {
+            sums.add(dxin, false, t->E, t->E, t->dbeta);
+            sums.add(prod, false, t->E, t->E, t->dgamma);
+        }
     }
-    if (want_ln_params && t->dbeta && (rc = column_sum(ctx, dxin, t->E, rows, t->E, t->dbeta, colsum_scratch))) return rc;
-    // dx (or, when only parameter gradients are wanted, a dump into the no longer needed LayerNorm(x) buffer);
-    // dxin is overwritten by dxin * xhat, whose column sums are dgamma
-    float* dx_out = want_dx ? t->dx : xin;
-    layer_norm_bwd_kernel<<<row_blocks, wpb * 32, 0, ctx->stream>>>(
-        dxin, t->x, t->ln_gamma, (want_dx && t->use_residual) ? g : nullptr, dx_out,
-        (want_ln_params && t->dgamma) ? dxin : nullptr, rows, t->E, 1e-5f);
-    LTCA_LAUNCH_OK(ctx, "layer_norm_bwd_kernel");
-    if (want_ln_params && t->dgamma && (rc = column_sum(ctx, dxin, t->E, rows, t->E, t->dgamma, colsum_scratch))) return rc;
-    return LTCA_OK;
+    return column_sums(ctx, sums, rows, colsum_scratch);
 }
 
-int ltca_tsa_fwd(ltca_ctx* ctx, const ltca_tsa_params* t) {
+// `outer` (or null): the FlashAttention form around this module; see tensor_forward.
+static int tsa_forward(ltca_ctx* ctx, const ltca_tsa_params* t, const ltca_tsa_params* outer, bool fused) {
     int rc = check(ctx, t);
     if (rc) return rc;
     LTCA_CUDA_OK(ctx, cudaSetDevice(ctx->device));
@@ -919,7 +1106,7 @@ int ltca_tsa_fwd(ltca_ctx* ctx, const ltca_tsa_params* t) {
     if (t->dropout_prob < 0.f || t->dropout_prob >= 1.f)
         return fail(ctx, LTCA_ERR_INVALID, "dropout_prob must be in [0, 1)");
     if (t->pre_norm) return prenorm_forward(ctx, t);
-    if (use_tensor(t, keeps_for_backward(t))) return tensor_forward(ctx, t);
+    if (use_tensor(t, keeps_for_backward(t))) return tensor_forward(ctx, t, outer, fused);
     Plan pl;
     if ((rc = make_plan(t, &pl))) return rc;
     size_t need = 0;
@@ -934,10 +1121,14 @@ int ltca_tsa_fwd(ltca_ctx* ctx, const ltca_tsa_params* t) {
     const int rows = (int)pl.rows;
     const Gemm32Problem proj = {fb.ctx, t->wo, t->bo, y, rows, t->E, pl.HW, pl.HW, t->E, t->E};
     if ((rc = gemm_fp32(ctx, &proj, 1, 0, 0, false))) return rc;
-    return residual_layer_norm(ctx, t, y, pl.rows);
+    return outer ? prenorm_finish(ctx, outer, y) : residual_layer_norm(ctx, t, y, pl.rows);
 }
 
-static int tsa_backward(ltca_ctx* ctx, const ltca_tsa_params* t, bool want_dx, bool want_dw) {
+int ltca_tsa_fwd(ltca_ctx* ctx, const ltca_tsa_params* t) { return tsa_forward(ctx, t, nullptr, false); }
+
+// `sums` (or null): the FlashAttention form around this module collects the bias gradients' column sums and runs them.
+static int tsa_backward(ltca_ctx* ctx, const ltca_tsa_params* t, bool want_dx, bool want_dw, ColSum* sums,
+                        const ltca_tsa_params* outer, float* outer_g) {
     int rc = check(ctx, t);
     if (rc) return rc;
     LTCA_CUDA_OK(ctx, cudaSetDevice(ctx->device));
@@ -954,7 +1145,13 @@ static int tsa_backward(ltca_ctx* ctx, const ltca_tsa_params* t, bool want_dx, b
         return fail(ctx, LTCA_ERR_WORKSPACE, "backward needs %zu bytes of workspace", need);
     float* colsum_scratch =
         reinterpret_cast<float*>(reinterpret_cast<char*>(t->workspace) + need - colsum_scratch_bytes(t));
-    if (use_tensor(t, true)) return tensor_backward(ctx, t, want_dx, want_dw, colsum_scratch);
+    ColSum own;
+    memset(&own, 0, sizeof(own));
+    ColSum* jobs = sums ? sums : &own;
+    if (use_tensor(t, true)) {
+        if ((rc = tensor_backward(ctx, t, want_dx, want_dw, jobs, outer, outer_g))) return rc;
+        return column_sums(ctx, own, (int64_t)t->B * t->S, colsum_scratch);
+    }
     Plan pl;
     if ((rc = make_plan(t, &pl))) return rc;
     if (!t->workspace || t->workspace_bytes < need)
@@ -981,10 +1178,10 @@ static int tsa_backward(ltca_ctx* ctx, const ltca_tsa_params* t, bool want_dx, b
     if ((rc = ltca_attn_bwd(ctx, &a))) return rc;
     if (want_dw) {
         // bias gradients (FlashAttention form): column sums of the projection outputs' gradients
-        if (t->dbq && (rc = column_sum(ctx, dq, HW, pl.rows, HW, t->dbq, colsum_scratch))) return rc;
-        if (t->dbk && (rc = column_sum(ctx, dk, HW, pl.rows, HW, t->dbk, colsum_scratch))) return rc;
-        if (t->dbv && (rc = column_sum(ctx, dv, HW, pl.rows, HW, t->dbv, colsum_scratch))) return rc;
-        if (t->dbo && (rc = column_sum(ctx, t->dy, E, pl.rows, E, t->dbo, colsum_scratch))) return rc;
+        jobs->add(dq, false, HW, HW, t->dbq);
+        jobs->add(dk, false, HW, HW, t->dbk);
+        jobs->add(dv, false, HW, HW, t->dbv);
+        jobs->add(t->dy, false, E, E, t->dbo);
     }
     if (want_dx) {
         const Gemm32Problem terms[3] = {{dq, t->wq, nullptr, t->dx, rows, E, HW, HW, HW, E},
@@ -1001,17 +1198,17 @@ static int tsa_backward(ltca_ctx* ctx, const ltca_tsa_params* t, bool want_dx, b
                                      {fb.ctx, t->dy, nullptr, t->dwo, HW, E, rows, HW, E, E}};
         if ((rc = gemm_fp32(ctx, dw, 4, 1, 0, false, dctx, pl.buf))) return rc;
     }
-    return LTCA_OK;
+    return column_sums(ctx, own, pl.rows, colsum_scratch);
 }
 
 int ltca_tsa_bwd_data(ltca_ctx* ctx, const ltca_tsa_params* t) {
-    return tsa_backward(ctx, t, true, false);
+    return tsa_backward(ctx, t, true, false, nullptr, nullptr, nullptr);
 }
 int ltca_tsa_bwd_weights(ltca_ctx* ctx, const ltca_tsa_params* t) {
-    return tsa_backward(ctx, t, false, true);
+    return tsa_backward(ctx, t, false, true, nullptr, nullptr, nullptr);
 }
 int ltca_tsa_bwd(ltca_ctx* ctx, const ltca_tsa_params* t) {
-    return tsa_backward(ctx, t, true, true);
+    return tsa_backward(ctx, t, true, true, nullptr, nullptr, nullptr);
 }
 
 }  // extern "C"
