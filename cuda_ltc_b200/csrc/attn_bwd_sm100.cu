@@ -25,6 +25,7 @@
 #include <type_traits>
 
 #include "host_common.h"
+#include "attn_mask.cuh"
 #include "sm100_ptx.cuh"
 #include "trace.cuh"
 
@@ -58,7 +59,7 @@ struct BwdArgs {
     const float* delta;              // [B*H, Sq_pad]
     void *dq, *dk, *dv;
     ltca_strides dqs, dks, dvs;
-    const float* keep_mask;
+    MaskArgs mask;
     const int32_t* kv_len;
     uint32_t* status;
 };
@@ -212,7 +213,7 @@ __device__ __forceinline__ void pack32(const uint32_t (&v)[32], uint32_t (&hi)[1
 // kSplit (fp32 gradients out): dS is written as two bf16 terms and the dQ contraction runs once
 // per term, so that the 2^-9 rounding of a single bf16 dS does not dominate the error of an fp32
 // result.
-template <typename OutT, bool kSplit>
+template <typename OutT, bool kSplit, bool kMask>
 __global__ void __launch_bounds__(kThreads, 1)
 attn_bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
                          const __grid_constant__ CUtensorMap tmap_do,
@@ -392,13 +393,15 @@ attn_bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
         const uint32_t tDS = tmem_base + lane_base + 384 + t * 32 + half * 16;
         const uint32_t tDSlo = tDS + 64;
         const float c2 = a.scale_log2;
-        const bool general = (a.keep_mask != nullptr) || (a.use_clamp != 0);
+        const bool general = kMask || (a.use_clamp != 0);
         const int64_t srow = ((int64_t)b * a.H + h) * a.Sq_pad + qi;      // qi < Sq_pad by construction
         const float lse2 = a.lse2[srow];
         const float dlt = a.delta[srow];
 
         bool ok = true;
         for (int j = 0; j < n_t; ++j) {
+            uint32_t keep = ~0u;
+            if (kMask) keep = mask_bits_of_queries(a.mask, b, q0 + wq * 32, j * kStep + half * 32);
             ok = mbar_wait_warp(bar_sdp_full(t), (uint32_t)(j & 1), wc, 0x60 + t);
             if (!ok) break;
             tc_fence_after_sync();
@@ -424,16 +427,12 @@ attn_bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
                 int lim = kvlen;
                 if (a.causal) lim = min(lim, qi + a.causal_off + 1);
                 lim -= k0 + half * 32;
-                const float* mrow = nullptr;
-                if (a.keep_mask && qi < a.Sq)
-                    mrow = a.keep_mask + ((int64_t)b * a.Sq + qi) * a.Sk + k0 + half * 32;
 #pragma unroll
                 for (int c = 0; c < 32; ++c) {
                     const float sv = __uint_as_float(s[c]);
                     const float p = fast_exp2(fmaf(sv, c2, -lse2));
                     float d = p * (__uint_as_float(dp[c]) - dlt);
-                    bool vis = c < lim;
-                    if (mrow && vis) vis = (__ldg(mrow + c) != 0.0f);
+                    const bool vis = c < lim && (keep >> c & 1u);
                     if (a.use_clamp && sv >= a.clamp_raw) d = 0.f;
                     dp[c] = __float_as_uint(vis ? d : 0.f);
                 }
@@ -509,7 +508,7 @@ attn_bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
 // (bf16 pairs in the first 16, the kSplit low-order term in the next 16), so neither thread
 // ever overwrites scores the other has not read yet.
 // ---------------------------------------------------------------------------------------------
-template <typename OutT, bool kSplit>
+template <typename OutT, bool kSplit, bool kMask>
 __global__ void __launch_bounds__(kThreads, 1)
 attn_bwd_dkv_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
                           const __grid_constant__ CUtensorMap tmap_do,
@@ -699,13 +698,15 @@ attn_bwd_dkv_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
         const uint32_t tDV = tmem_base + lane_base + t * 256 + 128 + half * 32;
         const uint32_t tDK = tDV + 64;
         const float c2 = a.scale_log2;
-        const bool general = (a.keep_mask != nullptr) || (a.use_clamp != 0);
+        const bool general = kMask || (a.use_clamp != 0);
         const bool key_live = kj < kvlen;
 
         bool ok = true;
         if (active[t]) {
             for (int j = j_begin[t]; j < n_q; ++j) {
                 const int it = j - j_begin[t];
+                uint32_t keep = ~0u;
+                if (kMask) keep = mask_bits_of_key(a.mask, b, j * kStep + half * 32, kj);
                 ok = mbar_wait_warp(bar_sdp_full(t), (uint32_t)(it & 1), wc, 0x90 + t);
                 if (!ok) break;
                 tc_fence_after_sync();
@@ -741,9 +742,7 @@ attn_bwd_dkv_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
                             const float sv = __uint_as_float(s[c]);
                             float p = fast_exp2(fmaf(sv, c2, -ls[e]));
                             float d = p * (__uint_as_float(dp[c]) - dl[e]);
-                            bool vis = key_live && (!a.causal || (kj <= q0 + c + a.causal_off));
-                            if (vis && a.keep_mask && (q0 + c) < a.Sq)
-                                vis = a.keep_mask[((int64_t)b * a.Sq + q0 + c) * a.Sk + kj] != 0.0f;
+                            const bool vis = key_live && (!a.causal || (kj <= q0 + c + a.causal_off)) && (keep >> c & 1u);
                             if (a.use_clamp && sv >= a.clamp_raw) {
                                 p = fast_exp2(a.clamp_log2 - ls[e]);
                                 d = 0.f;
@@ -879,6 +878,7 @@ __device__ __forceinline__ void store_row16_bf16(__nv_bfloat16* dst, const uint3
     }
 }
 
+template <bool kMask>
 __global__ void __launch_bounds__(kThreads, 1)
 attn_bwd_dkv4_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
                            const __grid_constant__ CUtensorMap tmap_do,
@@ -1104,7 +1104,7 @@ attn_bwd_dkv4_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
         const uint32_t tDV = tmem_base + lane_base + 384 + 16 * cq;
         const uint32_t tDK = tDV + 64;
         const float c2 = a.scale_log2;
-        const bool general = (a.keep_mask != nullptr) || (a.use_clamp != 0);
+        const bool general = kMask || (a.use_clamp != 0);
 
         int g = 0, na = 0;
         bool ok = true;
@@ -1130,6 +1130,8 @@ attn_bwd_dkv4_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
                 continue;
             }
             uint32_t s[32], dp[32];
+            uint32_t keep = ~0u;
+            if (kMask) keep = mask_bits_of_key(a.mask, b, j_begin * kQStep + cq * 32, kj);
             ok = mbar_wait_warp(bar_sdp_full, (uint32_t)(g & 1), wc, 0xc0);
             if (!ok) break;
             tc_fence_after_sync();
@@ -1164,9 +1166,7 @@ attn_bwd_dkv4_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
                             const float sv = __uint_as_float(s[c]);
                             float p = fast_exp2(fmaf(sv, c2, -ls[e]));
                             float d = p * (__uint_as_float(dp[c]) - dl[e]);
-                            bool vis = key_live && (!a.causal || (kj <= q0 + c + a.causal_off));
-                            if (vis && a.keep_mask && (q0 + c) < a.Sq)
-                                vis = a.keep_mask[((int64_t)b * a.Sq + q0 + c) * a.Sk + kj] != 0.0f;
+                            const bool vis = key_live && (!a.causal || (kj <= q0 + c + a.causal_off)) && (keep >> c & 1u);
                             if (a.use_clamp && sv >= a.clamp_raw) {
                                 p = fast_exp2(a.clamp_log2 - ls[e]);
                                 d = 0.f;
@@ -1230,6 +1230,7 @@ attn_bwd_dkv4_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
                 // (P^T and dS^T are announced before the next S^T / dP^T are awaited: the tensor pipe is
                 // the busier unit in this kernel and must get this step's accumulations as early as possible)
                 if (it + 1 < n_it) {
+                    if (kMask) keep = mask_bits_of_key(a.mask, b, (j + 1) * kQStep + cq * 32, kj);
                     ok = mbar_wait_warp(bar_sdp_full, (uint32_t)((g + 1) & 1), wc, 0xc0);
                     if (!ok) break;
                     tc_fence_after_sync();
@@ -1349,6 +1350,7 @@ static_assert(FusedSmem::kDynBytes <= 227 * 1024, "shared memory plan of the fus
 constexpr int kFusedCtrlRegs = 64;   // the MMA thread of dP^T / dK / dQ_j holds three more operand descriptors
 static_assert(512 * kMathRegs + 128 * kFusedCtrlRegs <= kThreads * kLaunchRegs, "register budget");
 
+template <bool kMask>
 __global__ void __launch_bounds__(kThreads, 1)
 attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
                             const __grid_constant__ CUtensorMap tmap_do,
@@ -1620,7 +1622,7 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
         const uint32_t tDV = tmem_base + lane_base + 384 + 16 * cq;
         const uint32_t tDK = tDV + 64;
         const float c2 = a.scale_log2;
-        const bool general = (a.keep_mask != nullptr) || (a.use_clamp != 0);
+        const bool general = kMask || (a.use_clamp != 0);
         // this thread's 64 bytes of its dS^T row (32 query columns of key `row`): block cq / 2, 16-byte chunks
         // 4 (cq % 2) .. + 3, swizzled with the row; the dQ_j staging uses the same geometry with fp32 columns
         // 16 cq .. + 15 of query `row`: box cq / 2, chunks 4 (cq % 2) .. + 3
@@ -1675,6 +1677,8 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
                 // S^T and dP^T of this step into registers (defined afresh in every iteration, so that they are
                 // not carried round the loop); the next step's may then be computed
                 uint32_t s[32], dp[32];
+                uint32_t keep = ~0u;
+                if (kMask) keep = mask_bits_of_key(a.mask, b, j * kQStep + cq * 32, kj);
                 ok = mbar_wait_warp(bar_sdp_full, (uint32_t)(g & 1), wc, 0xc0);
                 if (!ok) break;
                 LTCA_TRACE_EVT(0x10 + (g << 8));
@@ -1706,9 +1710,7 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
                             const float sv = __uint_as_float(s[c]);
                             float pv = fast_exp2(fmaf(sv, c2, -ls[e]));
                             float d = pv * (__uint_as_float(dp[c]) - dl[e]);
-                            bool vis = key_live && (!a.causal || (kj <= q0 + c + a.causal_off));
-                            if (vis && a.keep_mask && (q0 + c) < a.Sq)
-                                vis = a.keep_mask[((int64_t)b * a.Sq + q0 + c) * a.Sk + kj] != 0.0f;
+                            const bool vis = key_live && (!a.causal || (kj <= q0 + c + a.causal_off)) && (keep >> c & 1u);
                             if (a.use_clamp && sv >= a.clamp_raw) {
                                 pv = fast_exp2(a.clamp_log2 - ls[e]);
                                 d = 0.f;
@@ -1909,6 +1911,7 @@ struct Dq4Smem {
     static constexpr int kDynBytes = kMiscOff + 16 + 4 * kItemSlots + 1024;
 };
 
+template <bool kMask>
 __global__ void __launch_bounds__(kThreads, 1)
 attn_bwd_dq4_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
                           const __grid_constant__ CUtensorMap tmap_do,
@@ -2131,7 +2134,7 @@ attn_bwd_dq4_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
         const uint32_t tDP = tS + 128;
         const uint32_t tDQ = tmem_base + lane_base + 320 + 16 * cq;
         const float c2 = a.scale_log2;
-        const bool general = (a.keep_mask != nullptr) || (a.use_clamp != 0);
+        const bool general = kMask || (a.use_clamp != 0);
 
         int g = 0, na = 0;
         bool ok = true;
@@ -2157,6 +2160,8 @@ attn_bwd_dq4_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
             const float dlt = a.delta[srow];
 
             uint32_t s[32], dp[32];
+            uint32_t keep = ~0u;
+            if (kMask) keep = mask_bits_of_queries(a.mask, b, q0 + wq * 32, cq * 32);
             ok = mbar_wait_warp(bar_sdp_full, (uint32_t)(g & 1), wc, 0xf0);
             if (!ok) break;
             tc_fence_after_sync();
@@ -2176,16 +2181,12 @@ attn_bwd_dq4_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
                     int vis_lim = kvlen;
                     if (a.causal) vis_lim = min(vis_lim, qi + a.causal_off + 1);
                     vis_lim -= k0 + cq * 32;
-                    const float* mrow = nullptr;
-                    if (a.keep_mask && qi < a.Sq)
-                        mrow = a.keep_mask + ((int64_t)b * a.Sq + qi) * a.Sk + k0 + cq * 32;
 #pragma unroll
                     for (int c = 0; c < 32; ++c) {
                         const float sv = __uint_as_float(s[c]);
                         const float p = fast_exp2(fmaf(sv, c2, -lse2));
                         float d = p * (__uint_as_float(dp[c]) - dlt);
-                        bool vis = c < vis_lim;
-                        if (mrow && vis) vis = (__ldg(mrow + c) != 0.0f);
+                        const bool vis = c < vis_lim && (keep >> c & 1u);
                         if (a.use_clamp && sv >= a.clamp_raw) d = 0.f;
                         dp[c] = __float_as_uint(vis ? d : 0.f);
                     }
@@ -2214,6 +2215,7 @@ attn_bwd_dq4_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
                 // written below was released before S and dP of this step were even issued.)
                 const bool more = it + 1 < n_it;
                 if (more) {
+                    if (kMask) keep = mask_bits_of_queries(a.mask, b, q0 + wq * 32, (it + 1) * kKStep + cq * 32);
                     ok = mbar_wait_warp(bar_sdp_full, (uint32_t)((g + 1) & 1), wc, 0xf0);
                     if (!ok) break;
                     tc_fence_after_sync();
@@ -2307,8 +2309,8 @@ size_t dq_acc_bytes(const ltca_attn_params* p) {
 // the two paths are within 5 % of each other, in the fused kernel's favour when the inputs come from HBM.)
 bool use_fused(const ltca_attn_params* p) { return p->dtype == LTCA_BF16 && !p->bwd_deterministic; }
 
-template <typename OutT>
-int launch_main(ltca_ctx* ctx, const ltca_attn_params* p, const void* q, const void* k, const void* v,
+template <typename OutT, bool kMask>
+int launch_main(ltca_ctx* ctx, const ltca_attn_params* p, const void* mask_words, const void* q, const void* k, const void* v,
                 const void* dout, const ltca_strides& qs, const ltca_strides& ks, const ltca_strides& vs,
                 const ltca_strides& dos, const float* lse2, const float* delta, float* dq_acc) {
     CUtensorMap tq128, tdo128, tk64, tv64, tq64, tdo64, tk128, tv128;
@@ -2336,14 +2338,14 @@ int launch_main(ltca_ctx* ctx, const ltca_attn_params* p, const void* q, const v
     a.lse2 = lse2; a.delta = delta;
     a.dq = p->dq; a.dk = p->dk; a.dv = p->dv;
     a.dqs = p->dq_strides; a.dks = p->dk_strides; a.dvs = p->dv_strides;
-    a.keep_mask = p->keep_mask;
+    a.mask = mask_args(p, mask_words);
     a.kv_len = p->kv_len;
     a.status = ctx->d_status;
 
     if constexpr (sizeof(OutT) == 2) {
         if (dq_acc) {
             static SmemOptIn opt_fused;
-            LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(opt_fused, ctx->device, attn_bwd_fused_sm100_kernel,
+            LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(opt_fused, ctx->device, attn_bwd_fused_sm100_kernel<kMask>,
                                                   FusedSmem::kDynBytes));
             ItemGrid ig;
             ig.nblk = (p->Sk + kTile - 1) / kTile;
@@ -2357,7 +2359,7 @@ int launch_main(ltca_ctx* ctx, const ltca_attn_params* p, const void* q, const v
             if ((rc = make_tmap_bhsd(ctx, &tdv, p->dv, 2, p->B, p->H, p->Sk, kD, p->dv_strides, 64, kTile))) return rc;
             const ltca_strides accs{(int64_t)p->H * a.Sq_pad * kD, (int64_t)a.Sq_pad * kD, kD};
             if ((rc = make_tmap_bhsd(ctx, &tacc, dq_acc, 4, p->B, p->H, a.Sq_pad, kD, accs, 32, kTile))) return rc;
-            LTCA_CUDA_OK(ctx, launch_dependent_if(small_attention_call(p), attn_bwd_fused_sm100_kernel, dim3(n_cta), dim3(kThreads), FusedSmem::kDynBytes,
+            LTCA_CUDA_OK(ctx, launch_dependent_if(small_attention_call(p), attn_bwd_fused_sm100_kernel<kMask>, dim3(n_cta), dim3(kThreads), FusedSmem::kDynBytes,
                                                ctx->stream, tq128, tdo128, tk128, tv128, tdk, tdv, tacc, a, ig));
             LTCA_LAUNCH_OK(ctx, "attn_bwd_fused_sm100_kernel");
             kernel_timing_mark(ctx, 2);
@@ -2370,16 +2372,10 @@ int launch_main(ltca_ctx* ctx, const ltca_attn_params* p, const void* q, const v
             return LTCA_OK;
         }
     }
-    auto kdq = attn_bwd_dq_sm100_kernel<OutT, sizeof(OutT) == 4>;
-    auto kdkv = attn_bwd_dkv_sm100_kernel<OutT, sizeof(OutT) == 4>;
-    static SmemOptIn opt_dq, opt_dkv;         // one pair per template instantiation
-    LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(opt_dq, ctx->device, kdq, DqSmem::kDynBytes));
-    LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(opt_dkv, ctx->device, kdkv, DkvSmem::kDynBytes));
-    bool dq_launched = false;
     if constexpr (sizeof(OutT) == 2) {
         {
             static SmemOptIn opt_dq4;
-            LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(opt_dq4, ctx->device, attn_bwd_dq4_sm100_kernel, Dq4Smem::kDynBytes));
+            LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(opt_dq4, ctx->device, attn_bwd_dq4_sm100_kernel<kMask>, Dq4Smem::kDynBytes));
             ItemGrid ig;
             ig.nblk = (p->Sq + kTile - 1) / kTile;
             ig.H = p->H;
@@ -2389,22 +2385,14 @@ int launch_main(ltca_ctx* ctx, const ltca_attn_params* p, const void* q, const v
             const int n_cta = ig.n_items < ctx->sm_count ? ig.n_items : ctx->sm_count;
             CUtensorMap tdq;
             if ((rc = make_tmap_bhsd(ctx, &tdq, p->dq, 2, p->B, p->H, p->Sq, kD, p->dq_strides, 64, kTile))) return rc;
-            LTCA_CUDA_OK(ctx, launch_dependent_if(small_attention_call(p), attn_bwd_dq4_sm100_kernel, dim3(n_cta), dim3(kThreads), Dq4Smem::kDynBytes,
+            LTCA_CUDA_OK(ctx, launch_dependent_if(small_attention_call(p), attn_bwd_dq4_sm100_kernel<kMask>, dim3(n_cta), dim3(kThreads), Dq4Smem::kDynBytes,
                                                ctx->stream, tq128, tdo128, tk128, tv128, tdq, a, ig));
             LTCA_LAUNCH_OK(ctx, "attn_bwd_dq4_sm100_kernel");
-            dq_launched = true;
         }
-    }
-    if (!dq_launched) {
-        dim3 gq((p->Sq + 2 * kTile - 1) / (2 * kTile), p->H, p->B);
-        LTCA_CUDA_OK(ctx, launch_dependent_if(small_attention_call(p), kdq, gq, dim3(kThreads), DqSmem::kDynBytes, ctx->stream, tq128, tdo128, tk64, tv64, a));
-        LTCA_LAUNCH_OK(ctx, "attn_bwd_dq_sm100_kernel");
-    }
-    kernel_timing_mark(ctx, 2);
-    if constexpr (sizeof(OutT) == 2) {
+        kernel_timing_mark(ctx, 2);
         {
             static SmemOptIn opt_dkv4;
-            LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(opt_dkv4, ctx->device, attn_bwd_dkv4_sm100_kernel,
+            LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(opt_dkv4, ctx->device, attn_bwd_dkv4_sm100_kernel<kMask>,
                                                   Dkv4Smem::kDynBytes));
             ItemGrid ig;
             ig.nblk = (p->Sk + kTile - 1) / kTile;
@@ -2416,16 +2404,24 @@ int launch_main(ltca_ctx* ctx, const ltca_attn_params* p, const void* q, const v
             CUtensorMap tdk, tdv;
             if ((rc = make_tmap_bhsd(ctx, &tdk, p->dk, 2, p->B, p->H, p->Sk, kD, p->dk_strides, 64, kTile))) return rc;
             if ((rc = make_tmap_bhsd(ctx, &tdv, p->dv, 2, p->B, p->H, p->Sk, kD, p->dv_strides, 64, kTile))) return rc;
-            LTCA_CUDA_OK(ctx, launch_dependent_if(small_attention_call(p), attn_bwd_dkv4_sm100_kernel, dim3(n_cta), dim3(kThreads), Dkv4Smem::kDynBytes,
+            LTCA_CUDA_OK(ctx, launch_dependent_if(small_attention_call(p), attn_bwd_dkv4_sm100_kernel<kMask>, dim3(n_cta), dim3(kThreads), Dkv4Smem::kDynBytes,
                                                ctx->stream, tq128, tdo128, tk128, tv128, tdk, tdv, a, ig));
             LTCA_LAUNCH_OK(ctx, "attn_bwd_dkv4_sm100_kernel");
-            kernel_timing_mark(ctx, 3);
-            return LTCA_OK;
         }
+    } else {
+        auto kdq = attn_bwd_dq_sm100_kernel<OutT, sizeof(OutT) == 4, kMask>;
+        auto kdkv = attn_bwd_dkv_sm100_kernel<OutT, sizeof(OutT) == 4, kMask>;
+        static SmemOptIn opt_dq, opt_dkv;         // one pair per template instantiation
+        LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(opt_dq, ctx->device, kdq, DqSmem::kDynBytes));
+        LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(opt_dkv, ctx->device, kdkv, DkvSmem::kDynBytes));
+        dim3 gq((p->Sq + 2 * kTile - 1) / (2 * kTile), p->H, p->B);
+        LTCA_CUDA_OK(ctx, launch_dependent_if(small_attention_call(p), kdq, gq, dim3(kThreads), DqSmem::kDynBytes, ctx->stream, tq128, tdo128, tk64, tv64, a));
+        LTCA_LAUNCH_OK(ctx, "attn_bwd_dq_sm100_kernel");
+        kernel_timing_mark(ctx, 2);
+        dim3 gk((p->Sk + 2 * kTile - 1) / (2 * kTile), p->H, p->B);
+        LTCA_CUDA_OK(ctx, launch_dependent_if(small_attention_call(p), kdkv, gk, dim3(kThreads), DkvSmem::kDynBytes, ctx->stream, tq64, tdo64, tk128, tv128, a));
+        LTCA_LAUNCH_OK(ctx, "attn_bwd_dkv_sm100_kernel");
     }
-    dim3 gk((p->Sk + 2 * kTile - 1) / (2 * kTile), p->H, p->B);
-    LTCA_CUDA_OK(ctx, launch_dependent_if(small_attention_call(p), kdkv, gk, dim3(kThreads), DkvSmem::kDynBytes, ctx->stream, tq64, tdo64, tk128, tv128, a));
-    LTCA_LAUNCH_OK(ctx, "attn_bwd_dkv_sm100_kernel");
     kernel_timing_mark(ctx, 3);
     return LTCA_OK;
 }
@@ -2448,6 +2444,8 @@ int launch_attn_bwd_sm100(ltca_ctx* ctx, const ltca_attn_params* p) {
     const size_t pq = align_up((size_t)p->B * p->H * p->Sq * kD * 2, 256);
     const size_t pk = align_up((size_t)p->B * p->H * p->Sk * kD * 2, 256);
     if (p->dtype == LTCA_F32) need += 2 * pq + 2 * pk;
+    const void* words = nullptr;
+    if (int rc = mask_words_of(ctx, p, need, &words)) return rc;
     if (!p->workspace || p->workspace_bytes < need)
         return fail(ctx, LTCA_ERR_WORKSPACE, "tensor-pipe backward needs %zu bytes of workspace", need);
     const int es = elem_size(p->dtype);
@@ -2480,8 +2478,8 @@ int launch_attn_bwd_sm100(ltca_ctx* ctx, const ltca_attn_params* p) {
     if (p->dtype == LTCA_BF16) kernel_timing_mark(ctx, 1);
 
     if (p->dtype == LTCA_BF16)
-        return launch_main<__nv_bfloat16>(ctx, p, p->q, p->k, p->v, p->dout, p->q_strides, p->k_strides,
-                                          p->v_strides, p->do_strides, lse2, delta, dq_acc);
+        return (p->keep_mask ? launch_main<__nv_bfloat16, true> : launch_main<__nv_bfloat16, false>)(
+            ctx, p, words, p->q, p->k, p->v, p->dout, p->q_strides, p->k_strides, p->v_strides, p->do_strides, lse2, delta, dq_acc);
 
     // fp32 storage: bf16 copies of the four operands, fp32 gradients out
     void* qb = w;  w += pq;
@@ -2494,7 +2492,8 @@ int launch_attn_bwd_sm100(ltca_ctx* ctx, const ltca_attn_params* p) {
     kernel_timing_mark(ctx, 1);
     ltca_strides cq{(int64_t)p->H * p->Sq * kD, (int64_t)p->Sq * kD, kD};
     ltca_strides ck{(int64_t)p->H * p->Sk * kD, (int64_t)p->Sk * kD, kD};
-    return launch_main<float>(ctx, p, qb, kb, vb, gb, cq, ck, ck, cq, lse2, delta, nullptr);
+    return (p->keep_mask ? launch_main<float, true> : launch_main<float, false>)(ctx, p, words, qb, kb, vb, gb, cq, ck, ck, cq, lse2,
+                                                                                 delta, nullptr);
 }
 
 }  // namespace ltca

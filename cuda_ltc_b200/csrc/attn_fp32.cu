@@ -8,6 +8,7 @@
 // and row sums are half-warp shuffle reductions.
 #include <math.h>
 
+#include "attn_mask.cuh"
 #include "host_common.h"
 #include "sm100_ptx.cuh"
 
@@ -240,22 +241,6 @@ __device__ __forceinline__ void ld_row(float (&x)[NR], const float* p) {       /
         x[0] = v.x; x[1] = v.y;
     } else {
         x[0] = *p;
-    }
-}
-
-// Dense mask as bits: word (row, i) holds keys 32 i .. 32 i + 31 of a query row.  Both passes and all heads read the same
-// mask; packed once it is 1/32 of the traffic and one load for 32 keys.  One warp per word, coalesced reads and a vote.
-__global__ void __launch_bounds__(256) attn_mask_bits_kernel(const float* __restrict__ mask, uint32_t* __restrict__ words, int64_t rows,
-                                                             int Sk, int nw) {
-    grid_launch_dependents();
-    grid_dependency_wait();
-    const int lane = threadIdx.x & 31;
-    for (int64_t w = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); w < rows * nw; w += (int64_t)gridDim.x * 8) {
-        const int64_t r = w / nw;
-        const int k = (int)(w % nw) * 32 + lane;
-        const bool keep = k < Sk && __ldg(mask + r * Sk + k) != 0.f;
-        const uint32_t bits = __ballot_sync(0xffffffffu, keep);
-        if (lane == 0) words[w] = bits;
     }
 }
 
@@ -827,11 +812,6 @@ int run_rows(ltca_ctx* ctx, const CoreArgs& a, bool bwd) {
 template <typename T, int DP>
 int run_rows(ltca_ctx* ctx, const CoreArgs& a, bool bwd) {
     if (!a.keep_mask) return run_rows<T, DP, false>(ctx, a, bwd);
-    if (bwd) {
-        const int64_t rows = (int64_t)a.B * a.Sq, blocks = (rows * a.mask_nw + 7) / 8, most = 16ll * ctx->sm_device;
-        LTCA_CUDA_OK(ctx, launch_dependent(attn_mask_bits_kernel, dim3((unsigned)(blocks < most ? blocks : most)), dim3(256), 0,
-                                           ctx->stream, a.keep_mask, const_cast<uint32_t*>(a.mask_bits), rows, a.Sk, a.mask_nw));
-    }
     return run_rows<T, DP, true>(ctx, a, bwd);
 }
 
@@ -1043,9 +1023,7 @@ int dispatch(ltca_ctx* ctx, const CoreArgs& a, bool bwd) {
 // delta, and the dense mask as bits (the kernels for head_dim up to 128)
 static size_t delta_bytes(const ltca_attn_params* p) { return align_up((size_t)p->B * p->H * p->Sq * sizeof(float), 256); }
 size_t attn_bwd_fp32_workspace(const ltca_attn_params* p) {
-    size_t n = delta_bytes(p);
-    if (p->keep_mask && p->D <= 128) n += align_up((size_t)p->B * p->Sq * ((p->Sk + 31) / 32) * 4, 256);
-    return n;
+    return delta_bytes(p) + (p->D <= 128 ? mask_words_bytes(p) : 0);
 }
 
 int launch_attn_fwd_fp32(ltca_ctx* ctx, const ltca_attn_params* p) {
@@ -1063,8 +1041,13 @@ int launch_attn_bwd_fp32(ltca_ctx* ctx, const ltca_attn_params* p) {
                     attn_bwd_fp32_workspace(p));
     CoreArgs a = make_args(p);
     a.delta = reinterpret_cast<float*>(p->workspace);
-    a.mask_bits = reinterpret_cast<const uint32_t*>(reinterpret_cast<const char*>(p->workspace) + delta_bytes(p));
-    a.mask_nw = (p->Sk + 31) / 32;
+    if (p->D <= 128) {
+        const void* words = nullptr;
+        if (int rc = mask_words_of(ctx, p, delta_bytes(p), &words)) return rc;
+        const MaskArgs m = mask_args(p, words);
+        a.mask_bits = m.by_query;
+        a.mask_nw = m.nk;
+    }
     return p->dtype == LTCA_BF16 ? dispatch<__nv_bfloat16>(ctx, a, true) : dispatch<float>(ctx, a, true);
 }
 

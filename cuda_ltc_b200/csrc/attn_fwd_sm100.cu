@@ -28,6 +28,7 @@
 // split-P variant below), chosen so that everything fits the 512 tensor-memory columns:
 //   S0 S1 (kBN each) | O0 O1 (D each) | P0 P1 (kBN/2 each) | split-P only: Plo0 Plo1 (kBN/2 each)
 #include "host_common.h"
+#include "attn_mask.cuh"
 #include "sm100_ptx.cuh"
 #include "trace.cuh"
 
@@ -62,7 +63,7 @@ struct FwdArgs {
     void* o;
     int64_t o_sb, o_sh, o_ss;
     float* lse;
-    const float* keep_mask;
+    MaskArgs mask;
     const int32_t* kv_len;
     uint32_t* status;
 };
@@ -98,7 +99,7 @@ __device__ __forceinline__ float neg_inf() { return __int_as_float(0xff800000); 
 // kSplitP: P is written as two bf16 terms (p = hi + lo, 16 mantissa bits in total) and the
 // second contraction runs once per term; used when the output is stored as fp32, where the
 // 2^-9 rounding of a single bf16 P would be the largest error left.
-template <int D, typename OutT, bool kSplitP>
+template <int D, typename OutT, bool kSplitP, bool kMask>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
                       const __grid_constant__ CUtensorMap tmap_k,
@@ -310,7 +311,7 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
         const uint32_t tP = tmem_base + lane_base + L::kColP + t * (kBN / 2) + half * (kH / 2);
         const uint32_t tPlo = tmem_base + lane_base + L::kColPlo + t * (kBN / 2) + half * (kH / 2);
         const float c2 = a.scale_log2;
-        const bool general = (a.keep_mask != nullptr) || (a.use_clamp != 0);
+        const bool general = kMask || (a.use_clamp != 0);
         // exchange slots: [buffer][tile][half][row]
         auto xslot = [&](int buf, int hf) { return xchg + ((buf * 2 + t) * 2 + hf) * kBlockM + row; };
         uint32_t pair_phase = 0;
@@ -319,6 +320,10 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
         float l_run = 0.f;
         bool ok = true;
         for (int j = 0; j < n_t; ++j) {
+            uint32_t keep[kH / 32];              // dense mask of this thread's columns
+#pragma unroll
+            for (int w = 0; w < kH / 32; ++w)
+                keep[w] = kMask ? mask_bits_of_queries(a.mask, b, q0 + wq * 32, j * kBN + half * kH + 32 * w) : ~0u;
             ok = mbar_wait_warp(bar_s_full(t), (uint32_t)(j & 1), wc, 0x30 + t);
             if (!ok) break;
             tc_fence_after_sync();
@@ -340,15 +345,11 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
                 int lim = kvlen;
                 if (a.causal) lim = min(lim, qi + a.causal_off + 1);
                 lim -= k0 + half * kH;                  // own columns c < lim are visible
-                const float* mrow = nullptr;
-                if (a.keep_mask && qi < a.Sq)
-                    mrow = a.keep_mask + ((int64_t)b * a.Sq + qi) * a.Sk + k0 + half * kH;
 #pragma unroll
                 for (int c = 0; c < kH; ++c) {
                     float v = S_(c);
                     if (a.use_clamp) v = fminf(v, a.clamp_raw);
-                    bool vis = c < lim;
-                    if (mrow && vis) vis = (__ldg(mrow + c) != 0.0f);
+                    const bool vis = c < lim && (keep[c / 32] >> (c % 32) & 1u);
                     su[c] = __float_as_uint(vis ? v : neg_inf());
                 }
             } else if (edge) {
@@ -581,7 +582,7 @@ struct F4PCfg {
     static constexpr int kDynBytes = kMiscOff + 16 + 4 * kItemSlots + 1024;
 };
 
-template <bool kFold>
+template <bool kFold, bool kMask>
 __global__ void __launch_bounds__(kF4Threads, 1)
 attn_fwd4p_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
                         const __grid_constant__ CUtensorMap tmap_k,
@@ -842,7 +843,7 @@ attn_fwd4p_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
         const uint32_t tS = tmem_base + lane_base + t * kBN;
         const uint32_t tO = tmem_base + lane_base + 256 + t * D;
         const float c2 = a.scale_log2;
-        const bool general = (a.keep_mask != nullptr) || (a.use_clamp != 0);
+        const bool general = kMask || (a.use_clamp != 0);
         int scnt = 0;                       // s_full phases consumed
         int na = 0;                         // items with keys so far (selects the Q buffer)
         int ecnt = 0;                       // outputs this tile has staged
@@ -871,6 +872,10 @@ attn_fwd4p_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
             float m_run = neg_inf();
             float l_run = 0.f;
             for (int j = 0; j < n_t; ++j) {
+                uint32_t keep[2];                    // dense mask of this thread's 64 columns
+#pragma unroll
+                for (int w = 0; w < 2; ++w)
+                    keep[w] = kMask ? mask_bits_of_queries(a.mask, b_mask, tile_q0(it.m_block, t) + wq * 32, j * kBN + 32 * w) : ~0u;
                 ok = mbar_wait_warp(bar_s_full(t), (uint32_t)(scnt & 1), wc, 0x30 + t);
                 if (!ok) break;
                 ++scnt;
@@ -885,16 +890,11 @@ attn_fwd4p_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
                 if (general) {
                     const int k0 = j * kBN;
                     const int lim = lim_row - k0;           // columns c < lim are visible
-                    const int qi = tile_q0(it.m_block, t) + row;
-                    const float* mrow = nullptr;
-                    if (a.keep_mask && qi < a.Sq)
-                        mrow = a.keep_mask + ((int64_t)b_mask * a.Sq + qi) * a.Sk + k0;
 #pragma unroll
                     for (int c = 0; c < kBN; ++c) {
                         float v = S_(c);
                         if (a.use_clamp) v = fminf(v, a.clamp_raw);
-                        bool vis = c < lim;
-                        if (mrow && vis) vis = (__ldg(mrow + c) != 0.0f);
+                        const bool vis = c < lim && (keep[c / 32] >> (c % 32) & 1u);
                         su[c] = __float_as_uint(vis ? v : neg_inf());
                     }
                 } else if (j >= je) {
@@ -1068,9 +1068,6 @@ int launch_fwd4(ltca_ctx* ctx, const ltca_attn_params* p, const void* q, const v
     if ((rc = make_tmap_bhsd(ctx, &tk, k, 2, p->B, p->H, p->Sk, 64, ks, 64, kF4BN))) return rc;
     if ((rc = make_tmap_bhsd(ctx, &tv, v, 2, p->B, p->H, p->Sk, 64, vs, 64, kF4BN))) return rc;
     if ((rc = make_tmap_bhsd(ctx, &to, p->o, 2, p->B, p->H, p->Sq, 64, p->o_strides, 64, kBlockM))) return rc;
-    static SmemOptIn opt_in, opt_in_fold;
-    LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(opt_in, ctx->device, attn_fwd4p_sm100_kernel<false>, P::kDynBytes));
-    LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(opt_in_fold, ctx->device, attn_fwd4p_sm100_kernel<true>, P::kDynBytes));
     ItemGrid ig;
     ig.nblk = (p->Sq + kF4Tiles * kBlockM - 1) / (kF4Tiles * kBlockM);
     ig.H = p->H;
@@ -1080,18 +1077,18 @@ int launch_fwd4(ltca_ctx* ctx, const ltca_attn_params* p, const void* q, const v
     // (measured: B=1 H=16 S=4096, the bench workload dealt over eight GPUs: 92 us folded against 123 us)
     ig.fold = (a.causal && ig.nblk > 1 && ig.n_items <= ctx->sm_count) ? 1 : 0;
     const int n_cta = ig.n_items < ctx->sm_count ? ig.n_items : ctx->sm_count;
-    if (ig.fold)
-        LTCA_CUDA_OK(ctx, launch_dependent_if(small_attention_call(p), attn_fwd4p_sm100_kernel<true>, dim3(n_cta), dim3(kF4Threads), P::kDynBytes,
-                                           ctx->stream, tq, tk, tv, to, a, ig));
-    else
-        LTCA_CUDA_OK(ctx, launch_dependent_if(small_attention_call(p), attn_fwd4p_sm100_kernel<false>, dim3(n_cta), dim3(kF4Threads), P::kDynBytes,
-                                           ctx->stream, tq, tk, tv, to, a, ig));
+    static SmemOptIn opt_in[4];
+    auto kern = p->keep_mask ? (ig.fold ? attn_fwd4p_sm100_kernel<true, true> : attn_fwd4p_sm100_kernel<false, true>)
+                             : (ig.fold ? attn_fwd4p_sm100_kernel<true, false> : attn_fwd4p_sm100_kernel<false, false>);
+    LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(opt_in[(p->keep_mask ? 2 : 0) + ig.fold], ctx->device, kern, P::kDynBytes));
+    LTCA_CUDA_OK(ctx, launch_dependent_if(small_attention_call(p), kern, dim3(n_cta), dim3(kF4Threads), P::kDynBytes, ctx->stream, tq, tk,
+                                          tv, to, a, ig));
     LTCA_LAUNCH_OK(ctx, "attn_fwd4p_sm100_kernel");
     return LTCA_OK;
 }
 
 template <int D, typename OutT>
-int launch_fwd(ltca_ctx* ctx, const ltca_attn_params* p, const void* q, const void* k,
+int launch_fwd(ltca_ctx* ctx, const ltca_attn_params* p, const void* mask_words, const void* q, const void* k,
                const void* v, const ltca_strides& qs, const ltca_strides& ks,
                const ltca_strides& vs) {
     constexpr bool kSplitP = sizeof(OutT) == 4;
@@ -1113,7 +1110,7 @@ int launch_fwd(ltca_ctx* ctx, const ltca_attn_params* p, const void* q, const vo
     a.o = p->o;
     a.o_sb = p->o_strides.batch; a.o_sh = p->o_strides.head; a.o_ss = p->o_strides.seq;
     a.lse = p->lse;
-    a.keep_mask = p->keep_mask;
+    a.mask = mask_args(p, mask_words);
     a.kv_len = p->kv_len;
     a.status = ctx->d_status;
 
@@ -1137,9 +1134,9 @@ int launch_fwd(ltca_ctx* ctx, const ltca_attn_params* p, const void* q, const vo
         if (four) return launch_fwd4(ctx, p, q, k, v, qs, ks, vs, a);
     }
 
-    auto kern = attn_fwd_sm100_kernel<D, OutT, kSplitP>;
-    static SmemOptIn opt_in;                  // one per template instantiation
-    LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(opt_in, ctx->device, kern, L::kDynBytes));
+    auto kern = p->keep_mask ? attn_fwd_sm100_kernel<D, OutT, kSplitP, true> : attn_fwd_sm100_kernel<D, OutT, kSplitP, false>;
+    static SmemOptIn opt_in[2];               // one pair per template instantiation
+    LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(opt_in[p->keep_mask ? 1 : 0], ctx->device, kern, L::kDynBytes));
     dim3 grid((p->Sq + 2 * kBlockM - 1) / (2 * kBlockM), p->H, p->B);
     LTCA_CUDA_OK(ctx, launch_dependent(kern, grid, dim3(kFwdThreads), L::kDynBytes, ctx->stream, tq, tk, tv, a));
     LTCA_LAUNCH_OK(ctx, "attn_fwd_sm100_kernel");
@@ -1165,7 +1162,7 @@ bool attn_fwd_sm100_supported(const ltca_attn_params* p) {
 }
 
 // Expects bf16 Q, K, V (already converted when the caller's storage is fp32).
-int launch_attn_fwd_sm100_bf16in(ltca_ctx* ctx, const ltca_attn_params* p, const void* q,
+int launch_attn_fwd_sm100_bf16in(ltca_ctx* ctx, const ltca_attn_params* p, const void* mask_words, const void* q,
                                  const void* k, const void* v, const ltca_strides& qs,
                                  const ltca_strides& ks, const ltca_strides& vs) {
     const int oes = elem_size(p->dtype);
@@ -1173,11 +1170,11 @@ int launch_attn_fwd_sm100_bf16in(ltca_ctx* ctx, const ltca_attn_params* p, const
         ((p->o_strides.head * oes) & 15) || ((p->o_strides.batch * oes) & 15))
         return fail(ctx, LTCA_ERR_INVALID, "output base and strides must be 16-byte aligned");
     if (p->D == 64) {
-        return p->dtype == LTCA_BF16 ? launch_fwd<64, __nv_bfloat16>(ctx, p, q, k, v, qs, ks, vs)
-                                     : launch_fwd<64, float>(ctx, p, q, k, v, qs, ks, vs);
+        return p->dtype == LTCA_BF16 ? launch_fwd<64, __nv_bfloat16>(ctx, p, mask_words, q, k, v, qs, ks, vs)
+                                     : launch_fwd<64, float>(ctx, p, mask_words, q, k, v, qs, ks, vs);
     }
-    return p->dtype == LTCA_BF16 ? launch_fwd<128, __nv_bfloat16>(ctx, p, q, k, v, qs, ks, vs)
-                                 : launch_fwd<128, float>(ctx, p, q, k, v, qs, ks, vs);
+    return p->dtype == LTCA_BF16 ? launch_fwd<128, __nv_bfloat16>(ctx, p, mask_words, q, k, v, qs, ks, vs)
+                                 : launch_fwd<128, float>(ctx, p, mask_words, q, k, v, qs, ks, vs);
 }
 
 }  // namespace ltca

@@ -5,10 +5,11 @@
 
 #include "host_common.h"
 #include "sm100_ptx.cuh"
+#include "attn_mask.cuh"
 #include "attn_wide.h"
 
 namespace ltca {
-int launch_attn_fwd_sm100_bf16in(ltca_ctx* ctx, const ltca_attn_params* p, const void* q,
+int launch_attn_fwd_sm100_bf16in(ltca_ctx* ctx, const ltca_attn_params* p, const void* mask_words, const void* q,
                                  const void* k, const void* v, const ltca_strides& qs,
                                  const ltca_strides& ks, const ltca_strides& vs);
 
@@ -503,6 +504,7 @@ int ltca_attn_workspace_bytes(const ltca_attn_params* p, int backward, size_t* b
             if (backward) n += packed_bytes(p, p->Sq);                     // dO as bf16
         }
         if (backward) n += attn_bwd_sm100_workspace(p);
+        n += mask_words_bytes(p);                                          // behind everything else
     } else if (backward) {
         n += attn_bwd_fp32_workspace(p);
     }
@@ -520,11 +522,13 @@ int ltca_attn_fwd(ltca_ctx* ctx, const ltca_attn_params* p) {
                     "the tensor-pipe forward needs a head_dim that is a multiple of 8 with 16-byte aligned rows (got %d)",
                     p->D);
     if (!tensor_path(p, false)) return launch_attn_fwd_fp32(ctx, p);
-    if (p->dtype == LTCA_BF16)
-        return launch_attn_fwd_sm100_bf16in(ctx, p, p->q, p->k, p->v, p->q_strides, p->k_strides,
+    const void* words = nullptr;
+    if (p->dtype == LTCA_BF16) {
+        if ((rc = mask_words_of(ctx, p, 0, &words))) return rc;
+        return launch_attn_fwd_sm100_bf16in(ctx, p, words, p->q, p->k, p->v, p->q_strides, p->k_strides,
                                             p->v_strides);
-    size_t need = 0;
-    ltca_attn_workspace_bytes(p, 0, &need);
+    }
+    const size_t need = packed_bytes(p, p->Sq) + 2 * packed_bytes(p, p->Sk);
     if (!p->workspace || p->workspace_bytes < need)
         return fail(ctx, LTCA_ERR_WORKSPACE, "forward needs %zu bytes of workspace", need);
     if (reinterpret_cast<uintptr_t>(p->workspace) & 255)
@@ -536,7 +540,8 @@ int ltca_attn_fwd(ltca_ctx* ctx, const ltca_attn_params* p) {
     const PackJob jobs[3] = {{p->q, p->q_strides, qb, p->Sq}, {p->k, p->k_strides, kb, p->Sk},
                              {p->v, p->v_strides, vb, p->Sk}};
     if ((rc = pack_many_to_bf16(ctx, jobs, 3, p->B, p->H, p->D))) return rc;
-    return launch_attn_fwd_sm100_bf16in(ctx, p, qb, kb, vb, contiguous_strides(p->H, p->Sq, p->D),
+    if ((rc = mask_words_of(ctx, p, need, &words))) return rc;
+    return launch_attn_fwd_sm100_bf16in(ctx, p, words, qb, kb, vb, contiguous_strides(p->H, p->Sq, p->D),
                                         contiguous_strides(p->H, p->Sk, p->D),
                                         contiguous_strides(p->H, p->Sk, p->D));
 }

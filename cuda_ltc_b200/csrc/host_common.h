@@ -24,6 +24,9 @@ struct ltca_ctx {
     uint32_t* d_status = nullptr;     // device status word (allocated once at context creation)
     int* d_sched = nullptr;           // work-item counters of the persistent kernels (same allocation:
                                       // d_status + 4 .. ; two ints per kernel kind, kept at zero between launches)
+    // A module call's packed mask (attn_mask.cuh): set while the call launches its attention kernels, which all read it.
+    const float* mask_packed = nullptr;
+    const void* mask_words = nullptr;
     char err[512] = {0};
     // optional per-kernel timing of the backward pass (ltca_ctx_enable_kernel_timing)
     bool time_kernels = false;

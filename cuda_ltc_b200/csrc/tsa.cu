@@ -20,6 +20,7 @@
 // Backward follows the reference:
 // the incoming gradient passes through LayerNorm and the residual unchanged
 // (src/ml/cudnn_time_self_attention.cu:291-299), dx = dQ Wq^T + dK Wk^T + dV Wv^T.
+#include "attn_mask.cuh"
 #include "gemm_fp32.h"
 #include "gemm_sm100.h"
 #include "attn_wide.h"
@@ -268,6 +269,63 @@ __global__ void layer_norm_bwd_kernel(const float* __restrict__ g, const float* 
     const int lane = threadIdx.x & 31;
     const float* xr = x + row * E;
     const float* gr = g + row * E;
+    if ((E & 127) == 0 && E <= 1024 && aligned16(g, x, gamma, res, dx) && (reinterpret_cast<uintptr_t>(prod) & 15) == 0) {
+        // both rows stay in registers: every operand is read once, in 16-byte pieces
+        auto warp_sum = [](float v) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            return v;
+        };
+        const int n4 = E >> 7;
+        float4 xh[8], gv[8];
+        float s0 = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if (i < n4) {
+                xh[i] = __ldg(reinterpret_cast<const float4*>(xr) + lane + 32 * i);
+                gv[i] = __ldg(reinterpret_cast<const float4*>(gr) + lane + 32 * i);
+                s0 += (xh[i].x + xh[i].y) + (xh[i].z + xh[i].w);
+            }
+        const float mean = warp_sum(s0) / E;
+        float s1 = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if (i < n4) {
+                xh[i].x -= mean; xh[i].y -= mean; xh[i].z -= mean; xh[i].w -= mean;
+                s1 = fmaf(xh[i].x, xh[i].x, s1); s1 = fmaf(xh[i].y, xh[i].y, s1);
+                s1 = fmaf(xh[i].z, xh[i].z, s1); s1 = fmaf(xh[i].w, xh[i].w, s1);
+            }
+        const float inv_std = rsqrtf(warp_sum(s1) / E + eps);
+        float a1 = 0.f, a2 = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if (i < n4) {
+                const float4 gm = __ldg(reinterpret_cast<const float4*>(gamma) + lane + 32 * i);
+                xh[i].x *= inv_std; xh[i].y *= inv_std; xh[i].z *= inv_std; xh[i].w *= inv_std;
+                const float4 gg = make_float4(gv[i].x * gm.x, gv[i].y * gm.y, gv[i].z * gm.z, gv[i].w * gm.w);
+                a1 += (gg.x + gg.y) + (gg.z + gg.w);
+                a2 = fmaf(gg.x, xh[i].x, a2); a2 = fmaf(gg.y, xh[i].y, a2);
+                a2 = fmaf(gg.z, xh[i].z, a2); a2 = fmaf(gg.w, xh[i].w, a2);
+                if (prod)
+                    reinterpret_cast<float4*>(prod + row * E)[lane + 32 * i] =
+                        make_float4(gv[i].x * xh[i].x, gv[i].y * xh[i].y, gv[i].z * xh[i].z, gv[i].w * xh[i].w);
+                gv[i] = gg;
+            }
+        if (!dx) return;
+        const float m1 = warp_sum(a1) / E, m2 = warp_sum(a2) / E;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if (i < n4) {
+                float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (res) r = __ldg(reinterpret_cast<const float4*>(res + row * E) + lane + 32 * i);
+                r.x += inv_std * (gv[i].x - m1 - xh[i].x * m2);
+                r.y += inv_std * (gv[i].y - m1 - xh[i].y * m2);
+                r.z += inv_std * (gv[i].z - m1 - xh[i].z * m2);
+                r.w += inv_std * (gv[i].w - m1 - xh[i].w * m2);
+                reinterpret_cast<float4*>(dx + row * E)[lane + 32 * i] = r;
+            }
+        return;
+    }
     float sum = 0.f;
     for (int i = lane; i < E; i += 32) sum += xr[i];
 #pragma unroll
@@ -326,7 +384,7 @@ __device__ __forceinline__ float ld_f(const __nv_bfloat16* p) { return __bfloat1
 template <typename T>
 __device__ __forceinline__ float column_chunk(const T* src, int64_t ld, int64_t r0, int64_t r1) {
     float acc = 0.f;
-#pragma unroll 8
+#pragma unroll 16
     for (int64_t r = r0; r < r1; ++r) acc += ld_f(src + r * ld);
     return acc;
 }
@@ -646,6 +704,9 @@ void fill_wide(const ltca_tsa_params* t, const TBufs& tb, WideArgs* w) {
     w->grads_bf16 = 1;
 }
 
+// The attention scratch (TBufs::rest) of a call whose buffers start at w; not on the written-out-score path.
+char* scratch_of(const ltca_tsa_params* t, const TPlan& pl, char* w) { return t->saved ? w : w + tensor_saved_bytes(pl); }
+
 // bf16 copies, fused Q/K/V projection, attention forward.
 // `also_src` / `also_dst`: one more [rows, E] fp32 matrix (the backward's dy) to be rounded to bf16 by the same launch
 // that rounds x and the weights; *also_done says whether that happened (not on the paths that convert otherwise
@@ -833,6 +894,20 @@ int tensor_backward(ltca_ctx* ctx, const ltca_tsa_params* t, bool want_dx, bool 
     TBufs tb;
     // the forward is recomputed, as the reference's caller does before each backward
     // (src/ml/ml_liquid_net.cu:715-721)
+    // the recomputed attention and its backward read the same mask: packed once, behind what either uses of the scratch
+    struct PackedMask {
+        ltca_ctx* ctx;
+        ~PackedMask() { ctx->mask_packed = nullptr; ctx->mask_words = nullptr; }
+    } packed{ctx};
+    if (t->keep_mask && !pl.wide) {
+        ltca_attn_params a;
+        fill_attn_bf16(t, &a);
+        const size_t most = pl.attn_fwd > pl.attn_bwd ? pl.attn_fwd : pl.attn_bwd;
+        void* words = scratch_of(t, pl, w) + (most - mask_words_bytes(&a));
+        if ((rc = pack_mask_words(ctx, &a, words))) return rc;
+        ctx->mask_packed = t->keep_mask;
+        ctx->mask_words = words;
+    }
     bool dy_done = false;
     if ((rc = tensor_forward_core(ctx, t, pl, w, &tb, 1, t->dy, dyb, &dy_done, outer, outer_g))) return rc;
     const int rows = (int)pl.rows, E = t->E, HW = pl.HW, Ep = pl.Ep;
