@@ -1,32 +1,30 @@
 // Single-query attention over a key/value cache with per-sequence lengths.  The work is pure
 // streaming of K and V (about 0.5 FLOP per byte), so the kernel is built around wide coalesced
 // loads and keeps all arithmetic in fp32 registers:
-//   - a group of D/4 lanes owns one key at a time (each lane a 16-byte slice of the row), the
-//     score is a shuffle reduction inside the group, the value row is accumulated by the same
-//     lanes without further communication;
-//   - every group runs its own online softmax over the keys it visits; groups are merged once
-//     per CTA through shared memory;
-//   - when batch x heads cannot fill the GPU the key range is split across CTAs, partial
-//     (max, sum, output) triples go to a caller-provided scratch buffer and a second small
-//     kernel merges them;
-//   - when batch x heads does fill the GPU but the sequences have different lengths, each
-//     (batch, head) pair is a thread-block cluster of two or four CTAs that take alternate
-//     32-key blocks of ITS keys and merge through distributed shared memory (no scratch, no
-//     second kernel): the work per CTA is less uneven, which shortens the tail in which only
-//     the CTAs of the longest sequences are still streaming.
+//   - a group of lanes owns one key at a time (each lane 16 bytes of the row), the score is a shuffle
+//     reduction inside the group, the value row is accumulated by the same lanes without further
+//     communication; the next keys are loaded while these are multiplied;
+//   - every group runs its own online softmax over the keys it visits; a warp's groups are merged by
+//     shuffles, a CTA's warps through shared memory;
+//   - a pair's keys are split over several CTAs where batch x heads cannot fill the GPU, and over two
+//     or four where it does but the sequences differ in length (less of a tail in which only the
+//     longest are still streaming).  Up to 16 CTAs of a pair are one thread-block cluster whose
+//     first CTA receives the others' partial (max, sum, output) triples in its shared memory; more
+//     go through a caller-provided scratch buffer and a second small kernel.
 // The reference has no counterpart: its cuDNN call always passes currIdx = -1
 // (reference src/ml/cuDNN_ops.cu:206).
 #include <cooperative_groups.h>
 #include <math.h>
 
 #include "host_common.h"
+#include "sm100_ptx.cuh"
 
 namespace ltca {
 
 namespace {
 
-constexpr int kDecThreads = 128;
-constexpr int kUnroll = 4;
+constexpr int kMaxCluster = 16;             // CTAs of one (batch, head) pair that merge through shared memory
+constexpr int kUnroll = 4;                  // keys per group and iteration; two iterations are in flight
 
 struct DecodeArgs {
     int B, H, Sk, D;
@@ -39,28 +37,68 @@ struct DecodeArgs {
     const float* keep_mask;     // [B, 1, Sk]
     const int32_t* kv_len;
     int nsplit;
+    int vec16;                  // every K and V row starts on a 16-byte boundary
     float* partial;             // [B*H][nsplit][D + 2]; null when the splits are one cluster
 };
 
-__device__ __forceinline__ float4 ld4(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
-__device__ __forceinline__ float4 ld4(const __nv_bfloat16* p) {
-    const uint2 u = __ldg(reinterpret_cast<const uint2*>(p));
-    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x));
-    const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
-    return make_float4(a.x, a.y, b.x, b.y);
+// A lane's 16 bytes of a row: 4 fp32 or 8 bf16 values.
+template <typename T>
+constexpr int kLaneElems = 16 / (int)sizeof(T);
+template <typename T>
+__device__ __forceinline__ uint4 ld_lane(const T* p, bool vec16) {
+    if (sizeof(T) == 4 || vec16) return __ldg(reinterpret_cast<const uint4*>(p));
+    const uint2 a = __ldg(reinterpret_cast<const uint2*>(p)), b = __ldg(reinterpret_cast<const uint2*>(p) + 1);
+    return make_uint4(a.x, a.y, b.x, b.y);
+}
+__device__ __forceinline__ void unpack(const uint4& u, float (&v)[4]) {
+    v[0] = __uint_as_float(u.x); v[1] = __uint_as_float(u.y); v[2] = __uint_as_float(u.z); v[3] = __uint_as_float(u.w);
+}
+__device__ __forceinline__ void unpack(const uint4& u, float (&v)[8]) {
+    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        v[2 * i] = __uint_as_float(w[i] << 16);
+        v[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+    }
 }
 __device__ __forceinline__ void st1(float* p, float v) { *p = v; }
 __device__ __forceinline__ void st1(__nv_bfloat16* p, float v) { *p = __float2bfloat16_rn(v); }
 
-// kCluster: the nsplit CTAs of one (batch, head) pair form a thread-block cluster (1, nsplit, 1).
-template <typename T, int LPK, bool kCluster>
-__global__ void __launch_bounds__(kDecThreads) attn_decode_kernel(const DecodeArgs a) {
-    constexpr int D = 4 * LPK;
+// Result of a (batch, head) pair from n partials (max, sum, D unnormalised outputs), by the first D threads.
+template <typename T>
+__device__ __forceinline__ void merge_partials(const DecodeArgs& a, const float* part, int n, int b, int h) {
+    const int d = threadIdx.x, stride = a.D + 2;
+    float M = -INFINITY;
+    for (int s = 0; s < n; ++s) M = fmaxf(M, part[s * stride]);
+    const float Ms = (M == -INFINITY) ? 0.f : M;
+    float L = 0.f, acc = 0.f;
+    for (int s = 0; s < n; ++s) {
+        const float* ps = part + s * stride;
+        const float w = (ps[0] == -INFINITY) ? 0.f : expf(ps[0] - Ms);
+        L = fmaf(ps[1], w, L);
+        acc = fmaf(ps[2 + d], w, acc);
+    }
+    T* op = reinterpret_cast<T*>(a.o) + b * a.os.batch + h * a.os.head;
+    st1(op + d, L > 0.f ? acc / L : 0.f);
+    if (d == 0 && a.lse) a.lse[(int64_t)b * a.H + h] = L > 0.f ? M + logf(L) : -INFINITY;
+}
+
+// LPK lanes own one key at a time.  kSplit 0: one CTA per pair; 1: the nsplit CTAs of a pair form a cluster (1, nsplit, 1)
+// whose first CTA receives the others' partials in its shared memory; 2: partials go to scratch for a second kernel.
+template <typename T, int LPK, int W, int kSplit>
+__global__ void __launch_bounds__(32 * W) attn_decode_kernel(const DecodeArgs a) {
+    constexpr int EL = kLaneElems<T>;
+    constexpr int D = EL * LPK;
     constexpr int G = 32 / LPK;                         // key groups per warp
-    constexpr int NG = (kDecThreads / 32) * G;          // key groups per CTA
-    __shared__ float sm_o[NG][D];
-    __shared__ float sm_m[NG], sm_l[NG];
-    __shared__ float sm_part[D + 2];                    // this CTA's (max, sum, output) for the cluster merge
+    constexpr int NG = W * G;                           // key groups per CTA
+    __shared__ __align__(16) float sm_o[W][D];
+    __shared__ float sm_m[W], sm_l[W];
+    __shared__ float sm_part[kSplit == 1 ? kMaxCluster * (D + 2) : 1];
+    namespace cg = cooperative_groups;
+    grid_launch_dependents();
+    grid_dependency_wait();
+    // the other CTAs of the cluster may be written to once they have started: waited for behind the key loop
+    if (kSplit == 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
 
     const int bh = blockIdx.x;
     const int b = bh / a.H, h = bh % a.H;
@@ -69,199 +107,216 @@ __global__ void __launch_bounds__(kDecThreads) attn_decode_kernel(const DecodeAr
     const int g = warp * G + lane / LPK;
     const int sub = lane % LPK;
 
-    int kvlen = a.Sk;
-    if (a.kv_len) kvlen = min(max(a.kv_len[b], 0), a.Sk);
     // the CTA's splits interleave at the granularity of one iteration (NG * kUnroll keys), so only
     // the sequence's last iteration is ragged, whatever the split count
-    const int ks = 0, ke = kvlen;
-
-    const T* qp = reinterpret_cast<const T*>(a.q) + b * a.qs.batch + h * a.qs.head + 4 * sub;
-    const T* kp = reinterpret_cast<const T*>(a.k) + b * a.ks.batch + h * a.ks.head + 4 * sub;
-    const T* vp = reinterpret_cast<const T*>(a.v) + b * a.vs.batch + h * a.vs.head + 4 * sub;
+    int ke = a.Sk;
+    if (a.kv_len) ke = min(max(a.kv_len[b], 0), a.Sk);
+    const T* qp = reinterpret_cast<const T*>(a.q) + b * a.qs.batch + h * a.qs.head + EL * sub;
+    const T* kp = reinterpret_cast<const T*>(a.k) + b * a.ks.batch + h * a.ks.head + EL * sub;
+    const T* vp = reinterpret_cast<const T*>(a.v) + b * a.vs.batch + h * a.vs.head + EL * sub;
     const float* mrow = a.keep_mask ? a.keep_mask + (int64_t)b * a.Sk : nullptr;
-    float4 q4 = ld4(qp);
-    q4.x *= a.scale; q4.y *= a.scale; q4.z *= a.scale; q4.w *= a.scale;
+    const bool vec16 = a.vec16 != 0;
+    float q[EL];
+    unpack(ld_lane(qp, false), q);
+#pragma unroll
+    for (int i = 0; i < EL; ++i) q[i] *= a.scale;
 
-    float m = -INFINITY, l = 0.f;
-    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
-    const int iters = (ke - ks + NG * kUnroll - 1) / (NG * kUnroll);
-    for (int it = split; it < iters; it += a.nsplit) {
-        float4 kk[kUnroll], vv[kUnroll];
-        float s[kUnroll];
-        bool live[kUnroll];
+    float m = -INFINITY, l = 0.f, o[EL];
+#pragma unroll
+    for (int i = 0; i < EL; ++i) o[i] = 0.f;
+    const int iters = (ke + NG * kUnroll - 1) / (NG * kUnroll);
+
+    struct Keys { uint4 k[kUnroll], v[kUnroll]; };
+    auto fetch = [&](int it, Keys& x) {
 #pragma unroll
         for (int u = 0; u < kUnroll; ++u) {
-            const int j = ks + (it * kUnroll + u) * NG + g;
-            live[u] = j < ke;
-            const int jj = live[u] ? j : (ke - 1);            // in range: ke > ks here
-            kk[u] = ld4(kp + (int64_t)jj * a.ks.seq);
-            vv[u] = ld4(vp + (int64_t)jj * a.vs.seq);
-            if (live[u] && mrow && mrow[j] == 0.f) live[u] = false;
+            const int j = min((it * kUnroll + u) * NG + g, ke - 1);            // in range: ke > 0 here
+            x.k[u] = ld_lane(kp + (int64_t)j * a.ks.seq, vec16);
+            x.v[u] = ld_lane(vp + (int64_t)j * a.vs.seq, vec16);
         }
+    };
+    auto consume = [&](int it, const Keys& x) {
+        float s[kUnroll];
         float mt = m;
 #pragma unroll
         for (int u = 0; u < kUnroll; ++u) {
-            float d = q4.x * kk[u].x + q4.y * kk[u].y + q4.z * kk[u].z + q4.w * kk[u].w;
+            float kk[EL];
+            unpack(x.k[u], kk);
+            float d = q[0] * kk[0];
+#pragma unroll
+            for (int i = 1; i < EL; ++i) d = fmaf(q[i], kk[i], d);
 #pragma unroll
             for (int off = LPK / 2; off > 0; off >>= 1) d += __shfl_xor_sync(0xffffffffu, d, off);
             if (a.use_clamp) d = fminf(d, a.clamp);
-            s[u] = live[u] ? d : -INFINITY;
+            const int j = (it * kUnroll + u) * NG + g;
+            bool live = j < ke;
+            if (live && mrow && mrow[j] == 0.f) live = false;
+            s[u] = live ? d : -INFINITY;
             mt = fmaxf(mt, s[u]);
         }
         const float m_safe = (mt == -INFINITY) ? 0.f : mt;
         const float corr = (m == -INFINITY) ? 0.f : expf(m - m_safe);
         l *= corr;
-        o.x *= corr; o.y *= corr; o.z *= corr; o.w *= corr;
+#pragma unroll
+        for (int i = 0; i < EL; ++i) o[i] *= corr;
 #pragma unroll
         for (int u = 0; u < kUnroll; ++u) {
             const float p = expf(s[u] - m_safe);
             l += p;
-            o.x = fmaf(p, vv[u].x, o.x);
-            o.y = fmaf(p, vv[u].y, o.y);
-            o.z = fmaf(p, vv[u].z, o.z);
-            o.w = fmaf(p, vv[u].w, o.w);
+            float vv[EL];
+            unpack(x.v[u], vv);
+#pragma unroll
+            for (int i = 0; i < EL; ++i) o[i] = fmaf(p, vv[i], o[i]);
         }
         m = mt;
+    };
+    // the next iteration's keys are on their way while this one's are multiplied
+    Keys x, y;
+    int it = split;
+    if (it < iters) fetch(it, x);
+    while (it < iters) {
+        const int n1 = it + a.nsplit, n2 = n1 + a.nsplit;
+        if (n1 < iters) fetch(n1, y);
+        consume(it, x);
+        if (n1 >= iters) break;
+        if (n2 < iters) fetch(n2, x);
+        consume(n1, y);
+        it = n2;
     }
-    sm_o[g][4 * sub + 0] = o.x;
-    sm_o[g][4 * sub + 1] = o.y;
-    sm_o[g][4 * sub + 2] = o.z;
-    sm_o[g][4 * sub + 3] = o.w;
-    if (sub == 0) { sm_m[g] = m; sm_l[g] = l; }
+    // the groups of a warp, then the warps of the CTA
+#pragma unroll
+    for (int off = LPK; off < 32; off <<= 1) {
+        const float m2 = __shfl_xor_sync(0xffffffffu, m, off), l2 = __shfl_xor_sync(0xffffffffu, l, off);
+        const float mm = fmaxf(m, m2), ms = (mm == -INFINITY) ? 0.f : mm;
+        const float w1 = (m == -INFINITY) ? 0.f : expf(m - ms), w2 = (m2 == -INFINITY) ? 0.f : expf(m2 - ms);
+        l = l * w1 + l2 * w2;
+#pragma unroll
+        for (int i = 0; i < EL; ++i) o[i] = o[i] * w1 + __shfl_xor_sync(0xffffffffu, o[i], off) * w2;
+        m = mm;
+    }
+    if (lane < LPK) {
+#pragma unroll
+        for (int i = 0; i < EL; i += 4)
+            *reinterpret_cast<float4*>(&sm_o[warp][EL * sub + i]) = make_float4(o[i], o[i + 1], o[i + 2], o[i + 3]);
+    }
+    if (lane == 0) { sm_m[warp] = m; sm_l[warp] = l; }
     __syncthreads();
+    if (kSplit == 1) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
     if (threadIdx.x < D) {
         const int d = threadIdx.x;
         float M = -INFINITY;
 #pragma unroll
-        for (int i = 0; i < NG; ++i) M = fmaxf(M, sm_m[i]);
+        for (int i = 0; i < W; ++i) M = fmaxf(M, sm_m[i]);
         const float Ms = (M == -INFINITY) ? 0.f : M;
         float L = 0.f, acc = 0.f;
 #pragma unroll
-        for (int i = 0; i < NG; ++i) {
+        for (int i = 0; i < W; ++i) {
             const float w = (sm_m[i] == -INFINITY) ? 0.f : expf(sm_m[i] - Ms);
             L = fmaf(sm_l[i], w, L);
             acc = fmaf(sm_o[i][d], w, acc);
         }
-        if (kCluster) {
-            sm_part[2 + d] = acc;
-            if (d == 0) { sm_part[0] = M; sm_part[1] = L; }
-        } else if (a.nsplit == 1) {
+        if (kSplit == 0) {
             T* op = reinterpret_cast<T*>(a.o) + b * a.os.batch + h * a.os.head;
             st1(op + d, L > 0.f ? acc / L : 0.f);
             if (d == 0 && a.lse) a.lse[bh] = L > 0.f ? M + logf(L) : -INFINITY;
         } else {
-            float* part = a.partial + ((int64_t)bh * a.nsplit + split) * (D + 2);
+            float* part = kSplit == 1 ? cg::this_cluster().map_shared_rank(sm_part, 0) + split * (D + 2)
+                                      : a.partial + ((int64_t)bh * a.nsplit + split) * (D + 2);
             part[2 + d] = acc;
             if (d == 0) { part[0] = M; part[1] = L; }
         }
     }
-    if (kCluster) {
-        namespace cg = cooperative_groups;
-        cg::cluster_group cluster = cg::this_cluster();
-        cluster.sync();                                  // every CTA's partial is in its shared memory
-        if (cluster.block_rank() == 0 && threadIdx.x < D) {
-            const int d = threadIdx.x;
-            const int n = (int)cluster.num_blocks();
-            float M = -INFINITY;
-            for (int r = 0; r < n; ++r) M = fmaxf(M, cluster.map_shared_rank(sm_part, r)[0]);
-            const float Ms = (M == -INFINITY) ? 0.f : M;
-            float L = 0.f, acc = 0.f;
-            for (int r = 0; r < n; ++r) {
-                const float* ps = cluster.map_shared_rank(sm_part, r);
-                const float w = (ps[0] == -INFINITY) ? 0.f : expf(ps[0] - Ms);
-                L = fmaf(ps[1], w, L);
-                acc = fmaf(ps[2 + d], w, acc);
-            }
-            T* op = reinterpret_cast<T*>(a.o) + b * a.os.batch + h * a.os.head;
-            st1(op + d, L > 0.f ? acc / L : 0.f);
-            if (d == 0 && a.lse) a.lse[bh] = L > 0.f ? M + logf(L) : -INFINITY;
-        }
-        cluster.sync();                                  // nobody leaves while its partial may still be read
+    if (kSplit == 1) {
+        cg::this_cluster().sync();                       // every partial is in the first CTA's shared memory
+        if (split == 0 && threadIdx.x < D) merge_partials<T>(a, sm_part, a.nsplit, b, h);
     }
 }
 
 template <typename T>
-__global__ void attn_decode_merge_kernel(const DecodeArgs a) {
+__global__ void __launch_bounds__(128) attn_decode_merge_kernel(const DecodeArgs a) {
+    grid_launch_dependents();
+    grid_dependency_wait();
     const int bh = blockIdx.x;
-    const int b = bh / a.H, h = bh % a.H;
-    const int d = threadIdx.x;
-    if (d >= a.D) return;
-    const float* part = a.partial + (int64_t)bh * a.nsplit * (a.D + 2);
-    float M = -INFINITY;
-    for (int s = 0; s < a.nsplit; ++s) M = fmaxf(M, part[s * (a.D + 2)]);
-    const float Ms = (M == -INFINITY) ? 0.f : M;
-    float L = 0.f, acc = 0.f;
-    for (int s = 0; s < a.nsplit; ++s) {
-        const float* ps = part + s * (a.D + 2);
-        const float w = (ps[0] == -INFINITY) ? 0.f : expf(ps[0] - Ms);
-        L = fmaf(ps[1], w, L);
-        acc = fmaf(ps[2 + d], w, acc);
-    }
-    T* op = reinterpret_cast<T*>(a.o) + b * a.os.batch + h * a.os.head;
-    st1(op + d, L > 0.f ? acc / L : 0.f);
-    if (d == 0 && a.lse) a.lse[bh] = L > 0.f ? M + logf(L) : -INFINITY;
+    if ((int)threadIdx.x < a.D) merge_partials<T>(a, a.partial + (int64_t)bh * a.nsplit * (a.D + 2), a.nsplit, bh / a.H, bh % a.H);
 }
 
-int pick_splits(const ltca_attn_params* p, int sm_count) {
-    if (p->B < 1 || p->H < 1 || p->Sk < 1) return 1;      // nothing to split (and no division by zero below)
+// How a (batch, head) pair's keys are dealt out.  cluster: the splits merge through distributed shared memory; few: the
+// pairs alone do not fill the GPU.
+struct SplitPlan { int n; bool cluster; bool few; };
+SplitPlan plan_splits(const ltca_attn_params* p) {
+    SplitPlan s{1, false, false};
+    if (p->B < 1 || p->H < 1 || p->Sk < 1 || p->D < 1) return s;      // (nothing to split, no division by zero below)
+    constexpr int sms = kPlanSms;
     const int64_t bh = (int64_t)p->B * p->H;
-    if (sm_count <= 0) sm_count = kPlanSms;
-    if (bh >= 2 * sm_count) return 1;
-    int64_t want = (4 * (int64_t)sm_count + bh - 1) / bh;
-    int64_t cap = (p->Sk + 255) / 256;
+    if (bh >= 2 * sms) {
+        // With lengths that differ, two or four CTAs take alternate blocks of a pair's keys, so that the longest
+        // sequences do not stream alone at the end; measured at B=256 H=8 lengths U{1..1024}: 2 CTAs 6112 GB/s,
+        // 4: 6011, 8: 4869 (1: 4820).
+        if (p->kv_len && p->Sk >= 512) { s.n = p->Sk < 2048 ? 2 : 4; s.cluster = true; }
+        return s;
+    }
+    // About three CTAs of eight warps per SM, each with at least two iterations of keys.  Up to 16 splits are one
+    // cluster and one launch; where a pair has the keys and the GPU the room for more, scratch and a merge kernel.
+    s.few = true;
+    const int es = p->dtype == LTCA_BF16 ? 2 : 4;
+    const int64_t iter = 8 * kUnroll * 32 * 16 / ((int64_t)p->D * es);        // keys per iteration of an 8-warp CTA
+    const int64_t want = (3 * (int64_t)sms + bh - 1) / bh, cap = (p->Sk + 2 * iter - 1) / (2 * (iter > 0 ? iter : 1));
     int64_t n = want < cap ? want : cap;
-    if (n < 1) n = 1;
     if (n > 64) n = 64;
-    return (int)n;
+    if (n > kMaxCluster) {
+        s.n = (int)n;
+        return s;
+    }
+    while (s.n < n) s.n *= 2;
+    s.cluster = s.n > 1;
+    return s;
 }
 
-// Splits of one (batch, head) pair that run as one cluster (0: none).  Used when batch x heads
-// already fills the GPU (so the scratch path would not split) but the lengths differ.
-int pick_cluster(const ltca_attn_params* p, int sm_count) {
-#ifdef LTCA_DECODE_NO_CLUSTER
-    return 0;
-#endif
-    if (pick_splits(p, sm_count) != 1) return 0;
-    if (!p->kv_len || p->Sk < 512) return 0;
-    // measured at B=256 H=8 lengths U{1..1024}: 2 CTAs 6112 GB/s, 4: 6011, 8: 4869 (1: 4820)
-    return p->Sk < 2048 ? 2 : 4;
+template <typename T, int LPK, int W, int kSplit>
+int launch_decode(ltca_ctx* ctx, const DecodeArgs& a) {
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3(a.B * a.H, a.nsplit);
+    cfg.blockDim = dim3(32 * W);
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = 1;
+    attr[1].val.clusterDim.y = (unsigned)a.nsplit;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = kSplit == 1 ? 2 : 1;
+    if (kSplit == 1 && a.nsplit > 8) {
+        static SmemOptIn once;      // clusters of more than eight CTAs are an opt-in of a kernel on one device
+        const uint64_t bit = (ctx->device >= 0 && ctx->device < 64) ? (1ull << ctx->device) : 0ull;
+        if (!bit || !(once.done.load(std::memory_order_acquire) & bit)) {
+            LTCA_CUDA_OK(ctx, cudaFuncSetAttribute(attn_decode_kernel<T, LPK, W, kSplit>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+            once.done.fetch_or(bit, std::memory_order_release);
+        }
+    }
+    LTCA_CUDA_OK(ctx, cudaLaunchKernelEx(&cfg, attn_decode_kernel<T, LPK, W, kSplit>, a));
+    return LTCA_OK;
 }
 
 template <typename T, int LPK>
-int run_decode(ltca_ctx* ctx, const DecodeArgs& a) {
-    dim3 grid(a.B * a.H, a.nsplit);
-    if (a.nsplit > 1 && !a.partial) {
-        cudaLaunchConfig_t cfg;
-        memset(&cfg, 0, sizeof(cfg));
-        cfg.gridDim = grid;
-        cfg.blockDim = dim3(kDecThreads);
-        cfg.stream = ctx->stream;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = 1;
-        attr[0].val.clusterDim.y = (unsigned)a.nsplit;
-        attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        LTCA_CUDA_OK(ctx, cudaLaunchKernelEx(&cfg, attn_decode_kernel<T, LPK, true>, a));
-        return LTCA_OK;
-    }
-    attn_decode_kernel<T, LPK, false><<<grid, kDecThreads, 0, ctx->stream>>>(a);
-    LTCA_LAUNCH_OK(ctx, "attn_decode_kernel");
-    if (a.nsplit > 1) {
-        attn_decode_merge_kernel<T><<<a.B * a.H, 128, 0, ctx->stream>>>(a);
-        LTCA_LAUNCH_OK(ctx, "attn_decode_merge_kernel");
-    }
+int run_decode(ltca_ctx* ctx, const DecodeArgs& a, const SplitPlan& plan) {
+    if (plan.cluster) return plan.few ? launch_decode<T, LPK, 8, 1>(ctx, a) : launch_decode<T, LPK, 4, 1>(ctx, a);
+    if (plan.n == 1) return plan.few ? launch_decode<T, LPK, 8, 0>(ctx, a) : launch_decode<T, LPK, 4, 0>(ctx, a);
+    if (int rc = launch_decode<T, LPK, 8, 2>(ctx, a)) return rc;
+    LTCA_CUDA_OK(ctx, launch_dependent(attn_decode_merge_kernel<T>, dim3(a.B * a.H), dim3(128), 0, ctx->stream, a));
     return LTCA_OK;
 }
 
 template <typename T>
-int dispatch_decode(ltca_ctx* ctx, const DecodeArgs& a) {
+int dispatch_decode(ltca_ctx* ctx, const DecodeArgs& a, const SplitPlan& plan) {
+    constexpr int EL = kLaneElems<T>;
     switch (a.D) {
-        case 16: return run_decode<T, 4>(ctx, a);
-        case 32: return run_decode<T, 8>(ctx, a);
-        case 64: return run_decode<T, 16>(ctx, a);
-        case 128: return run_decode<T, 32>(ctx, a);
+        case 16: return run_decode<T, 16 / EL>(ctx, a, plan);
+        case 32: return run_decode<T, 32 / EL>(ctx, a, plan);
+        case 64: return run_decode<T, 64 / EL>(ctx, a, plan);
+        case 128: return run_decode<T, 128 / EL>(ctx, a, plan);
     }
     return fail(ctx, LTCA_ERR_UNSUPPORTED, "decode supports head_dim 16, 32, 64, 128 (got %d)", a.D);
 }
@@ -270,11 +325,21 @@ int dispatch_decode(ltca_ctx* ctx, const DecodeArgs& a) {
 
 // The split count must not depend on the context, so that the size query (which has no
 // context) and the launch agree.  Non-positive shapes need no scratch (the launch refuses them).
+// A clustered call uses no scratch; the query still answers what its partials would take at one CTA per 256 keys, the
+// size by which ltca_attn_decode_static has always told large shapes from small ones.
 size_t attn_decode_workspace(const ltca_attn_params* p) {
     if (p->B < 1 || p->H < 1 || p->Sk < 1 || p->D < 1) return 0;
-    const int ns = pick_splits(p, kPlanSms);
-    if (ns <= 1) return 0;
-    return align_up((size_t)p->B * p->H * ns * (p->D + 2) * sizeof(float), 256);
+    const SplitPlan s = plan_splits(p);
+    if (!s.few) return 0;
+    const int64_t bh = (int64_t)p->B * p->H;
+    int64_t n = s.n;
+    if (s.cluster || n == 1) {
+        const int64_t want = (4 * (int64_t)kPlanSms + bh - 1) / bh, cap = (p->Sk + 255) / 256;
+        n = want < cap ? want : cap;
+        if (n > 64) n = 64;
+        if (n <= 1) return 0;
+    }
+    return align_up((size_t)bh * n * (p->D + 2) * sizeof(float), 256);
 }
 
 int launch_attn_decode(ltca_ctx* ctx, const ltca_attn_params* p) {
@@ -299,17 +364,20 @@ int launch_attn_decode(ltca_ctx* ctx, const ltca_attn_params* p) {
     a.lse = p->lse;
     a.keep_mask = p->keep_mask;
     a.kv_len = p->kv_len;
-    a.nsplit = pick_splits(p, kPlanSms);
-    if (pick_cluster(p, kPlanSms) > 1) {
-        a.nsplit = pick_cluster(p, kPlanSms);       // merged inside the cluster: a.partial stays null
-    } else if (a.nsplit > 1) {
+    a.vec16 = 1;
+    for (const ltca_strides* st : {&p->k_strides, &p->v_strides})
+        if ((st->seq * es) % 16 || (st->head * es) % 16 || (st->batch * es) % 16) a.vec16 = 0;
+    if ((reinterpret_cast<uintptr_t>(p->k) | reinterpret_cast<uintptr_t>(p->v)) % 16) a.vec16 = 0;
+    const SplitPlan plan = plan_splits(p);
+    a.nsplit = plan.n;
+    if (plan.n > 1 && !plan.cluster) {
         const size_t need = attn_decode_workspace(p);
         if (!p->workspace || p->workspace_bytes < need)
             return fail(ctx, LTCA_ERR_WORKSPACE, "decode needs %zu bytes of workspace", need);
         a.partial = reinterpret_cast<float*>(p->workspace);
     }
-    return p->dtype == LTCA_BF16 ? dispatch_decode<__nv_bfloat16>(ctx, a)
-                                 : dispatch_decode<float>(ctx, a);
+    return p->dtype == LTCA_BF16 ? dispatch_decode<__nv_bfloat16>(ctx, a, plan)
+                                 : dispatch_decode<float>(ctx, a, plan);
 }
 
 }  // namespace ltca
