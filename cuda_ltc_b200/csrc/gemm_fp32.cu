@@ -5,7 +5,7 @@
 // What bounds them: the small modules this pipeline serves (model widths of 32 to 256, up to a few thousand rows) are
 // launches and latency, the larger ones the FMA pipe.  So the products of one step (Q, K and V; the four weight gradients;
 // the three terms of dx) share a launch, the tile shrinks until the tiles occupy the SMs, and operands arrive by
-// 16-byte cp.async two steps ahead in whatever order they are stored: an operand whose rows run along the contraction is
+// 16-byte cp.async some steps ahead in whatever order they are stored: an operand whose rows run along the contraction is
 // read as vectors of four contraction steps, one whose rows run across it as vectors of four rows or columns, so
 // nothing is transposed on the way.
 // Measured at B8 S32 E32 with 4 heads of 32: 21 launches of one 128 x 128 tile kernel took 8 to 24 us each and 241 us a
@@ -18,7 +18,6 @@ namespace ltca {
 namespace {
 
 constexpr int kPad = 4;
-constexpr int kStages = 3;
 
 struct Gemm32Args {
     Gemm32Problem p[kMaxGemm32];
@@ -96,6 +95,9 @@ struct Frag {
 template <int TM, int TN, int NT>
 struct Gemm32Tile {
     static constexpr int KC = TM >= 128 ? 16 : 32;
+    // A 32 x 32 tile multiplies a step in a fraction of the latency of its loads and nothing else runs beside it (such
+    // launches have few CTAs): five steps in flight instead of two.
+    static constexpr int kStages = TM <= 32 ? 6 : 3;
     static constexpr int TY = NT / 16, RM = TM / TY, CN = TN / 16;
     static constexpr int VM = RM < 4 ? RM : 4, VN = CN < 4 ? CN : 4;
     template <bool TA> static constexpr int a_floats() { return TA ? KC * (TM + kPad) : TM * (KC + kPad); }
@@ -107,7 +109,7 @@ __global__ void __launch_bounds__(NT) gemm_fp32_kernel(const __grid_constant__ G
     grid_launch_dependents();
     grid_dependency_wait();
     using G = Gemm32Tile<TM, TN, NT>;
-    constexpr int KC = G::KC, RM = G::RM, CN = G::CN;
+    constexpr int KC = G::KC, RM = G::RM, CN = G::CN, kStages = G::kStages;
     constexpr int kA = G::template a_floats<TA>(), kB = G::template b_floats<TB>();
     extern __shared__ __align__(16) float sm[];
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
@@ -203,6 +205,98 @@ __global__ void __launch_bounds__(NT) gemm_fp32_kernel(const __grid_constant__ G
     }
 }
 
+// Small products whose sums may run in any order (gradients with respect to x and to the weights, the output projection):
+// 32 x 32 tiles whose four warps split every step of the contraction between them, each holding the whole tile (8 x 4
+// outputs per thread), and add their shares at the end.  A launch of a few such tiles is one chain of steps per CTA, and
+// this makes the chain four times shorter: at B8 S32 E32 with 4 heads of 32 dx takes 4 us instead of 11.  Two groups of
+// products, of different operand forms, share a launch (the steps behind the attention backward).
+constexpr int kSmallStages = 6, kSmallK = 32;
+struct Gemm32Pair {
+    Gemm32Args g[2];
+    int tiles_x[2], tiles_y[2], blocks[2];      // blocks[i] = tiles x products of group i
+    int form[2];                                // 0: A [M,K] B [K,N];  1: A [M,K] B [N,K];  2: A [K,M] B [K,N]
+};
+constexpr int kSmallFloats = kSmallStages * 2 * 32 * (32 + kPad);
+
+template <bool TA, bool TB>
+__device__ __forceinline__ void small_product(const Gemm32Args& g, int tx0, int ty0, int z, float* sm) {
+    constexpr int KC = kSmallK, LD = 32 + kPad, kTile = 32 * LD, S = kSmallStages;
+    const int warp = threadIdx.x >> 5, tx = threadIdx.x & 7, ty = (threadIdx.x >> 3) & 3;
+    const int first = g.sum ? 0 : z, terms = g.sum ? g.n : 1;
+    const int M = g.p[first].M, N = g.p[first].N, K = g.p[first].K;
+    const int m0 = ty0 * 32, n0 = tx0 * 32;
+    if (m0 >= M || n0 >= N) return;
+    const int steps = (K + KC - 1) / KC, all = steps * terms;
+    const bool vec = g.vec != 0;
+    auto fetch = [&](int it) {
+        if (it < all) {
+            const Gemm32Problem& p = g.p[first + it / steps];
+            const int k0 = (it % steps) * KC;
+            float* as = sm + (it % S) * 2 * kTile;
+            if constexpr (TA) load_block<KC, 32, 128>(as, p.A, p.lda, k0, K, m0, M, vec);
+            else load_block<32, KC, 128>(as, p.A, p.lda, m0, M, k0, K, vec);
+            if constexpr (TB) load_block<32, KC, 128>(as + kTile, p.B, p.ldb, n0, N, k0, K, vec);
+            else load_block<KC, 32, 128>(as + kTile, p.B, p.ldb, k0, K, n0, N, vec);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    float acc[8][4];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+#pragma unroll
+    for (int s = 0; s < S - 1; ++s) fetch(s);
+    for (int it = 0; it < all; ++it) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(S - 2) : "memory");
+        __syncthreads();
+        fetch(it + S - 1);
+        const float* as = sm + (it % S) * 2 * kTile;
+#pragma unroll
+        for (int k = 0; k < KC / 4; k += 4) {
+            Frag<!TA, 8, TA ? 4 : 1, TA ? 16 : 4> a;
+            Frag<TB, 4, TB ? 1 : 4, TB ? 8 : 32> b;
+            a.template load<LD>(as, TA ? 4 * ty : ty, warp * (KC / 4) + k);
+            b.template load<LD>(as + kTile, TB ? tx : 4 * tx, warp * (KC / 4) + k);
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a.v[e][i], b.v[e][j], acc[i][j]);
+        }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int r = TA ? (i / 4) * 16 + 4 * ty + i % 4 : ty + 4 * i, c = TB ? tx + 8 * j : 4 * tx + j;
+            sm[warp * kTile + r * LD + c] = acc[i][j];
+        }
+    __syncthreads();
+    const Gemm32Problem& p = g.p[first];
+    for (int e = threadIdx.x; e < 32 * 32; e += 128) {
+        const int r = e / 32, c = e % 32, gm = m0 + r, gn = n0 + c;
+        if (gm >= M || gn >= N) continue;
+        float v = (sm[r * LD + c] + sm[kTile + r * LD + c]) + (sm[2 * kTile + r * LD + c] + sm[3 * kTile + r * LD + c]);
+        if (p.bias) v += __ldg(p.bias + gn);
+        p.C[(int64_t)gm * p.ldc + gn] = v;
+    }
+}
+__global__ void __launch_bounds__(128) gemm_fp32_small_kernel(const __grid_constant__ Gemm32Pair a) {
+    grid_launch_dependents();
+    grid_dependency_wait();
+    extern __shared__ __align__(16) float sm[];
+    const int grp = (int)blockIdx.x < a.blocks[0] ? 0 : 1;
+    const int block = blockIdx.x - (grp ? a.blocks[0] : 0);
+    const int x = block % a.tiles_x[grp], y = block / a.tiles_x[grp] % a.tiles_y[grp], z = block / (a.tiles_x[grp] * a.tiles_y[grp]);
+    if (a.form[grp] == 0) small_product<false, false>(a.g[grp], x, y, z, sm);
+    else if (a.form[grp] == 1) small_product<false, true>(a.g[grp], x, y, z, sm);
+    else small_product<true, false>(a.g[grp], x, y, z, sm);
+}
+
 // C[m][n] = sum over slices, in slice order, of the partial results; blockIdx.y picks the product.
 __global__ void __launch_bounds__(256) gemm_fp32_reduce_kernel(const __grid_constant__ Gemm32Args g) {
     grid_launch_dependents();
@@ -220,7 +314,7 @@ __global__ void __launch_bounds__(256) gemm_fp32_reduce_kernel(const __grid_cons
 template <bool TA, bool TB, int TM, int TN, int NT>
 int launch(ltca_ctx* ctx, const Gemm32Args& g, int max_m, int max_n) {
     using G = Gemm32Tile<TM, TN, NT>;
-    constexpr int smem = kStages * (G::template a_floats<TA>() + G::template b_floats<TB>()) * (int)sizeof(float);
+    constexpr int smem = G::kStages * (G::template a_floats<TA>() + G::template b_floats<TB>()) * (int)sizeof(float);
     static SmemOptIn once;
     if (smem > 48 * 1024) LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(once, ctx->device, gemm_fp32_kernel<TA, TB, TM, TN, NT>, smem));
     dim3 grid((max_n + TN - 1) / TN, (max_m + TM - 1) / TM, (g.sum ? 1 : g.n) * g.slices);
@@ -235,11 +329,15 @@ int launch_tile(ltca_ctx* ctx, const Gemm32Args& g, int tile, int max_m, int max
     return launch<TA, TB, 32, 32, 128>(ctx, g, max_m, max_n);
 }
 
-}  // namespace
-
-int gemm_fp32(ltca_ctx* ctx, const Gemm32Problem* p, int n, int ta, int tb, bool sum, float* scratch, size_t scratch_bytes) {
-    if (n < 1 || n > kMaxGemm32) return fail(ctx, LTCA_ERR_INVALID, "gemm_fp32 takes 1 to %d products", kMaxGemm32);
+// Tile, slices and operand checks of one group of products.
+struct Plan32 {
     Gemm32Args g;
+    int tile, max_m, max_n;
+    int64_t tiles32;        // 32 x 32 tiles of the launch
+};
+int plan_gemm(ltca_ctx* ctx, Plan32* pl, const Gemm32Problem* p, int n, bool sum, float* scratch, size_t scratch_bytes) {
+    if (n < 1 || n > kMaxGemm32) return fail(ctx, LTCA_ERR_INVALID, "gemm_fp32 takes 1 to %d products", kMaxGemm32);
+    Gemm32Args& g = pl->g;
     memset(&g, 0, sizeof(g));
     g.n = n;
     g.sum = sum && n > 1 ? 1 : 0;
@@ -288,18 +386,72 @@ int gemm_fp32(ltca_ctx* ctx, const Gemm32Problem* p, int n, int ta, int tb, bool
             }
         }
     }
+    pl->tile = tile;
+    pl->max_m = max_m;
+    pl->max_n = max_n;
+    pl->tiles32 = tiles(32);
+    return LTCA_OK;
+}
+
+int launch_plan(ltca_ctx* ctx, const Plan32& pl, int ta, int tb) {
+    const Gemm32Args& g = pl.g;
     int rc;
-    if (!ta && !tb) rc = launch_tile<false, false>(ctx, g, tile, max_m, max_n);
-    else if (!ta && tb) rc = launch_tile<false, true>(ctx, g, tile, max_m, max_n);
-    else if (ta && !tb) rc = launch_tile<true, false>(ctx, g, tile, max_m, max_n);
+    if (!ta && !tb) rc = launch_tile<false, false>(ctx, g, pl.tile, pl.max_m, pl.max_n);
+    else if (!ta && tb) rc = launch_tile<false, true>(ctx, g, pl.tile, pl.max_m, pl.max_n);
+    else if (ta && !tb) rc = launch_tile<true, false>(ctx, g, pl.tile, pl.max_m, pl.max_n);
     else return fail(ctx, LTCA_ERR_UNSUPPORTED, "gemm_fp32: A stored [K, M] with B stored [N, K] is not built");
     if (rc || !g.partial) return rc;
     int64_t mn = 0;
-    for (int i = 0; i < n; ++i) if ((int64_t)p[i].M * p[i].N > mn) mn = (int64_t)p[i].M * p[i].N;
-    const int64_t blocks = (mn + 255) / 256;
-    LTCA_CUDA_OK(ctx, launch_dependent(gemm_fp32_reduce_kernel, dim3((unsigned)(blocks < 8 * sms ? blocks : 8 * sms), n), dim3(256), 0,
+    for (int i = 0; i < g.n; ++i) if ((int64_t)g.p[i].M * g.p[i].N > mn) mn = (int64_t)g.p[i].M * g.p[i].N;
+    const int64_t blocks = (mn + 255) / 256, most = 8 * (ctx->sm_device > 0 ? ctx->sm_device : kPlanSms);
+    LTCA_CUDA_OK(ctx, launch_dependent(gemm_fp32_reduce_kernel, dim3((unsigned)(blocks < most ? blocks : most), g.n), dim3(256), 0,
                                        ctx->stream, g));
     return LTCA_OK;
+}
+
+// Launches one or two groups of small products (see gemm_fp32_small_kernel).
+int launch_small(ltca_ctx* ctx, const Plan32* pl, const int* form, int groups) {
+    Gemm32Pair a;
+    memset(&a, 0, sizeof(a));
+    for (int i = 0; i < groups; ++i) {
+        a.g[i] = pl[i].g;
+        a.tiles_x[i] = (pl[i].max_n + 31) / 32;
+        a.tiles_y[i] = (pl[i].max_m + 31) / 32;
+        a.blocks[i] = a.tiles_x[i] * a.tiles_y[i] * (a.g[i].sum ? 1 : a.g[i].n);
+        a.form[i] = form[i];
+    }
+    constexpr int smem = kSmallFloats * (int)sizeof(float);
+    static SmemOptIn once;
+    LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(once, ctx->device, gemm_fp32_small_kernel, smem));
+    LTCA_CUDA_OK(ctx, launch_dependent(gemm_fp32_small_kernel, dim3((unsigned)(a.blocks[0] + a.blocks[1])), dim3(128), smem, ctx->stream, a));
+    return LTCA_OK;
+}
+// 32-wide tiles and an unsliced contraction: the launch is a chain of latencies.
+bool small_plan(const Plan32& pl) { return pl.tile == 32 && pl.g.slices == 1; }
+
+}  // namespace
+
+int gemm_fp32(ltca_ctx* ctx, const Gemm32Problem* p, int n, int ta, int tb, bool sum, bool any_order, float* scratch,
+              size_t scratch_bytes) {
+    Plan32 pl;
+    if (int rc = plan_gemm(ctx, &pl, p, n, sum, scratch, scratch_bytes)) return rc;
+    const int form = ta ? 2 : tb ? 1 : 0;
+    if (any_order && small_plan(pl) && !(ta && tb)) return launch_small(ctx, &pl, &form, 1);
+    return launch_plan(ctx, pl, ta, tb);
+}
+
+int gemm_fp32_grads(ltca_ctx* ctx, const Gemm32Problem* dx, int n_dx, const Gemm32Problem* dw, int n_dw, float* scratch,
+                    size_t scratch_bytes) {
+    Plan32 pl[2];
+    int rc;
+    if ((rc = plan_gemm(ctx, &pl[0], dx, n_dx, true, nullptr, 0))) return rc;
+    if ((rc = plan_gemm(ctx, &pl[1], dw, n_dw, false, scratch, scratch_bytes))) return rc;
+    if (small_plan(pl[0]) && small_plan(pl[1])) {
+        const int form[2] = {1, 2};
+        return launch_small(ctx, pl, form, 2);
+    }
+    if ((rc = gemm_fp32(ctx, dx, n_dx, 0, 1, true, true))) return rc;
+    return gemm_fp32(ctx, dw, n_dw, 1, 0, false, true, scratch, scratch_bytes);
 }
 
 }  // namespace ltca

@@ -20,7 +20,13 @@ constexpr int kMaxGemm32 = 4;
 // A launch whose contraction is long against its tiles is cut into slices that a second kernel sums in slice order, so the
 // result does not depend on the launch; `scratch` (or null) holds the slice results, with too little of it the slices
 // get longer.
-int gemm_fp32(ltca_ctx* ctx, const Gemm32Problem* p, int n, int ta, int tb, bool sum, float* scratch = nullptr,
+//   any_order: the sums need not run in ascending order of the contraction.  What the attention kernels read (the Q, K, V
+//   projections, the gradient at the context) keeps that order, so that it does not depend on the tile a launch takes.
+int gemm_fp32(ltca_ctx* ctx, const Gemm32Problem* p, int n, int ta, int tb, bool sum, bool any_order, float* scratch = nullptr,
               size_t scratch_bytes = 0);
+// The gradients behind the attention backward: dx = sum of n_dx products A [M,K] B [N,K], and n_dw products A [K,M] B [K,N];
+// one launch for both where they are small.
+int gemm_fp32_grads(ltca_ctx* ctx, const Gemm32Problem* dx, int n_dx, const Gemm32Problem* dw, int n_dw, float* scratch,
+                    size_t scratch_bytes);
 
 }  // namespace ltca

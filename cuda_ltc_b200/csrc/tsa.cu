@@ -564,7 +564,7 @@ int forward_core(ltca_ctx* ctx, const ltca_tsa_params* t, const Plan& pl, char* 
     const Gemm32Problem qkv[3] = {{t->x, t->wq, t->bq, fb->q, rows, HW, E, E, HW, HW},
                                   {t->x, t->wk, t->bk, fb->k, rows, HW, E, E, HW, HW},
                                   {t->x, t->wv, t->bv, fb->v, rows, HW, E, E, HW, HW}};
-    if ((rc = gemm_fp32(ctx, qkv, 3, 0, 0, false))) return rc;
+    if ((rc = gemm_fp32(ctx, qkv, 3, 0, 0, false, false))) return rc;
     ltca_attn_params a;
     fill_attn(t, &a);
     a.q = fb->q; a.k = fb->k; a.v = fb->v; a.o = fb->ctx; a.lse = fb->lse;
@@ -1195,7 +1195,7 @@ static int tsa_forward(ltca_ctx* ctx, const ltca_tsa_params* t, const ltca_tsa_p
     if ((rc = forward_core(ctx, t, pl, w, &fb, pl.attn_fwd))) return rc;
     const int rows = (int)pl.rows;
     const Gemm32Problem proj = {fb.ctx, t->wo, t->bo, y, rows, t->E, pl.HW, pl.HW, t->E, t->E};
-    if ((rc = gemm_fp32(ctx, &proj, 1, 0, 0, false))) return rc;
+    if ((rc = gemm_fp32(ctx, &proj, 1, 0, 0, false, true))) return rc;
     return outer ? prenorm_finish(ctx, outer, y) : residual_layer_norm(ctx, t, y, pl.rows);
 }
 
@@ -1243,7 +1243,7 @@ static int tsa_backward(ltca_ctx* ctx, const ltca_tsa_params* t, bool want_dx, b
     const int rows = (int)pl.rows, E = t->E, HW = pl.HW;
     // dctx = dy Wo^T
     const Gemm32Problem back = {t->dy, t->wo, nullptr, dctx, rows, HW, E, E, E, HW};
-    if ((rc = gemm_fp32(ctx, &back, 1, 0, 1, false))) return rc;
+    if ((rc = gemm_fp32(ctx, &back, 1, 0, 1, false, false))) return rc;
     ltca_attn_params a;
     fill_attn(t, &a);
     a.q = fb.q; a.k = fb.k; a.v = fb.v; a.o = fb.ctx; a.lse = fb.lse;
@@ -1258,21 +1258,19 @@ static int tsa_backward(ltca_ctx* ctx, const ltca_tsa_params* t, bool want_dx, b
         jobs->add(dv, false, HW, HW, t->dbv);
         jobs->add(t->dy, false, E, E, t->dbo);
     }
-    if (want_dx) {
-        const Gemm32Problem terms[3] = {{dq, t->wq, nullptr, t->dx, rows, E, HW, HW, HW, E},
-                                        {dk, t->wk, nullptr, t->dx, rows, E, HW, HW, HW, E},
-                                        {dv, t->wv, nullptr, t->dx, rows, E, HW, HW, HW, E}};
-        if ((rc = gemm_fp32(ctx, terms, 3, 0, 1, true))) return rc;
-    }
-    if (want_dw) {
-        // dW = x^T dQ  ([E, rows] x [rows, HW]),  dWo = ctx^T dy  ([HW, rows] x [rows, E])
-        // dctx is dead once the attention backward has run: it holds the contraction slices
-        const Gemm32Problem dw[4] = {{t->x, dq, nullptr, t->dwq, E, HW, rows, E, HW, HW},
-                                     {t->x, dk, nullptr, t->dwk, E, HW, rows, E, HW, HW},
-                                     {t->x, dv, nullptr, t->dwv, E, HW, rows, E, HW, HW},
-                                     {fb.ctx, t->dy, nullptr, t->dwo, HW, E, rows, HW, E, E}};
-        if ((rc = gemm_fp32(ctx, dw, 4, 1, 0, false, dctx, pl.buf))) return rc;
-    }
+    const Gemm32Problem terms[3] = {{dq, t->wq, nullptr, t->dx, rows, E, HW, HW, HW, E},
+                                    {dk, t->wk, nullptr, t->dx, rows, E, HW, HW, HW, E},
+                                    {dv, t->wv, nullptr, t->dx, rows, E, HW, HW, HW, E}};
+    // dW = x^T dQ  ([E, rows] x [rows, HW]),  dWo = ctx^T dy  ([HW, rows] x [rows, E])
+    // dctx is dead once the attention backward has run: it holds the contraction slices
+    const Gemm32Problem dw[4] = {{t->x, dq, nullptr, t->dwq, E, HW, rows, E, HW, HW},
+                                 {t->x, dk, nullptr, t->dwk, E, HW, rows, E, HW, HW},
+                                 {t->x, dv, nullptr, t->dwv, E, HW, rows, E, HW, HW},
+                                 {fb.ctx, t->dy, nullptr, t->dwo, HW, E, rows, HW, E, E}};
+    if (want_dx && want_dw) rc = gemm_fp32_grads(ctx, terms, 3, dw, 4, dctx, pl.buf);
+    else if (want_dx) rc = gemm_fp32(ctx, terms, 3, 0, 1, true, true);
+    else if (want_dw) rc = gemm_fp32(ctx, dw, 4, 1, 0, false, true, dctx, pl.buf);
+    if (rc) return rc;
     return column_sums(ctx, own, pl.rows, colsum_scratch);
 }
 
