@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(NT) gemm_fp32_kernel(const __grid_constant__ G
     for (int i = 0; i < RM; ++i)
 #pragma unroll
         for (int j = 0; j < CN; ++j) { acc[i][j] = 0.f; total[i][j] = 0.f; }
-#pragma unroll
+#pragma unroll 1
     for (int s = 0; s < kStages - 1; ++s) fetch(s);
     for (int it = 0; it < all; ++it) {
         asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(NT) gemm_fp32_kernel(const __grid_constant__ G
         fetch(it + kStages - 1);
         const float* as = sm + (it % kStages) * (kA + kB);
         const float* bs = as + kA;
-#pragma unroll
+#pragma unroll(TM <= 32 ? 1 : KC / 4)
         for (int k = 0; k < KC; k += 4) {
             Frag<!TA, RM, G::VM, G::VM * G::TY> a;
             Frag<TB, CN, VN, VN * 16> b;
@@ -206,11 +206,13 @@ __global__ void __launch_bounds__(NT) gemm_fp32_kernel(const __grid_constant__ G
 }
 
 // Small products whose sums may run in any order (gradients with respect to x and to the weights, the output projection):
-// 32 x 32 tiles whose four warps split every step of the contraction between them, each holding the whole tile (8 x 4
-// outputs per thread), and add their shares at the end.  A launch of a few such tiles is one chain of steps per CTA, and
-// this makes the chain four times shorter: at B8 S32 E32 with 4 heads of 32 dx takes 4 us instead of 11.  Two groups of
-// products, of different operand forms, share a launch (the steps behind the attention backward).
-constexpr int kSmallStages = 6, kSmallK = 32;
+// 32 x 32 tiles whose eight warps split every step of the contraction between them, each holding the whole tile (8 x 4
+// outputs per thread), and add their shares at the end: a launch of a few such tiles is one chain of steps per CTA, and
+// this makes the chain eight times shorter.  The loops are not unrolled: such a launch meets a cold instruction cache,
+// and fetching straight-line code took longer than running it (B8 S32 E32 with 4 heads of 32: dx and the weight gradients
+// 24 us as launches of their own, 11.5 unrolled with four warps, 10 rolled).  Two groups of products, of different operand
+// forms, share a launch (the steps behind the attention backward).
+constexpr int kSmallStages = 6, kSmallK = 32, kSmallWarps = 8, kSmallThreads = 32 * kSmallWarps;
 struct Gemm32Pair {
     Gemm32Args g[2];
     int tiles_x[2], tiles_y[2], blocks[2];      // blocks[i] = tiles x products of group i
@@ -220,7 +222,7 @@ constexpr int kSmallFloats = kSmallStages * 2 * 32 * (32 + kPad);
 
 template <bool TA, bool TB>
 __device__ __forceinline__ void small_product(const Gemm32Args& g, int tx0, int ty0, int z, float* sm) {
-    constexpr int KC = kSmallK, LD = 32 + kPad, kTile = 32 * LD, S = kSmallStages;
+    constexpr int KC = kSmallK, KW = KC / kSmallWarps, LD = 32 + kPad, kTile = 32 * LD, S = kSmallStages;
     const int warp = threadIdx.x >> 5, tx = threadIdx.x & 7, ty = (threadIdx.x >> 3) & 3;
     const int first = g.sum ? 0 : z, terms = g.sum ? g.n : 1;
     const int M = g.p[first].M, N = g.p[first].N, K = g.p[first].K;
@@ -233,10 +235,10 @@ __device__ __forceinline__ void small_product(const Gemm32Args& g, int tx0, int 
             const Gemm32Problem& p = g.p[first + it / steps];
             const int k0 = (it % steps) * KC;
             float* as = sm + (it % S) * 2 * kTile;
-            if constexpr (TA) load_block<KC, 32, 128>(as, p.A, p.lda, k0, K, m0, M, vec);
-            else load_block<32, KC, 128>(as, p.A, p.lda, m0, M, k0, K, vec);
-            if constexpr (TB) load_block<32, KC, 128>(as + kTile, p.B, p.ldb, n0, N, k0, K, vec);
-            else load_block<KC, 32, 128>(as + kTile, p.B, p.ldb, k0, K, n0, N, vec);
+            if constexpr (TA) load_block<KC, 32, kSmallThreads>(as, p.A, p.lda, k0, K, m0, M, vec);
+            else load_block<32, KC, kSmallThreads>(as, p.A, p.lda, m0, M, k0, K, vec);
+            if constexpr (TB) load_block<32, KC, kSmallThreads>(as + kTile, p.B, p.ldb, n0, N, k0, K, vec);
+            else load_block<KC, 32, kSmallThreads>(as + kTile, p.B, p.ldb, k0, K, n0, N, vec);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
@@ -245,19 +247,19 @@ __device__ __forceinline__ void small_product(const Gemm32Args& g, int tx0, int 
     for (int i = 0; i < 8; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
-#pragma unroll
+#pragma unroll 1
     for (int s = 0; s < S - 1; ++s) fetch(s);
     for (int it = 0; it < all; ++it) {
         asm volatile("cp.async.wait_group %0;" ::"n"(S - 2) : "memory");
         __syncthreads();
         fetch(it + S - 1);
         const float* as = sm + (it % S) * 2 * kTile;
-#pragma unroll
-        for (int k = 0; k < KC / 4; k += 4) {
+#pragma unroll 1
+        for (int k = 0; k < KW; k += 4) {
             Frag<!TA, 8, TA ? 4 : 1, TA ? 16 : 4> a;
             Frag<TB, 4, TB ? 1 : 4, TB ? 8 : 32> b;
-            a.template load<LD>(as, TA ? 4 * ty : ty, warp * (KC / 4) + k);
-            b.template load<LD>(as + kTile, TB ? tx : 4 * tx, warp * (KC / 4) + k);
+            a.template load<LD>(as, TA ? 4 * ty : ty, warp * KW + k);
+            b.template load<LD>(as + kTile, TB ? tx : 4 * tx, warp * KW + k);
 #pragma unroll
             for (int e = 0; e < 4; ++e)
 #pragma unroll
@@ -277,15 +279,17 @@ __device__ __forceinline__ void small_product(const Gemm32Args& g, int tx0, int 
         }
     __syncthreads();
     const Gemm32Problem& p = g.p[first];
-    for (int e = threadIdx.x; e < 32 * 32; e += 128) {
+    for (int e = threadIdx.x; e < 32 * 32; e += kSmallThreads) {
         const int r = e / 32, c = e % 32, gm = m0 + r, gn = n0 + c;
         if (gm >= M || gn >= N) continue;
-        float v = (sm[r * LD + c] + sm[kTile + r * LD + c]) + (sm[2 * kTile + r * LD + c] + sm[3 * kTile + r * LD + c]);
+        float v = 0.f;
+#pragma unroll
+        for (int w = 0; w < kSmallWarps; ++w) v += sm[w * kTile + r * LD + c];
         if (p.bias) v += __ldg(p.bias + gn);
         p.C[(int64_t)gm * p.ldc + gn] = v;
     }
 }
-__global__ void __launch_bounds__(128) gemm_fp32_small_kernel(const __grid_constant__ Gemm32Pair a) {
+__global__ void __launch_bounds__(kSmallThreads) gemm_fp32_small_kernel(const __grid_constant__ Gemm32Pair a) {
     grid_launch_dependents();
     grid_dependency_wait();
     extern __shared__ __align__(16) float sm[];
@@ -423,7 +427,7 @@ int launch_small(ltca_ctx* ctx, const Plan32* pl, const int* form, int groups) {
     constexpr int smem = kSmallFloats * (int)sizeof(float);
     static SmemOptIn once;
     LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(once, ctx->device, gemm_fp32_small_kernel, smem));
-    LTCA_CUDA_OK(ctx, launch_dependent(gemm_fp32_small_kernel, dim3((unsigned)(a.blocks[0] + a.blocks[1])), dim3(128), smem, ctx->stream, a));
+    LTCA_CUDA_OK(ctx, launch_dependent(gemm_fp32_small_kernel, dim3((unsigned)(a.blocks[0] + a.blocks[1])), dim3(kSmallThreads), smem, ctx->stream, a));
     return LTCA_OK;
 }
 // 32-wide tiles and an unsliced contraction: the launch is a chain of latencies.
