@@ -78,8 +78,8 @@ __global__ void bf16_to_f32_kernel(const __nv_bfloat16* __restrict__ s, float* _
         d[i] = __bfloat162float(s[i]);
 }
 
-// Strided fp32 [B,H,S,D] -> contiguous bf16 [B,H,S,D]; one thread per 4 elements (D % 4 == 0).  blockIdx.y picks
-// the tensor, so the operands of one attention call are packed by one launch.
+// Strided fp32 [B,H,S,D] -> contiguous bf16 [B,H,S,D].  blockIdx.y picks the tensor, so the operands of one attention
+// call are packed by one launch.
 struct PackJobs {
     const float* src[kMaxPackJobs];
     __nv_bfloat16* dst[kMaxPackJobs];
@@ -87,38 +87,60 @@ struct PackJobs {
     ltca_strides st[kMaxPackJobs];
     int S[kMaxPackJobs];
 };
-__global__ void pack_bf16_kernel(const __grid_constant__ PackJobs jobs, int BH, int H, int D) {
-    grid_launch_dependents();
+
+// four values in bf16, and what the rounding left of each
+__device__ __forceinline__ uint2 round4(const float4& v) {
+    const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+    return make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+}
+__device__ __forceinline__ float4 rest4(const float4& v, const uint2& r) {
+    const __nv_bfloat162 a = *reinterpret_cast<const __nv_bfloat162*>(&r.x), b = *reinterpret_cast<const __nv_bfloat162*>(&r.y);
+    return make_float4(v.x - __low2float(a), v.y - __high2float(a), v.z - __low2float(b), v.w - __high2float(b));
+}
+
+// Bound by memory.  A block takes kPackChunks * 256 consecutive pieces of 4 * kVec values: kVec = 2 wherever head_dim is
+// a multiple of 8, so that a piece is one 16-byte store; all loads of a thread are issued before its first store.  The
+// place of a piece is found with 32-bit arithmetic from the block's first row.
+// The kernel after this one may be placed when a block's loads are done, not before: released at the start, the
+// attention kernel's CTAs settled four at a time on the SMs that had room first (B2 H8 S2800 D64 causal 109 us against
+// 74), where 352 of them should spread over 148 SMs.  50 MB of fp32 to bf16: 20 us with a piece of 16 bytes per thread and
+// step, 64-bit divisions and the release at the start, 12 us so.
+constexpr int kPackChunks = 4;
+template <int kVec>
+__global__ void __launch_bounds__(256) pack_bf16_kernel(const __grid_constant__ PackJobs jobs, int BH, int H, int D) {
     grid_dependency_wait();
     const int j = blockIdx.y;
     const float* __restrict__ src = jobs.src[j];
-    __nv_bfloat16* __restrict__ dst = jobs.dst[j];
-    __nv_bfloat16* __restrict__ low = jobs.lo[j];
     const ltca_strides st = jobs.st[j];
-    const int S = jobs.S[j];
-    const int d4 = D / 4;
-    const size_t n4 = (size_t)BH * S * d4;
-    const size_t stride = (size_t)gridDim.x * blockDim.x;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += stride) {
-        const int dd = (int)(i % d4);
-        size_t r = i / d4;
-        const int s = (int)(r % S); r /= S;
-        const int h = (int)(r % H);
-        const int64_t b = (int64_t)(r / H);
-        const float4 v = *reinterpret_cast<const float4*>(src + b * st.batch + h * st.head + (int64_t)s * st.seq + 4 * dd);
-        __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
-        uint2 u;
-        u.x = *reinterpret_cast<uint32_t*>(&lo);
-        u.y = *reinterpret_cast<uint32_t*>(&hi);
-        reinterpret_cast<uint2*>(dst)[i] = u;
-        if (low) {
-            const __nv_bfloat162 l0 = __floats2bfloat162_rn(v.x - __low2float(lo), v.y - __high2float(lo));
-            const __nv_bfloat162 l1 = __floats2bfloat162_rn(v.z - __low2float(hi), v.w - __high2float(hi));
-            uint2 w;
-            w.x = *reinterpret_cast<const uint32_t*>(&l0);
-            w.y = *reinterpret_cast<const uint32_t*>(&l1);
-            reinterpret_cast<uint2*>(low)[i] = w;
-        }
+    const unsigned S = (unsigned)jobs.S[j], per_row = (unsigned)D / (4 * kVec);
+    const uint64_t total = (uint64_t)BH * S * per_row, first = (uint64_t)blockIdx.x * (kPackChunks * 256);
+    const unsigned row0 = (unsigned)(first / per_row), in_row0 = (unsigned)(first - (uint64_t)row0 * per_row);
+    float4 v[kPackChunks][kVec];
+#pragma unroll
+    for (int c = 0; c < kPackChunks; ++c) {
+        const unsigned local = c * 256 + threadIdx.x;
+        if (first + local >= total) break;
+        const unsigned at = in_row0 + local, r = at / per_row, row = row0 + r, piece = at - r * per_row;
+        const unsigned bh = row / S, s = row - bh * S, b = bh / (unsigned)H, h = bh - b * (unsigned)H;
+        const float4* p = reinterpret_cast<const float4*>(src + (int64_t)b * st.batch + (int64_t)h * st.head + (int64_t)s * st.seq) + piece * kVec;
+#pragma unroll
+        for (int e = 0; e < kVec; ++e) v[c][e] = __ldg(p + e);
+    }
+    grid_launch_dependents();
+#pragma unroll
+    for (int c = 0; c < kPackChunks; ++c) {
+        const uint64_t i = first + c * 256 + threadIdx.x;
+        if (i >= total) break;
+        uint2 r[kVec], w[kVec];
+#pragma unroll
+        for (int e = 0; e < kVec; ++e) r[e] = round4(v[c][e]);
+        if constexpr (kVec == 2) reinterpret_cast<uint4*>(jobs.dst[j])[i] = make_uint4(r[0].x, r[0].y, r[1].x, r[1].y);
+        else reinterpret_cast<uint2*>(jobs.dst[j])[i] = r[0];
+        if (!jobs.lo[j]) continue;
+#pragma unroll
+        for (int e = 0; e < kVec; ++e) w[e] = round4(rest4(v[c][e], r[e]));
+        if constexpr (kVec == 2) reinterpret_cast<uint4*>(jobs.lo[j])[i] = make_uint4(w[0].x, w[0].y, w[1].x, w[1].y);
+        else reinterpret_cast<uint2*>(jobs.lo[j])[i] = w[0];
     }
 }
 
@@ -377,12 +399,11 @@ int pack_many_to_bf16(ltca_ctx* ctx, const PackJob* jobs, int count, int B, int 
         k.S[j] = jobs[j].S;
         if (jobs[j].S > s_max) s_max = jobs[j].S;
     }
-    // the grid is sized for the longest tensor; 16 blocks per SM over all the tensors together
-    const size_t n4 = (size_t)B * H * s_max * D / 4;
-    int bx = blocks_for(n4, 256, ctx->sm_count);
-    const int cap = (ctx->sm_count > 0 ? ctx->sm_count : kPlanSms) * 16 / count;
-    if (bx > cap) bx = cap;
-    LTCA_CUDA_OK(ctx, launch_dependent(pack_bf16_kernel, dim3((unsigned)bx, (unsigned)count), dim3(256), 0, ctx->stream, k,
+    const int vec = D % 8 ? 1 : 2;
+    const uint64_t pieces = (uint64_t)B * H * s_max * (D / (4 * vec)), blocks = (pieces + kPackChunks * 256 - 1) / (kPackChunks * 256);
+    if (blocks > 0x7fffffffull) return fail(ctx, LTCA_ERR_INVALID, "pack: tensor too large");
+    const dim3 grid((unsigned)blocks, (unsigned)count);               // sized for the longest tensor
+    LTCA_CUDA_OK(ctx, launch_dependent(vec == 2 ? pack_bf16_kernel<2> : pack_bf16_kernel<1>, grid, dim3(256), 0, ctx->stream, k,
                                        B * H, H, D));
     LTCA_LAUNCH_OK(ctx, "pack_bf16_kernel");
     return LTCA_OK;
