@@ -6,7 +6,8 @@
 // contract (scale, keep-mask with 0 = hidden, optional score clamp), plus a causal flag and
 // per-sequence key lengths, computed as a true online softmax.
 //
-// Shape of the kernel
+// Two kernels: attn_fwd_tile_sm100_kernel, a CTA per 128-row query tile (further down), and, for calls of few tiles with
+// long keys at head_dim 64, attn_fwd_sm100_kernel:
 //   - one CTA per (256 query rows, head, batch): two 128-row query tiles share every K/V tile
 //     that TMA brings in, which halves the L2 -> shared traffic per FLOP;
 //   - 16 softmax warps: a query row belongs to TWO threads, each owning half of the step's key
@@ -23,10 +24,10 @@
 //     epilogue;
 //   - K and V tiles travel through one ring of shared-memory slots in the order
 //     K0 V0 K1 V1 ..., each slot guarded by a full/empty mbarrier pair.
-//
-// Keys per step (kBN): 128 for head_dim 64 with a bf16 result, else 64 (head_dim 128, or the
-// split-P variant below), chosen so that everything fits the 512 tensor-memory columns:
-//   S0 S1 (kBN each) | O0 O1 (D each) | P0 P1 (kBN/2 each) | split-P only: Plo0 Plo1 (kBN/2 each)
+// Its keys per step: 128 for a bf16 result, else 64 (the split-P variant), chosen so that everything fits the 512
+// tensor-memory columns: S0 S1 (kBN each) | O0 O1 (D each) | P0 P1 (kBN/2 each) | split-P only: Plo0 Plo1 (kBN/2 each)
+#include <type_traits>
+
 #include "host_common.h"
 #include "attn_mask.cuh"
 #include "sm100_ptx.cuh"
@@ -38,7 +39,6 @@ namespace ltca {
 namespace {
 
 constexpr int kBlockM = 128;        // query rows per tile
-constexpr int kFwd4MinSq = 256;     // queries above which the four-tile persistent kernel is used
 // Two threads share one query row (each owns half of the step's key columns): 16 softmax warps, four per
 // scheduler, row maxima exchanged through shared memory.  (One thread per row, 8 warps, hid no latency.)
 constexpr int kRowSplit = 2;
@@ -533,104 +533,75 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
 }
 
 // ---------------------------------------------------------------------------------------------
-// Four-tile persistent kernel (head_dim 64, bf16 result): the kernel used for long query ranges.
+// One-tile kernel: a CTA is ONE 128-row query tile, four CTAs to an SM at head_dim 64, two at 128.
 //
-// Every scheduler of the SM holds four softmax warps that belong to four DIFFERENT query tiles;
-// a tile's warps only ever wait for that tile's own barriers, so while one tile sits in a
-// barrier round trip, a tensor-memory load or the tensor pipe's queue, the other three keep the
-// special-function unit busy (measured on B200: four independent warps per scheduler hide every
-// one of those latencies, two dependent ones hide almost none).
-//   - steps of 64 keys; tile t: S_t = Q_t K_j^T in columns [64 t, 64 t + 64), O_t in
-//     [256 + 64 t, 256 + 64 t + 64); P_t (bf16) overwrites the first 32 columns of S_t, so the
-//     issuer queues O_t += P_t V_j and S_t = Q_t K_{j+1}^T back to back (the tensor pipe runs one
-//     thread's MMAs in order) and one commit tells the tile both "S ready" and "O up to date";
-//   - warps 0-15: softmax, one query row per thread (tile = warp / 4); warp 16 issues the
-//     contractions of tiles 0 and 1, warp 17 those of tiles 2 and 3; warp 18: TMA producer.
-//
-// Persistent: one CTA per SM takes (512 query rows, head, batch)
-// items from a global counter (ItemQueue; grouped heavy-first order).  Barriers, tensor memory
-// and tensor maps are set up once per CTA; the Q tiles are double-buffered and the K/V ring runs
-// straight from one item's last keys into the next item's first, so the pipeline never drains:
-// a tile that has finished its rows of item i (the early tiles of a causal block have fewer key
-// steps) writes its output and starts on item i+1 while the later tiles still work on item i.
-// (A one-CTA-per-block version of this kernel spent 8.6 us per 512-row block on set-up, pipeline fill and drain.)
-// Barrier phases run on per-role counters; every completion of a reused barrier depends on the
-// waiter of the previous one, so a parity wait cannot alias:
-//   s_full(t)    one commit per key step + one at the start and one at the end of an item
-//   p_full(t)    one arrival per softmax warp per step
-//   tile_free(t) the tile's warps have read O of the previous item out of tensor memory
-//   q_full/q_empty[2], kv_full/kv_empty[8] as usual (both MMA threads release a slot).
+// Softmax warps of several tiles share every scheduler, as latencies between the two contractions of a step need (a step
+// leaves a tile's warps idle for about 1300 cycles while P is multiplied and the next scores are formed), and the tiles
+// are independent work: a causal tile of two key steps leaves after two and the next takes its place, and a call is
+// dealt out in pieces of 128 rows.  A persistent kernel with four tiles on one key stream, which this replaces, made the
+// early tiles of 512 causal rows wait for the late ones' keys: B64 H8 S512 causal 68 us against 49, B8 H16 S4096 causal
+// 440 against 392.  What it pays is a set-up per tile and a K/V read per tile from L2 (20 bytes per clock and SM).
+//   - head_dim 64: warps 0-3 softmax, one row per thread, 64 keys per step; tensor memory S [0, 64), O [64, 128);
+//   - head_dim 128: warps 0-7, two threads per row, each 64 of the 128 keys of a step and 64 of the output columns (the row
+//     maxima meet through shared memory); S [0, 128), O [128, 256);
+//   - P overwrites the first half of S, its second bf16 term (kSplitP: results stored as fp32) the other half;
+//   - of the last four warps one issues the contractions and one is the TMA producer (the others complete the
+//     warpgroup that gives registers up);
+//   - the result leaves through the Q slot (fp32: and the ring) and a TMA store.
 // ---------------------------------------------------------------------------------------------
-constexpr int kF4Tiles = 4;
-constexpr int kF4BN = 64;
-constexpr int kF4Threads = 640;
-constexpr int kF4LaunchRegs = 96;
-constexpr int kF4CtrlRegs = 56;
-constexpr int kF4MathRegs = 104;
-static_assert(512 * kF4MathRegs + 128 * kF4CtrlRegs <= kF4Threads * kF4LaunchRegs, "register budget");
-
-struct F4PCfg {
-    static constexpr int kQTileBytes = kBlockM * 64 * 2;       // 16 KB
-    static constexpr int kKvTileBytes = kF4BN * 64 * 2;        // 8 KB
-    static constexpr int kStages = 8;
-    static constexpr int kQBufBytes = kF4Tiles * kQTileBytes;  // 64 KB, two of them
-    static constexpr int kRingOff = 2 * kQBufBytes;
-    static constexpr int kBarOff = kRingOff + kStages * kKvTileBytes;
-    // q_full[2], q_empty[2], kv_full[S], kv_empty[S], s_full[4], p_full[4], tile_free[4], staged[4], item full/empty
-    static constexpr int kNumBars = 4 + 2 * kStages + 4 * kF4Tiles + 2 * kItemSlots;
+template <int D>
+struct TileCfg {
+    static constexpr int kRowSplit = D / 64;                       // threads per row
+    static constexpr int kMathWarps = 4 * kRowSplit;
+    static constexpr int kThreads = 32 * (kMathWarps + 4);
+    static constexpr int kCtas = 4 / kRowSplit;                    // per SM
+    static constexpr int kLaunchRegs = 65536 / (kCtas * kThreads) / 8 * 8;
+    static constexpr int kMathRegs = 104, kCtrlRegs = D == 64 ? 24 : 32;
+    static_assert(32 * kMathWarps * kMathRegs + 128 * kCtrlRegs <= kThreads * kLaunchRegs, "register budget");
+    static constexpr int kBN = D;                                  // keys per step
+    static constexpr int kBlocks = D / 64;                         // 128-byte column blocks of a row
+    static constexpr int kQBytes = kBlockM * D * 2;
+    static constexpr int kKvBytes = kBN * D * 2;
+    static constexpr int kStages = D == 64 ? 4 : 2;                // ring slots: K0 V0 K1 V1 ...
+    static constexpr int kRingOff = kQBytes;
+    static constexpr int kXchgOff = kRingOff + kStages * kKvBytes; // row maxima [2 buffers][2 halves][128], row sums [2][128]
+    static constexpr int kBarOff = kXchgOff + (kRowSplit > 1 ? 3 * 2 * kBlockM * 4 : 0);
+    static constexpr int kNumBars = 1 + 2 * kStages + 3 + 4;       // q_full, kv_full[], kv_empty[], s_full, p_full, staged, pair[4]
     static constexpr int kMiscOff = kBarOff + kNumBars * 8;
-    static constexpr int kDynBytes = kMiscOff + 16 + 4 * kItemSlots + 1024;
+    static constexpr int kDynBytes = kMiscOff + 16 + 1024;
+    static_assert(kCtas * (kDynBytes + 1024) <= 228 * 1024, "shared memory");
+    static constexpr uint32_t kTmemCols = 2 * D;
 };
 
-template <bool kFold, bool kMask>
-__global__ void __launch_bounds__(kF4Threads, 1)
-attn_fwd4p_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
-                        const __grid_constant__ CUtensorMap tmap_k,
-                        const __grid_constant__ CUtensorMap tmap_v,
-                        const __grid_constant__ CUtensorMap tmap_o, const FwdArgs a, const ItemGrid grid) {
-    using L = F4PCfg;
-    constexpr int D = 64;
-    constexpr int kBN = kF4BN;
+template <int D, bool kSplitP, bool kMask>
+__global__ void __launch_bounds__(TileCfg<D>::kThreads, TileCfg<D>::kCtas)
+attn_fwd_tile_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
+                           const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_o, const FwdArgs a) {
+    using L = TileCfg<D>;
+    constexpr int kBN = L::kBN, kRS = L::kRowSplit, kMmaWarp = L::kMathWarps, kTmaWarp = L::kMathWarps + 1;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
-    const uint32_t q_smem = smem_base;
-    const uint32_t ring_smem = smem_base + L::kRingOff;
+    const uint32_t ring = smem_base + L::kRingOff;
     const uint32_t bar_base = smem_base + L::kBarOff;
-    auto bar_q_full = [&](int r) { return bar_base + 8u * r; };
-    auto bar_q_empty = [&](int r) { return bar_base + 8u * (2 + r); };
-    auto bar_kv_full = [&](int s) { return bar_base + 8u * (4 + s); };
-    auto bar_kv_empty = [&](int s) { return bar_base + 8u * (4 + L::kStages + s); };
-    auto bar_s_full = [&](int t) { return bar_base + 8u * (4 + 2 * L::kStages + t); };
-    auto bar_p_full = [&](int t) { return bar_base + 8u * (4 + 2 * L::kStages + kF4Tiles + t); };
-    auto bar_tile_free = [&](int t) { return bar_base + 8u * (4 + 2 * L::kStages + 2 * kF4Tiles + t); };
-    auto bar_staged = [&](int t) { return bar_base + 8u * (4 + 2 * L::kStages + 3 * kF4Tiles + t); };
-    const uint32_t bar_item0 = bar_base + 8u * (4 + 2 * L::kStages + 4 * kF4Tiles);
+    auto bar_kv_full = [&](int s) { return bar_base + 8u * (1 + s); };
+    auto bar_kv_empty = [&](int s) { return bar_base + 8u * (1 + L::kStages + s); };
+    const uint32_t bar_q_full = bar_base, bar_s_full = bar_base + 8u * (1 + 2 * L::kStages), bar_p_full = bar_s_full + 8,
+                   bar_staged = bar_s_full + 16, bar_pair0 = bar_s_full + 24;
     volatile uint32_t* misc = reinterpret_cast<volatile uint32_t*>(smem_gen + L::kMiscOff);
-    const ItemQueue iq{bar_item0, bar_item0 + 8u * kItemSlots,
-                       reinterpret_cast<volatile int*>(smem_gen + L::kMiscOff + 16)};
-
-    const int warp = threadIdx.x >> 5;
-    const int lane = threadIdx.x & 31;
-    LTCA_TRACE_DECL(blockIdx.x == 5);
-    LTCA_TRACE_EVT(0x01);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
     if (threadIdx.x == 0) {
-        // a Q buffer is free again when both MMA threads are done with it and every tile's output,
-        // which is staged in the tile's own Q slot, has been read by its TMA store
-        for (int r = 0; r < 2; ++r) { mbar_init(bar_q_full(r), 1); mbar_init(bar_q_empty(r), 2 + kF4Tiles); }
-        for (int s = 0; s < L::kStages; ++s) { mbar_init(bar_kv_full(s), 1); mbar_init(bar_kv_empty(s), 2); }
-        for (int t = 0; t < kF4Tiles; ++t) {
-            mbar_init(bar_s_full(t), 1);
-            mbar_init(bar_p_full(t), 4);
-            mbar_init(bar_tile_free(t), 4);
-            mbar_init(bar_staged(t), 4);
-        }
-        for (int i = 0; i < kItemSlots; ++i) { mbar_init(iq.full(i), 1); mbar_init(iq.empty(i), 18); }
+        mbar_init(bar_q_full, 1);
+        for (int s = 0; s < L::kStages; ++s) { mbar_init(bar_kv_full(s), 1); mbar_init(bar_kv_empty(s), 1); }
+        mbar_init(bar_s_full, 1);
+        mbar_init(bar_p_full, L::kMathWarps);
+        mbar_init(bar_staged, L::kMathWarps);
+        for (int i = 0; i < 4; ++i) mbar_init(bar_pair0 + 8u * i, 2);
         misc[1] = 0u;
         mbar_fence_init();
     }
-    if (warp == 16) { tmem_alloc(smem_u32(const_cast<uint32_t*>(&misc[0])), kTmemCols); tmem_relinquish(); }
+    if (warp == kMmaWarp) { tmem_alloc(smem_u32(const_cast<uint32_t*>(&misc[0])), L::kTmemCols); tmem_relinquish(); }
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
@@ -638,452 +609,281 @@ attn_fwd4p_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
     const WaitCtx wc{&misc[1], a.status};
     grid_dependency_wait();                    // the operands are complete once the kernel before this one has ended
 
-    // the item's block, its (head, batch), and the number of 64-key steps of each tile
-    struct Item { int m_block, h, b, kvlen, n_max; };
-    // First query row of tile t of block m.  Plain: four neighbouring tiles.  Folded (a causal launch with no more
-    // items than SMs, where the launch lasts as long as its heaviest item): tiles 2m and 2m + 1 from the start of
-    // the padded tile range and the two tiles that mirror them at its end, so that every item carries the same
-    // work; the early tiles finish their few key steps and wait, the late ones run on with the SM to themselves.
-    auto tile_q0 = [&](int m, int t) {
-        if (!kFold) return (m * kF4Tiles + t) * kBlockM;
-        const int tile = t < 2 ? 2 * m + t : grid.nblk * kF4Tiles - 2 * m - 4 + t;
-        return tile * kBlockM;
-    };
-    auto steps_of = [&](const Item& it, int t) {
-        const int q0 = tile_q0(it.m_block, t);
-        int lim = 0;
-        if (q0 < a.Sq) {
-            lim = it.kvlen;
-            if (a.causal) lim = min(lim, min(q0 + kBlockM - 1, a.Sq - 1) + a.causal_off + 1);
-        }
-        return lim > 0 ? (lim + kBN - 1) / kBN : 0;
-    };
-    auto decode = [&](int linear, Item& it) {
-        int rank;
-        sched_item(grid, linear, rank, it.h, it.b);
-        it.m_block = grid.nblk - 1 - rank;              // heavy (late) causal blocks first
-        it.kvlen = a.Sk;
-        if (a.kv_len) it.kvlen = min(max(a.kv_len[it.b], 0), a.Sk);
-        it.n_max = 0;
-#pragma unroll
-        for (int t = 0; t < kF4Tiles; ++t) it.n_max = max(it.n_max, steps_of(it, t));
-    };
-    auto slot_of = [&](int e) { return e % L::kStages; };
-    auto phase_of = [&](int e) { return (uint32_t)((e / L::kStages) & 1); };
+    int rank, h, b;
+    sched_block(rank, h, b);
+    const int q0 = ((int)gridDim.x - 1 - rank) * kBlockM;          // heavy (late) causal tiles first
+    int kvlen = a.Sk;
+    if (a.kv_len) kvlen = min(max(a.kv_len[b], 0), a.Sk);
+    int lim = kvlen;
+    if (a.causal) lim = min(lim, min(q0 + kBlockM - 1, a.Sq - 1) + a.causal_off + 1);
+    const int n_t = lim > 0 ? (lim + kBN - 1) / kBN : 0;
+    auto slot_of = [](int e) { return e % L::kStages; };
+    auto phase_of = [](int e) { return (uint32_t)((e / L::kStages) & 1); };
 
-    if (warp >= 16) {
-        reg_dealloc<kF4CtrlRegs>();
-        if (warp == 18) {
-            // ------------------------------ TMA producer --------------------------------------
-            if (lane == 0) {
-                tma_prefetch_desc(&tmap_q);
-                tma_prefetch_desc(&tmap_k);
-                tma_prefetch_desc(&tmap_v);
-                bool ok = true;
-                int nq = 0, na = 0, kve = 0;
-                auto load_q = [&](const Item& it, int use) {     // `use`: ordinal among the items that have keys
-                    const int r = use & 1;
-                    if (!mbar_wait(bar_q_empty(r), (uint32_t)(((use >> 1) & 1) ^ 1), wc, 0x11)) return false;
-                    mbar_arrive_expect_tx(bar_q_full(r), (uint32_t)L::kQBufBytes);
-                    for (int t = 0; t < kF4Tiles; ++t)
-                        tma_load_4d(q_smem + r * L::kQBufBytes + t * L::kQTileBytes, &tmap_q, bar_q_full(r), 0,
-                                    tile_q0(it.m_block, t), it.h, it.b);
-                    LTCA_TRACE_EVT(0x31);
-                    return true;
-                };
-                Item cur, nxt;
-                int lin = iq.produce(nq++, grid.counters, grid.n_items, wc);
-                bool cur_q = false;
-                while (ok && lin >= 0) {
-                    decode(lin, cur);
-                    if (cur.n_max > 0 && !cur_q) ok = load_q(cur, na);
-                    // the next item is fetched (a global atomic) towards the end of this item's key stream and
-                    // its Q tiles are loaded under this item's last keys
-                    int lin_next = -1;
-                    bool have_lin_next = false;
-                    bool nxt_q = false;
-                    bool nxt_active = false;
-                    auto fetch_next = [&]() {
-                        lin_next = iq.produce(nq++, grid.counters, grid.n_items, wc);
-                        have_lin_next = true;
-                        if (lin_next == -2) { ok = false; return; }
-                        LTCA_TRACE_EVT(0x32);
-                        if (lin_next >= 0) { decode(lin_next, nxt); nxt_active = nxt.n_max > 0; }
-                    };
-                    if (cur.n_max > 0) {
-                        const int use_next = na + 1;
-                        for (int j = 0; j < cur.n_max && ok; ++j) {
-#pragma unroll
-                            for (int which = 0; which < 2; ++which, ++kve) {     // 0: K_j, 1: V_j
-                                const int slot = slot_of(kve);
-                                ok = ok && mbar_wait(bar_kv_empty(slot), phase_of(kve) ^ 1u, wc, 0x10);
-                                if (!ok) break;
-                                mbar_arrive_expect_tx(bar_kv_full(slot), (uint32_t)L::kKvTileBytes);
-                                tma_load_4d(ring_smem + slot * L::kKvTileBytes, which == 0 ? &tmap_k : &tmap_v,
-                                            bar_kv_full(slot), 0, j * kBN, cur.h, cur.b);
-                            }
-                            LTCA_TRACE_EVT(0x30 + (j << 8));
-                            // (late: an item taken long before it is started is an item that an SM which
-                            // becomes idle earlier can no longer take; two steps before the end of the key stream
-                            // still leaves the consumers' four steps of ring depth to fetch it and load its Q)
-                            if (ok && !have_lin_next && j + 2 >= cur.n_max) fetch_next();
-                            // Q of the next item as soon as its buffer has been released, without
-                            // ever holding up the key stream
-                            if (ok && nxt_active && !nxt_q &&
-                                mbar_try_wait(bar_q_empty(use_next & 1), (uint32_t)(((use_next >> 1) & 1) ^ 1))) {
-                                ok = load_q(nxt, use_next);
-                                nxt_q = true;
-                            }
-                        }
-                        ++na;
-                    }
-                    if (ok && !have_lin_next) fetch_next();
-                    cur_q = nxt_q;
-                    lin = lin_next;
-                }
+    if (warp >= L::kMathWarps) {
+        reg_dealloc<L::kCtrlRegs>();
+        if (warp == kTmaWarp && lane == 0 && n_t > 0) {
+            mbar_arrive_expect_tx(bar_q_full, (uint32_t)L::kQBytes);
+            for (int kb = 0; kb < L::kBlocks; ++kb) tma_load_4d(smem_base + kb * (kBlockM * 128), &tmap_q, bar_q_full, kb * 64, q0, h, b);
+            bool ok = true;
+            for (int e = 0; e < 2 * n_t && ok; ++e) {              // K0 V0 K1 V1 ...
+                const int s = slot_of(e);
+                ok = mbar_wait(bar_kv_empty(s), phase_of(e) ^ 1u, wc, 0x50);
+                if (!ok) break;
+                mbar_arrive_expect_tx(bar_kv_full(s), (uint32_t)L::kKvBytes);
+                for (int kb = 0; kb < L::kBlocks; ++kb)
+                    tma_load_4d(ring + s * L::kKvBytes + kb * (kBN * 128), (e & 1) ? &tmap_v : &tmap_k, bar_kv_full(s), kb * 64,
+                                (e >> 1) * kBN, h, b);
             }
-        } else if (warp == 16 || warp == 17) {
-            // ------------------------------ MMA issuer of tiles 2i, 2i+1 ----------------------
-            const int t0 = 2 * (warp - 16);
-            if (lane == 0) {
-                constexpr uint32_t idesc_qk = make_idesc_bf16(kBlockM, kBN, 0, 0);
-                constexpr uint32_t idesc_pv = make_idesc_bf16(kBlockM, D, 0, 1);
-                const uint64_t q_desc = make_smem_desc_sw128(q_smem, 16, 1024);
-                const uint64_t k_desc = make_smem_desc_sw128(ring_smem, 16, 1024);
-                const uint64_t v_desc = make_smem_desc_sw128(ring_smem, kBN * 128, 1024);
-                auto issue_qk = [&](int t, int slot, int r) {
-                    const uint64_t qd = q_desc + (uint64_t)((r * L::kQBufBytes + t * L::kQTileBytes) >> 4);
-                    const uint64_t kd = k_desc + (uint64_t)((slot * L::kKvTileBytes) >> 4);
+        } else if (warp == kMmaWarp && lane == 0 && n_t > 0) {
+            constexpr uint32_t idesc_qk = make_idesc_bf16(kBlockM, kBN, 0, 0);
+            constexpr uint32_t idesc_pv = make_idesc_bf16(kBlockM, D, 0, 1);
+            const uint32_t q_lo = smem_desc_lo(smem_base, 16), k_lo = smem_desc_lo(ring, 16), v_lo = smem_desc_lo(ring, kBN * 128);
+            auto issue_qk = [&](int s) {
 #pragma unroll
-                    for (int k = 0; k < D / 16; ++k)
-                        mma_ss(tmem_base + t * kBN, qd + 2 * k, kd + 2 * k, idesc_qk, k > 0 ? 1u : 0u);
-                };
-                auto issue_pv = [&](int t, int slot, bool acc) {
-                    const uint64_t vd = v_desc + (uint64_t)((slot * L::kKvTileBytes) >> 4);
+                for (int k = 0; k < D / 16; ++k)
+                    mma_ss_lo(tmem_base, q_lo + (k / 4) * (kBlockM * 8) + (k % 4) * 2,
+                              k_lo + ((s * L::kKvBytes) >> 4) + (k / 4) * (kBN * 8) + (k % 4) * 2, idesc_qk, k > 0 ? 1u : 0u);
+            };
+            bool ok = mbar_wait(bar_q_full, 0, wc, 0x51) && mbar_wait(bar_kv_full(0), 0, wc, 0x52);
+            if (ok) {
+                tc_fence_after_sync();
+                issue_qk(0);
+                mma_commit(bar_s_full);
+                mma_commit(bar_kv_empty(0));
+            }
+            for (int j = 0; j < n_t && ok; ++j) {
+                const int e_v = 2 * j + 1, e_k = 2 * j + 2;
+                const bool more = j + 1 < n_t;
+                ok = mbar_wait(bar_kv_full(slot_of(e_v)), phase_of(e_v), wc, 0x53);
+                if (more) ok = ok && mbar_wait(bar_kv_full(slot_of(e_k)), phase_of(e_k), wc, 0x54);
+                ok = ok && mbar_wait(bar_p_full, (uint32_t)(j & 1), wc, 0x55);
+                if (!ok) break;
+                tc_fence_after_sync();
+                const uint32_t vd = v_lo + ((slot_of(e_v) * L::kKvBytes) >> 4);
+#pragma unroll
+                for (int t = 0; t < (kSplitP ? 2 : 1); ++t)
 #pragma unroll
                     for (int k = 0; k < kBN / 16; ++k)
-                        mma_ts(tmem_base + 256 + t * D, tmem_base + t * kBN + k * 8, vd + 128 * k, idesc_pv,
-                               (acc || k > 0) ? 1u : 0u);
-                };
-                bool ok = true;
-                int na = 0, kve = 0;
-                int uses[2] = {0, 0};       // items in which tile t0 + i had keys
-                int pcnt[2] = {0, 0};       // p_full phases consumed
-                Item it;
-                for (int nq = 0; ok; ++nq) {
-                    const int lin = iq.consume(nq, wc);
-                    if (lin < 0) break;
-                    decode(lin, it);
-                    if (it.n_max == 0) continue;
-                    const int nt0 = steps_of(it, t0), nt1 = steps_of(it, t0 + 1);
-                    const int r = na & 1;
-                    ok = mbar_wait(bar_q_full(r), (uint32_t)((na >> 1) & 1), wc, 0x20);
-                    ok = ok && mbar_wait(bar_kv_full(slot_of(kve)), phase_of(kve), wc, 0x21);
-                    if (!ok) break;
-                    LTCA_TRACE_EVT(0x28);
-                    tc_fence_after_sync();
-#pragma unroll
-                    for (int i = 0; i < 2; ++i) {
-                        const int t = t0 + i;
-                        if (ok && (i == 0 ? nt0 : nt1) > 0) {
-                            // S and O of the tile's previous item must have been read out
-                            if (uses[i] > 0) {
-                                ok = mbar_wait(bar_tile_free(t), (uint32_t)((uses[i] - 1) & 1), wc, 0x2c + t);
-                                if (!ok) break;
-                                tc_fence_after_sync();
-                            }
-                            ++uses[i];
-                            LTCA_TRACE_EVT(0x29 + (i << 8));
-                            issue_qk(t, slot_of(kve), r);
-                            mma_commit(bar_s_full(t));
-                        }
-                    }
-                    if (!ok) break;
-                    mma_commit(bar_kv_empty(slot_of(kve)));
-                    for (int j = 0; j < it.n_max && ok; ++j) {
-                        const int e_v = kve + 2 * j + 1, e_k = kve + 2 * j + 2;
-                        const bool have_next = (j + 1 < it.n_max);
-                        ok = mbar_wait(bar_kv_full(slot_of(e_v)), phase_of(e_v), wc, 0x22);
-                        if (have_next) ok = ok && mbar_wait(bar_kv_full(slot_of(e_k)), phase_of(e_k), wc, 0x23);
-                        LTCA_TRACE_EVT(0x24 + (j << 8));
-#pragma unroll
-                        for (int i = 0; i < 2; ++i) {
-                            const int t = t0 + i;
-                            const int nt = i == 0 ? nt0 : nt1;
-                            if (ok && j < nt) {
-                                ok = mbar_wait(bar_p_full(t), (uint32_t)(pcnt[i] & 1), wc, 0x24 + t);
-                                if (!ok) break;
-                                ++pcnt[i];
-                                LTCA_TRACE_EVT(0x20 + i + (j << 8));
-                                tc_fence_after_sync();
-                                issue_pv(t, slot_of(e_v), j > 0);
-                                if (j + 1 < nt) issue_qk(t, slot_of(e_k), r);
-                                mma_commit(bar_s_full(t));     // S of step j+1 ready, O holds steps 0..j
-                                LTCA_TRACE_EVT(0x22 + i + (j << 8));
-                            }
-                        }
-                        if (!ok) break;
-                        mma_commit(bar_kv_empty(slot_of(e_v)));
-                        if (have_next) mma_commit(bar_kv_empty(slot_of(e_k)));
-                    }
-                    if (!ok) break;
-                    mma_commit(bar_q_empty(r));             // this thread's last read of the item's Q tiles
-                    kve += 2 * it.n_max;
-                    ++na;
-                }
+                        mma_ts_lo(tmem_base + kBN, tmem_base + (kBN / 2) * t + k * 8, vd + 128 * k, idesc_pv,
+                                  (j > 0 || t > 0 || k > 0) ? 1u : 0u);
+                if (more) issue_qk(slot_of(e_k));
+                mma_commit(bar_s_full);                            // S of step j + 1 ready, O holds steps 0 .. j
+                mma_commit(bar_kv_empty(slot_of(e_v)));
+                if (more) mma_commit(bar_kv_empty(slot_of(e_k)));
             }
         }
     } else {
-        // ------------------------------ softmax / correction / epilogue ------------------------
-        reg_alloc<kF4MathRegs>();
-        const int t = warp >> 2;
-        const int wq = warp & 3;
+        reg_alloc<L::kMathRegs>();
+        const int wq = warp & 3, half = kRS > 1 ? warp >> 2 : 0;
         const int row = wq * 32 + lane;
         const uint32_t lane_base = (uint32_t)(wq * 32) << 16;
-        const uint32_t tS = tmem_base + lane_base + t * kBN;
-        const uint32_t tO = tmem_base + lane_base + 256 + t * D;
+        const uint32_t tS = tmem_base + lane_base + half * 64, tO = tmem_base + lane_base + kBN + half * 64;
+        const uint32_t tP = tmem_base + lane_base + half * 32, tPlo = tP + kBN / 2;
+        float* xchg = reinterpret_cast<float*>(smem_gen + L::kXchgOff);
+        auto xslot = [&](int buf, int hf) { return xchg + (buf * 2 + hf) * kBlockM + row; };
+        // the row's other thread has published its value too
+        uint32_t pair_phase = 0;
+        auto meet = [&]() {
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_pair0 + 8u * wq);
+            const bool met = mbar_wait_warp(bar_pair0 + 8u * wq, pair_phase, wc, 0x59);
+            pair_phase ^= 1u;
+            return met;
+        };
         const float c2 = a.scale_log2;
         const bool general = kMask || (a.use_clamp != 0);
-        int scnt = 0;                       // s_full phases consumed
-        int na = 0;                         // items with keys so far (selects the Q buffer)
-        int ecnt = 0;                       // outputs this tile has staged
+        // per row: number of visible keys; per tile: the first step that needs masking at all
+        int lim_row = kvlen, je = n_t;
+        if (a.causal) lim_row = min(lim_row, q0 + row + a.causal_off + 1);
+        if (kvlen % kBN) je = min(je, kvlen / kBN);
+        if (a.causal) {
+            const int v = q0 + a.causal_off - (kBN - 1);           // step j is cut by the diagonal when j * kBN > v
+            je = min(je, v < 0 ? 0 : v / kBN + 1);
+        }
+        float m_run = neg_inf(), l_run = 0.f;
         bool ok = true;
-        Item it;
-        for (int nq = 0; ok; ++nq) {
-            const int lin = iq.consume_warp(nq, wc);
-            if (lin < 0) break;
-            decode(lin, it);
-            const int n_t = steps_of(it, t);
-            const int n_max = it.n_max;
-            const int b_mask = it.b;
-            // per row: number of visible keys; per tile: the first step that needs masking at all
-            int lim_row, je = n_t;
-            {
-                const int q0 = tile_q0(it.m_block, t);
-                lim_row = it.kvlen;
-                if (a.causal) lim_row = min(lim_row, q0 + row + a.causal_off + 1);
-                if (it.kvlen % kBN) je = min(je, it.kvlen / kBN);
-                if (a.causal) {
-                    const int v = q0 + a.causal_off - (kBN - 1);      // step j is cut by the diagonal when j * kBN > v
-                    je = min(je, v < 0 ? 0 : v / kBN + 1);
-                }
-            }
-
-            float m_run = neg_inf();
-            float l_run = 0.f;
-            for (int j = 0; j < n_t; ++j) {
-                uint32_t keep[2];                    // dense mask of this thread's 64 columns
+        for (int j = 0; j < n_t; ++j) {
+            uint32_t keep[2];                                      // dense mask of this thread's 64 columns
 #pragma unroll
-                for (int w = 0; w < 2; ++w)
-                    keep[w] = kMask ? mask_bits_of_queries(a.mask, b_mask, tile_q0(it.m_block, t) + wq * 32, j * kBN + 32 * w) : ~0u;
-                ok = mbar_wait_warp(bar_s_full(t), (uint32_t)(scnt & 1), wc, 0x30 + t);
-                if (!ok) break;
-                ++scnt;
-                LTCA_TRACE_EVT(0x10 + (j << 8));
-                tc_fence_after_sync();
-                uint32_t su[kBN];
-                tmem_ld32(tS, reinterpret_cast<uint32_t(&)[32]>(su[0]));
-                tmem_ld32(tS + 32, reinterpret_cast<uint32_t(&)[32]>(su[32]));
-                tmem_wait_ld();
-                LTCA_TRACE_EVT(0x11 + (j << 8));
-#define S_(c) __uint_as_float(su[(c)])
-                if (general) {
-                    const int k0 = j * kBN;
-                    const int lim = lim_row - k0;           // columns c < lim are visible
-#pragma unroll
-                    for (int c = 0; c < kBN; ++c) {
-                        float v = S_(c);
-                        if (a.use_clamp) v = fminf(v, a.clamp_raw);
-                        const bool vis = c < lim && (keep[c / 32] >> (c % 32) & 1u);
-                        su[c] = __float_as_uint(vis ? v : neg_inf());
-                    }
-                } else if (j >= je) {
-                    // causal diagonal or end of the keys, no dense mask: a select per column, no branches
-                    const int lim = lim_row - j * kBN;
-#pragma unroll
-                    for (int c = 0; c < kBN; ++c) su[c] = (c < lim) ? su[c] : 0xff800000u;
-                }
-                float mx[4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) mx[i] = fmaxf(S_(2 * i), S_(2 * i + 1));
-#pragma unroll
-                for (int c = 8; c < kBN; c += 8)
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) mx[i] = fmax3(mx[i], S_(c + 2 * i), S_(c + 2 * i + 1));
-                const float mt = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
-
-                // Lazy rescale: keep the stale maximum while the new one exceeds it by less than
-                // 2^8 in the exponent; P stays below 256 and fp32 sums keep their accuracy.
-                float factor = 1.0f;
-                bool need = false;
-                if (j == 0) {
-                    m_run = mt;
-                } else if ((mt - m_run) * c2 > 8.0f) {
-                    factor = fast_exp2((m_run - mt) * c2);
-                    m_run = mt;
-                    need = true;
-                }
-                if (j > 0 && __any_sync(0xffffffffu, need)) {
-                    // O already holds every earlier step: the commit behind s_full covered it
-                    // (rare: not unrolled, or its four 16-register pieces push the step's scores out of registers)
-#pragma unroll 1
-                    for (int c0 = 0; c0 < D; c0 += 16) {
-                        uint32_t o[16];
-                        tmem_ld16(tO + c0, o);
-                        tmem_wait_ld();
-#pragma unroll
-                        for (int c = 0; c < 16; ++c) o[c] = __float_as_uint(__uint_as_float(o[c]) * factor);
-                        tmem_st16(tO + c0, o);
-                    }
-                    l_run *= factor;
-                }
-                const float m_safe = (m_run == neg_inf()) ? 0.f : m_run;
-                const float mneg = -m_safe * c2;
-                float sum0 = 0.f, sum1 = 0.f, sum2 = 0.f, sum3 = 0.f;
-#pragma unroll
-                for (int ch = 0; ch < kBN / 32; ++ch) {
-                    uint32_t hi[16];
-#pragma unroll
-                    for (int cc = 0; cc < 32; cc += 4) {
-                        const int c = ch * 32 + cc;
-                        const float p0 = fast_exp2(fmaf(S_(c), c2, mneg));
-                        const float p1 = fast_exp2(fmaf(S_(c + 1), c2, mneg));
-                        const float p2 = fast_exp2(fmaf(S_(c + 2), c2, mneg));
-                        const float p3 = fast_exp2(fmaf(S_(c + 3), c2, mneg));
-                        sum0 += p0; sum1 += p1; sum2 += p2; sum3 += p3;
-                        hi[cc / 2] = pack_bf16x2(p0, p1);
-                        hi[cc / 2 + 1] = pack_bf16x2(p2, p3);
-                    }
-                    tmem_st16(tS + ch * 16, hi);      // P over the first columns of S (all of S is in registers)
-                }
-                l_run += (sum0 + sum1) + (sum2 + sum3);
-                tmem_wait_st();
-                tc_fence_before_sync();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(bar_p_full(t));
-                LTCA_TRACE_EVT(0x12 + (j << 8));
-#undef S_
-            }
+            for (int w = 0; w < 2; ++w)
+                keep[w] = kMask ? mask_bits_of_queries(a.mask, b, q0 + wq * 32, j * kBN + half * 64 + 32 * w) : ~0u;
+            ok = mbar_wait_warp(bar_s_full, (uint32_t)(j & 1), wc, 0x56);
             if (!ok) break;
-
-            // epilogue: O / l and lse; the tile's tensor memory is handed back before the stores
-            decode(lin, it);                    // (re-derived here rather than kept in registers across the key loop)
-            const int b = it.b, h = it.h;
-            const int q0 = tile_q0(it.m_block, t);
-            const int qi = q0 + row;
-            if (it.n_max > 0) {
-                const int r = na & 1;
-                ++na;
-                if (n_t > 0) {
-                    ok = mbar_wait_warp(bar_s_full(t), (uint32_t)(scnt & 1), wc, 0x34 + t);
-                    if (!ok) break;
-                    ++scnt;
-                    LTCA_TRACE_EVT(0x18);
-                    tc_fence_after_sync();
-                    uint32_t o[D];
-                    tmem_ld32(tO, reinterpret_cast<uint32_t(&)[32]>(o[0]));
-                    tmem_ld32(tO + 32, reinterpret_cast<uint32_t(&)[32]>(o[32]));
-                    tmem_wait_ld();
-                    tc_fence_before_sync();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(bar_tile_free(t));
-                    LTCA_TRACE_EVT(0x19);
-                    float inv = 0.f;
-                    float lse = neg_inf();
-                    if (l_run > 0.f) {
-                        inv = 1.0f / l_run;
-                        lse = m_run * a.scale + __logf(l_run);
-                    }
-                    // this row, bf16, into the tile's Q slot in the layout of a 128-byte-swizzled TMA box
-                    uint8_t* stage = smem_gen + r * L::kQBufBytes + t * L::kQTileBytes + row * 128;
+            tc_fence_after_sync();
+            uint32_t su[64];
+            tmem_ld32(tS, reinterpret_cast<uint32_t(&)[32]>(su[0]));
+            tmem_ld32(tS + 32, reinterpret_cast<uint32_t(&)[32]>(su[32]));
+            tmem_wait_ld();
+#define S_(c) __uint_as_float(su[(c)])
+            const int lim_c = lim_row - j * kBN - half * 64;       // own columns c < lim_c are visible
+            if (general) {
 #pragma unroll
-                    for (int v = 0; v < D / 8; ++v) {
-                        uint4 w;
+                for (int c = 0; c < 64; ++c) {
+                    float v = S_(c);
+                    if (a.use_clamp) v = fminf(v, a.clamp_raw);
+                    const bool vis = c < lim_c && (keep[c / 32] >> (c % 32) & 1u);
+                    su[c] = __float_as_uint(vis ? v : neg_inf());
+                }
+            } else if (j >= je) {
+#pragma unroll
+                for (int c = 0; c < 64; ++c) su[c] = (c < lim_c) ? su[c] : 0xff800000u;
+            }
+            float mx[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) mx[i] = fmaxf(S_(2 * i), S_(2 * i + 1));
+#pragma unroll
+            for (int c = 8; c < 64; c += 8)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) mx[i] = fmax3(mx[i], S_(c + 2 * i), S_(c + 2 * i + 1));
+            float mt = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+            if constexpr (kRS > 1) {
+                // (behind this meeting both halves of S are in registers: P may overwrite them)
+                *xslot(j & 1, half) = mt;
+                ok = meet();
+                if (!ok) break;
+                mt = fmaxf(mt, *xslot(j & 1, half ^ 1));
+            }
+            // lazy rescale, as in the kernels above
+            float factor = 1.0f;
+            bool need = false;
+            if (j == 0) {
+                m_run = mt;
+            } else if ((mt - m_run) * c2 > 8.0f) {
+                factor = fast_exp2((m_run - mt) * c2);
+                m_run = mt;
+                need = true;
+            }
+            if (j > 0 && __any_sync(0xffffffffu, need)) {
+#pragma unroll 1
+                for (int c0 = 0; c0 < 64; c0 += 16) {
+                    uint32_t o[16];
+                    tmem_ld16(tO + c0, o);
+                    tmem_wait_ld();
+#pragma unroll
+                    for (int c = 0; c < 16; ++c) o[c] = __float_as_uint(__uint_as_float(o[c]) * factor);
+                    tmem_st16(tO + c0, o);
+                }
+                l_run *= factor;
+            }
+            const float m_safe = (m_run == neg_inf()) ? 0.f : m_run;
+            const float mneg = -m_safe * c2;
+            float sum0 = 0.f, sum1 = 0.f, sum2 = 0.f, sum3 = 0.f;
+#pragma unroll
+            for (int ch = 0; ch < 2; ++ch) {
+                uint32_t hi[16], lo[16];
+#pragma unroll
+                for (int cc = 0; cc < 32; cc += 4) {
+                    const int c = ch * 32 + cc;
+                    const float p0 = fast_exp2(fmaf(S_(c), c2, mneg));
+                    const float p1 = fast_exp2(fmaf(S_(c + 1), c2, mneg));
+                    const float p2 = fast_exp2(fmaf(S_(c + 2), c2, mneg));
+                    const float p3 = fast_exp2(fmaf(S_(c + 3), c2, mneg));
+                    sum0 += p0; sum1 += p1; sum2 += p2; sum3 += p3;
+                    const uint32_t h01 = pack_bf16x2(p0, p1), h23 = pack_bf16x2(p2, p3);
+                    hi[cc / 2] = h01;
+                    hi[cc / 2 + 1] = h23;
+                    if constexpr (kSplitP) {
+                        lo[cc / 2] = pack_bf16x2(p0 - __uint_as_float(h01 << 16), p1 - __uint_as_float(h01 & 0xffff0000u));
+                        lo[cc / 2 + 1] = pack_bf16x2(p2 - __uint_as_float(h23 << 16), p3 - __uint_as_float(h23 & 0xffff0000u));
+                    }
+                }
+                tmem_st16(tP + ch * 16, hi);                       // P over S (all of S is in registers)
+                if constexpr (kSplitP) tmem_st16(tPlo + ch * 16, lo);
+            }
+            l_run += (sum0 + sum1) + (sum2 + sum3);
+            tmem_wait_st();
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_p_full);
+#undef S_
+        }
+        grid_launch_dependents();
+        const int qi = q0 + row;
+        const int64_t stat = ((int64_t)b * a.H + h) * a.Sq + qi;
+        if (n_t > 0) {
+            if constexpr (kRS > 1) {
+                *xslot(2, half) = l_run;
+                ok = ok && meet();
+                if (ok) l_run += *xslot(2, half ^ 1);
+            }
+            ok = ok && mbar_wait_warp(bar_s_full, (uint32_t)(n_t & 1), wc, 0x57);
+            tc_fence_after_sync();
+            uint32_t o[64];
+            if (ok) {
+                tmem_ld32(tO, reinterpret_cast<uint32_t(&)[32]>(o[0]));
+                tmem_ld32(tO + 32, reinterpret_cast<uint32_t(&)[32]>(o[32]));
+                tmem_wait_ld();
+            }
+            float inv = 0.f, lse = neg_inf();
+            if (l_run > 0.f) {
+                inv = 1.0f / l_run;
+                lse = m_run * a.scale + __logf(l_run);
+            }
+            if (ok) {
+                // every operand has been read: Q's slot (and the ring) take the result as 128-byte-swizzled boxes
+#pragma unroll
+                for (int v = 0; v < (kSplitP ? 16 : 8); ++v) {
+                    uint4 w;
+                    if constexpr (kSplitP) {
+                        w = make_uint4(__float_as_uint(__uint_as_float(o[4 * v]) * inv), __float_as_uint(__uint_as_float(o[4 * v + 1]) * inv),
+                                       __float_as_uint(__uint_as_float(o[4 * v + 2]) * inv),
+                                       __float_as_uint(__uint_as_float(o[4 * v + 3]) * inv));
+                    } else {
                         w.x = pack_bf16x2(__uint_as_float(o[8 * v + 0]) * inv, __uint_as_float(o[8 * v + 1]) * inv);
                         w.y = pack_bf16x2(__uint_as_float(o[8 * v + 2]) * inv, __uint_as_float(o[8 * v + 3]) * inv);
                         w.z = pack_bf16x2(__uint_as_float(o[8 * v + 4]) * inv, __uint_as_float(o[8 * v + 5]) * inv);
                         w.w = pack_bf16x2(__uint_as_float(o[8 * v + 6]) * inv, __uint_as_float(o[8 * v + 7]) * inv);
-                        *reinterpret_cast<uint4*>(stage + ((v ^ (row & 7)) << 4)) = w;
                     }
-                    fence_proxy_async_smem();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(bar_staged(t));
-                    if (a.lse && qi < a.Sq) a.lse[((int64_t)b * a.H + h) * a.Sq + qi] = lse;
-                    if (wq == 0 && lane == 0) {
-                        // one thread stores the tile once all four warps have staged their rows
-                        // (rows past the end of the sequence are clipped by the tensor map)
-                        if (mbar_wait(bar_staged(t), (uint32_t)(ecnt & 1), wc, 0x38 + t)) {
-                            tma_store_4d(&tmap_o, q_smem + r * L::kQBufBytes + t * L::kQTileBytes, 0, q0, h, b);
-                            tma_store_commit();
-                            tma_store_wait_read<0>();
-                        }
-                        mbar_arrive(bar_q_empty(r));
-                    }
-                    ++ecnt;
-                } else {
-                    // no key is visible to these rows: zeros and -inf
-                    if (q0 < a.Sq && qi < a.Sq) {
-                        __nv_bfloat16* orow = reinterpret_cast<__nv_bfloat16*>(a.o) + b * a.o_sb + h * a.o_sh +
-                                              (int64_t)qi * a.o_ss;
-                        uint4* dst = reinterpret_cast<uint4*>(orow);
-#pragma unroll
-                        for (int v = 0; v < D / 8; ++v) dst[v] = make_uint4(0u, 0u, 0u, 0u);
-                        if (a.lse) a.lse[((int64_t)b * a.H + h) * a.Sq + qi] = neg_inf();
-                    }
-                    if (wq == 0 && lane == 0) mbar_arrive(bar_q_empty(r));
+                    const int box = half * (kSplitP ? 2 : 1) + v / 8;
+                    *reinterpret_cast<uint4*>(smem_gen + box * (kBlockM * 128) + row * 128 + (((v % 8) ^ (row & 7)) << 4)) = w;
                 }
-            } else if (q0 < a.Sq && qi < a.Sq) {
-                __nv_bfloat16* orow = reinterpret_cast<__nv_bfloat16*>(a.o) + b * a.o_sb + h * a.o_sh +
-                                      (int64_t)qi * a.o_ss;
-                uint4* dst = reinterpret_cast<uint4*>(orow);
-#pragma unroll
-                for (int v = 0; v < D / 8; ++v) dst[v] = make_uint4(0u, 0u, 0u, 0u);
-                if (a.lse) a.lse[((int64_t)b * a.H + h) * a.Sq + qi] = neg_inf();
+                fence_proxy_async_smem();
             }
-            LTCA_TRACE_EVT(0x1a);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_staged);
+            if (half == 0 && a.lse && qi < a.Sq) a.lse[stat] = lse;
+            if (warp == 0 && lane == 0 && ok && mbar_wait(bar_staged, 0, wc, 0x58)) {
+                constexpr int kCols = kSplitP ? 32 : 64;           // of a 128-byte box
+                for (int i = 0; i < D / kCols; ++i) tma_store_4d(&tmap_o, smem_base + i * (kBlockM * 128), i * kCols, q0, h, b);
+                tma_store_commit();
+                tma_store_wait_read<0>();
+            }
+        } else if (qi < a.Sq) {
+            // no key is visible to these rows: zeros and -inf
+            using OutT = typename std::conditional<kSplitP, float, __nv_bfloat16>::type;
+            uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<OutT*>(a.o) + b * a.o_sb + h * a.o_sh + (int64_t)qi * a.o_ss +
+                                                  half * 64);
+#pragma unroll
+            for (int v = 0; v < (kSplitP ? 16 : 8); ++v) dst[v] = make_uint4(0u, 0u, 0u, 0u);
+            if (half == 0 && a.lse) a.lse[stat] = neg_inf();
         }
     }
-
-    // ------------------------------ tear-down -------------------------------------------------
-    // Out of work: only now may the kernel after this one place its CTAs (released at the start, its blocks would
-    // sit beside this kernel's CTAs for the whole run, waiting for it to end).
-    grid_launch_dependents();
     tc_fence_before_sync();
     __syncthreads();
-    if (threadIdx.x == 0) item_counters_release(grid.counters);
-    if (warp == 16) {
+    if (warp == kMmaWarp) {
         __syncwarp();
         if (misc[1]) __nanosleep(200000);    // aborted: give copies and MMAs in flight time to land
         tc_fence_after_sync();
-        tmem_dealloc(tmem_base, kTmemCols);
+        tmem_dealloc(tmem_base, L::kTmemCols);
     }
 }
 
-int launch_fwd4(ltca_ctx* ctx, const ltca_attn_params* p, const void* q, const void* k, const void* v,
-                const ltca_strides& qs, const ltca_strides& ks, const ltca_strides& vs, const FwdArgs& a) {
-    using P = F4PCfg;
+template <int D, bool kSplitP>
+int launch_fwd_tile(ltca_ctx* ctx, const ltca_attn_params* p, const void* q, const void* k, const void* v, const ltca_strides& qs,
+                    const ltca_strides& ks, const ltca_strides& vs, const FwdArgs& a) {
+    using L = TileCfg<D>;
     CUtensorMap tq, tk, tv, to;
     int rc;
-    if ((rc = make_tmap_bhsd(ctx, &tq, q, 2, p->B, p->H, p->Sq, 64, qs, 64, kBlockM))) return rc;
-    if ((rc = make_tmap_bhsd(ctx, &tk, k, 2, p->B, p->H, p->Sk, 64, ks, 64, kF4BN))) return rc;
-    if ((rc = make_tmap_bhsd(ctx, &tv, v, 2, p->B, p->H, p->Sk, 64, vs, 64, kF4BN))) return rc;
-    if ((rc = make_tmap_bhsd(ctx, &to, p->o, 2, p->B, p->H, p->Sq, 64, p->o_strides, 64, kBlockM))) return rc;
-    ItemGrid ig;
-    ig.nblk = (p->Sq + kF4Tiles * kBlockM - 1) / (kF4Tiles * kBlockM);
-    ig.H = p->H;
-    ig.BH = p->B * p->H;
-    ig.n_items = ig.nblk * ig.BH;
-    ig.counters = ctx->d_sched + 6;             // ints 6,7: the forward kernel's item counters
-    // (measured: B=1 H=16 S=4096, the bench workload dealt over eight GPUs: 92 us folded against 123 us)
-    ig.fold = (a.causal && ig.nblk > 1 && ig.n_items <= ctx->sm_count) ? 1 : 0;
-    const int n_cta = ig.n_items < ctx->sm_count ? ig.n_items : ctx->sm_count;
-    static SmemOptIn opt_in[4];
-    auto kern = p->keep_mask ? (ig.fold ? attn_fwd4p_sm100_kernel<true, true> : attn_fwd4p_sm100_kernel<false, true>)
-                             : (ig.fold ? attn_fwd4p_sm100_kernel<true, false> : attn_fwd4p_sm100_kernel<false, false>);
-    LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(opt_in[(p->keep_mask ? 2 : 0) + ig.fold], ctx->device, kern, P::kDynBytes));
-    LTCA_CUDA_OK(ctx, launch_dependent_if(small_attention_call(p), kern, dim3(n_cta), dim3(kF4Threads), P::kDynBytes, ctx->stream, tq, tk,
-                                          tv, to, a, ig));
-    LTCA_LAUNCH_OK(ctx, "attn_fwd4p_sm100_kernel");
+    if ((rc = make_tmap_bhsd(ctx, &tq, q, 2, p->B, p->H, p->Sq, D, qs, 64, kBlockM))) return rc;
+    if ((rc = make_tmap_bhsd(ctx, &tk, k, 2, p->B, p->H, p->Sk, D, ks, 64, L::kBN))) return rc;
+    if ((rc = make_tmap_bhsd(ctx, &tv, v, 2, p->B, p->H, p->Sk, D, vs, 64, L::kBN))) return rc;
+    if ((rc = make_tmap_bhsd(ctx, &to, p->o, kSplitP ? 4 : 2, p->B, p->H, p->Sq, D, p->o_strides, kSplitP ? 32 : 64, kBlockM))) return rc;
+    auto kern = p->keep_mask ? attn_fwd_tile_sm100_kernel<D, kSplitP, true> : attn_fwd_tile_sm100_kernel<D, kSplitP, false>;
+    static SmemOptIn opt_in[2];
+    LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(opt_in[p->keep_mask ? 1 : 0], ctx->device, kern, L::kDynBytes));
+    dim3 grid((p->Sq + kBlockM - 1) / kBlockM, p->H, p->B);
+    LTCA_CUDA_OK(ctx, launch_dependent_if(small_attention_call(p), kern, grid, dim3(L::kThreads), L::kDynBytes, ctx->stream, tq, tk, tv, to, a));
     return LTCA_OK;
 }
 
@@ -1092,13 +892,6 @@ int launch_fwd(ltca_ctx* ctx, const ltca_attn_params* p, const void* mask_words,
                const void* v, const ltca_strides& qs, const ltca_strides& ks,
                const ltca_strides& vs) {
     constexpr bool kSplitP = sizeof(OutT) == 4;
-    using L = FwdCfg<D, kSplitP>;
-    CUtensorMap tq, tk, tv;
-    int rc;
-    if ((rc = make_tmap_bhsd(ctx, &tq, q, 2, p->B, p->H, p->Sq, D, qs, 64, kBlockM))) return rc;
-    if ((rc = make_tmap_bhsd(ctx, &tk, k, 2, p->B, p->H, p->Sk, D, ks, 64, L::kBN))) return rc;
-    if ((rc = make_tmap_bhsd(ctx, &tv, v, 2, p->B, p->H, p->Sk, D, vs, 64, L::kBN))) return rc;
-
     FwdArgs a;
     a.B = p->B; a.H = p->H; a.Sq = p->Sq; a.Sk = p->Sk;
     a.causal = p->causal ? 1 : 0;
@@ -1114,32 +907,32 @@ int launch_fwd(ltca_ctx* ctx, const ltca_attn_params* p, const void* mask_words,
     a.kv_len = p->kv_len;
     a.status = ctx->d_status;
 
-    if constexpr (D == 64 && sizeof(OutT) == 2) {
-        // long query ranges: four independent tiles per CTA (see attn_fwd4p_sm100_kernel)
-        // ... unless its work items (512 queries of one batch entry and head) leave SMs idle where the CTAs of the
-        // two-tile kernel (256 queries) would fill them: B=4 H=16 Sq=512 Sk=4096 takes 129 us on 64 of 148 SMs
-        // against 75 us on 128, B=1 H=8 S=4096 causal 92 against 70 us.  Per tile the four-tile kernel is the
-        // faster one (16 pairs of S=4096, causal: 99 against 112 us), so it keeps the case unless the other fills
-        // the SMs a quarter better.  The device's SM count decides, not a limit set on the context: the choice,
-        // and with it the bits of the result, does not move with the launch width.
-        bool four = p->Sq > kFwd4MinSq;
-        const int64_t bh = (int64_t)p->B * p->H;
-        const int64_t items4 = bh * ((p->Sq + 4 * kBlockM - 1) / (4 * kBlockM));
-        const int64_t sms = ctx->sm_device > 0 ? ctx->sm_device : kPlanSms;
-        if (four && items4 < sms) {
-            const int64_t ctas2 = bh * ((p->Sq + 2 * kBlockM - 1) / (2 * kBlockM));
-            const int64_t waves2 = (ctas2 + sms - 1) / sms;
-            four = (double)ctas2 / (double)(waves2 * sms) < 1.25 * (double)items4 / (double)sms;
-        }
-        if (four) return launch_fwd4(ctx, p, q, k, v, qs, ks, vs, a);
-    }
+    // The one-tile kernel, except where head_dim is 64 and the call has so few tiles that two-tile CTAs run in one wave and
+    // keys enough that a tile's own step time decides: there two threads per row shorten the step (B=1 H=8 S=4096 causal
+    // 60 us against 65, B=4 H=16 Sq=512 Sk=4096 64 against 78; at S=512 the one-tile kernel is the faster one again, 11.2
+    // against 12.0 for B=4 H=8).  The device's SM count decides, not a limit set on the context: the choice, and with it
+    // the bits of the result, does not move with the launch width.
+    const int64_t ctas2 = (int64_t)p->B * p->H * ((p->Sq + 2 * kBlockM - 1) / (2 * kBlockM));
+    const int64_t sms = ctx->sm_device > 0 ? ctx->sm_device : kPlanSms;
+    // Where the caller asks for the two-tile kernel's order of additions (ctx->fwd_pairs), short queries keep it too.
+    const bool few = ctas2 <= sms && p->Sk > 512;
+    const bool ordered = ctx->fwd_pairs && (ctas2 <= sms || p->Sq <= 2 * kBlockM);
+    if (D != 64 || !(few || ordered)) return launch_fwd_tile<D, kSplitP>(ctx, p, q, k, v, qs, ks, vs, a);
 
-    auto kern = p->keep_mask ? attn_fwd_sm100_kernel<D, OutT, kSplitP, true> : attn_fwd_sm100_kernel<D, OutT, kSplitP, false>;
-    static SmemOptIn opt_in[2];               // one pair per template instantiation
-    LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(opt_in[p->keep_mask ? 1 : 0], ctx->device, kern, L::kDynBytes));
-    dim3 grid((p->Sq + 2 * kBlockM - 1) / (2 * kBlockM), p->H, p->B);
-    LTCA_CUDA_OK(ctx, launch_dependent(kern, grid, dim3(kFwdThreads), L::kDynBytes, ctx->stream, tq, tk, tv, a));
-    LTCA_LAUNCH_OK(ctx, "attn_fwd_sm100_kernel");
+    if constexpr (D == 64) {
+        using L = FwdCfg<D, kSplitP>;
+        CUtensorMap tq, tk, tv;
+        int rc;
+        if ((rc = make_tmap_bhsd(ctx, &tq, q, 2, p->B, p->H, p->Sq, D, qs, 64, kBlockM))) return rc;
+        if ((rc = make_tmap_bhsd(ctx, &tk, k, 2, p->B, p->H, p->Sk, D, ks, 64, L::kBN))) return rc;
+        if ((rc = make_tmap_bhsd(ctx, &tv, v, 2, p->B, p->H, p->Sk, D, vs, 64, L::kBN))) return rc;
+        auto kern = p->keep_mask ? attn_fwd_sm100_kernel<D, OutT, kSplitP, true> : attn_fwd_sm100_kernel<D, OutT, kSplitP, false>;
+        static SmemOptIn opt_in[2];               // one pair per template instantiation
+        LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(opt_in[p->keep_mask ? 1 : 0], ctx->device, kern, L::kDynBytes));
+        dim3 grid((p->Sq + 2 * kBlockM - 1) / (2 * kBlockM), p->H, p->B);
+        LTCA_CUDA_OK(ctx, launch_dependent(kern, grid, dim3(kFwdThreads), L::kDynBytes, ctx->stream, tq, tk, tv, a));
+        LTCA_LAUNCH_OK(ctx, "attn_fwd_sm100_kernel");
+    }
     return LTCA_OK;
 }
 

@@ -27,6 +27,10 @@ struct ltca_ctx {
     // A module call's packed mask (attn_mask.cuh): set while the call launches its attention kernels, which all read it.
     const float* mask_packed = nullptr;
     const void* mask_words = nullptr;
+    // Set while the FlashAttention form's backward recomputes its forward: the gradient of the key bias is zero but for the
+    // rounding of that forward (a shift of all keys does not move a softmax), so every digit of it follows the order in
+    // which one kernel adds; short calls then stay with the two-tile kernel (launch_fwd, attn_fwd_sm100.cu).
+    bool fwd_pairs = false;
     char err[512] = {0};
     // optional per-kernel timing of the backward pass (ltca_ctx_enable_kernel_timing)
     bool time_kernels = false;

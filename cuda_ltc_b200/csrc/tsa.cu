@@ -895,10 +895,11 @@ int tensor_backward(ltca_ctx* ctx, const ltca_tsa_params* t, bool want_dx, bool 
     // the forward is recomputed, as the reference's caller does before each backward
     // (src/ml/ml_liquid_net.cu:715-721)
     // the recomputed attention and its backward read the same mask: packed once, behind what either uses of the scratch
-    struct PackedMask {
+    struct Hints {
         ltca_ctx* ctx;
-        ~PackedMask() { ctx->mask_packed = nullptr; ctx->mask_words = nullptr; }
-    } packed{ctx};
+        ~Hints() { ctx->mask_packed = nullptr; ctx->mask_words = nullptr; ctx->fwd_pairs = false; }
+    } hints{ctx};
+    ctx->fwd_pairs = t->bk != nullptr;
     if (t->keep_mask && !pl.wide) {
         ltca_attn_params a;
         fill_attn_bf16(t, &a);
