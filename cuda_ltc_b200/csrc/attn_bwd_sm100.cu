@@ -77,6 +77,7 @@ struct StatsArgs {
     const float* lse;
     float *lse2, *delta;
     float* dq_acc;           // optional: fp32 [B*H, Sq_pad, 64] accumulator of the fused kernel, cleared here
+    uint4* dout_bf16;        // fp32 storage: dO rounded to bf16, [B*H, Sq, 64], for the contractions
 };
 
 __device__ __forceinline__ void load8(const __nv_bfloat16* p, float (&f)[8]) {
@@ -95,17 +96,18 @@ __device__ __forceinline__ void load8(const float* p, float (&f)[8]) {
     f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
 }
 
+// Bound by memory (o and dO are read once).  A block takes kStatsRows consecutive rows of one (batch, head) pair (Sq_pad
+// is a multiple of 256), so the pair comes from two 32-bit divisions by block; with a row's place from 64-bit ones per
+// thread 134 MB each of o and dO took 44 us, 38 so.  More rows per thread were slower (64 rows a block 43 us, 128 54).
+constexpr int kStatsRows = 32;
 template <typename T>
-__global__ void __launch_bounds__(256) attn_bwd_stats_kernel(const StatsArgs a) {
+__global__ void __launch_bounds__(8 * kStatsRows) attn_bwd_stats_kernel(const StatsArgs a) {
     grid_launch_dependents();
     grid_dependency_wait();
-    const int64_t row = (int64_t)blockIdx.x * 32 + (threadIdx.x >> 3);
-    const int sub = threadIdx.x & 7;
-    const int64_t total = (int64_t)a.B * a.H * a.Sq_pad;
-    if (row >= total) return;                    // whole 8-lane groups leave together
-    const int qi = (int)(row % a.Sq_pad);
-    const int64_t bh = row / a.Sq_pad;
-    const int h = (int)(bh % a.H), b = (int)(bh / a.H);
+    const unsigned per_pair = (unsigned)a.Sq_pad / kStatsRows, bh = blockIdx.x / per_pair;
+    const unsigned b = bh / (unsigned)a.H, h = bh - b * (unsigned)a.H;
+    const int qi = (int)(blockIdx.x - bh * per_pair) * kStatsRows + (threadIdx.x >> 3), sub = threadIdx.x & 7;
+    const int64_t row = (int64_t)bh * a.Sq_pad + qi;
     if (a.dq_acc) {
         float4* z = reinterpret_cast<float4*>(a.dq_acc + row * kD + 8 * sub);
         z[0] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -121,8 +123,14 @@ __global__ void __launch_bounds__(256) attn_bwd_stats_kernel(const StatsArgs a) 
         // fp32 storage: the contractions see dO rounded to bf16, and sum_j P_ij dP_ij equals
         // delta_i only when delta is formed from the same rounded dO
         if constexpr (sizeof(T) == 4) {
+            uint32_t w[4];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) fg[i] = __bfloat162float(__float2bfloat16_rn(fg[i]));
+            for (int i = 0; i < 4; ++i) {
+                w[i] = pack_bf16x2(fg[2 * i], fg[2 * i + 1]);
+                fg[2 * i] = __uint_as_float(w[i] << 16);
+                fg[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+            }
+            a.dout_bf16[((int64_t)bh * a.Sq + qi) * 8 + sub] = make_uint4(w[0], w[1], w[2], w[3]);
         }
 #pragma unroll
         for (int i = 0; i < 8; ++i) acc = fmaf(fo[i], fg[i], acc);
@@ -133,7 +141,7 @@ __global__ void __launch_bounds__(256) attn_bwd_stats_kernel(const StatsArgs a) 
     if (sub == 0) {
         float l2 = pos_inf();
         if (qi < a.Sq) {
-            const float l = a.lse[bh * a.Sq + qi];
+            const float l = a.lse[(int64_t)bh * a.Sq + qi];
             l2 = (l == neg_inf()) ? pos_inf() : l * 1.4426950408889634f;
         }
         a.lse2[row] = l2;
@@ -2467,13 +2475,15 @@ int launch_attn_bwd_sm100(ltca_ctx* ctx, const ltca_attn_params* p) {
     s.B = p->B; s.H = p->H; s.Sq = p->Sq; s.Sq_pad = (int)align_up((size_t)p->Sq, 256);
     s.o = p->o; s.dout = p->dout; s.os = p->o_strides; s.dos = p->do_strides;
     s.lse = p->lse; s.lse2 = lse2; s.delta = delta; s.dq_acc = dq_acc;
-    const int64_t rows = (int64_t)p->B * p->H * s.Sq_pad;
-    const unsigned blocks = (unsigned)((rows + 31) / 32);
+    // fp32 storage: bf16 copies of the four operands (dO's comes with the statistics), fp32 gradients out
+    void *qb = w, *kb = w + pq, *vb = w + pq + pk, *gb = w + pq + 2 * pk;
+    s.dout_bf16 = reinterpret_cast<uint4*>(gb);
+    const unsigned blocks = (unsigned)((int64_t)p->B * p->H * (s.Sq_pad / kStatsRows));
     kernel_timing_mark(ctx, 0);
     if (p->dtype == LTCA_BF16)
-        LTCA_CUDA_OK(ctx, launch_dependent_if(small_attention_call(p), attn_bwd_stats_kernel<__nv_bfloat16>, dim3(blocks), dim3(256), 0, ctx->stream, s));
+        LTCA_CUDA_OK(ctx, launch_dependent_if(small_attention_call(p), attn_bwd_stats_kernel<__nv_bfloat16>, dim3(blocks), dim3(8 * kStatsRows), 0, ctx->stream, s));
     else
-        LTCA_CUDA_OK(ctx, launch_dependent_if(small_attention_call(p), attn_bwd_stats_kernel<float>, dim3(blocks), dim3(256), 0, ctx->stream, s));
+        LTCA_CUDA_OK(ctx, launch_dependent_if(small_attention_call(p), attn_bwd_stats_kernel<float>, dim3(blocks), dim3(8 * kStatsRows), 0, ctx->stream, s));
     LTCA_LAUNCH_OK(ctx, "attn_bwd_stats_kernel");
     if (p->dtype == LTCA_BF16) kernel_timing_mark(ctx, 1);
 
@@ -2481,14 +2491,8 @@ int launch_attn_bwd_sm100(ltca_ctx* ctx, const ltca_attn_params* p) {
         return (p->keep_mask ? launch_main<__nv_bfloat16, true> : launch_main<__nv_bfloat16, false>)(
             ctx, p, words, p->q, p->k, p->v, p->dout, p->q_strides, p->k_strides, p->v_strides, p->do_strides, lse2, delta, dq_acc);
 
-    // fp32 storage: bf16 copies of the four operands, fp32 gradients out
-    void* qb = w;  w += pq;
-    void* kb = w;  w += pk;
-    void* vb = w;  w += pk;
-    void* gb = w;
-    const PackJob jobs[4] = {{p->q, p->q_strides, qb, p->Sq}, {p->k, p->k_strides, kb, p->Sk},
-                             {p->v, p->v_strides, vb, p->Sk}, {p->dout, p->do_strides, gb, p->Sq}};
-    if (int rc = pack_many_to_bf16(ctx, jobs, 4, p->B, p->H, kD)) return rc;
+    const PackJob jobs[3] = {{p->q, p->q_strides, qb, p->Sq}, {p->k, p->k_strides, kb, p->Sk}, {p->v, p->v_strides, vb, p->Sk}};
+    if (int rc = pack_many_to_bf16(ctx, jobs, 3, p->B, p->H, kD)) return rc;
     kernel_timing_mark(ctx, 1);
     ltca_strides cq{(int64_t)p->H * p->Sq * kD, (int64_t)p->Sq * kD, kD};
     ltca_strides ck{(int64_t)p->H * p->Sk * kD, (int64_t)p->Sk * kD, kD};

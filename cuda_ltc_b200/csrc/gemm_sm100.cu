@@ -482,11 +482,16 @@ __global__ void cvt_rows_bf16_kernel(const float* __restrict__ src, int64_t ld_s
     }
 }
 
+constexpr int kCvtBatch = 4;                   // loads in flight per thread (67 MB to 34: 16.6 us with one, 15.9 so)
 __global__ void cvt_rows_bf16_vec_kernel(const float4* __restrict__ src, uint2* __restrict__ dst, int64_t n4) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (int64_t)gridDim.x * blockDim.x) {
-        const float4 v = __ldg(src + i);
-        dst[i] = make_uint2(pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w));
-    }
+    const int64_t first = (int64_t)blockIdx.x * (kCvtBatch * 256) + threadIdx.x;
+    float4 v[kCvtBatch];
+#pragma unroll
+    for (int e = 0; e < kCvtBatch; ++e)
+        if (first + e * 256 < n4) v[e] = __ldg(src + first + e * 256);
+#pragma unroll
+    for (int e = 0; e < kCvtBatch; ++e)
+        if (first + e * 256 < n4) dst[first + e * 256] = make_uint2(pack_bf16x2(v[e].x, v[e].y), pack_bf16x2(v[e].z, v[e].w));
 }
 
 // Several matrices of any sizes in ONE launch (the activations and the weights of a module call).
@@ -617,7 +622,7 @@ int convert_rows_bf16(ltca_ctx* ctx, const float* src, int64_t ld_src, void* dst
     if (ld_src == cols && ld_dst == cols && (n & 3) == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0 &&
         (reinterpret_cast<uintptr_t>(dst) & 7) == 0) {
         const int64_t n4 = n / 4;
-        const unsigned blocks = (unsigned)((n4 + 255) / 256 < 2368 ? (n4 + 255) / 256 : 2368);
+        const unsigned blocks = (unsigned)((n4 + kCvtBatch * 256 - 1) / (kCvtBatch * 256));
         cvt_rows_bf16_vec_kernel<<<blocks, 256, 0, ctx->stream>>>(reinterpret_cast<const float4*>(src),
                                                                   reinterpret_cast<uint2*>(dst), n4);
     } else {
