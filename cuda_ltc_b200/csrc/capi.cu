@@ -108,6 +108,7 @@ __device__ __forceinline__ float4 rest4(const float4& v, const uint2& r) {
 constexpr int kPackChunks = 4;
 template <int kVec>
 __global__ void __launch_bounds__(256) pack_bf16_kernel(const __grid_constant__ PackJobs jobs, int BH, int H, int D) {
+    if (gridDim.x * gridDim.y <= kPlanSms) grid_launch_dependents();   // a block per SM at most: nothing to crowd out
     grid_dependency_wait();
     const int j = blockIdx.y;
     const float* __restrict__ src = jobs.src[j];

@@ -14,15 +14,17 @@
 // so no operand is ever transposed in memory: the instruction descriptor's major bits select the
 // form and the shared-memory descriptors follow the layout the TMA boxes produce.
 //
-// Persistent CTAs (one per SM) walk a list of 128 x 256 tiles of C: warp 0 is the TMA producer (ring of four
-// 48 KB (A, B) stages), warp 1 issues the MMAs (M128 N256 K16) into one of two 256-column accumulators in tensor
-// memory, warps 2-5 are the epilogue (one accumulator row per thread: tcgen05.ld, bias, convert; the tile is
-// staged in shared memory as 128-byte-swizzled boxes and stored with TMA), which works on tile i while the MMAs
-// of tile i+1 run.  Measured at the module's sizes (device time line of one CTA): a ring stage of 48 KB arrives
+// Persistent CTAs (one per SM) walk a list of tiles of C: warp 0 is the TMA producer (ring of (A, B) stages of 64 K
+// values), warp 1 issues the MMAs (K16 steps) into one of two accumulators in tensor memory, warps 2-5 are the epilogue
+// (one accumulator row per thread: tcgen05.ld, bias, convert; the tile is staged in shared memory as 128-byte-swizzled
+// boxes and stored with TMA), which works on tile i while the MMAs of tile i+1 run.  Tiles are 128 x 256 (four stages of
+// 48 KB), 128 x 128 (six of 32 KB) or, for two CTAs of a cluster, 256 x 256 (six of 32 KB: each CTA holds its 128 rows of A
+// and half the columns of B); pick_tile says which.  Measured at the module's sizes: a ring stage of 48 KB arrives
 // every 600 - 700 cycles (about 80 bytes per cycle and SM from L2: every 128-row block of A is re-read once per
-// N tile and every weight matrix once per M tile) against 512 cycles of MMAs, which is why the tile is 256 wide;
-// the epilogue of a tile takes 4700 cycles (bf16) to 7200 (fp32) and is hidden behind the next tile's main loop
-// except for the last tile of a CTA.
+// N tile and every weight matrix once per M tile) against 512 cycles of MMAs; the epilogue of a tile takes 4700 cycles
+// (bf16) to 7200 (fp32) and is hidden behind the next tile's main loop except for the last tile of a CTA.  Without any
+// epilogue M=32768, N=3 x 512, K=512 takes 41 of 51 us, without its stores 47; eight epilogue warps, stores of 32 bytes
+// per thread straight from registers and stores of whole lines through shared memory all took as long or longer.
 // The tile list runs over independent problems (Q, K and V projections share one launch) and/or splits of K
 // (weight gradients: K = batch x time is long and M x N is small, so the K range is cut into
 // slices whose partial tiles go to scratch and are summed in a fixed order by a second kernel).
@@ -40,11 +42,8 @@ namespace ltca {
 
 namespace {
 
-constexpr int kBM = 128, kBN = 256, kBK = 64;
-constexpr int kStages = 4;                         // operand ring: 4 x (16 KB of A + 32 KB of B)
+constexpr int kBM = 128, kBK = 64;                 // rows of A per CTA, contraction per ring stage
 constexpr int kATileBytes = kBM * kBK * 2;         // 16 KB
-constexpr int kBTileBytes = kBN * kBK * 2;         // 32 KB
-constexpr int kStageBytes = kATileBytes + kBTileBytes;
 // The result tile leaves through two staging boxes of 128 rows x 128 bytes (64 bf16 or 32 fp32 columns) that
 // alternate.  A tiled TMA store reads shared memory at 32 bytes per cycle (513 cycles per box, measured with one
 // and with 148 CTAs storing, whatever the number of stores in flight), so a second pair of boxes buys nothing,
@@ -52,14 +51,21 @@ constexpr int kStageBytes = kATileBytes + kBTileBytes;
 constexpr int kStageBoxes = 2;
 constexpr int kStageOutBytes = kBM * 128 * kStageBoxes;
 constexpr int kGemmThreads = 192;
-constexpr int kOutOff = kStages * kStageBytes;
-constexpr int kBarOff = kOutOff + kStageOutBytes;
-constexpr int kNumBars = 2 * kStages + 4;          // full[S], empty[S], acc_full[2], acc_empty[2]
-constexpr int kMiscOff = kBarOff + kNumBars * 8;
-constexpr int kBiasOff = kMiscOff + 16;            // this tile's kBN bias values
-constexpr int kDynBytes = kBiasOff + kBN * 4 + 1024;
-static_assert(kDynBytes <= 227 * 1024, "shared memory");
-constexpr uint32_t kAccCols = 2 * kBN;             // two accumulators
+template <int kBN, bool kPair>
+struct GemmCfg {
+    static constexpr int kTileM = kPair ? 2 * kBM : kBM;           // rows of C per work item
+    static constexpr int kBRows = kPair ? kBN / 2 : kBN;           // columns of the tile whose B this CTA holds
+    static constexpr int kStageBytes = kATileBytes + kBRows * kBK * 2;
+    static constexpr int kStages = kStageBytes > 32768 ? 4 : 6;    // operand ring
+    static constexpr int kOutOff = kStages * kStageBytes;
+    static constexpr int kBarOff = kOutOff + kStageOutBytes;
+    static constexpr int kNumBars = 2 * kStages + 4;               // full[S], empty[S], acc_full[2], acc_empty[2]
+    static constexpr int kMiscOff = kBarOff + kNumBars * 8;
+    static constexpr int kBiasOff = kMiscOff + 16;                 // this tile's kBN bias values
+    static constexpr int kDynBytes = kBiasOff + kBN * 4 + 1024;
+    static_assert(kDynBytes <= 227 * 1024, "shared memory");
+    static constexpr uint32_t kAccCols = 2 * kBN;                  // two accumulators
+};
 
 struct GemmKArgs {
     int M, N, K;
@@ -82,7 +88,8 @@ struct GemmTile {
     int m0, n0, problem, slice, kb_begin, kb_end, pair_begin, n_pairs, n_iters;
     int bh, bb;                      // batch entry
 };
-__device__ __forceinline__ GemmTile gemm_tile(const GemmKArgs& g, int linear) {
+template <int kBN, int kTileM>
+__device__ __forceinline__ GemmTile gemm_tile(const GemmKArgs& g, int linear, int rank) {
     GemmTile t;
     const int x = linear % g.tiles_x;
     const int yz = linear / g.tiles_x;
@@ -91,7 +98,7 @@ __device__ __forceinline__ GemmTile gemm_tile(const GemmKArgs& g, int linear) {
     t.bh = w % g.batch_h;
     t.bb = w / g.batch_h;
     t.n0 = x * kBN;
-    t.m0 = y * kBM;
+    t.m0 = y * kTileM + rank * kBM;
     t.problem = z / g.ksplit;
     t.slice = z % g.ksplit;
     const int nkb = (g.K + kBK - 1) / kBK;
@@ -104,43 +111,50 @@ __device__ __forceinline__ GemmTile gemm_tile(const GemmKArgs& g, int linear) {
     return t;
 }
 
-// Persistent: CTA c computes tiles c, c + gridDim.x, ... of the list (N tiles fastest, so neighbouring CTAs
+// Persistent: CTA (or pair) c computes tiles c, c + their number, ... of the list (N tiles fastest, so neighbouring CTAs
 // share their rows of A in L2).  The two accumulators alternate: while the epilogue warps read tile i out of
 // tensor memory, convert it and hand it to the TMA store, the MMA thread is already accumulating tile i+1 and
 // the producer is loading tile i+2's operands.
-template <bool kAMn, bool kBMn>
+template <bool kAMn, bool kBMn, int kBN, bool kPair>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CUtensorMap ta1,
                        const __grid_constant__ CUtensorMap ta2, const __grid_constant__ CUtensorMap tb0,
                        const __grid_constant__ CUtensorMap tb1, const __grid_constant__ CUtensorMap tb2,
                        const __grid_constant__ CUtensorMap tc0, const __grid_constant__ CUtensorMap tc1,
                        const __grid_constant__ CUtensorMap tc2, const GemmKArgs g) {
+    using L = GemmCfg<kBN, kPair>;
+    constexpr int kStages = L::kStages, kStageBytes = L::kStageBytes;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
-    const uint32_t bar_base = smem_base + kBarOff;
+    const uint32_t bar_base = smem_base + L::kBarOff;
     auto a_smem = [&](int s) { return smem_base + (uint32_t)(s * kStageBytes); };
     auto b_smem = [&](int s) { return smem_base + (uint32_t)(s * kStageBytes + kATileBytes); };
     auto bar_full = [&](int s) { return bar_base + 8u * s; };
     auto bar_empty = [&](int s) { return bar_base + 8u * (kStages + s); };
     auto bar_acc_full = [&](int b) { return bar_base + 8u * (2 * kStages + b); };
     auto bar_acc_empty = [&](int b) { return bar_base + 8u * (2 * kStages + 2 + b); };
-    volatile uint32_t* misc = reinterpret_cast<volatile uint32_t*>(smem_gen + kMiscOff);
+    volatile uint32_t* misc = reinterpret_cast<volatile uint32_t*>(smem_gen + L::kMiscOff);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n_tiles = g.tiles_x * g.tiles_y * g.tiles_z * g.batch_h * g.batch_b;
+    const int rank = kPair ? (int)cluster_rank() : 0;             // rank 0 issues the pair's MMAs
     LTCA_TRACE_DECL(blockIdx.x == 5 && g.tiles_z == LTCA_TRACE_GEMM_Z);
     LTCA_TRACE_EVT(0x01);
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) { mbar_init(bar_full(s), 1); mbar_init(bar_empty(s), 1); }
-        for (int b = 0; b < 2; ++b) { mbar_init(bar_acc_full(b), 1); mbar_init(bar_acc_empty(b), 4); }
+        for (int b = 0; b < 2; ++b) { mbar_init(bar_acc_full(b), 1); mbar_init(bar_acc_empty(b), kPair ? 8 : 4); }
         misc[1] = 0u;
         mbar_fence_init();
     }
-    if (warp == 1) { tmem_alloc(smem_u32(const_cast<uint32_t*>(&misc[0])), kAccCols); tmem_relinquish(); }
+    if (warp == 1) {
+        if constexpr (kPair) { tmem_alloc_pair(smem_u32(const_cast<uint32_t*>(&misc[0])), L::kAccCols); tmem_relinquish_pair(); }
+        else { tmem_alloc(smem_u32(const_cast<uint32_t*>(&misc[0])), L::kAccCols); tmem_relinquish(); }
+    }
     tc_fence_before_sync();
     __syncthreads();
+    if constexpr (kPair) cluster_sync();                          // the other CTA's barriers may be signalled
     tc_fence_after_sync();
     const uint32_t tmem_base = misc[0];
     const WaitCtx wc{&misc[1], g.status};
@@ -156,8 +170,8 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_con
             tma_prefetch_desc(&tb0);
             bool ok = true;
             int it = 0;
-            for (int lin = blockIdx.x; lin < n_tiles && ok; lin += gridDim.x) {
-                const GemmTile t = gemm_tile(g, lin);
+            for (int lin = kPair ? blockIdx.x >> 1 : blockIdx.x; lin < n_tiles && ok; lin += kPair ? gridDim.x >> 1 : gridDim.x) {
+                const GemmTile t = gemm_tile<kBN, L::kTileM>(g, lin, rank);
                 for (int p = 0; p < t.n_pairs && ok; ++p) {
                     const int pair = t.pair_begin + p;
                     const CUtensorMap* ta = pair == 0 ? &ta0 : (pair == 1 ? &ta1 : &ta2);
@@ -167,30 +181,36 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_con
                         ok = mbar_wait(bar_empty(s), (uint32_t)(((it / kStages) & 1) ^ 1), wc, 0xd0);
                         if (!ok) break;
                         LTCA_TRACE_EVT(0x10 + (it << 8));
-                        mbar_arrive_expect_tx(bar_full(s), (uint32_t)kStageBytes);
-                        const int k0 = kb * kBK;
+                        // a pair's loads all signal the issuing CTA's barrier
+                        if (rank == 0) mbar_arrive_expect_tx(bar_full(s), (uint32_t)(kPair ? 2 : 1) * kStageBytes);
+                        const uint32_t bar = kPair ? map_shared(bar_full(s), 0) : bar_full(s);
+                        auto load = [&](uint32_t dst, const CUtensorMap* map, int c0, int c1) {
+                            if constexpr (kPair) tma_load_4d_pair(dst, map, bar, c0, c1, t.bh, t.bb);
+                            else tma_load_4d(dst, map, bar, c0, c1, t.bh, t.bb);
+                        };
+                        const int k0 = kb * kBK, n0 = t.n0 + rank * L::kBRows;
                         if (kAMn) {
-                            tma_load_4d(a_smem(s), ta, bar_full(s), t.m0, k0, t.bh, t.bb);
-                            tma_load_4d(a_smem(s) + 8192, ta, bar_full(s), t.m0 + 64, k0, t.bh, t.bb);
+                            load(a_smem(s), ta, t.m0, k0);
+                            load(a_smem(s) + 8192, ta, t.m0 + 64, k0);
                         } else {
-                            tma_load_4d(a_smem(s), ta, bar_full(s), k0, t.m0, t.bh, t.bb);
+                            load(a_smem(s), ta, k0, t.m0);
                         }
                         if (kBMn) {
 #pragma unroll
-                            for (int pn = 0; pn < kBN / 64; ++pn)     // 64-column blocks of 64 K rows, 8 KB each
-                                tma_load_4d(b_smem(s) + pn * 8192, tb, bar_full(s), t.n0 + 64 * pn, k0, t.bh, t.bb);
+                            for (int pn = 0; pn < L::kBRows / 64; ++pn)     // 64-column blocks of 64 K rows, 8 KB each
+                                load(b_smem(s) + pn * 8192, tb, n0 + 64 * pn, k0);
                         } else {
-                            // 256 rows of 128 bytes, as two boxes of 128 rows
-                            tma_load_4d(b_smem(s), tb, bar_full(s), k0, t.n0, t.bh, t.bb);
-                            tma_load_4d(b_smem(s) + kBTileBytes / 2, tb, bar_full(s), k0, t.n0 + 128, t.bh, t.bb);
+#pragma unroll
+                            for (int pn = 0; pn < L::kBRows / 128; ++pn)    // boxes of 128 rows of 128 bytes
+                                load(b_smem(s) + pn * 16384, tb, k0, n0 + 128 * pn);
                         }
                     }
                 }
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            constexpr uint32_t idesc = make_idesc_bf16(kBM, kBN, kAMn ? 1 : 0, kBMn ? 1 : 0);
+        if (lane == 0 && rank == 0) {
+            constexpr uint32_t idesc = make_idesc_bf16(L::kTileM, kBN, kAMn ? 1 : 0, kBMn ? 1 : 0);
             // K-major tile: 128 rows of 128 bytes, 8-row groups 1024 bytes apart, 32 bytes per K step.
             // MN-major tile: two blocks of 64 columns, 8192 bytes apart, each 64 K rows of 128 bytes;
             // a K step of 16 rows advances 2048 bytes.
@@ -201,8 +221,8 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_con
             constexpr uint64_t a_step = kAMn ? 128 : 2, b_step = kBMn ? 128 : 2;
             bool ok = true;
             int it = 0, na = 0;                         // ring position; tiles that used an accumulator
-            for (int lin = blockIdx.x; lin < n_tiles && ok; lin += gridDim.x) {
-                const GemmTile t = gemm_tile(g, lin);
+            for (int lin = kPair ? blockIdx.x >> 1 : blockIdx.x; lin < n_tiles && ok; lin += kPair ? gridDim.x >> 1 : gridDim.x) {
+                const GemmTile t = gemm_tile<kBN, L::kTileM>(g, lin, rank);
                 if (t.n_iters == 0) continue;
                 const int buf = na & 1;
                 // the epilogue has read this accumulator's previous tile out
@@ -219,11 +239,16 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_con
                     const uint64_t ad = a_desc0 + (uint64_t)((s * kStageBytes) >> 4);
                     const uint64_t bd = b_desc0 + (uint64_t)((s * kStageBytes) >> 4);
 #pragma unroll
-                    for (int k = 0; k < kBK / 16; ++k)
-                        mma_ss(acc, ad + a_step * k, bd + b_step * k, idesc, (i > 0 || k > 0) ? 1u : 0u);
-                    mma_commit(bar_empty(s));
+                    for (int k = 0; k < kBK / 16; ++k) {
+                        const uint32_t more = (i > 0 || k > 0) ? 1u : 0u;
+                        if constexpr (kPair) mma_ss_pair(acc, ad + a_step * k, bd + b_step * k, idesc, more);
+                        else mma_ss(acc, ad + a_step * k, bd + b_step * k, idesc, more);
+                    }
+                    if constexpr (kPair) mma_commit_pair(bar_empty(s));
+                    else mma_commit(bar_empty(s));
                 }
-                if (ok) mma_commit(bar_acc_full(buf));
+                if constexpr (kPair) { if (ok) mma_commit_pair(bar_acc_full(buf)); }
+                else { if (ok) mma_commit(bar_acc_full(buf)); }
                 LTCA_TRACE_EVT(0x22 + (na << 8));
                 ++na;
             }
@@ -232,13 +257,21 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_con
         // epilogue: warp w reads the 32 accumulator rows of its lane quarter (w % 4)
         const int qd = warp & 3;
         const int row = qd * 32 + lane;
-        uint8_t* stage = smem_gen + kOutOff;
-        const uint32_t stage_addr = smem_base + kOutOff;
+        uint8_t* stage = smem_gen + L::kOutOff;
+        const uint32_t stage_addr = smem_base + L::kOutOff;
         const int box_cols = g.out_bf16 ? 64 : 32;
+        auto release_acc = [&](int buf) {                    // the accumulator is in registers
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) {
+                if constexpr (kPair) mbar_arrive_cluster(map_shared(bar_acc_empty(buf), 0));
+                else mbar_arrive(bar_acc_empty(buf));
+            }
+        };
         bool ok = true;
         int na = 0, pc = 0;                                 // accumulators used; boxes staged
-        for (int lin = blockIdx.x; lin < n_tiles; lin += gridDim.x) {
-            const GemmTile t = gemm_tile(g, lin);
+        for (int lin = kPair ? blockIdx.x >> 1 : blockIdx.x; lin < n_tiles; lin += kPair ? gridDim.x >> 1 : gridDim.x) {
+            const GemmTile t = gemm_tile<kBN, L::kTileM>(g, lin, rank);
             const int gm = t.m0 + row;
             const int buf = na & 1;
             const bool have = t.n_iters > 0;
@@ -250,8 +283,7 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_con
             }
             const uint32_t tacc = tmem_base + (uint32_t)kBN * buf + ((uint32_t)(qd * 32) << 16);
             const float* bias = (g.ksplit == 1) ? g.bias[t.problem] : nullptr;
-            const bool staged = g.tma_store && g.ksplit == 1;
-            if (staged) {
+            if (g.tma_store) {
                 // The tile leaves box by box: 128 rows of 128 bytes (64 bf16 or 32 fp32 columns) go to shared memory
                 // in the layout of a 128-byte swizzled TMA box and one thread stores the box; the tensor map clips
                 // rows and columns past the end of C.  (Storing a row's 16-byte pieces straight from registers costs
@@ -296,7 +328,7 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_con
                 };
                 // The tile's bias goes through shared memory once: read per row from global memory it was 32 uniform
                 // loads per 32 columns and thread, 7 us of a product of 3200 x 256 x 256.
-                float* bias_s = reinterpret_cast<float*>(smem_gen + kBiasOff);
+                float* bias_s = reinterpret_cast<float*>(smem_gen + L::kBiasOff);
                 if (bias) {
                     // (the last reads of the tile before lie before that tile's last barrier)
                     for (int c = row; c < kBN; c += 128) bias_s[c] = t.n0 + c < g.N ? __ldg(bias + t.n0 + c) : 0.f;
@@ -335,9 +367,11 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_con
                     fence_proxy_async_smem();
                     asm volatile("bar.sync 1, 128;" ::: "memory");    // the four epilogue warps have staged their rows
                     if (warp == 2 && lane == 0) {
-                        const CUtensorMap* tc = t.problem == 0 ? &tc0 : (t.problem == 1 ? &tc1 : &tc2);
-                        if (gn0 < g.N) {
-                            tma_store_4d(tc, stage_addr + hb * (kBM * 128), gn0, t.m0, t.bh, t.bb);
+                        // (partial tiles are one [problem][slice][M][N] tensor)
+                        const CUtensorMap* tc = t.problem == 0 || g.ksplit > 1 ? &tc0 : (t.problem == 1 ? &tc1 : &tc2);
+                        if (gn0 < g.N && t.m0 < g.M) {
+                            tma_store_4d(tc, stage_addr + hb * (kBM * 128), gn0, t.m0, g.ksplit > 1 ? t.slice : t.bh,
+                                         g.ksplit > 1 ? t.problem : t.bb);
                             if (g.c_lo) tma_store_4d(&tc1, stage_addr + (hb + 1) * (kBM * 128), gn0, t.m0, t.bh, t.bb);
                         }
                         tma_store_commit();
@@ -362,10 +396,7 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_con
                     if (pi + 2 < n_pieces) {
                         load_piece(pi + 2, va0, va1);
                     } else if (have) {
-                        // the accumulator is in registers: the MMA thread may start the tile after next in it
-                        tc_fence_before_sync();
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(bar_acc_empty(buf));
+                        release_acc(buf);              // the MMA thread may start the tile after next in it
                     }
                     put_piece(pi + 1, vb0, vb1);
                 }
@@ -383,11 +414,7 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_con
 #pragma unroll
                     for (int c = 0; c < 32; ++c) v[c] = 0u;
                 }
-                if (have && c0 + 32 == kBN) {
-                    tc_fence_before_sync();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(bar_acc_empty(buf));
-                }
+                if (have && c0 + 32 == kBN) release_acc(buf);
                 const int gn0 = t.n0 + c0;
                 if (bias) {
 #pragma unroll
@@ -437,11 +464,13 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_con
     tc_fence_before_sync();
     __syncthreads();
     LTCA_TRACE_EVT(0x3f);
+    if (misc[1]) __nanosleep(200000);        // aborted: give copies and MMAs in flight time to land
+    if constexpr (kPair) cluster_sync();     // nothing of the other CTA's is on its way here any more
     if (warp == 1) {
         __syncwarp();
-        if (misc[1]) __nanosleep(200000);    // aborted: give copies and MMAs in flight time to land
         tc_fence_after_sync();
-        tmem_dealloc(tmem_base, kAccCols);
+        if constexpr (kPair) tmem_dealloc_pair(tmem_base, L::kAccCols);
+        else tmem_dealloc(tmem_base, L::kAccCols);
     }
 }
 
@@ -457,19 +486,36 @@ namespace ltca {
 namespace {
 #endif
 
-// C[problem][i] = sum over slices of partial[problem][slice][i], in slice order.
-__global__ void gemm_splitk_reduce_kernel(const float* __restrict__ partial, float* c0, float* c1, float* c2,
-                                          int64_t mn, int ksplit) {
+// C[problem][i] = sum over slices of partial[problem][slice][i], in slice order; kVec consecutive i per thread, the loads
+// of four slices in flight at once: four values where that still leaves a thousand threads per SM (3 x 512 x 512 from four
+// slices: 4.8 us with one value and one load at a time, 3.7 so), else one (512 x 512 from 16 slices: 7.6 us with four).
+template <int kVec>
+__global__ void __launch_bounds__(256) gemm_splitk_reduce_kernel(const float* __restrict__ partial, float* c0, float* c1, float* c2,
+                                                                 int64_t mn, int ksplit) {
     grid_launch_dependents();
     grid_dependency_wait();
     const int problem = blockIdx.y;
     float* c = problem == 0 ? c0 : (problem == 1 ? c1 : c2);
-    const float* p = partial + (int64_t)problem * ksplit * mn;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < mn; i += (int64_t)gridDim.x * blockDim.x) {
-        float acc = 0.f;
-        for (int s = 0; s < ksplit; ++s) acc += p[(int64_t)s * mn + i];
-        c[i] = acc;
+    const int64_t i = ((int64_t)blockIdx.x * 256 + threadIdx.x) * kVec;
+    if (i >= mn) return;
+    const float* p = partial + (int64_t)problem * ksplit * mn + i;
+    float acc[kVec] = {};
+    for (int s = 0; s < ksplit; s += 4) {
+        float v[4][kVec];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            if (s + e >= ksplit) continue;
+            if constexpr (kVec == 4) *reinterpret_cast<float4*>(v[e]) = __ldg(reinterpret_cast<const float4*>(p + (int64_t)(s + e) * mn));
+            else v[e][0] = __ldg(p + (int64_t)(s + e) * mn);
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+#pragma unroll
+            for (int j = 0; j < kVec; ++j)
+                if (s + e < ksplit) acc[j] += v[e][j];
     }
+    if constexpr (kVec == 4) *reinterpret_cast<float4*>(c + i) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+    else c[i] = acc[0];
 }
 
 __global__ void cvt_rows_bf16_kernel(const float* __restrict__ src, int64_t ld_src, __nv_bfloat16* __restrict__ dst,
@@ -510,6 +556,53 @@ int make_operand_map(ltca_ctx* ctx, CUtensorMap* map, const GemmOperand& o, int 
     return make_tmap_bhsd(ctx, map, o.ptr, 2, batch_b, batch_h, mn_extent, k_extent, st, 64, 128);
 }
 
+// Which tile a product takes.
+//   - 128 x 128: all its tiles fit beside one another on the SMs.  One wave either way, and the smaller tile is spread over
+//     twice as many SMs and has half the epilogue behind its last MMA (M=3200 N=256 K=256: 9.3 us with 128 x 256, 7.1 so;
+//     three such products of K=3200 in four slices 12.0, 9.0).  With a second wave the traffic per MMA decides against it
+//     (M=8192, N=3 x 512, K=512: 17.4 us against 22.4), unless the other tile's second half would be empty anyway.
+//   - pairs: contractions of kPairMinBlocks ring stages or more whose tiles fill the pairs' waves as well.  The pair loads a
+//     third less per MMA (M=8192 N=4096, three pairs of K=512: 87 us and 76; dW of 3 x 512 x 512, K=32768: 60 and 52).  A
+//     short contraction spends its time on the results, and there the two CTAs only wait for one another (M=32768,
+//     N=3 x 512, K=512: 51 us and 56; 256 products of 256 x 256 x 512: 29 and 37).
+//   - 128 x 256 otherwise.
+enum GemmTileKind { kTile128, kTile256, kTilePair };
+constexpr int kPairMinBlocks = 16;
+GemmTileKind pick_tile(int M, int N, int64_t blocks, int64_t z, int sms) {
+    auto up = [](int64_t a, int64_t b) { return (a + b - 1) / b; };
+    if (N <= 128 || up(M, 128) * up(N, 128) * z <= sms) return kTile128;
+    if (sms < 2 || blocks < kPairMinBlocks) return kTile256;
+    const int64_t waves_pair = up(up(M, 256) * up(N, 256) * z, sms / 2), waves_256 = up(up(M, 128) * up(N, 256) * z, sms);
+    return waves_pair <= waves_256 ? kTilePair : kTile256;
+}
+
+struct GemmMaps { CUtensorMap a[3], b[3], c[3]; };
+template <int kBN, bool kPair>
+int launch_gemm(ltca_ctx* ctx, const GemmMaps& m, const GemmKArgs& g, bool amn, bool bmn, int64_t n_tiles, int sms) {
+    using L = GemmCfg<kBN, kPair>;
+    auto kern = !bmn ? gemm_bf16_sm100_kernel<false, false, kBN, kPair>
+                     : (amn ? gemm_bf16_sm100_kernel<true, true, kBN, kPair> : gemm_bf16_sm100_kernel<false, true, kBN, kPair>);
+    static SmemOptIn opt_in[3];
+    LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(opt_in[!bmn ? 0 : (amn ? 2 : 1)], ctx->device, kern, L::kDynBytes));
+    const int64_t units = kPair ? sms / 2 : sms;
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3((unsigned)((n_tiles < units ? n_tiles : units) * (kPair ? 2 : 1)));
+    cfg.blockDim = dim3(kGemmThreads);
+    cfg.dynamicSmemBytes = L::kDynBytes;
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = 2; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = kPair ? 2 : 1;
+    LTCA_CUDA_OK(ctx, cudaLaunchKernelEx(&cfg, kern, m.a[0], m.a[1], m.a[2], m.b[0], m.b[1], m.b[2], m.c[0], m.c[1], m.c[2], g));
+    LTCA_LAUNCH_OK(ctx, "gemm_bf16_sm100_kernel");
+    return LTCA_OK;
+}
+
 }  // namespace
 
 size_t gemm_sm100_partial_bytes(int M, int N, int n_problems, int ksplit) {
@@ -518,7 +611,7 @@ size_t gemm_sm100_partial_bytes(int M, int N, int n_problems, int ksplit) {
 }
 
 int gemm_sm100_pick_ksplit(int M, int N, int K, int n_problems, int sm_count) {
-    const int tiles = ((M + kBM - 1) / kBM) * ((N + kBN - 1) / kBN) * n_problems;
+    const int tiles = ((M + kBM - 1) / kBM) * ((N + 255) / 256) * n_problems;
     const int nkb = (K + kBK - 1) / kBK;
     if (sm_count <= 0) sm_count = kPlanSms;
     int ks = 1;
@@ -560,19 +653,21 @@ int gemm_sm100(ltca_ctx* ctx, const GemmProblem& gp) {
     g.batch_h = gp.batch_h; g.batch_b = gp.batch_b;
     g.c_bs[0] = gp.c_bs[0]; g.c_bs[1] = gp.c_bs[1];
     const int ces = gp.out_bf16 ? 2 : 4;
-    g.tma_store = (g.ksplit == 1 && ((gp.ldc * ces) % 16) == 0 && ((gp.c_bs[0] * ces) % 16) == 0 &&
-                   ((gp.c_bs[1] * ces) % 16) == 0) ? 1 : 0;
-    for (int i = 0; i < gp.n_problems && g.tma_store; ++i)
-        if (reinterpret_cast<uintptr_t>(gp.c[i]) & 15) g.tma_store = 0;
-    if (reinterpret_cast<uintptr_t>(gp.c_lo) & 15) g.tma_store = 0;
     CUtensorMap tc[3];
     memset(tc, 0, sizeof(tc));
-    if (g.tma_store) {
-        ltca_strides cs;
-        cs.batch = gp.c_bs[1]; cs.head = gp.c_bs[0]; cs.seq = gp.ldc;
-        for (int i = 0; i < 3; ++i) {
-            const int j = i < gp.n_problems ? i : 0;
-            void* dst = (i == 1 && gp.c_lo) ? gp.c_lo : gp.c[j];
+    if (g.ksplit > 1) {
+        const int64_t mn = (int64_t)gp.M * gp.N;
+        const ltca_strides ps{mn * g.ksplit, mn, gp.N};
+        g.tma_store = (gp.N & 3) == 0 && (reinterpret_cast<uintptr_t>(gp.partial) & 15) == 0;
+        if (g.tma_store && (rc = make_tmap_bhsd(ctx, &tc[0], gp.partial, 4, gp.n_problems, g.ksplit, gp.M, gp.N, ps, 32, kBM))) return rc;
+    } else {
+        g.tma_store = ((gp.ldc * ces) % 16) == 0 && ((gp.c_bs[0] * ces) % 16) == 0 && ((gp.c_bs[1] * ces) % 16) == 0 &&
+                      (reinterpret_cast<uintptr_t>(gp.c_lo) & 15) == 0;
+        for (int i = 0; i < gp.n_problems; ++i)
+            if (reinterpret_cast<uintptr_t>(gp.c[i]) & 15) g.tma_store = 0;
+        const ltca_strides cs{gp.c_bs[1], gp.c_bs[0], gp.ldc};
+        for (int i = 0; i < 3 && g.tma_store; ++i) {
+            void* dst = (i == 1 && gp.c_lo) ? gp.c_lo : gp.c[i < gp.n_problems ? i : 0];
             if ((rc = make_tmap_bhsd(ctx, &tc[i], dst, ces, gp.batch_b, gp.batch_h, gp.M, gp.N, cs,
                                      gp.out_bf16 ? 64 : 32, kBM))) return rc;
         }
@@ -583,33 +678,34 @@ int gemm_sm100(ltca_ctx* ctx, const GemmProblem& gp) {
         for (int i = 0; i < gp.n_problems; ++i)
             if (gp.bias[i]) return fail(ctx, LTCA_ERR_INVALID, "gemm: split K takes no bias");
     }
-    g.tiles_x = (gp.N + kBN - 1) / kBN;
-    g.tiles_y = (gp.M + kBM - 1) / kBM;
-    g.tiles_z = gp.n_problems * g.ksplit;
-    const int64_t n_tiles = (int64_t)g.tiles_x * g.tiles_y * g.tiles_z * g.batch_h * g.batch_b;
-    if (n_tiles > 0x7fffffff) return fail(ctx, LTCA_ERR_UNSUPPORTED, "gemm: too many tiles");
     const int sms = ctx->sm_count > 0 ? ctx->sm_count : kPlanSms;
-    dim3 grid((unsigned)(n_tiles < sms ? n_tiles : sms));
+    const int64_t z = (int64_t)gp.n_problems * g.ksplit * gp.batch_h * gp.batch_b;
+    const GemmTileKind kind = pick_tile(gp.M, gp.N, (int64_t)((gp.K + kBK - 1) / kBK) / g.ksplit * g.n_sum, z, sms);
+    const int tile_m = kind == kTilePair ? 2 * kBM : kBM, tile_n = kind == kTile128 ? 128 : 256;
+    g.tiles_x = (gp.N + tile_n - 1) / tile_n;
+    g.tiles_y = (gp.M + tile_m - 1) / tile_m;
+    g.tiles_z = gp.n_problems * g.ksplit;
+    const int64_t n_tiles = g.tiles_x * (g.tiles_y * z);
+    if (n_tiles > 0x7fffffff) return fail(ctx, LTCA_ERR_UNSUPPORTED, "gemm: too many tiles");
     const bool amn = gp.a[0].mn_major != 0, bmn = gp.b[0].mn_major != 0;
-    auto launch = [&](auto kern) -> int {
-        LTCA_CUDA_OK(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kDynBytes));
-        LTCA_CUDA_OK(ctx, launch_dependent(kern, grid, dim3(kGemmThreads), kDynBytes, ctx->stream, ta[0], ta[1], ta[2], tb[0],
-                                           tb[1], tb[2], tc[0], tc[1], tc[2], g));
-        LTCA_LAUNCH_OK(ctx, "gemm_bf16_sm100_kernel");
-        return LTCA_OK;
-    };
-    if (!amn && !bmn) rc = launch(gemm_bf16_sm100_kernel<false, false>);
-    else if (!amn && bmn) rc = launch(gemm_bf16_sm100_kernel<false, true>);
-    else if (amn && bmn) rc = launch(gemm_bf16_sm100_kernel<true, true>);
-    else return fail(ctx, LTCA_ERR_UNSUPPORTED, "gemm: A stored [K, M] with B stored [N, K] is not built");
+    if (amn && !bmn) return fail(ctx, LTCA_ERR_UNSUPPORTED, "gemm: A stored [K, M] with B stored [N, K] is not built");
+    const GemmMaps maps{{ta[0], ta[1], ta[2]}, {tb[0], tb[1], tb[2]}, {tc[0], tc[1], tc[2]}};
+    if (kind == kTilePair) rc = launch_gemm<256, true>(ctx, maps, g, amn, bmn, n_tiles, sms);
+    else if (kind == kTile256) rc = launch_gemm<256, false>(ctx, maps, g, amn, bmn, n_tiles, sms);
+    else rc = launch_gemm<128, false>(ctx, maps, g, amn, bmn, n_tiles, sms);
     if (rc) return rc;
     if (g.ksplit > 1) {
         const int64_t mn = (int64_t)gp.M * gp.N;
-        dim3 rg((unsigned)((mn + 255) / 256 < 1184 ? (mn + 255) / 256 : 1184), gp.n_problems);
-        LTCA_CUDA_OK(ctx, launch_dependent(gemm_splitk_reduce_kernel, rg, dim3(256), 0, ctx->stream, (const float*)gp.partial,
-                                           reinterpret_cast<float*>(gp.c[0]),
-                                           reinterpret_cast<float*>(gp.c[gp.n_problems > 1 ? 1 : 0]),
-                                           reinterpret_cast<float*>(gp.c[gp.n_problems > 2 ? 2 : 0]), mn, g.ksplit));
+        float* c[3];
+        bool vec = (mn & 3) == 0 && (reinterpret_cast<uintptr_t>(gp.partial) & 15) == 0 && mn / 4 * gp.n_problems >= (int64_t)kPlanSms * 1024;
+        for (int i = 0; i < 3; ++i) {
+            c[i] = reinterpret_cast<float*>(gp.c[i < gp.n_problems ? i : 0]);
+            vec = vec && (reinterpret_cast<uintptr_t>(c[i]) & 15) == 0;
+        }
+        const int64_t per = vec ? 1024 : 256;
+        const dim3 rg((unsigned)((mn + per - 1) / per), gp.n_problems);
+        LTCA_CUDA_OK(ctx, launch_dependent(vec ? gemm_splitk_reduce_kernel<4> : gemm_splitk_reduce_kernel<1>, rg, dim3(256), 0, ctx->stream,
+                                           (const float*)gp.partial, c[0], c[1], c[2], mn, g.ksplit));
         LTCA_LAUNCH_OK(ctx, "gemm_splitk_reduce_kernel");
     }
     return LTCA_OK;
