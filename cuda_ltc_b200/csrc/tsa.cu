@@ -137,6 +137,13 @@ __global__ void residual_layer_norm_kernel(const float* __restrict__ y, const fl
     if (row >= rows) return;
     const RowOut o{out, nullptr, E, 0};
     layer_norm_row(y, x, gamma, beta, o, row, E, use_res != 0, use_ln != 0, eps, aligned16(y, x, gamma, beta, out));
+    // y is scratch and this was its only reader: whole lines of it that still lie in L2 need not be written to HBM
+    // (32768 x 512: 45.3 -> 43.6 us, and the module forward of 8192 rows 58.6 -> 57.1).  The row's stores above depend on
+    // every lane's loads, so nothing of it is still on its way.
+    if ((E & 31) == 0 && (reinterpret_cast<uintptr_t>(y) & 127) == 0) {
+        __syncwarp();
+        for (int l = threadIdx.x & 31; l < E / 32; l += 32) discard_line(y + row * E + 32 * l);
+    }
 }
 
 int residual_layer_norm(ltca_ctx* ctx, const ltca_tsa_params* t, const float* y, int64_t rows) {
