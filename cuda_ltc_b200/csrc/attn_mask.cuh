@@ -38,6 +38,34 @@ inline MaskArgs mask_args(const ltca_attn_params* p, const void* words) {
     return m;
 }
 
+// Packs the dense mask into m's words: one warp per block of 32 queries x 32 keys, blocks first, first + step, ...  Lane l
+// reads key l of each query (coalesced); the vote over a query's 32 values is its row word, the values a lane has seen are
+// its key's column word.
+__device__ __forceinline__ void write_mask_words(const MaskArgs& m, int B, int64_t first, int64_t step) {
+    const int lane = threadIdx.x & 31, Sq = m.Sq, Sk = m.Sk, nq = m.nq, nk = m.nk;
+    uint32_t* by_query = const_cast<uint32_t*>(m.by_query);
+    uint32_t* by_key = const_cast<uint32_t*>(m.by_key);
+    for (int64_t w = first; w < (int64_t)B * nq * nk; w += step) {
+        const int kw = (int)(w % nk), qw = (int)(w / nk % nq);
+        const int64_t b = w / ((int64_t)nk * nq);
+        const int q0 = qw * 32, k = kw * 32 + lane;
+        const float* src = m.dense + (b * Sq + q0) * Sk + k;
+        float v[32];
+#pragma unroll
+        for (int i = 0; i < 32; ++i) v[i] = (k < Sk && q0 + i < Sq) ? __ldg(src + (int64_t)i * Sk) : 0.f;
+        uint32_t row = 0, col = 0;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+            const bool keep = v[i] != 0.f;
+            const uint32_t bits = __ballot_sync(0xffffffffu, keep);
+            if (lane == i) row = bits;
+            col |= (keep ? 1u : 0u) << i;
+        }
+        if (q0 + lane < Sq) by_query[(b * Sq + q0 + lane) * nk + kw] = row;
+        if (k < Sk) by_key[(b * Sk + k) * nq + qw] = col;
+    }
+}
+
 // Bit c of the result: key k + c is kept for query q0 + lane (k a multiple of 32).  Whole-warp call.
 __device__ __forceinline__ uint32_t mask_bits_of_queries(const MaskArgs& m, int b, int q0, int k) {
     if (!m.dense) return ~0u;

@@ -172,9 +172,10 @@ __device__ __forceinline__ float dropout(float v, int64_t i, float p, float scal
     return dropout_uniform(seed, (uint64_t)i) >= p ? v * scale : 0.f;
 }
 
-// Everything the FlashAttention form does before its first product, in one launch whose blocks take one of three parts:
-// LayerNorm of the input rows, dropout of the incoming gradient, rounding of the weights to bf16.  As launches of their
-// own (with a separate rounding of the first two results) these were four of 12 kernels of a few microseconds.
+// Everything the FlashAttention form does before its first product, in one launch whose blocks take one of four parts:
+// packing of the dense mask, LayerNorm of the input rows, dropout of the incoming gradient, rounding of the weights to
+// bf16.  As launches of their own (with a separate rounding of LayerNorm's and dropout's results) these were five of 13
+// kernels of a few microseconds; the mask's took 6.5 us of latency in each direction of B16 S200.
 struct PrepareArgs {
     const float *x, *gamma, *beta;      // rows [rows, E]; LayerNorm when use_ln, else a copy
     RowOut xo;
@@ -184,7 +185,9 @@ struct PrepareArgs {
     int E, use_ln;
     float eps, p;
     uint64_t seed;
-    int row_blocks, dy_blocks;          // blocks of the first two parts
+    MaskArgs mask;                      // words to write, or no mask
+    int B;
+    int mask_blocks, row_blocks, dy_blocks;      // blocks of the first three parts
     CvtMany w;                          // matrices to round
 };
 constexpr int kPrepareThreads = 256;
@@ -192,6 +195,11 @@ __global__ void __launch_bounds__(kPrepareThreads) prenorm_prepare_kernel(const 
     grid_launch_dependents();
     grid_dependency_wait();
     int block = blockIdx.x;
+    if (block < a.mask_blocks) {
+        write_mask_words(a.mask, a.B, (int64_t)block * (kPrepareThreads / 32) + (threadIdx.x >> 5), (int64_t)a.mask_blocks * (kPrepareThreads / 32));
+        return;
+    }
+    block -= a.mask_blocks;
     if (block < a.row_blocks) {
         const int64_t row = (int64_t)block * (kPrepareThreads / 32) + (threadIdx.x >> 5);
         if (row >= a.rows) return;
@@ -228,7 +236,7 @@ __global__ void __launch_bounds__(kPrepareThreads) prenorm_prepare_kernel(const 
     }
     block -= a.dy_blocks;
     cvt_many_pieces(a.w, (uint32_t)block * kPrepareThreads + threadIdx.x,
-                    (gridDim.x - a.row_blocks - a.dy_blocks) * kPrepareThreads);
+                    (gridDim.x - a.mask_blocks - a.row_blocks - a.dy_blocks) * kPrepareThreads);
 }
 
 // out = dropout(y (+ x)): the end of the FlashAttention form's forward.
@@ -427,8 +435,10 @@ size_t colsum_scratch_bytes(const ltca_tsa_params* t) {
     return align_up((size_t)kMaxColJobs * kColChunks * (hw > t->E ? hw : t->E) * sizeof(float), 256);
 }
 
-// `xo` receives LayerNorm(x) (or x), `go` the gradient behind the dropout (null outputs: no such part); w: matrices to round.
-int prenorm_prepare(ltca_ctx* ctx, const ltca_tsa_params* t, const RowOut& xo, const RowOut* go, const CvtMany* w) {
+// `xo` receives LayerNorm(x) (or x), `go` the gradient behind the dropout (null outputs: no such part); w: matrices to
+// round; mask: words to write (null: no such part).
+int prenorm_prepare(ltca_ctx* ctx, const ltca_tsa_params* t, const RowOut& xo, const RowOut* go, const CvtMany* w,
+                    const MaskArgs* mask = nullptr) {
     PrepareArgs a;
     memset(&a, 0, sizeof(a));
     a.x = t->x; a.gamma = t->ln_gamma; a.beta = t->ln_beta;
@@ -454,8 +464,15 @@ int prenorm_prepare(ltca_ctx* ctx, const ltca_tsa_params* t, const RowOut& xo, c
         const uint32_t blocks = (w->start4[w->n] + 2 * kPrepareThreads - 1) / (2 * kPrepareThreads);
         w_blocks = blocks < 4u * sms ? (int)blocks : 4 * sms;
     }
-    if (a.row_blocks + a.dy_blocks + w_blocks == 0) return LTCA_OK;
-    LTCA_CUDA_OK(ctx, launch_dependent(prenorm_prepare_kernel, dim3((unsigned)(a.row_blocks + a.dy_blocks + w_blocks)),
+    if (mask) {
+        a.mask = *mask;
+        a.B = t->B;
+        const int64_t blocks = ((int64_t)t->B * mask->nq * mask->nk + kPrepareThreads / 32 - 1) / (kPrepareThreads / 32);
+        a.mask_blocks = (int)(blocks < 8 * sms ? blocks : 8 * sms);
+    }
+    const int blocks = a.mask_blocks + a.row_blocks + a.dy_blocks + w_blocks;
+    if (blocks == 0) return LTCA_OK;
+    LTCA_CUDA_OK(ctx, launch_dependent(prenorm_prepare_kernel, dim3((unsigned)blocks),
                                        dim3(kPrepareThreads), 0, ctx->stream, a));
     return LTCA_OK;
 }
@@ -714,6 +731,27 @@ void fill_wide(const ltca_tsa_params* t, const TBufs& tb, WideArgs* w) {
 // The attention scratch (TBufs::rest) of a call whose buffers start at w; not on the written-out-score path.
 char* scratch_of(const ltca_tsa_params* t, const TPlan& pl, char* w) { return t->saved ? w : w + tensor_saved_bytes(pl); }
 
+// What a module call tells its kernels through the context, taken back when the call returns.
+struct CallHints {
+    ltca_ctx* ctx;
+    ~CallHints() { ctx->mask_packed = nullptr; ctx->mask_words = nullptr; ctx->fwd_pairs = false; }
+};
+// The packed form of the call's dense mask lies in the last bytes of the `bytes` of scratch that its attention kernels
+// share; `later`: the call's prepare launch writes it (prenorm_prepare), else it is written now.
+int place_mask_words(ltca_ctx* ctx, const ltca_tsa_params* t, const TPlan& pl, char* scratch, size_t bytes, bool later) {
+    if (!t->keep_mask || pl.wide) return LTCA_OK;
+    ltca_attn_params a;
+    fill_attn_bf16(t, &a);
+    const size_t need = mask_words_bytes(&a);
+    if (bytes < need) return LTCA_OK;
+    void* words = scratch + (bytes - need);
+    int rc;
+    if (!later && (rc = pack_mask_words(ctx, &a, words))) return rc;
+    ctx->mask_packed = t->keep_mask;
+    ctx->mask_words = words;
+    return LTCA_OK;
+}
+
 // bf16 copies, fused Q/K/V projection, attention forward.
 // `also_src` / `also_dst`: one more [rows, E] fp32 matrix (the backward's dy) to be rounded to bf16 by the same launch
 // that rounds x and the weights; *also_done says whether that happened (not on the paths that convert otherwise
@@ -787,7 +825,12 @@ int tensor_forward_core(ltca_ctx* ctx, const ltca_tsa_params* t, const TPlan& pl
             const bool one = make_cvt_many(&wm, n - 1, src + 1, ld_src + 1, dst + 1, ld_dst + 1, nrows + 1, ncols + 1, nullptr);
             if (!one && n > 1 && (rc = convert_many_bf16(ctx, n - 1, src + 1, ld_src + 1, dst + 1, ld_dst + 1, nrows + 1, ncols + 1)))
                 return rc;
-            if ((rc = prenorm_prepare(ctx, outer, xo, also_src ? &go : nullptr, one ? &wm : nullptr))) return rc;
+            // (the mask's words go where the context says that the call's kernels will find them)
+            ltca_attn_params ap;
+            fill_attn_bf16(t, &ap);
+            const MaskArgs words = mask_args(&ap, ctx->mask_words);
+            const bool mask = t->keep_mask && ctx->mask_packed == t->keep_mask;
+            if ((rc = prenorm_prepare(ctx, outer, xo, also_src ? &go : nullptr, one ? &wm : nullptr, mask ? &words : nullptr))) return rc;
             if (also_done) *also_done = true;
             n = 0;
         } else if (also_src) {
@@ -870,6 +913,8 @@ int tensor_forward(ltca_ctx* ctx, const ltca_tsa_params* t, const ltca_tsa_param
     float* y = reinterpret_cast<float*>(w);
     w += pl.y;
     TBufs tb;
+    CallHints hints{ctx};
+    if (fused && (rc = place_mask_words(ctx, t, pl, scratch_of(t, pl, w), pl.attn_fwd, true))) return rc;
     if ((rc = tensor_forward_core(ctx, t, pl, w, &tb, 0, nullptr, nullptr, nullptr, fused ? outer : nullptr))) return rc;
     GemmProblem gp;
     gp.M = (int)pl.rows; gp.N = t->E; gp.K = pl.HW;
@@ -902,20 +947,10 @@ int tensor_backward(ltca_ctx* ctx, const ltca_tsa_params* t, bool want_dx, bool 
     // the forward is recomputed, as the reference's caller does before each backward
     // (src/ml/ml_liquid_net.cu:715-721)
     // the recomputed attention and its backward read the same mask: packed once, behind what either uses of the scratch
-    struct Hints {
-        ltca_ctx* ctx;
-        ~Hints() { ctx->mask_packed = nullptr; ctx->mask_words = nullptr; ctx->fwd_pairs = false; }
-    } hints{ctx};
+    CallHints hints{ctx};
     ctx->fwd_pairs = t->bk != nullptr;
-    if (t->keep_mask && !pl.wide) {
-        ltca_attn_params a;
-        fill_attn_bf16(t, &a);
-        const size_t most = pl.attn_fwd > pl.attn_bwd ? pl.attn_fwd : pl.attn_bwd;
-        void* words = scratch_of(t, pl, w) + (most - mask_words_bytes(&a));
-        if ((rc = pack_mask_words(ctx, &a, words))) return rc;
-        ctx->mask_packed = t->keep_mask;
-        ctx->mask_words = words;
-    }
+    const size_t most = pl.attn_fwd > pl.attn_bwd ? pl.attn_fwd : pl.attn_bwd;
+    if ((rc = place_mask_words(ctx, t, pl, scratch_of(t, pl, w), most, outer && !(t->saved && t->reuse_forward)))) return rc;
     bool dy_done = false;
     if ((rc = tensor_forward_core(ctx, t, pl, w, &tb, 1, t->dy, dyb, &dy_done, outer, outer_g))) return rc;
     const int rows = (int)pl.rows, E = t->E, HW = pl.HW, Ep = pl.Ep;
