@@ -67,6 +67,8 @@ struct GemmCfg {
     static constexpr uint32_t kAccCols = 2 * kBN;                  // two accumulators
 };
 
+struct GemmMaps { CUtensorMap a[kMaxGemmProblems], b[kMaxGemmProblems], c[kMaxGemmProblems]; };
+
 struct GemmKArgs {
     int M, N, K;
     int n_sum, ksplit;
@@ -76,9 +78,9 @@ struct GemmKArgs {
     int64_t ldc;
     int out_bf16;
     int tma_store;           // results leave through shared memory and a TMA store (needs 16-byte aligned rows)
-    void* C[3];
-    void* c_lo;              // second bf16 term of the (single) result, or null; its tensor map is tc1
-    const float* bias[3];
+    void* C[kMaxGemmProblems];
+    void* c_lo;              // second bf16 term of the (single) result, or null; its tensor map is c[1]
+    const float* bias[kMaxGemmProblems];
     float* partial;          // [problem][slice][M][N] when ksplit > 1
     uint32_t* status;
 };
@@ -117,11 +119,7 @@ __device__ __forceinline__ GemmTile gemm_tile(const GemmKArgs& g, int linear, in
 // the producer is loading tile i+2's operands.
 template <bool kAMn, bool kBMn, int kBN, bool kPair>
 __global__ void __launch_bounds__(kGemmThreads, 1)
-gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CUtensorMap ta1,
-                       const __grid_constant__ CUtensorMap ta2, const __grid_constant__ CUtensorMap tb0,
-                       const __grid_constant__ CUtensorMap tb1, const __grid_constant__ CUtensorMap tb2,
-                       const __grid_constant__ CUtensorMap tc0, const __grid_constant__ CUtensorMap tc1,
-                       const __grid_constant__ CUtensorMap tc2, const GemmKArgs g) {
+gemm_bf16_sm100_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ GemmKArgs g) {
     using L = GemmCfg<kBN, kPair>;
     constexpr int kStages = L::kStages, kStageBytes = L::kStageBytes;
     extern __shared__ uint8_t smem_raw[];
@@ -166,16 +164,16 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_con
 
     if (warp == 0) {
         if (lane == 0) {
-            tma_prefetch_desc(&ta0);
-            tma_prefetch_desc(&tb0);
+            tma_prefetch_desc(&maps.a[0]);
+            tma_prefetch_desc(&maps.b[0]);
             bool ok = true;
             int it = 0;
             for (int lin = kPair ? blockIdx.x >> 1 : blockIdx.x; lin < n_tiles && ok; lin += kPair ? gridDim.x >> 1 : gridDim.x) {
                 const GemmTile t = gemm_tile<kBN, L::kTileM>(g, lin, rank);
                 for (int p = 0; p < t.n_pairs && ok; ++p) {
                     const int pair = t.pair_begin + p;
-                    const CUtensorMap* ta = pair == 0 ? &ta0 : (pair == 1 ? &ta1 : &ta2);
-                    const CUtensorMap* tb = pair == 0 ? &tb0 : (pair == 1 ? &tb1 : &tb2);
+                    const CUtensorMap* ta = &maps.a[pair];
+                    const CUtensorMap* tb = &maps.b[pair];
                     for (int kb = t.kb_begin; kb < t.kb_end; ++kb, ++it) {
                         const int s = it % kStages;
                         ok = mbar_wait(bar_empty(s), (uint32_t)(((it / kStages) & 1) ^ 1), wc, 0xd0);
@@ -368,11 +366,11 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_con
                     asm volatile("bar.sync 1, 128;" ::: "memory");    // the four epilogue warps have staged their rows
                     if (warp == 2 && lane == 0) {
                         // (partial tiles are one [problem][slice][M][N] tensor)
-                        const CUtensorMap* tc = t.problem == 0 || g.ksplit > 1 ? &tc0 : (t.problem == 1 ? &tc1 : &tc2);
+                        const CUtensorMap* tc = &maps.c[g.ksplit > 1 ? 0 : t.problem];
                         if (gn0 < g.N && t.m0 < g.M) {
                             tma_store_4d(tc, stage_addr + hb * (kBM * 128), gn0, t.m0, g.ksplit > 1 ? t.slice : t.bh,
                                          g.ksplit > 1 ? t.problem : t.bb);
-                            if (g.c_lo) tma_store_4d(&tc1, stage_addr + (hb + 1) * (kBM * 128), gn0, t.m0, t.bh, t.bb);
+                            if (g.c_lo) tma_store_4d(&maps.c[1], stage_addr + (hb + 1) * (kBM * 128), gn0, t.m0, t.bh, t.bb);
                         }
                         tma_store_commit();
                         // the box that the next piece takes has been read
@@ -491,11 +489,11 @@ namespace {
 // slices: 4.8 us with one value and one load at a time, 3.7 so), else one (512 x 512 from 16 slices: 7.6 us with four).
 template <int kVec>
 __global__ void __launch_bounds__(256) gemm_splitk_reduce_kernel(const float* __restrict__ partial, float* c0, float* c1, float* c2,
-                                                                 int64_t mn, int ksplit) {
+                                                                 float* c3, int64_t mn, int ksplit) {
     grid_launch_dependents();
     grid_dependency_wait();
     const int problem = blockIdx.y;
-    float* c = problem == 0 ? c0 : (problem == 1 ? c1 : c2);
+    float* c = problem == 0 ? c0 : (problem == 1 ? c1 : (problem == 2 ? c2 : c3));
     const int64_t i = ((int64_t)blockIdx.x * 256 + threadIdx.x) * kVec;
     if (i >= mn) return;
     const float* p = partial + (int64_t)problem * ksplit * mn + i;
@@ -576,7 +574,6 @@ GemmTileKind pick_tile(int M, int N, int64_t blocks, int64_t z, int sms) {
     return waves_pair <= waves_256 ? kTilePair : kTile256;
 }
 
-struct GemmMaps { CUtensorMap a[3], b[3], c[3]; };
 template <int kBN, bool kPair>
 int launch_gemm(ltca_ctx* ctx, const GemmMaps& m, const GemmKArgs& g, bool amn, bool bmn, int64_t n_tiles, int sms) {
     using L = GemmCfg<kBN, kPair>;
@@ -598,7 +595,7 @@ int launch_gemm(ltca_ctx* ctx, const GemmMaps& m, const GemmKArgs& g, bool amn, 
     attr[1].val.clusterDim.x = 2; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = kPair ? 2 : 1;
-    LTCA_CUDA_OK(ctx, cudaLaunchKernelEx(&cfg, kern, m.a[0], m.a[1], m.a[2], m.b[0], m.b[1], m.b[2], m.c[0], m.c[1], m.c[2], g));
+    LTCA_CUDA_OK(ctx, cudaLaunchKernelEx(&cfg, kern, m, g));
     LTCA_LAUNCH_OK(ctx, "gemm_bf16_sm100_kernel");
     return LTCA_OK;
 }
@@ -621,22 +618,21 @@ int gemm_sm100_pick_ksplit(int M, int N, int K, int n_problems, int sm_count) {
 }
 
 int gemm_sm100(ltca_ctx* ctx, const GemmProblem& gp) {
-    if (gp.n_problems < 1 || gp.n_problems > 3 || gp.n_sum < 1 || gp.n_sum > 3 ||
+    if (gp.n_problems < 1 || gp.n_problems > kMaxGemmProblems || gp.n_sum < 1 || gp.n_sum > 3 ||
         (gp.n_sum > 1 && gp.n_problems != 1))
-        return fail(ctx, LTCA_ERR_INVALID, "gemm: between 1 and 3 problems, or one problem of up to 3 summed pairs");
+        return fail(ctx, LTCA_ERR_INVALID, "gemm: between 1 and 4 problems, or one problem of up to 3 summed pairs");
     if (gp.M < 1 || gp.N < 1 || gp.K < 1) return fail(ctx, LTCA_ERR_INVALID, "gemm: empty problem");
     const bool batched = gp.batch_h > 1 || gp.batch_b > 1;
     if (gp.batch_h < 1 || gp.batch_b < 1 || (batched && (gp.n_problems != 1 || gp.ksplit > 1)))
         return fail(ctx, LTCA_ERR_INVALID, "gemm: a batch takes one problem (or one sum of pairs) and no split of K");
     const int n_pairs = gp.n_sum > 1 ? gp.n_sum : gp.n_problems;
-    CUtensorMap ta[3], tb[3];
+    GemmMaps maps;
     int rc;
-    for (int i = 0; i < 3; ++i) {
-        const int j = i < n_pairs ? i : 0;
-        if (gp.a[j].mn_major != gp.a[0].mn_major || gp.b[j].mn_major != gp.b[0].mn_major)
+    for (int i = 0; i < n_pairs; ++i) {
+        if (gp.a[i].mn_major != gp.a[0].mn_major || gp.b[i].mn_major != gp.b[0].mn_major)
             return fail(ctx, LTCA_ERR_INVALID, "gemm: all pairs of one launch share the operand forms");
-        if ((rc = make_operand_map(ctx, &ta[i], gp.a[j], gp.M, gp.K, gp.batch_h, gp.batch_b, gp.a_bs))) return rc;
-        if ((rc = make_operand_map(ctx, &tb[i], gp.b[j], gp.N, gp.K, gp.batch_h, gp.batch_b, gp.b_bs))) return rc;
+        if ((rc = make_operand_map(ctx, &maps.a[i], gp.a[i], gp.M, gp.K, gp.batch_h, gp.batch_b, gp.a_bs))) return rc;
+        if ((rc = make_operand_map(ctx, &maps.b[i], gp.b[i], gp.N, gp.K, gp.batch_h, gp.batch_b, gp.b_bs))) return rc;
     }
     GemmKArgs g;
     g.M = gp.M; g.N = gp.N; g.K = gp.K;
@@ -647,28 +643,26 @@ int gemm_sm100(ltca_ctx* ctx, const GemmProblem& gp) {
     g.c_lo = gp.c_lo;
     if (gp.c_lo && (!gp.out_bf16 || gp.n_problems != 1 || gp.ksplit > 1))
         return fail(ctx, LTCA_ERR_INVALID, "gemm: a second result term needs one bf16 problem and no split of K");
-    for (int i = 0; i < 3; ++i) { g.C[i] = gp.c[i < gp.n_problems ? i : 0]; g.bias[i] = i < gp.n_problems ? gp.bias[i] : nullptr; }
+    for (int i = 0; i < kMaxGemmProblems; ++i) { g.C[i] = gp.c[i < gp.n_problems ? i : 0]; g.bias[i] = i < gp.n_problems ? gp.bias[i] : nullptr; }
     g.partial = gp.partial;
     g.status = ctx->d_status;
     g.batch_h = gp.batch_h; g.batch_b = gp.batch_b;
     g.c_bs[0] = gp.c_bs[0]; g.c_bs[1] = gp.c_bs[1];
     const int ces = gp.out_bf16 ? 2 : 4;
-    CUtensorMap tc[3];
-    memset(tc, 0, sizeof(tc));
     if (g.ksplit > 1) {
         const int64_t mn = (int64_t)gp.M * gp.N;
         const ltca_strides ps{mn * g.ksplit, mn, gp.N};
         g.tma_store = (gp.N & 3) == 0 && (reinterpret_cast<uintptr_t>(gp.partial) & 15) == 0;
-        if (g.tma_store && (rc = make_tmap_bhsd(ctx, &tc[0], gp.partial, 4, gp.n_problems, g.ksplit, gp.M, gp.N, ps, 32, kBM))) return rc;
+        if (g.tma_store && (rc = make_tmap_bhsd(ctx, &maps.c[0], gp.partial, 4, gp.n_problems, g.ksplit, gp.M, gp.N, ps, 32, kBM))) return rc;
     } else {
         g.tma_store = ((gp.ldc * ces) % 16) == 0 && ((gp.c_bs[0] * ces) % 16) == 0 && ((gp.c_bs[1] * ces) % 16) == 0 &&
                       (reinterpret_cast<uintptr_t>(gp.c_lo) & 15) == 0;
         for (int i = 0; i < gp.n_problems; ++i)
             if (reinterpret_cast<uintptr_t>(gp.c[i]) & 15) g.tma_store = 0;
         const ltca_strides cs{gp.c_bs[1], gp.c_bs[0], gp.ldc};
-        for (int i = 0; i < 3 && g.tma_store; ++i) {
-            void* dst = (i == 1 && gp.c_lo) ? gp.c_lo : gp.c[i < gp.n_problems ? i : 0];
-            if ((rc = make_tmap_bhsd(ctx, &tc[i], dst, ces, gp.batch_b, gp.batch_h, gp.M, gp.N, cs,
+        for (int i = 0; i < (gp.c_lo ? 2 : gp.n_problems) && g.tma_store; ++i) {
+            void* dst = (i == 1 && gp.c_lo) ? gp.c_lo : gp.c[i];
+            if ((rc = make_tmap_bhsd(ctx, &maps.c[i], dst, ces, gp.batch_b, gp.batch_h, gp.M, gp.N, cs,
                                      gp.out_bf16 ? 64 : 32, kBM))) return rc;
         }
     }
@@ -689,23 +683,22 @@ int gemm_sm100(ltca_ctx* ctx, const GemmProblem& gp) {
     if (n_tiles > 0x7fffffff) return fail(ctx, LTCA_ERR_UNSUPPORTED, "gemm: too many tiles");
     const bool amn = gp.a[0].mn_major != 0, bmn = gp.b[0].mn_major != 0;
     if (amn && !bmn) return fail(ctx, LTCA_ERR_UNSUPPORTED, "gemm: A stored [K, M] with B stored [N, K] is not built");
-    const GemmMaps maps{{ta[0], ta[1], ta[2]}, {tb[0], tb[1], tb[2]}, {tc[0], tc[1], tc[2]}};
     if (kind == kTilePair) rc = launch_gemm<256, true>(ctx, maps, g, amn, bmn, n_tiles, sms);
     else if (kind == kTile256) rc = launch_gemm<256, false>(ctx, maps, g, amn, bmn, n_tiles, sms);
     else rc = launch_gemm<128, false>(ctx, maps, g, amn, bmn, n_tiles, sms);
     if (rc) return rc;
     if (g.ksplit > 1) {
         const int64_t mn = (int64_t)gp.M * gp.N;
-        float* c[3];
+        float* c[kMaxGemmProblems];
         bool vec = (mn & 3) == 0 && (reinterpret_cast<uintptr_t>(gp.partial) & 15) == 0 && mn / 4 * gp.n_problems >= (int64_t)kPlanSms * 1024;
-        for (int i = 0; i < 3; ++i) {
+        for (int i = 0; i < kMaxGemmProblems; ++i) {
             c[i] = reinterpret_cast<float*>(gp.c[i < gp.n_problems ? i : 0]);
             vec = vec && (reinterpret_cast<uintptr_t>(c[i]) & 15) == 0;
         }
         const int64_t per = vec ? 1024 : 256;
         const dim3 rg((unsigned)((mn + per - 1) / per), gp.n_problems);
         LTCA_CUDA_OK(ctx, launch_dependent(vec ? gemm_splitk_reduce_kernel<4> : gemm_splitk_reduce_kernel<1>, rg, dim3(256), 0, ctx->stream,
-                                           (const float*)gp.partial, c[0], c[1], c[2], mn, g.ksplit));
+                                           (const float*)gp.partial, c[0], c[1], c[2], c[3], mn, g.ksplit));
         LTCA_LAUNCH_OK(ctx, "gemm_splitk_reduce_kernel");
     }
     return LTCA_OK;

@@ -16,13 +16,14 @@ struct GemmOperand {
 
 // C_i[M,N] = A_i B_i (+ bias_i) for i < n_problems (n_sum == 1), or
 // C_0[M,N] = sum_{p < n_sum} A_p B_p (+ bias_0)            (n_problems == 1).
+constexpr int kMaxGemmProblems = 4;
 struct GemmProblem {
     int M = 0, N = 0, K = 0;
     int n_problems = 1, n_sum = 1;
     int ksplit = 1;                 // > 1: K range cut into slices, summed in order from `partial`
-    GemmOperand a[3] = {}, b[3] = {};
-    void* c[3] = {nullptr, nullptr, nullptr};
-    const float* bias[3] = {nullptr, nullptr, nullptr};
+    GemmOperand a[kMaxGemmProblems] = {}, b[kMaxGemmProblems] = {};
+    void* c[kMaxGemmProblems] = {};
+    const float* bias[kMaxGemmProblems] = {};
     int64_t ldc = 0;
     int out_bf16 = 0;               // result element type: bf16 or fp32
     void* c_lo = nullptr;           // with out_bf16, one problem, no split of K: also write bf16(x - bf16(x)) here,

@@ -643,7 +643,7 @@ struct TPlan {
     int HW, Ep;
     size_t xb, w_in, w_out, act, lse, y;
     size_t attn_fwd, attn_bwd, partial;
-    int ks_in, ks_out;
+    int ks_in, ks_out, n_dw;
     // materialised-score path: low-order parts of x, Wq, Wk, q, k; fp32 projection scratch; score matrices
     bool wide;
     size_t mat32, mat16;
@@ -674,9 +674,12 @@ int make_tplan(const ltca_tsa_params* t, TPlan* pl, bool backward) {
         if ((rc = ltca_attn_workspace_bytes(&a, 1, &pl->attn_bwd))) return rc;
     }
     const int rows = (int)pl->rows;
-    pl->ks_in = gemm_sm100_pick_ksplit(t->E, pl->HW, rows, 3, kPlanSms);
+    // dWq, dWk, dWv are one launch, and dWo with them where it has their shape: 64 pairs of CTAs with work instead of 48 and
+    // then 64 with a quarter of it (32768 x 512 x 512: 51 + 21 us and two reductions of 4 and 5, so 55 and one of 4)
+    pl->n_dw = t->E == pl->HW ? 4 : 3;
+    pl->ks_in = gemm_sm100_pick_ksplit(t->E, pl->HW, rows, pl->n_dw, kPlanSms);
     pl->ks_out = gemm_sm100_pick_ksplit(pl->HW, t->E, rows, 1, kPlanSms);
-    const size_t p_in = gemm_sm100_partial_bytes(t->E, pl->HW, 3, pl->ks_in);
+    const size_t p_in = gemm_sm100_partial_bytes(t->E, pl->HW, pl->n_dw, pl->ks_in);
     const size_t p_out = gemm_sm100_partial_bytes(pl->HW, t->E, 1, pl->ks_out);
     pl->partial = p_in > p_out ? p_in : p_out;
     return LTCA_OK;
@@ -1005,7 +1008,7 @@ int tensor_backward(ltca_ctx* ctx, const ltca_tsa_params* t, bool want_dx, bool 
         {   // dW = x^T dq : x is stored [rows, E] = [K, M], dq [rows, HW] = [K, N]
             GemmProblem gp;
             gp.M = E; gp.N = HW; gp.K = rows;
-            gp.n_problems = 3;
+            gp.n_problems = pl.n_dw;
             gp.ksplit = pl.ks_in;
             void* dst[3] = {t->dwq, t->dwk, t->dwv};
             for (int i = 0; i < 3; ++i) {
@@ -1013,11 +1016,16 @@ int tensor_backward(ltca_ctx* ctx, const ltca_tsa_params* t, bool want_dx, bool 
                 gp.b[i] = GemmOperand{grads[i], HW, 1};
                 gp.c[i] = dst[i];
             }
+            if (gp.n_problems == 4) {
+                gp.a[3] = GemmOperand{tb.ctx, HW, 1};
+                gp.b[3] = GemmOperand{dyb, Ep, 1};
+                gp.c[3] = t->dwo;
+            }
             gp.ldc = HW;
             gp.partial = partial;
             if ((rc = gemm_sm100(ctx, gp))) return rc;
         }
-        {   // dWo = ctx^T dy
+        if (pl.n_dw == 3) {   // dWo = ctx^T dy
             GemmProblem gp;
             gp.M = HW; gp.N = E; gp.K = rows;
             gp.ksplit = pl.ks_out;
