@@ -102,7 +102,6 @@ __device__ __forceinline__ void load8(const float* p, float (&f)[8]) {
 constexpr int kStatsRows = 32;
 template <typename T>
 __global__ void __launch_bounds__(8 * kStatsRows) attn_bwd_stats_kernel(const StatsArgs a) {
-    grid_launch_dependents();
     grid_dependency_wait();
     const unsigned per_pair = (unsigned)a.Sq_pad / kStatsRows, bh = blockIdx.x / per_pair;
     const unsigned b = bh / (unsigned)a.H, h = bh - b * (unsigned)a.H;
@@ -284,7 +283,6 @@ attn_bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
     tc_fence_after_sync();
     const uint32_t tmem_base = misc[0];
     const WaitCtx wc{&misc[1], a.status};
-    grid_launch_dependents();                  // (set up: the next kernel may place its CTAs)
     grid_dependency_wait();                    // the operands are complete once the kernel before this one has ended
     auto slot_of = [&](int item) { return item % L::kStages; };
     auto phase_of = [&](int item) { return (uint32_t)((item / L::kStages) & 1); };
@@ -579,7 +577,6 @@ attn_bwd_dkv_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
     tc_fence_after_sync();
     const uint32_t tmem_base = misc[0];
     const WaitCtx wc{&misc[1], a.status};
-    grid_launch_dependents();                  // (set up: the next kernel may place its CTAs)
     grid_dependency_wait();                    // the operands are complete once the kernel before this one has ended
     // ring items are numbered from the first streamed step of this CTA
     auto slot_of = [&](int j) { return (j - j_first) % L::kStages; };
@@ -1296,9 +1293,6 @@ attn_bwd_dkv4_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
         }
     }
 
-    // Out of work: only now may the kernel after this one place its CTAs (released at the start, its blocks would
-    // sit beside this kernel's CTAs for the whole run, waiting for it to end).
-    grid_launch_dependents();
     tc_fence_before_sync();
     __syncthreads();
     if (threadIdx.x == 0) item_counters_release(grid.counters);
@@ -1855,9 +1849,6 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
         }
     }
 
-    // Out of work: only now may the kernel after this one place its CTAs (released at the start, its blocks would
-    // sit beside this kernel's CTAs for the whole run, waiting for it to end).
-    grid_launch_dependents();
     tc_fence_before_sync();
     __syncthreads();
     if (threadIdx.x == 0) item_counters_release(grid.counters);
@@ -1873,7 +1864,6 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
 __global__ void __launch_bounds__(256) attn_bwd_dq_convert_kernel(const float* __restrict__ acc, void* dq,
                                                                   ltca_strides dqs, int B, int H, int Sq, int Sq_pad,
                                                                   float scale) {
-    grid_launch_dependents();
     grid_dependency_wait();
     const int64_t idx = (int64_t)blockIdx.x * 32 + (threadIdx.x >> 3);       // row among B * H * Sq
     const int sub = threadIdx.x & 7;
@@ -2277,9 +2267,6 @@ attn_bwd_dq4_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
         }
     }
 
-    // Out of work: only now may the kernel after this one place its CTAs (released at the start, its blocks would
-    // sit beside this kernel's CTAs for the whole run, waiting for it to end).
-    grid_launch_dependents();
     tc_fence_before_sync();
     __syncthreads();
     if (threadIdx.x == 0) item_counters_release(grid.counters);

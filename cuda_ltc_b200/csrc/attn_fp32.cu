@@ -278,7 +278,6 @@ __device__ __forceinline__ float half_warp_sum(float v) {
 // ----------------------------------------------------------------------------------------------
 template <typename T, int DP, int TM, int NT, bool kMask>
 __global__ void __launch_bounds__(NT, TM < 64 ? 4 : DP <= 32 ? 4 : DP <= 64 ? 3 : 1) attn_fwd_fp32_kernel(const CoreArgs a) {
-    if (TM < 64) grid_launch_dependents();       // (see run_rows)
     grid_dependency_wait();
     constexpr int KN = 64, LD = DP + kPad, LP = KN + kPad, RS = NT / 16, RM = TM / RS, CN = KN / 16;
     using Lt = AccLayout<DP, TM, NT>;
@@ -412,7 +411,6 @@ __global__ void __launch_bounds__(NT, TM < 64 ? 4 : DP <= 32 ? 4 : DP <= 64 ? 3 
         if (more) load_padded<DP, KN, NT>(Vs, vb, a.vs.seq, k0 + KN, a.Sk, a.D, vec);
         cp_async_commit();
     }
-    if (TM == 64) grid_launch_dependents();
     cp_async_wait<0>();
 
 #pragma unroll
@@ -469,7 +467,6 @@ __global__ void attn_bwd_delta_kernel(const CoreArgs a) {
 // pass 1: delta = rowsum(dO o O), left for pass 2, and dQ.  One CTA per TM query rows, KN keys per step.
 template <typename T, int DP, int TM, int KN, int NT, bool kMask>
 __global__ void __launch_bounds__(NT, NT == 128 ? 3 : 1) attn_bwd_dq_fp32_kernel(const CoreArgs a) {
-    if (TM < 64) grid_launch_dependents();       // (see run_rows)
     grid_dependency_wait();
     constexpr int LD = DP + kPad, LP = KN + kPad, RS = NT / 16, RM = TM / RS, CN = KN / 16, NW = KN / 32;
     using Lt = AccLayout<DP, TM, NT>;
@@ -582,7 +579,6 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 3 : 1) attn_bwd_dq_fp32_kernel
         if (more) load_padded<DP, KN, NT>(Ks, kb, a.ks.seq, k0 + KN, a.Sk, a.D, vec);
         cp_async_commit();
     }
-    if (TM == 64) grid_launch_dependents();
     cp_async_wait<0>();
     if (!L.active) return;
     T* dqb = reinterpret_cast<T*>(a.dq) + b * a.dqs.batch + h * a.dqs.head;
@@ -601,7 +597,6 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 3 : 1) attn_bwd_dq_fp32_kernel
 // pass 2: dK and dV.  One CTA per TK keys, QN query rows per step; a thread accumulates NR neighbouring keys.
 template <typename T, int DP, int TK, int QN, int NT, bool kMask>
 __global__ void __launch_bounds__(NT, TK < 64 ? 3 : DP <= 32 ? 3 : DP <= 64 ? 2 : 1) attn_bwd_dkv_fp32_kernel(const CoreArgs a) {
-    if (TK < 64) grid_launch_dependents();       // (see run_rows)
     grid_dependency_wait();
     constexpr int LD = DP + kPad, LP = TK + kPad, RS = NT / 16, RM = QN / RS, CN = TK / 16, NW = (TK + 31) / 32;
     using Lt = AccLayout<DP, TK, NT>;
@@ -715,7 +710,6 @@ __global__ void __launch_bounds__(NT, TK < 64 ? 3 : DP <= 32 ? 3 : DP <= 64 ? 2 
         }
         __syncthreads();
     }
-    if (TK == 64) grid_launch_dependents();
     cp_async_wait<0>();
     if (!L.active) return;
     T* dkb = reinterpret_cast<T*>(a.dk) + b * a.dks.batch + h * a.dks.head;
@@ -800,8 +794,8 @@ int run_dkv(ltca_ctx* ctx, const CoreArgs& a) {
     return LTCA_OK;
 }
 
-// (The 64-row kernels let the next kernel's CTAs be placed when their loops are done: released at the start these take
-// whatever slots are left and sit unevenly on the SMs, 82 us instead of 67 for a B16 H8 S100 D32 step.)
+// (None of these kernels lets the next one's CTAs be placed before it ends: released at the start, or when the tile loop is
+// done, they take whatever slots are left and sit unevenly on the SMs, 82 or 62 us instead of 57 for B16 H8 S100 D32.)
 // Tiles of 64 rows reuse what they load most; where they would leave SMs idle, tiles of 16 rows give four times the CTAs
 // and a quarter of the serial work.
 template <typename T, int DP, bool kMask>

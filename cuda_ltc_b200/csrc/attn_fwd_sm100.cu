@@ -180,7 +180,6 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
     const WaitCtx wc{&misc[1], a.status};
     LTCA_TRACE_DECL(blockIdx.x == 0 && blockIdx.y == 5 && blockIdx.z == 0);
     LTCA_TRACE_EVT(0x01);
-    grid_launch_dependents();                  // (set up: the next kernel may place its CTAs)
     grid_dependency_wait();                    // q, k, v are complete once the kernel before this one has ended
 
     if (warp >= kMathWarps) {

@@ -6,7 +6,6 @@ namespace ltca {
 namespace {
 
 __global__ void __launch_bounds__(256) mask_words_kernel(const MaskArgs m, int B) {
-    grid_launch_dependents();
     grid_dependency_wait();
     write_mask_words(m, B, (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5), (int64_t)gridDim.x * 8);
 }

@@ -106,7 +106,6 @@ struct Gemm32Tile {
 
 template <bool TA, bool TB, int TM, int TN, int NT>
 __global__ void __launch_bounds__(NT) gemm_fp32_kernel(const __grid_constant__ Gemm32Args g) {
-    grid_launch_dependents();
     grid_dependency_wait();
     using G = Gemm32Tile<TM, TN, NT>;
     constexpr int KC = G::KC, RM = G::RM, CN = G::CN, kStages = G::kStages;
@@ -290,7 +289,6 @@ __device__ __forceinline__ void small_product(const Gemm32Args& g, int tx0, int 
     }
 }
 __global__ void __launch_bounds__(kSmallThreads) gemm_fp32_small_kernel(const __grid_constant__ Gemm32Pair a) {
-    grid_launch_dependents();
     grid_dependency_wait();
     extern __shared__ __align__(16) float sm[];
     const int grp = (int)blockIdx.x < a.blocks[0] ? 0 : 1;
@@ -303,7 +301,6 @@ __global__ void __launch_bounds__(kSmallThreads) gemm_fp32_small_kernel(const __
 
 // C[m][n] = sum over slices, in slice order, of the partial results; blockIdx.y picks the product.
 __global__ void __launch_bounds__(256) gemm_fp32_reduce_kernel(const __grid_constant__ Gemm32Args g) {
-    grid_launch_dependents();
     grid_dependency_wait();
     const Gemm32Problem& p = g.p[blockIdx.y];
     const int64_t mn = (int64_t)p.M * p.N;

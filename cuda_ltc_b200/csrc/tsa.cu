@@ -131,7 +131,6 @@ __global__ void residual_layer_norm_kernel(const float* __restrict__ y, const fl
                                            const float* __restrict__ gamma,
                                            const float* __restrict__ beta, float* __restrict__ out,
                                            int64_t rows, int E, int use_res, int use_ln, float eps) {
-    grid_launch_dependents();
     grid_dependency_wait();
     const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (row >= rows) return;
@@ -192,7 +191,6 @@ struct PrepareArgs {
 };
 constexpr int kPrepareThreads = 256;
 __global__ void __launch_bounds__(kPrepareThreads) prenorm_prepare_kernel(const __grid_constant__ PrepareArgs a) {
-    grid_launch_dependents();
     grid_dependency_wait();
     int block = blockIdx.x;
     if (block < a.mask_blocks) {
@@ -242,7 +240,6 @@ __global__ void __launch_bounds__(kPrepareThreads) prenorm_prepare_kernel(const 
 // out = dropout(y (+ x)): the end of the FlashAttention form's forward.
 __global__ void __launch_bounds__(256) residual_dropout_kernel(const float* __restrict__ y, const float* __restrict__ x, float* __restrict__ out,
                                                                int64_t n, int use_res, float p, uint64_t seed) {
-    grid_launch_dependents();
     grid_dependency_wait();
     const float scale = 1.0f / (1.0f - p);
     const int64_t first = (int64_t)blockIdx.x * 256 + threadIdx.x, step = (int64_t)gridDim.x * 256;
@@ -277,7 +274,6 @@ __global__ void layer_norm_bwd_kernel(const float* __restrict__ g, const float* 
                                       const float* __restrict__ gamma, const float* __restrict__ res,
                                       float* __restrict__ dx, float* __restrict__ prod, int64_t rows, int E,
                                       float eps) {
-    grid_launch_dependents();
     grid_dependency_wait();
     const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (row >= rows) return;
@@ -404,7 +400,6 @@ __device__ __forceinline__ float column_chunk(const T* src, int64_t ld, int64_t 
     return acc;
 }
 __global__ void __launch_bounds__(128) column_sum_partial_kernel(const __grid_constant__ ColSum a) {
-    grid_launch_dependents();
     grid_dependency_wait();
     const int j = blockIdx.z, c = blockIdx.x * 128 + threadIdx.x;
     if (c >= a.cols[j]) return;
@@ -415,7 +410,6 @@ __global__ void __launch_bounds__(128) column_sum_partial_kernel(const __grid_co
                   : column_chunk(static_cast<const float*>(a.src[j]) + c, a.ld[j], r0, r1);
 }
 __global__ void __launch_bounds__(128) column_sum_final_kernel(const __grid_constant__ ColSum a) {
-    grid_launch_dependents();
     grid_dependency_wait();
     const int j = blockIdx.y, c = blockIdx.x * 128 + threadIdx.x;
     if (c >= a.cols[j]) return;
