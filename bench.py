@@ -860,7 +860,7 @@ def main():
         # Algorithmic FLOPs per launch: one contraction over the causal half is f_fwd / 2.  Forward =
         # 2 contractions; the dK/dV kernel is charged S^T, dP^T, dV, dK (4), the dQ kernel only dQ (1; its
         # own S and dP are recomputation): together the 2.5 x forward of the backward pass.
-        kernels = {"attn_fwd4p_sm100_kernel": {"ms": fwd_ms, "flops": f_fwd}}
+        kernels = {"attn_fwd_tile_sm100_kernel": {"ms": fwd_ms, "flops": f_fwd}}
         if kern_ms:
             # bf16 storage takes the fused backward: row statistics (which also clear the fp32 dQ accumulator),
             # one kernel with the five contractions (2.5 x forward), and the conversion of the accumulator
