@@ -404,7 +404,8 @@ int pack_many_to_bf16(ltca_ctx* ctx, const PackJob* jobs, int count, int B, int 
     const uint64_t pieces = (uint64_t)B * H * s_max * (D / (4 * vec)), blocks = (pieces + kPackChunks * 256 - 1) / (kPackChunks * 256);
     if (blocks > 0x7fffffffull) return fail(ctx, LTCA_ERR_INVALID, "pack: tensor too large");
     const dim3 grid((unsigned)blocks, (unsigned)count);               // sized for the longest tensor
-    LTCA_CUDA_OK(ctx, launch_dependent(vec == 2 ? pack_bf16_kernel<2> : pack_bf16_kernel<1>, grid, dim3(256), 0, ctx->stream, k,
+    auto kern = vec == 2 ? pack_bf16_kernel<2> : pack_bf16_kernel<1>;
+    LTCA_CUDA_OK(ctx, launch_dependent(kern, grid, dim3(256), 0, ctx->stream, k,
                                        B * H, H, D));
     LTCA_LAUNCH_OK(ctx, "pack_bf16_kernel");
     return LTCA_OK;

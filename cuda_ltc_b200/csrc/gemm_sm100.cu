@@ -697,7 +697,8 @@ int gemm_sm100(ltca_ctx* ctx, const GemmProblem& gp) {
         }
         const int64_t per = vec ? 1024 : 256;
         const dim3 rg((unsigned)((mn + per - 1) / per), gp.n_problems);
-        LTCA_CUDA_OK(ctx, launch_dependent(vec ? gemm_splitk_reduce_kernel<4> : gemm_splitk_reduce_kernel<1>, rg, dim3(256), 0, ctx->stream,
+        auto kern = vec ? gemm_splitk_reduce_kernel<4> : gemm_splitk_reduce_kernel<1>;
+        LTCA_CUDA_OK(ctx, launch_dependent(kern, rg, dim3(256), 0, ctx->stream,
                                            (const float*)gp.partial, c[0], c[1], c[2], c[3], mn, g.ksplit));
         LTCA_LAUNCH_OK(ctx, "gemm_splitk_reduce_kernel");
     }
