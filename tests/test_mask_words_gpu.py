@@ -14,7 +14,7 @@ from util import bf16_round, keep_mask, randn
 pytestmark = pytest.mark.gpu
 
 
-# (1, 2, 700, 97): the four-tile forward; (2, 80, 300, 161): more work items than SMs
+# (1, 2, 700, 97): several query tiles; (2, 80, 300, 161): more work items than SMs
 @pytest.mark.parametrize("shape", [(2, 2, 1, 1), (1, 3, 31, 33), (2, 2, 64, 65), (1, 2, 129, 31), (1, 2, 700, 97), (2, 80, 300, 161)])
 @pytest.mark.parametrize("storage", ["bf16", "f32"])
 def test_masked_forward_and_backward(ctx, shape, storage):
