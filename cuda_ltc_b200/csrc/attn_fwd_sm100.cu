@@ -737,10 +737,13 @@ attn_fwd_tile_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
                 for (int i = 0; i < 4; ++i) mx[i] = fmax3(mx[i], S_(c + 2 * i), S_(c + 2 * i + 1));
             float mt = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
             if constexpr (kRS > 1) {
-                // (behind this meeting both halves of S are in registers: P may overwrite them)
+                // Behind this meeting both halves of S are in registers: P may overwrite them.  The columns that this warp
+                // writes were read by the row's other warp, hence the fences of a hand-over of tensor memory.
                 *xslot(j & 1, half) = mt;
+                tc_fence_before_sync();
                 ok = meet();
                 if (!ok) break;
+                tc_fence_after_sync();
                 mt = fmaxf(mt, *xslot(j & 1, half ^ 1));
             }
             // lazy rescale, as in the kernels above

@@ -77,3 +77,12 @@ def test_waiting_kernels_touch_no_kernel_argument_memory_before_the_wait():
                 continue
             before = body[:k]
             assert not re.search(r"\ba\.\w+\[|\bg\.\w+\[[^\]]*\]\s*[^;=]*;|__ldg\(|atomic\w+\(", before), name
+
+
+def test_columns_that_two_warps_share_are_handed_over_with_fences():
+    """The wider forward tile: P overwrites score columns that the row's other warp has loaded, so the meeting of the two
+    lies between the two halves of a tensor-memory hand-over."""
+    body = _kernel_bodies(_sources()["attn_fwd_sm100.cu"])["attn_fwd_tile_sm100_kernel"]
+    steps = body[body.index("*xslot(j & 1, half) = mt;"):]
+    order = [steps.index(s) for s in ("tc_fence_before_sync()", "meet()", "tc_fence_after_sync()", "tmem_st16(tP")]
+    assert order == sorted(order)
