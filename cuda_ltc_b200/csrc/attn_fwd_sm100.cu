@@ -547,6 +547,14 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
 //   - of the last four warps one issues the contractions and one is the TMA producer (the others complete the
 //     warpgroup that gives registers up);
 //   - the result leaves through the Q slot (fp32: and the ring) and a TMA store.
+//
+// kTeams > 1 is the form for a context whose SMs are limited (ltca_ctx_set_sm_limit): CTAs of a tile each settle on every
+// SM that has room, so there one CTA per SM holds the same number of tiles side by side, a team of warps each with its own
+// ring, barriers and accumulators, and the teams take tiles from a counter until there are none left.  A tile's
+// arithmetic, and with it every bit of the result, is that of the plain form; a team waits for its slowest warp between
+// tiles and loads nothing of the next tile before that.  On 16 SMs B8 H16 S4096 causal takes 4.00 ms, 434 us scaled to 148,
+// where the plain form takes 396 there (four tiles that start together stay in step); on 132 SMs 516 us, B8 H16 S1024
+// causal 56, B64 H8 S512 causal 61.
 // ---------------------------------------------------------------------------------------------
 template <int D>
 struct TileCfg {
@@ -566,20 +574,29 @@ struct TileCfg {
     static constexpr int kXchgOff = kRingOff + kStages * kKvBytes; // row maxima [2 buffers][2 halves][128], row sums [2][128]
     static constexpr int kBarOff = kXchgOff + (kRowSplit > 1 ? 3 * 2 * kBlockM * 4 : 0);
     static constexpr int kNumBars = 1 + 2 * kStages + 3 + 4;       // q_full, kv_full[], kv_empty[], s_full, p_full, staged, pair[4]
-    static constexpr int kMiscOff = kBarOff + kNumBars * 8;
-    static constexpr int kDynBytes = kMiscOff + 16 + 1024;
+    static constexpr int kMiscOff = kBarOff + kNumBars * 8;        // tmem base, abort flag, a team's next tile
+    static constexpr int kDynBytes = kMiscOff + 32 + 1024;
     static_assert(kCtas * (kDynBytes + 1024) <= 228 * 1024, "shared memory");
+    static constexpr int kTeamBytes = (kMiscOff + 32 + 1023) / 1024 * 1024;
+    static constexpr int kTeamsDynBytes = kCtas * kTeamBytes + 1024;
+    static_assert(kTeamsDynBytes <= 227 * 1024, "shared memory");
     static constexpr uint32_t kTmemCols = 2 * D;
 };
 
-template <int D, bool kSplitP, bool kMask>
-__global__ void __launch_bounds__(TileCfg<D>::kThreads, TileCfg<D>::kCtas)
+template <int D, bool kSplitP, bool kMask, int kTeams>
+__global__ void __launch_bounds__(TileCfg<D>::kThreads * kTeams, kTeams > 1 ? 1 : TileCfg<D>::kCtas)
 attn_fwd_tile_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
-                           const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_o, const FwdArgs a) {
+                           const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_o, const FwdArgs a,
+                           const ItemGrid items) {
     using L = TileCfg<D>;
+    // (the teams share the registers and the tensor memory that as many CTAs of the plain form have on an SM)
+    static_assert(kTeams == 1 || kTeams == L::kCtas, "one CTA or an SM's worth of them");
     constexpr int kBN = L::kBN, kRS = L::kRowSplit, kMmaWarp = L::kMathWarps, kTmaWarp = L::kMathWarps + 1;
     extern __shared__ uint8_t smem_raw[];
-    const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    // (through a shuffle: what follows from it is then known to be the same in a whole warp, which the operands of the
+    // tensor-core instructions have to be)
+    const int team = kTeams > 1 ? __shfl_sync(0xffffffffu, (int)threadIdx.x / L::kThreads, 0) : 0, tid = threadIdx.x - team * L::kThreads;
+    const uint32_t smem_cta = (smem_u32(smem_raw) + 1023u) & ~1023u, smem_base = smem_cta + team * L::kTeamBytes;
     uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
     const uint32_t ring = smem_base + L::kRingOff;
     const uint32_t bar_base = smem_base + L::kBarOff;
@@ -588,9 +605,10 @@ attn_fwd_tile_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
     const uint32_t bar_q_full = bar_base, bar_s_full = bar_base + 8u * (1 + 2 * L::kStages), bar_p_full = bar_s_full + 8,
                    bar_staged = bar_s_full + 16, bar_pair0 = bar_s_full + 24;
     volatile uint32_t* misc = reinterpret_cast<volatile uint32_t*>(smem_gen + L::kMiscOff);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    volatile uint32_t* misc_cta = reinterpret_cast<volatile uint32_t*>(smem_raw + (smem_cta - smem_u32(smem_raw)) + L::kMiscOff);
+    const int warp = kTeams > 1 ? __shfl_sync(0xffffffffu, tid >> 5, 0) : tid >> 5, lane = tid & 31;
 
-    if (threadIdx.x == 0) {
+    if (tid == 0) {
         mbar_init(bar_q_full, 1);
         for (int s = 0; s < L::kStages; ++s) { mbar_init(bar_kv_full(s), 1); mbar_init(bar_kv_empty(s), 1); }
         mbar_init(bar_s_full, 1);
@@ -600,78 +618,121 @@ attn_fwd_tile_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
         misc[1] = 0u;
         mbar_fence_init();
     }
-    if (warp == kMmaWarp) { tmem_alloc(smem_u32(const_cast<uint32_t*>(&misc[0])), L::kTmemCols); tmem_relinquish(); }
+    if (warp == kMmaWarp && team == 0) { tmem_alloc(smem_u32(const_cast<uint32_t*>(&misc[0])), kTeams * L::kTmemCols); tmem_relinquish(); }
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
-    const uint32_t tmem_base = misc[0];
+    const uint32_t tmem_base = misc_cta[0] + team * L::kTmemCols;
     const WaitCtx wc{&misc[1], a.status};
     grid_dependency_wait();                    // the operands are complete once the kernel before this one has ended
 
-    int rank, h, b;
-    sched_block(rank, h, b);
-    const int q0 = ((int)gridDim.x - 1 - rank) * kBlockM;          // heavy (late) causal tiles first
-    int kvlen = a.Sk;
-    if (a.kv_len) kvlen = min(max(a.kv_len[b], 0), a.Sk);
-    int lim = kvlen;
-    if (a.causal) lim = min(lim, min(q0 + kBlockM - 1, a.Sq - 1) + a.causal_off + 1);
-    const int n_t = lim > 0 ? (lim + kBN - 1) / kBN : 0;
+    // The tile at hand, and what of this team's barriers and ring went before it: key steps, and tiles with any.
+    int h, b, q0, kvlen, n_t = 0, steps = 0, tiles = 0;
+    bool started = false;
     auto slot_of = [](int e) { return e % L::kStages; };
     auto phase_of = [](int e) { return (uint32_t)((e / L::kStages) & 1); };
+    auto take = [&](int rank, int nblk) {
+        q0 = (nblk - 1 - rank) * kBlockM;      // heavy (late) causal tiles first
+        kvlen = a.Sk;
+        if (a.kv_len) kvlen = min(max(a.kv_len[b], 0), a.Sk);
+        int lim = kvlen;
+        if (a.causal) lim = min(lim, min(q0 + kBlockM - 1, a.Sq - 1) + a.causal_off + 1);
+        n_t = lim > 0 ? (lim + kBN - 1) / kBN : 0;
+    };
+    // Whole-team call: false when there is no further tile (or a wait of this team gave up).
+    auto next_tile = [&]() {
+        int rank;
+        if constexpr (kTeams > 1) {
+            auto team_sync = [&]() {
+                __syncwarp();
+                asm volatile("bar.sync %0, %1;" ::"r"(1 + team), "n"(L::kThreads) : "memory");
+            };
+            steps = (steps + n_t) & 1023;      // (only their place in the ring and their parities matter)
+            tiles = (tiles + (n_t > 0 ? 1 : 0)) & 1;
+            tc_fence_before_sync();
+            team_sync();                       // every warp is done with the tile before
+            if (tid == 0) {
+                // The first tiles are dealt out there and back, so that a CTA gets heavy and light ones; then the counter.
+                const int dealt = team * gridDim.x + ((team & 1) ? gridDim.x - 1 - blockIdx.x : blockIdx.x);
+                int item = items.n_items;
+                if (!misc[1]) item = started ? (int)(kTeams * gridDim.x) + atomicAdd(items.counters, 1) : dealt;
+                started = true;
+                if (item < items.n_items) {
+                    sched_item(items, item, rank, h, b);
+                    take(rank, items.nblk);
+                    misc[3] = (uint32_t)q0; misc[4] = (uint32_t)h; misc[5] = (uint32_t)b;
+                    misc[6] = (uint32_t)kvlen; misc[7] = (uint32_t)n_t;
+                }
+                misc[2] = item < items.n_items ? 1u : 0u;
+            }
+            team_sync();
+            tc_fence_after_sync();
+            if (!misc[2]) return false;
+            q0 = (int)misc[3]; h = (int)misc[4]; b = (int)misc[5]; kvlen = (int)misc[6]; n_t = (int)misc[7];
+        } else {
+            sched_block(rank, h, b);
+            take(rank, (int)gridDim.x);
+        }
+        return true;
+    };
 
     if (warp >= L::kMathWarps) {
         reg_dealloc<L::kCtrlRegs>();
-        if (warp == kTmaWarp && lane == 0 && n_t > 0) {
-            mbar_arrive_expect_tx(bar_q_full, (uint32_t)L::kQBytes);
-            for (int kb = 0; kb < L::kBlocks; ++kb) tma_load_4d(smem_base + kb * (kBlockM * 128), &tmap_q, bar_q_full, kb * 64, q0, h, b);
-            bool ok = true;
-            for (int e = 0; e < 2 * n_t && ok; ++e) {              // K0 V0 K1 V1 ...
-                const int s = slot_of(e);
-                ok = mbar_wait(bar_kv_empty(s), phase_of(e) ^ 1u, wc, 0x50);
-                if (!ok) break;
-                mbar_arrive_expect_tx(bar_kv_full(s), (uint32_t)L::kKvBytes);
-                for (int kb = 0; kb < L::kBlocks; ++kb)
-                    tma_load_4d(ring + s * L::kKvBytes + kb * (kBN * 128), (e & 1) ? &tmap_v : &tmap_k, bar_kv_full(s), kb * 64,
-                                (e >> 1) * kBN, h, b);
+        do {
+            if (!next_tile()) break;
+            const int e0 = 2 * steps;                                  // ring entries that went before
+            if (warp == kTmaWarp && lane == 0 && n_t > 0) {
+                mbar_arrive_expect_tx(bar_q_full, (uint32_t)L::kQBytes);
+                for (int kb = 0; kb < L::kBlocks; ++kb) tma_load_4d(smem_base + kb * (kBlockM * 128), &tmap_q, bar_q_full, kb * 64, q0, h, b);
+                bool ok = true;
+                for (int e = 0; e < 2 * n_t && ok; ++e) {              // K0 V0 K1 V1 ...
+                    const int s = slot_of(e0 + e);
+                    ok = mbar_wait(bar_kv_empty(s), phase_of(e0 + e) ^ 1u, wc, 0x50);
+                    if (!ok) break;
+                    mbar_arrive_expect_tx(bar_kv_full(s), (uint32_t)L::kKvBytes);
+                    for (int kb = 0; kb < L::kBlocks; ++kb)
+                        tma_load_4d(ring + s * L::kKvBytes + kb * (kBN * 128), (e & 1) ? &tmap_v : &tmap_k, bar_kv_full(s), kb * 64,
+                                    (e >> 1) * kBN, h, b);
+                }
+            } else if (warp == kMmaWarp && lane == 0 && n_t > 0) {
+                constexpr uint32_t idesc_qk = make_idesc_bf16(kBlockM, kBN, 0, 0);
+                constexpr uint32_t idesc_pv = make_idesc_bf16(kBlockM, D, 0, 1);
+                const uint32_t q_lo = smem_desc_lo(smem_base, 16), k_lo = smem_desc_lo(ring, 16), v_lo = smem_desc_lo(ring, kBN * 128);
+                auto issue_qk = [&](int s) {
+    #pragma unroll
+                    for (int k = 0; k < D / 16; ++k)
+                        mma_ss_lo(tmem_base, q_lo + (k / 4) * (kBlockM * 8) + (k % 4) * 2,
+                                  k_lo + ((s * L::kKvBytes) >> 4) + (k / 4) * (kBN * 8) + (k % 4) * 2, idesc_qk, k > 0 ? 1u : 0u);
+                };
+                bool ok = mbar_wait(bar_q_full, (uint32_t)(tiles & 1), wc, 0x51) && mbar_wait(bar_kv_full(slot_of(e0)), phase_of(e0), wc, 0x52);
+                if (ok) {
+                    tc_fence_after_sync();
+                    issue_qk(slot_of(e0));
+                    mma_commit(bar_s_full);
+                    mma_commit(bar_kv_empty(slot_of(e0)));
+                }
+                for (int j = 0; j < n_t && ok; ++j) {
+                    const int e_v = e0 + 2 * j + 1, e_k = e0 + 2 * j + 2;
+                    const bool more = j + 1 < n_t;
+                    ok = mbar_wait(bar_kv_full(slot_of(e_v)), phase_of(e_v), wc, 0x53);
+                    if (more) ok = ok && mbar_wait(bar_kv_full(slot_of(e_k)), phase_of(e_k), wc, 0x54);
+                    ok = ok && mbar_wait(bar_p_full, (uint32_t)((steps + j) & 1), wc, 0x55);
+                    if (!ok) break;
+                    tc_fence_after_sync();
+                    const uint32_t vd = v_lo + ((slot_of(e_v) * L::kKvBytes) >> 4);
+    #pragma unroll
+                    for (int t = 0; t < (kSplitP ? 2 : 1); ++t)
+    #pragma unroll
+                        for (int k = 0; k < kBN / 16; ++k)
+                            mma_ts_lo(tmem_base + kBN, tmem_base + (kBN / 2) * t + k * 8, vd + 128 * k, idesc_pv,
+                                      (j > 0 || t > 0 || k > 0) ? 1u : 0u);
+                    if (more) issue_qk(slot_of(e_k));
+                    mma_commit(bar_s_full);                            // S of step j + 1 ready, O holds steps 0 .. j
+                    mma_commit(bar_kv_empty(slot_of(e_v)));
+                    if (more) mma_commit(bar_kv_empty(slot_of(e_k)));
+                }
             }
-        } else if (warp == kMmaWarp && lane == 0 && n_t > 0) {
-            constexpr uint32_t idesc_qk = make_idesc_bf16(kBlockM, kBN, 0, 0);
-            constexpr uint32_t idesc_pv = make_idesc_bf16(kBlockM, D, 0, 1);
-            const uint32_t q_lo = smem_desc_lo(smem_base, 16), k_lo = smem_desc_lo(ring, 16), v_lo = smem_desc_lo(ring, kBN * 128);
-            auto issue_qk = [&](int s) {
-#pragma unroll
-                for (int k = 0; k < D / 16; ++k)
-                    mma_ss_lo(tmem_base, q_lo + (k / 4) * (kBlockM * 8) + (k % 4) * 2,
-                              k_lo + ((s * L::kKvBytes) >> 4) + (k / 4) * (kBN * 8) + (k % 4) * 2, idesc_qk, k > 0 ? 1u : 0u);
-            };
-            bool ok = mbar_wait(bar_q_full, 0, wc, 0x51) && mbar_wait(bar_kv_full(0), 0, wc, 0x52);
-            if (ok) {
-                tc_fence_after_sync();
-                issue_qk(0);
-                mma_commit(bar_s_full);
-                mma_commit(bar_kv_empty(0));
-            }
-            for (int j = 0; j < n_t && ok; ++j) {
-                const int e_v = 2 * j + 1, e_k = 2 * j + 2;
-                const bool more = j + 1 < n_t;
-                ok = mbar_wait(bar_kv_full(slot_of(e_v)), phase_of(e_v), wc, 0x53);
-                if (more) ok = ok && mbar_wait(bar_kv_full(slot_of(e_k)), phase_of(e_k), wc, 0x54);
-                ok = ok && mbar_wait(bar_p_full, (uint32_t)(j & 1), wc, 0x55);
-                if (!ok) break;
-                tc_fence_after_sync();
-                const uint32_t vd = v_lo + ((slot_of(e_v) * L::kKvBytes) >> 4);
-#pragma unroll
-                for (int t = 0; t < (kSplitP ? 2 : 1); ++t)
-#pragma unroll
-                    for (int k = 0; k < kBN / 16; ++k)
-                        mma_ts_lo(tmem_base + kBN, tmem_base + (kBN / 2) * t + k * 8, vd + 128 * k, idesc_pv,
-                                  (j > 0 || t > 0 || k > 0) ? 1u : 0u);
-                if (more) issue_qk(slot_of(e_k));
-                mma_commit(bar_s_full);                            // S of step j + 1 ready, O holds steps 0 .. j
-                mma_commit(bar_kv_empty(slot_of(e_v)));
-                if (more) mma_commit(bar_kv_empty(slot_of(e_k)));
-            }
-        }
+        } while (kTeams > 1);
     } else {
         reg_alloc<L::kMathRegs>();
         const int wq = warp & 3, half = kRS > 1 ? warp >> 2 : 0;
@@ -692,182 +753,191 @@ attn_fwd_tile_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
         };
         const float c2 = a.scale_log2;
         const bool general = kMask || (a.use_clamp != 0);
-        // per row: number of visible keys; per tile: the first step that needs masking at all
-        int lim_row = kvlen, je = n_t;
-        if (a.causal) lim_row = min(lim_row, q0 + row + a.causal_off + 1);
-        if (kvlen % kBN) je = min(je, kvlen / kBN);
-        if (a.causal) {
-            const int v = q0 + a.causal_off - (kBN - 1);           // step j is cut by the diagonal when j * kBN > v
-            je = min(je, v < 0 ? 0 : v / kBN + 1);
-        }
-        float m_run = neg_inf(), l_run = 0.f;
-        bool ok = true;
-        for (int j = 0; j < n_t; ++j) {
-            uint32_t keep[2];                                      // dense mask of this thread's 64 columns
-#pragma unroll
-            for (int w = 0; w < 2; ++w)
-                keep[w] = kMask ? mask_bits_of_queries(a.mask, b, q0 + wq * 32, j * kBN + half * 64 + 32 * w) : ~0u;
-            ok = mbar_wait_warp(bar_s_full, (uint32_t)(j & 1), wc, 0x56);
-            if (!ok) break;
-            tc_fence_after_sync();
-            uint32_t su[64];
-            tmem_ld32(tS, reinterpret_cast<uint32_t(&)[32]>(su[0]));
-            tmem_ld32(tS + 32, reinterpret_cast<uint32_t(&)[32]>(su[32]));
-            tmem_wait_ld();
-#define S_(c) __uint_as_float(su[(c)])
-            const int lim_c = lim_row - j * kBN - half * 64;       // own columns c < lim_c are visible
-            if (general) {
-#pragma unroll
-                for (int c = 0; c < 64; ++c) {
-                    float v = S_(c);
-                    if (a.use_clamp) v = fminf(v, a.clamp_raw);
-                    const bool vis = c < lim_c && (keep[c / 32] >> (c % 32) & 1u);
-                    su[c] = __float_as_uint(vis ? v : neg_inf());
-                }
-            } else if (j >= je) {
-#pragma unroll
-                for (int c = 0; c < 64; ++c) su[c] = (c < lim_c) ? su[c] : 0xff800000u;
+        do {
+            if (!next_tile()) break;
+            const int s_full0 = steps + tiles;                         // score tiles that went before (one more than steps each)
+            // per row: number of visible keys; per tile: the first step that needs masking at all
+            int lim_row = kvlen, je = n_t;
+            if (a.causal) lim_row = min(lim_row, q0 + row + a.causal_off + 1);
+            if (kvlen % kBN) je = min(je, kvlen / kBN);
+            if (a.causal) {
+                const int v = q0 + a.causal_off - (kBN - 1);           // step j is cut by the diagonal when j * kBN > v
+                je = min(je, v < 0 ? 0 : v / kBN + 1);
             }
-            float mx[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) mx[i] = fmaxf(S_(2 * i), S_(2 * i + 1));
-#pragma unroll
-            for (int c = 8; c < 64; c += 8)
-#pragma unroll
-                for (int i = 0; i < 4; ++i) mx[i] = fmax3(mx[i], S_(c + 2 * i), S_(c + 2 * i + 1));
-            float mt = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
-            if constexpr (kRS > 1) {
-                // Behind this meeting both halves of S are in registers: P may overwrite them.  The columns that this warp
-                // writes were read by the row's other warp, hence the fences of a hand-over of tensor memory.
-                *xslot(j & 1, half) = mt;
-                tc_fence_before_sync();
-                ok = meet();
+            float m_run = neg_inf(), l_run = 0.f;
+            bool ok = true;
+            for (int j = 0; j < n_t; ++j) {
+                uint32_t keep[2];                                      // dense mask of this thread's 64 columns
+    #pragma unroll
+                for (int w = 0; w < 2; ++w)
+                    keep[w] = kMask ? mask_bits_of_queries(a.mask, b, q0 + wq * 32, j * kBN + half * 64 + 32 * w) : ~0u;
+                ok = mbar_wait_warp(bar_s_full, (uint32_t)((s_full0 + j) & 1), wc, 0x56);
                 if (!ok) break;
                 tc_fence_after_sync();
-                mt = fmaxf(mt, *xslot(j & 1, half ^ 1));
-            }
-            // lazy rescale, as in the kernels above
-            float factor = 1.0f;
-            bool need = false;
-            if (j == 0) {
-                m_run = mt;
-            } else if ((mt - m_run) * c2 > 8.0f) {
-                factor = fast_exp2((m_run - mt) * c2);
-                m_run = mt;
-                need = true;
-            }
-            if (j > 0 && __any_sync(0xffffffffu, need)) {
-#pragma unroll 1
-                for (int c0 = 0; c0 < 64; c0 += 16) {
-                    uint32_t o[16];
-                    tmem_ld16(tO + c0, o);
-                    tmem_wait_ld();
-#pragma unroll
-                    for (int c = 0; c < 16; ++c) o[c] = __float_as_uint(__uint_as_float(o[c]) * factor);
-                    tmem_st16(tO + c0, o);
-                }
-                l_run *= factor;
-            }
-            const float m_safe = (m_run == neg_inf()) ? 0.f : m_run;
-            const float mneg = -m_safe * c2;
-            float sum0 = 0.f, sum1 = 0.f, sum2 = 0.f, sum3 = 0.f;
-#pragma unroll
-            for (int ch = 0; ch < 2; ++ch) {
-                uint32_t hi[16], lo[16];
-#pragma unroll
-                for (int cc = 0; cc < 32; cc += 4) {
-                    const int c = ch * 32 + cc;
-                    const float p0 = fast_exp2(fmaf(S_(c), c2, mneg));
-                    const float p1 = fast_exp2(fmaf(S_(c + 1), c2, mneg));
-                    const float p2 = fast_exp2(fmaf(S_(c + 2), c2, mneg));
-                    const float p3 = fast_exp2(fmaf(S_(c + 3), c2, mneg));
-                    sum0 += p0; sum1 += p1; sum2 += p2; sum3 += p3;
-                    const uint32_t h01 = pack_bf16x2(p0, p1), h23 = pack_bf16x2(p2, p3);
-                    hi[cc / 2] = h01;
-                    hi[cc / 2 + 1] = h23;
-                    if constexpr (kSplitP) {
-                        lo[cc / 2] = pack_bf16x2(p0 - __uint_as_float(h01 << 16), p1 - __uint_as_float(h01 & 0xffff0000u));
-                        lo[cc / 2 + 1] = pack_bf16x2(p2 - __uint_as_float(h23 << 16), p3 - __uint_as_float(h23 & 0xffff0000u));
-                    }
-                }
-                tmem_st16(tP + ch * 16, hi);                       // P over S (all of S is in registers)
-                if constexpr (kSplitP) tmem_st16(tPlo + ch * 16, lo);
-            }
-            l_run += (sum0 + sum1) + (sum2 + sum3);
-            tmem_wait_st();
-            tc_fence_before_sync();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bar_p_full);
-#undef S_
-        }
-        grid_launch_dependents();
-        const int qi = q0 + row;
-        const int64_t stat = ((int64_t)b * a.H + h) * a.Sq + qi;
-        if (n_t > 0) {
-            if constexpr (kRS > 1) {
-                *xslot(2, half) = l_run;
-                ok = ok && meet();
-                if (ok) l_run += *xslot(2, half ^ 1);
-            }
-            ok = ok && mbar_wait_warp(bar_s_full, (uint32_t)(n_t & 1), wc, 0x57);
-            tc_fence_after_sync();
-            uint32_t o[64];
-            if (ok) {
-                tmem_ld32(tO, reinterpret_cast<uint32_t(&)[32]>(o[0]));
-                tmem_ld32(tO + 32, reinterpret_cast<uint32_t(&)[32]>(o[32]));
+                uint32_t su[64];
+                tmem_ld32(tS, reinterpret_cast<uint32_t(&)[32]>(su[0]));
+                tmem_ld32(tS + 32, reinterpret_cast<uint32_t(&)[32]>(su[32]));
                 tmem_wait_ld();
-            }
-            float inv = 0.f, lse = neg_inf();
-            if (l_run > 0.f) {
-                inv = 1.0f / l_run;
-                lse = m_run * a.scale + __logf(l_run);
-            }
-            if (ok) {
-                // every operand has been read: Q's slot (and the ring) take the result as 128-byte-swizzled boxes
-#pragma unroll
-                for (int v = 0; v < (kSplitP ? 16 : 8); ++v) {
-                    uint4 w;
-                    if constexpr (kSplitP) {
-                        w = make_uint4(__float_as_uint(__uint_as_float(o[4 * v]) * inv), __float_as_uint(__uint_as_float(o[4 * v + 1]) * inv),
-                                       __float_as_uint(__uint_as_float(o[4 * v + 2]) * inv),
-                                       __float_as_uint(__uint_as_float(o[4 * v + 3]) * inv));
-                    } else {
-                        w.x = pack_bf16x2(__uint_as_float(o[8 * v + 0]) * inv, __uint_as_float(o[8 * v + 1]) * inv);
-                        w.y = pack_bf16x2(__uint_as_float(o[8 * v + 2]) * inv, __uint_as_float(o[8 * v + 3]) * inv);
-                        w.z = pack_bf16x2(__uint_as_float(o[8 * v + 4]) * inv, __uint_as_float(o[8 * v + 5]) * inv);
-                        w.w = pack_bf16x2(__uint_as_float(o[8 * v + 6]) * inv, __uint_as_float(o[8 * v + 7]) * inv);
+    #define S_(c) __uint_as_float(su[(c)])
+                const int lim_c = lim_row - j * kBN - half * 64;       // own columns c < lim_c are visible
+                if (general) {
+    #pragma unroll
+                    for (int c = 0; c < 64; ++c) {
+                        float v = S_(c);
+                        if (a.use_clamp) v = fminf(v, a.clamp_raw);
+                        const bool vis = c < lim_c && (keep[c / 32] >> (c % 32) & 1u);
+                        su[c] = __float_as_uint(vis ? v : neg_inf());
                     }
-                    const int box = half * (kSplitP ? 2 : 1) + v / 8;
-                    *reinterpret_cast<uint4*>(smem_gen + box * (kBlockM * 128) + row * 128 + (((v % 8) ^ (row & 7)) << 4)) = w;
+                } else if (j >= je) {
+    #pragma unroll
+                    for (int c = 0; c < 64; ++c) su[c] = (c < lim_c) ? su[c] : 0xff800000u;
                 }
-                fence_proxy_async_smem();
+                float mx[4];
+    #pragma unroll
+                for (int i = 0; i < 4; ++i) mx[i] = fmaxf(S_(2 * i), S_(2 * i + 1));
+    #pragma unroll
+                for (int c = 8; c < 64; c += 8)
+    #pragma unroll
+                    for (int i = 0; i < 4; ++i) mx[i] = fmax3(mx[i], S_(c + 2 * i), S_(c + 2 * i + 1));
+                float mt = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+                if constexpr (kRS > 1) {
+                    // Behind this meeting both halves of S are in registers: P may overwrite them.  The columns that this warp
+                    // writes were read by the row's other warp, hence the fences of a hand-over of tensor memory.
+                    *xslot(j & 1, half) = mt;
+                    tc_fence_before_sync();
+                    ok = meet();
+                    if (!ok) break;
+                    tc_fence_after_sync();
+                    mt = fmaxf(mt, *xslot(j & 1, half ^ 1));
+                }
+                // lazy rescale, as in the kernels above
+                float factor = 1.0f;
+                bool need = false;
+                if (j == 0) {
+                    m_run = mt;
+                } else if ((mt - m_run) * c2 > 8.0f) {
+                    factor = fast_exp2((m_run - mt) * c2);
+                    m_run = mt;
+                    need = true;
+                }
+                if (j > 0 && __any_sync(0xffffffffu, need)) {
+    #pragma unroll 1
+                    for (int c0 = 0; c0 < 64; c0 += 16) {
+                        uint32_t o[16];
+                        tmem_ld16(tO + c0, o);
+                        tmem_wait_ld();
+    #pragma unroll
+                        for (int c = 0; c < 16; ++c) o[c] = __float_as_uint(__uint_as_float(o[c]) * factor);
+                        tmem_st16(tO + c0, o);
+                    }
+                    l_run *= factor;
+                }
+                const float m_safe = (m_run == neg_inf()) ? 0.f : m_run;
+                const float mneg = -m_safe * c2;
+                float sum0 = 0.f, sum1 = 0.f, sum2 = 0.f, sum3 = 0.f;
+    #pragma unroll
+                for (int ch = 0; ch < 2; ++ch) {
+                    uint32_t hi[16], lo[16];
+    #pragma unroll
+                    for (int cc = 0; cc < 32; cc += 4) {
+                        const int c = ch * 32 + cc;
+                        const float p0 = fast_exp2(fmaf(S_(c), c2, mneg));
+                        const float p1 = fast_exp2(fmaf(S_(c + 1), c2, mneg));
+                        const float p2 = fast_exp2(fmaf(S_(c + 2), c2, mneg));
+                        const float p3 = fast_exp2(fmaf(S_(c + 3), c2, mneg));
+                        sum0 += p0; sum1 += p1; sum2 += p2; sum3 += p3;
+                        const uint32_t h01 = pack_bf16x2(p0, p1), h23 = pack_bf16x2(p2, p3);
+                        hi[cc / 2] = h01;
+                        hi[cc / 2 + 1] = h23;
+                        if constexpr (kSplitP) {
+                            lo[cc / 2] = pack_bf16x2(p0 - __uint_as_float(h01 << 16), p1 - __uint_as_float(h01 & 0xffff0000u));
+                            lo[cc / 2 + 1] = pack_bf16x2(p2 - __uint_as_float(h23 << 16), p3 - __uint_as_float(h23 & 0xffff0000u));
+                        }
+                    }
+                    tmem_st16(tP + ch * 16, hi);                       // P over S (all of S is in registers)
+                    if constexpr (kSplitP) tmem_st16(tPlo + ch * 16, lo);
+                }
+                l_run += (sum0 + sum1) + (sum2 + sum3);
+                tmem_wait_st();
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_p_full);
+    #undef S_
             }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bar_staged);
-            if (half == 0 && a.lse && qi < a.Sq) a.lse[stat] = lse;
-            if (warp == 0 && lane == 0 && ok && mbar_wait(bar_staged, 0, wc, 0x58)) {
-                constexpr int kCols = kSplitP ? 32 : 64;           // of a 128-byte box
-                for (int i = 0; i < D / kCols; ++i) tma_store_4d(&tmap_o, smem_base + i * (kBlockM * 128), i * kCols, q0, h, b);
-                tma_store_commit();
-                tma_store_wait_read<0>();
+            if constexpr (kTeams == 1) grid_launch_dependents();
+            const int qi = q0 + row;
+            const int64_t stat = ((int64_t)b * a.H + h) * a.Sq + qi;
+            if (n_t > 0) {
+                if constexpr (kRS > 1) {
+                    *xslot(2, half) = l_run;
+                    ok = ok && meet();
+                    if (ok) l_run += *xslot(2, half ^ 1);
+                }
+                ok = ok && mbar_wait_warp(bar_s_full, (uint32_t)((s_full0 + n_t) & 1), wc, 0x57);
+                tc_fence_after_sync();
+                float inv = 0.f, lse = neg_inf();
+                if (l_run > 0.f) {
+                    inv = 1.0f / l_run;
+                    lse = m_run * a.scale + __logf(l_run);
+                }
+                if (ok) {
+                    uint32_t o[64];
+                    tmem_ld32(tO, reinterpret_cast<uint32_t(&)[32]>(o[0]));
+                    tmem_ld32(tO + 32, reinterpret_cast<uint32_t(&)[32]>(o[32]));
+                    tmem_wait_ld();
+                    // every operand has been read: Q's slot (and the ring) take the result as 128-byte-swizzled boxes
+    #pragma unroll
+                    for (int v = 0; v < (kSplitP ? 16 : 8); ++v) {
+                        uint4 w;
+                        if constexpr (kSplitP) {
+                            w = make_uint4(__float_as_uint(__uint_as_float(o[4 * v]) * inv), __float_as_uint(__uint_as_float(o[4 * v + 1]) * inv),
+                                           __float_as_uint(__uint_as_float(o[4 * v + 2]) * inv),
+                                           __float_as_uint(__uint_as_float(o[4 * v + 3]) * inv));
+                        } else {
+                            w.x = pack_bf16x2(__uint_as_float(o[8 * v + 0]) * inv, __uint_as_float(o[8 * v + 1]) * inv);
+                            w.y = pack_bf16x2(__uint_as_float(o[8 * v + 2]) * inv, __uint_as_float(o[8 * v + 3]) * inv);
+                            w.z = pack_bf16x2(__uint_as_float(o[8 * v + 4]) * inv, __uint_as_float(o[8 * v + 5]) * inv);
+                            w.w = pack_bf16x2(__uint_as_float(o[8 * v + 6]) * inv, __uint_as_float(o[8 * v + 7]) * inv);
+                        }
+                        const int box = half * (kSplitP ? 2 : 1) + v / 8;
+                        *reinterpret_cast<uint4*>(smem_gen + box * (kBlockM * 128) + row * 128 + (((v % 8) ^ (row & 7)) << 4)) = w;
+                    }
+                    fence_proxy_async_smem();
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_staged);
+                if (half == 0 && a.lse && qi < a.Sq) a.lse[stat] = lse;
+                if (warp == 0 && lane == 0 && ok && mbar_wait(bar_staged, (uint32_t)(tiles & 1), wc, 0x58)) {
+                    constexpr int kCols = kSplitP ? 32 : 64;           // of a 128-byte box
+                    for (int i = 0; i < D / kCols; ++i) tma_store_4d(&tmap_o, smem_base + i * (kBlockM * 128), i * kCols, q0, h, b);
+                    tma_store_commit();
+                    tma_store_wait_read<0>();
+                }
+            } else if (qi < a.Sq) {
+                // no key is visible to these rows: zeros and -inf
+                using OutT = typename std::conditional<kSplitP, float, __nv_bfloat16>::type;
+                uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<OutT*>(a.o) + b * a.o_sb + h * a.o_sh + (int64_t)qi * a.o_ss +
+                                                      half * 64);
+    #pragma unroll
+                for (int v = 0; v < (kSplitP ? 16 : 8); ++v) dst[v] = make_uint4(0u, 0u, 0u, 0u);
+                if (half == 0 && a.lse) a.lse[stat] = neg_inf();
             }
-        } else if (qi < a.Sq) {
-            // no key is visible to these rows: zeros and -inf
-            using OutT = typename std::conditional<kSplitP, float, __nv_bfloat16>::type;
-            uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<OutT*>(a.o) + b * a.o_sb + h * a.o_sh + (int64_t)qi * a.o_ss +
-                                                  half * 64);
-#pragma unroll
-            for (int v = 0; v < (kSplitP ? 16 : 8); ++v) dst[v] = make_uint4(0u, 0u, 0u, 0u);
-            if (half == 0 && a.lse) a.lse[stat] = neg_inf();
-        }
+        } while (kTeams > 1);
     }
     tc_fence_before_sync();
-    __syncthreads();
-    if (warp == kMmaWarp) {
+    bool gave_up;
+    if constexpr (kTeams > 1) {
+        gave_up = __syncthreads_or(misc[1] != 0);
+        if (threadIdx.x == 0) item_counters_release(items.counters);
+    } else {
+        __syncthreads();
+        gave_up = misc[1] != 0;
+    }
+    if (warp == kMmaWarp && team == 0) {
         __syncwarp();
-        if (misc[1]) __nanosleep(200000);    // aborted: give copies and MMAs in flight time to land
+        if (gave_up) __nanosleep(200000);    // aborted: give copies and MMAs in flight time to land
         tc_fence_after_sync();
-        tmem_dealloc(tmem_base, L::kTmemCols);
+        tmem_dealloc(tmem_base, kTeams * L::kTmemCols);
     }
 }
 
@@ -881,11 +951,31 @@ int launch_fwd_tile(ltca_ctx* ctx, const ltca_attn_params* p, const void* q, con
     if ((rc = make_tmap_bhsd(ctx, &tk, k, 2, p->B, p->H, p->Sk, D, ks, 64, L::kBN))) return rc;
     if ((rc = make_tmap_bhsd(ctx, &tv, v, 2, p->B, p->H, p->Sk, D, vs, 64, L::kBN))) return rc;
     if ((rc = make_tmap_bhsd(ctx, &to, p->o, kSplitP ? 4 : 2, p->B, p->H, p->Sq, D, p->o_strides, kSplitP ? 32 : 64, kBlockM))) return rc;
-    auto kern = p->keep_mask ? attn_fwd_tile_sm100_kernel<D, kSplitP, true> : attn_fwd_tile_sm100_kernel<D, kSplitP, false>;
+    ItemGrid items;
+    memset(&items, 0, sizeof(items));
+    // bf16 results at head_dim 64 keep to the SMs that the context allows: what a sequence-sharded run computes while slices
+    // are on their way between the GPUs.
+    if constexpr (D == 64 && !kSplitP) {
+        items.nblk = (p->Sq + kBlockM - 1) / kBlockM;
+        items.H = p->H;
+        items.BH = p->B * p->H;
+        const int64_t n = (int64_t)items.nblk * items.BH, ctas = (n + L::kCtas - 1) / L::kCtas;
+        if (ctx->sm_count < ctx->sm_device && n <= 0x7fffffff - 2ll * L::kCtas * ctx->sm_device) {
+            items.n_items = (int)n;
+            items.counters = ctx->d_sched + 6;        // ints 6,7: the forward's
+            auto kern = p->keep_mask ? attn_fwd_tile_sm100_kernel<D, kSplitP, true, L::kCtas> : attn_fwd_tile_sm100_kernel<D, kSplitP, false, L::kCtas>;
+            static SmemOptIn opt_in[2];
+            LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(opt_in[p->keep_mask ? 1 : 0], ctx->device, kern, L::kTeamsDynBytes));
+            LTCA_CUDA_OK(ctx, launch_dependent_if(small_attention_call(p), kern, dim3((unsigned)(ctas < ctx->sm_count ? ctas : ctx->sm_count)),
+                                                  dim3(L::kThreads * L::kCtas), L::kTeamsDynBytes, ctx->stream, tq, tk, tv, to, a, items));
+            return LTCA_OK;
+        }
+    }
+    auto kern = p->keep_mask ? attn_fwd_tile_sm100_kernel<D, kSplitP, true, 1> : attn_fwd_tile_sm100_kernel<D, kSplitP, false, 1>;
     static SmemOptIn opt_in[2];
     LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(opt_in[p->keep_mask ? 1 : 0], ctx->device, kern, L::kDynBytes));
     dim3 grid((p->Sq + kBlockM - 1) / kBlockM, p->H, p->B);
-    LTCA_CUDA_OK(ctx, launch_dependent_if(small_attention_call(p), kern, grid, dim3(L::kThreads), L::kDynBytes, ctx->stream, tq, tk, tv, to, a));
+    LTCA_CUDA_OK(ctx, launch_dependent_if(small_attention_call(p), kern, grid, dim3(L::kThreads), L::kDynBytes, ctx->stream, tq, tk, tv, to, a, items));
     return LTCA_OK;
 }
 

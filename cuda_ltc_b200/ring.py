@@ -82,9 +82,10 @@ class CudaOps:
     """The steps' arithmetic on this library's kernels (``Context``); raises if the library is missing."""
 
     def __init__(self, ctx, scale=None, mode=None, comm_sms=16):
-        """``comm_sms``: SMs left free while slices are in flight.  The attention kernels are persistent (one
-        CTA per SM for the whole launch), so without free SMs the communication library's copy kernels would
-        only start when an attention kernel ends and the exchange would not overlap the arithmetic."""
+        """``comm_sms``: SMs left free while slices are in flight.  The attention kernels fill every SM, the backward
+        for the whole launch and the forward until its last tile is placed, so without free SMs the communication
+        library's copy kernels would only start when an attention kernel ends and the exchange would not overlap the
+        arithmetic.  (Under the limit the bf16 forward at head_dim 64 keeps to the SMs it is given, as the backward does.)"""
         from . import _lib
         self.ctx, self.scale, self.comm_sms = ctx, scale, comm_sms
         self.mode = _lib.MODE_AUTO if mode is None else mode

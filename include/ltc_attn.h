@@ -157,10 +157,12 @@ int ltca_device_status(ltca_ctx* ctx, uint32_t* status_out);
  * The kernel returns on its own; ltca_device_status then reports LTCA_ERR_DEVICE with the time-out bit
  * (status & 1) and barrier code 0x7f in bits 8..23, and the context stays usable. */
 int ltca_selftest_bounded_wait(ltca_ctx* ctx, uint32_t limit_us);
-/* The persistent kernels of this context launch one CTA per SM; n_sms caps that number so that other work
- * on the GPU (a communication library's copy kernels while slices are exchanged between GPUs) finds free SMs
- * at once instead of waiting for a whole kernel to end.  n_sms <= 0 or above the device's count restores the
- * default (all SMs).  Takes effect from the next launch. */
+/* The persistent kernels of this context (tensor-pipe products, bf16 backward) launch one CTA per SM; n_sms caps that
+ * number so that other work on the GPU (a communication library's copy kernels while slices are exchanged between
+ * GPUs) finds free SMs at once instead of waiting for a whole kernel to end.  Under a cap the forward with bf16
+ * storage at head_dim 64 keeps to as many SMs too (except calls of so few tiles that they are one wave anyway), with
+ * the same results; the remaining kernels are short and take no notice of it.  n_sms <= 0 or above the device's count
+ * restores the default (all SMs).  Takes effect from the next launch. */
 int ltca_ctx_set_sm_limit(ltca_ctx* ctx, int32_t n_sms);
 
 /* ---- attention core --------------------------------------------------------------------- */

@@ -478,7 +478,7 @@ def test_sm_limit_changes_the_launch_width_not_the_results(ctx):
     must leave forward and backward results bit-identical; 0 restores the default."""
     import torch
     g = torch.Generator(device="cuda").manual_seed(4)
-    # (4 x 40 pairs of 512 queries: 160 work items of the persistent forward kernel, more than there are SMs)
+    # (4 x 40 pairs of 512 queries: 640 tiles, more than the forward's teams on the allowed SMs)
     q, k, v, do = ((torch.randn((4, 40, 512, 64), generator=g, device="cuda") * 0.5).bfloat16() for _ in range(4))
     o, lse = ctx.attn_fwd(q, k, v, causal=True)
     grads = ctx.attn_bwd(q, k, v, o, lse, do, causal=True, deterministic=True)

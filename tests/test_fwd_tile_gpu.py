@@ -42,3 +42,57 @@ def test_forward_tiles(ctx, case, storage, D):
     fin, got = np.isfinite(lse_ref), lse.cpu().numpy()
     assert (np.isfinite(got) == fin).all()
     assert max_abs(got[fin], lse_ref[fin]) < 2e-3
+
+
+LIMIT_CASES = [
+    # B, H, Sq, Sk, causal, lengths, mask
+    (1, 1, 1, 1, False, False, False),          # fewer tiles than one CTA has teams
+    (3, 67, 260, 200, True, True, False),       # 603 tiles, some without keys, odd numbers of key steps
+    (2, 40, 515, 515, True, False, True),
+]
+
+
+@pytest.mark.parametrize("n_sms", [1, 100])
+@pytest.mark.parametrize("case", LIMIT_CASES)
+def test_forward_under_an_sm_limit_has_the_same_bits(ctx, case, n_sms):
+    B, H, Sq, Sk, causal, use_len, use_mask = case
+    q, k, v = (torch.from_numpy(randn((B, H, n, 64), 60 + i, 0.5)).cuda().bfloat16() for i, n in enumerate((Sq, Sk, Sk)))
+    kw = dict(causal=causal, mode=_lib.MODE_BF16)
+    if use_len:
+        kw["kv_len"] = torch.tensor([(0, Sk // 2 + 1, Sk)[i % 3] for i in range(B)], dtype=torch.int32, device="cuda")
+    if use_mask:
+        kw.update(keep_mask=(torch.rand((B, Sq, Sk), device="cuda") > 0.2).float(), score_clamp=1.0)
+    want = ctx.attn_fwd(q, k, v, **kw)
+    try:
+        ctx.set_sm_limit(n_sms)
+        got = [ctx.attn_fwd(q, k, v, **kw) for _ in range(2)]      # (twice: the tile counter is back at zero)
+    finally:
+        ctx.set_sm_limit(0)
+    torch.cuda.synchronize()
+    assert ctx.device_status() == 0
+    for o, lse in got:
+        assert torch.equal(o, want[0]) and torch.equal(lse, want[1])
+
+
+def test_forward_keeps_to_the_sm_limit(ctx):
+    """On an eighteenth of the SMs a call that fills the GPU many times over takes far longer."""
+    q, k, v = ((torch.randn((4, 40, 1024, 64), device="cuda") * 0.5).bfloat16() for _ in range(3))
+
+    def best():
+        times = []
+        for _ in range(5):
+            a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            a.record()
+            ctx.attn_fwd(q, k, v, mode=_lib.MODE_BF16)
+            b.record()
+            b.synchronize()
+            times.append(a.elapsed_time(b))
+        return min(times)
+
+    free = best()
+    try:
+        ctx.set_sm_limit(8)
+        held = best()
+    finally:
+        ctx.set_sm_limit(0)
+    assert held > 4 * free, (held, free)
