@@ -36,7 +36,7 @@ struct CoreArgs {
     float* delta;
     const float* keep_mask;
     const int32_t* kv_len;
-    const uint32_t* mask_bits;  // backward: the dense mask packed, [B, Sq, mask_nw]
+    const uint32_t* mask_bits;  // backward: the dense mask packed, [B, Sq, mask_nw]; null: no room for it
     int mask_nw;
     int vec;            // every row starts on a 16-byte (fp32) or 8-byte (bf16) boundary and holds a multiple of 4 elements
 };
@@ -106,6 +106,23 @@ __device__ __forceinline__ void store4(T* row, int d, int D, float4 v, bool vec)
         if (d + 2 < D) st_elem(row + d + 2, v.z);
         if (d + 3 < D) st_elem(row + d + 3, v.w);
     }
+}
+
+// How the backward kernels meet a dense mask: not at all, as packed words, or (a workspace sized without the mask has no room
+// for the words) as it is.
+constexpr int kNoMask = 0, kWords = 1, kDense = 2;
+// Word w of query qi's row: bit c = key 32 w + c is kept; 0 beyond the tensor.
+template <int kMask>
+__device__ __forceinline__ uint32_t mask_word(const CoreArgs& a, int b, int qi, int w) {
+    if (qi >= a.Sq || w >= a.mask_nw) return 0u;
+    const int64_t row = (int64_t)b * a.Sq + qi;
+    if constexpr (kMask == kWords) return a.mask_bits[row * a.mask_nw + w];
+    const float* m = a.keep_mask + row * a.Sk + 32 * w;
+    const int n = min(32, a.Sk - 32 * w);
+    uint32_t bits = 0;
+#pragma unroll 1
+    for (int c = 0; c < n; ++c) bits |= (__ldg(m + c) != 0.f ? 1u : 0u) << c;
+    return bits;
 }
 
 __device__ __forceinline__ bool key_visible(const CoreArgs& a, int b, int qi, int kj, int kvlen) {
@@ -465,7 +482,7 @@ __global__ void attn_bwd_delta_kernel(const CoreArgs a) {
 // backward
 // ----------------------------------------------------------------------------------------------
 // pass 1: delta = rowsum(dO o O), left for pass 2, and dQ.  One CTA per TM query rows, KN keys per step.
-template <typename T, int DP, int TM, int KN, int NT, bool kMask>
+template <typename T, int DP, int TM, int KN, int NT, int kMask>
 __global__ void __launch_bounds__(NT, NT == 128 ? 3 : 1) attn_bwd_dq_fp32_kernel(const CoreArgs a) {
     grid_dependency_wait();
     constexpr int LD = DP + kPad, LP = KN + kPad, RS = NT / 16, RM = TM / RS, CN = KN / 16, NW = KN / 32;
@@ -545,7 +562,7 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 3 : 1) attn_bwd_dq_fp32_kernel
 #pragma unroll
                 for (int w = 0; w < NW; ++w) {
                     const int qi = q0 + row0 + RS * i, kw = k0 / 32 + w;
-                    words[i][w] = (qi < a.Sq && kw < a.mask_nw) ? a.mask_bits[((int64_t)b * a.Sq + qi) * a.mask_nw + kw] : 0u;
+                    words[i][w] = mask_word<kMask>(a, b, qi, kw);
                 }
         }
         float s[RM][CN], dp[RM][CN];
@@ -595,7 +612,7 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 3 : 1) attn_bwd_dq_fp32_kernel
 }
 
 // pass 2: dK and dV.  One CTA per TK keys, QN query rows per step; a thread accumulates NR neighbouring keys.
-template <typename T, int DP, int TK, int QN, int NT, bool kMask>
+template <typename T, int DP, int TK, int QN, int NT, int kMask>
 __global__ void __launch_bounds__(NT, TK < 64 ? 3 : DP <= 32 ? 3 : DP <= 64 ? 2 : 1) attn_bwd_dkv_fp32_kernel(const CoreArgs a) {
     grid_dependency_wait();
     constexpr int LD = DP + kPad, LP = TK + kPad, RS = NT / 16, RM = QN / RS, CN = TK / 16, NW = (TK + 31) / 32;
@@ -654,7 +671,7 @@ __global__ void __launch_bounds__(NT, TK < 64 ? 3 : DP <= 32 ? 3 : DP <= 64 ? 2 
 #pragma unroll
                 for (int w = 0; w < NW; ++w) {
                     const int qi = q0 + row0 + RS * i, kw = k0 / 32 + w;
-                    uint32_t x = (qi < a.Sq && kw < a.mask_nw) ? a.mask_bits[((int64_t)b * a.Sq + qi) * a.mask_nw + kw] : 0u;
+                    const uint32_t x = mask_word<kMask>(a, b, qi, kw);
                     words[i][w] = TK < 32 ? x >> (k0 % 32) : x;
                 }
         }
@@ -773,7 +790,7 @@ int run_fwd(ltca_ctx* ctx, const CoreArgs& a) {
     return LTCA_OK;
 }
 
-template <typename T, int DP, int TM, int KN, int NT, bool kMask>
+template <typename T, int DP, int TM, int KN, int NT, int kMask>
 int run_dq(ltca_ctx* ctx, const CoreArgs& a) {
     static SmemOptIn once;
     constexpr size_t smem = ((size_t)(2 * TM + 2 * KN) * (DP + kPad) + TM * (KN + kPad) + TM) * sizeof(float);
@@ -783,7 +800,7 @@ int run_dq(ltca_ctx* ctx, const CoreArgs& a) {
     LTCA_CUDA_OK(ctx, launch_dependent(attn_bwd_dq_fp32_kernel<T, DP, TM, KN, NT, kMask>, grid, dim3(NT), smem, ctx->stream, a));
     return LTCA_OK;
 }
-template <typename T, int DP, int TK, int QN, int NT, bool kMask>
+template <typename T, int DP, int TK, int QN, int NT, int kMask>
 int run_dkv(ltca_ctx* ctx, const CoreArgs& a) {
     static SmemOptIn once;
     constexpr size_t smem = ((size_t)(2 * TK + 2 * QN) * (DP + kPad) + 2 * QN * (TK + kPad) + 2 * QN) * sizeof(float);
@@ -805,8 +822,13 @@ int run_rows(ltca_ctx* ctx, const CoreArgs& a, bool bwd) {
     constexpr int NT = DP > 64 ? 256 : 128;         // at DP = 128 eight columns per thread need the wider CTA
     if (!bwd) return fills(a.Sq) ? run_fwd<T, DP, 64, NT, kMask>(ctx, a) : run_fwd<T, DP, 16, 128, kMask>(ctx, a);
     int rc;
-    if ((rc = fills(a.Sq) ? run_dq<T, DP, 64, 64, NT, kMask>(ctx, a) : run_dq<T, DP, 16, 32, 128, kMask>(ctx, a))) return rc;
-    return fills(a.Sk) ? run_dkv<T, DP, 64, 64, NT, kMask>(ctx, a) : run_dkv<T, DP, 16, 32, 128, kMask>(ctx, a);
+    if constexpr (kMask) {
+        // without room for the mask's words: the small tiles alone, whose results have the same bits
+        if (!a.mask_bits) return (rc = run_dq<T, DP, 16, 32, 128, kDense>(ctx, a)) ? rc : run_dkv<T, DP, 16, 32, 128, kDense>(ctx, a);
+    }
+    constexpr int kM = kMask ? kWords : kNoMask;
+    if ((rc = fills(a.Sq) ? run_dq<T, DP, 64, 64, NT, kM>(ctx, a) : run_dq<T, DP, 16, 32, 128, kM>(ctx, a))) return rc;
+    return fills(a.Sk) ? run_dkv<T, DP, 64, 64, NT, kM>(ctx, a) : run_dkv<T, DP, 16, 32, 128, kM>(ctx, a);
 }
 template <typename T, int DP>
 int run_rows(ltca_ctx* ctx, const CoreArgs& a, bool bwd) {
@@ -1035,9 +1057,8 @@ int launch_attn_fwd_fp32(ltca_ctx* ctx, const ltca_attn_params* p) {
 int launch_attn_bwd_fp32(ltca_ctx* ctx, const ltca_attn_params* p) {
     if (p->D < 1 || p->D > kWideMaxD)
         return fail(ctx, LTCA_ERR_UNSUPPORTED, "fp32 attention supports head_dim 1..%d, got %d", kWideMaxD, p->D);
-    if (p->workspace_bytes < attn_bwd_fp32_workspace(p) || !p->workspace)
-        return fail(ctx, LTCA_ERR_WORKSPACE, "backward needs %zu bytes of workspace",
-                    attn_bwd_fp32_workspace(p));
+    if (p->workspace_bytes < delta_bytes(p) || !p->workspace)
+        return fail(ctx, LTCA_ERR_WORKSPACE, "backward needs %zu bytes of workspace", delta_bytes(p));
     CoreArgs a = make_args(p);
     a.delta = reinterpret_cast<float*>(p->workspace);
     if (p->D <= 128) {

@@ -728,6 +728,15 @@ void fill_wide(const ltca_tsa_params* t, const TBufs& tb, WideArgs* w) {
 // The attention scratch (TBufs::rest) of a call whose buffers start at w; not on the written-out-score path.
 char* scratch_of(const ltca_tsa_params* t, const TPlan& pl, char* w) { return t->saved ? w : w + tensor_saved_bytes(pl); }
 
+// The call as its workspace is laid out.  Packed mask words are part of what ltca_tsa_workspace_bytes asks for, but a
+// workspace that was sized without the mask is laid out without them: the attention kernels then read the dense values.
+ltca_tsa_params laid_out(const ltca_tsa_params* t, int which) {
+    ltca_tsa_params l = *t;
+    size_t need = 0;
+    if (l.keep_mask && (ltca_tsa_workspace_bytes(&l, which, &need) || l.workspace_bytes < need)) l.keep_mask = nullptr;
+    return l;
+}
+
 // What a module call tells its kernels through the context, taken back when the call returns.
 struct CallHints {
     ltca_ctx* ctx;
@@ -902,7 +911,8 @@ int tensor_forward_core(ltca_ctx* ctx, const ltca_tsa_params* t, const TPlan& pl
 int tensor_forward(ltca_ctx* ctx, const ltca_tsa_params* t, const ltca_tsa_params* outer, bool fused) {
     TPlan pl;
     int rc;
-    if ((rc = make_tplan(t, &pl, keeps_for_backward(t)))) return rc;
+    const ltca_tsa_params layout = laid_out(t, 0);
+    if ((rc = make_tplan(&layout, &pl, keeps_for_backward(t)))) return rc;
     const size_t need = tensor_workspace(pl, 0);
     if (!t->workspace || t->workspace_bytes < need)
         return fail(ctx, LTCA_ERR_WORKSPACE, "forward needs %zu bytes of workspace", need);
@@ -911,7 +921,7 @@ int tensor_forward(ltca_ctx* ctx, const ltca_tsa_params* t, const ltca_tsa_param
     w += pl.y;
     TBufs tb;
     CallHints hints{ctx};
-    if (fused && (rc = place_mask_words(ctx, t, pl, scratch_of(t, pl, w), pl.attn_fwd, true))) return rc;
+    if (fused && (rc = place_mask_words(ctx, &layout, pl, scratch_of(t, pl, w), pl.attn_fwd, true))) return rc;
     if ((rc = tensor_forward_core(ctx, t, pl, w, &tb, 0, nullptr, nullptr, nullptr, fused ? outer : nullptr))) return rc;
     GemmProblem gp;
     gp.M = (int)pl.rows; gp.N = t->E; gp.K = pl.HW;
@@ -929,7 +939,8 @@ int tensor_backward(ltca_ctx* ctx, const ltca_tsa_params* t, bool want_dx, bool 
                     const ltca_tsa_params* outer, float* outer_g) {
     TPlan pl;
     int rc;
-    if ((rc = make_tplan(t, &pl, true))) return rc;
+    const ltca_tsa_params layout = laid_out(t, 1);
+    if ((rc = make_tplan(&layout, &pl, true))) return rc;
     const size_t need = tensor_workspace(pl, 1);
     if (!t->workspace || t->workspace_bytes < need)
         return fail(ctx, LTCA_ERR_WORKSPACE, "backward needs %zu bytes of workspace", need);
@@ -947,7 +958,7 @@ int tensor_backward(ltca_ctx* ctx, const ltca_tsa_params* t, bool want_dx, bool 
     CallHints hints{ctx};
     ctx->fwd_pairs = t->bk != nullptr;
     const size_t most = pl.attn_fwd > pl.attn_bwd ? pl.attn_fwd : pl.attn_bwd;
-    if ((rc = place_mask_words(ctx, t, pl, scratch_of(t, pl, w), most, outer && !(t->saved && t->reuse_forward)))) return rc;
+    if ((rc = place_mask_words(ctx, &layout, pl, scratch_of(t, pl, w), most, outer && !(t->saved && t->reuse_forward)))) return rc;
     bool dy_done = false;
     if ((rc = tensor_forward_core(ctx, t, pl, w, &tb, 1, t->dy, dyb, &dy_done, outer, outer_g))) return rc;
     const int rows = (int)pl.rows, E = t->E, HW = pl.HW, Ep = pl.Ep;
@@ -1141,7 +1152,8 @@ static bool fuses_prenorm(const ltca_tsa_params* c, bool backward) {
 // FlashAttention form, forward: LayerNorm on the input, the core module, residual with the raw input, dropout.
 static int prenorm_forward(ltca_ctx* ctx, const ltca_tsa_params* t) {
     size_t need = 0;
-    int rc = ltca_tsa_workspace_bytes(t, 0, &need);
+    const ltca_tsa_params layout = laid_out(t, 0);
+    int rc = ltca_tsa_workspace_bytes(&layout, 0, &need);
     if (rc) return rc;
     if (!t->workspace || t->workspace_bytes < need)
         return fail(ctx, LTCA_ERR_WORKSPACE, "forward needs %zu bytes of workspace", need);
@@ -1163,7 +1175,8 @@ static int prenorm_forward(ltca_ctx* ctx, const ltca_tsa_params* t) {
 // FlashAttention form, backward (an extension: the reference class has no backward pass).
 static int prenorm_backward(ltca_ctx* ctx, const ltca_tsa_params* t, bool want_dx, bool want_dw) {
     size_t need = 0;
-    int rc = ltca_tsa_workspace_bytes(t, 1, &need);
+    const ltca_tsa_params layout = laid_out(t, 1);
+    int rc = ltca_tsa_workspace_bytes(&layout, 1, &need);
     if (rc) return rc;
     if (!t->workspace || t->workspace_bytes < need)
         return fail(ctx, LTCA_ERR_WORKSPACE, "backward needs %zu bytes of workspace", need);
@@ -1228,9 +1241,10 @@ static int tsa_forward(ltca_ctx* ctx, const ltca_tsa_params* t, const ltca_tsa_p
     if (t->pre_norm) return prenorm_forward(ctx, t);
     if (use_tensor(t, keeps_for_backward(t))) return tensor_forward(ctx, t, outer, fused);
     Plan pl;
-    if ((rc = make_plan(t, &pl))) return rc;
+    const ltca_tsa_params layout = laid_out(t, 0);
+    if ((rc = make_plan(&layout, &pl))) return rc;
     size_t need = 0;
-    ltca_tsa_workspace_bytes(t, 0, &need);
+    ltca_tsa_workspace_bytes(&layout, 0, &need);
     if (!t->workspace || t->workspace_bytes < need)
         return fail(ctx, LTCA_ERR_WORKSPACE, "forward needs %zu bytes of workspace", need);
     char* w = reinterpret_cast<char*>(t->workspace);
@@ -1260,7 +1274,8 @@ static int tsa_backward(ltca_ctx* ctx, const ltca_tsa_params* t, bool want_dx, b
         return fail(ctx, LTCA_ERR_INVALID, "dropout_prob must be in [0, 1)");
     if (t->pre_norm) return prenorm_backward(ctx, t, want_dx, want_dw);
     size_t need = 0;
-    ltca_tsa_workspace_bytes(t, 1, &need);
+    const ltca_tsa_params layout = laid_out(t, 1);
+    ltca_tsa_workspace_bytes(&layout, 1, &need);
     if (!t->workspace || t->workspace_bytes < need)
         return fail(ctx, LTCA_ERR_WORKSPACE, "backward needs %zu bytes of workspace", need);
     float* colsum_scratch =
@@ -1273,9 +1288,7 @@ static int tsa_backward(ltca_ctx* ctx, const ltca_tsa_params* t, bool want_dx, b
         return column_sums(ctx, own, (int64_t)t->B * t->S, colsum_scratch);
     }
     Plan pl;
-    if ((rc = make_plan(t, &pl))) return rc;
-    if (!t->workspace || t->workspace_bytes < need)
-        return fail(ctx, LTCA_ERR_WORKSPACE, "backward needs %zu bytes of workspace", need);
+    if ((rc = make_plan(&layout, &pl))) return rc;
     char* w = reinterpret_cast<char*>(t->workspace);
     float* dctx = reinterpret_cast<float*>(w); w += pl.buf;
     float* dq = reinterpret_cast<float*>(w);   w += pl.buf;

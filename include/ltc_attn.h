@@ -167,7 +167,9 @@ int ltca_ctx_set_sm_limit(ltca_ctx* ctx, int32_t n_sms);
 
 /* ---- attention core --------------------------------------------------------------------- */
 
-/* Scratch needed by ltca_attn_fwd (backward = 0) or ltca_attn_bwd (backward = 1). */
+/* Scratch needed by ltca_attn_fwd (backward = 0) or ltca_attn_bwd (backward = 1).  With keep_mask set the answer holds
+ * room for the mask packed into bits; a call whose workspace was sized without the mask runs too, on the mask as it is
+ * (the same for the module's entry points below). */
 int ltca_attn_workspace_bytes(const ltca_attn_params* p, int backward, size_t* bytes_out);
 
 /* 1 if the tensor-pipe (tcgen05) kernels cover this problem, 0 if it runs on the fp32 path. */
