@@ -77,6 +77,15 @@ inline int64_t integer(PyObject* o) {
     if (v == -1 && PyErr_Occurred()) throw PyErrorSet();
     return v;
 }
+// Any whole number, modulo 2^64 (what a ctypes field of that type takes).
+inline uint64_t word64(PyObject* o) {
+    PyObject* i = PyNumber_Long(o);
+    if (!i) throw PyErrorSet();
+    const unsigned long long v = PyLong_AsUnsignedLongLongMask(i);
+    Py_DECREF(i);
+    if (v == (unsigned long long)-1 && PyErr_Occurred()) throw PyErrorSet();
+    return v;
+}
 inline int truth(PyObject* o) {
     const int v = PyObject_IsTrue(o);
     if (v < 0) throw PyErrorSet();
@@ -359,7 +368,7 @@ void fill_fa(ltca_tsa_params& p, PyObject* const* a) {
     fill_module(p, a);
     p.pre_norm = 1;
     p.dropout_prob = (float)number(a[kModuleArgs]);
-    p.dropout_seed = (uint64_t)integer(a[kModuleArgs + 1]);
+    p.dropout_seed = word64(a[kModuleArgs + 1]);
     p.score_clamp = (float)number(a[kModuleArgs + 2]);
 }
 

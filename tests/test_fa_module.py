@@ -94,3 +94,19 @@ def test_cuda_flash_attention_module(ctx, case):
         assert torch.equal(got[name], again[name]), f"{name}: two runs differ"
         mag = bias_mag if name in ("dbq", "dbk", "dbv") else float(np.abs(r).max())
         assert np.abs(g - r).max() < tol * max(1.0, mag), f"{name}: {np.abs(g - r).max()} vs {mag}"
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("seed", [2 ** 63, 2 ** 64 - 3, -5])
+def test_dropout_seeds_use_all_64_bits(ctx, seed):
+    import torch
+    B, S, E, H, D = 1, 8, 32, 2, 16
+    x, dy, wq, wk, wv, wo, _, gamma, beta, _ = make(B, S, E, H, D, 5, False)
+    args = [torch.from_numpy(a).cuda() for a in (x, wq, wk, wv, wo)]
+    kw = dict(gamma=torch.from_numpy(gamma).cuda(), beta=torch.from_numpy(beta).cuda(), dropout_prob=0.5, dropout_seed=seed)
+    out = ctx.fa_fwd(*args, B, S, H, D, **kw)
+    keep = oracle.dropout_keep(seed % 2 ** 64, B * S * E, 0.5).reshape(B * S, E)
+    assert ((out.cpu().numpy() != 0) == (keep != 0)).all()
+    g = ctx.fa_bwd(*args, torch.from_numpy(dy).cuda(), B, S, H, D, **kw)
+    # dbo sums the gradient behind the dropout (at most 8 fp32 terms per column)
+    assert np.allclose(g["dbo"].cpu().numpy(), (dy * keep * 2.0).sum(0), rtol=0, atol=1e-5)
