@@ -6,8 +6,10 @@
 // the host about 18 us per forward and 25 us per decode step - the calls were bound by the interpreter.  Here a call
 // is one argument vector, two allocations without the dispatcher, and the launch itself.
 //
-// Every function takes its arguments by position (the Python methods of Context give them names and defaults), holds
-// the GIL, and enqueues on the context's stream like the C ABI does.
+// Every function takes its arguments by position (the Python methods of Context give them names and defaults) and enqueues
+// on the context's stream like the C ABI does.  The C call itself runs without the interpreter lock, as calls through
+// ctypes do: threads that drive contexts of their own enqueue side by side, and a launch queue that is full holds up only
+// the thread that met it.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
@@ -51,6 +53,16 @@ void check(const Host* h, int rc) {
         Py_DECREF(e);
     }
     throw PyErrorSet();
+}
+
+// f() without the interpreter lock; it touches no Python object, and whatever it reads is held by the caller.
+template <typename F>
+int unlocked(F f) {
+    struct Release {
+        PyThreadState* state = PyEval_SaveThread();
+        ~Release() { PyEval_RestoreThread(state); }
+    } release;
+    return f();
 }
 
 // ---- argument access ---------------------------------------------------------------------------
@@ -109,13 +121,15 @@ inline PyObject* result(PyObject* given_obj, const at::Tensor& t) {
     return wrap(t);
 }
 
-const at::Tensor* workspace(Host* h, size_t bytes) {
-    if (bytes == 0) return nullptr;
+// Undefined for zero bytes.  The result is a reference of its own: while the lock is released another thread may have
+// the scratch of this context grow.
+at::Tensor workspace(Host* h, size_t bytes) {
+    if (bytes == 0) return at::Tensor();
     if (!h->ws->defined() || (size_t)h->ws->numel() < bytes) {
         *h->ws = at::Tensor();           // give the old block back before the larger one is taken
         *h->ws = empty(h, {(int64_t)bytes}, at::kByte);
     }
-    return h->ws;
+    return *h->ws;
 }
 
 // ---- the attention core ------------------------------------------------------------------------
@@ -170,11 +184,15 @@ void fill(Core& c, const at::Tensor& q, const at::Tensor& k, const at::Tensor& v
     }
 }
 
-inline void attach(Host* h, ltca_attn_params& p, size_t bytes) {
-    if (const at::Tensor* ws = workspace(h, bytes)) {
-        p.workspace = ws->data_ptr();
-        p.workspace_bytes = (size_t)ws->numel();
+// The scratch of a call, which keeps it until it returns.
+template <typename Params>
+at::Tensor attach(Host* h, Params& p, size_t bytes) {
+    at::Tensor ws = workspace(h, bytes);
+    if (ws.defined()) {
+        p.workspace = ws.data_ptr();
+        p.workspace_bytes = (size_t)ws.numel();
     }
+    return ws;
 }
 
 // out / lse: the caller's tensors, or new ones of the shape that the call writes.
@@ -196,8 +214,8 @@ PyObject* attn_fwd(Host* h, PyObject* const* a) {
     outputs(h, c, a[9], a[10], o, lse);
     size_t need = 0;
     ltca_attn_workspace_bytes(&c.p, 0, &need);
-    attach(h, c.p, need);
-    check(h, ltca_attn_fwd(h->ctx, &c.p));
+    const at::Tensor ws = attach(h, c.p, need);
+    check(h, unlocked([&] { return ltca_attn_fwd(h->ctx, &c.p); }));
     return Py_BuildValue("NN", result(a[9], o), result(a[10], lse));
 }
 
@@ -209,8 +227,8 @@ PyObject* attn_decode(Host* h, PyObject* const* a) {
     outputs(h, c, a[7], a[8], o, lse);
     size_t need = 0;
     ltca_attn_decode_workspace_bytes(&c.p, &need);
-    attach(h, c.p, need);
-    check(h, ltca_attn_decode(h->ctx, &c.p));
+    const at::Tensor ws = attach(h, c.p, need);
+    check(h, unlocked([&] { return ltca_attn_decode(h->ctx, &c.p); }));
     return Py_BuildValue("NN", result(a[7], o), result(a[8], lse));
 }
 
@@ -239,8 +257,8 @@ PyObject* attn_bwd(Host* h, PyObject* const* a) {
     p.bwd_deterministic = truth(a[15]);
     size_t need = 0;
     ltca_attn_workspace_bytes(&p, 1, &need);
-    attach(h, p, need);
-    check(h, ltca_attn_bwd(h->ctx, &p));
+    const at::Tensor ws = attach(h, p, need);
+    check(h, unlocked([&] { return ltca_attn_bwd(h->ctx, &p); }));
     return Py_BuildValue("NNN", result(a[12], g[0]), result(a[13], g[1]), result(a[14], g[2]));
 }
 
@@ -291,36 +309,34 @@ void attach_saved(ltca_tsa_params& p, PyObject* saved, int reuse) {
     p.saved_bytes = (size_t)s.numel();
     p.reuse_forward = reuse;
 }
-// weight_cache: None or (buffer, valid)
-void attach_weight_cache(ltca_tsa_params& p, PyObject* cache) {
-    if (!given(cache)) return;
+// weight_cache: None or (buffer, valid).  The result keeps the buffer for the call.
+at::Tensor attach_weight_cache(ltca_tsa_params& p, PyObject* cache) {
+    if (!given(cache)) return at::Tensor();
     PyObject* buf = PySequence_GetItem(cache, 0);
     PyObject* valid = buf ? PySequence_GetItem(cache, 1) : nullptr;
     if (!valid) { Py_XDECREF(buf); throw PyErrorSet(); }
-    // the caller's tuple keeps the buffer alive for the call
-    const at::Tensor* t = THPVariable_Check(buf) ? &THPVariable_Unpack(buf) : nullptr;
+    at::Tensor t;
+    if (THPVariable_Check(buf)) t = THPVariable_Unpack(buf);
     const int v = PyObject_IsTrue(valid);
-    if (t) { p.weight_cache = t->data_ptr(); p.weight_cache_bytes = (size_t)t->numel(); p.weight_cache_valid = v; }
+    if (t.defined()) { p.weight_cache = t.data_ptr(); p.weight_cache_bytes = (size_t)t.numel(); p.weight_cache_valid = v; }
     Py_DECREF(buf);
     Py_DECREF(valid);
-    if (!t) raise(PyExc_TypeError, "weight_cache is (buffer, valid)");
+    if (!t.defined()) raise(PyExc_TypeError, "weight_cache is (buffer, valid)");
     if (v < 0) throw PyErrorSet();
+    return t;
 }
 
-void attach_module(Host* h, ltca_tsa_params& p, int which) {
+at::Tensor attach_module(Host* h, ltca_tsa_params& p, int which) {
     size_t need = 0;
     check(h, ltca_tsa_workspace_bytes(&p, which, &need));
-    if (const at::Tensor* ws = workspace(h, need)) {
-        p.workspace = ws->data_ptr();
-        p.workspace_bytes = (size_t)ws->numel();
-    }
+    return attach(h, p, need);
 }
 
 PyObject* module_forward(Host* h, ltca_tsa_params& p, const at::Tensor& x) {
     at::Tensor out = empty(h, x.sizes(), at::kFloat);
     p.out = static_cast<float*>(out.data_ptr());
-    attach_module(h, p, 0);
-    check(h, ltca_tsa_fwd(h->ctx, &p));
+    const at::Tensor ws = attach_module(h, p, 0);
+    check(h, unlocked([&] { return ltca_tsa_fwd(h->ctx, &p); }));
     return wrap(std::move(out));
 }
 
@@ -328,7 +344,7 @@ PyObject* module_forward(Host* h, ltca_tsa_params& p, const at::Tensor& x) {
 PyObject* tsa_fwd(Host* h, PyObject* const* a) {
     ltca_tsa_params p;
     fill_module(p, a);
-    attach_weight_cache(p, a[kModuleArgs + 1]);
+    const at::Tensor cache = attach_weight_cache(p, a[kModuleArgs + 1]);
     attach_saved(p, a[kModuleArgs], 0);
     return module_forward(h, p, tensor(a[0]));
 }
@@ -338,7 +354,7 @@ PyObject* tsa_bwd(Host* h, PyObject* const* a) {
     ltca_tsa_params p;
     fill_module(p, a);
     const at::Tensor& dy = tensor(a[kModuleArgs]);
-    attach_weight_cache(p, a[kModuleArgs + 3]);
+    const at::Tensor cache = attach_weight_cache(p, a[kModuleArgs + 3]);
     attach_saved(p, a[kModuleArgs + 1], truth(a[kModuleArgs + 2]));
     const at::Tensor& x = tensor(a[0]);
     at::Tensor dx = empty(h, x.sizes(), at::kFloat);
@@ -350,8 +366,8 @@ PyObject* tsa_bwd(Host* h, PyObject* const* a) {
     p.dy = static_cast<const float*>(dy.data_ptr());
     p.dx = static_cast<float*>(dx.data_ptr());
     p.dwq = base; p.dwk = base + E * HW; p.dwv = base + 2 * E * HW; p.dwo = base + 3 * E * HW;
-    attach_module(h, p, 3);
-    check(h, ltca_tsa_bwd(h->ctx, &p));
+    const at::Tensor ws = attach_module(h, p, 3);
+    check(h, unlocked([&] { return ltca_tsa_bwd(h->ctx, &p); }));
     PyObject* out[5] = {wrap(std::move(dx)), nullptr, nullptr, nullptr, nullptr};
     for (int i = 0; i < 4; ++i) {
         const int64_t size[2] = {i < 3 ? E : HW, i < 3 ? HW : E}, stride[2] = {size[1], 1};
@@ -396,8 +412,8 @@ PyObject* fa_bwd(Host* h, PyObject* const* a) {
     const int n = p.use_layer_norm ? 11 : 9;
     if (n == 11) { g[9].t = f32({E}); g[10].t = f32({E}); }
     for (int i = 0; i < n; ++i) *g[i].slot = static_cast<float*>(g[i].t.data_ptr());
-    attach_module(h, p, 3);
-    check(h, ltca_tsa_bwd(h->ctx, &p));
+    const at::Tensor ws = attach_module(h, p, 3);
+    check(h, unlocked([&] { return ltca_tsa_bwd(h->ctx, &p); }));
     PyObject* d = PyDict_New();
     if (!d) throw PyErrorSet();
     for (int i = 0; i < n; ++i) {
@@ -410,9 +426,9 @@ PyObject* fa_bwd(Host* h, PyObject* const* a) {
 
 // (nbytes): the context's scratch, at least that large; None for zero bytes.
 PyObject* host_workspace(Host* h, PyObject* const* a) {
-    const at::Tensor* ws = workspace(h, (size_t)integer(a[0]));
-    if (!ws) Py_RETURN_NONE;
-    return wrap(*ws);
+    at::Tensor ws = workspace(h, (size_t)integer(a[0]));
+    if (!ws.defined()) Py_RETURN_NONE;
+    return wrap(std::move(ws));
 }
 
 // (): the context is gone; later calls fail with LTCA_ERR_INVALID.
