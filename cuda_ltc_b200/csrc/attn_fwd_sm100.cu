@@ -1006,7 +1006,7 @@ int launch_fwd(ltca_ctx* ctx, const ltca_attn_params* p, const void* mask_words,
     // the bits of the result, does not move with the launch width.
     const int64_t ctas2 = (int64_t)p->B * p->H * ((p->Sq + 2 * kBlockM - 1) / (2 * kBlockM));
     const int64_t sms = ctx->sm_device > 0 ? ctx->sm_device : kPlanSms;
-    // Where the caller asks for the two-tile kernel's order of additions (ctx->fwd_pairs), short queries keep it too.
+    // Module calls with a key bias (ctx->fwd_pairs) keep it for short queries too.
     const bool few = ctas2 <= sms && p->Sk > 512;
     const bool ordered = ctx->fwd_pairs && (ctas2 <= sms || p->Sq <= 2 * kBlockM);
     if (D != 64 || !(few || ordered)) return launch_fwd_tile<D, kSplitP>(ctx, p, q, k, v, qs, ks, vs, a);

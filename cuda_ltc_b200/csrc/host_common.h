@@ -27,9 +27,10 @@ struct ltca_ctx {
     // A module call's packed mask (attn_mask.cuh): set while the call launches its attention kernels, which all read it.
     const float* mask_packed = nullptr;
     const void* mask_words = nullptr;
-    // Set while the FlashAttention form's backward recomputes its forward: the gradient of the key bias is zero but for the
-    // rounding of that forward (a shift of all keys does not move a softmax), so every digit of it follows the order in
-    // which one kernel adds; short calls then stay with the two-tile kernel (launch_fwd, attn_fwd_sm100.cu).
+    // Set by a module call with a key bias, forward and backward alike: short calls then take the two-tile kernel
+    // (launch_fwd, attn_fwd_sm100.cu).  Where no score is clamped the terms of that bias's gradient cancel (a shift of all
+    // keys does not move a softmax) and what is left of it follows the order in which one kernel adds, so that order is held
+    // fixed; and the backward recomputes what the forward computed.
     bool fwd_pairs = false;
     char err[512] = {0};
     // optional per-kernel timing of the backward pass (ltca_ctx_enable_kernel_timing)

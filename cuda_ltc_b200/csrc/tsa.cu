@@ -921,6 +921,7 @@ int tensor_forward(ltca_ctx* ctx, const ltca_tsa_params* t, const ltca_tsa_param
     w += pl.y;
     TBufs tb;
     CallHints hints{ctx};
+    ctx->fwd_pairs = t->bk != nullptr;
     if (fused && (rc = place_mask_words(ctx, &layout, pl, scratch_of(t, pl, w), pl.attn_fwd, true))) return rc;
     if ((rc = tensor_forward_core(ctx, t, pl, w, &tb, 0, nullptr, nullptr, nullptr, fused ? outer : nullptr))) return rc;
     GemmProblem gp;

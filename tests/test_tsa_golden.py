@@ -368,3 +368,25 @@ def test_materialised_score_path_matches_reference_cudnn_module(ctx, path):
     assert np.abs(got[0].cpu().numpy() - d["dx"]).max() < tol * max(1.0, np.abs(d["dx"]).max())
     for name, g, r in zip(("dwq", "dwk", "dwv", "dwo"), got[1:], reference_weight_grads(d, E, H)):
         assert np.abs(g.cpu().numpy() - r).max() < tol * max(1.0, np.abs(r).max()), name
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bias", [False, True])
+@pytest.mark.parametrize("S", [64, 200, 300])
+def test_backward_recomputes_what_the_forward_computed(ctx, S, bias):
+    """The gradients from a kept forward and from the backward's own recomputation of it, bit for bit: both calls take the
+    same attention kernel, with and without biases."""
+    import torch
+    B, E, H, W = 3, 128, 2, 64
+    r = lambda *n, amp=1.0: torch.from_numpy((np.random.default_rng(n[0] + 7 * len(n)).standard_normal(n) * amp).astype(np.float32)).cuda()
+    x, dy = r(B * S, E), r(B * S, E).roll(1, 0)
+    w = [r(E, H * W, amp=E ** -0.5).roll(i, 0) for i in range(3)] + [r(H * W, E, amp=E ** -0.5)]
+    kw = dict(scale=W ** -0.5, time_major=False)
+    if bias:
+        kw.update({n: 0.1 * r(H * W).roll(i) for i, n in enumerate(("bq", "bk", "bv"))})
+    saved = ctx.tsa_saved_buffer(x, *w, B, S, H, W)
+    ctx.tsa_fwd(x, *w, B, S, H, W, use_layer_norm=False, saved=saved, **kw)
+    kept = ctx.tsa_bwd(x, *w, dy, B, S, H, W, saved=saved, reuse_forward=True, **kw)
+    again = ctx.tsa_bwd(x, *w, dy, B, S, H, W, **kw)
+    for a, b in zip(kept, again):
+        assert torch.equal(a, b)
