@@ -29,42 +29,45 @@ def _kernel_bodies(text):
     return bodies
 
 
+def _launched(text, bodies):
+    """(launch, kernels) for every dependent launch of a source file.  A kernel picked at run time goes by a local name:
+    it stands for every kernel named between its declaration and the launch."""
+    spots = [(m, m.group(1)) for m in re.finditer(r"launch_dependent\(\s*([\w<>:, ]+?),\s*\S*(?:dim3|grid|rg)\b", text)]
+    spots += [(m, m.group(1)) for m in re.finditer(r"launch_dependent_if\([^;]*?\),\s*([\w<>:, ]+?),\s*\S*(?:dim3|grid|gq|gk)\b", text)]
+    spots += [(m, m.group(1)) for m in re.finditer(r"cudaLaunchKernelEx\(&cfg,\s*(\w+)", text)
+              if "cudaLaunchAttributeProgrammaticStreamSerialization" in text]
+    for m, name in spots:
+        base = re.sub(r"<.*", "", name).strip()
+        if base in bodies:
+            yield m.group(0), {base}
+            continue
+        declared = text.rfind(f"auto {base} =", 0, m.start())
+        assert declared >= 0, f"{m.group(0)}: {base} is neither a kernel nor a local name for one"
+        named = set(re.findall(r"\b\w+_kernel\b", text[declared:m.start()])) & set(bodies)
+        assert named, f"{m.group(0)}: no kernel found behind {base}"
+        yield m.group(0), named
+
+
 def test_every_dependent_launch_targets_a_kernel_that_waits():
     src = _sources()
     bodies = {}
     for text in src.values():
         bodies.update(_kernel_bodies(text))
-    launched = set()
+    seen = set()
     for name, text in src.items():
-        for m in re.finditer(r"launch_dependent(?:_if)?\(\s*([^;]*?);", text, flags=re.S):
-            args = m.group(1)
-            if args.startswith(("bool dependent", "void (*kern)", "true, kern")):
-                continue                                    # the helpers' own definitions
-            first = args.split(",")[1] if "launch_dependent_if" in m.group(0) else args.split(",")[0]
-            launched.add(first.strip())
-    assert launched, "no dependent launch found: the pattern of this test is out of date"
-    # local aliases of kernels (function pointers picked at run time) and the kernels they stand for
-    alias = {
-        "kern": None,                                        # resolved below, per file
-        "kdq": "attn_bwd_dq_sm100_kernel", "kdkv": "attn_bwd_dkv_sm100_kernel",
-        "fwd_kernel": "wide_softmax_fwd_rows_kernel", "bwd_kernel": "wide_softmax_bwd_rows_kernel",
-    }
-    names = set()
-    for k in launched:
-        base = re.sub(r"<.*", "", k)
-        if base == "kern":
-            names.update({"gemm_bf16_sm100_kernel", "attn_fwd_sm100_kernel"})
-        elif base in alias:
-            names.add(alias[base])
-            if base == "fwd_kernel":
-                names.add("wide_softmax_fwd_kernel")
-            if base == "bwd_kernel":
-                names.add("wide_softmax_bwd_kernel")
-        else:
-            names.add(base)
-    for k in sorted(names):
-        assert k in bodies, f"{k}: launched as a dependent kernel but not found"
-        assert "grid_dependency_wait()" in bodies[k], f"{k} is launched as a dependent kernel but never waits"
+        if name == "host_common.h":
+            continue                                        # the helpers' own definitions
+        found = list(_launched(text, bodies))
+        # the pattern has to see every launch of the file
+        direct = text.count("cudaLaunchKernelEx(") if "cudaLaunchAttributeProgrammaticStreamSerialization" in text else 0
+        assert len(found) == len(re.findall(r"launch_dependent(?:_if)?\(", text)) + direct, name
+        for launch, kernels in found:
+            for k in kernels:
+                assert "grid_dependency_wait()" in bodies[k], f"{name}: {k} is launched as a dependent kernel but never waits"
+            seen |= kernels
+    # kernels that are picked at run time or launched directly
+    assert {"attn_fwd_tile_sm100_kernel", "gemm_bf16_sm100_kernel", "attn_decode_kernel", "pack_bf16_kernel",
+            "gemm_splitk_reduce_kernel", "wide_softmax_fwd_rows_kernel", "attn_bwd_dkv_sm100_kernel"} <= seen
 
 
 def test_waiting_kernels_touch_no_kernel_argument_memory_before_the_wait():
