@@ -3,7 +3,7 @@ torch front end, with g++ against torch's headers.
 
 Run as ``python -m cuda_ltc_b200.build`` or call :func:`build_library`.  Objects go to
 ``cuda_ltc_b200/build/``, the libraries to ``cuda_ltc_b200/``; a source file is recompiled only when it
-or one of the headers is newer than its object.
+or one of the headers is newer than its object, _host.so also when torch or the interpreter is another one.
 """
 from __future__ import annotations
 
@@ -48,12 +48,17 @@ def _compile(src: str, obj: str) -> str:
 
 
 def _build_host(force: bool = False) -> None:
-    """_host.so finds libltc_attn.so beside itself; torch's libraries are already in a process that imports it."""
+    """_host.so finds libltc_attn.so beside itself; torch's libraries are already in a process that imports it.  It is
+    built against one torch and one interpreter, whose ABI it shares: a stamp beside the objects says which."""
     header = os.path.join(HERE, "..", "include", "ltc_attn.h")
-    if not force and os.path.exists(HOST_OUT) and os.path.getmtime(HOST_OUT) >= max(
-            os.path.getmtime(HOST_SRC), os.path.getmtime(header)):
-        return
     import torch
+    built_for = f"torch {torch.__version__} at {os.path.dirname(torch.__file__)}, python {sys.version}\n"
+    stamp = os.path.join(OBJ_DIR, "_host.stamp")
+    if not force and os.path.exists(HOST_OUT) and os.path.exists(stamp) and os.path.getmtime(HOST_OUT) >= max(
+            os.path.getmtime(HOST_SRC), os.path.getmtime(header)):
+        with open(stamp) as f:
+            if f.read() == built_for:
+                return
     from torch.utils import cpp_extension
     lib_dir = os.path.join(os.path.dirname(torch.__file__), "lib")
     includes = [*cpp_extension.include_paths(), sysconfig.get_paths()["include"], "/usr/local/cuda/include"]
@@ -63,6 +68,8 @@ def _build_host(force: bool = False) -> None:
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError("g++ failed for host_binding.cpp:\n" + r.stdout + r.stderr)
+    with open(stamp, "w") as f:
+        f.write(built_for)
 
 
 def build_library(force: bool = False, verbose: bool = False) -> str:

@@ -143,3 +143,21 @@ def test_decode_size_query_and_static_entry_reject_bad_shapes_on_the_host(lib):
         assert lib.ltca_attn_decode_static(None, C.byref(p), err, len(err)) == -1
         assert b"bad decode arguments" in err.value
     assert lib.ltca_attn_decode_static(None, None, err, len(err)) == -1
+
+
+def test_the_native_front_end_is_rebuilt_for_another_torch(lib, monkeypatch, tmp_path):
+    """_host.so shares torch's ABI, so a binary that was built against another torch is not kept."""
+    import types
+    import torch
+    from cuda_ltc_b200 import build
+    ran = []
+    monkeypatch.setattr(build, "OBJ_DIR", str(tmp_path))
+    monkeypatch.setattr(build.subprocess, "run",
+                        lambda cmd, **kw: ran.append(cmd) or types.SimpleNamespace(returncode=0, stdout="", stderr=""))
+    build._build_host()                     # nothing says what the present one was built against
+    assert len(ran) == 1
+    build._build_host()
+    assert len(ran) == 1
+    monkeypatch.setattr(torch, "__version__", "0.0.0")
+    build._build_host()
+    assert len(ran) == 2
