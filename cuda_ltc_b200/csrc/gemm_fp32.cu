@@ -1,6 +1,6 @@
-// Products of the module's exact pipeline: fp32 operands, fp32 FMA arithmetic, every sum in ascending order of the
-// contraction (the arithmetic of the reference's cublasSgemm with tensor cores off,
-// src/ml/flash_attention.cu:531-536).
+// Products of the module's exact pipeline: fp32 operands, fp32 FMA arithmetic (that of the reference's cublasSgemm with
+// tensor cores off, src/ml/flash_attention.cu:531-536).  The sums run in ascending order of the contraction, but for
+// sliced contractions (slice by slice) and the small products that may run in any order (eight interleaved shares).
 //
 // What bounds them: the small modules this pipeline serves (model widths of 32 to 256, up to a few thousand rows) are
 // launches and latency, the larger ones the FMA pipe.  So the products of one step (Q, K and V; the four weight gradients;
@@ -381,6 +381,8 @@ int plan_gemm(ltca_ctx* ctx, Plan32* pl, const Gemm32Problem* p, int n, bool sum
             g.kper = (int)(((K + s - 1) / s + 31) / 32 * 32);
             g.slices = (K + g.kper - 1) / g.kper;
             if (g.slices > 1) {
+                for (int i = 0; i < n; ++i)
+                    if (p[i].bias) return fail(ctx, LTCA_ERR_INVALID, "gemm_fp32: a sliced contraction takes no bias");
                 g.partial = scratch;
                 int64_t off = 0;
                 for (int i = 0; i < n; ++i) { g.part_off[i] = off; off += (int64_t)g.slices * p[i].M * p[i].N; }
