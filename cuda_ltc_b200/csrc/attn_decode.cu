@@ -374,25 +374,27 @@ int dispatch_decode(ltca_ctx* ctx, const DecodeArgs& a, const SplitPlan& plan) {
     return fail(ctx, LTCA_ERR_UNSUPPORTED, "decode supports head_dim 16, 32, 64, 128 (got %d)", a.D);
 }
 
+// Bytes of the partial results of n splits per pair.
+size_t partial_bytes(const ltca_attn_params* p, int64_t n) {
+    return n > 1 ? align_up((size_t)p->B * p->H * n * (p->D + 2) * sizeof(float), 256) : 0;
+}
+
 }  // namespace
 
 // The split count must not depend on the context, so that the size query (which has no
 // context) and the launch agree.  Non-positive shapes need no scratch (the launch refuses them).
-// A clustered call uses no scratch; the query still answers what its partials would take at one CTA per 256 keys, the
-// size by which ltca_attn_decode_static has always told large shapes from small ones.
+// The answer is never below what the partials would take at one CTA per 256 keys and four per SM, although splits that
+// merge inside a cluster use no scratch: by that size ltca_attn_decode_static tells the shapes it takes from those it
+// refuses, and which it takes does not move with the split.
 size_t attn_decode_workspace(const ltca_attn_params* p) {
     if (p->B < 1 || p->H < 1 || p->Sk < 1 || p->D < 1) return 0;
     const SplitPlan s = plan_splits(p);
     if (!s.few) return 0;
-    const int64_t bh = (int64_t)p->B * p->H;
-    int64_t n = s.n;
-    if (s.cluster || n == 1) {
-        const int64_t want = (4 * (int64_t)kPlanSms + bh - 1) / bh, cap = (p->Sk + 255) / 256;
-        n = want < cap ? want : cap;
-        if (n > 64) n = 64;
-        if (n <= 1) return 0;
-    }
-    return align_up((size_t)bh * n * (p->D + 2) * sizeof(float), 256);
+    const int64_t bh = (int64_t)p->B * p->H, want = (4 * (int64_t)kPlanSms + bh - 1) / bh, cap = (p->Sk + 255) / 256;
+    int64_t n = want < cap ? want : cap;
+    if (n > 64) n = 64;
+    if (!s.cluster && s.n > n) n = s.n;
+    return partial_bytes(p, n);
 }
 
 int launch_attn_decode(ltca_ctx* ctx, const ltca_attn_params* p) {
@@ -424,7 +426,7 @@ int launch_attn_decode(ltca_ctx* ctx, const ltca_attn_params* p) {
     const SplitPlan plan = plan_splits(p);
     a.nsplit = plan.n;
     if (plan.n > 1 && !plan.cluster) {
-        const size_t need = attn_decode_workspace(p);
+        const size_t need = partial_bytes(p, plan.n);
         if (!p->workspace || p->workspace_bytes < need)
             return fail(ctx, LTCA_ERR_WORKSPACE, "decode needs %zu bytes of workspace", need);
         a.partial = reinterpret_cast<float*>(p->workspace);
@@ -479,7 +481,7 @@ extern "C" int ltca_attn_decode_static(void* stream, const ltca_attn_params* p, 
     if (need > kStaticScratchBytes) {
         char msg[200];
         snprintf(msg, sizeof(msg),
-                 "this decode shape needs %zu bytes of split scratch, the built-in array holds %zu; "
+                 "ltca_attn_decode_workspace_bytes answers %zu for this shape, this entry point takes up to %zu; "
                  "use ltca_attn_decode with a caller-provided workspace", need, kStaticScratchBytes);
         set_err(err, err_len, msg);
         return LTCA_ERR_WORKSPACE;

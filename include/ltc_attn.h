@@ -188,8 +188,8 @@ int ltca_attn_bwd(ltca_ctx* ctx, const ltca_attn_params* p);
  * each sequence.  The reference has no such call; the closest hook is the currIdx argument
  * of cudnnMultiHeadAttnForward, always -1 there (src/ml/cuDNN_ops.cu:206). */
 int ltca_attn_decode(ltca_ctx* ctx, const ltca_attn_params* p);
-/* Scratch needed by ltca_attn_decode: zero when batch x heads alone fills the GPU, otherwise
- * room for the partial results of the key-range split. */
+/* Scratch for ltca_attn_decode: zero when batch x heads alone fills the GPU, otherwise at least room for the
+ * partial results of the key-range split (calls whose splits merge inside a thread-block cluster use none of it). */
 int ltca_attn_decode_workspace_bytes(const ltca_attn_params* p, size_t* bytes_out);
 
 /*
@@ -207,7 +207,7 @@ int ltca_attn_decode_workspace_bytes(const ltca_attn_params* p, size_t* bytes_ou
  *  - Works on the calling thread's CURRENT device and enqueues on `stream` (cudaStream_t as void*).
  *  - The first call on each device looks up the device address of the built-in array
  *    (cudaGetSymbolAddress); make that first call before starting any stream capture.
- *  - Shapes whose split scratch (ltca_attn_decode_workspace_bytes) exceeds 256 KiB are refused
+ *  - Shapes for which ltca_attn_decode_workspace_bytes answers more than 256 KiB are refused
  *    with LTCA_ERR_WORKSPACE and a message in `err`; nothing is launched.
  *  - All calls share the one array.  Each call overwrites every slot it later reads, so stale
  *    contents of an earlier call are harmless and nothing has to be cleared, but two calls

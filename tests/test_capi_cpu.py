@@ -161,3 +161,24 @@ def test_the_native_front_end_is_rebuilt_for_another_torch(lib, monkeypatch, tmp
     monkeypatch.setattr(torch, "__version__", "0.0.0")
     build._build_host()
     assert len(ran) == 2
+
+
+@pytest.mark.parametrize("B,H,Sk,D,refused", [(1, 8, 32768, 128, True),      # more splits than a cluster holds
+                                              (50, 4, 16384, 128, True),     # splits of one cluster
+                                              (1, 8, 2048, 128, False), (4, 64, 8192, 64, False)])
+def test_static_decode_takes_the_shapes_below_its_size(lib, B, H, Sk, D, refused):
+    """Which shapes the allocation-free decode takes follows a size that the split does not move: four splits per SM over the
+    pairs, one per 256 keys, 64 at most."""
+    from cuda_ltc_b200 import _lib
+    dummy = (C.c_float * 64)()
+    p = _lib.AttnParams()
+    p.B, p.H, p.Sq, p.Sk, p.D = B, H, 1, Sk, D
+    p.dtype, p.mode, p.scale = _lib.LTCA_F32, _lib.MODE_FP32, 0.125
+    n = C.c_size_t(0)
+    assert lib.ltca_attn_decode_workspace_bytes(C.byref(p), C.byref(n)) == 0
+    splits = min(-(-4 * 148 // (B * H)), -(-Sk // 256), 64)
+    assert n.value >= B * H * splits * (D + 2) * 4 and (n.value > 256 << 10) == refused
+    if refused:                                              # (on the host; nothing is launched or read)
+        p.q = p.k = p.v = p.o = C.addressof(dummy)
+        err = C.create_string_buffer(256)
+        assert lib.ltca_attn_decode_static(None, C.byref(p), err, len(err)) == -4 and b"262144" in err.value
