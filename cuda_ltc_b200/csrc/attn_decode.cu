@@ -283,7 +283,6 @@ __global__ void __launch_bounds__(32 * W) attn_decode_kernel(const DecodeArgs a)
 
 template <typename T>
 __global__ void __launch_bounds__(128) attn_decode_merge_kernel(const DecodeArgs a) {
-    grid_launch_dependents();
     grid_dependency_wait();
     const int bh = blockIdx.x;
     if ((int)threadIdx.x < a.D) merge_partials<T>(a, a.partial + (int64_t)bh * a.nsplit * (a.D + 2), a.nsplit, bh / a.H, bh % a.H);

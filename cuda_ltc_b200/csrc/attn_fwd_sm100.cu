@@ -864,7 +864,6 @@ attn_fwd_tile_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
                 if (lane == 0) mbar_arrive(bar_p_full);
     #undef S_
             }
-            if constexpr (kTeams == 1) grid_launch_dependents();
             const int qi = q0 + row;
             const int64_t stat = ((int64_t)b * a.H + h) * a.Sq + qi;
             if (n_t > 0) {

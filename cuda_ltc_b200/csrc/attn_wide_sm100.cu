@@ -55,7 +55,6 @@ struct SoftmaxArgs {
 // One warp per (batch, head, query) row: scale, clamp (the reference clamps scaled scores at 10,
 // src/ml/flash_attention.cu:167), visibility (keep-mask value 0 hides, :161-164; causal; key lengths), softmax.
 __global__ void __launch_bounds__(256) wide_softmax_fwd_kernel(const SoftmaxArgs a) {
-    grid_launch_dependents();
     grid_dependency_wait();
     const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
@@ -103,7 +102,6 @@ __global__ void __launch_bounds__(256) wide_softmax_fwd_kernel(const SoftmaxArgs
 
 // dS = scale * P o (dP - sum_j P dP), zero where the score was clamped; written to dS (P itself by default).
 __global__ void __launch_bounds__(256) wide_softmax_bwd_kernel(const SoftmaxArgs a) {
-    grid_launch_dependents();
     grid_dependency_wait();
     const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
@@ -144,7 +142,6 @@ __device__ __forceinline__ void unpack4_bf16(uint2 w, float* v) {
 // (kChunks groups of four neighbouring columns), so every matrix is read once, 16 bytes per lane and access.
 template <int kChunks>
 __global__ void __launch_bounds__(256) wide_softmax_fwd_rows_kernel(const SoftmaxArgs a) {
-    grid_launch_dependents();
     grid_dependency_wait();
     const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
@@ -209,7 +206,6 @@ __global__ void __launch_bounds__(256) wide_softmax_fwd_rows_kernel(const Softma
 
 template <int kChunks>
 __global__ void __launch_bounds__(256) wide_softmax_bwd_rows_kernel(const SoftmaxArgs a) {
-    grid_launch_dependents();
     grid_dependency_wait();
     const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;

@@ -538,7 +538,9 @@ __global__ void cvt_rows_bf16_vec_kernel(const float4* __restrict__ src, uint2* 
         if (first + e * 256 < n4) dst[first + e * 256] = make_uint2(pack_bf16x2(v[e].x, v[e].y), pack_bf16x2(v[e].z, v[e].w));
 }
 
-// Several matrices of any sizes in ONE launch (the activations and the weights of a module call).
+// Several matrices of any sizes in ONE launch (the activations and the weights of a module call).  Releases the projection
+// behind it at its start: that kernel's CTAs are one to an SM and cannot settle unevenly (module forward B32 S256 E512 54.9
+// us, 55.1 without; module step B64 S512 equal within 0.2 %).
 __global__ void cvt_many_bf16_kernel(const __grid_constant__ CvtMany b) {
     grid_launch_dependents();
     grid_dependency_wait();
