@@ -68,10 +68,12 @@ struct FwdArgs {
     uint32_t* status;
 };
 
-template <int D, bool kSplitP>
+// The two-tile kernel, head_dim 64.
+constexpr int kPairD = 64;
+template <bool kSplitP>
 struct FwdCfg {
-    static constexpr int kBN = (D == 64 && !kSplitP) ? 128 : 64;   // keys per step
-    static constexpr int kDimBlocks = D / 64;                      // 64-element (128 B) column blocks
+    static constexpr int D = kPairD;
+    static constexpr int kBN = kSplitP ? 64 : 128;                 // keys per step
     static constexpr int kQTileBytes = kBlockM * D * 2;
     static constexpr int kKvTileBytes = kBN * D * 2;
     static constexpr int kStages = 8;                              // ring slots
@@ -99,13 +101,14 @@ __device__ __forceinline__ float neg_inf() { return __int_as_float(0xff800000); 
 // kSplitP: P is written as two bf16 terms (p = hi + lo, 16 mantissa bits in total) and the
 // second contraction runs once per term; used when the output is stored as fp32, where the
 // 2^-9 rounding of a single bf16 P would be the largest error left.
-template <int D, typename OutT, bool kSplitP, bool kMask>
+template <bool kSplitP, bool kMask>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
                       const __grid_constant__ CUtensorMap tmap_k,
                       const __grid_constant__ CUtensorMap tmap_v, const FwdArgs a) {
-    using L = FwdCfg<D, kSplitP>;
-    constexpr int kBN = L::kBN;
+    using L = FwdCfg<kSplitP>;
+    using OutT = typename std::conditional<kSplitP, float, __nv_bfloat16>::type;
+    constexpr int D = kPairD, kBN = L::kBN;
     constexpr int kH = kBN / kRowSplit;  // key columns per thread and step
     constexpr int kDH = D / kRowSplit;   // output columns per thread
     extern __shared__ uint8_t smem_raw[];
@@ -194,9 +197,7 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
                 tma_prefetch_desc(&tmap_v);
                 mbar_arrive_expect_tx(bar_q_full(), 2u * L::kQTileBytes);
                 for (int t = 0; t < 2; ++t)
-                    for (int kb = 0; kb < L::kDimBlocks; ++kb)
-                        tma_load_4d(q_smem + t * L::kQTileBytes + kb * (kBlockM * 128), &tmap_q,
-                                    bar_q_full(), kb * 64, m_block * 2 * kBlockM + t * kBlockM, h, b);
+                    tma_load_4d(q_smem + t * L::kQTileBytes, &tmap_q, bar_q_full(), 0, m_block * 2 * kBlockM + t * kBlockM, h, b);
                 bool ok = true;
                 for (int j = 0; j < n_max && ok; ++j) {
 #pragma unroll
@@ -206,10 +207,8 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
                         ok = ok && mbar_wait(bar_kv_empty(slot), phase_of(item) ^ 1u, wc, 0x10 + which);
                         if (!ok) break;
                         mbar_arrive_expect_tx(bar_kv_full(slot), (uint32_t)L::kKvTileBytes);
-                        for (int kb = 0; kb < L::kDimBlocks; ++kb)
-                            tma_load_4d(ring_smem + slot * L::kKvTileBytes + kb * (kBN * 128),
-                                        which == 0 ? &tmap_k : &tmap_v, bar_kv_full(slot), kb * 64,
-                                        j * kBN, h, b);
+                        tma_load_4d(ring_smem + slot * L::kKvTileBytes, which == 0 ? &tmap_k : &tmap_v, bar_kv_full(slot), 0,
+                                    j * kBN, h, b);
                     }
                 }
             }
@@ -231,11 +230,8 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
                 auto issue_qk = [&](int slot) {
                     const uint64_t kd = k_desc + (uint64_t)((slot * L::kKvTileBytes) >> 4);
 #pragma unroll
-                    for (int k = 0; k < D / 16; ++k) {
-                        const uint32_t qoff = (k / 4) * (kBlockM * 128) + (k % 4) * 32;
-                        const uint32_t koff = (k / 4) * (kBN * 128) + (k % 4) * 32;
-                        mma_ss(s_tmem, q_desc + (qoff >> 4), kd + (koff >> 4), idesc_qk, k > 0 ? 1u : 0u);
-                    }
+                    for (int k = 0; k < D / 16; ++k)
+                        mma_ss(s_tmem, q_desc + 2 * k, kd + 2 * k, idesc_qk, k > 0 ? 1u : 0u);
                 };
                 auto issue_pv = [&](int slot, bool acc) {
                     const uint64_t vd = v_desc + (uint64_t)((slot * L::kKvTileBytes) >> 4);
@@ -1011,13 +1007,13 @@ int launch_fwd(ltca_ctx* ctx, const ltca_attn_params* p, const void* mask_words,
     if (D != 64 || !(few || ordered)) return launch_fwd_tile<D, kSplitP>(ctx, p, q, k, v, qs, ks, vs, a);
 
     if constexpr (D == 64) {
-        using L = FwdCfg<D, kSplitP>;
+        using L = FwdCfg<kSplitP>;
         CUtensorMap tq, tk, tv;
         int rc;
         if ((rc = make_tmap_bhsd(ctx, &tq, q, 2, p->B, p->H, p->Sq, D, qs, 64, kBlockM))) return rc;
         if ((rc = make_tmap_bhsd(ctx, &tk, k, 2, p->B, p->H, p->Sk, D, ks, 64, L::kBN))) return rc;
         if ((rc = make_tmap_bhsd(ctx, &tv, v, 2, p->B, p->H, p->Sk, D, vs, 64, L::kBN))) return rc;
-        auto kern = p->keep_mask ? attn_fwd_sm100_kernel<D, OutT, kSplitP, true> : attn_fwd_sm100_kernel<D, OutT, kSplitP, false>;
+        auto kern = p->keep_mask ? attn_fwd_sm100_kernel<kSplitP, true> : attn_fwd_sm100_kernel<kSplitP, false>;
         static SmemOptIn opt_in[2];               // one pair per template instantiation
         LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(opt_in[p->keep_mask ? 1 : 0], ctx->device, kern, L::kDynBytes));
         dim3 grid((p->Sq + 2 * kBlockM - 1) / (2 * kBlockM), p->H, p->B);
