@@ -109,21 +109,20 @@ TC_CASES = [
     (32, 8, 256, 256, 64, True, False, False, 0.0),     # config 2 core
     (1, 2, 512, 512, 128, True, False, False, 0.0),
     (1, 1, 300, 300, 128, False, True, False, 0.0),
-    # few (batch, head) pairs and long query ranges: the two-tile kernel over several 256-row blocks (the
-    # four-tile kernel's 512-row work items would leave most SMs idle)
+    # few (batch, head) pairs and long query ranges: the two-tile kernel (head_dim 64, its CTAs of 256 rows run in one
+    # wave, more than 512 keys) over several blocks
     (1, 2, 1100, 1100, 64, True, False, False, 0.0),
     (2, 2, 2048, 2048, 64, True, False, False, 0.0),
     (1, 3, 1536, 1000, 64, True, False, False, 0.0),    # more queries than keys: the early tiles see nothing
     (1, 2, 1000, 1500, 64, True, True, False, 0.0),     # key lengths
     (1, 2, 640, 640, 64, True, False, True, 5.0),       # dense mask and clamp
-    # enough pairs that the four-tile kernel's items fill the SMs about as well, and still no more items than SMs:
-    # causal launches take its folded tile mapping (two early and two late query tiles per item)
-    (5, 8, 1100, 1100, 64, True, False, False, 0.0),    # nine tiles in three blocks: three padded tile slots
+    # enough pairs that those CTAs are more than one wave: the one-tile kernel over several tiles of 128 rows
+    (5, 8, 1100, 1100, 64, True, False, False, 0.0),    # nine tiles, the last one ragged
     (4, 8, 2048, 2048, 64, True, False, False, 0.0),
     (5, 8, 1536, 1000, 64, True, False, False, 0.0),
     (5, 8, 1000, 1500, 64, True, True, False, 0.0),
     (8, 8, 640, 640, 64, True, False, True, 5.0),
-    (10, 16, 512, 700, 64, False, True, False, 0.0),    # more items than SMs: the plain mapping, items from a queue
+    (10, 16, 512, 700, 64, False, True, False, 0.0),    # more tiles than the GPU holds at once
 ]
 
 

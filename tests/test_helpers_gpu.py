@@ -88,8 +88,8 @@ def test_contexts_on_two_devices_of_one_process():
             g = torch.Generator(device=f"cuda:{dev}").manual_seed(9)
             q, k, v, do = ((torch.randn((1, 2, 640, 64), generator=g, device=f"cuda:{dev}") * 0.5).bfloat16()
                            for _ in range(4))
-            o, lse = c.attn_fwd(q, k, v, causal=True, mode=_lib.MODE_BF16)          # persistent 4-tile kernel
-            o2, _ = c.attn_fwd(q[:, :, :200], k, v, mode=_lib.MODE_BF16)             # 2-tile kernel
+            o, lse = c.attn_fwd(q, k, v, causal=True, mode=_lib.MODE_BF16)          # two-tile kernel (more than 512 keys)
+            o2, _ = c.attn_fwd(q[:, :, :200], k, v, mode=_lib.MODE_BF16)             # the same without a causal mask
             grads = c.attn_bwd(q, k, v, o, lse, do, causal=True)
             qf = q.float()
             of, lf = c.attn_fwd(qf, k.float(), v.float(), causal=True, mode=_lib.MODE_FP32)
