@@ -2343,6 +2343,7 @@ int launch_main(ltca_ctx* ctx, const ltca_attn_params* p, const void* mask_words
             LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(opt_fused, ctx->device, attn_bwd_fused_sm100_kernel<kMask>,
                                                   FusedSmem::kDynBytes));
             ItemGrid ig;
+            ig.group = kSchedGroup;
             ig.nblk = (p->Sk + kTile - 1) / kTile;
             ig.H = p->H;
             ig.BH = p->H * p->B;
@@ -2372,6 +2373,7 @@ int launch_main(ltca_ctx* ctx, const ltca_attn_params* p, const void* mask_words
             static SmemOptIn opt_dq4;
             LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(opt_dq4, ctx->device, attn_bwd_dq4_sm100_kernel<kMask>, Dq4Smem::kDynBytes));
             ItemGrid ig;
+            ig.group = kSchedGroup;
             ig.nblk = (p->Sq + kTile - 1) / kTile;
             ig.H = p->H;
             ig.BH = p->H * p->B;
@@ -2390,6 +2392,7 @@ int launch_main(ltca_ctx* ctx, const ltca_attn_params* p, const void* mask_words
             LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(opt_dkv4, ctx->device, attn_bwd_dkv4_sm100_kernel<kMask>,
                                                   Dkv4Smem::kDynBytes));
             ItemGrid ig;
+            ig.group = kSchedGroup;
             ig.nblk = (p->Sk + kTile - 1) / kTile;
             ig.H = p->H;
             ig.BH = p->H * p->B;

@@ -41,31 +41,8 @@ struct CoreArgs {
     int vec;            // every row starts on a 16-byte (fp32) or 8-byte (bf16) boundary and holds a multiple of 4 elements
 };
 
-// ---- packed fp32 pairs --------------------------------------------------------------------------
-// One instruction multiplies and adds two pairs of fp32 values, each half rounded as fmaf rounds it.  The products of
-// these kernels are bound by issue slots (loads, masks and exponentials share them with the multiply-adds), so halving
-// the number of multiply-add instructions is worth the second accumulator.
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-    f32x2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
-    f32x2 d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ f32x2 pair(float x, float y) {
-    f32x2 d;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(x), "f"(y));
-    return d;
-}
-__device__ __forceinline__ float2 halves(f32x2 v) {
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
+// The products of these kernels take packed fp32 pairs: they are bound by issue slots (loads, masks and exponentials share
+// them with the multiply-adds), so halving the number of multiply-add instructions is worth the second accumulator.
 
 // 16-byte asynchronous copy global -> shared; nothing is read and zeros are written when `bytes` is 0.
 __device__ __forceinline__ void cp_async16(float* dst, const void* src, int bytes) {

@@ -536,10 +536,16 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
 // dealt out in pieces of 128 rows.  A persistent kernel with four tiles on one key stream, which this replaces, made the
 // early tiles of 512 causal rows wait for the late ones' keys: B64 H8 S512 causal 68 us against 49, B8 H16 S4096 causal
 // 440 against 392.  What it pays is a set-up per tile and a K/V read per tile from L2 (20 bytes per clock and SM).
-//   - head_dim 64: warps 0-3 softmax, one row per thread, 64 keys per step; tensor memory S [0, 64), O [64, 128);
-//   - head_dim 128: warps 0-7, two threads per row, each 64 of the 128 keys of a step and 64 of the output columns (the row
-//     maxima meet through shared memory); S [0, 128), O [128, 256);
-//   - P overwrites the first half of S, its second bf16 term (kSplitP: results stored as fp32) the other half;
+//   - warps 0-3 softmax, one row per thread, head_dim keys per step; tensor memory S [0, D), O [D, 2 D).  At head_dim 128 a
+//     thread so holds 128 scores in its 216 registers and two warps share a scheduler; two threads per row, 64 scores each,
+//     had four of them but met once a step to agree on the row's maximum (B8 H16 S4096 causal 568 us, one per row 525).
+//     fp32 results at head_dim 128 have two threads per row (warps 0-7), which share the work of P's second term, and the
+//     halves of P below are one thread's each (B8 H16 S2048 causal 325 -> 319 us);
+//   - P overwrites the first half of S, its second bf16 term (kSplitP: results stored as fp32) the other half.  It is handed
+//     to the contraction in two halves of the keys, so that the first products run under the second half's exponentials
+//     (B8 H16 S4096 D64, not causal: one hand-over 721 us, two 698);
+//   - a step's V slot is returned before the next S is issued: with two slots at head_dim 128 the next V then arrives a
+//     contraction earlier (B1 H8 S4096 76 -> 65);
 //   - of the last four warps one issues the contractions and one is the TMA producer (the others complete the
 //     warpgroup that gives registers up);
 //   - the result leaves through the Q slot (fp32: and the ring) and a TMA store.
@@ -552,16 +558,17 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
 // where the plain form takes 396 there (four tiles that start together stay in step); on 132 SMs 516 us, B8 H16 S1024
 // causal 56, B64 H8 S512 causal 61.
 // ---------------------------------------------------------------------------------------------
-template <int D>
+template <int D, bool kSplitP>
 struct TileCfg {
-    static constexpr int kRowSplit = D / 64;                       // threads per row
+    static constexpr int kBN = D;                                  // keys per step
+    static constexpr int kRowSplit = D == 128 && kSplitP ? 2 : 1;  // threads per row
+    static constexpr int kCols = kBN / kRowSplit;                  // score columns of a thread
     static constexpr int kMathWarps = 4 * kRowSplit;
     static constexpr int kThreads = 32 * (kMathWarps + 4);
-    static constexpr int kCtas = 4 / kRowSplit;                    // per SM
+    static constexpr int kCtas = D == 64 ? 4 : 2;                  // per SM
     static constexpr int kLaunchRegs = 65536 / (kCtas * kThreads) / 8 * 8;
-    static constexpr int kMathRegs = 104, kCtrlRegs = D == 64 ? 24 : 32;
+    static constexpr int kMathRegs = kCols == 64 ? 104 : 216, kCtrlRegs = D == 64 ? 24 : kCols == 64 ? 32 : 40;
     static_assert(32 * kMathWarps * kMathRegs + 128 * kCtrlRegs <= kThreads * kLaunchRegs, "register budget");
-    static constexpr int kBN = D;                                  // keys per step
     static constexpr int kBlocks = D / 64;                         // 128-byte column blocks of a row
     static constexpr int kQBytes = kBlockM * D * 2;
     static constexpr int kKvBytes = kBN * D * 2;
@@ -569,7 +576,7 @@ struct TileCfg {
     static constexpr int kRingOff = kQBytes;
     static constexpr int kXchgOff = kRingOff + kStages * kKvBytes; // row maxima [2 buffers][2 halves][128], row sums [2][128]
     static constexpr int kBarOff = kXchgOff + (kRowSplit > 1 ? 3 * 2 * kBlockM * 4 : 0);
-    static constexpr int kNumBars = 1 + 2 * kStages + 3 + 4;       // q_full, kv_full[], kv_empty[], s_full, p_full, staged, pair[4]
+    static constexpr int kNumBars = 1 + 2 * kStages + 4 + 4;       // q_full, kv_full[], kv_empty[], s_full, p_full[2], staged, pair[4]
     static constexpr int kMiscOff = kBarOff + kNumBars * 8;        // tmem base, abort flag, a team's next tile
     static constexpr int kDynBytes = kMiscOff + 32 + 1024;
     static_assert(kCtas * (kDynBytes + 1024) <= 228 * 1024, "shared memory");
@@ -580,14 +587,14 @@ struct TileCfg {
 };
 
 template <int D, bool kSplitP, bool kMask, int kTeams>
-__global__ void __launch_bounds__(TileCfg<D>::kThreads * kTeams, kTeams > 1 ? 1 : TileCfg<D>::kCtas)
+__global__ void __launch_bounds__(TileCfg<D, kSplitP>::kThreads * kTeams, kTeams > 1 ? 1 : TileCfg<D, kSplitP>::kCtas)
 attn_fwd_tile_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                            const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_o, const FwdArgs a,
                            const ItemGrid items) {
-    using L = TileCfg<D>;
+    using L = TileCfg<D, kSplitP>;
     // (the teams share the registers and the tensor memory that as many CTAs of the plain form have on an SM)
     static_assert(kTeams == 1 || kTeams == L::kCtas, "one CTA or an SM's worth of them");
-    constexpr int kBN = L::kBN, kRS = L::kRowSplit, kMmaWarp = L::kMathWarps, kTmaWarp = L::kMathWarps + 1;
+    constexpr int kBN = L::kBN, kRS = L::kRowSplit, kC = L::kCols, kMmaWarp = L::kMathWarps, kTmaWarp = L::kMathWarps + 1;
     extern __shared__ uint8_t smem_raw[];
     // (through a shuffle: what follows from it is then known to be the same in a whole warp, which the operands of the
     // tensor-core instructions have to be)
@@ -599,7 +606,7 @@ attn_fwd_tile_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
     auto bar_kv_full = [&](int s) { return bar_base + 8u * (1 + s); };
     auto bar_kv_empty = [&](int s) { return bar_base + 8u * (1 + L::kStages + s); };
     const uint32_t bar_q_full = bar_base, bar_s_full = bar_base + 8u * (1 + 2 * L::kStages), bar_p_full = bar_s_full + 8,
-                   bar_staged = bar_s_full + 16, bar_pair0 = bar_s_full + 24;
+                   bar_staged = bar_s_full + 24, bar_pair0 = bar_s_full + 32;
     volatile uint32_t* misc = reinterpret_cast<volatile uint32_t*>(smem_gen + L::kMiscOff);
     volatile uint32_t* misc_cta = reinterpret_cast<volatile uint32_t*>(smem_raw + (smem_cta - smem_u32(smem_raw)) + L::kMiscOff);
     const int warp = kTeams > 1 ? __shfl_sync(0xffffffffu, tid >> 5, 0) : tid >> 5, lane = tid & 31;
@@ -608,7 +615,8 @@ attn_fwd_tile_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
         mbar_init(bar_q_full, 1);
         for (int s = 0; s < L::kStages; ++s) { mbar_init(bar_kv_full(s), 1); mbar_init(bar_kv_empty(s), 1); }
         mbar_init(bar_s_full, 1);
-        mbar_init(bar_p_full, L::kMathWarps);
+        mbar_init(bar_p_full, 4);
+        mbar_init(bar_p_full + 8u, 4);
         mbar_init(bar_staged, L::kMathWarps);
         for (int i = 0; i < 4; ++i) mbar_init(bar_pair0 + 8u * i, 2);
         misc[1] = 0u;
@@ -666,7 +674,7 @@ attn_fwd_tile_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
             if (!misc[2]) return false;
             q0 = (int)misc[3]; h = (int)misc[4]; b = (int)misc[5]; kvlen = (int)misc[6]; n_t = (int)misc[7];
         } else {
-            sched_block(rank, h, b);
+            sched_block(rank, h, b, items.group);
             take(rank, (int)gridDim.x);
         }
         return true;
@@ -700,32 +708,41 @@ attn_fwd_tile_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
                         mma_ss_lo(tmem_base, q_lo + (k / 4) * (kBlockM * 8) + (k % 4) * 2,
                                   k_lo + ((s * L::kKvBytes) >> 4) + (k / 4) * (kBN * 8) + (k % 4) * 2, idesc_qk, k > 0 ? 1u : 0u);
                 };
+                auto issue_pv = [&](int s, int part, bool first) {     // one half of the step's keys
+                    constexpr int kSteps = kBN / 32;
+                    const uint32_t vd = v_lo + ((s * L::kKvBytes) >> 4);
+    #pragma unroll
+                    for (int t = 0; t < (kSplitP ? 2 : 1); ++t)
+    #pragma unroll
+                        for (int k = 0; k < kSteps; ++k)
+                            mma_ts_lo(tmem_base + kBN, tmem_base + (kBN / 2) * t + (part * kSteps + k) * 8, vd + 128 * (part * kSteps + k),
+                                      idesc_pv, (!first || t > 0 || k > 0) ? 1u : 0u);
+                };
                 bool ok = mbar_wait(bar_q_full, (uint32_t)(tiles & 1), wc, 0x51) && mbar_wait(bar_kv_full(slot_of(e0)), phase_of(e0), wc, 0x52);
                 if (ok) {
                     tc_fence_after_sync();
                     issue_qk(slot_of(e0));
-                    mma_commit(bar_s_full);
                     mma_commit(bar_kv_empty(slot_of(e0)));
+                    mma_commit(bar_s_full);
                 }
                 for (int j = 0; j < n_t && ok; ++j) {
                     const int e_v = e0 + 2 * j + 1, e_k = e0 + 2 * j + 2;
                     const bool more = j + 1 < n_t;
                     ok = mbar_wait(bar_kv_full(slot_of(e_v)), phase_of(e_v), wc, 0x53);
                     if (more) ok = ok && mbar_wait(bar_kv_full(slot_of(e_k)), phase_of(e_k), wc, 0x54);
-                    ok = ok && mbar_wait(bar_p_full, (uint32_t)((steps + j) & 1), wc, 0x55);
+                    for (int part = 0; part < 2 && ok; ++part) {
+                        ok = mbar_wait(bar_p_full + 8u * part, (uint32_t)((steps + j) & 1), wc, 0x55);
+                        if (!ok) break;
+                        tc_fence_after_sync();
+                        issue_pv(slot_of(e_v), part, j == 0 && part == 0);
+                    }
                     if (!ok) break;
-                    tc_fence_after_sync();
-                    const uint32_t vd = v_lo + ((slot_of(e_v) * L::kKvBytes) >> 4);
-    #pragma unroll
-                    for (int t = 0; t < (kSplitP ? 2 : 1); ++t)
-    #pragma unroll
-                        for (int k = 0; k < kBN / 16; ++k)
-                            mma_ts_lo(tmem_base + kBN, tmem_base + (kBN / 2) * t + k * 8, vd + 128 * k, idesc_pv,
-                                      (j > 0 || t > 0 || k > 0) ? 1u : 0u);
-                    if (more) issue_qk(slot_of(e_k));
-                    mma_commit(bar_s_full);                            // S of step j + 1 ready, O holds steps 0 .. j
                     mma_commit(bar_kv_empty(slot_of(e_v)));
-                    if (more) mma_commit(bar_kv_empty(slot_of(e_k)));
+                    if (more) {
+                        issue_qk(slot_of(e_k));
+                        mma_commit(bar_kv_empty(slot_of(e_k)));
+                    }
+                    mma_commit(bar_s_full);                            // S of step j + 1 ready, O holds steps 0 .. j
                 }
             }
         } while (kTeams > 1);
@@ -734,8 +751,8 @@ attn_fwd_tile_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
         const int wq = warp & 3, half = kRS > 1 ? warp >> 2 : 0;
         const int row = wq * 32 + lane;
         const uint32_t lane_base = (uint32_t)(wq * 32) << 16;
-        const uint32_t tS = tmem_base + lane_base + half * 64, tO = tmem_base + lane_base + kBN + half * 64;
-        const uint32_t tP = tmem_base + lane_base + half * 32, tPlo = tP + kBN / 2;
+        const uint32_t tS = tmem_base + lane_base + half * kC, tO = tmem_base + lane_base + kBN + half * (D / kRS);
+        const uint32_t tP = tmem_base + lane_base + half * (kC / 2), tPlo = tP + kBN / 2;
         float* xchg = reinterpret_cast<float*>(smem_gen + L::kXchgOff);
         auto xslot = [&](int buf, int hf) { return xchg + (buf * 2 + hf) * kBlockM + row; };
         // the row's other thread has published its value too
@@ -763,22 +780,24 @@ attn_fwd_tile_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
             float m_run = neg_inf(), l_run = 0.f;
             bool ok = true;
             for (int j = 0; j < n_t; ++j) {
-                uint32_t keep[2];                                      // dense mask of this thread's 64 columns
+                uint32_t keep[kC / 32];                                // dense mask of this thread's columns
     #pragma unroll
-                for (int w = 0; w < 2; ++w)
-                    keep[w] = kMask ? mask_bits_of_queries(a.mask, b, q0 + wq * 32, j * kBN + half * 64 + 32 * w) : ~0u;
+                for (int w = 0; w < kC / 32; ++w)
+                    keep[w] = kMask ? mask_bits_of_queries(a.mask, b, q0 + wq * 32, j * kBN + half * kC + 32 * w) : ~0u;
                 ok = mbar_wait_warp(bar_s_full, (uint32_t)((s_full0 + j) & 1), wc, 0x56);
                 if (!ok) break;
                 tc_fence_after_sync();
-                uint32_t su[64];
-                tmem_ld32(tS, reinterpret_cast<uint32_t(&)[32]>(su[0]));
-                tmem_ld32(tS + 32, reinterpret_cast<uint32_t(&)[32]>(su[32]));
+                uint32_t su[kC];
+    #pragma unroll
+                for (int c = 0; c < kC; c += 32) tmem_ld32(tS + c, reinterpret_cast<uint32_t(&)[32]>(su[c]));
                 tmem_wait_ld();
+    #pragma unroll
+                for (int c = 0; c < kC; c += 32) tmem_ld_fence(reinterpret_cast<uint32_t(&)[32]>(su[c]));
     #define S_(c) __uint_as_float(su[(c)])
-                const int lim_c = lim_row - j * kBN - half * 64;       // own columns c < lim_c are visible
+                const int lim_c = lim_row - j * kBN - half * kC;       // own columns c < lim_c are visible
                 if (general) {
     #pragma unroll
-                    for (int c = 0; c < 64; ++c) {
+                    for (int c = 0; c < kC; ++c) {
                         float v = S_(c);
                         if (a.use_clamp) v = fminf(v, a.clamp_raw);
                         const bool vis = c < lim_c && (keep[c / 32] >> (c % 32) & 1u);
@@ -786,13 +805,13 @@ attn_fwd_tile_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
                     }
                 } else if (j >= je) {
     #pragma unroll
-                    for (int c = 0; c < 64; ++c) su[c] = (c < lim_c) ? su[c] : 0xff800000u;
+                    for (int c = 0; c < kC; ++c) su[c] = (c < lim_c) ? su[c] : 0xff800000u;
                 }
                 float mx[4];
     #pragma unroll
                 for (int i = 0; i < 4; ++i) mx[i] = fmaxf(S_(2 * i), S_(2 * i + 1));
     #pragma unroll
-                for (int c = 8; c < 64; c += 8)
+                for (int c = 8; c < kC; c += 8)
     #pragma unroll
                     for (int i = 0; i < 4; ++i) mx[i] = fmax3(mx[i], S_(c + 2 * i), S_(c + 2 * i + 1));
                 float mt = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
@@ -818,7 +837,7 @@ attn_fwd_tile_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
                 }
                 if (j > 0 && __any_sync(0xffffffffu, need)) {
     #pragma unroll 1
-                    for (int c0 = 0; c0 < 64; c0 += 16) {
+                    for (int c0 = 0; c0 < D / kRS; c0 += 16) {
                         uint32_t o[16];
                         tmem_ld16(tO + c0, o);
                         tmem_wait_ld();
@@ -829,19 +848,19 @@ attn_fwd_tile_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
                     l_run *= factor;
                 }
                 const float m_safe = (m_run == neg_inf()) ? 0.f : m_run;
-                const float mneg = -m_safe * c2;
-                float sum0 = 0.f, sum1 = 0.f, sum2 = 0.f, sum3 = 0.f;
+                const f32x2 c2_2 = pair(c2, c2), mneg_2 = pair(-m_safe * c2, -m_safe * c2);
+                f32x2 sum01 = pair(0.f, 0.f), sum23 = sum01;
     #pragma unroll
-                for (int ch = 0; ch < 2; ++ch) {
+                for (int ch = 0; ch < kC / 32; ++ch) {
                     uint32_t hi[16], lo[16];
     #pragma unroll
                     for (int cc = 0; cc < 32; cc += 4) {
                         const int c = ch * 32 + cc;
-                        const float p0 = fast_exp2(fmaf(S_(c), c2, mneg));
-                        const float p1 = fast_exp2(fmaf(S_(c + 1), c2, mneg));
-                        const float p2 = fast_exp2(fmaf(S_(c + 2), c2, mneg));
-                        const float p3 = fast_exp2(fmaf(S_(c + 3), c2, mneg));
-                        sum0 += p0; sum1 += p1; sum2 += p2; sum3 += p3;
+                        const float2 x01 = halves(fma2(pair(S_(c), S_(c + 1)), c2_2, mneg_2));
+                        const float2 x23 = halves(fma2(pair(S_(c + 2), S_(c + 3)), c2_2, mneg_2));
+                        const float p0 = fast_exp2(x01.x), p1 = fast_exp2(x01.y), p2 = fast_exp2(x23.x), p3 = fast_exp2(x23.y);
+                        sum01 = add2(sum01, pair(p0, p1));
+                        sum23 = add2(sum23, pair(p2, p3));
                         const uint32_t h01 = pack_bf16x2(p0, p1), h23 = pack_bf16x2(p2, p3);
                         hi[cc / 2] = h01;
                         hi[cc / 2 + 1] = h23;
@@ -852,12 +871,16 @@ attn_fwd_tile_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
                     }
                     tmem_st16(tP + ch * 16, hi);                       // P over S (all of S is in registers)
                     if constexpr (kSplitP) tmem_st16(tPlo + ch * 16, lo);
+                    constexpr int kHalf = kBN / 64;                    // pieces in one half of the step's keys
+                    if (ch % kHalf == kHalf - 1) {                     // their contraction may begin
+                        tmem_wait_st();
+                        tc_fence_before_sync();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(bar_p_full + 8u * (half + ch / kHalf));
+                    }
                 }
-                l_run += (sum0 + sum1) + (sum2 + sum3);
-                tmem_wait_st();
-                tc_fence_before_sync();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(bar_p_full);
+                const float2 s01 = halves(sum01), s23 = halves(sum23);
+                l_run += (s01.x + s01.y) + (s23.x + s23.y);
     #undef S_
             }
             const int qi = q0 + row;
@@ -876,26 +899,32 @@ attn_fwd_tile_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
                     lse = m_run * a.scale + __logf(l_run);
                 }
                 if (ok) {
-                    uint32_t o[64];
-                    tmem_ld32(tO, reinterpret_cast<uint32_t(&)[32]>(o[0]));
-                    tmem_ld32(tO + 32, reinterpret_cast<uint32_t(&)[32]>(o[32]));
-                    tmem_wait_ld();
                     // every operand has been read: Q's slot (and the ring) take the result as 128-byte-swizzled boxes
     #pragma unroll
-                    for (int v = 0; v < (kSplitP ? 16 : 8); ++v) {
-                        uint4 w;
-                        if constexpr (kSplitP) {
-                            w = make_uint4(__float_as_uint(__uint_as_float(o[4 * v]) * inv), __float_as_uint(__uint_as_float(o[4 * v + 1]) * inv),
-                                           __float_as_uint(__uint_as_float(o[4 * v + 2]) * inv),
-                                           __float_as_uint(__uint_as_float(o[4 * v + 3]) * inv));
-                        } else {
-                            w.x = pack_bf16x2(__uint_as_float(o[8 * v + 0]) * inv, __uint_as_float(o[8 * v + 1]) * inv);
-                            w.y = pack_bf16x2(__uint_as_float(o[8 * v + 2]) * inv, __uint_as_float(o[8 * v + 3]) * inv);
-                            w.z = pack_bf16x2(__uint_as_float(o[8 * v + 4]) * inv, __uint_as_float(o[8 * v + 5]) * inv);
-                            w.w = pack_bf16x2(__uint_as_float(o[8 * v + 6]) * inv, __uint_as_float(o[8 * v + 7]) * inv);
+                    for (int ob = 0; ob < D / 64 / kRS; ++ob) {
+                        uint32_t o[64];
+                        tmem_ld32(tO + ob * 64, reinterpret_cast<uint32_t(&)[32]>(o[0]));
+                        tmem_ld32(tO + ob * 64 + 32, reinterpret_cast<uint32_t(&)[32]>(o[32]));
+                        tmem_wait_ld();
+                        tmem_ld_fence(reinterpret_cast<uint32_t(&)[32]>(o[0]));
+                        tmem_ld_fence(reinterpret_cast<uint32_t(&)[32]>(o[32]));
+    #pragma unroll
+                        for (int v = 0; v < (kSplitP ? 16 : 8); ++v) {
+                            uint4 w;
+                            if constexpr (kSplitP) {
+                                w = make_uint4(__float_as_uint(__uint_as_float(o[4 * v]) * inv),
+                                               __float_as_uint(__uint_as_float(o[4 * v + 1]) * inv),
+                                               __float_as_uint(__uint_as_float(o[4 * v + 2]) * inv),
+                                               __float_as_uint(__uint_as_float(o[4 * v + 3]) * inv));
+                            } else {
+                                w.x = pack_bf16x2(__uint_as_float(o[8 * v + 0]) * inv, __uint_as_float(o[8 * v + 1]) * inv);
+                                w.y = pack_bf16x2(__uint_as_float(o[8 * v + 2]) * inv, __uint_as_float(o[8 * v + 3]) * inv);
+                                w.z = pack_bf16x2(__uint_as_float(o[8 * v + 4]) * inv, __uint_as_float(o[8 * v + 5]) * inv);
+                                w.w = pack_bf16x2(__uint_as_float(o[8 * v + 6]) * inv, __uint_as_float(o[8 * v + 7]) * inv);
+                            }
+                            const int box = (half + ob) * (kSplitP ? 2 : 1) + v / 8;
+                            *reinterpret_cast<uint4*>(smem_gen + box * (kBlockM * 128) + row * 128 + (((v % 8) ^ (row & 7)) << 4)) = w;
                         }
-                        const int box = half * (kSplitP ? 2 : 1) + v / 8;
-                        *reinterpret_cast<uint4*>(smem_gen + box * (kBlockM * 128) + row * 128 + (((v % 8) ^ (row & 7)) << 4)) = w;
                     }
                     fence_proxy_async_smem();
                 }
@@ -912,9 +941,9 @@ attn_fwd_tile_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
                 // no key is visible to these rows: zeros and -inf
                 using OutT = typename std::conditional<kSplitP, float, __nv_bfloat16>::type;
                 uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<OutT*>(a.o) + b * a.o_sb + h * a.o_sh + (int64_t)qi * a.o_ss +
-                                                      half * 64);
+                                                      half * (D / kRS));
     #pragma unroll
-                for (int v = 0; v < (kSplitP ? 16 : 8); ++v) dst[v] = make_uint4(0u, 0u, 0u, 0u);
+                for (int v = 0; v < D / kRS * (int)sizeof(OutT) / 16; ++v) dst[v] = make_uint4(0u, 0u, 0u, 0u);
                 if (half == 0 && a.lse) a.lse[stat] = neg_inf();
             }
         } while (kTeams > 1);
@@ -939,7 +968,7 @@ attn_fwd_tile_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
 template <int D, bool kSplitP>
 int launch_fwd_tile(ltca_ctx* ctx, const ltca_attn_params* p, const void* q, const void* k, const void* v, const ltca_strides& qs,
                     const ltca_strides& ks, const ltca_strides& vs, const FwdArgs& a) {
-    using L = TileCfg<D>;
+    using L = TileCfg<D, kSplitP>;
     CUtensorMap tq, tk, tv, to;
     int rc;
     if ((rc = make_tmap_bhsd(ctx, &tq, q, 2, p->B, p->H, p->Sq, D, qs, 64, kBlockM))) return rc;
@@ -948,6 +977,7 @@ int launch_fwd_tile(ltca_ctx* ctx, const ltca_attn_params* p, const void* q, con
     if ((rc = make_tmap_bhsd(ctx, &to, p->o, kSplitP ? 4 : 2, p->B, p->H, p->Sq, D, p->o_strides, kSplitP ? 32 : 64, kBlockM))) return rc;
     ItemGrid items;
     memset(&items, 0, sizeof(items));
+    items.group = sched_group((int64_t)p->B * p->H, 4ll * p->Sk * D);
     // bf16 results at head_dim 64 keep to the SMs that the context allows: what a sequence-sharded run computes while slices
     // are on their way between the GPUs.
     if constexpr (D == 64 && !kSplitP) {

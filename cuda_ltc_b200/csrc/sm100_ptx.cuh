@@ -422,18 +422,18 @@ __device__ __forceinline__ void reg_dealloc() {
 
 // ---- CTA order for causal work ----------------------------------------------------------------
 // Thread blocks start in the order of their linear index.  The (batch, head) pairs are taken in
-// groups of kSchedGroup; inside a group every pair's heaviest block starts first, then every
+// groups (kSchedGroup of them, or what sched_group says); inside a group every pair's heaviest block starts first, then every
 // pair's second heaviest, and so on, so the long blocks of a launch never start last (short
 // tail), while one group's K / V / Q / dO (a few tens of MB) stay resident in L2.
 constexpr int kSchedGroup = 16;
-__device__ __forceinline__ void sched_block(int& rank, int& h, int& b) {
+__device__ __forceinline__ void sched_block(int& rank, int& h, int& b, int group) {
     const int nblk = gridDim.x, H = gridDim.y, BH = gridDim.y * gridDim.z;
     const int linear = blockIdx.x + nblk * (blockIdx.y + H * blockIdx.z);
-    const int g = linear / (kSchedGroup * nblk);
-    const int n_in = min(kSchedGroup, BH - g * kSchedGroup);
-    const int local = linear - g * kSchedGroup * nblk;
+    const int g = linear / (group * nblk);
+    const int n_in = min(group, BH - g * group);
+    const int local = linear - g * group * nblk;
     rank = local / n_in;
-    const int bh = g * kSchedGroup + local % n_in;
+    const int bh = g * group + local % n_in;
     h = bh % H;
     b = bh / H;
 }
@@ -488,17 +488,59 @@ __device__ __forceinline__ void item_counters_release(int* counters) {
 }
 
 // The item list of a persistent kernel: nblk row blocks for each of BH (batch, head) pairs.
-struct ItemGrid { int nblk, H, BH, n_items; int* counters; };
+struct ItemGrid { int nblk, H, BH, n_items; int* counters; int group; };
+
+// The forward's group: as many pairs as leave 48 MB of K and V for a group's tiles to share in L2 (whose 126 MB also see the
+// queries and the results go by), the pairs dealt out evenly: with a small last group the launch ends on its few tiles.
+// Tiles are short (128 rows), so more pairs side by side mean a shorter tail.  B8 H16 S4096 D64 causal 406 us in groups of 16
+// pairs, 374 in three of 43 (395 with 48, 48 and 32); B16 H16 S1024 82 and 72; the ragged prefill B4 H16 S1500 D128 51.3
+// and 49.2.  The backward kernels, whose blocks take five tensors through L2, gained nothing and keep kSchedGroup.
+inline int sched_group(int64_t pairs, int64_t kv_bytes_per_pair) {
+    int64_t n = (int64_t(48) << 20) / (kv_bytes_per_pair > 0 ? kv_bytes_per_pair : 1);
+    if (n < kSchedGroup) n = kSchedGroup;
+    const int64_t groups = (pairs + n - 1) / n;           // of equal size
+    return (int)((pairs + groups - 1) / groups);
+}
 
 // Entry `linear` of the grouped heavy-first order (see sched_block): rank 0 is the heaviest block.
 __device__ __forceinline__ void sched_item(const ItemGrid& g, int linear, int& rank, int& h, int& b) {
-    const int grp = linear / (kSchedGroup * g.nblk);
-    const int n_in = min(kSchedGroup, g.BH - grp * kSchedGroup);
-    const int local = linear - grp * kSchedGroup * g.nblk;
+    const int grp = linear / (g.group * g.nblk);
+    const int n_in = min(g.group, g.BH - grp * g.group);
+    const int local = linear - grp * g.group * g.nblk;
     rank = local / n_in;
-    const int bh = grp * kSchedGroup + local % n_in;
+    const int bh = grp * g.group + local % n_in;
     h = bh % g.H;
     b = bh / g.H;
+}
+
+// ---- packed fp32 pairs ------------------------------------------------------------------------
+// One instruction works on two pairs of fp32 values, each half rounded as the single instruction rounds it.  A pair takes
+// its unit as long as two single instructions do, but one issue slot instead of two.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ f32x2 pair(float x, float y) {
+    f32x2 d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(x), "f"(y));
+    return d;
+}
+__device__ __forceinline__ float2 halves(f32x2 v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
 }
 
 // ---- small math helpers -----------------------------------------------------------------------
