@@ -6,7 +6,8 @@
 
 namespace ltca {
 
-// All matrices are bf16 views [batch, head, seq, width] given by element strides (multiples of 8).
+// All matrices are bf16 views [batch, head, seq, width] given by element strides (multiples of 8); a head stride of 0 is one
+// matrix for all heads.
 struct WideArgs {
     int B = 0, H = 0, Sq = 0, Sk = 0, D = 0;
     int causal = 0;
@@ -27,7 +28,7 @@ struct WideArgs {
     // backward
     const void* dout = nullptr; ltca_strides dos{};
     const void* doutl = nullptr;                // optional low-order part of dO (same strides)
-    void *dq = nullptr, *dk = nullptr, *dv = nullptr;
+    void *dq = nullptr, *dk = nullptr, *dv = nullptr;       // (dk may be null)
     ltca_strides dqs{}, dks{}, dvs{};
     int grads_bf16 = 1;
     float* dP = nullptr;                        // scratch fp32 [B*H, Sq, Skp]
@@ -45,5 +46,7 @@ bool wide_supported(int D, const ltca_strides& qs, const ltca_strides& ks, const
 int wide_attn_fwd(ltca_ctx* ctx, const WideArgs& w);
 // dQ, dK, dV from dO; expects `scores` and `P` as wide_attn_fwd left them for the same inputs.
 int wide_attn_bwd(ltca_ctx* ctx, const WideArgs& w);
+// its last step, dK = dS^T Q, alone
+int wide_key_grad(ltca_ctx* ctx, const WideArgs& w);
 
 }  // namespace ltca

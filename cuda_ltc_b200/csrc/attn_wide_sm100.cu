@@ -326,6 +326,7 @@ int batched(ltca_ctx* ctx, const WideArgs& w, int M, int N, int K, const Mat* a,
     }
     gp.a_bs[0] = a[0].hs; gp.a_bs[1] = a[0].bs;
     gp.b_bs[0] = b[0].hs; gp.b_bs[1] = b[0].bs;
+    gp.a_shared = a[0].hs == 0; gp.b_shared = b[0].hs == 0;    // one matrix for all heads
     gp.c[0] = c;
     gp.ldc = ldc;
     gp.c_bs[0] = c_hs; gp.c_bs[1] = c_bs;
@@ -450,15 +451,20 @@ int wide_attn_bwd(ltca_ctx* ctx, const WideArgs& w) {
                           w.grads_bf16)))
             return rc;
     }
-    {   // dK = dS^T Q : dS stored [Sq, Sk] = [K, M], Q stored [Sq, D] = [K, N]
-        Mat a[3] = {{sa.dS, Skp, 1, mat, mat_b}, {sa.dSlo, Skp, 1, mat, mat_b}, {sa.dS, Skp, 1, mat, mat_b}};
-        Mat b[3] = {{w.qh, w.qs.seq, 1, w.qs.head, w.qs.batch}, {w.qh, w.qs.seq, 1, w.qs.head, w.qs.batch},
-                    {w.ql, w.qs.seq, 1, w.qs.head, w.qs.batch}};
-        if ((rc = batched(ctx, w, w.Sk, w.D, w.Sq, a, b, full ? 3 : terms, w.dk, w.dks.seq, w.dks.head, w.dks.batch,
-                          w.grads_bf16)))
-            return rc;
-    }
-    return LTCA_OK;
+    return w.dk ? wide_key_grad(ctx, w) : LTCA_OK;
+}
+
+int wide_key_grad(ltca_ctx* ctx, const WideArgs& w) {
+    const int Skp = wide_padded_keys(w.Sk);
+    const int64_t mat = (int64_t)w.Sq * Skp, mat_b = (int64_t)w.H * mat;
+    const bool full = w.Plo && w.vl && w.doutl && w.ql && w.kl;
+    const SoftmaxArgs sa = softmax_args(w);
+    // dS stored [Sq, Sk] = [K, M], Q stored [Sq, D] = [K, N]
+    Mat a[3] = {{sa.dS, Skp, 1, mat, mat_b}, {sa.dSlo, Skp, 1, mat, mat_b}, {sa.dS, Skp, 1, mat, mat_b}};
+    Mat b[3] = {{w.qh, w.qs.seq, 1, w.qs.head, w.qs.batch}, {w.qh, w.qs.seq, 1, w.qs.head, w.qs.batch},
+                {w.ql, w.qs.seq, 1, w.qs.head, w.qs.batch}};
+    return batched(ctx, w, w.Sk, w.D, w.Sq, a, b, full ? 3 : (w.Plo ? 2 : 1), w.dk, w.dks.seq, w.dks.head, w.dks.batch,
+                   w.grads_bf16);
 }
 
 }  // namespace ltca

@@ -29,6 +29,8 @@
 // (weight gradients: K = batch x time is long and M x N is small, so the K range is cut into
 // slices whose partial tiles go to scratch and are summed in a fixed order by a second kernel).
 // `n_sum` > 1 accumulates several operand pairs into one tile (dx = dq Wq^T + dk Wk^T + dv Wv^T).
+#include <type_traits>
+
 #include "host_common.h"
 #include "gemm_sm100.h"
 #include "attn_wide.h"
@@ -68,20 +70,29 @@ struct GemmCfg {
 };
 
 struct GemmMaps { CUtensorMap a[kMaxGemmProblems], b[kMaxGemmProblems], c[kMaxGemmProblems]; };
+// A group's: up to three terms each, second terms of the results behind the first.
+struct GemmGroupMaps {
+    CUtensorMap a[3 * kMaxGemmProblems], b[3 * kMaxGemmProblems], c[2 * kMaxGemmProblems];
+    int first[kMaxGemmProblems + 1];   // a member's pairs
+    int form[kMaxGemmProblems];        // ... and operand forms (bit 0: A stored [K, M], bit 1: B stored [K, N])
+};
 
 struct GemmKArgs {
     int M, N, K;
     int n_sum, ksplit;
     int tiles_x, tiles_y, tiles_z;   // N tiles, M tiles, problems x K slices
     int batch_h, batch_b;            // independent products of the same shape (slowest index of the tile list)
+    int sum_h;                       // heads whose products one tile sums up
+    int a_head, b_head;              // 0: the heads share the operand
+    int out_bf16;
+    int tma_store;                   // results leave through shared memory and a TMA store (needs 16-byte aligned rows)
+    int add_to_c;
     int64_t c_bs[2];                 // element strides of C over (h, b)
     int64_t ldc;
-    int out_bf16;
-    int tma_store;           // results leave through shared memory and a TMA store (needs 16-byte aligned rows)
     void* C[kMaxGemmProblems];
-    void* c_lo;              // second bf16 term of the (single) result, or null; its tensor map is c[1]
+    void* c_lo;                      // second bf16 term of the (single) result, or null; its tensor map is c[1]
     const float* bias[kMaxGemmProblems];
-    float* partial;          // [problem][slice][M][N] when ksplit > 1
+    float* partial;                  // [problem][slice][M][N] when ksplit > 1
     uint32_t* status;
 };
 
@@ -90,8 +101,8 @@ struct GemmTile {
     int m0, n0, problem, slice, kb_begin, kb_end, pair_begin, n_pairs, n_iters;
     int bh, bb;                      // batch entry
 };
-template <int kBN, int kTileM>
-__device__ __forceinline__ GemmTile gemm_tile(const GemmKArgs& g, int linear, int rank) {
+template <int kBN, int kTileM, typename Maps>
+__device__ __forceinline__ GemmTile gemm_tile(const Maps& maps, const GemmKArgs& g, int sum_h, int linear, int rank) {
     GemmTile t;
     const int x = linear % g.tiles_x;
     const int yz = linear / g.tiles_x;
@@ -107,20 +118,40 @@ __device__ __forceinline__ GemmTile gemm_tile(const GemmKArgs& g, int linear, in
     const int per = (nkb + g.ksplit - 1) / g.ksplit;
     t.kb_begin = min(t.slice * per, nkb);
     t.kb_end = min(t.kb_begin + per, nkb);
-    t.pair_begin = g.n_sum > 1 ? 0 : t.problem;
-    t.n_pairs = g.n_sum > 1 ? g.n_sum : 1;
-    t.n_iters = t.n_pairs * (t.kb_end - t.kb_begin);
+    if constexpr (std::is_same<Maps, GemmGroupMaps>::value) {
+        t.pair_begin = maps.first[t.problem];
+        t.n_pairs = maps.first[t.problem + 1] - t.pair_begin;
+    } else {
+        t.pair_begin = g.n_sum > 1 ? 0 : t.problem;
+        t.n_pairs = g.n_sum > 1 ? g.n_sum : 1;
+    }
+    t.n_iters = t.n_pairs * sum_h * (t.kb_end - t.kb_begin);
     return t;
+}
+
+template <bool kByMember, bool kMn, typename Maps>
+__device__ __forceinline__ bool is_mn(const Maps& maps, int problem, int bit) {
+    if constexpr (kByMember) return (maps.form[problem] & bit) != 0;
+    return kMn;
 }
 
 // Persistent: CTA (or pair) c computes tiles c, c + their number, ... of the list (N tiles fastest, so neighbouring CTAs
 // share their rows of A in L2).  The two accumulators alternate: while the epilogue warps read tile i out of
 // tensor memory, convert it and hand it to the TMA store, the MMA thread is already accumulating tile i+1 and
 // the producer is loading tile i+2's operands.
-template <bool kAMn, bool kBMn, int kBN, bool kPair>
+// kKind: kHeads has operands that heads share, sums over heads and results that are added to C (the plain kernel is free of
+// them: they cost it 0.1 us a launch); the members of a kGroup differ in their operand forms (kAMn, kBMn do not count) and
+// their number of terms.  Four weight gradients of 8 x 512 x 512 x 512 with three and two terms: 55 us as four launches, 31 as
+// one.
+enum GemmKind { kPlain, kHeads, kGroup };
+template <bool kAMn, bool kBMn, int kBN, bool kPair, int kKind>
 __global__ void __launch_bounds__(kGemmThreads, 1)
-gemm_bf16_sm100_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ GemmKArgs g) {
+gemm_bf16_sm100_kernel(const __grid_constant__ typename std::conditional<kKind == kGroup, GemmGroupMaps, GemmMaps>::type maps,
+                       const __grid_constant__ GemmKArgs g) {
+    const int sum_h = kKind == kHeads ? g.sum_h : 1;
+    const bool add_to_c = kKind == kHeads && g.add_to_c;
     using L = GemmCfg<kBN, kPair>;
+    static_assert(kKind != kGroup || !kPair, "groups run on single CTAs");
     constexpr int kStages = L::kStages, kStageBytes = L::kStageBytes;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -170,11 +201,13 @@ gemm_bf16_sm100_kernel(const __grid_constant__ GemmMaps maps, const __grid_const
             bool ok = true;
             int it = 0;
             for (int lin = kPair ? blockIdx.x >> 1 : blockIdx.x; lin < n_tiles && ok; lin += kPair ? gridDim.x >> 1 : gridDim.x) {
-                const GemmTile t = gemm_tile<kBN, L::kTileM>(g, lin, rank);
-                for (int p = 0; p < t.n_pairs && ok; ++p) {
+                const GemmTile t = gemm_tile<kBN, L::kTileM>(maps, g, sum_h, lin, rank);
+                const bool amn = is_mn<kKind == kGroup, kAMn>(maps, t.problem, 1), bmn = is_mn<kKind == kGroup, kBMn>(maps, t.problem, 2);
+                for (int p = 0, head = t.bh; p < t.n_pairs && ok; ++head == t.bh + sum_h ? (++p, head = t.bh) : 0) {
                     const int pair = t.pair_begin + p;
                     const CUtensorMap* ta = &maps.a[pair];
                     const CUtensorMap* tb = &maps.b[pair];
+                    const int ha = kKind == kHeads && !g.a_head ? 0 : head, hb = kKind == kHeads && !g.b_head ? 0 : head;
                     for (int kb = t.kb_begin; kb < t.kb_end; ++kb, ++it) {
                         const int s = it % kStages;
                         ok = mbar_wait(bar_empty(s), (uint32_t)(((it / kStages) & 1) ^ 1), wc, 0xd0);
@@ -183,25 +216,25 @@ gemm_bf16_sm100_kernel(const __grid_constant__ GemmMaps maps, const __grid_const
                         // a pair's loads all signal the issuing CTA's barrier
                         if (rank == 0) mbar_arrive_expect_tx(bar_full(s), (uint32_t)(kPair ? 2 : 1) * kStageBytes);
                         const uint32_t bar = kPair ? map_shared(bar_full(s), 0) : bar_full(s);
-                        auto load = [&](uint32_t dst, const CUtensorMap* map, int c0, int c1) {
-                            if constexpr (kPair) tma_load_4d_pair(dst, map, bar, c0, c1, t.bh, t.bb);
-                            else tma_load_4d(dst, map, bar, c0, c1, t.bh, t.bb);
+                        auto load = [&](uint32_t dst, const CUtensorMap* map, int c0, int c1, int h) {
+                            if constexpr (kPair) tma_load_4d_pair(dst, map, bar, c0, c1, h, t.bb);
+                            else tma_load_4d(dst, map, bar, c0, c1, h, t.bb);
                         };
                         const int k0 = kb * kBK, n0 = t.n0 + rank * L::kBRows;
-                        if (kAMn) {
-                            load(a_smem(s), ta, t.m0, k0);
-                            load(a_smem(s) + 8192, ta, t.m0 + 64, k0);
+                        if (amn) {
+                            load(a_smem(s), ta, t.m0, k0, ha);
+                            load(a_smem(s) + 8192, ta, t.m0 + 64, k0, ha);
                         } else {
-                            load(a_smem(s), ta, k0, t.m0);
+                            load(a_smem(s), ta, k0, t.m0, ha);
                         }
-                        if (kBMn) {
+                        if (bmn) {
 #pragma unroll
                             for (int pn = 0; pn < L::kBRows / 64; ++pn)     // 64-column blocks of 64 K rows, 8 KB each
-                                load(b_smem(s) + pn * 8192, tb, n0 + 64 * pn, k0);
+                                load(b_smem(s) + pn * 8192, tb, n0 + 64 * pn, k0, hb);
                         } else {
 #pragma unroll
                             for (int pn = 0; pn < L::kBRows / 128; ++pn)    // boxes of 128 rows of 128 bytes
-                                load(b_smem(s) + pn * 16384, tb, k0, n0 + 128 * pn);
+                                load(b_smem(s) + pn * 16384, tb, k0, n0 + 128 * pn, hb);
                         }
                     }
                 }
@@ -209,19 +242,13 @@ gemm_bf16_sm100_kernel(const __grid_constant__ GemmMaps maps, const __grid_const
         }
     } else if (warp == 1) {
         if (lane == 0 && rank == 0) {
-            constexpr uint32_t idesc = make_idesc_bf16(L::kTileM, kBN, kAMn ? 1 : 0, kBMn ? 1 : 0);
             // K-major tile: 128 rows of 128 bytes, 8-row groups 1024 bytes apart, 32 bytes per K step.
             // MN-major tile: two blocks of 64 columns, 8192 bytes apart, each 64 K rows of 128 bytes;
             // a K step of 16 rows advances 2048 bytes.
-            const uint64_t a_desc0 = kAMn ? make_smem_desc_sw128(a_smem(0), 8192, 1024)
-                                          : make_smem_desc_sw128(a_smem(0), 16, 1024);
-            const uint64_t b_desc0 = kBMn ? make_smem_desc_sw128(b_smem(0), 8192, 1024)
-                                          : make_smem_desc_sw128(b_smem(0), 16, 1024);
-            constexpr uint64_t a_step = kAMn ? 128 : 2, b_step = kBMn ? 128 : 2;
             bool ok = true;
             int it = 0, na = 0;                         // ring position; tiles that used an accumulator
             for (int lin = kPair ? blockIdx.x >> 1 : blockIdx.x; lin < n_tiles && ok; lin += kPair ? gridDim.x >> 1 : gridDim.x) {
-                const GemmTile t = gemm_tile<kBN, L::kTileM>(g, lin, rank);
+                const GemmTile t = gemm_tile<kBN, L::kTileM>(maps, g, sum_h, lin, rank);
                 if (t.n_iters == 0) continue;
                 const int buf = na & 1;
                 // the epilogue has read this accumulator's previous tile out
@@ -229,6 +256,11 @@ gemm_bf16_sm100_kernel(const __grid_constant__ GemmMaps maps, const __grid_const
                 if (!ok) break;
                 LTCA_TRACE_EVT(0x20 + (na << 8));
                 const uint32_t acc = tmem_base + (uint32_t)kBN * buf;
+                const bool amn = is_mn<kKind == kGroup, kAMn>(maps, t.problem, 1), bmn = is_mn<kKind == kGroup, kBMn>(maps, t.problem, 2);
+                const uint32_t idesc = make_idesc_bf16(L::kTileM, kBN, amn ? 1 : 0, bmn ? 1 : 0);
+                const uint64_t a_desc0 = make_smem_desc_sw128(a_smem(0), amn ? 8192 : 16, 1024);
+                const uint64_t b_desc0 = make_smem_desc_sw128(b_smem(0), bmn ? 8192 : 16, 1024);
+                const uint64_t a_step = amn ? 128 : 2, b_step = bmn ? 128 : 2;
                 for (int i = 0; i < t.n_iters && ok; ++i, ++it) {
                     const int s = it % kStages;
                     ok = mbar_wait(bar_full(s), (uint32_t)((it / kStages) & 1), wc, 0xd1);
@@ -270,7 +302,7 @@ gemm_bf16_sm100_kernel(const __grid_constant__ GemmMaps maps, const __grid_const
         bool ok = true;
         int na = 0, pc = 0;                                 // accumulators used; boxes staged
         for (int lin = kPair ? blockIdx.x >> 1 : blockIdx.x; lin < n_tiles; lin += kPair ? gridDim.x >> 1 : gridDim.x) {
-            const GemmTile t = gemm_tile<kBN, L::kTileM>(g, lin, rank);
+            const GemmTile t = gemm_tile<kBN, L::kTileM>(maps, g, sum_h, lin, rank);
             const int gm = t.m0 + row;
             const int buf = na & 1;
             const bool have = t.n_iters > 0;
@@ -369,9 +401,10 @@ gemm_bf16_sm100_kernel(const __grid_constant__ GemmMaps maps, const __grid_const
                         // (partial tiles are one [problem][slice][M][N] tensor)
                         const CUtensorMap* tc = &maps.c[g.ksplit > 1 ? 0 : t.problem];
                         if (gn0 < g.N && t.m0 < g.M) {
-                            tma_store_4d(tc, stage_addr + hb * (kBM * 128), gn0, t.m0, g.ksplit > 1 ? t.slice : t.bh,
-                                         g.ksplit > 1 ? t.problem : t.bb);
-                            if (g.c_lo) tma_store_4d(&maps.c[1], stage_addr + (hb + 1) * (kBM * 128), gn0, t.m0, t.bh, t.bb);
+                            if (add_to_c) tma_reduce_add_4d(tc, stage_addr + hb * (kBM * 128), gn0, t.m0, t.bh, t.bb);
+                            else tma_store_4d(tc, stage_addr + hb * (kBM * 128), gn0, t.m0, g.ksplit > 1 ? t.slice : t.bh,
+                                              g.ksplit > 1 ? t.problem : t.bb);
+                            if (g.c_lo) tma_store_4d(&maps.c[kKind == kGroup ? kMaxGemmProblems + t.problem : 1], stage_addr + (hb + 1) * (kBM * 128), gn0, t.m0, t.bh, t.bb);
                         }
                         tma_store_commit();
                         // the box that the next piece takes has been read
@@ -452,7 +485,7 @@ gemm_bf16_sm100_kernel(const __grid_constant__ GemmMaps maps, const __grid_const
                                  (int64_t)gm * g.ldc + gn0;
 #pragma unroll
                     for (int c = 0; c < 32; ++c)
-                        if (gn0 + c < g.N) dst[c] = __uint_as_float(v[c]);
+                        if (gn0 + c < g.N) dst[c] = (add_to_c ? dst[c] : 0.f) + __uint_as_float(v[c]);
                 }
             }
         }
@@ -548,7 +581,8 @@ __global__ void cvt_many_bf16_kernel(const __grid_constant__ CvtMany b) {
 }
 
 int make_operand_map(ltca_ctx* ctx, CUtensorMap* map, const GemmOperand& o, int mn_extent, int k_extent,
-                     int batch_h, int batch_b, const int64_t* bs) {
+                     int batch_h, int batch_b, const int64_t* bs, bool shared) {
+    if (shared) batch_h = 1;
     ltca_strides st;
     st.batch = bs[1]; st.head = bs[0]; st.seq = o.ld;
     if (o.mn_major)   // stored [K, MN]: rows are K, 64 x 64 boxes
@@ -576,11 +610,11 @@ GemmTileKind pick_tile(int M, int N, int64_t blocks, int64_t z, int sms) {
     return waves_pair <= waves_256 ? kTilePair : kTile256;
 }
 
-template <int kBN, bool kPair>
+template <int kBN, bool kPair, int kKind>
 int launch_gemm(ltca_ctx* ctx, const GemmMaps& m, const GemmKArgs& g, bool amn, bool bmn, int64_t n_tiles, int sms) {
     using L = GemmCfg<kBN, kPair>;
-    auto kern = !bmn ? gemm_bf16_sm100_kernel<false, false, kBN, kPair>
-                     : (amn ? gemm_bf16_sm100_kernel<true, true, kBN, kPair> : gemm_bf16_sm100_kernel<false, true, kBN, kPair>);
+    auto kern = !bmn ? gemm_bf16_sm100_kernel<false, false, kBN, kPair, kKind>
+                     : (amn ? gemm_bf16_sm100_kernel<true, true, kBN, kPair, kKind> : gemm_bf16_sm100_kernel<false, true, kBN, kPair, kKind>);
     static SmemOptIn opt_in[3];
     LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(opt_in[!bmn ? 0 : (amn ? 2 : 1)], ctx->device, kern, L::kDynBytes));
     const int64_t units = kPair ? sms / 2 : sms;
@@ -625,6 +659,10 @@ int gemm_sm100(ltca_ctx* ctx, const GemmProblem& gp) {
         return fail(ctx, LTCA_ERR_INVALID, "gemm: between 1 and 4 problems, or one problem of up to 3 summed pairs");
     if (gp.M < 1 || gp.N < 1 || gp.K < 1) return fail(ctx, LTCA_ERR_INVALID, "gemm: empty problem");
     const bool batched = gp.batch_h > 1 || gp.batch_b > 1;
+    if (gp.sum_h < 1 || (gp.sum_h > 1 && (gp.batch_h != 1 || gp.n_problems != 1 || gp.ksplit > 1)))
+        return fail(ctx, LTCA_ERR_INVALID, "gemm: a sum over heads takes one problem, no batch of heads and no split of K");
+    if (gp.add_to_c && (gp.out_bf16 || gp.ksplit > 1)) return fail(ctx, LTCA_ERR_INVALID, "gemm: adding to C needs fp32 results, no split of K");
+    const int heads = gp.sum_h > 1 ? gp.sum_h : gp.batch_h;
     if (gp.batch_h < 1 || gp.batch_b < 1 || (batched && (gp.n_problems != 1 || gp.ksplit > 1)))
         return fail(ctx, LTCA_ERR_INVALID, "gemm: a batch takes one problem (or one sum of pairs) and no split of K");
     const int n_pairs = gp.n_sum > 1 ? gp.n_sum : gp.n_problems;
@@ -633,8 +671,8 @@ int gemm_sm100(ltca_ctx* ctx, const GemmProblem& gp) {
     for (int i = 0; i < n_pairs; ++i) {
         if (gp.a[i].mn_major != gp.a[0].mn_major || gp.b[i].mn_major != gp.b[0].mn_major)
             return fail(ctx, LTCA_ERR_INVALID, "gemm: all pairs of one launch share the operand forms");
-        if ((rc = make_operand_map(ctx, &maps.a[i], gp.a[i], gp.M, gp.K, gp.batch_h, gp.batch_b, gp.a_bs))) return rc;
-        if ((rc = make_operand_map(ctx, &maps.b[i], gp.b[i], gp.N, gp.K, gp.batch_h, gp.batch_b, gp.b_bs))) return rc;
+        if ((rc = make_operand_map(ctx, &maps.a[i], gp.a[i], gp.M, gp.K, heads, gp.batch_b, gp.a_bs, gp.a_shared != 0))) return rc;
+        if ((rc = make_operand_map(ctx, &maps.b[i], gp.b[i], gp.N, gp.K, heads, gp.batch_b, gp.b_bs, gp.b_shared != 0))) return rc;
     }
     GemmKArgs g;
     g.M = gp.M; g.N = gp.N; g.K = gp.K;
@@ -649,6 +687,9 @@ int gemm_sm100(ltca_ctx* ctx, const GemmProblem& gp) {
     g.partial = gp.partial;
     g.status = ctx->d_status;
     g.batch_h = gp.batch_h; g.batch_b = gp.batch_b;
+    g.sum_h = gp.sum_h;
+    g.a_head = gp.a_shared ? 0 : 1; g.b_head = gp.b_shared ? 0 : 1;
+    g.add_to_c = gp.add_to_c;
     g.c_bs[0] = gp.c_bs[0]; g.c_bs[1] = gp.c_bs[1];
     const int ces = gp.out_bf16 ? 2 : 4;
     if (g.ksplit > 1) {
@@ -676,7 +717,7 @@ int gemm_sm100(ltca_ctx* ctx, const GemmProblem& gp) {
     }
     const int sms = ctx->sm_count > 0 ? ctx->sm_count : kPlanSms;
     const int64_t z = (int64_t)gp.n_problems * g.ksplit * gp.batch_h * gp.batch_b;
-    const GemmTileKind kind = pick_tile(gp.M, gp.N, (int64_t)((gp.K + kBK - 1) / kBK) / g.ksplit * g.n_sum, z, sms);
+    const GemmTileKind kind = pick_tile(gp.M, gp.N, (int64_t)((gp.K + kBK - 1) / kBK) / g.ksplit * g.n_sum * g.sum_h, z, sms);
     const int tile_m = kind == kTilePair ? 2 * kBM : kBM, tile_n = kind == kTile128 ? 128 : 256;
     g.tiles_x = (gp.N + tile_n - 1) / tile_n;
     g.tiles_y = (gp.M + tile_m - 1) / tile_m;
@@ -685,9 +726,10 @@ int gemm_sm100(ltca_ctx* ctx, const GemmProblem& gp) {
     if (n_tiles > 0x7fffffff) return fail(ctx, LTCA_ERR_UNSUPPORTED, "gemm: too many tiles");
     const bool amn = gp.a[0].mn_major != 0, bmn = gp.b[0].mn_major != 0;
     if (amn && !bmn) return fail(ctx, LTCA_ERR_UNSUPPORTED, "gemm: A stored [K, M] with B stored [N, K] is not built");
-    if (kind == kTilePair) rc = launch_gemm<256, true>(ctx, maps, g, amn, bmn, n_tiles, sms);
-    else if (kind == kTile256) rc = launch_gemm<256, false>(ctx, maps, g, amn, bmn, n_tiles, sms);
-    else rc = launch_gemm<128, false>(ctx, maps, g, amn, bmn, n_tiles, sms);
+    auto launch = kind == kTilePair ? launch_gemm<256, true, kPlain> : kind == kTile256 ? launch_gemm<256, false, kPlain> : launch_gemm<128, false, kPlain>;
+    if (g.sum_h > 1 || g.add_to_c || !g.a_head || !g.b_head)
+        launch = kind == kTilePair ? launch_gemm<256, true, kHeads> : kind == kTile256 ? launch_gemm<256, false, kHeads> : launch_gemm<128, false, kHeads>;
+    rc = launch(ctx, maps, g, amn, bmn, n_tiles, sms);
     if (rc) return rc;
     if (g.ksplit > 1) {
         const int64_t mn = (int64_t)gp.M * gp.N;
@@ -705,6 +747,75 @@ int gemm_sm100(ltca_ctx* ctx, const GemmProblem& gp) {
         LTCA_LAUNCH_OK(ctx, "gemm_splitk_reduce_kernel");
     }
     return LTCA_OK;
+}
+
+bool gemm_group_aligned(const GemmGroup& gg) {
+    const int ces = gg.out_bf16 ? 2 : 4;
+    for (int i = 0; i < gg.n; ++i) {
+        const GemmGroup::Member& m = gg.m[i];
+        if (((m.ldc * ces) & 15) || (gg.heads > 1 && ((m.c_hs * ces) & 15)) || (reinterpret_cast<uintptr_t>(m.c) & 15) ||
+            (reinterpret_cast<uintptr_t>(m.c_lo) & 15))
+            return false;
+    }
+    return true;
+}
+
+template <int kBN>
+static int launch_group(ltca_ctx* ctx, const GemmGroupMaps& m, const GemmKArgs& g, int64_t n_tiles, int sms) {
+    using L = GemmCfg<kBN, false>;
+    auto kern = gemm_bf16_sm100_kernel<false, false, kBN, false, kGroup>;
+    static SmemOptIn opt_in;
+    LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(opt_in, ctx->device, kern, L::kDynBytes));
+    LTCA_CUDA_OK(ctx, launch_dependent(kern, dim3((unsigned)(n_tiles < sms ? n_tiles : sms)), dim3(kGemmThreads), L::kDynBytes, ctx->stream,
+                                       m, g));
+    LTCA_LAUNCH_OK(ctx, "gemm_bf16_sm100_kernel");
+    return LTCA_OK;
+}
+
+int gemm_sm100_group(ltca_ctx* ctx, const GemmGroup& gg) {
+    if (gg.M < 1 || gg.N < 1 || gg.K < 1 || gg.heads < 1 || gg.n < 1 || gg.n > kMaxGemmProblems || !gemm_group_aligned(gg))
+        return fail(ctx, LTCA_ERR_INVALID, "gemm: between 1 and 4 members with 16-byte aligned results");
+    GemmGroupMaps maps;
+    GemmKArgs g;
+    memset(&maps, 0, sizeof(maps));
+    memset(&g, 0, sizeof(g));
+    g.M = gg.M; g.N = gg.N; g.K = gg.K;
+    g.n_sum = 1; g.ksplit = 1; g.sum_h = 1;
+    g.batch_h = gg.heads; g.batch_b = 1;
+    g.a_head = g.b_head = 1;
+    g.out_bf16 = gg.out_bf16;
+    g.tma_store = 1;
+    g.c_lo = gg.m[0].c_lo;
+    g.status = ctx->d_status;
+    int rc;
+    for (int i = 0; i < gg.n; ++i) {
+        const GemmGroup::Member& m = gg.m[i];
+        if (m.terms < 1 || m.terms > 3 || (m.c_lo != nullptr) != (g.c_lo != nullptr) || (m.c_lo && !gg.out_bf16))
+            return fail(ctx, LTCA_ERR_INVALID, "gemm: a member has one to three terms, and a second result term as the others");
+        const int64_t as[2] = {m.a_hs, 0}, bs[2] = {m.b_hs, 0};
+        maps.first[i + 1] = maps.first[i] + m.terms;
+        maps.form[i] = (m.a[0].mn_major ? 1 : 0) | (m.b[0].mn_major ? 2 : 0);
+        for (int t = 0; t < m.terms; ++t) {
+            if (m.a[t].mn_major != m.a[0].mn_major || m.b[t].mn_major != m.b[0].mn_major)
+                return fail(ctx, LTCA_ERR_INVALID, "gemm: the terms of a member share the operand forms");
+            if ((rc = make_operand_map(ctx, &maps.a[maps.first[i] + t], m.a[t], gg.M, gg.K, gg.heads, 1, as, false))) return rc;
+            if ((rc = make_operand_map(ctx, &maps.b[maps.first[i] + t], m.b[t], gg.N, gg.K, gg.heads, 1, bs, false))) return rc;
+        }
+        const ltca_strides cs{0, m.c_hs, m.ldc};
+        for (int l = 0; l < (m.c_lo ? 2 : 1); ++l)
+            if ((rc = make_tmap_bhsd(ctx, &maps.c[l * kMaxGemmProblems + i], l ? m.c_lo : m.c, gg.out_bf16 ? 2 : 4, 1, gg.heads, gg.M, gg.N, cs,
+                                     gg.out_bf16 ? 64 : 32, kBM))) return rc;
+        g.C[i] = m.c;
+    }
+    const int sms = ctx->sm_count > 0 ? ctx->sm_count : kPlanSms;
+    const int64_t z = (int64_t)gg.n * gg.heads;
+    const bool wide = pick_tile(gg.M, gg.N, 0, z, sms) != kTile128;    // (0: no pairs)
+    g.tiles_x = (gg.N + (wide ? 255 : 127)) / (wide ? 256 : 128);
+    g.tiles_y = (gg.M + kBM - 1) / kBM;
+    g.tiles_z = gg.n;
+    const int64_t n_tiles = g.tiles_x * (g.tiles_y * z);
+    if (n_tiles > 0x7fffffff) return fail(ctx, LTCA_ERR_UNSUPPORTED, "gemm: too many tiles");
+    return wide ? launch_group<256>(ctx, maps, g, n_tiles, sms) : launch_group<128>(ctx, maps, g, n_tiles, sms);
 }
 
 int convert_rows_bf16(ltca_ctx* ctx, const float* src, int64_t ld_src, void* dst, int64_t ld_dst, int64_t rows,

@@ -34,9 +34,31 @@ struct GemmProblem {
     // Needs n_problems == 1 and ksplit == 1 (n_sum is allowed); strides must keep 16-byte alignment.
     int batch_h = 1, batch_b = 1;
     int64_t a_bs[2] = {0, 0}, b_bs[2] = {0, 0}, c_bs[2] = {0, 0};
+    int a_shared = 0, b_shared = 0; // every head of the batch (or of the sum) reads the same A / B
+    int sum_h = 1;                  // > 1, batch_h == 1: C_b = sum over h < sum_h of A_hb B_hb, the heads one after the other in
+                                    // one accumulator (a_bs[0], b_bs[0] as in a batch)
+    int add_to_c = 0;               // fp32 results without a split of K: C += ... (one add per element, so the bits are
+                                    // those of any other run)
 };
 
 int gemm_sm100(ltca_ctx* ctx, const GemmProblem& gp);
+
+// Up to four products of the same shape in one launch, each of its own operand forms and number of summed terms, for every one
+// of `heads` (strides a_hs, b_hs, c_hs between them).  c_lo as in GemmProblem, for all members or for none.  Results need
+// 16-byte aligned rows (gemm_group_aligned).
+struct GemmGroup {
+    struct Member {
+        int terms = 1;
+        GemmOperand a[3] = {}, b[3] = {};
+        int64_t a_hs = 0, b_hs = 0, c_hs = 0, ldc = 0;
+        void* c = nullptr;
+        void* c_lo = nullptr;
+    };
+    int M = 0, N = 0, K = 0, heads = 1, n = 0, out_bf16 = 0;
+    Member m[kMaxGemmProblems];
+};
+bool gemm_group_aligned(const GemmGroup& gg);
+int gemm_sm100_group(ltca_ctx* ctx, const GemmGroup& gg);
 int gemm_sm100_pick_ksplit(int M, int N, int K, int n_problems, int sm_count);
 size_t gemm_sm100_partial_bytes(int M, int N, int n_problems, int ksplit);
 // dst[r, c] = bf16(src[r, c]) for a [rows, cols] block with row pitches ld_src / ld_dst (elements).

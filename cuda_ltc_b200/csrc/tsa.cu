@@ -632,6 +632,27 @@ bool use_tensor(const ltca_tsa_params* t, bool backward) {
     return true;
 }
 
+// Whether the written-out-score path runs on per-head products of the weights: heads as wide as the model (the reference's
+// form) and enough rows.  With M_h = Wq_h Wk_h^T and N_h = Wv_h Wo_h, both [E, E],
+//   scores   q_h k_h^T = (x M_h) x^T            output   sum_h P_h v_h Wo_h = sum_h P_h (x N_h)
+// so k, ctx and the output projection are never formed, and in the backward, with dS and dP as before,
+//   dP_h = dy z_h^T, dz_h = P_h^T dy, dT_h = dS_h x        (T_h = x M_h, z_h = x N_h)
+//   dx = sum_h dT_h M_h^T + dz_h N_h^T + dS_h^T T_h        dM_h = x^T dT_h, dN_h = x^T dz_h
+//   dWq_h = dM_h Wk_h, dWk_h = dM_h^T Wq_h, dWv_h = dN_h Wo_h^T, dWo_h = Wv_h^T dN_h.
+// In units of rows x E x (H E) multiply-adds the projections cost 4 instead of 8 forward (T counts three, its operands have two
+// terms) and 4 instead of 8 backward; products of weights add 6 and 10 in units of E x E x (H E), and three launches.  From
+// four rows per column of x on that is the faster path: forward and backward of a kept forward, us, B32 S256 E512 H8 365 + 407
+// -> 271 + 307; at the line, B8 S256 E512 H8 155 + 183 -> 125 + 159, B32 S32 E256 H4 65 + 82 -> 60 + 79; half as many rows
+// gained nothing (B4 S256 E512 H8).  Fewer bf16 roundings lie between the inputs and a result than on the other path, and the
+// products of weights have two terms, as q and k have there: errors against 64 bits 4.0e-3 -> 3.2e-3 (output), 5.7e-3 ->
+// 4.8e-3 (dx), 5.8e-3 -> 5.2e-3 (dWq, dWk), 4.0e-3 -> 3.6e-3 (dWv, dWo), the like at every size.
+// (A choice by shape, mode and biases, which are the same in a forward and the backward that reuses it.)
+constexpr int kComposedRows = 4;
+bool composed_shape(const ltca_tsa_params* t) {
+    return t->head_width == t->E && (int64_t)t->B * t->S >= (int64_t)kComposedRows * t->E && use_wide(t, false);
+}
+bool use_composed(const ltca_tsa_params* t) { return composed_shape(t) && !t->bq && !t->bk && !t->bv; }
+
 struct TPlan {
     int64_t rows;
     int HW, Ep;
@@ -641,6 +662,10 @@ struct TPlan {
     // materialised-score path: low-order parts of x, Wq, Wk, q, k; fp32 projection scratch; score matrices
     bool wide;
     size_t mat32, mat16;
+    // ... on products of the weights: one [E, H * E] matrix in bf16
+    bool composed;
+    size_t me;
+    int ks_m;
 };
 
 int make_tplan(const ltca_tsa_params* t, TPlan* pl, bool backward) {
@@ -654,6 +679,8 @@ int make_tplan(const ltca_tsa_params* t, TPlan* pl, bool backward) {
     pl->lse = align_up((size_t)t->B * t->H * t->S * sizeof(float), 256);
     pl->y = align_up((size_t)pl->rows * t->E * sizeof(float), 256);
     pl->wide = use_wide(t, backward);
+    pl->composed = pl->wide && use_composed(t);
+    pl->me = align_up((size_t)t->E * t->H * t->E * 2, 256);
     pl->mat32 = pl->mat16 = 0;
     pl->attn_fwd = pl->attn_bwd = 0;
     int rc;
@@ -676,6 +703,28 @@ int make_tplan(const ltca_tsa_params* t, TPlan* pl, bool backward) {
     const size_t p_in = gemm_sm100_partial_bytes(t->E, pl->HW, pl->n_dw, pl->ks_in);
     const size_t p_out = gemm_sm100_partial_bytes(pl->HW, t->E, 1, pl->ks_out);
     pl->partial = p_in > p_out ? p_in : p_out;
+    pl->ks_m = 1;
+    if (pl->composed) {
+        pl->ks_m = gemm_sm100_pick_ksplit(t->E, pl->HW, rows, 2, kPlanSms);
+        pl->partial = gemm_sm100_partial_bytes(t->E, pl->HW, 2, pl->ks_m);
+    }
+    return LTCA_OK;
+}
+
+// A size is asked for before the biases are known: the larger one of a plan with and one without them.
+template <typename Size>
+int planned_bytes(const ltca_tsa_params* t, bool backward, Size size, size_t* bytes_out) {
+    TPlan pl;
+    int rc = make_tplan(t, &pl, backward);
+    if (rc) return rc;
+    *bytes_out = size(pl);
+    if (!composed_shape(t)) return LTCA_OK;
+    ltca_tsa_params other = *t;
+    const float present = 0.f;                         // (only whether there is a bias is looked at)
+    other.bq = use_composed(t) ? &present : nullptr;
+    other.bk = other.bv = nullptr;
+    if ((rc = make_tplan(&other, &pl, backward))) return rc;
+    if (size(pl) > *bytes_out) *bytes_out = size(pl);
     return LTCA_OK;
 }
 
@@ -688,7 +737,18 @@ size_t wide_extra(const TPlan& pl, int which) {
     return wide_kept(pl) + (which == 0 ? 0 : pl.mat32 + pl.mat16);     // backward: dP and dS
 }
 
+// On products of the weights: what a forward keeps (x, the weights with the second terms of Wq and Wk, M, N, T, z, lse, scores,
+// probabilities) and what no later call needs (the other second terms).
+size_t composed_kept(const TPlan& pl) { return pl.xb + 5 * pl.w_in + pl.w_out + 2 * pl.me + 2 * pl.act + pl.lse + pl.mat32 + pl.mat16; }
+size_t composed_scratch(const TPlan& pl) { return pl.xb + pl.w_in + pl.w_out + 2 * pl.me + pl.act; }
+
 size_t tensor_workspace(const TPlan& pl, int which) {
+    if (pl.composed) {
+        const size_t n = composed_kept(pl) + composed_scratch(pl);
+        if (which == 0) return n + pl.y;
+        // dy; dT, dz and two more for bias gradients; dP, dS; dM and dN in fp32 and in two terms each
+        return n + pl.xb + 4 * pl.act + pl.mat32 + pl.mat16 + 4 * pl.me + 4 * pl.me + pl.partial;
+    }
     // x, the four weight matrices, q, k, v, ctx, lse
     size_t n = pl.xb + 3 * pl.w_in + pl.w_out + 4 * pl.act + pl.lse + wide_extra(pl, which);
     if (which == 0) return n + pl.y + pl.attn_fwd;
@@ -698,6 +758,7 @@ size_t tensor_workspace(const TPlan& pl, int which) {
 }
 
 size_t tensor_saved_bytes(const TPlan& pl) {
+    if (pl.composed) return composed_kept(pl);
     return pl.xb + 3 * pl.w_in + pl.w_out + 4 * pl.act + pl.lse + wide_kept(pl);
 }
 
@@ -708,6 +769,8 @@ struct TBufs {
     // materialised-score path
     void *xl, *wql, *wkl, *ql, *kl, *P, *dS;
     float *scores, *dP;
+    // ... on products of the weights
+    void *wvl, *wol, *m, *ml, *n, *nl, *t, *tl, *z;
 };
 
 // The attention problem of the module for the materialised-score path (bf16 views of the projection outputs).
@@ -723,6 +786,22 @@ void fill_wide(const ltca_tsa_params* t, const TBufs& tb, WideArgs* w) {
     w->o = tb.ctx; w->o_bf16 = 1; w->lse = tb.lse;
     w->scores = tb.scores; w->P = tb.P; w->dP = tb.dP; w->dS = tb.dS;
     w->grads_bf16 = 1;
+}
+
+// The same on products of the weights: T and z in the places of q and v, x in that of k, for every head.
+ltca_strides x_strides(const ltca_tsa_params* t, int64_t ld) {
+    ltca_strides st;
+    st.head = 0;
+    st.batch = t->time_major ? ld : (int64_t)t->S * ld;
+    st.seq = t->time_major ? (int64_t)t->B * ld : ld;
+    return st;
+}
+void fill_composed(const ltca_tsa_params* t, const TPlan& pl, const TBufs& tb, WideArgs* w) {
+    fill_wide(t, tb, w);
+    w->qh = tb.t; w->ql = tb.tl;
+    w->kh = tb.xb; w->kl = tb.xl; w->ks = x_strides(t, pl.Ep);
+    w->v = tb.z;
+    w->o = nullptr;
 }
 
 // The attention scratch (TBufs::rest) of a call whose buffers start at w; not on the written-out-score path.
@@ -755,6 +834,254 @@ int place_mask_words(ltca_ctx* ctx, const ltca_tsa_params* t, const TPlan& pl, c
     if (!later && (rc = pack_mask_words(ctx, &a, words))) return rc;
     ctx->mask_packed = t->keep_mask;
     ctx->mask_words = words;
+    return LTCA_OK;
+}
+
+// The steps of tensor_forward_core on products of the weights, up to z and the probabilities.  (No FlashAttention form runs
+// its first steps in here: fuses_prenorm.)
+int composed_forward_core(ltca_ctx* ctx, const ltca_tsa_params* t, const TPlan& pl, char* w, TBufs* tb, const float* also_src,
+                          void* also_dst, bool* also_done) {
+    char* r = w;
+    if (t->saved) w = reinterpret_cast<char*>(t->saved);
+    tb->xb = w;  w += pl.xb;
+    tb->wq = w;  w += pl.w_in;
+    tb->wk = w;  w += pl.w_in;
+    tb->wv = w;  w += pl.w_in;
+    tb->wo = w;  w += pl.w_out;
+    tb->wql = w; w += pl.w_in;
+    tb->wkl = w; w += pl.w_in;
+    tb->m = w;   w += pl.me;
+    tb->n = w;   w += pl.me;
+    tb->t = w;   w += pl.act;
+    tb->z = w;   w += pl.act;
+    tb->lse = reinterpret_cast<float*>(w);    w += pl.lse;
+    tb->scores = reinterpret_cast<float*>(w); w += pl.mat32;
+    tb->P = w;   w += pl.mat16;
+    if (!t->saved) r = w;
+    tb->xl = r;  r += pl.xb;
+    tb->wvl = r; r += pl.w_in;
+    tb->wol = r; r += pl.w_out;
+    tb->ml = r;  r += pl.me;
+    tb->nl = r;  r += pl.me;
+    tb->tl = r;  r += pl.act;
+    tb->rest = r;
+    tb->q = tb->k = tb->v = tb->ctx = tb->ql = tb->kl = tb->dS = nullptr;
+    tb->dP = nullptr;
+    const bool cached = t->weight_cache != nullptr;
+    if (cached) {                                      // laid out as on the other path
+        char* c = reinterpret_cast<char*>(t->weight_cache);
+        tb->wq = c;  c += pl.w_in;
+        tb->wk = c;  c += pl.w_in;
+        tb->wv = c;  c += pl.w_in;
+        tb->wo = c;  c += pl.w_out;
+        tb->wql = c; c += pl.w_in;
+        tb->wkl = c; c += pl.w_in;
+        tb->wvl = c; c += pl.w_in;
+        tb->wol = c;
+    }
+    if (t->saved && t->reuse_forward) return LTCA_OK;
+    const int E = t->E, HW = pl.HW, Ep = pl.Ep, rows = (int)pl.rows;
+    int rc;
+    {
+        const float* src[6] = {t->x, t->wq, t->wk, t->wv, t->wo, nullptr};
+        void* dst[6] = {tb->xb, tb->wq, tb->wk, tb->wv, tb->wo, nullptr};
+        void* lo[6] = {tb->xl, tb->wql, tb->wkl, tb->wvl, tb->wol, nullptr};
+        int64_t ld_src[6] = {E, HW, HW, HW, E, E}, ld_dst[6] = {Ep, HW, HW, HW, Ep, Ep};
+        int64_t nrows[6] = {pl.rows, E, E, E, HW, pl.rows};
+        int ncols[6] = {E, HW, HW, HW, E, E};
+        int n = cached && t->weight_cache_valid ? 1 : 5;
+        if (also_src) {
+            src[n] = also_src; dst[n] = also_dst; lo[n] = nullptr;
+            ld_src[n] = E; ld_dst[n] = Ep; nrows[n] = pl.rows; ncols[n] = E;
+            ++n;
+            *also_done = true;
+        }
+        if ((rc = convert_many_bf16(ctx, n, src, ld_src, dst, ld_dst, nrows, ncols, lo))) return rc;
+    }
+    {   // M_h = Wq_h Wk_h^T : both stored [E, HW], the head's columns contiguous; N_h = Wv_h Wo_h : Wo_h is rows [h E, (h + 1) E)
+        GemmGroup gg;
+        gg.M = gg.N = gg.K = E;
+        gg.heads = t->H; gg.n = 2; gg.out_bf16 = 1;
+        GemmGroup::Member &m = gg.m[0], &n = gg.m[1];
+        m.terms = n.terms = 3;
+        m.a[0] = GemmOperand{tb->wq, HW, 0};  m.b[0] = GemmOperand{tb->wk, HW, 0};
+        m.a[1] = GemmOperand{tb->wq, HW, 0};  m.b[1] = GemmOperand{tb->wkl, HW, 0};
+        m.a[2] = GemmOperand{tb->wql, HW, 0}; m.b[2] = GemmOperand{tb->wk, HW, 0};
+        m.a_hs = m.b_hs = E;
+        m.c = tb->m; m.c_lo = tb->ml;
+        n.a[0] = GemmOperand{tb->wv, HW, 0};  n.b[0] = GemmOperand{tb->wo, Ep, 1};
+        n.a[1] = GemmOperand{tb->wv, HW, 0};  n.b[1] = GemmOperand{tb->wol, Ep, 1};
+        n.a[2] = GemmOperand{tb->wvl, HW, 0}; n.b[2] = GemmOperand{tb->wo, Ep, 1};
+        n.a_hs = E; n.b_hs = (int64_t)E * Ep;
+        n.c = tb->n; n.c_lo = tb->nl;
+        m.ldc = n.ldc = HW;
+        m.c_hs = n.c_hs = E;
+        if ((rc = gemm_sm100_group(ctx, gg))) return rc;
+    }
+    {   // T = x M, in two terms
+        GemmProblem gp;
+        gp.M = rows; gp.N = HW; gp.K = E;
+        gp.n_sum = 3;
+        gp.a[0] = GemmOperand{tb->xb, Ep, 0}; gp.b[0] = GemmOperand{tb->m, HW, 1};
+        gp.a[1] = GemmOperand{tb->xb, Ep, 0}; gp.b[1] = GemmOperand{tb->ml, HW, 1};
+        gp.a[2] = GemmOperand{tb->xl, Ep, 0}; gp.b[2] = GemmOperand{tb->m, HW, 1};
+        gp.c[0] = tb->t; gp.c_lo = tb->tl;
+        gp.out_bf16 = 1;
+        gp.ldc = HW;
+        if ((rc = gemm_sm100(ctx, gp))) return rc;
+    }
+    {   // z = x N
+        GemmProblem gp;
+        gp.M = rows; gp.N = HW; gp.K = E;
+        gp.a[0] = GemmOperand{tb->xb, Ep, 0}; gp.b[0] = GemmOperand{tb->n, HW, 1};
+        gp.c[0] = tb->z;
+        gp.out_bf16 = 1;
+        gp.ldc = HW;
+        if ((rc = gemm_sm100(ctx, gp))) return rc;
+    }
+    WideArgs wa;
+    fill_composed(t, pl, *tb, &wa);
+    return wide_attn_fwd(ctx, wa);
+}
+
+// C_b = sum over the heads of op(S_hb) R_hb for one [S, E] matrix of rows per sequence: S_hb a score-shaped matrix (mn_major:
+// taken transposed), R the activations [rows, H E]; `add`: to what C holds.
+int sum_over_heads(ltca_ctx* ctx, const ltca_tsa_params* t, const TPlan& pl, const void* score, int mn_major, const void* act,
+                   float* c, const float* bias, bool add) {
+    ltca_attn_params a;
+    fill_attn_bf16(t, &a);
+    const ltca_strides cs = x_strides(t, t->E);
+    const int Skp = wide_padded_keys(t->S);
+    GemmProblem gp;
+    gp.M = t->S; gp.N = t->E; gp.K = t->S;
+    gp.a[0] = GemmOperand{score, Skp, mn_major};
+    gp.b[0] = GemmOperand{act, a.q_strides.seq, 1};
+    gp.sum_h = t->H; gp.batch_b = t->B;
+    gp.a_bs[0] = (int64_t)t->S * Skp;   gp.a_bs[1] = (int64_t)t->H * t->S * Skp;
+    gp.b_bs[0] = a.q_strides.head;      gp.b_bs[1] = a.q_strides.batch;
+    gp.c_bs[1] = cs.batch;
+    gp.c[0] = c;
+    gp.ldc = cs.seq;
+    gp.bias[0] = bias;
+    gp.add_to_c = add ? 1 : 0;
+    return gemm_sm100(ctx, gp);
+}
+
+// A product for every head between two of [E, H E] / [rows, H E] / [HW, E] matrices: C_h[M, N] = sum over the terms.
+int per_head(ltca_ctx* ctx, const ltca_tsa_params* t, int M, int n_sum, const GemmOperand* a, int64_t a_hs, const GemmOperand* b,
+             int64_t b_hs, void* c, int64_t ldc, int64_t c_hs, int out_bf16) {
+    GemmProblem gp;
+    gp.M = M; gp.N = t->E; gp.K = t->E;
+    gp.n_sum = n_sum;
+    for (int i = 0; i < n_sum; ++i) { gp.a[i] = a[i]; gp.b[i] = b[i]; }
+    gp.batch_h = t->H;
+    gp.a_bs[0] = a_hs; gp.b_bs[0] = b_hs; gp.c_bs[0] = c_hs;
+    gp.c[0] = c;
+    gp.ldc = ldc;
+    gp.out_bf16 = out_bf16;
+    return gemm_sm100(ctx, gp);
+}
+
+// The backward behind composed_forward_core; w: the workspace behind what the forward laid out there.
+int composed_backward(ltca_ctx* ctx, const ltca_tsa_params* t, const TPlan& pl, const TBufs& tb, const void* dyb, char* w,
+                      bool want_dx, bool want_dw, ColSum* sums) {
+    const int rows = (int)pl.rows, E = t->E, HW = pl.HW, Ep = pl.Ep;
+    void* dt = w;     w += pl.act;
+    void* dz = w;     w += pl.act;
+    void* dq = w;     w += pl.act;
+    void* dv = w;     w += pl.act;
+    WideArgs wa;
+    fill_composed(t, pl, tb, &wa);
+    wa.dP = reinterpret_cast<float*>(w); w += pl.mat32;
+    wa.dS = w;        w += pl.mat16;
+    float* dm32 = reinterpret_cast<float*>(w); w += 2 * pl.me;
+    float* dn32 = reinterpret_cast<float*>(w); w += 2 * pl.me;
+    void* dm = w;     w += pl.me;
+    void* dml = w;    w += pl.me;
+    void* dn = w;     w += pl.me;
+    void* dnl = w;    w += pl.me;
+    float* partial = reinterpret_cast<float*>(w);
+    int rc;
+    // dP = dy z^T, dz = P^T dy, dS, dT = dS x
+    wa.dout = dyb; wa.dos = x_strides(t, Ep);
+    wa.dq = dt; wa.dv = dz;
+    if ((rc = wide_attn_bwd(ctx, wa))) return rc;
+    if (want_dx) {
+        GemmProblem gp;                                // M and N are stored [E, H E] = [N, K]
+        gp.M = rows; gp.N = E; gp.K = HW;
+        gp.n_sum = 2;
+        gp.a[0] = GemmOperand{dt, HW, 0}; gp.b[0] = GemmOperand{tb.m, HW, 0};
+        gp.a[1] = GemmOperand{dz, HW, 0}; gp.b[1] = GemmOperand{tb.n, HW, 0};
+        gp.c[0] = t->dx;
+        gp.ldc = E;
+        if ((rc = gemm_sm100(ctx, gp))) return rc;
+        if ((rc = sum_over_heads(ctx, t, pl, wa.dS, 1, tb.t, t->dx, nullptr, true))) return rc;
+    }
+    if (!want_dw) return LTCA_OK;
+    {   // dM = x^T dT, dN = x^T dz
+        GemmProblem gp;
+        gp.M = E; gp.N = HW; gp.K = rows;
+        gp.n_problems = 2;
+        gp.ksplit = pl.ks_m;
+        gp.a[0] = gp.a[1] = GemmOperand{tb.xb, Ep, 1};
+        gp.b[0] = GemmOperand{dt, HW, 1}; gp.b[1] = GemmOperand{dz, HW, 1};
+        gp.c[0] = dm32; gp.c[1] = dn32;
+        gp.ldc = HW;
+        gp.partial = partial;
+        if ((rc = gemm_sm100(ctx, gp))) return rc;
+        const float* src[2] = {dm32, dn32};
+        void *hi[2] = {dm, dn}, *lo[2] = {dml, dnl};
+        const int64_t ld[2] = {HW, HW}, nrows[2] = {E, E};
+        const int ncols[2] = {HW, HW};
+        if ((rc = convert_many_bf16(ctx, 2, src, ld, hi, ld, nrows, ncols, lo))) return rc;
+    }
+    const int64_t wo_h = (int64_t)E * Ep;
+    {
+        GemmGroup gg;
+        gg.M = gg.N = gg.K = E;
+        gg.heads = t->H; gg.n = 4;
+        void* dst[4] = {t->dwq, t->dwk, t->dwv, t->dwo};
+        for (int i = 0; i < 4; ++i) {
+            GemmGroup::Member& m = gg.m[i];
+            const void *hi = i < 2 ? dm : dn, *lo = i < 2 ? dml : dnl;
+            m.terms = i < 2 ? 3 : 2;
+            m.a_hs = m.b_hs = m.c_hs = E;
+            m.c = dst[i];
+            m.ldc = HW;
+            for (int k = 0; k < m.terms; ++k) {
+                const void* d = k == 1 ? lo : hi;
+                if (i == 0) { m.a[k] = GemmOperand{d, HW, 0}; m.b[k] = GemmOperand{k == 2 ? tb.wkl : tb.wk, HW, 1}; }
+                if (i == 1) { m.a[k] = GemmOperand{d, HW, 1}; m.b[k] = GemmOperand{k == 2 ? tb.wql : tb.wq, HW, 1}; }
+                if (i == 2) { m.a[k] = GemmOperand{d, HW, 0}; m.b[k] = GemmOperand{tb.wo, Ep, 0}; }
+                if (i == 3) { m.a[k] = GemmOperand{tb.wv, HW, 1}; m.b[k] = GemmOperand{d, HW, 1}; }
+            }
+            if (i == 2) m.b_hs = wo_h;
+            if (i == 3) { m.ldc = E; m.c_hs = (int64_t)E * E; }
+        }
+        // results whose rows cannot be stored by TMA: one launch each
+        if (gemm_group_aligned(gg)) {
+            if ((rc = gemm_sm100_group(ctx, gg))) return rc;
+        } else {
+            for (const GemmGroup::Member& m : gg.m)
+                if ((rc = per_head(ctx, t, E, m.terms, m.a, m.a_hs, m.b, m.b_hs, m.c, m.ldc, m.c_hs, 0))) return rc;
+        }
+    }
+    sums->add(t->dy, false, E, E, t->dbo);
+    if (t->dbq || t->dbk || t->dbv) {
+        // Gradients of biases that the module does not have: column sums of dq = dT Wk, dv = dz Wo^T and dk = (dS^T x) Wq.
+        const GemmOperand qa = {dt, HW, 0}, qb = {tb.wk, HW, 1}, va = {dz, HW, 0}, vb = {tb.wo, Ep, 0};
+        if ((rc = per_head(ctx, t, rows, 1, &qa, E, &qb, E, dq, HW, E, 1))) return rc;
+        if ((rc = per_head(ctx, t, rows, 1, &va, E, &vb, wo_h, dv, HW, E, 1))) return rc;
+        WideArgs wk = wa;
+        wk.qh = tb.xb; wk.ql = nullptr; wk.qs = x_strides(t, Ep);
+        wk.dk = dt;
+        if ((rc = wide_key_grad(ctx, wk))) return rc;
+        const GemmOperand ka = {dt, HW, 0}, kb = {tb.wq, HW, 1};
+        if ((rc = per_head(ctx, t, rows, 1, &ka, E, &kb, E, dz, HW, E, 1))) return rc;
+        sums->add(dq, true, HW, HW, t->dbq);
+        sums->add(dz, true, HW, HW, t->dbk);
+        sums->add(dv, true, HW, HW, t->dbv);
+    }
     return LTCA_OK;
 }
 
@@ -799,6 +1126,7 @@ int tensor_forward_core(ltca_ctx* ctx, const ltca_tsa_params* t, const TPlan& pl
         }
     }
     tb->rest = r;
+    tb->wvl = tb->wol = nullptr;
     // the weights' copies live in the caller's cache when there is one
     const bool cached = t->weight_cache != nullptr;
     if (cached) {
@@ -808,6 +1136,8 @@ int tensor_forward_core(ltca_ctx* ctx, const ltca_tsa_params* t, const TPlan& pl
         tb->wv = c;  c += pl.w_in;
         tb->wo = c;  c += pl.w_out;
         if (pl.wide) { tb->wql = c; c += pl.w_in; tb->wkl = c; c += pl.w_in; }
+        // (a call without biases may find this block valid: composed_forward_core)
+        if (composed_shape(t)) { tb->wvl = c; c += pl.w_in; tb->wol = c; }
     }
     const bool convert_weights = !(cached && t->weight_cache_valid);
     if (saved && t->reuse_forward) return LTCA_OK;
@@ -819,7 +1149,7 @@ int tensor_forward_core(ltca_ctx* ctx, const ltca_tsa_params* t, const TPlan& pl
         const float* src[6] = {t->x, t->wq, t->wk, t->wv, t->wo, nullptr};
         void* dst[6] = {tb->xb, tb->wq, tb->wk, tb->wv, tb->wo, nullptr};
         void* lo[6] = {pl.wide ? tb->xl : nullptr, pl.wide ? tb->wql : nullptr, pl.wide ? tb->wkl : nullptr,
-                       nullptr, nullptr, nullptr};
+                       tb->wvl, tb->wol, nullptr};
         int64_t ld_src[6] = {E, HW, HW, HW, E, E}, ld_dst[6] = {Ep, HW, HW, HW, Ep, Ep};
         int64_t nrows[6] = {pl.rows, E, E, E, HW, pl.rows};
         int ncols[6] = {E, HW, HW, HW, E, E};
@@ -923,6 +1253,11 @@ int tensor_forward(ltca_ctx* ctx, const ltca_tsa_params* t, const ltca_tsa_param
     CallHints hints{ctx};
     ctx->fwd_pairs = t->bk != nullptr;
     if (fused && (rc = place_mask_words(ctx, &layout, pl, scratch_of(t, pl, w), pl.attn_fwd, true))) return rc;
+    if (pl.composed) {
+        if ((rc = composed_forward_core(ctx, t, pl, w, &tb, nullptr, nullptr, nullptr))) return rc;
+        if ((rc = sum_over_heads(ctx, t, pl, tb.P, 0, tb.z, y, t->bo, false))) return rc;
+        return outer ? prenorm_finish(ctx, outer, y) : residual_layer_norm(ctx, t, y, pl.rows);
+    }
     if ((rc = tensor_forward_core(ctx, t, pl, w, &tb, 0, nullptr, nullptr, nullptr, fused ? outer : nullptr))) return rc;
     GemmProblem gp;
     gp.M = (int)pl.rows; gp.N = t->E; gp.K = pl.HW;
@@ -947,6 +1282,13 @@ int tensor_backward(ltca_ctx* ctx, const ltca_tsa_params* t, bool want_dx, bool 
         return fail(ctx, LTCA_ERR_WORKSPACE, "backward needs %zu bytes of workspace", need);
     char* w = reinterpret_cast<char*>(t->workspace);
     void* dyb = w;   w += pl.xb;
+    if (pl.composed) {
+        TBufs tb;
+        bool dy_done = false;
+        if ((rc = composed_forward_core(ctx, t, pl, w, &tb, t->dy, dyb, &dy_done))) return rc;
+        if (!dy_done && (rc = convert_rows_bf16(ctx, t->dy, t->E, dyb, pl.Ep, pl.rows, t->E))) return rc;
+        return composed_backward(ctx, t, pl, tb, dyb, tb.rest, want_dx, want_dw, sums);
+    }
     void* dctx = w;  w += pl.act;
     void* dq = w;    w += pl.act;
     void* dk = w;    w += pl.act;
@@ -1056,11 +1398,8 @@ extern "C" {
 // Workspace of the TimeSelfAttention form (no input LayerNorm, no dropout), without the column-sum scratch.
 static int inner_workspace(const ltca_tsa_params* t, int which, size_t* bytes_out) {
     if (use_tensor(t, which != 0 || keeps_for_backward(t))) {
-        TPlan tp;
-        int trc = make_tplan(t, &tp, which != 0 || keeps_for_backward(t));
-        if (trc) return trc;
-        *bytes_out = tensor_workspace(tp, which);
-        return LTCA_OK;
+        return planned_bytes(t, which != 0 || keeps_for_backward(t), [&](const TPlan& tp) { return tensor_workspace(tp, which); },
+                             bytes_out);
     }
     Plan pl;
     int rc = make_plan(t, &pl);
@@ -1098,11 +1437,7 @@ int ltca_tsa_saved_bytes(const ltca_tsa_params* t, size_t* bytes_out) {
     ltca_tsa_params probe = *t;
     probe.saved = nullptr;
     if (use_tensor(&probe, true)) {
-        TPlan tp;
-        int rc = make_tplan(&probe, &tp, true);
-        if (rc) return rc;
-        *bytes_out = tensor_saved_bytes(tp);
-        return LTCA_OK;
+        return planned_bytes(&probe, true, [](const TPlan& tp) { return tensor_saved_bytes(tp); }, bytes_out);
     }
     Plan pl;
     int rc = make_plan(&probe, &pl);
@@ -1119,7 +1454,7 @@ int ltca_tsa_weight_cache_bytes(const ltca_tsa_params* t, size_t* bytes_out) {
     TPlan tp;
     int rc = make_tplan(t, &tp, true);
     if (rc) return rc;
-    *bytes_out = 3 * tp.w_in + tp.w_out + (tp.wide ? 2 * tp.w_in : 0);
+    *bytes_out = 3 * tp.w_in + tp.w_out + (tp.wide ? 2 * tp.w_in : 0) + (composed_shape(t) ? tp.w_in + tp.w_out : 0);
     return LTCA_OK;
 }
 

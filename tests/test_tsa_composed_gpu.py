@@ -1,0 +1,104 @@
+"""The reference's form of the module (heads as wide as the model) where it runs on per-head products of the weights
+(Wq_h Wk_h^T, Wv_h Wo_h): from four rows per column of x on.  Both sides of that line, ragged lengths, every mask kind and
+the calls that share a kept forward, against the fp64 oracle.  Bounds as in tests/test_tsa_golden.py: no result has more
+bf16 roundings behind it than on the path through q, k, v and ctx."""
+import numpy as np
+import pytest
+
+import oracle
+from util import rel_l2
+
+MODULE_REL_L2, MODULE_GRAD_REL_L2, MODULE_MAX_ABS = 5e-3, 7e-3, 2.0 ** -7
+
+# B, S, E, H, causal, time_major, mask, mode
+CASES = [
+    (4, 136, 136, 2, False, True, False, "auto"),       # exactly four rows per column; one tile and a remainder everywhere
+    (5, 109, 136, 2, True, False, False, "auto"),       # one row more, odd length
+    (4, 135, 136, 2, False, True, False, "auto"),       # just below: q, k, v and ctx
+    (9, 33, 72, 3, False, False, True, "bf16"),         # tiles wider than every matrix, dense mask
+    (3, 300, 200, 1, True, True, False, "auto"),        # one head; more keys than a row kernel's first form
+    (16, 64, 256, 4, False, True, False, "auto"),       # the smallest of a model's sizes
+]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("case", CASES)
+def test_module_on_products_of_the_weights(case):
+    import torch
+    import cuda_ltc_b200 as ltc
+    from cuda_ltc_b200 import _lib
+    B, S, E, H, causal, time_major, use_mask, mode_name = case
+    mode = _lib.MODE_AUTO if mode_name == "auto" else _lib.MODE_BF16
+    ctx = ltc.Context(0)
+    rng = np.random.default_rng(7)
+    lim = np.sqrt(3.0 / E)
+    x = (0.5 * rng.standard_normal((B * S, E))).astype(np.float32)
+    dy = rng.standard_normal((B * S, E)).astype(np.float32)
+    wq, wk = (rng.uniform(-lim, lim, (E, H * E)).astype(np.float32) * 0.5 for _ in range(2))
+    wv = rng.uniform(-lim, lim, (E, H * E)).astype(np.float32)
+    wo = rng.uniform(-lim, lim, (H * E, E)).astype(np.float32)
+    m = None
+    if use_mask:
+        m = (rng.random((B, S, S)) < 0.8).astype(np.float32)
+        m[:, np.arange(S), np.arange(S)] = 1.0
+    _, y_ref = oracle.tsa_fwd(x, wq, wk, wv, wo, B, S, H, E, 1.0, causal, time_major, True, True, np.ones(E, np.float32),
+                              np.zeros(E, np.float32), None, None, None, None, m)
+    gref = oracle.tsa_bwd(x, wq, wk, wv, wo, dy, B, S, H, E, 1.0, causal, time_major, None, None, None, m)
+    dev = lambda a: None if a is None else torch.from_numpy(a).cuda()
+    args = tuple(dev(a) for a in (x, wq, wk, wv, wo))
+    kw = dict(scale=1.0, causal=causal, time_major=time_major, mode=mode, keep_mask=dev(m))
+    plain = dict(use_residual=False, use_layer_norm=False, **kw)
+    y = ctx.tsa_fwd(*args, B, S, H, E, **plain)
+    got = ctx.tsa_bwd(*args, dev(dy), B, S, H, E, **kw)
+    cache = ctx.tsa_weight_cache(*args, B, S, H, E, mode=mode, causal=causal)
+    assert rel_l2(y.cpu().numpy(), y_ref) < MODULE_REL_L2
+    assert np.abs(y.cpu().numpy() - y_ref).max() < MODULE_MAX_ABS * max(1.0, np.abs(y_ref).max())
+    for name, g, r in zip(("dx", "dwq", "dwk", "dwv", "dwo"), got, gref):
+        gh = g.cpu().numpy().astype(np.float64)
+        assert rel_l2(gh, r) < MODULE_GRAD_REL_L2, f"{name}: rel-L2 {rel_l2(gh, r)}"
+        assert np.abs(gh - r).max() < MODULE_MAX_ABS * max(1.0, np.abs(r).max()), name
+    # a kept forward, twice, and kept weights: the same bits
+    saved = ctx.tsa_saved_buffer(*args, B, S, H, E, mode=mode, causal=causal)
+    assert torch.equal(y, ctx.tsa_fwd(*args, B, S, H, E, saved=saved, weight_cache=(cache, False), **plain))
+    for valid in (True, True):
+        kept = ctx.tsa_bwd(*args, dev(dy), B, S, H, E, saved=saved, reuse_forward=True, weight_cache=(cache, valid), **kw)
+        for a, b in zip(got, kept):
+            assert torch.equal(a, b)
+    # biases go through q, k and v, in blocks sized without them
+    bias = [(0.1 * rng.standard_normal(H * E)).astype(np.float32) for _ in range(3)]
+    bkw = dict(bq=dev(bias[0]), bk=dev(bias[1]), bv=dev(bias[2]))
+    _, yb_ref = oracle.tsa_fwd(x, wq, wk, wv, wo, B, S, H, E, 1.0, causal, time_major, True, True, np.ones(E, np.float32),
+                               np.zeros(E, np.float32), *bias, None, m)
+    yb = ctx.tsa_fwd(*args, B, S, H, E, saved=saved, **bkw, **plain)
+    assert rel_l2(yb.cpu().numpy(), yb_ref) < MODULE_REL_L2
+    torch.cuda.synchronize()
+    assert ctx.device_status() == 0
+
+
+@pytest.mark.gpu
+def test_bias_gradients_without_biases():
+    """The FlashAttention form asks for bias gradients whether it has biases or not."""
+    import torch
+    import cuda_ltc_b200 as ltc
+    from cuda_ltc_b200 import _lib
+    B, S, E = 8, 140, 200
+    ctx = ltc.Context(0)
+    rng = np.random.default_rng(9)
+    lim = np.sqrt(3.0 / E)
+    x, dy = ((0.5 * rng.standard_normal((B * S, E))).astype(np.float32) for _ in range(2))
+    w = [rng.uniform(-lim, lim, (E, E)).astype(np.float32) for _ in range(4)]
+    dev = lambda a: torch.from_numpy(a).cuda()
+    args = (dev(x), *(dev(a) for a in w))
+    one, zero = torch.ones(E, device="cuda"), torch.zeros(E, device="cuda")
+    kw = dict(gamma=one, beta=zero, mode=_lib.MODE_AUTO)
+    got = ctx.fa_bwd(*args, dev(dy), B, S, 1, E, **kw)
+    # zero biases take the path through q, k and v
+    ref = ctx.fa_bwd(*args, dev(dy), B, S, 1, E, biases=(zero, zero, zero, zero), **kw)
+    out, out_ref = (ctx.fa_fwd(*args, B, S, 1, E, biases=b, **kw) for b in ((None,) * 4, (zero, zero, zero, zero)))
+    assert rel_l2(out.cpu().numpy(), out_ref.cpu().numpy()) < MODULE_REL_L2
+    for name in ("dx", "dwq", "dwk", "dwv", "dwo", "dbq", "dbv", "dbo", "dgamma", "dbeta"):
+        assert rel_l2(got[name].cpu().numpy(), ref[name].cpu().numpy()) < 2 * MODULE_GRAD_REL_L2, name
+    # (dbk: the terms of a key bias's gradient cancel, both are rounding errors of sums of |dS| |q|)
+    assert got["dbk"].abs().max() < 0.05 * ref["dbq"].abs().max()
+    torch.cuda.synchronize()
+    assert ctx.device_status() == 0
