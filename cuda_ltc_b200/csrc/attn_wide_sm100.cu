@@ -52,6 +52,16 @@ struct SoftmaxArgs {
     __nv_bfloat16 *dS, *dSlo;    // where dS goes (P / Plo themselves when the caller gave no separate buffer)
 };
 
+// Query and batch of a row, in 32 bits where the rows allow it (65536 rows of 256 keys: 24.4 us with two 64-bit divisions, 22.8).
+struct RowPlace { int i, b; };
+__device__ __forceinline__ RowPlace row_place(const SoftmaxArgs& a, int64_t row) {
+    if ((int64_t)a.B * a.H * a.Sq <= 0xffffffffll) {
+        const uint32_t r = (uint32_t)row, bh = r / (uint32_t)a.Sq;
+        return {(int)(r - bh * (uint32_t)a.Sq), (int)(bh / (uint32_t)a.H)};
+    }
+    return {(int)(row % a.Sq), (int)(row / ((int64_t)a.H * a.Sq))};
+}
+
 // One warp per (batch, head, query) row: scale, clamp (the reference clamps scaled scores at 10,
 // src/ml/flash_attention.cu:167), visibility (keep-mask value 0 hides, :161-164; causal; key lengths), softmax.
 __global__ void __launch_bounds__(256) wide_softmax_fwd_kernel(const SoftmaxArgs a) {
@@ -59,8 +69,8 @@ __global__ void __launch_bounds__(256) wide_softmax_fwd_kernel(const SoftmaxArgs
     const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (row >= (int64_t)a.B * a.H * a.Sq) return;
-    const int i = (int)(row % a.Sq);
-    const int b = (int)(row / ((int64_t)a.H * a.Sq));
+    const RowPlace at = row_place(a, row);
+    const int i = at.i, b = at.b;
     int lim = a.Sk;
     if (a.kv_len) lim = min(max(a.kv_len[b], 0), a.Sk);
     if (a.causal) lim = min(lim, i + a.causal_off + 1);
@@ -146,8 +156,8 @@ __global__ void __launch_bounds__(256) wide_softmax_fwd_rows_kernel(const Softma
     const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (row >= (int64_t)a.B * a.H * a.Sq) return;
-    const int i = (int)(row % a.Sq);
-    const int b = (int)(row / ((int64_t)a.H * a.Sq));
+    const RowPlace at = row_place(a, row);
+    const int i = at.i, b = at.b;
     int lim = a.Sk;
     if (a.kv_len) lim = min(max(a.kv_len[b], 0), a.Sk);
     if (a.causal) lim = min(lim, i + a.causal_off + 1);

@@ -46,8 +46,78 @@ __device__ __forceinline__ void put1(const RowOut& o, int64_t row, int c, float 
     if (o.bf16) o.bf16[row * o.ld_bf16 + c] = __float2bfloat16_rn(v);
 }
 
+__device__ __forceinline__ float warp_total(float v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+__device__ __forceinline__ float4 ldg4(const float* row, int i) { return __ldg(reinterpret_cast<const float4*>(row) + i); }
+
+// Rows of up to 1024 floats that stay in a warp's registers, E / 128 pieces of 16 bytes per lane: kN4 of them, where the loads of
+// a row all go out before the first is waited for, or (0) as many as E says, one after the other.  With few rows per SM a row
+// kernel lasts as long as one row's chain of loads and sums: residual + LayerNorm of 32768 x 512 37.5 us with one piece at a
+// time, 28.2 so (192 MB); 8192 x 512 12.3 and 10.3.  (The prepare launch below, whose other parts need the warps that the
+// registers would cost, 7.7 us with one at a time, 9.8 with all.)
+template <int kN4>
+struct RowPieces {
+    static constexpr int kMax = kN4 > 0 ? kN4 : 8;
+    int n;
+    __device__ __forceinline__ explicit RowPieces(int E) : n(kN4 > 0 ? kN4 : E >> 7) {}
+    __device__ __forceinline__ bool has(int i) const { return kN4 > 0 || i < n; }
+};
+
+template <int kN4>
+__device__ __forceinline__ void layer_norm_pieces(const float* __restrict__ yr, const float* __restrict__ xr, const float* __restrict__ gamma,
+                                                  const float* __restrict__ beta, const RowOut& out, int64_t row, int E, bool use_res,
+                                                  float eps) {
+    const RowPieces<kN4> p(E);
+    constexpr int kMax = RowPieces<kN4>::kMax;
+    constexpr bool kEarly = kN4 > 0 && kN4 <= 4;       // gamma and beta with the row
+    const int lane = threadIdx.x & 31;
+    float4 v[kMax], r[kMax], gm[kEarly ? kMax : 1], bt[kEarly ? kMax : 1];
+    const float4 one = make_float4(1.f, 1.f, 1.f, 1.f), zero = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < kMax; ++i)
+        if (p.has(i)) {
+            v[i] = ldg4(yr, lane + 32 * i);
+            r[i] = use_res ? ldg4(xr, lane + 32 * i) : zero;
+        }
+    if constexpr (kEarly) {
+#pragma unroll
+        for (int i = 0; i < kMax; ++i) {
+            gm[i] = gamma ? ldg4(gamma, lane + 32 * i) : one;
+            bt[i] = beta ? ldg4(beta, lane + 32 * i) : zero;
+        }
+    }
+    float sum = 0.f;
+#pragma unroll
+    for (int i = 0; i < kMax; ++i)
+        if (p.has(i)) {
+            if (use_res) { v[i].x += r[i].x; v[i].y += r[i].y; v[i].z += r[i].z; v[i].w += r[i].w; }
+            sum += (v[i].x + v[i].y) + (v[i].z + v[i].w);
+        }
+    const float mean = warp_total(sum) / E;
+    float var = 0.f;
+#pragma unroll
+    for (int i = 0; i < kMax; ++i)
+        if (p.has(i)) {
+            const float a = v[i].x - mean, b = v[i].y - mean, c = v[i].z - mean, d = v[i].w - mean;
+            var = fmaf(a, a, var); var = fmaf(b, b, var); var = fmaf(c, c, var); var = fmaf(d, d, var);
+        }
+    const float inv = rsqrtf(warp_total(var) / E + eps);
+#pragma unroll
+    for (int i = 0; i < kMax; ++i)
+        if (p.has(i)) {
+            const float4 g = kEarly ? gm[kEarly ? i : 0] : gamma ? ldg4(gamma, lane + 32 * i) : one;
+            const float4 t = kEarly ? bt[kEarly ? i : 0] : beta ? ldg4(beta, lane + 32 * i) : zero;
+            put4(out, row, 4 * (lane + 32 * i), make_float4((v[i].x - mean) * inv * g.x + t.x, (v[i].y - mean) * inv * g.y + t.y,
+                                                            (v[i].z - mean) * inv * g.z + t.z, (v[i].w - mean) * inv * g.w + t.w));
+        }
+}
+
 // One row by one warp: LayerNorm(y (+ x)), or just the sum / a copy.  `vec`: every row of every operand starts on a
-// 16-byte boundary and E is a multiple of 4.
+// 16-byte boundary and E is a multiple of 4.  kBatch: a kernel that does nothing else spends registers on a row's loads.
+template <bool kBatch>
 __device__ __forceinline__ void layer_norm_row(const float* __restrict__ y, const float* __restrict__ x,
                                                const float* __restrict__ gamma, const float* __restrict__ beta, const RowOut& out,
                                                int64_t row, int E, bool use_res, bool use_ln, float eps, bool vec) {
@@ -55,49 +125,11 @@ __device__ __forceinline__ void layer_norm_row(const float* __restrict__ y, cons
     const float* yr = y + row * E;
     const float* xr = x + row * E;
     if (use_ln && vec && (E & 127) == 0 && E <= 1024) {
-        // the row stays in registers: one read of y and x, one write of the result
-        float4 v[8];
-        const int n4 = E >> 7;                        // float4 per lane
-        float sum4 = 0.f;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            if (i < n4) {
-                v[i] = __ldg(reinterpret_cast<const float4*>(yr) + lane + 32 * i);
-                if (use_res) {
-                    const float4 r = __ldg(reinterpret_cast<const float4*>(xr) + lane + 32 * i);
-                    v[i].x += r.x; v[i].y += r.y; v[i].z += r.z; v[i].w += r.w;
-                }
-                sum4 += (v[i].x + v[i].y) + (v[i].z + v[i].w);
-            }
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) sum4 += __shfl_xor_sync(0xffffffffu, sum4, o);
-        const float mean4 = sum4 / E;
-        float var4 = 0.f;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            if (i < n4) {
-                const float a = v[i].x - mean4, b = v[i].y - mean4, c = v[i].z - mean4, d = v[i].w - mean4;
-                var4 = fmaf(a, a, var4); var4 = fmaf(b, b, var4); var4 = fmaf(c, c, var4); var4 = fmaf(d, d, var4);
-            }
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) var4 += __shfl_xor_sync(0xffffffffu, var4, o);
-        const float inv4 = rsqrtf(var4 / E + eps);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            if (i < n4) {
-                float4 gm = make_float4(1.f, 1.f, 1.f, 1.f), bt = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (gamma) gm = __ldg(reinterpret_cast<const float4*>(gamma) + lane + 32 * i);
-                if (beta) bt = __ldg(reinterpret_cast<const float4*>(beta) + lane + 32 * i);
-                float4 o4;
-                o4.x = (v[i].x - mean4) * inv4 * gm.x + bt.x;
-                o4.y = (v[i].y - mean4) * inv4 * gm.y + bt.y;
-                o4.z = (v[i].z - mean4) * inv4 * gm.z + bt.z;
-                o4.w = (v[i].w - mean4) * inv4 * gm.w + bt.w;
-                put4(out, row, 4 * (lane + 32 * i), o4);
-            }
-        }
+        // one read of y and x, one write of the result
+        if (kBatch && E == 512) layer_norm_pieces<4>(yr, xr, gamma, beta, out, row, E, use_res, eps);
+        else if (kBatch && E == 256) layer_norm_pieces<2>(yr, xr, gamma, beta, out, row, E, use_res, eps);
+        else if (kBatch && E == 128) layer_norm_pieces<1>(yr, xr, gamma, beta, out, row, E, use_res, eps);
+        else layer_norm_pieces<0>(yr, xr, gamma, beta, out, row, E, use_res, eps);
         return;
     }
     auto value = [&](int i) { return yr[i] + (use_res ? xr[i] : 0.f); };
@@ -135,7 +167,7 @@ __global__ void residual_layer_norm_kernel(const float* __restrict__ y, const fl
     const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (row >= rows) return;
     const RowOut o{out, nullptr, E, 0};
-    layer_norm_row(y, x, gamma, beta, o, row, E, use_res != 0, use_ln != 0, eps, aligned16(y, x, gamma, beta, out));
+    layer_norm_row<true>(y, x, gamma, beta, o, row, E, use_res != 0, use_ln != 0, eps, aligned16(y, x, gamma, beta, out));
     // y is scratch and this was its only reader: whole lines of it that still lie in L2 need not be written to HBM
     // (32768 x 512: 45.3 -> 43.6 us, and the module forward of 8192 rows 58.6 -> 57.1).  The row's stores above depend on
     // every lane's loads, so nothing of it is still on its way.
@@ -202,7 +234,7 @@ __global__ void __launch_bounds__(kPrepareThreads) prenorm_prepare_kernel(const 
         const int64_t row = (int64_t)block * (kPrepareThreads / 32) + (threadIdx.x >> 5);
         if (row >= a.rows) return;
         const bool vec = aligned16(a.x, a.gamma, a.beta, a.xo.f32, a.xo.bf16);
-        layer_norm_row(a.x, a.x, a.gamma, a.beta, a.xo, row, a.E, false, a.use_ln != 0, a.eps, vec);
+        layer_norm_row<false>(a.x, a.x, a.gamma, a.beta, a.xo, row, a.E, false, a.use_ln != 0, a.eps, vec);
         return;
     }
     block -= a.row_blocks;
@@ -267,6 +299,64 @@ __global__ void __launch_bounds__(256) residual_dropout_kernel(const float* __re
     }
 }
 
+// Its registers form: both rows are read once, in 16-byte pieces.
+template <int kN4>
+__device__ __forceinline__ void layer_norm_bwd_pieces(const float* __restrict__ gr, const float* __restrict__ xr, const float* __restrict__ gamma,
+                                                      const float* __restrict__ res, float* __restrict__ dx, float* __restrict__ prod, int E,
+                                                      float eps) {
+    const RowPieces<kN4> p(E);
+    constexpr int kMax = RowPieces<kN4>::kMax;
+    const int lane = threadIdx.x & 31;
+    float4 xh[kMax], gv[kMax], gm[kMax], r[kMax];
+#pragma unroll
+    for (int i = 0; i < kMax; ++i)
+        if (p.has(i)) {
+            xh[i] = ldg4(xr, lane + 32 * i);
+            gv[i] = ldg4(gr, lane + 32 * i);
+            gm[i] = ldg4(gamma, lane + 32 * i);
+            r[i] = dx && res ? ldg4(res, lane + 32 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    float s0 = 0.f;
+#pragma unroll
+    for (int i = 0; i < kMax; ++i)
+        if (p.has(i)) s0 += (xh[i].x + xh[i].y) + (xh[i].z + xh[i].w);
+    const float mean = warp_total(s0) / E;
+    float s1 = 0.f;
+#pragma unroll
+    for (int i = 0; i < kMax; ++i)
+        if (p.has(i)) {
+            xh[i].x -= mean; xh[i].y -= mean; xh[i].z -= mean; xh[i].w -= mean;
+            s1 = fmaf(xh[i].x, xh[i].x, s1); s1 = fmaf(xh[i].y, xh[i].y, s1);
+            s1 = fmaf(xh[i].z, xh[i].z, s1); s1 = fmaf(xh[i].w, xh[i].w, s1);
+        }
+    const float inv_std = rsqrtf(warp_total(s1) / E + eps);
+    float a1 = 0.f, a2 = 0.f;
+#pragma unroll
+    for (int i = 0; i < kMax; ++i)
+        if (p.has(i)) {
+            xh[i].x *= inv_std; xh[i].y *= inv_std; xh[i].z *= inv_std; xh[i].w *= inv_std;
+            const float4 gg = make_float4(gv[i].x * gm[i].x, gv[i].y * gm[i].y, gv[i].z * gm[i].z, gv[i].w * gm[i].w);
+            a1 += (gg.x + gg.y) + (gg.z + gg.w);
+            a2 = fmaf(gg.x, xh[i].x, a2); a2 = fmaf(gg.y, xh[i].y, a2);
+            a2 = fmaf(gg.z, xh[i].z, a2); a2 = fmaf(gg.w, xh[i].w, a2);
+            if (prod)
+                reinterpret_cast<float4*>(prod)[lane + 32 * i] =
+                    make_float4(gv[i].x * xh[i].x, gv[i].y * xh[i].y, gv[i].z * xh[i].z, gv[i].w * xh[i].w);
+            gv[i] = gg;
+        }
+    if (!dx) return;
+    const float m1 = warp_total(a1) / E, m2 = warp_total(a2) / E;
+#pragma unroll
+    for (int i = 0; i < kMax; ++i)
+        if (p.has(i)) {
+            r[i].x += inv_std * (gv[i].x - m1 - xh[i].x * m2);
+            r[i].y += inv_std * (gv[i].y - m1 - xh[i].y * m2);
+            r[i].z += inv_std * (gv[i].z - m1 - xh[i].z * m2);
+            r[i].w += inv_std * (gv[i].w - m1 - xh[i].w * m2);
+            reinterpret_cast<float4*>(dx)[lane + 32 * i] = r[i];
+        }
+}
+
 // LayerNorm backward, one warp per row.  g = gradient at the LayerNorm output, x = its input.
 //   dx = inv_std * (g*gamma - mean(g*gamma) - xhat * mean(g*gamma*xhat))  (+ res[row] when res != null)
 // dx and prod are optional; prod receives g * xhat, whose column sums are dgamma.
@@ -281,60 +371,12 @@ __global__ void layer_norm_bwd_kernel(const float* __restrict__ g, const float* 
     const float* xr = x + row * E;
     const float* gr = g + row * E;
     if ((E & 127) == 0 && E <= 1024 && aligned16(g, x, gamma, res, dx) && (reinterpret_cast<uintptr_t>(prod) & 15) == 0) {
-        // both rows stay in registers: every operand is read once, in 16-byte pieces
-        auto warp_sum = [](float v) {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            return v;
-        };
-        const int n4 = E >> 7;
-        float4 xh[8], gv[8];
-        float s0 = 0.f;
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-            if (i < n4) {
-                xh[i] = __ldg(reinterpret_cast<const float4*>(xr) + lane + 32 * i);
-                gv[i] = __ldg(reinterpret_cast<const float4*>(gr) + lane + 32 * i);
-                s0 += (xh[i].x + xh[i].y) + (xh[i].z + xh[i].w);
-            }
-        const float mean = warp_sum(s0) / E;
-        float s1 = 0.f;
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-            if (i < n4) {
-                xh[i].x -= mean; xh[i].y -= mean; xh[i].z -= mean; xh[i].w -= mean;
-                s1 = fmaf(xh[i].x, xh[i].x, s1); s1 = fmaf(xh[i].y, xh[i].y, s1);
-                s1 = fmaf(xh[i].z, xh[i].z, s1); s1 = fmaf(xh[i].w, xh[i].w, s1);
-            }
-        const float inv_std = rsqrtf(warp_sum(s1) / E + eps);
-        float a1 = 0.f, a2 = 0.f;
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-            if (i < n4) {
-                const float4 gm = __ldg(reinterpret_cast<const float4*>(gamma) + lane + 32 * i);
-                xh[i].x *= inv_std; xh[i].y *= inv_std; xh[i].z *= inv_std; xh[i].w *= inv_std;
-                const float4 gg = make_float4(gv[i].x * gm.x, gv[i].y * gm.y, gv[i].z * gm.z, gv[i].w * gm.w);
-                a1 += (gg.x + gg.y) + (gg.z + gg.w);
-                a2 = fmaf(gg.x, xh[i].x, a2); a2 = fmaf(gg.y, xh[i].y, a2);
-                a2 = fmaf(gg.z, xh[i].z, a2); a2 = fmaf(gg.w, xh[i].w, a2);
-                if (prod)
-                    reinterpret_cast<float4*>(prod + row * E)[lane + 32 * i] =
-                        make_float4(gv[i].x * xh[i].x, gv[i].y * xh[i].y, gv[i].z * xh[i].z, gv[i].w * xh[i].w);
-                gv[i] = gg;
-            }
-        if (!dx) return;
-        const float m1 = warp_sum(a1) / E, m2 = warp_sum(a2) / E;
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-            if (i < n4) {
-                float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (res) r = __ldg(reinterpret_cast<const float4*>(res + row * E) + lane + 32 * i);
-                r.x += inv_std * (gv[i].x - m1 - xh[i].x * m2);
-                r.y += inv_std * (gv[i].y - m1 - xh[i].y * m2);
-                r.z += inv_std * (gv[i].z - m1 - xh[i].z * m2);
-                r.w += inv_std * (gv[i].w - m1 - xh[i].w * m2);
-                reinterpret_cast<float4*>(dx + row * E)[lane + 32 * i] = r;
-            }
+        const float* rr = res ? res + row * E : nullptr;
+        float *dr = dx ? dx + row * E : nullptr, *pr = prod ? prod + row * E : nullptr;
+        if (E == 512) layer_norm_bwd_pieces<4>(gr, xr, gamma, rr, dr, pr, E, eps);
+        else if (E == 256) layer_norm_bwd_pieces<2>(gr, xr, gamma, rr, dr, pr, E, eps);
+        else if (E == 128) layer_norm_bwd_pieces<1>(gr, xr, gamma, rr, dr, pr, E, eps);
+        else layer_norm_bwd_pieces<0>(gr, xr, gamma, rr, dr, pr, E, eps);
         return;
     }
     float sum = 0.f;
