@@ -38,6 +38,10 @@ struct CoreArgs {
     const int32_t* kv_len;
     const uint32_t* mask_bits;  // backward: the dense mask packed, [B, Sq, mask_nw]; null: no room for it
     int mask_nw;
+    // dq kernel: dO is not there yet, it is dy Wo_h^T (see FromOutput); dO's rows are written for the dK/dV kernel
+    const float *dy, *wo;
+    int64_t dy_batch, dy_seq;
+    int E;
     int vec;            // every row starts on a 16-byte (fp32) or 8-byte (bf16) boundary and holds a multiple of 4 elements
 };
 
@@ -458,8 +462,41 @@ __global__ void attn_bwd_delta_kernel(const CoreArgs a) {
 // ----------------------------------------------------------------------------------------------
 // backward
 // ----------------------------------------------------------------------------------------------
+// dst[r][c] = dO[r0 + r][c] = sum over e of dy[r0 + r][e] Wo[h D + c][e], e ascending as in the product that this replaces, also
+// written to dO's rows.  A thread keeps a row of Wo's head for its column c and goes down the tile's rows, whose dy its warp
+// reads at one address.
+template <int DP, int ROWS, int NT>
+__device__ __forceinline__ void form_dout(float* dst, const CoreArgs& a, int b, int h, int r0) {
+    constexpr int LD = DP + kPad, RT = NT / DP, NR = ROWS / RT;
+    const int c = threadIdx.x % DP, rt = threadIdx.x / DP;
+    const float* w = a.wo + ((int64_t)h * a.D + min(c, a.D - 1)) * a.E;
+    const float* d = a.dy + b * a.dy_batch;
+    float g[NR];
+#pragma unroll
+    for (int i = 0; i < NR; ++i) g[i] = 0.f;
+    for (int e = 0; e < a.E; e += 8) {                         // (a multiple of 8)
+        const float4 w0 = ld4(w + e), w1 = ld4(w + e + 4);
+#pragma unroll
+        for (int i = 0; i < NR; ++i) {
+            const float* row = d + (int64_t)min(r0 + rt + RT * i, a.Sq - 1) * a.dy_seq + e;
+            const float4 x0 = ld4(row), x1 = ld4(row + 4);
+            g[i] = fmaf(x0.x, w0.x, g[i]); g[i] = fmaf(x0.y, w0.y, g[i]); g[i] = fmaf(x0.z, w0.z, g[i]); g[i] = fmaf(x0.w, w0.w, g[i]);
+            g[i] = fmaf(x1.x, w1.x, g[i]); g[i] = fmaf(x1.y, w1.y, g[i]); g[i] = fmaf(x1.z, w1.z, g[i]); g[i] = fmaf(x1.w, w1.w, g[i]);
+        }
+    }
+    float* out = const_cast<float*>(reinterpret_cast<const float*>(a.dout)) + b * a.dos.batch + h * a.dos.head + c;
+#pragma unroll
+    for (int i = 0; i < NR; ++i) {
+        const int r = rt + RT * i;
+        const bool in = r0 + r < a.Sq && c < a.D;
+        dst[r * LD + c] = in ? g[i] : 0.f;
+        if (in) out[(int64_t)(r0 + r) * a.dos.seq] = g[i];
+    }
+}
+
 // pass 1: delta = rowsum(dO o O), left for pass 2, and dQ.  One CTA per TM query rows, KN keys per step.
-template <typename T, int DP, int TM, int KN, int NT, int kMask>
+// kForm: dO is formed here (a kernel of its own, since form_dout takes registers: without it twice as many CTAs fit on an SM).
+template <typename T, int DP, int TM, int KN, int NT, int kMask, bool kForm>
 __global__ void __launch_bounds__(NT, NT == 128 ? 3 : 1) attn_bwd_dq_fp32_kernel(const CoreArgs a) {
     grid_dependency_wait();
     constexpr int LD = DP + kPad, LP = KN + kPad, RS = NT / 16, RM = TM / RS, CN = KN / 16, NW = KN / 32;
@@ -485,10 +522,11 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 3 : 1) attn_bwd_dq_fp32_kernel
     const T* gb = reinterpret_cast<const T*>(a.dout) + b * a.dos.batch + h * a.dos.head;
     const T* ob = reinterpret_cast<const T*>(a.o_in) + b * a.os.batch + h * a.os.head;
     load_padded<DP, TM, NT>(Qs, qb, a.qs.seq, q0, a.Sq, a.D, vec);
-    load_padded<DP, TM, NT>(Gs, gb, a.dos.seq, q0, a.Sq, a.D, vec);
+    if constexpr (!kForm) load_padded<DP, TM, NT>(Gs, gb, a.dos.seq, q0, a.Sq, a.D, vec);
     load_padded<DP, KN, NT>(Ks, kb, a.ks.seq, 0, a.Sk, a.D, vec);
     load_padded<DP, KN, NT>(Vs, vb, a.vs.seq, 0, a.Sk, a.D, vec);
     cp_async_commit();
+    if constexpr (kForm) form_dout<DP, TM, NT>(Gs, a, b, h, q0);
     cp_async_wait<0>();
     __syncthreads();
 
@@ -767,14 +805,14 @@ int run_fwd(ltca_ctx* ctx, const CoreArgs& a) {
     return LTCA_OK;
 }
 
-template <typename T, int DP, int TM, int KN, int NT, int kMask>
+template <typename T, int DP, int TM, int KN, int NT, int kMask, bool kForm = false>
 int run_dq(ltca_ctx* ctx, const CoreArgs& a) {
     static SmemOptIn once;
     constexpr size_t smem = ((size_t)(2 * TM + 2 * KN) * (DP + kPad) + TM * (KN + kPad) + TM) * sizeof(float);
-    int rc = set_smem(ctx, attn_bwd_dq_fp32_kernel<T, DP, TM, KN, NT, kMask>, smem, once);
+    int rc = set_smem(ctx, attn_bwd_dq_fp32_kernel<T, DP, TM, KN, NT, kMask, kForm>, smem, once);
     if (rc) return rc;
     dim3 grid((a.Sq + TM - 1) / TM, a.H, a.B);
-    LTCA_CUDA_OK(ctx, launch_dependent(attn_bwd_dq_fp32_kernel<T, DP, TM, KN, NT, kMask>, grid, dim3(NT), smem, ctx->stream, a));
+    LTCA_CUDA_OK(ctx, launch_dependent(attn_bwd_dq_fp32_kernel<T, DP, TM, KN, NT, kMask, kForm>, grid, dim3(NT), smem, ctx->stream, a));
     return LTCA_OK;
 }
 template <typename T, int DP, int TK, int QN, int NT, int kMask>
@@ -792,19 +830,26 @@ int run_dkv(ltca_ctx* ctx, const CoreArgs& a) {
 // done, they take whatever slots are left and sit unevenly on the SMs, 82 or 62 us instead of 57 for B16 H8 S100 D32.)
 // Tiles of 64 rows reuse what they load most; where they would leave SMs idle, tiles of 16 rows give four times the CTAs
 // and a quarter of the serial work.
+template <typename T, int DP, int kMask>
+int run_small_dq(ltca_ctx* ctx, const CoreArgs& a) {
+    if constexpr (sizeof(T) == 4 && DP <= 64) {
+        if (a.dy) return run_dq<T, DP, 16, 32, 128, kMask, true>(ctx, a);
+    }
+    return run_dq<T, DP, 16, 32, 128, kMask>(ctx, a);
+}
+bool fills_sms(const ltca_ctx* ctx, int B, int H, int S) { return (int64_t)B * H * ((S + 63) / 64) >= ctx->sm_device; }
 template <typename T, int DP, bool kMask>
 int run_rows(ltca_ctx* ctx, const CoreArgs& a, bool bwd) {
-    const int64_t bh = (int64_t)a.B * a.H;
-    auto fills = [&](int S) { return bh * ((S + 63) / 64) >= ctx->sm_device; };
+    auto fills = [&](int S) { return fills_sms(ctx, a.B, a.H, S); };
     constexpr int NT = DP > 64 ? 256 : 128;         // at DP = 128 eight columns per thread need the wider CTA
     if (!bwd) return fills(a.Sq) ? run_fwd<T, DP, 64, NT, kMask>(ctx, a) : run_fwd<T, DP, 16, 128, kMask>(ctx, a);
     int rc;
     if constexpr (kMask) {
         // without room for the mask's words: the small tiles alone, whose results have the same bits
-        if (!a.mask_bits) return (rc = run_dq<T, DP, 16, 32, 128, kDense>(ctx, a)) ? rc : run_dkv<T, DP, 16, 32, 128, kDense>(ctx, a);
+        if (!a.mask_bits) return (rc = run_small_dq<T, DP, kDense>(ctx, a)) ? rc : run_dkv<T, DP, 16, 32, 128, kDense>(ctx, a);
     }
     constexpr int kM = kMask ? kWords : kNoMask;
-    if ((rc = fills(a.Sq) ? run_dq<T, DP, 64, 64, NT, kM>(ctx, a) : run_dq<T, DP, 16, 32, 128, kM>(ctx, a))) return rc;
+    if ((rc = fills(a.Sq) ? run_dq<T, DP, 64, 64, NT, kM>(ctx, a) : run_small_dq<T, DP, kM>(ctx, a))) return rc;
     return fills(a.Sk) ? run_dkv<T, DP, 64, 64, NT, kM>(ctx, a) : run_dkv<T, DP, 16, 32, 128, kM>(ctx, a);
 }
 template <typename T, int DP>
@@ -1031,13 +1076,23 @@ int launch_attn_fwd_fp32(ltca_ctx* ctx, const ltca_attn_params* p) {
     return p->dtype == LTCA_BF16 ? dispatch<__nv_bfloat16>(ctx, a, false) : dispatch<float>(ctx, a, false);
 }
 
-int launch_attn_bwd_fp32(ltca_ctx* ctx, const ltca_attn_params* p) {
+bool attn_bwd_fp32_forms_dout(const ltca_ctx* ctx, const ltca_attn_params* p, const FromOutput& f) {
+    const auto al = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
+    return p->dtype == LTCA_F32 && p->D <= 64 && !fills_sms(ctx, p->B, p->H, p->Sq) && f.E <= kFormDoutMaxE && (f.E % 8) == 0 &&
+           (int64_t)p->B * p->Sq <= kFormDoutRows && al(f.dy) && al(f.wo);
+}
+
+int launch_attn_bwd_fp32(ltca_ctx* ctx, const ltca_attn_params* p, const FromOutput* from) {
     if (p->D < 1 || p->D > kWideMaxD)
         return fail(ctx, LTCA_ERR_UNSUPPORTED, "fp32 attention supports head_dim 1..%d, got %d", kWideMaxD, p->D);
     if (p->workspace_bytes < delta_bytes(p) || !p->workspace)
         return fail(ctx, LTCA_ERR_WORKSPACE, "backward needs %zu bytes of workspace", delta_bytes(p));
     CoreArgs a = make_args(p);
     a.delta = reinterpret_cast<float*>(p->workspace);
+    if (from) {
+        a.dy = from->dy; a.wo = from->wo; a.E = from->E;
+        a.dy_batch = from->batch; a.dy_seq = from->seq;
+    }
     if (p->D <= 128) {
         const void* words = nullptr;
         if (int rc = mask_words_of(ctx, p, delta_bytes(p), &words)) return rc;

@@ -410,6 +410,10 @@ int pack_many_to_bf16(ltca_ctx* ctx, const PackJob* jobs, int count, int B, int 
     LTCA_LAUNCH_OK(ctx, "pack_bf16_kernel");
     return LTCA_OK;
 }
+
+bool attn_bwd_exact(const ltca_attn_params* p) {
+    return p->mode != LTCA_MODE_BF16 && !wide_core_path(p, true) && !tensor_path(p, true);
+}
 }  // namespace ltca
 
 using namespace ltca;

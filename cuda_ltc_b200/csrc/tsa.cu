@@ -74,13 +74,13 @@ __device__ __forceinline__ void layer_norm_pieces(const float* __restrict__ yr, 
     constexpr int kMax = RowPieces<kN4>::kMax;
     constexpr bool kEarly = kN4 > 0 && kN4 <= 4;       // gamma and beta with the row
     const int lane = threadIdx.x & 31;
-    float4 v[kMax], r[kMax], gm[kEarly ? kMax : 1], bt[kEarly ? kMax : 1];
+    float4 v[kMax], r[kN4 > 0 ? kMax : 1], gm[kEarly ? kMax : 1], bt[kEarly ? kMax : 1];
     const float4 one = make_float4(1.f, 1.f, 1.f, 1.f), zero = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
     for (int i = 0; i < kMax; ++i)
         if (p.has(i)) {
             v[i] = ldg4(yr, lane + 32 * i);
-            r[i] = use_res ? ldg4(xr, lane + 32 * i) : zero;
+            if constexpr (kN4 > 0) r[i] = use_res ? ldg4(xr, lane + 32 * i) : zero;
         }
     if constexpr (kEarly) {
 #pragma unroll
@@ -93,7 +93,10 @@ __device__ __forceinline__ void layer_norm_pieces(const float* __restrict__ yr, 
 #pragma unroll
     for (int i = 0; i < kMax; ++i)
         if (p.has(i)) {
-            if (use_res) { v[i].x += r[i].x; v[i].y += r[i].y; v[i].z += r[i].z; v[i].w += r[i].w; }
+            if (use_res) {
+                const float4 x = kN4 > 0 ? r[kN4 > 0 ? i : 0] : ldg4(xr, lane + 32 * i);
+                v[i].x += x.x; v[i].y += x.y; v[i].z += x.z; v[i].w += x.w;
+            }
             sum += (v[i].x + v[i].y) + (v[i].z + v[i].w);
         }
     const float mean = warp_total(sum) / E;
@@ -116,8 +119,8 @@ __device__ __forceinline__ void layer_norm_pieces(const float* __restrict__ yr, 
 }
 
 // One row by one warp: LayerNorm(y (+ x)), or just the sum / a copy.  `vec`: every row of every operand starts on a
-// 16-byte boundary and E is a multiple of 4.  kBatch: a kernel that does nothing else spends registers on a row's loads.
-template <bool kBatch>
+// 16-byte boundary and E is a multiple of 4.  kN4 > 0: rows of 128 kN4 floats, all of a row's loads in flight (see RowPieces).
+template <int kN4>
 __device__ __forceinline__ void layer_norm_row(const float* __restrict__ y, const float* __restrict__ x,
                                                const float* __restrict__ gamma, const float* __restrict__ beta, const RowOut& out,
                                                int64_t row, int E, bool use_res, bool use_ln, float eps, bool vec) {
@@ -126,10 +129,7 @@ __device__ __forceinline__ void layer_norm_row(const float* __restrict__ y, cons
     const float* xr = x + row * E;
     if (use_ln && vec && (E & 127) == 0 && E <= 1024) {
         // one read of y and x, one write of the result
-        if (kBatch && E == 512) layer_norm_pieces<4>(yr, xr, gamma, beta, out, row, E, use_res, eps);
-        else if (kBatch && E == 256) layer_norm_pieces<2>(yr, xr, gamma, beta, out, row, E, use_res, eps);
-        else if (kBatch && E == 128) layer_norm_pieces<1>(yr, xr, gamma, beta, out, row, E, use_res, eps);
-        else layer_norm_pieces<0>(yr, xr, gamma, beta, out, row, E, use_res, eps);
+        layer_norm_pieces<kN4>(yr, xr, gamma, beta, out, row, E, use_res, eps);
         return;
     }
     auto value = [&](int i) { return yr[i] + (use_res ? xr[i] : 0.f); };
@@ -159,6 +159,7 @@ __device__ __forceinline__ bool aligned16(const void* a, const void* b, const vo
              reinterpret_cast<uintptr_t>(d) | reinterpret_cast<uintptr_t>(e)) & 15) == 0;
 }
 
+template <int kN4>
 __global__ void residual_layer_norm_kernel(const float* __restrict__ y, const float* __restrict__ x,
                                            const float* __restrict__ gamma,
                                            const float* __restrict__ beta, float* __restrict__ out,
@@ -167,7 +168,7 @@ __global__ void residual_layer_norm_kernel(const float* __restrict__ y, const fl
     const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (row >= rows) return;
     const RowOut o{out, nullptr, E, 0};
-    layer_norm_row<true>(y, x, gamma, beta, o, row, E, use_res != 0, use_ln != 0, eps, aligned16(y, x, gamma, beta, out));
+    layer_norm_row<kN4>(y, x, gamma, beta, o, row, E, use_res != 0, use_ln != 0, eps, aligned16(y, x, gamma, beta, out));
     // y is scratch and this was its only reader: whole lines of it that still lie in L2 need not be written to HBM
     // (32768 x 512: 45.3 -> 43.6 us, and the module forward of 8192 rows 58.6 -> 57.1).  The row's stores above depend on
     // every lane's loads, so nothing of it is still on its way.
@@ -179,9 +180,93 @@ __global__ void residual_layer_norm_kernel(const float* __restrict__ y, const fl
 
 int residual_layer_norm(ltca_ctx* ctx, const ltca_tsa_params* t, const float* y, int64_t rows) {
     const int wpb = 8;
-    LTCA_CUDA_OK(ctx, launch_dependent(residual_layer_norm_kernel, dim3((unsigned)((rows + wpb - 1) / wpb)), dim3(wpb * 32),
+    auto kern = t->E == 512 ? residual_layer_norm_kernel<4> : t->E == 256 ? residual_layer_norm_kernel<2>
+              : t->E == 128 ? residual_layer_norm_kernel<1> : residual_layer_norm_kernel<0>;
+    LTCA_CUDA_OK(ctx, launch_dependent(kern, dim3((unsigned)((rows + wpb - 1) / wpb)), dim3(wpb * 32),
                                        0, ctx->stream, y, t->x, t->ln_gamma, t->ln_beta, t->out, rows, t->E,
                                        t->use_residual, t->use_layer_norm, 1e-5f));
+    return LTCA_OK;
+}
+
+// The end of a small exact forward in one launch: out = LayerNorm(x + ctx Wo + bo), a warp to a row of at most 64 columns, Wo in
+// shared memory.  As a product and a row kernel these were two of the eight dependent launches of a small training step, each
+// of which costs 3 to 4 us whatever it computes: step of B8 S32 E32 H4 32.3 -> 29.3 us, forward of B32 S128 E32 H4 34.8 -> 33.8.
+// Every block reads all of Wo: with 64 KB of it 2048 rows of the forward B32 S64 E64 H8 width 32 take 33.9 us instead of 32.7,
+// so it is limited to 32 KB, and to 4096 rows.
+constexpr int kProjThreads = 256, kProjMaxE = 64, kProjMaxWeights = 8192, kProjRows = 4096;
+__global__ void __launch_bounds__(kProjThreads) project_norm_kernel(const float* __restrict__ ctx, const float* __restrict__ wo,
+                                                                    const float* __restrict__ bo, const float* __restrict__ x,
+                                                                    const float* __restrict__ gamma, const float* __restrict__ beta,
+                                                                    float* __restrict__ out, int rows, int HW, int E, int use_res, int use_ln,
+                                                                    float eps) {
+    grid_dependency_wait();
+    extern __shared__ __align__(16) float proj_sm[];
+    float* ws = proj_sm;                                       // [HW][E]
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    float* cs = proj_sm + HW * E + warp * HW;                  // this warp's row of ctx
+    const int row = blockIdx.x * (kProjThreads / 32) + warp;
+    const bool live = row < rows;
+    for (int i = threadIdx.x; i < HW * E / 4; i += kProjThreads)
+        reinterpret_cast<float4*>(ws)[i] = __ldg(reinterpret_cast<const float4*>(wo) + i);
+    if (live)
+        for (int i = lane; i < HW / 4; i += 32)
+            reinterpret_cast<float4*>(cs)[i] = __ldg(reinterpret_cast<const float4*>(ctx + (int64_t)row * HW) + i);
+    float v[kProjMaxE / 32], res[kProjMaxE / 32], gm[kProjMaxE / 32], bt[kProjMaxE / 32];
+#pragma unroll
+    for (int j = 0; j < kProjMaxE / 32; ++j) {
+        const int c = lane + 32 * j;
+        const bool in = live && c < E;
+        res[j] = (in && use_res ? __ldg(x + (int64_t)row * E + c) : 0.f) + (in && bo ? __ldg(bo + c) : 0.f);
+        gm[j] = in && gamma ? __ldg(gamma + c) : 1.f;
+        bt[j] = in && beta ? __ldg(beta + c) : 0.f;
+    }
+    __syncthreads();
+    if (!live) return;
+#pragma unroll
+    for (int j = 0; j < kProjMaxE / 32; ++j) {
+        const int c = lane + 32 * j;
+        float acc[4] = {0.f, 0.f, 0.f, 0.f};
+        if (c < E) {
+#pragma unroll 4
+            for (int k = 0; k < HW; k += 4) {
+                const float4 a = *reinterpret_cast<const float4*>(cs + k);
+                acc[0] = fmaf(a.x, ws[k * E + c], acc[0]);
+                acc[1] = fmaf(a.y, ws[(k + 1) * E + c], acc[1]);
+                acc[2] = fmaf(a.z, ws[(k + 2) * E + c], acc[2]);
+                acc[3] = fmaf(a.w, ws[(k + 3) * E + c], acc[3]);
+            }
+        }
+        v[j] = (acc[0] + acc[1]) + (acc[2] + acc[3]) + res[j];
+    }
+    float mean = 0.f, inv = 1.f;
+    if (use_ln) {
+        float sum = 0.f, var = 0.f;
+#pragma unroll
+        for (int j = 0; j < kProjMaxE / 32; ++j) sum += v[j];      // (columns beyond E hold zeros)
+        mean = warp_total(sum) / E;
+#pragma unroll
+        for (int j = 0; j < kProjMaxE / 32; ++j)
+            if (lane + 32 * j < E) var = fmaf(v[j] - mean, v[j] - mean, var);
+        inv = rsqrtf(warp_total(var) / E + eps);
+    }
+#pragma unroll
+    for (int j = 0; j < kProjMaxE / 32; ++j)
+        if (lane + 32 * j < E) out[(int64_t)row * E + lane + 32 * j] = use_ln ? fmaf((v[j] - mean) * inv, gm[j], bt[j]) : v[j];
+}
+// Whether that kernel takes the call (ctx is the library's own buffer, aligned and contiguous).
+bool projects_and_norms(const ltca_tsa_params* t, int64_t rows, int HW) {
+    return t->E <= kProjMaxE && (t->E % 4) == 0 && (HW % 4) == 0 && HW * t->E <= kProjMaxWeights && rows <= kProjRows &&
+           (reinterpret_cast<uintptr_t>(t->wo) & 15) == 0;
+}
+int project_norm(ltca_ctx* ctx, const ltca_tsa_params* t, const float* core, int64_t rows, int HW) {
+    static SmemOptIn once;
+    constexpr int kMost = (kProjMaxWeights + kProjThreads / 32 * kProjMaxWeights / 4) * (int)sizeof(float);   // HW <= kProjMaxWeights / 4
+    const int smem = (HW * t->E + kProjThreads / 32 * HW) * (int)sizeof(float);
+    LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(once, ctx->device, project_norm_kernel, kMost));
+    constexpr int wpb = kProjThreads / 32;
+    LTCA_CUDA_OK(ctx, launch_dependent(project_norm_kernel, dim3((unsigned)((rows + wpb - 1) / wpb)), dim3(kProjThreads), smem, ctx->stream,
+                                       core, t->wo, t->bo, t->x, t->ln_gamma, t->ln_beta, t->out, (int)rows, HW, t->E, t->use_residual,
+                                       t->use_layer_norm, 1e-5f));
     return LTCA_OK;
 }
 
@@ -234,7 +319,7 @@ __global__ void __launch_bounds__(kPrepareThreads) prenorm_prepare_kernel(const 
         const int64_t row = (int64_t)block * (kPrepareThreads / 32) + (threadIdx.x >> 5);
         if (row >= a.rows) return;
         const bool vec = aligned16(a.x, a.gamma, a.beta, a.xo.f32, a.xo.bf16);
-        layer_norm_row<false>(a.x, a.x, a.gamma, a.beta, a.xo, row, a.E, false, a.use_ln != 0, a.eps, vec);
+        layer_norm_row<0>(a.x, a.x, a.gamma, a.beta, a.xo, row, a.E, false, a.use_ln != 0, a.eps, vec);
         return;
     }
     block -= a.row_blocks;
@@ -307,14 +392,18 @@ __device__ __forceinline__ void layer_norm_bwd_pieces(const float* __restrict__ 
     const RowPieces<kN4> p(E);
     constexpr int kMax = RowPieces<kN4>::kMax;
     const int lane = threadIdx.x & 31;
-    float4 xh[kMax], gv[kMax], gm[kMax], r[kMax];
+    constexpr bool kEarly = kN4 > 0;                   // gamma and the residual with the rows
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 xh[kMax], gv[kMax], gm[kEarly ? kMax : 1], r[kEarly ? kMax : 1];
 #pragma unroll
     for (int i = 0; i < kMax; ++i)
         if (p.has(i)) {
             xh[i] = ldg4(xr, lane + 32 * i);
             gv[i] = ldg4(gr, lane + 32 * i);
-            gm[i] = ldg4(gamma, lane + 32 * i);
-            r[i] = dx && res ? ldg4(res, lane + 32 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
+            if constexpr (kEarly) {
+                gm[i] = ldg4(gamma, lane + 32 * i);
+                r[i] = dx && res ? ldg4(res, lane + 32 * i) : zero;
+            }
         }
     float s0 = 0.f;
 #pragma unroll
@@ -335,7 +424,8 @@ __device__ __forceinline__ void layer_norm_bwd_pieces(const float* __restrict__ 
     for (int i = 0; i < kMax; ++i)
         if (p.has(i)) {
             xh[i].x *= inv_std; xh[i].y *= inv_std; xh[i].z *= inv_std; xh[i].w *= inv_std;
-            const float4 gg = make_float4(gv[i].x * gm[i].x, gv[i].y * gm[i].y, gv[i].z * gm[i].z, gv[i].w * gm[i].w);
+            const float4 m = kEarly ? gm[kEarly ? i : 0] : ldg4(gamma, lane + 32 * i);
+            const float4 gg = make_float4(gv[i].x * m.x, gv[i].y * m.y, gv[i].z * m.z, gv[i].w * m.w);
             a1 += (gg.x + gg.y) + (gg.z + gg.w);
             a2 = fmaf(gg.x, xh[i].x, a2); a2 = fmaf(gg.y, xh[i].y, a2);
             a2 = fmaf(gg.z, xh[i].z, a2); a2 = fmaf(gg.w, xh[i].w, a2);
@@ -349,17 +439,19 @@ __device__ __forceinline__ void layer_norm_bwd_pieces(const float* __restrict__ 
 #pragma unroll
     for (int i = 0; i < kMax; ++i)
         if (p.has(i)) {
-            r[i].x += inv_std * (gv[i].x - m1 - xh[i].x * m2);
-            r[i].y += inv_std * (gv[i].y - m1 - xh[i].y * m2);
-            r[i].z += inv_std * (gv[i].z - m1 - xh[i].z * m2);
-            r[i].w += inv_std * (gv[i].w - m1 - xh[i].w * m2);
-            reinterpret_cast<float4*>(dx)[lane + 32 * i] = r[i];
+            float4 d = kEarly ? r[kEarly ? i : 0] : res ? ldg4(res, lane + 32 * i) : zero;
+            d.x += inv_std * (gv[i].x - m1 - xh[i].x * m2);
+            d.y += inv_std * (gv[i].y - m1 - xh[i].y * m2);
+            d.z += inv_std * (gv[i].z - m1 - xh[i].z * m2);
+            d.w += inv_std * (gv[i].w - m1 - xh[i].w * m2);
+            reinterpret_cast<float4*>(dx)[lane + 32 * i] = d;
         }
 }
 
 // LayerNorm backward, one warp per row.  g = gradient at the LayerNorm output, x = its input.
 //   dx = inv_std * (g*gamma - mean(g*gamma) - xhat * mean(g*gamma*xhat))  (+ res[row] when res != null)
 // dx and prod are optional; prod receives g * xhat, whose column sums are dgamma.
+template <int kN4>
 __global__ void layer_norm_bwd_kernel(const float* __restrict__ g, const float* __restrict__ x,
                                       const float* __restrict__ gamma, const float* __restrict__ res,
                                       float* __restrict__ dx, float* __restrict__ prod, int64_t rows, int E,
@@ -373,10 +465,7 @@ __global__ void layer_norm_bwd_kernel(const float* __restrict__ g, const float* 
     if ((E & 127) == 0 && E <= 1024 && aligned16(g, x, gamma, res, dx) && (reinterpret_cast<uintptr_t>(prod) & 15) == 0) {
         const float* rr = res ? res + row * E : nullptr;
         float *dr = dx ? dx + row * E : nullptr, *pr = prod ? prod + row * E : nullptr;
-        if (E == 512) layer_norm_bwd_pieces<4>(gr, xr, gamma, rr, dr, pr, E, eps);
-        else if (E == 256) layer_norm_bwd_pieces<2>(gr, xr, gamma, rr, dr, pr, E, eps);
-        else if (E == 128) layer_norm_bwd_pieces<1>(gr, xr, gamma, rr, dr, pr, E, eps);
-        else layer_norm_bwd_pieces<0>(gr, xr, gamma, rr, dr, pr, E, eps);
+        layer_norm_bwd_pieces<kN4>(gr, xr, gamma, rr, dr, pr, E, eps);
         return;
     }
     float sum = 0.f;
@@ -1595,7 +1684,9 @@ static int prenorm_backward(ltca_ctx* ctx, const ltca_tsa_params* t, bool want_d
         // LayerNorm(x) is no longer needed: its buffer takes dxin * xhat, whose column sums are dgamma
         float* prod = (want_ln_params && t->dgamma) ? xin : nullptr;
         const int wpb = 8;
-        LTCA_CUDA_OK(ctx, launch_dependent(layer_norm_bwd_kernel, dim3((unsigned)((rows + wpb - 1) / wpb)), dim3(wpb * 32), 0, ctx->stream,
+        auto kern = t->E == 512 ? layer_norm_bwd_kernel<4> : t->E == 256 ? layer_norm_bwd_kernel<2>
+                  : t->E == 128 ? layer_norm_bwd_kernel<1> : layer_norm_bwd_kernel<0>;
+        LTCA_CUDA_OK(ctx, launch_dependent(kern, dim3((unsigned)((rows + wpb - 1) / wpb)), dim3(wpb * 32), 0, ctx->stream,
                                            (const float*)dxin, t->x, t->ln_gamma, (want_dx && t->use_residual) ? g : nullptr,
                                            want_dx ? t->dx : nullptr, prod, rows, t->E, 1e-5f));
         if (want_ln_params) {
@@ -1630,6 +1721,7 @@ static int tsa_forward(ltca_ctx* ctx, const ltca_tsa_params* t, const ltca_tsa_p
     w += pl.y;
     FwdBufs fb;
     if ((rc = forward_core(ctx, t, pl, w, &fb, pl.attn_fwd))) return rc;
+    if (!outer && projects_and_norms(t, pl.rows, pl.HW)) return project_norm(ctx, t, fb.ctx, pl.rows, pl.HW);
     const int rows = (int)pl.rows;
     const Gemm32Problem proj = {fb.ctx, t->wo, t->bo, y, rows, t->E, pl.HW, pl.HW, t->E, t->E};
     if ((rc = gemm_fp32(ctx, &proj, 1, 0, 0, false, true))) return rc;
@@ -1677,16 +1769,22 @@ static int tsa_backward(ltca_ctx* ctx, const ltca_tsa_params* t, bool want_dx, b
     // (src/ml/ml_liquid_net.cu:715-721)
     if ((rc = forward_core(ctx, t, pl, w, &fb, pl.attn_fwd))) return rc;
     const int rows = (int)pl.rows, E = t->E, HW = pl.HW;
-    // dctx = dy Wo^T
-    const Gemm32Problem back = {t->dy, t->wo, nullptr, dctx, rows, HW, E, E, E, HW};
-    if ((rc = gemm_fp32(ctx, &back, 1, 0, 1, false, false))) return rc;
     ltca_attn_params a;
     fill_attn(t, &a);
     a.q = fb.q; a.k = fb.k; a.v = fb.v; a.o = fb.ctx; a.lse = fb.lse;
     a.dout = dctx; a.dq = dq; a.dk = dk; a.dv = dv;
     a.workspace = pl.attn_bwd ? fb.rest : nullptr;
     a.workspace_bytes = pl.attn_bwd;
-    if ((rc = ltca_attn_bwd(ctx, &a))) return rc;
+    // dctx = dy Wo^T
+    const ltca_strides dys = x_strides(t, E);
+    const FromOutput from = {t->dy, t->wo, E, dys.batch, dys.seq};
+    if (attn_bwd_exact(&a) && attn_bwd_fp32_forms_dout(ctx, &a, from)) {
+        if ((rc = launch_attn_bwd_fp32(ctx, &a, &from))) return rc;
+    } else {
+        const Gemm32Problem back = {t->dy, t->wo, nullptr, dctx, rows, HW, E, E, E, HW};
+        if ((rc = gemm_fp32(ctx, &back, 1, 0, 1, false, false))) return rc;
+        if ((rc = ltca_attn_bwd(ctx, &a))) return rc;
+    }
     if (want_dw) {
         // bias gradients (FlashAttention form): column sums of the projection outputs' gradients
         jobs->add(dq, false, HW, HW, t->dbq);
