@@ -496,8 +496,9 @@ __device__ __forceinline__ void form_dout(float* dst, const CoreArgs& a, int b, 
 
 // pass 1: delta = rowsum(dO o O), left for pass 2, and dQ.  One CTA per TM query rows, KN keys per step.
 // kForm: dO is formed here (a kernel of its own, since form_dout takes registers: without it twice as many CTAs fit on an SM).
-template <typename T, int DP, int TM, int KN, int NT, int kMask, bool kForm>
-__global__ void __launch_bounds__(NT, NT == 128 ? 3 : 1) attn_bwd_dq_fp32_kernel(const CoreArgs a) {
+// kCtas: how many share an SM; four leave no registers for the rows' deltas.
+template <typename T, int DP, int TM, int KN, int NT, int kMask, bool kForm, int kCtas>
+__global__ void __launch_bounds__(NT, kCtas) attn_bwd_dq_fp32_kernel(const CoreArgs a) {
     grid_dependency_wait();
     constexpr int LD = DP + kPad, LP = KN + kPad, RS = NT / 16, RM = TM / RS, CN = KN / 16, NW = KN / 32;
     using Lt = AccLayout<DP, TM, NT>;
@@ -556,7 +557,7 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 3 : 1) attn_bwd_dq_fp32_kernel
         const int r = row0 + RS * i;
         const float l = q0 + r < a.Sq ? a.lse_in[stat0 + q0 + r] : kNegInf;
         lse[i] = l == kNegInf ? INFINITY : l;
-        dlt[i] = row_delta[r];
+        if constexpr (kCtas < 4) dlt[i] = row_delta[r];
     }
 #pragma unroll
     for (int i = 0; i < Lt::NR; ++i)
@@ -599,7 +600,7 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 3 : 1) attn_bwd_dq_fp32_kernel
                 bool zero = !(visible >> j & 1u);
                 if (a.use_clamp && v >= a.clamp) { v = a.clamp; zero = true; }     // the gradient of a clamped score
                 const float p = expf(v - lse[i]);
-                Ss[r * LP + tx + 16 * j] = zero ? 0.f : p * (dp[i][j] - dlt[i]) * a.scale;
+                Ss[r * LP + tx + 16 * j] = zero ? 0.f : p * (dp[i][j] - (kCtas < 4 ? dlt[i] : row_delta[r])) * a.scale;
             }
         }
         __syncthreads();
@@ -627,8 +628,8 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 3 : 1) attn_bwd_dq_fp32_kernel
 }
 
 // pass 2: dK and dV.  One CTA per TK keys, QN query rows per step; a thread accumulates NR neighbouring keys.
-template <typename T, int DP, int TK, int QN, int NT, int kMask>
-__global__ void __launch_bounds__(NT, TK < 64 ? 3 : DP <= 32 ? 3 : DP <= 64 ? 2 : 1) attn_bwd_dkv_fp32_kernel(const CoreArgs a) {
+template <typename T, int DP, int TK, int QN, int NT, int kMask, int kCtas>
+__global__ void __launch_bounds__(NT, kCtas) attn_bwd_dkv_fp32_kernel(const CoreArgs a) {
     grid_dependency_wait();
     constexpr int LD = DP + kPad, LP = TK + kPad, RS = NT / 16, RM = QN / RS, CN = TK / 16, NW = (TK + 31) / 32;
     using Lt = AccLayout<DP, TK, NT>;
@@ -805,24 +806,24 @@ int run_fwd(ltca_ctx* ctx, const CoreArgs& a) {
     return LTCA_OK;
 }
 
-template <typename T, int DP, int TM, int KN, int NT, int kMask, bool kForm = false>
+template <typename T, int DP, int TM, int KN, int NT, int kMask, bool kForm = false, int kCtas = NT == 128 ? 3 : 1>
 int run_dq(ltca_ctx* ctx, const CoreArgs& a) {
     static SmemOptIn once;
     constexpr size_t smem = ((size_t)(2 * TM + 2 * KN) * (DP + kPad) + TM * (KN + kPad) + TM) * sizeof(float);
-    int rc = set_smem(ctx, attn_bwd_dq_fp32_kernel<T, DP, TM, KN, NT, kMask, kForm>, smem, once);
+    int rc = set_smem(ctx, attn_bwd_dq_fp32_kernel<T, DP, TM, KN, NT, kMask, kForm, kCtas>, smem, once);
     if (rc) return rc;
     dim3 grid((a.Sq + TM - 1) / TM, a.H, a.B);
-    LTCA_CUDA_OK(ctx, launch_dependent(attn_bwd_dq_fp32_kernel<T, DP, TM, KN, NT, kMask, kForm>, grid, dim3(NT), smem, ctx->stream, a));
+    LTCA_CUDA_OK(ctx, launch_dependent(attn_bwd_dq_fp32_kernel<T, DP, TM, KN, NT, kMask, kForm, kCtas>, grid, dim3(NT), smem, ctx->stream, a));
     return LTCA_OK;
 }
-template <typename T, int DP, int TK, int QN, int NT, int kMask>
+template <typename T, int DP, int TK, int QN, int NT, int kMask, int kCtas = TK < 64 || DP <= 32 ? 3 : DP <= 64 ? 2 : 1>
 int run_dkv(ltca_ctx* ctx, const CoreArgs& a) {
     static SmemOptIn once;
     constexpr size_t smem = ((size_t)(2 * TK + 2 * QN) * (DP + kPad) + 2 * QN * (TK + kPad) + 2 * QN) * sizeof(float);
-    int rc = set_smem(ctx, attn_bwd_dkv_fp32_kernel<T, DP, TK, QN, NT, kMask>, smem, once);
+    int rc = set_smem(ctx, attn_bwd_dkv_fp32_kernel<T, DP, TK, QN, NT, kMask, kCtas>, smem, once);
     if (rc) return rc;
     dim3 grid((a.Sk + TK - 1) / TK, a.H, a.B);
-    LTCA_CUDA_OK(ctx, launch_dependent(attn_bwd_dkv_fp32_kernel<T, DP, TK, QN, NT, kMask>, grid, dim3(NT), smem, ctx->stream, a));
+    LTCA_CUDA_OK(ctx, launch_dependent(attn_bwd_dkv_fp32_kernel<T, DP, TK, QN, NT, kMask, kCtas>, grid, dim3(NT), smem, ctx->stream, a));
     return LTCA_OK;
 }
 
@@ -830,6 +831,7 @@ int run_dkv(ltca_ctx* ctx, const CoreArgs& a) {
 // done, they take whatever slots are left and sit unevenly on the SMs, 82 or 62 us instead of 57 for B16 H8 S100 D32.)
 // Tiles of 64 rows reuse what they load most; where they would leave SMs idle, tiles of 16 rows give four times the CTAs
 // and a quarter of the serial work.
+constexpr int kFourTilesCausalKeys = 256;
 template <typename T, int DP, int kMask>
 int run_small_dq(ltca_ctx* ctx, const CoreArgs& a) {
     if constexpr (sizeof(T) == 4 && DP <= 64) {
@@ -849,6 +851,18 @@ int run_rows(ltca_ctx* ctx, const CoreArgs& a, bool bwd) {
         if (!a.mask_bits) return (rc = run_small_dq<T, DP, kDense>(ctx, a)) ? rc : run_dkv<T, DP, 16, 32, 128, kDense>(ctx, a);
     }
     constexpr int kM = kMask ? kWords : kNoMask;
+    // Narrow heads: four 64-row tiles to an SM instead of three, in 128 registers a thread, where three would not take all tiles
+    // at once.  (B16 H8 S250 D32 175 us -> 152, B64 H8 S128 causal 151 -> 136, B32 H16 S60 D16 59 -> 44; with one wave of
+    // either, B4 H8 S400, 134 and 140.)  Not where the tiles of a pair last unevenly long (B8 H8 S512 causal 206 and 220), nor
+    // with a mask, whose words do not fit the registers either (B20 H16 S100 D24 120 and 132), except at the narrowest heads
+    // (B16 H8 S200 D16 126 and 108).
+    if constexpr (DP <= 16 || (DP <= 32 && kM == kNoMask)) {
+        const bool many = (int64_t)a.B * a.H * (((a.Sq < a.Sk ? a.Sq : a.Sk) + 63) / 64) > 3ll * ctx->sm_device;
+        if (many && (!a.causal || a.Sk <= kFourTilesCausalKeys)) {
+            if ((rc = run_dq<T, DP, 64, 64, NT, kM, false, 4>(ctx, a))) return rc;
+            return run_dkv<T, DP, 64, 64, NT, kM, 4>(ctx, a);
+        }
+    }
     if ((rc = fills(a.Sq) ? run_dq<T, DP, 64, 64, NT, kM>(ctx, a) : run_small_dq<T, DP, kM>(ctx, a))) return rc;
     return fills(a.Sk) ? run_dkv<T, DP, 64, 64, NT, kM>(ctx, a) : run_dkv<T, DP, 16, 32, 128, kM>(ctx, a);
 }
