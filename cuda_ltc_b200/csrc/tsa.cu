@@ -779,8 +779,10 @@ bool use_tensor(const ltca_tsa_params* t, bool backward) {
 // 4.8e-3 (dx), 5.8e-3 -> 5.2e-3 (dWq, dWk), 4.0e-3 -> 3.6e-3 (dWv, dWo), the like at every size.
 // (A choice by shape, mode and biases, which are the same in a forward and the backward that reuses it.)
 constexpr int kComposedRows = 4;
+// (Kept weights serve calls of any number of rows, so a weight cache has what either path needs from E and the mode alone.)
+bool composed_weights(const ltca_tsa_params* t) { return t->head_width == t->E && use_wide(t, false); }
 bool composed_shape(const ltca_tsa_params* t) {
-    return t->head_width == t->E && (int64_t)t->B * t->S >= (int64_t)kComposedRows * t->E && use_wide(t, false);
+    return composed_weights(t) && (int64_t)t->B * t->S >= (int64_t)kComposedRows * t->E;
 }
 bool use_composed(const ltca_tsa_params* t) { return composed_shape(t) && !t->bq && !t->bk && !t->bv; }
 
@@ -1267,8 +1269,8 @@ int tensor_forward_core(ltca_ctx* ctx, const ltca_tsa_params* t, const TPlan& pl
         tb->wv = c;  c += pl.w_in;
         tb->wo = c;  c += pl.w_out;
         if (pl.wide) { tb->wql = c; c += pl.w_in; tb->wkl = c; c += pl.w_in; }
-        // (a call without biases may find this block valid: composed_forward_core)
-        if (composed_shape(t)) { tb->wvl = c; c += pl.w_in; tb->wol = c; }
+        // (a call without biases, or with more rows, may find this block valid: composed_forward_core)
+        if (composed_weights(t)) { tb->wvl = c; c += pl.w_in; tb->wol = c; }
     }
     const bool convert_weights = !(cached && t->weight_cache_valid);
     if (saved && t->reuse_forward) return LTCA_OK;
@@ -1585,7 +1587,7 @@ int ltca_tsa_weight_cache_bytes(const ltca_tsa_params* t, size_t* bytes_out) {
     TPlan tp;
     int rc = make_tplan(t, &tp, true);
     if (rc) return rc;
-    *bytes_out = 3 * tp.w_in + tp.w_out + (tp.wide ? 2 * tp.w_in : 0) + (composed_shape(t) ? tp.w_in + tp.w_out : 0);
+    *bytes_out = 3 * tp.w_in + tp.w_out + (tp.wide ? 2 * tp.w_in : 0) + (composed_weights(t) ? tp.w_in + tp.w_out : 0);
     return LTCA_OK;
 }
 

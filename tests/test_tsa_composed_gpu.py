@@ -64,6 +64,11 @@ def test_module_on_products_of_the_weights(case):
         kept = ctx.tsa_bwd(*args, dev(dy), B, S, H, E, saved=saved, reuse_forward=True, weight_cache=(cache, valid), **kw)
         for a, b in zip(got, kept):
             assert torch.equal(a, b)
+    # kept weights also serve other numbers of rows
+    few = ctx.tsa_weight_cache(x_few := args[0][:S], *args[1:], 1, S, H, E, mode=mode, causal=causal)
+    fkw = dict(plain, keep_mask=None if m is None else dev(m[:1]))
+    ctx.tsa_fwd(x_few, *args[1:], 1, S, H, E, weight_cache=(few, False), **fkw)
+    assert torch.equal(y, ctx.tsa_fwd(*args, B, S, H, E, weight_cache=(few, True), **plain))
     # biases go through q, k and v, in blocks sized without them
     bias = [(0.1 * rng.standard_normal(H * E)).astype(np.float32) for _ in range(3)]
     bkw = dict(bq=dev(bias[0]), bk=dev(bias[1]), bv=dev(bias[2]))
