@@ -615,7 +615,7 @@ attn_fwd_tile_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
         mbar_init(bar_q_full, 1);
         for (int s = 0; s < L::kStages; ++s) { mbar_init(bar_kv_full(s), 1); mbar_init(bar_kv_empty(s), 1); }
         mbar_init(bar_s_full, 1);
-        mbar_init(bar_p_full, 4);
+        mbar_init(bar_p_full, L::kMathWarps);  // the first half of P, and O at its scale in all columns
         mbar_init(bar_p_full + 8u, 4);
         mbar_init(bar_staged, L::kMathWarps);
         for (int i = 0; i < 4; ++i) mbar_init(bar_pair0 + 8u * i, 2);
@@ -846,6 +846,16 @@ attn_fwd_tile_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
                         tmem_st16(tO + c0, o);
                     }
                     l_run *= factor;
+                }
+                if constexpr (kRS > 1) {
+                    // The product of P's first half adds to every column of O, so it waits for the warps that hold the
+                    // second half of P and of O's columns too.
+                    if (half == 1) {
+                        tmem_wait_st();
+                        tc_fence_before_sync();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(bar_p_full);
+                    }
                 }
                 const float m_safe = (m_run == neg_inf()) ? 0.f : m_run;
                 const f32x2 c2_2 = pair(c2, c2), mneg_2 = pair(-m_safe * c2, -m_safe * c2);

@@ -44,6 +44,33 @@ def test_forward_tiles(ctx, case, storage, D):
     assert max_abs(got[fin], lse_ref[fin]) < 2e-3
 
 
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("storage", ["bf16", "f32"])
+@pytest.mark.parametrize("causal", [False, True])
+def test_forward_tiles_that_rescale_at_every_step(ctx, causal, storage, D):
+    """Scores that grow along the keys, by more than the 2^8 a row's running maximum may lag behind in every step of 64 or
+    128 keys, so that each step rescales what it has summed up."""
+    B, H, S = 2, 24, 1000
+    dt = torch.bfloat16 if storage == "bf16" else torch.float32
+    q, k, v = (randn((B, H, S, D), 70 + i, 0.5) for i in range(3))
+    q[..., 0], k[..., 0] = 1.0, 0.125 * np.arange(S)           # natural units: 8 in 64 keys, log(2^8) = 5.5
+    q, k, v = (bf16_round(a) for a in (q, k, v))
+    tq, tk, tv = (torch.from_numpy(a).cuda().to(dt) for a in (q, k, v))
+    o, lse = ctx.attn_fwd(tq, tk, tv, scale=1.0, causal=causal, mode=_lib.MODE_BF16)
+    o_ref, lse_ref = oracle.attn_fwd(q, k, v, 1.0, causal)
+    # Exact bf16 inputs.  Results stored as bf16: probabilities and results rounded once each to 8 significant bits, which is
+    # 2^-8 of sum P |v| and of the result.  fp32: two terms of the probabilities, 2^-16.  Both: scores up to 200 in fp32, whose rounding reaches the exponent as
+    # 200 x 2^-23 at most, and the exponential's own error, together below 1e-4 of sum P |v|.
+    mag = oracle.attn_fwd(q, k, np.abs(v), 1.0, causal)[0]
+    bound = (2.0 ** -8 + 1e-4) * mag + 2.0 ** -8 * np.abs(o_ref) if storage == "bf16" else (2.0 ** -16 + 1e-4) * mag
+    err = np.abs(o.float().cpu().numpy() - o_ref)
+    assert (err <= bound + 1e-6).all(), (err.max(), (err / (bound + 1e-6)).max())
+    assert max_abs(lse.cpu().numpy(), lse_ref) < 1e-3
+    for _ in range(20):
+        again = ctx.attn_fwd(tq, tk, tv, scale=1.0, causal=causal, mode=_lib.MODE_BF16)
+        assert torch.equal(o, again[0]) and torch.equal(lse, again[1])
+
+
 LIMIT_CASES = [
     # B, H, Sq, Sk, causal, lengths, mask
     (1, 1, 1, 1, False, False, False),          # fewer tiles than one CTA has teams

@@ -89,3 +89,14 @@ def test_columns_that_two_warps_share_are_handed_over_with_fences():
     steps = body[body.index("*xslot(j & 1, half) = mt;"):]
     order = [steps.index(s) for s in ("tc_fence_before_sync()", "meet()", "tc_fence_after_sync()", "tmem_st16(tP")]
     assert order == sorted(order)
+
+
+def test_first_product_of_a_step_waits_for_every_warp_that_rescales():
+    """The forward tile's products add to all columns of O: the barrier in front of a step's first product counts every math
+    warp, and where a row's columns belong to two warps the second one arrives on it behind its rescale."""
+    body = _kernel_bodies(_sources()["attn_fwd_sm100.cu"])["attn_fwd_tile_sm100_kernel"]
+    assert "mbar_init(bar_p_full, L::kMathWarps)" in body
+    steps = body[body.index("tmem_st16(tO + c0, o);"):]
+    order = [steps.index(s) for s in ("if (half == 1) {", "tmem_wait_st();", "tc_fence_before_sync();", "mbar_arrive(bar_p_full);",
+                                      "tmem_st16(tP")]
+    assert order == sorted(order)
