@@ -28,9 +28,12 @@ struct WideArgs {
     // backward
     const void* dout = nullptr; ltca_strides dos{};
     const void* doutl = nullptr;                // optional low-order part of dO (same strides)
-    void *dq = nullptr, *dk = nullptr, *dv = nullptr;       // (dk may be null)
+    void *dq = nullptr, *dk = nullptr, *dv = nullptr;
     ltca_strides dqs{}, dks{}, dvs{};
     int grads_bf16 = 1;
+    // the forward's softmax leaves this value here (or null)
+    uint32_t* mark = nullptr;
+    uint32_t mark_value = 0;
     float* dP = nullptr;                        // scratch fp32 [B*H, Sq, Skp]
     void* dS = nullptr;                         // optional bf16 [B*H, Sq, Skp] for dS (null: dS overwrites P, and Plo its
     void* dSlo = nullptr;                       // second term); with it the probabilities survive the backward
@@ -46,7 +49,10 @@ bool wide_supported(int D, const ltca_strides& qs, const ltca_strides& ks, const
 int wide_attn_fwd(ltca_ctx* ctx, const WideArgs& w);
 // dQ, dK, dV from dO; expects `scores` and `P` as wide_attn_fwd left them for the same inputs.
 int wide_attn_bwd(ltca_ctx* ctx, const WideArgs& w);
-// its last step, dK = dS^T Q, alone
+// its steps one by one: dP and dV, dS, dQ, dK
+int wide_score_value_grads(ltca_ctx* ctx, const WideArgs& w);
+int wide_softmax_grad(ltca_ctx* ctx, const WideArgs& w);
+int wide_query_grad(ltca_ctx* ctx, const WideArgs& w);
 int wide_key_grad(ltca_ctx* ctx, const WideArgs& w);
 
 }  // namespace ltca

@@ -50,7 +50,12 @@ struct SoftmaxArgs {
     // backward
     const float* dP;             // [B*H, Sq, Skp]
     __nv_bfloat16 *dS, *dSlo;    // where dS goes (P / Plo themselves when the caller gave no separate buffer)
+    uint32_t* mark;              // forward: takes mark_value (or null)
+    uint32_t mark_value;
 };
+__device__ __forceinline__ void leave_mark(const SoftmaxArgs& a) {
+    if (a.mark && blockIdx.x == 0 && threadIdx.x == 0) *a.mark = a.mark_value;
+}
 
 // Query and batch of a row, in 32 bits where the rows allow it (65536 rows of 256 keys: 24.4 us with two 64-bit divisions, 22.8).
 struct RowPlace { int i, b; };
@@ -66,6 +71,7 @@ __device__ __forceinline__ RowPlace row_place(const SoftmaxArgs& a, int64_t row)
 // src/ml/flash_attention.cu:167), visibility (keep-mask value 0 hides, :161-164; causal; key lengths), softmax.
 __global__ void __launch_bounds__(256) wide_softmax_fwd_kernel(const SoftmaxArgs a) {
     grid_dependency_wait();
+    leave_mark(a);
     const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (row >= (int64_t)a.B * a.H * a.Sq) return;
@@ -153,6 +159,7 @@ __device__ __forceinline__ void unpack4_bf16(uint2 w, float* v) {
 template <int kChunks>
 __global__ void __launch_bounds__(256) wide_softmax_fwd_rows_kernel(const SoftmaxArgs a) {
     grid_dependency_wait();
+    leave_mark(a);
     const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (row >= (int64_t)a.B * a.H * a.Sq) return;
@@ -314,6 +321,8 @@ SoftmaxArgs softmax_args(const WideArgs& w) {
     a.Plo = reinterpret_cast<__nv_bfloat16*>(w.Plo);
     a.dS = reinterpret_cast<__nv_bfloat16*>(w.dS ? w.dS : w.P);
     a.dSlo = reinterpret_cast<__nv_bfloat16*>(w.dS ? w.dSlo : w.Plo);
+    a.mark = w.mark;
+    a.mark_value = w.mark_value;
     return a;
 }
 
@@ -417,16 +426,23 @@ int wide_attn_fwd(ltca_ctx* ctx, const WideArgs& w) {
 }
 
 int wide_attn_bwd(ltca_ctx* ctx, const WideArgs& w) {
+    int rc;
+    if ((rc = wide_score_value_grads(ctx, w)) || (rc = wide_softmax_grad(ctx, w)) || (rc = wide_query_grad(ctx, w))) return rc;
+    return wide_key_grad(ctx, w);
+}
+
+// every operand in two terms: three-term products (hi hi, lo hi, hi lo); else P and dS have one or two terms
+static bool wide_full(const WideArgs& w) { return w.Plo && w.vl && w.doutl && w.ql && w.kl; }
+static int wide_terms(const WideArgs& w) { return wide_full(w) ? 3 : (w.Plo ? 2 : 1); }
+
+int wide_score_value_grads(ltca_ctx* ctx, const WideArgs& w) {
     const int Skp = wide_padded_keys(w.Sk);
-    const int64_t mat = (int64_t)w.Sq * Skp;
-    const int64_t mat_b = (int64_t)w.H * mat;
-    const int terms = w.Plo ? 2 : 1;                 // P (then dS) as one or two bf16 terms
-    const bool full = w.Plo && w.vl && w.doutl && w.ql && w.kl;    // every operand in two terms: three-term products
+    const int64_t mat = (int64_t)w.Sq * Skp, mat_b = (int64_t)w.H * mat;
+    const bool full = wide_full(w);
     if ((w.vl || w.doutl) && !full)
         return fail(ctx, LTCA_ERR_INVALID, "low-order parts of V and dO come with those of Q, K and the probabilities");
     if (w.dS && w.Plo && !w.dSlo) return fail(ctx, LTCA_ERR_INVALID, "two-term probabilities need a two-term dS buffer");
     int rc;
-    // (three-term products: hi hi, lo hi, hi lo)
     {   // dP = dO V^T : both K-major
         Mat a[3] = {{w.dout, w.dos.seq, 0, w.dos.head, w.dos.batch}, {w.doutl, w.dos.seq, 0, w.dos.head, w.dos.batch},
                     {w.dout, w.dos.seq, 0, w.dos.head, w.dos.batch}};
@@ -434,14 +450,15 @@ int wide_attn_bwd(ltca_ctx* ctx, const WideArgs& w) {
                     {w.vl, w.vs.seq, 0, w.vs.head, w.vs.batch}};
         if ((rc = batched(ctx, w, w.Sq, w.Sk, w.D, a, b, full ? 3 : 1, w.dP, Skp, mat, mat_b, 0))) return rc;
     }
-    {   // dV = P^T dO : P stored [Sq, Sk] = [K, M], dO stored [Sq, D] = [K, N]
-        Mat a[3] = {{w.P, Skp, 1, mat, mat_b}, {w.Plo, Skp, 1, mat, mat_b}, {w.P, Skp, 1, mat, mat_b}};
-        Mat b[3] = {{w.dout, w.dos.seq, 1, w.dos.head, w.dos.batch}, {w.dout, w.dos.seq, 1, w.dos.head, w.dos.batch},
-                    {w.doutl, w.dos.seq, 1, w.dos.head, w.dos.batch}};
-        if ((rc = batched(ctx, w, w.Sk, w.D, w.Sq, a, b, full ? 3 : terms, w.dv, w.dvs.seq, w.dvs.head, w.dvs.batch,
-                          w.grads_bf16)))
-            return rc;
-    }
+    // dV = P^T dO : P stored [Sq, Sk] = [K, M], dO stored [Sq, D] = [K, N]
+    Mat a[3] = {{w.P, Skp, 1, mat, mat_b}, {w.Plo, Skp, 1, mat, mat_b}, {w.P, Skp, 1, mat, mat_b}};
+    Mat b[3] = {{w.dout, w.dos.seq, 1, w.dos.head, w.dos.batch}, {w.dout, w.dos.seq, 1, w.dos.head, w.dos.batch},
+                {w.doutl, w.dos.seq, 1, w.dos.head, w.dos.batch}};
+    return batched(ctx, w, w.Sk, w.D, w.Sq, a, b, wide_terms(w), w.dv, w.dvs.seq, w.dvs.head, w.dvs.batch, w.grads_bf16);
+}
+
+int wide_softmax_grad(ltca_ctx* ctx, const WideArgs& w) {
+    const int Skp = wide_padded_keys(w.Sk);
     const SoftmaxArgs sa = softmax_args(w);
     const int64_t rows = (int64_t)w.B * w.H * w.Sq;
     const unsigned sblocks = (unsigned)((rows + 7) / 8);
@@ -453,28 +470,29 @@ int wide_attn_bwd(ltca_ctx* ctx, const WideArgs& w) {
     else if (vec && Skp <= 1024) bwd_kernel = wide_softmax_bwd_rows_kernel<8>;
     LTCA_CUDA_OK(ctx, launch_dependent(bwd_kernel, dim3(sblocks), dim3(256), 0, ctx->stream, sa));
     LTCA_LAUNCH_OK(ctx, "wide_softmax_bwd_kernel");
-    {   // dQ = dS K : dS K-major, K stored [Sk, D] = [K, N]
-        Mat a[3] = {{sa.dS, Skp, 0, mat, mat_b}, {sa.dSlo, Skp, 0, mat, mat_b}, {sa.dS, Skp, 0, mat, mat_b}};
-        Mat b[3] = {{w.kh, w.ks.seq, 1, w.ks.head, w.ks.batch}, {w.kh, w.ks.seq, 1, w.ks.head, w.ks.batch},
-                    {w.kl, w.ks.seq, 1, w.ks.head, w.ks.batch}};
-        if ((rc = batched(ctx, w, w.Sq, w.D, w.Sk, a, b, full ? 3 : terms, w.dq, w.dqs.seq, w.dqs.head, w.dqs.batch,
-                          w.grads_bf16)))
-            return rc;
-    }
-    return w.dk ? wide_key_grad(ctx, w) : LTCA_OK;
+    return LTCA_OK;
+}
+
+int wide_query_grad(ltca_ctx* ctx, const WideArgs& w) {
+    const int Skp = wide_padded_keys(w.Sk);
+    const int64_t mat = (int64_t)w.Sq * Skp, mat_b = (int64_t)w.H * mat;
+    const SoftmaxArgs sa = softmax_args(w);
+    // dQ = dS K : dS K-major, K stored [Sk, D] = [K, N]
+    Mat a[3] = {{sa.dS, Skp, 0, mat, mat_b}, {sa.dSlo, Skp, 0, mat, mat_b}, {sa.dS, Skp, 0, mat, mat_b}};
+    Mat b[3] = {{w.kh, w.ks.seq, 1, w.ks.head, w.ks.batch}, {w.kh, w.ks.seq, 1, w.ks.head, w.ks.batch},
+                {w.kl, w.ks.seq, 1, w.ks.head, w.ks.batch}};
+    return batched(ctx, w, w.Sq, w.D, w.Sk, a, b, wide_terms(w), w.dq, w.dqs.seq, w.dqs.head, w.dqs.batch, w.grads_bf16);
 }
 
 int wide_key_grad(ltca_ctx* ctx, const WideArgs& w) {
     const int Skp = wide_padded_keys(w.Sk);
     const int64_t mat = (int64_t)w.Sq * Skp, mat_b = (int64_t)w.H * mat;
-    const bool full = w.Plo && w.vl && w.doutl && w.ql && w.kl;
     const SoftmaxArgs sa = softmax_args(w);
     // dS stored [Sq, Sk] = [K, M], Q stored [Sq, D] = [K, N]
     Mat a[3] = {{sa.dS, Skp, 1, mat, mat_b}, {sa.dSlo, Skp, 1, mat, mat_b}, {sa.dS, Skp, 1, mat, mat_b}};
     Mat b[3] = {{w.qh, w.qs.seq, 1, w.qs.head, w.qs.batch}, {w.qh, w.qs.seq, 1, w.qs.head, w.qs.batch},
                 {w.ql, w.qs.seq, 1, w.qs.head, w.qs.batch}};
-    return batched(ctx, w, w.Sk, w.D, w.Sq, a, b, full ? 3 : (w.Plo ? 2 : 1), w.dk, w.dks.seq, w.dks.head, w.dks.batch,
-                   w.grads_bf16);
+    return batched(ctx, w, w.Sk, w.D, w.Sq, a, b, wide_terms(w), w.dk, w.dks.seq, w.dks.head, w.dks.batch, w.grads_bf16);
 }
 
 }  // namespace ltca

@@ -94,6 +94,7 @@ struct GemmKArgs {
     const float* bias[kMaxGemmProblems];
     float* partial;                  // [problem][slice][M][N] when ksplit > 1
     uint32_t* status;
+    RunIf run_if;
 };
 
 // One tile of the work list of a CTA.
@@ -150,6 +151,7 @@ gemm_bf16_sm100_kernel(const __grid_constant__ typename std::conditional<kKind =
                        const __grid_constant__ GemmKArgs g) {
     const int sum_h = kKind == kHeads ? g.sum_h : 1;
     const bool add_to_c = kKind == kHeads && g.add_to_c;
+    if (skipped(g.run_if)) return;
     using L = GemmCfg<kBN, kPair>;
     static_assert(kKind != kGroup || !kPair, "groups run on single CTAs");
     constexpr int kStages = L::kStages, kStageBytes = L::kStageBytes;
@@ -523,7 +525,8 @@ namespace {
 // slices: 4.8 us with one value and one load at a time, 3.7 so), else one (512 x 512 from 16 slices: 7.6 us with four).
 template <int kVec>
 __global__ void __launch_bounds__(256) gemm_splitk_reduce_kernel(const float* __restrict__ partial, float* c0, float* c1, float* c2,
-                                                                 float* c3, int64_t mn, int ksplit) {
+                                                                 float* c3, int64_t mn, int ksplit, const RunIf run_if) {
+    if (skipped(run_if)) return;
     grid_dependency_wait();
     const int problem = blockIdx.y;
     float* c = problem == 0 ? c0 : (problem == 1 ? c1 : (problem == 2 ? c2 : c3));
@@ -686,6 +689,7 @@ int gemm_sm100(ltca_ctx* ctx, const GemmProblem& gp) {
     for (int i = 0; i < kMaxGemmProblems; ++i) { g.C[i] = gp.c[i < gp.n_problems ? i : 0]; g.bias[i] = i < gp.n_problems ? gp.bias[i] : nullptr; }
     g.partial = gp.partial;
     g.status = ctx->d_status;
+    g.run_if = ctx->run_if;
     g.batch_h = gp.batch_h; g.batch_b = gp.batch_b;
     g.sum_h = gp.sum_h;
     g.a_head = gp.a_shared ? 0 : 1; g.b_head = gp.b_shared ? 0 : 1;
@@ -743,7 +747,7 @@ int gemm_sm100(ltca_ctx* ctx, const GemmProblem& gp) {
         const dim3 rg((unsigned)((mn + per - 1) / per), gp.n_problems);
         auto kern = vec ? gemm_splitk_reduce_kernel<4> : gemm_splitk_reduce_kernel<1>;
         LTCA_CUDA_OK(ctx, launch_dependent(kern, rg, dim3(256), 0, ctx->stream,
-                                           (const float*)gp.partial, c[0], c[1], c[2], c[3], mn, g.ksplit));
+                                           (const float*)gp.partial, c[0], c[1], c[2], c[3], mn, g.ksplit, ctx->run_if));
         LTCA_LAUNCH_OK(ctx, "gemm_splitk_reduce_kernel");
     }
     return LTCA_OK;
@@ -787,6 +791,7 @@ int gemm_sm100_group(ltca_ctx* ctx, const GemmGroup& gg) {
     g.tma_store = 1;
     g.c_lo = gg.m[0].c_lo;
     g.status = ctx->d_status;
+    g.run_if = ctx->run_if;
     int rc;
     for (int i = 0; i < gg.n; ++i) {
         const GemmGroup::Member& m = gg.m[i];

@@ -15,6 +15,14 @@
 
 #include "../../include/ltc_attn.h"
 
+namespace ltca {
+// Kernels that run only where a word of device memory says so (null: always); see skipped (sm100_ptx.cuh).
+struct RunIf {
+    const uint32_t* word = nullptr;
+    uint32_t value = 0;
+};
+}  // namespace ltca
+
 struct ltca_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -32,6 +40,9 @@ struct ltca_ctx {
     // keys does not move a softmax) and what is left of it follows the order in which one kernel adds, so that order is held
     // fixed; and the backward recomputes what the forward computed.
     bool fwd_pairs = false;
+    // Set by a module backward that takes a kept forward of either form (tensor_backward, tsa.cu) while it launches the
+    // kernels of one of them.
+    ltca::RunIf run_if;
     char err[512] = {0};
     // optional per-kernel timing of the backward pass (ltca_ctx_enable_kernel_timing)
     bool time_kernels = false;

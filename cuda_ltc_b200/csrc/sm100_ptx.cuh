@@ -121,6 +121,17 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, co
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// The first thing a kernel with a RunIf asks: true where the word says that it is not to run.  It then lets the kernel after it
+// start and leaves, behind the kernel before it.  The word is read before the wait, which saves a skipped kernel its set-up:
+// whoever sets ctx->run_if launches something that is not a dependent launch first, so that the word's writer has completed
+// before any of these kernels can start.
+__device__ __forceinline__ bool skipped(const RunIf& r) {
+    if (!r.word || *r.word == r.value) return false;
+    grid_launch_dependents();
+    grid_dependency_wait();
+    return true;
+}
+
 // The 128-byte line at p (aligned) holds nothing that is read again: its content becomes undefined, and a line that is only
 // in L2 is dropped there instead of being written back.
 __device__ __forceinline__ void discard_line(const void* p) {

@@ -777,7 +777,6 @@ bool use_tensor(const ltca_tsa_params* t, bool backward) {
 // gained nothing (B4 S256 E512 H8).  Fewer bf16 roundings lie between the inputs and a result than on the other path, and the
 // products of weights have two terms, as q and k have there: errors against 64 bits 4.0e-3 -> 3.2e-3 (output), 5.7e-3 ->
 // 4.8e-3 (dx), 5.8e-3 -> 5.2e-3 (dWq, dWk), 4.0e-3 -> 3.6e-3 (dWv, dWo), the like at every size.
-// (A choice by shape, mode and biases, which are the same in a forward and the backward that reuses it.)
 constexpr int kComposedRows = 4;
 // (Kept weights serve calls of any number of rows, so a weight cache has what either path needs from E and the mode alone.)
 bool composed_weights(const ltca_tsa_params* t) { return t->head_width == t->E && use_wide(t, false); }
@@ -785,6 +784,11 @@ bool composed_shape(const ltca_tsa_params* t) {
     return composed_weights(t) && (int64_t)t->B * t->S >= (int64_t)kComposedRows * t->E;
 }
 bool use_composed(const ltca_tsa_params* t) { return composed_shape(t) && !t->bq && !t->bk && !t->bv; }
+// Where a call's biases decide between the two paths, a kept forward has either form.  Its block's first word says which: the
+// backward that reuses it need not be given the biases, for which it has no use.
+enum KeptForm : uint32_t { kKeptProjections = 1, kKeptComposed = 2 };
+size_t kept_word_bytes(const ltca_tsa_params* t) { return composed_shape(t) ? 256 : 0; }
+char* kept_block(const ltca_tsa_params* t) { return reinterpret_cast<char*>(t->saved) + kept_word_bytes(t); }
 
 struct TPlan {
     int64_t rows;
@@ -801,7 +805,7 @@ struct TPlan {
     int ks_m;
 };
 
-int make_tplan(const ltca_tsa_params* t, TPlan* pl, bool backward) {
+int make_tplan_as(const ltca_tsa_params* t, TPlan* pl, bool backward, bool composed) {
     pl->rows = (int64_t)t->B * t->S;
     pl->HW = t->H * t->head_width;
     pl->Ep = (t->E + 7) / 8 * 8;
@@ -812,7 +816,7 @@ int make_tplan(const ltca_tsa_params* t, TPlan* pl, bool backward) {
     pl->lse = align_up((size_t)t->B * t->H * t->S * sizeof(float), 256);
     pl->y = align_up((size_t)pl->rows * t->E * sizeof(float), 256);
     pl->wide = use_wide(t, backward);
-    pl->composed = pl->wide && use_composed(t);
+    pl->composed = pl->wide && composed;
     pl->me = align_up((size_t)t->E * t->H * t->E * 2, 256);
     pl->mat32 = pl->mat16 = 0;
     pl->attn_fwd = pl->attn_bwd = 0;
@@ -843,20 +847,17 @@ int make_tplan(const ltca_tsa_params* t, TPlan* pl, bool backward) {
     }
     return LTCA_OK;
 }
+int make_tplan(const ltca_tsa_params* t, TPlan* pl, bool backward) { return make_tplan_as(t, pl, backward, use_composed(t)); }
 
 // A size is asked for before the biases are known: the larger one of a plan with and one without them.
 template <typename Size>
 int planned_bytes(const ltca_tsa_params* t, bool backward, Size size, size_t* bytes_out) {
     TPlan pl;
-    int rc = make_tplan(t, &pl, backward);
+    int rc = make_tplan_as(t, &pl, backward, false);
     if (rc) return rc;
     *bytes_out = size(pl);
     if (!composed_shape(t)) return LTCA_OK;
-    ltca_tsa_params other = *t;
-    const float present = 0.f;                         // (only whether there is a bias is looked at)
-    other.bq = use_composed(t) ? &present : nullptr;
-    other.bk = other.bv = nullptr;
-    if ((rc = make_tplan(&other, &pl, backward))) return rc;
+    if ((rc = make_tplan_as(t, &pl, backward, true))) return rc;
     if (size(pl) > *bytes_out) *bytes_out = size(pl);
     return LTCA_OK;
 }
@@ -900,11 +901,19 @@ struct TBufs {
     float* lse;
     char* rest;
     // materialised-score path
-    void *xl, *wql, *wkl, *ql, *kl, *P, *dS;
-    float *scores, *dP;
+    void *xl, *wql, *wkl, *ql, *kl, *P;
+    float* scores;
     // ... on products of the weights
     void *wvl, *wol, *m, *ml, *n, *nl, *t, *tl, *z;
 };
+
+// What both forms of the module on the written-out-score path have alike comes first.
+char* place_scores(const TPlan& pl, char* w, TBufs* tb) {
+    tb->lse = reinterpret_cast<float*>(w);    w += pl.lse;
+    tb->scores = reinterpret_cast<float*>(w); w += pl.mat32;
+    tb->P = w;                                w += pl.mat16;
+    return w;
+}
 
 // The attention problem of the module for the materialised-score path (bf16 views of the projection outputs).
 void fill_wide(const ltca_tsa_params* t, const TBufs& tb, WideArgs* w) {
@@ -917,8 +926,12 @@ void fill_wide(const ltca_tsa_params* t, const TBufs& tb, WideArgs* w) {
     w->qs = w->ks = w->vs = w->os = a.q_strides;
     w->dos = w->dqs = w->dks = w->dvs = a.q_strides;
     w->o = tb.ctx; w->o_bf16 = 1; w->lse = tb.lse;
-    w->scores = tb.scores; w->P = tb.P; w->dP = tb.dP; w->dS = tb.dS;
+    w->scores = tb.scores; w->P = tb.P;
     w->grads_bf16 = 1;
+    if (t->saved && kept_word_bytes(t)) {
+        w->mark = reinterpret_cast<uint32_t*>(t->saved);
+        w->mark_value = kKeptProjections;
+    }
 }
 
 // The same on products of the weights: T and z in the places of q and v, x in that of k, for every head.
@@ -935,6 +948,7 @@ void fill_composed(const ltca_tsa_params* t, const TPlan& pl, const TBufs& tb, W
     w->kh = tb.xb; w->kl = tb.xl; w->ks = x_strides(t, pl.Ep);
     w->v = tb.z;
     w->o = nullptr;
+    w->mark_value = kKeptComposed;
 }
 
 // The attention scratch (TBufs::rest) of a call whose buffers start at w; not on the written-out-score path.
@@ -952,7 +966,7 @@ ltca_tsa_params laid_out(const ltca_tsa_params* t, int which) {
 // What a module call tells its kernels through the context, taken back when the call returns.
 struct CallHints {
     ltca_ctx* ctx;
-    ~CallHints() { ctx->mask_packed = nullptr; ctx->mask_words = nullptr; ctx->fwd_pairs = false; }
+    ~CallHints() { ctx->mask_packed = nullptr; ctx->mask_words = nullptr; ctx->fwd_pairs = false; ctx->run_if = RunIf(); }
 };
 // The packed form of the call's dense mask lies in the last bytes of the `bytes` of scratch that its attention kernels
 // share; `later`: the call's prepare launch writes it (prenorm_prepare), else it is written now.
@@ -975,7 +989,8 @@ int place_mask_words(ltca_ctx* ctx, const ltca_tsa_params* t, const TPlan& pl, c
 int composed_forward_core(ltca_ctx* ctx, const ltca_tsa_params* t, const TPlan& pl, char* w, TBufs* tb, const float* also_src,
                           void* also_dst, bool* also_done) {
     char* r = w;
-    if (t->saved) w = reinterpret_cast<char*>(t->saved);
+    if (t->saved) w = kept_block(t);
+    w = place_scores(pl, w, tb);
     tb->xb = w;  w += pl.xb;
     tb->wq = w;  w += pl.w_in;
     tb->wk = w;  w += pl.w_in;
@@ -987,9 +1002,6 @@ int composed_forward_core(ltca_ctx* ctx, const ltca_tsa_params* t, const TPlan& 
     tb->n = w;   w += pl.me;
     tb->t = w;   w += pl.act;
     tb->z = w;   w += pl.act;
-    tb->lse = reinterpret_cast<float*>(w);    w += pl.lse;
-    tb->scores = reinterpret_cast<float*>(w); w += pl.mat32;
-    tb->P = w;   w += pl.mat16;
     if (!t->saved) r = w;
     tb->xl = r;  r += pl.xb;
     tb->wvl = r; r += pl.w_in;
@@ -998,8 +1010,7 @@ int composed_forward_core(ltca_ctx* ctx, const ltca_tsa_params* t, const TPlan& 
     tb->nl = r;  r += pl.me;
     tb->tl = r;  r += pl.act;
     tb->rest = r;
-    tb->q = tb->k = tb->v = tb->ctx = tb->ql = tb->kl = tb->dS = nullptr;
-    tb->dP = nullptr;
+    tb->q = tb->k = tb->v = tb->ctx = tb->ql = tb->kl = nullptr;
     const bool cached = t->weight_cache != nullptr;
     if (cached) {                                      // laid out as on the other path
         char* c = reinterpret_cast<char*>(t->weight_cache);
@@ -1100,6 +1111,12 @@ int sum_over_heads(ltca_ctx* ctx, const ltca_tsa_params* t, const TPlan& pl, con
     return gemm_sm100(ctx, gp);
 }
 
+// What a backward of either form works on first: dy in bf16, four activations, and on the written-out-score path dP and dS (not in
+// P's place: the probabilities stay valid for the next backward from the same forward).
+struct BwdBufs { void *dyb, *dctx, *dq, *dk, *dv; float* dP; void* dS; };
+// A backward's two parts lie before and behind the step from dP to dS, which is the same in both forms.
+enum BwdPart { kUpToScores = 1, kFromScores = 2, kWhole = 3 };
+
 // A product for every head between two of [E, H E] / [rows, H E] / [HW, E] matrices: C_h[M, N] = sum over the terms.
 int per_head(ltca_ctx* ctx, const ltca_tsa_params* t, int M, int n_sum, const GemmOperand* a, int64_t a_hs, const GemmOperand* b,
              int64_t b_hs, void* c, int64_t ldc, int64_t c_hs, int out_bf16) {
@@ -1115,30 +1132,33 @@ int per_head(ltca_ctx* ctx, const ltca_tsa_params* t, int M, int n_sum, const Ge
     return gemm_sm100(ctx, gp);
 }
 
-// The backward behind composed_forward_core; w: the workspace behind what the forward laid out there.
-int composed_backward(ltca_ctx* ctx, const ltca_tsa_params* t, const TPlan& pl, const TBufs& tb, const void* dyb, char* w,
-                      bool want_dx, bool want_dw, ColSum* sums) {
+// tensor_backward on products of the weights; arguments as projected_backward has them.
+int composed_backward(ltca_ctx* ctx, const ltca_tsa_params* t, const TPlan& pl, const BwdBufs& g, char* w, BwdPart part, bool want_dx,
+                      bool want_dw) {
     const int rows = (int)pl.rows, E = t->E, HW = pl.HW, Ep = pl.Ep;
-    void* dt = w;     w += pl.act;
-    void* dz = w;     w += pl.act;
-    void* dq = w;     w += pl.act;
-    void* dv = w;     w += pl.act;
-    WideArgs wa;
-    fill_composed(t, pl, tb, &wa);
-    wa.dP = reinterpret_cast<float*>(w); w += pl.mat32;
-    wa.dS = w;        w += pl.mat16;
+    void *dyb = g.dyb, *dt = g.dctx, *dz = g.dk, *dq = g.dq, *dv = g.dv;
     float* dm32 = reinterpret_cast<float*>(w); w += 2 * pl.me;
     float* dn32 = reinterpret_cast<float*>(w); w += 2 * pl.me;
     void* dm = w;     w += pl.me;
     void* dml = w;    w += pl.me;
     void* dn = w;     w += pl.me;
     void* dnl = w;    w += pl.me;
-    float* partial = reinterpret_cast<float*>(w);
+    float* partial = reinterpret_cast<float*>(w); w += pl.partial;
+    TBufs tb;
     int rc;
+    bool dy_done = part != kWhole;
+    if ((rc = composed_forward_core(ctx, t, pl, w, &tb, dy_done ? nullptr : t->dy, dyb, &dy_done))) return rc;
+    if (!dy_done && (rc = convert_rows_bf16(ctx, t->dy, E, dyb, Ep, pl.rows, E))) return rc;
+    WideArgs wa;
+    fill_composed(t, pl, tb, &wa);
+    wa.dP = g.dP; wa.dS = g.dS;
     // dP = dy z^T, dz = P^T dy, dS, dT = dS x
     wa.dout = dyb; wa.dos = x_strides(t, Ep);
     wa.dq = dt; wa.dv = dz;
-    if ((rc = wide_attn_bwd(ctx, wa))) return rc;
+    if ((part & kUpToScores) && (rc = wide_score_value_grads(ctx, wa))) return rc;
+    if (part == kWhole && (rc = wide_softmax_grad(ctx, wa))) return rc;
+    if (!(part & kFromScores)) return LTCA_OK;
+    if ((rc = wide_query_grad(ctx, wa))) return rc;
     if (want_dx) {
         GemmProblem gp;                                // M and N are stored [E, H E] = [N, K]
         gp.M = rows; gp.N = E; gp.K = HW;
@@ -1199,9 +1219,9 @@ int composed_backward(ltca_ctx* ctx, const ltca_tsa_params* t, const TPlan& pl, 
                 if ((rc = per_head(ctx, t, E, m.terms, m.a, m.a_hs, m.b, m.b_hs, m.c, m.ldc, m.c_hs, 0))) return rc;
         }
     }
-    sums->add(t->dy, false, E, E, t->dbo);
     if (t->dbq || t->dbk || t->dbv) {
-        // Gradients of biases that the module does not have: column sums of dq = dT Wk, dv = dz Wo^T and dk = (dS^T x) Wq.
+        // Gradients of biases that the module does not have: column sums of dq = dT Wk, dv = dz Wo^T and dk = (dS^T x) Wq.  dk takes
+        // dz's place once dv is there, so that the three lie where projected_backward has them.
         const GemmOperand qa = {dt, HW, 0}, qb = {tb.wk, HW, 1}, va = {dz, HW, 0}, vb = {tb.wo, Ep, 0};
         if ((rc = per_head(ctx, t, rows, 1, &qa, E, &qb, E, dq, HW, E, 1))) return rc;
         if ((rc = per_head(ctx, t, rows, 1, &va, E, &vb, wo_h, dv, HW, E, 1))) return rc;
@@ -1211,9 +1231,6 @@ int composed_backward(ltca_ctx* ctx, const ltca_tsa_params* t, const TPlan& pl, 
         if ((rc = wide_key_grad(ctx, wk))) return rc;
         const GemmOperand ka = {dt, HW, 0}, kb = {tb.wq, HW, 1};
         if ((rc = per_head(ctx, t, rows, 1, &ka, E, &kb, E, dz, HW, E, 1))) return rc;
-        sums->add(dq, true, HW, HW, t->dbq);
-        sums->add(dz, true, HW, HW, t->dbk);
-        sums->add(dv, true, HW, HW, t->dbv);
     }
     return LTCA_OK;
 }
@@ -1224,12 +1241,13 @@ int composed_backward(ltca_ctx* ctx, const ltca_tsa_params* t, const TPlan& pl, 
 // or not at all).
 // `outer`: the FlashAttention form around this module; its LayerNorm (of outer->x) and its dropout (of outer->dy, into
 // outer_g as fp32 and into also_dst) take the place of those conversions, in the same launch as the weights'.
-int tensor_forward_core(ltca_ctx* ctx, const ltca_tsa_params* t, const TPlan& pl, char* w, TBufs* tb, int which,
+int tensor_forward_core(ltca_ctx* ctx, const ltca_tsa_params* t, const TPlan& pl, char* w, TBufs* tb,
                         const float* also_src = nullptr, void* also_dst = nullptr, bool* also_done = nullptr,
                         const ltca_tsa_params* outer = nullptr, float* outer_g = nullptr) {
     char* rest = w;
     const bool saved = t->saved != nullptr;
-    if (saved) w = reinterpret_cast<char*>(t->saved);
+    if (saved) w = kept_block(t);
+    w = place_scores(pl, w, tb);
     tb->xb = w;  w += pl.xb;
     tb->wq = w;  w += pl.w_in;
     tb->wk = w;  w += pl.w_in;
@@ -1239,26 +1257,14 @@ int tensor_forward_core(ltca_ctx* ctx, const ltca_tsa_params* t, const TPlan& pl
     tb->k = w;   w += pl.act;
     tb->v = w;   w += pl.act;
     tb->ctx = w; w += pl.act;
-    tb->lse = reinterpret_cast<float*>(w); w += pl.lse;
     if (pl.wide) {
         tb->xl = w;  w += pl.xb;
         tb->wql = w; w += pl.w_in;
         tb->wkl = w; w += pl.w_in;
         tb->ql = w;  w += pl.act;
         tb->kl = w;  w += pl.act;
-        tb->scores = reinterpret_cast<float*>(w); w += pl.mat32;
-        tb->P = w;   w += pl.mat16;
     }
-    char* r = saved ? rest : w;                        // what follows is never kept
-    if (pl.wide) {
-        tb->dP = nullptr; tb->dS = nullptr;
-        if (which != 0) {
-            // dS gets its own buffer: the probabilities stay valid for the next backward call from the same forward
-            tb->dP = reinterpret_cast<float*>(r); r += pl.mat32;
-            tb->dS = r; r += pl.mat16;
-        }
-    }
-    tb->rest = r;
+    tb->rest = saved ? rest : w;
     tb->wvl = tb->wol = nullptr;
     // the weights' copies live in the caller's cache when there is one
     const bool cached = t->weight_cache != nullptr;
@@ -1391,7 +1397,7 @@ int tensor_forward(ltca_ctx* ctx, const ltca_tsa_params* t, const ltca_tsa_param
         if ((rc = sum_over_heads(ctx, t, pl, tb.P, 0, tb.z, y, t->bo, false))) return rc;
         return outer ? prenorm_finish(ctx, outer, y) : residual_layer_norm(ctx, t, y, pl.rows);
     }
-    if ((rc = tensor_forward_core(ctx, t, pl, w, &tb, 0, nullptr, nullptr, nullptr, fused ? outer : nullptr))) return rc;
+    if ((rc = tensor_forward_core(ctx, t, pl, w, &tb, nullptr, nullptr, nullptr, fused ? outer : nullptr))) return rc;
     GemmProblem gp;
     gp.M = (int)pl.rows; gp.N = t->E; gp.K = pl.HW;
     gp.a[0] = GemmOperand{tb.ctx, pl.HW, 0};
@@ -1403,43 +1409,25 @@ int tensor_forward(ltca_ctx* ctx, const ltca_tsa_params* t, const ltca_tsa_param
     return outer ? prenorm_finish(ctx, outer, y) : residual_layer_norm(ctx, t, y, pl.rows);
 }
 
-// `sums` collects the bias gradients (column sums of buffers that stay as they are until the call ends).
-int tensor_backward(ltca_ctx* ctx, const ltca_tsa_params* t, bool want_dx, bool want_dw, ColSum* sums,
-                    const ltca_tsa_params* outer, float* outer_g) {
-    TPlan pl;
+// tensor_backward on q, k, v and ctx.  `w`: the workspace behind `g`.  In parts only on the written-out-score path, from a kept forward and
+// with dy's bf16 copy in its place.
+int projected_backward(ltca_ctx* ctx, const ltca_tsa_params* t, const ltca_tsa_params& layout, const TPlan& pl, const BwdBufs& g, char* w,
+                       BwdPart part, bool want_dx, bool want_dw, const ltca_tsa_params* outer, float* outer_g) {
+    void *dyb = g.dyb, *dctx = g.dctx, *dq = g.dq, *dk = g.dk, *dv = g.dv;
     int rc;
-    const ltca_tsa_params layout = laid_out(t, 1);
-    if ((rc = make_tplan(&layout, &pl, true))) return rc;
-    const size_t need = tensor_workspace(pl, 1);
-    if (!t->workspace || t->workspace_bytes < need)
-        return fail(ctx, LTCA_ERR_WORKSPACE, "backward needs %zu bytes of workspace", need);
-    char* w = reinterpret_cast<char*>(t->workspace);
-    void* dyb = w;   w += pl.xb;
-    if (pl.composed) {
-        TBufs tb;
-        bool dy_done = false;
-        if ((rc = composed_forward_core(ctx, t, pl, w, &tb, t->dy, dyb, &dy_done))) return rc;
-        if (!dy_done && (rc = convert_rows_bf16(ctx, t->dy, t->E, dyb, pl.Ep, pl.rows, t->E))) return rc;
-        return composed_backward(ctx, t, pl, tb, dyb, tb.rest, want_dx, want_dw, sums);
-    }
-    void* dctx = w;  w += pl.act;
-    void* dq = w;    w += pl.act;
-    void* dk = w;    w += pl.act;
-    void* dv = w;    w += pl.act;
     float* partial = reinterpret_cast<float*>(w); w += pl.partial;
     TBufs tb;
     // the forward is recomputed, as the reference's caller does before each backward
     // (src/ml/ml_liquid_net.cu:715-721)
     // the recomputed attention and its backward read the same mask: packed once, behind what either uses of the scratch
-    CallHints hints{ctx};
     ctx->fwd_pairs = t->bk != nullptr;
     const size_t most = pl.attn_fwd > pl.attn_bwd ? pl.attn_fwd : pl.attn_bwd;
     if ((rc = place_mask_words(ctx, &layout, pl, scratch_of(t, pl, w), most, outer && !(t->saved && t->reuse_forward)))) return rc;
-    bool dy_done = false;
-    if ((rc = tensor_forward_core(ctx, t, pl, w, &tb, 1, t->dy, dyb, &dy_done, outer, outer_g))) return rc;
+    bool dy_done = part != kWhole;
+    if ((rc = tensor_forward_core(ctx, t, pl, w, &tb, dy_done ? nullptr : t->dy, dyb, &dy_done, outer, outer_g))) return rc;
     const int rows = (int)pl.rows, E = t->E, HW = pl.HW, Ep = pl.Ep;
     if (!dy_done && (rc = convert_rows_bf16(ctx, t->dy, E, dyb, Ep, pl.rows, E))) return rc;
-    {   // dctx = dy Wo^T : Wo is stored [HW, E] = [N, K]
+    if (part & kUpToScores) {   // dctx = dy Wo^T : Wo is stored [HW, E] = [N, K]
         GemmProblem gp;
         gp.M = rows; gp.N = HW; gp.K = E;
         gp.a[0] = GemmOperand{dyb, Ep, 0};
@@ -1453,7 +1441,11 @@ int tensor_backward(ltca_ctx* ctx, const ltca_tsa_params* t, bool want_dx, bool 
         WideArgs wa;
         fill_wide(t, tb, &wa);
         wa.dout = dctx; wa.dq = dq; wa.dk = dk; wa.dv = dv;
-        if ((rc = wide_attn_bwd(ctx, wa))) return rc;
+        wa.dP = g.dP; wa.dS = g.dS;
+        if ((part & kUpToScores) && (rc = wide_score_value_grads(ctx, wa))) return rc;
+        if (part == kWhole && (rc = wide_softmax_grad(ctx, wa))) return rc;
+        if (!(part & kFromScores)) return LTCA_OK;
+        if ((rc = wide_query_grad(ctx, wa)) || (rc = wide_key_grad(ctx, wa))) return rc;
     } else {
         ltca_attn_params a;
         fill_attn_bf16(t, &a);
@@ -1464,13 +1456,6 @@ int tensor_backward(ltca_ctx* ctx, const ltca_tsa_params* t, bool want_dx, bool 
         if ((rc = ltca_attn_bwd(ctx, &a))) return rc;
     }
     const void* grads[3] = {dq, dk, dv};
-    if (want_dw) {
-        // bias gradients (FlashAttention form): column sums of the projection outputs' gradients
-        sums->add(dq, true, HW, HW, t->dbq);
-        sums->add(dk, true, HW, HW, t->dbk);
-        sums->add(dv, true, HW, HW, t->dbv);
-        sums->add(t->dy, false, E, E, t->dbo);
-    }
     if (want_dx) {
         // dx = dq Wq^T + dk Wk^T + dv Wv^T : each W is stored [E, HW] = [N, K]; one accumulator tile
         GemmProblem gp;
@@ -1517,6 +1502,72 @@ int tensor_backward(ltca_ctx* ctx, const ltca_tsa_params* t, bool want_dx, bool 
             gp.partial = partial;
             if ((rc = gemm_sm100(ctx, gp))) return rc;
         }
+    }
+    return LTCA_OK;
+}
+
+// `sums` collects the bias gradients (column sums of buffers that stay as they are until the call ends).
+int tensor_backward(ltca_ctx* ctx, const ltca_tsa_params* t, bool want_dx, bool want_dw, ColSum* sums,
+                    const ltca_tsa_params* outer, float* outer_g) {
+    TPlan pl[2];                                       // projections; products of the weights
+    int rc;
+    const ltca_tsa_params layout = laid_out(t, 1);
+    // A kept forward of either form: both backwards are launched, each to run where the block is its own.  (What the other one's
+    // eight or nine launches cost: backward of B32 S256 E512 H8 313 us and 299 without them, B16 S256 E256 H4 113 and 93; by itself
+    // the path through q, k, v and ctx takes 405 and 106.)
+    const bool either = t->saved && t->reuse_forward && composed_shape(t);
+    const bool composed = use_composed(t);
+    size_t need = 0;
+    for (int i = 0; i < 2; ++i) {
+        if (!either && i != (composed ? 1 : 0)) continue;
+        if ((rc = make_tplan_as(&layout, &pl[i], true, i == 1))) return rc;
+        const size_t n = tensor_workspace(pl[i], 1);
+        if (n > need) need = n;
+    }
+    if (!t->workspace || t->workspace_bytes < need)
+        return fail(ctx, LTCA_ERR_WORKSPACE, "backward needs %zu bytes of workspace", need);
+    const TPlan& any = pl[composed ? 1 : 0];
+    char* w = reinterpret_cast<char*>(t->workspace);
+    BwdBufs g;
+    g.dyb = w;  w += any.xb;
+    g.dctx = w; w += any.act;
+    g.dq = w;   w += any.act;
+    g.dk = w;   w += any.act;
+    g.dv = w;   w += any.act;
+    g.dP = reinterpret_cast<float*>(w); w += any.mat32;
+    g.dS = w;   w += any.mat16;
+    CallHints hints{ctx};
+    if (either) {
+        // (an ordinary launch, as the kernels that look at the word need before them: skipped, sm100_ptx.cuh)
+        if ((rc = convert_rows_bf16(ctx, t->dy, t->E, g.dyb, any.Ep, any.rows, t->E))) return rc;
+        for (BwdPart part : {kUpToScores, kFromScores}) {
+            if (part == kFromScores) {
+                ctx->run_if = RunIf();
+                TBufs tb{};
+                WideArgs wa;
+                place_scores(any, kept_block(t), &tb);
+                fill_wide(t, tb, &wa);
+                wa.dP = g.dP; wa.dS = g.dS;
+                if ((rc = wide_softmax_grad(ctx, wa))) return rc;
+            }
+            ctx->run_if.word = reinterpret_cast<const uint32_t*>(t->saved);
+            ctx->run_if.value = kKeptProjections;
+            if ((rc = projected_backward(ctx, t, layout, pl[0], g, w, part, want_dx, want_dw, outer, outer_g))) return rc;
+            ctx->run_if.value = kKeptComposed;
+            if ((rc = composed_backward(ctx, t, pl[1], g, w, part, want_dx, want_dw))) return rc;
+        }
+        ctx->run_if = RunIf();
+    } else if (composed) {
+        if ((rc = composed_backward(ctx, t, pl[1], g, w, kWhole, want_dx, want_dw))) return rc;
+    } else {
+        if ((rc = projected_backward(ctx, t, layout, pl[0], g, w, kWhole, want_dx, want_dw, outer, outer_g))) return rc;
+    }
+    if (want_dw) {
+        // bias gradients (FlashAttention form): column sums of the projection outputs' gradients
+        sums->add(g.dq, true, any.HW, any.HW, t->dbq);
+        sums->add(g.dk, true, any.HW, any.HW, t->dbk);
+        sums->add(g.dv, true, any.HW, any.HW, t->dbv);
+        sums->add(t->dy, false, t->E, t->E, t->dbo);
     }
     return LTCA_OK;
 }
@@ -1570,7 +1621,7 @@ int ltca_tsa_saved_bytes(const ltca_tsa_params* t, size_t* bytes_out) {
     ltca_tsa_params probe = *t;
     probe.saved = nullptr;
     if (use_tensor(&probe, true)) {
-        return planned_bytes(&probe, true, [](const TPlan& tp) { return tensor_saved_bytes(tp); }, bytes_out);
+        return planned_bytes(&probe, true, [&](const TPlan& tp) { return kept_word_bytes(&probe) + tensor_saved_bytes(tp); }, bytes_out);
     }
     Plan pl;
     int rc = make_plan(&probe, &pl);

@@ -272,8 +272,9 @@ typedef struct {
      * forward() to backward(), so its caller runs forward() again before every backward()
      * (src/ml/ml_liquid_net.cu:715-721) and the backward entry points here recompute it once more by default.
      * A caller that gives the SAME `saved` block (ltca_tsa_saved_bytes, 256-byte aligned) to ltca_tsa_fwd and
-     * then, with x, the weights and biases, the shape and the mode unchanged, to a backward call with
-     * reuse_forward = 1 skips that recomputation.  Not available with pre_norm.  With `saved` set the forward takes the pipeline
+     * then, with x, the weights, the shape and the mode unchanged, to a backward call with reuse_forward = 1 skips
+     * that recomputation.  (The block says itself what it holds: it may be copied, and the backward needs no
+     * biases.)  Not available with pre_norm.  With `saved` set the forward takes the pipeline
      * the backward will take. */
     void*   saved;
     size_t  saved_bytes;

@@ -107,3 +107,72 @@ def test_bias_gradients_without_biases():
     assert got["dbk"].abs().max() < 0.05 * ref["dbq"].abs().max()
     torch.cuda.synchronize()
     assert ctx.device_status() == 0
+
+
+def _bias_gradients(ctx, p, dy, saved, bias, HW, E):
+    """dbq, dbk, dbv, dbo and dwq of a backward that reuses `saved`, `bias` (or None) given to the call."""
+    import ctypes as C
+    import torch
+    out = {n: torch.full((HW if n != "dbo" else E,), float("nan"), device="cuda") for n in ("dbq", "dbk", "dbv", "dbo")}
+    dw = {n: torch.empty(HW * E, device="cuda") for n in ("dwq", "dwk", "dwv", "dwo")}
+    for n, t in (*out.items(), *dw.items()):
+        setattr(p, n, t.data_ptr())
+    for n in ("bq", "bk", "bv"):
+        setattr(p, n, bias[n].data_ptr() if bias else None)
+    p.dy, p.saved, p.saved_bytes, p.reuse_forward = dy.data_ptr(), saved.data_ptr(), saved.numel(), 1
+    need = C.c_size_t(0)
+    ctx.check(ctx.lib.ltca_tsa_workspace_bytes(C.byref(p), 2, C.byref(need)))
+    ws = torch.empty(need.value, dtype=torch.uint8, device="cuda")
+    p.workspace, p.workspace_bytes = ws.data_ptr(), need.value
+    ctx.check(ctx.lib.ltca_tsa_bwd_weights(ctx.handle, C.byref(p)))
+    torch.cuda.synchronize()
+    return [*out.values(), dw["dwq"]]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("case", [(4, 136, 136, 2, False, True), (8, 140, 200, 1, True, False), (4, 135, 136, 2, False, True)])
+def test_kept_forward_is_read_in_the_form_it_was_written(case):
+    """The backward that reuses a kept forward needs no biases: whether it is given them or not, it takes the block as the
+    forward wrote it, by another context and from a copy of the block too."""
+    import torch
+    import cuda_ltc_b200 as ltc
+    from cuda_ltc_b200 import _lib
+    B, S, E, H, causal, time_major = case
+    ctx, other = ltc.Context(0), ltc.Context(0)
+    g = torch.Generator(device="cuda").manual_seed(3)
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda")
+    lim = (3.0 / E) ** 0.5
+    x, dy = 0.5 * rnd(B * S, E), rnd(B * S, E)
+    w = [lim * 0.5 * rnd(E, H * E) for _ in range(3)] + [lim * 0.5 * rnd(H * E, E)]
+    biases = {n: 0.3 * rnd(H * E) for n in ("bq", "bk", "bv")}
+    kw = dict(causal=causal, time_major=time_major)
+    plain = dict(use_residual=False, use_layer_norm=False, **kw)
+    saved = ctx.tsa_saved_buffer(x, *w, B, S, H, E, causal=causal)
+    want = {}
+    for name, b in (("biased", biases), ("unbiased", {})):
+        want[name] = ctx.tsa_bwd(x, *w, dy, B, S, H, E, **kw, **b)                # recomputes the forward
+    assert rel_l2(want["biased"][1].cpu().numpy(), want["unbiased"][1].cpu().numpy()) > 0.05
+    for name, b in (("biased", biases), ("unbiased", {}), ("biased", biases)):
+        ctx.tsa_fwd(x, *w, B, S, H, E, saved=saved, **plain, **b)
+        torch.cuda.synchronize()
+        for c, block in ((ctx, saved), (other, saved), (ctx, saved.clone())):
+            for given in ({}, biases):
+                got = c.tsa_bwd(x, *w, dy, B, S, H, E, saved=block, reuse_forward=True, **kw, **given)
+                torch.cuda.synchronize()
+                for a, r in zip(got, want[name]):
+                    assert torch.equal(a, r), (name, bool(given))
+        p = ctx._tsa_sizes(x, *w, B, S, H, E, _lib.MODE_AUTO, causal)
+        p.time_major = int(time_major)
+        p.x, p.wq, p.wk, p.wv, p.wo = (t.data_ptr() for t in (x, *w))
+        sums = [_bias_gradients(ctx, p, dy, saved, given, H * E, E) for given in (None, biases)]
+        for a, r in zip(*sums):
+            assert torch.isfinite(a).all() and torch.equal(a, r), name
+        assert rel_l2(sums[0][3].cpu().numpy(), dy.sum(0, dtype=torch.float64).cpu().numpy()) < 1e-5
+        assert torch.equal(sums[0][4].view(E, H * E), want[name][1])
+    # a backward that recomputes into the block leaves it in its own call's form
+    got = ctx.tsa_bwd(x, *w, dy, B, S, H, E, saved=saved, **kw)
+    again = ctx.tsa_bwd(x, *w, dy, B, S, H, E, saved=saved, reuse_forward=True, **kw, **biases)
+    for a, b, r in zip(got, again, want["unbiased"]):
+        assert torch.equal(a, r) and torch.equal(b, r)
+    torch.cuda.synchronize()
+    assert ctx.device_status() == 0 and other.device_status() == 0
