@@ -778,8 +778,10 @@ bool use_tensor(const ltca_tsa_params* t, bool backward) {
 // products of weights have two terms, as q and k have there: errors against 64 bits 4.0e-3 -> 3.2e-3 (output), 5.7e-3 ->
 // 4.8e-3 (dx), 5.8e-3 -> 5.2e-3 (dWq, dWk), 4.0e-3 -> 3.6e-3 (dWv, dWo), the like at every size.
 constexpr int kComposedRows = 4;
-// (Kept weights serve calls of any number of rows, so a weight cache has what either path needs from E and the mode alone.)
-bool composed_weights(const ltca_tsa_params* t) { return t->head_width == t->E && use_wide(t, false); }
+// Kept weights serve calls of any number of rows, so a weight cache has what either path needs from E and the mode alone.  Heads of up
+// to 128, which come here on explicit request, keep the block of their q, k, v and ctx (B16 S256 E128 H2 step 112 us, on products
+// of the weights 102: the block would have to grow for it).
+bool composed_weights(const ltca_tsa_params* t) { return t->head_width == t->E && t->head_width > 128 && use_wide(t, false); }
 bool composed_shape(const ltca_tsa_params* t) {
     return composed_weights(t) && (int64_t)t->B * t->S >= (int64_t)kComposedRows * t->E;
 }

@@ -280,14 +280,14 @@ typedef struct {
     size_t  saved_bytes;
     int32_t reuse_forward;
     /* Optional: keep the reduced-precision copies of the four weight matrices across calls.  The tensor-pipe
-     * pipelines round wq, wk, wv, wo to bf16 (the materialised-score path also splits wq and wk into two terms)
-     * at the start of every call; the reference's module never changes its projection weights after
+     * pipelines round wq, wk, wv, wo to bf16 (the materialised-score path also splits wq and wk into two terms,
+     * and all four where heads are as wide as the model and wider than 128) at the start of every call; the reference's module never changes its projection weights after
      * construction or loadWeights (getParameters exposes the LayerNorm pair only,
      * src/ml/cudnn_time_self_attention.cu:436-450), so a caller can keep the copies.  With weight_cache set
      * (ltca_tsa_weight_cache_bytes, 256-byte aligned) a call with weight_cache_valid = 0 writes the copies there
      * and uses them; a call with weight_cache_valid = 1 uses them as they are and does not read wq..wo for the
-     * projections.  The caller clears the flag whenever the weights, the shape, the head width or the mode
-     * change.  Ignored by the exact pipeline. */
+     * projections.  The caller clears the flag whenever the weights, E, H, the head width or the mode
+     * change; calls of any B and S, with and without biases, share one block.  Ignored by the exact pipeline. */
     void*   weight_cache;
     size_t  weight_cache_bytes;
     int32_t weight_cache_valid;
