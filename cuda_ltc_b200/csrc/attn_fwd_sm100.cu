@@ -540,7 +540,9 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
 //     thread so holds 128 scores in its 216 registers and two warps share a scheduler; two threads per row, 64 scores each,
 //     had four of them but met once a step to agree on the row's maximum (B8 H16 S4096 causal 568 us, one per row 525).
 //     fp32 results at head_dim 128 have two threads per row (warps 0-7), which share the work of P's second term, and the
-//     halves of P below are one thread's each (B8 H16 S2048 causal 325 -> 319 us);
+//     halves of P below are one thread's each (B8 H16 S2048 causal 325 -> 319 us).  Not with a mask, whose words no longer fit
+//     their 104 registers: what is spilled goes out to L2, since the tiles leave an SM next to no L1 (masked B64 H8 S200 126 us
+//     with two threads per row, 97 with one; B4 H16 S1500 298 and 247);
 //   - P overwrites the first half of S, its second bf16 term (kSplitP: results stored as fp32) the other half.  It is handed
 //     to the contraction in two halves of the keys, so that the first products run under the second half's exponentials
 //     (B8 H16 S4096 D64, not causal: one hand-over 721 us, two 698);
@@ -558,10 +560,10 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
 // where the plain form takes 396 there (four tiles that start together stay in step); on 132 SMs 516 us, B8 H16 S1024
 // causal 56, B64 H8 S512 causal 61.
 // ---------------------------------------------------------------------------------------------
-template <int D, bool kSplitP>
+template <int D, bool kSplitP, bool kMask>
 struct TileCfg {
     static constexpr int kBN = D;                                  // keys per step
-    static constexpr int kRowSplit = D == 128 && kSplitP ? 2 : 1;  // threads per row
+    static constexpr int kRowSplit = D == 128 && kSplitP && !kMask ? 2 : 1;    // threads per row
     static constexpr int kCols = kBN / kRowSplit;                  // score columns of a thread
     static constexpr int kMathWarps = 4 * kRowSplit;
     static constexpr int kThreads = 32 * (kMathWarps + 4);
@@ -587,11 +589,11 @@ struct TileCfg {
 };
 
 template <int D, bool kSplitP, bool kMask, int kTeams>
-__global__ void __launch_bounds__(TileCfg<D, kSplitP>::kThreads * kTeams, kTeams > 1 ? 1 : TileCfg<D, kSplitP>::kCtas)
+__global__ void __launch_bounds__(TileCfg<D, kSplitP, kMask>::kThreads * kTeams, kTeams > 1 ? 1 : TileCfg<D, kSplitP, kMask>::kCtas)
 attn_fwd_tile_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                            const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_o, const FwdArgs a,
                            const ItemGrid items) {
-    using L = TileCfg<D, kSplitP>;
+    using L = TileCfg<D, kSplitP, kMask>;
     // (the teams share the registers and the tensor memory that as many CTAs of the plain form have on an SM)
     static_assert(kTeams == 1 || kTeams == L::kCtas, "one CTA or an SM's worth of them");
     constexpr int kBN = L::kBN, kRS = L::kRowSplit, kC = L::kCols, kMmaWarp = L::kMathWarps, kTmaWarp = L::kMathWarps + 1;
@@ -975,10 +977,10 @@ attn_fwd_tile_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
     }
 }
 
-template <int D, bool kSplitP>
+template <int D, bool kSplitP, bool kMask>
 int launch_fwd_tile(ltca_ctx* ctx, const ltca_attn_params* p, const void* q, const void* k, const void* v, const ltca_strides& qs,
                     const ltca_strides& ks, const ltca_strides& vs, const FwdArgs& a) {
-    using L = TileCfg<D, kSplitP>;
+    using L = TileCfg<D, kSplitP, kMask>;
     CUtensorMap tq, tk, tv, to;
     int rc;
     if ((rc = make_tmap_bhsd(ctx, &tq, q, 2, p->B, p->H, p->Sq, D, qs, 64, kBlockM))) return rc;
@@ -998,17 +1000,17 @@ int launch_fwd_tile(ltca_ctx* ctx, const ltca_attn_params* p, const void* q, con
         if (ctx->sm_count < ctx->sm_device && n <= 0x7fffffff - 2ll * L::kCtas * ctx->sm_device) {
             items.n_items = (int)n;
             items.counters = ctx->d_sched + 6;        // ints 6,7: the forward's
-            auto kern = p->keep_mask ? attn_fwd_tile_sm100_kernel<D, kSplitP, true, L::kCtas> : attn_fwd_tile_sm100_kernel<D, kSplitP, false, L::kCtas>;
-            static SmemOptIn opt_in[2];
-            LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(opt_in[p->keep_mask ? 1 : 0], ctx->device, kern, L::kTeamsDynBytes));
+            auto kern = attn_fwd_tile_sm100_kernel<D, kSplitP, kMask, L::kCtas>;
+            static SmemOptIn opt_in;
+            LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(opt_in, ctx->device, kern, L::kTeamsDynBytes));
             LTCA_CUDA_OK(ctx, launch_dependent_if(small_attention_call(p), kern, dim3((unsigned)(ctas < ctx->sm_count ? ctas : ctx->sm_count)),
                                                   dim3(L::kThreads * L::kCtas), L::kTeamsDynBytes, ctx->stream, tq, tk, tv, to, a, items));
             return LTCA_OK;
         }
     }
-    auto kern = p->keep_mask ? attn_fwd_tile_sm100_kernel<D, kSplitP, true, 1> : attn_fwd_tile_sm100_kernel<D, kSplitP, false, 1>;
-    static SmemOptIn opt_in[2];
-    LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(opt_in[p->keep_mask ? 1 : 0], ctx->device, kern, L::kDynBytes));
+    auto kern = attn_fwd_tile_sm100_kernel<D, kSplitP, kMask, 1>;
+    static SmemOptIn opt_in;
+    LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(opt_in, ctx->device, kern, L::kDynBytes));
     dim3 grid((p->Sq + kBlockM - 1) / kBlockM, p->H, p->B);
     LTCA_CUDA_OK(ctx, launch_dependent_if(small_attention_call(p), kern, grid, dim3(L::kThreads), L::kDynBytes, ctx->stream, tq, tk, tv, to, a, items));
     return LTCA_OK;
@@ -1044,7 +1046,9 @@ int launch_fwd(ltca_ctx* ctx, const ltca_attn_params* p, const void* mask_words,
     // Module calls with a key bias (ctx->fwd_pairs) keep it for short queries too.
     const bool few = ctas2 <= sms && p->Sk > 512;
     const bool ordered = ctx->fwd_pairs && (ctas2 <= sms || p->Sq <= 2 * kBlockM);
-    if (D != 64 || !(few || ordered)) return launch_fwd_tile<D, kSplitP>(ctx, p, q, k, v, qs, ks, vs, a);
+    if (D != 64 || !(few || ordered))
+        return p->keep_mask ? launch_fwd_tile<D, kSplitP, true>(ctx, p, q, k, v, qs, ks, vs, a)
+                            : launch_fwd_tile<D, kSplitP, false>(ctx, p, q, k, v, qs, ks, vs, a);
 
     if constexpr (D == 64) {
         using L = FwdCfg<kSplitP>;

@@ -8,7 +8,7 @@ import torch
 
 import oracle
 from cuda_ltc_b200 import _lib
-from util import bf16_round, max_abs, randn
+from util import bf16_round, keep_mask, max_abs, randn
 
 pytestmark = pytest.mark.gpu
 
@@ -69,6 +69,36 @@ def test_forward_tiles_that_rescale_at_every_step(ctx, causal, storage, D):
     for _ in range(20):
         again = ctx.attn_fwd(tq, tk, tv, scale=1.0, causal=causal, mode=_lib.MODE_BF16)
         assert torch.equal(o, again[0]) and torch.equal(lse, again[1])
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("storage", ["bf16", "f32"])
+@pytest.mark.parametrize("case", [(1, 1, 1, 1, False, False), (2, 3, 129, 65, False, False), (2, 2, 128, 256, True, False),
+                                  (2, 2, 257, 130, True, True), (3, 67, 200, 200, False, False), (2, 3, 300, 1000, False, False)])
+def test_forward_tiles_with_a_mask(ctx, case, storage, D):
+    """A dense mask with a hidden row, short lengths and, from 1000 keys on, scores that grow by more than 2^8 in every step, so
+    that each step rescales what it has summed up."""
+    B, H, Sq, Sk, causal, use_len = case
+    dt = torch.bfloat16 if storage == "bf16" else torch.float32
+    q, k, v = (randn((B, H, n, D), 80 + i, 0.5) for i, n in enumerate((Sq, Sk, Sk)))
+    if Sk >= 1000:
+        q[..., 0], k[..., 0] = 1.0, 0.125 * np.arange(Sk)
+    q, k, v = (bf16_round(a) for a in (q, k, v))
+    m = keep_mask(B, Sq, Sk, 7)
+    L = np.array([(Sk // 2 + 1, Sk)[i % 2] for i in range(B)], dtype=np.int32) if use_len else None
+    dev = lambda a: None if a is None else torch.from_numpy(a).cuda()
+    tq, tk, tv = (dev(a).to(dt) for a in (q, k, v))
+    o, lse = ctx.attn_fwd(tq, tk, tv, scale=0.5, causal=causal, keep_mask=dev(m), kv_len=dev(L), mode=_lib.MODE_BF16)
+    o_ref, lse_ref = oracle.attn_fwd(q, k, v, 0.5, causal, m, L)
+    # as in the test above: exact bf16 inputs, probabilities in one term or two, scores up to 100
+    mag = oracle.attn_fwd(q, k, np.abs(v), 0.5, causal, m, L)[0]
+    bound = (2.0 ** -8 + 1e-4) * mag + 2.0 ** -8 * np.abs(o_ref) if storage == "bf16" else (2.0 ** -16 + 1e-4) * mag
+    err = np.abs(o.float().cpu().numpy() - o_ref)
+    assert (err <= bound + 1e-6).all(), (err.max(), (err / (bound + 1e-6)).max())
+    fin, got = np.isfinite(lse_ref), lse.cpu().numpy()
+    assert not fin[0, :, 0].any() and (np.isfinite(got) == fin).all()
+    assert max_abs(got[fin], lse_ref[fin]) < 1e-3
+    assert ctx.device_status() == 0
 
 
 LIMIT_CASES = [
