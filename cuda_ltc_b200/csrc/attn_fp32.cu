@@ -8,6 +8,8 @@
 // and row sums are half-warp shuffle reductions.
 #include <math.h>
 
+#include <numeric>
+
 #include "attn_mask.cuh"
 #include "host_common.h"
 #include "sm100_ptx.cuh"
@@ -496,7 +498,7 @@ __device__ __forceinline__ void form_dout(float* dst, const CoreArgs& a, int b, 
 
 // pass 1: delta = rowsum(dO o O), left for pass 2, and dQ.  One CTA per TM query rows, KN keys per step.
 // kForm: dO is formed here (a kernel of its own, since form_dout takes registers: without it twice as many CTAs fit on an SM).
-// kCtas: how many share an SM; four leave no registers for the rows' deltas.
+// kCtas: how many share an SM (their registers); four leave no registers for the rows' deltas.
 template <typename T, int DP, int TM, int KN, int NT, int kMask, bool kForm, int kCtas>
 __global__ void __launch_bounds__(NT, kCtas) attn_bwd_dq_fp32_kernel(const CoreArgs a) {
     grid_dependency_wait();
@@ -806,10 +808,14 @@ int run_fwd(ltca_ctx* ctx, const CoreArgs& a) {
     return LTCA_OK;
 }
 
+// Whether four CTAs of that much dynamic shared memory are resident on one SM at once.
+constexpr bool four_fit_sm(size_t smem) { return 4 * (smem + 1024) <= 228 * 1024; }
+
 template <typename T, int DP, int TM, int KN, int NT, int kMask, bool kForm = false, int kCtas = NT == 128 ? 3 : 1>
 int run_dq(ltca_ctx* ctx, const CoreArgs& a) {
     static SmemOptIn once;
     constexpr size_t smem = ((size_t)(2 * TM + 2 * KN) * (DP + kPad) + TM * (KN + kPad) + TM) * sizeof(float);
+    static_assert(kCtas != 4 || four_fit_sm(smem), "four CTAs to an SM");
     int rc = set_smem(ctx, attn_bwd_dq_fp32_kernel<T, DP, TM, KN, NT, kMask, kForm, kCtas>, smem, once);
     if (rc) return rc;
     dim3 grid((a.Sq + TM - 1) / TM, a.H, a.B);
@@ -820,6 +826,7 @@ template <typename T, int DP, int TK, int QN, int NT, int kMask, int kCtas = TK 
 int run_dkv(ltca_ctx* ctx, const CoreArgs& a) {
     static SmemOptIn once;
     constexpr size_t smem = ((size_t)(2 * TK + 2 * QN) * (DP + kPad) + 2 * QN * (TK + kPad) + 2 * QN) * sizeof(float);
+    static_assert(kCtas != 4 || four_fit_sm(smem), "four CTAs to an SM");
     int rc = set_smem(ctx, attn_bwd_dkv_fp32_kernel<T, DP, TK, QN, NT, kMask, kCtas>, smem, once);
     if (rc) return rc;
     dim3 grid((a.Sk + TK - 1) / TK, a.H, a.B);
@@ -831,7 +838,6 @@ int run_dkv(ltca_ctx* ctx, const CoreArgs& a) {
 // done, they take whatever slots are left and sit unevenly on the SMs, 82 or 62 us instead of 57 for B16 H8 S100 D32.)
 // Tiles of 64 rows reuse what they load most; where they would leave SMs idle, tiles of 16 rows give four times the CTAs
 // and a quarter of the serial work.
-constexpr int kFourTilesCausalKeys = 256;
 template <typename T, int DP, int kMask>
 int run_small_dq(ltca_ctx* ctx, const CoreArgs& a) {
     if constexpr (sizeof(T) == 4 && DP <= 64) {
@@ -840,6 +846,26 @@ int run_small_dq(ltca_ctx* ctx, const CoreArgs& a) {
     return run_dq<T, DP, 16, 32, 128, kMask>(ctx, a);
 }
 bool fills_sms(const ltca_ctx* ctx, int B, int H, int S) { return (int64_t)B * H * ((S + 63) / 64) >= ctx->sm_device; }
+// Whether the 64-row backward tiles of a narrow head go four to an SM, in 128 registers a thread, instead of three.  (Figures:
+// backward, us, three and four.)
+//   - Tiles of one length: where that saves a wave.  B16 H8 S250 D32 151 and 135, B32 H8 S512 D32 878 and 857, B64 H8 S64 D16
+//     47 and 33; without a wave saved B12 H8 S400 D32 275 and 291, with a dense mask at D16 215 and 223.  Two tiles to a causal
+//     pair count as one length: B32 H8 S128 causal D16 59 and 52, D32 74 and 69.
+//   - Longer causal rows: what three to an SM even out as they go, four to an SM start side by side, and an SM takes about every
+//     sm_device-th tile, which is a pair's same tile over and over where that number and the tiles of a pair have a divisor in
+//     common (B16 H8 S256 D16 87 and 91, D32 115 and 118; B8 H8 S512 D32 193 and 204).  So where they have none and more
+//     than a few tiles are left over by three (B14 H8 S320 D16 109 and 92, D32 149 and 138; B12 H8 S448 D32 227 and 221; four
+//     left over, B8 H8 S448, 153 and 161), or where an SM has more than five tiles (B24 H8 S256 D16 117 and 111, D32 157 and 157;
+//     B64 H8 S512 D16 784 and 729, D32 1090 and 1062).
+//   - Key lengths, each pair's own: from five tiles on at the narrowest heads (uniform lengths, B32 H8 S256 D16 129 and 111; B10
+//     H8 S384 D16 109 and 120); three at others (B32 H8 S256 D32 180 and 183).
+bool four_tiles(const ltca_ctx* ctx, const CoreArgs& a, bool narrowest) {
+    const int64_t sms = ctx->sm_device, per_pair = ((a.Sq < a.Sk ? a.Sq : a.Sk) + 63) / 64, n = (int64_t)a.B * a.H * per_pair;
+    const bool many = n > 5 * sms;
+    if (a.kv_len) return many && narrowest;
+    if (a.causal && per_pair > 2) return many || (5 * n > 16 * sms && std::gcd(per_pair, sms) == 1);
+    return (n + 4 * sms - 1) / (4 * sms) < (n + 3 * sms - 1) / (3 * sms);
+}
 template <typename T, int DP, bool kMask>
 int run_rows(ltca_ctx* ctx, const CoreArgs& a, bool bwd) {
     auto fills = [&](int S) { return fills_sms(ctx, a.B, a.H, S); };
@@ -851,16 +877,13 @@ int run_rows(ltca_ctx* ctx, const CoreArgs& a, bool bwd) {
         if (!a.mask_bits) return (rc = run_small_dq<T, DP, kDense>(ctx, a)) ? rc : run_dkv<T, DP, 16, 32, 128, kDense>(ctx, a);
     }
     constexpr int kM = kMask ? kWords : kNoMask;
-    // Narrow heads: four 64-row tiles to an SM instead of three, in 128 registers a thread, where three would not take all tiles
-    // at once.  (B16 H8 S250 D32 175 us -> 152, B64 H8 S128 causal 151 -> 136, B32 H16 S60 D16 59 -> 44; with one wave of
-    // either, B4 H8 S400, 134 and 140.)  Not where the tiles of a pair last unevenly long (B8 H8 S512 causal 206 and 220), nor
-    // with a mask, whose words do not fit the registers either (B20 H16 S100 D24 120 and 132), except at the narrowest heads
-    // (B16 H8 S200 D16 126 and 108).
+    // Four tiles to an SM for the narrowest heads (D16), and for dQ up to D32: the shared memory of four dK/dV tiles is more than
+    // an SM's there, and in 128 registers three of them are slower (B16 H8 S250 D32 139 us, in 168 136).  With a dense mask at
+    // D32 the words do not fit the registers either (B20 H16 S100 D24 120 and 132).
     if constexpr (DP <= 16 || (DP <= 32 && kM == kNoMask)) {
-        const bool many = (int64_t)a.B * a.H * (((a.Sq < a.Sk ? a.Sq : a.Sk) + 63) / 64) > 3ll * ctx->sm_device;
-        if (many && (!a.causal || a.Sk <= kFourTilesCausalKeys)) {
+        if (four_tiles(ctx, a, DP <= 16)) {
             if ((rc = run_dq<T, DP, 64, 64, NT, kM, false, 4>(ctx, a))) return rc;
-            return run_dkv<T, DP, 64, 64, NT, kM, 4>(ctx, a);
+            return run_dkv<T, DP, 64, 64, NT, kM, DP <= 16 ? 4 : 3>(ctx, a);
         }
     }
     if ((rc = fills(a.Sq) ? run_dq<T, DP, 64, 64, NT, kM>(ctx, a) : run_small_dq<T, DP, kM>(ctx, a))) return rc;
