@@ -56,8 +56,10 @@ __device__ __forceinline__ float4 ldg4(const float* row, int i) { return __ldg(r
 // Rows of up to 1024 floats that stay in a warp's registers, E / 128 pieces of 16 bytes per lane: kN4 of them, where the loads of
 // a row all go out before the first is waited for, or (0) as many as E says, one after the other.  With few rows per SM a row
 // kernel lasts as long as one row's chain of loads and sums: residual + LayerNorm of 32768 x 512 37.5 us with one piece at a
-// time, 28.2 so (192 MB); 8192 x 512 12.3 and 10.3.  (The prepare launch below, whose other parts need the warps that the
-// registers would cost, 7.7 us with one at a time, 9.8 with all.)
+// time, 28.2 so (192 MB); 8192 x 512 12.3 and 10.3; module forward of 32768 rows of 128 52.9 and 47.1, of 384 139 and 135, of 1024
+// 398 and 390.  (The prepare launch below, whose other parts need the warps that the registers would cost, 7.7 us with one at a
+// time, 9.8 with all.)
+int row_pieces(int E) { return (E & 127) == 0 && E <= 1024 ? E >> 7 : 0; }
 template <int kN4>
 struct RowPieces {
     static constexpr int kMax = kN4 > 0 ? kN4 : 8;
@@ -72,7 +74,7 @@ __device__ __forceinline__ void layer_norm_pieces(const float* __restrict__ yr, 
                                                   float eps) {
     const RowPieces<kN4> p(E);
     constexpr int kMax = RowPieces<kN4>::kMax;
-    constexpr bool kEarly = kN4 > 0 && kN4 <= 4;       // gamma and beta with the row
+    constexpr bool kEarly = kN4 > 0 && kN4 <= 4;       // gamma and beta with the row, while registers last
     const int lane = threadIdx.x & 31;
     float4 v[kMax], r[kN4 > 0 ? kMax : 1], gm[kEarly ? kMax : 1], bt[kEarly ? kMax : 1];
     const float4 one = make_float4(1.f, 1.f, 1.f, 1.f), zero = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -180,8 +182,17 @@ __global__ void residual_layer_norm_kernel(const float* __restrict__ y, const fl
 
 int residual_layer_norm(ltca_ctx* ctx, const ltca_tsa_params* t, const float* y, int64_t rows) {
     const int wpb = 8;
-    auto kern = t->E == 512 ? residual_layer_norm_kernel<4> : t->E == 256 ? residual_layer_norm_kernel<2>
-              : t->E == 128 ? residual_layer_norm_kernel<1> : residual_layer_norm_kernel<0>;
+    auto kern = residual_layer_norm_kernel<0>;
+    switch (row_pieces(t->E)) {
+        case 1: kern = residual_layer_norm_kernel<1>; break;
+        case 2: kern = residual_layer_norm_kernel<2>; break;
+        case 3: kern = residual_layer_norm_kernel<3>; break;
+        case 4: kern = residual_layer_norm_kernel<4>; break;
+        case 5: kern = residual_layer_norm_kernel<5>; break;
+        case 6: kern = residual_layer_norm_kernel<6>; break;
+        case 7: kern = residual_layer_norm_kernel<7>; break;
+        case 8: kern = residual_layer_norm_kernel<8>; break;
+    }
     LTCA_CUDA_OK(ctx, launch_dependent(kern, dim3((unsigned)((rows + wpb - 1) / wpb)), dim3(wpb * 32),
                                        0, ctx->stream, y, t->x, t->ln_gamma, t->ln_beta, t->out, rows, t->E,
                                        t->use_residual, t->use_layer_norm, 1e-5f));
@@ -384,68 +395,57 @@ __global__ void __launch_bounds__(256) residual_dropout_kernel(const float* __re
     }
 }
 
-// Its registers form: both rows are read once, in 16-byte pieces.
+// Its registers form: rows of 128 kN4 floats, read once in 16-byte pieces, with gamma and the residual in flight beside them.
 template <int kN4>
 __device__ __forceinline__ void layer_norm_bwd_pieces(const float* __restrict__ gr, const float* __restrict__ xr, const float* __restrict__ gamma,
                                                       const float* __restrict__ res, float* __restrict__ dx, float* __restrict__ prod, int E,
                                                       float eps) {
-    const RowPieces<kN4> p(E);
-    constexpr int kMax = RowPieces<kN4>::kMax;
     const int lane = threadIdx.x & 31;
-    constexpr bool kEarly = kN4 > 0;                   // gamma and the residual with the rows
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    float4 xh[kMax], gv[kMax], gm[kEarly ? kMax : 1], r[kEarly ? kMax : 1];
+    float4 xh[kN4], gv[kN4], gm[kN4], r[kN4];
 #pragma unroll
-    for (int i = 0; i < kMax; ++i)
-        if (p.has(i)) {
-            xh[i] = ldg4(xr, lane + 32 * i);
-            gv[i] = ldg4(gr, lane + 32 * i);
-            if constexpr (kEarly) {
-                gm[i] = ldg4(gamma, lane + 32 * i);
-                r[i] = dx && res ? ldg4(res, lane + 32 * i) : zero;
-            }
-        }
+    for (int i = 0; i < kN4; ++i) {
+        xh[i] = ldg4(xr, lane + 32 * i);
+        gv[i] = ldg4(gr, lane + 32 * i);
+        gm[i] = ldg4(gamma, lane + 32 * i);
+        r[i] = dx && res ? ldg4(res, lane + 32 * i) : zero;
+    }
     float s0 = 0.f;
 #pragma unroll
-    for (int i = 0; i < kMax; ++i)
-        if (p.has(i)) s0 += (xh[i].x + xh[i].y) + (xh[i].z + xh[i].w);
+    for (int i = 0; i < kN4; ++i) s0 += (xh[i].x + xh[i].y) + (xh[i].z + xh[i].w);
     const float mean = warp_total(s0) / E;
     float s1 = 0.f;
 #pragma unroll
-    for (int i = 0; i < kMax; ++i)
-        if (p.has(i)) {
-            xh[i].x -= mean; xh[i].y -= mean; xh[i].z -= mean; xh[i].w -= mean;
-            s1 = fmaf(xh[i].x, xh[i].x, s1); s1 = fmaf(xh[i].y, xh[i].y, s1);
-            s1 = fmaf(xh[i].z, xh[i].z, s1); s1 = fmaf(xh[i].w, xh[i].w, s1);
-        }
+    for (int i = 0; i < kN4; ++i) {
+        xh[i].x -= mean; xh[i].y -= mean; xh[i].z -= mean; xh[i].w -= mean;
+        s1 = fmaf(xh[i].x, xh[i].x, s1); s1 = fmaf(xh[i].y, xh[i].y, s1);
+        s1 = fmaf(xh[i].z, xh[i].z, s1); s1 = fmaf(xh[i].w, xh[i].w, s1);
+    }
     const float inv_std = rsqrtf(warp_total(s1) / E + eps);
     float a1 = 0.f, a2 = 0.f;
 #pragma unroll
-    for (int i = 0; i < kMax; ++i)
-        if (p.has(i)) {
-            xh[i].x *= inv_std; xh[i].y *= inv_std; xh[i].z *= inv_std; xh[i].w *= inv_std;
-            const float4 m = kEarly ? gm[kEarly ? i : 0] : ldg4(gamma, lane + 32 * i);
-            const float4 gg = make_float4(gv[i].x * m.x, gv[i].y * m.y, gv[i].z * m.z, gv[i].w * m.w);
-            a1 += (gg.x + gg.y) + (gg.z + gg.w);
-            a2 = fmaf(gg.x, xh[i].x, a2); a2 = fmaf(gg.y, xh[i].y, a2);
-            a2 = fmaf(gg.z, xh[i].z, a2); a2 = fmaf(gg.w, xh[i].w, a2);
-            if (prod)
-                reinterpret_cast<float4*>(prod)[lane + 32 * i] =
-                    make_float4(gv[i].x * xh[i].x, gv[i].y * xh[i].y, gv[i].z * xh[i].z, gv[i].w * xh[i].w);
-            gv[i] = gg;
-        }
+    for (int i = 0; i < kN4; ++i) {
+        xh[i].x *= inv_std; xh[i].y *= inv_std; xh[i].z *= inv_std; xh[i].w *= inv_std;
+        const float4 gg = make_float4(gv[i].x * gm[i].x, gv[i].y * gm[i].y, gv[i].z * gm[i].z, gv[i].w * gm[i].w);
+        a1 += (gg.x + gg.y) + (gg.z + gg.w);
+        a2 = fmaf(gg.x, xh[i].x, a2); a2 = fmaf(gg.y, xh[i].y, a2);
+        a2 = fmaf(gg.z, xh[i].z, a2); a2 = fmaf(gg.w, xh[i].w, a2);
+        if (prod)
+            reinterpret_cast<float4*>(prod)[lane + 32 * i] =
+                make_float4(gv[i].x * xh[i].x, gv[i].y * xh[i].y, gv[i].z * xh[i].z, gv[i].w * xh[i].w);
+        gv[i] = gg;
+    }
     if (!dx) return;
     const float m1 = warp_total(a1) / E, m2 = warp_total(a2) / E;
 #pragma unroll
-    for (int i = 0; i < kMax; ++i)
-        if (p.has(i)) {
-            float4 d = kEarly ? r[kEarly ? i : 0] : res ? ldg4(res, lane + 32 * i) : zero;
-            d.x += inv_std * (gv[i].x - m1 - xh[i].x * m2);
-            d.y += inv_std * (gv[i].y - m1 - xh[i].y * m2);
-            d.z += inv_std * (gv[i].z - m1 - xh[i].z * m2);
-            d.w += inv_std * (gv[i].w - m1 - xh[i].w * m2);
-            reinterpret_cast<float4*>(dx)[lane + 32 * i] = d;
-        }
+    for (int i = 0; i < kN4; ++i) {
+        float4 d = r[i];
+        d.x += inv_std * (gv[i].x - m1 - xh[i].x * m2);
+        d.y += inv_std * (gv[i].y - m1 - xh[i].y * m2);
+        d.z += inv_std * (gv[i].z - m1 - xh[i].z * m2);
+        d.w += inv_std * (gv[i].w - m1 - xh[i].w * m2);
+        reinterpret_cast<float4*>(dx)[lane + 32 * i] = d;
+    }
 }
 
 // LayerNorm backward, one warp per row.  g = gradient at the LayerNorm output, x = its input.
@@ -462,11 +462,13 @@ __global__ void layer_norm_bwd_kernel(const float* __restrict__ g, const float* 
     const int lane = threadIdx.x & 31;
     const float* xr = x + row * E;
     const float* gr = g + row * E;
-    if ((E & 127) == 0 && E <= 1024 && aligned16(g, x, gamma, res, dx) && (reinterpret_cast<uintptr_t>(prod) & 15) == 0) {
-        const float* rr = res ? res + row * E : nullptr;
-        float *dr = dx ? dx + row * E : nullptr, *pr = prod ? prod + row * E : nullptr;
-        layer_norm_bwd_pieces<kN4>(gr, xr, gamma, rr, dr, pr, E, eps);
-        return;
+    if constexpr (kN4 > 0) {
+        if (aligned16(g, x, gamma, res, dx) && (reinterpret_cast<uintptr_t>(prod) & 15) == 0) {
+            const float* rr = res ? res + row * E : nullptr;
+            float *dr = dx ? dx + row * E : nullptr, *pr = prod ? prod + row * E : nullptr;
+            layer_norm_bwd_pieces<kN4>(gr, xr, gamma, rr, dr, pr, E, eps);
+            return;
+        }
     }
     float sum = 0.f;
     for (int i = lane; i < E; i += 32) sum += xr[i];
@@ -1739,8 +1741,17 @@ static int prenorm_backward(ltca_ctx* ctx, const ltca_tsa_params* t, bool want_d
         // LayerNorm(x) is no longer needed: its buffer takes dxin * xhat, whose column sums are dgamma
         float* prod = (want_ln_params && t->dgamma) ? xin : nullptr;
         const int wpb = 8;
-        auto kern = t->E == 512 ? layer_norm_bwd_kernel<4> : t->E == 256 ? layer_norm_bwd_kernel<2>
-                  : t->E == 128 ? layer_norm_bwd_kernel<1> : layer_norm_bwd_kernel<0>;
+        auto kern = layer_norm_bwd_kernel<0>;
+        switch (row_pieces(t->E)) {
+            case 1: kern = layer_norm_bwd_kernel<1>; break;
+            case 2: kern = layer_norm_bwd_kernel<2>; break;
+            case 3: kern = layer_norm_bwd_kernel<3>; break;
+            case 4: kern = layer_norm_bwd_kernel<4>; break;
+            case 5: kern = layer_norm_bwd_kernel<5>; break;
+            case 6: kern = layer_norm_bwd_kernel<6>; break;
+            case 7: kern = layer_norm_bwd_kernel<7>; break;
+            case 8: kern = layer_norm_bwd_kernel<8>; break;
+        }
         LTCA_CUDA_OK(ctx, launch_dependent(kern, dim3((unsigned)((rows + wpb - 1) / wpb)), dim3(wpb * 32), 0, ctx->stream,
                                            (const float*)dxin, t->x, t->ln_gamma, (want_dx && t->use_residual) ? g : nullptr,
                                            want_dx ? t->dx : nullptr, prod, rows, t->E, 1e-5f));
