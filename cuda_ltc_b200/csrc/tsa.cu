@@ -203,8 +203,11 @@ int residual_layer_norm(ltca_ctx* ctx, const ltca_tsa_params* t, const float* y,
 // shared memory.  As a product and a row kernel these were two of the eight dependent launches of a small training step, each
 // of which costs 3 to 4 us whatever it computes: step of B8 S32 E32 H4 32.3 -> 29.3 us, forward of B32 S128 E32 H4 34.8 -> 33.8.
 // Every block reads all of Wo: with 64 KB of it 2048 rows of the forward B32 S64 E64 H8 width 32 take 33.9 us instead of 32.7,
-// so it is limited to 32 KB, and to 4096 rows.
+// so it is limited to 32 KB and 4096 rows, and to the multiply-adds of 3072 rows with 32 KB.  Forward of 3072 rows with 8192
+// weights 25.1 -> 24.5 us, of 4096 with 6144 34.7 -> 34.4, with 512 (E4) 22.7 -> 21.0; of 4096 with 7680 40.2 -> 41.8, with
+// 8192 27.3 -> 28.3.
 constexpr int kProjThreads = 256, kProjMaxE = 64, kProjMaxWeights = 8192, kProjRows = 4096;
+constexpr int64_t kProjProducts = 3072ll * kProjMaxWeights;
 __global__ void __launch_bounds__(kProjThreads) project_norm_kernel(const float* __restrict__ ctx, const float* __restrict__ wo,
                                                                     const float* __restrict__ bo, const float* __restrict__ x,
                                                                     const float* __restrict__ gamma, const float* __restrict__ beta,
@@ -267,7 +270,7 @@ __global__ void __launch_bounds__(kProjThreads) project_norm_kernel(const float*
 // Whether that kernel takes the call (ctx is the library's own buffer, aligned and contiguous).
 bool projects_and_norms(const ltca_tsa_params* t, int64_t rows, int HW) {
     return t->E <= kProjMaxE && (t->E % 4) == 0 && (HW % 4) == 0 && HW * t->E <= kProjMaxWeights && rows <= kProjRows &&
-           (reinterpret_cast<uintptr_t>(t->wo) & 15) == 0;
+           rows * HW * t->E <= kProjProducts && (reinterpret_cast<uintptr_t>(t->wo) & 15) == 0;
 }
 int project_norm(ltca_ctx* ctx, const ltca_tsa_params* t, const float* core, int64_t rows, int HW) {
     static SmemOptIn once;

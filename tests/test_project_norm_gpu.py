@@ -7,11 +7,13 @@ import pytest
 import oracle
 
 
-# B, S, E, H, W: one row, a ragged last block, E no multiple of a warp, the most columns, the most weights, beyond either
+# B, S, E, H, W: one row, a ragged last block, E no multiple of a warp, the most columns, the most weights, beyond either, the
+# most products, beyond them, the widest context
 @pytest.mark.gpu
 @pytest.mark.parametrize("shape", [(1, 1, 32, 4, 32), (3, 7, 32, 2, 16), (2, 9, 36, 3, 12), (2, 20, 64, 4, 32), (1, 33, 64, 8, 16),
                                    (2, 10, 64, 2, 68),
-                                   (2, 8, 68, 2, 16), (64, 65, 32, 2, 16)])
+                                   (2, 8, 68, 2, 16), (64, 65, 32, 2, 16), (64, 64, 32, 4, 48), (61, 64, 48, 4, 40),
+                                   (3, 11, 4, 4, 512)])
 @pytest.mark.parametrize("norm", [False, True])
 def test_projection_residual_norm(shape, norm):
     import torch
