@@ -74,7 +74,8 @@ struct GemmMaps { CUtensorMap a[kMaxGemmProblems], b[kMaxGemmProblems], c[kMaxGe
 struct GemmGroupMaps {
     CUtensorMap a[3 * kMaxGemmProblems], b[3 * kMaxGemmProblems], c[2 * kMaxGemmProblems];
     int first[kMaxGemmProblems + 1];   // a member's pairs
-    int form[kMaxGemmProblems];        // ... and operand forms (bit 0: A stored [K, M], bit 1: B stored [K, N])
+    int form[kMaxGemmProblems];        // ... operand forms (bit 0: A stored [K, M], bit 1: B stored [K, N]), and whether its
+                                       // result has a second term (bit 2; where any has one)
 };
 
 struct GemmKArgs {
@@ -130,6 +131,8 @@ __device__ __forceinline__ GemmTile gemm_tile(const Maps& maps, const GemmKArgs&
     return t;
 }
 
+__device__ __forceinline__ bool has_second_term(const GemmMaps&, int) { return true; }
+__device__ __forceinline__ bool has_second_term(const GemmGroupMaps& maps, int problem) { return (maps.form[problem] & 4) != 0; }
 template <bool kByMember, bool kMn, typename Maps>
 __device__ __forceinline__ bool is_mn(const Maps& maps, int problem, int bit) {
     if constexpr (kByMember) return (maps.form[problem] & bit) != 0;
@@ -406,7 +409,8 @@ gemm_bf16_sm100_kernel(const __grid_constant__ typename std::conditional<kKind =
                             if (add_to_c) tma_reduce_add_4d(tc, stage_addr + hb * (kBM * 128), gn0, t.m0, t.bh, t.bb);
                             else tma_store_4d(tc, stage_addr + hb * (kBM * 128), gn0, t.m0, g.ksplit > 1 ? t.slice : t.bh,
                                               g.ksplit > 1 ? t.problem : t.bb);
-                            if (g.c_lo) tma_store_4d(&maps.c[kKind == kGroup ? kMaxGemmProblems + t.problem : 1], stage_addr + (hb + 1) * (kBM * 128), gn0, t.m0, t.bh, t.bb);
+                            if (g.c_lo && has_second_term(maps, t.problem))
+                                tma_store_4d(&maps.c[kKind == kGroup ? kMaxGemmProblems + t.problem : 1], stage_addr + (hb + 1) * (kBM * 128), gn0, t.m0, t.bh, t.bb);
                         }
                         tma_store_commit();
                         // the box that the next piece takes has been read
@@ -789,17 +793,18 @@ int gemm_sm100_group(ltca_ctx* ctx, const GemmGroup& gg) {
     g.a_head = g.b_head = 1;
     g.out_bf16 = gg.out_bf16;
     g.tma_store = 1;
-    g.c_lo = gg.m[0].c_lo;
+    for (int i = 0; i < gg.n; ++i)
+        if (gg.m[i].c_lo) g.c_lo = gg.m[i].c_lo;       // (whether any is there: the stores go by the members' tensor maps)
     g.status = ctx->d_status;
     g.run_if = ctx->run_if;
     int rc;
     for (int i = 0; i < gg.n; ++i) {
         const GemmGroup::Member& m = gg.m[i];
-        if (m.terms < 1 || m.terms > 3 || (m.c_lo != nullptr) != (g.c_lo != nullptr) || (m.c_lo && !gg.out_bf16))
-            return fail(ctx, LTCA_ERR_INVALID, "gemm: a member has one to three terms, and a second result term as the others");
+        if (m.terms < 1 || m.terms > 3 || (m.c_lo && !gg.out_bf16))
+            return fail(ctx, LTCA_ERR_INVALID, "gemm: a member has one to three terms, and a second term of its result in bf16 only");
         const int64_t as[2] = {m.a_hs, 0}, bs[2] = {m.b_hs, 0};
         maps.first[i + 1] = maps.first[i] + m.terms;
-        maps.form[i] = (m.a[0].mn_major ? 1 : 0) | (m.b[0].mn_major ? 2 : 0);
+        maps.form[i] = (m.a[0].mn_major ? 1 : 0) | (m.b[0].mn_major ? 2 : 0) | (m.c_lo ? 4 : 0);
         for (int t = 0; t < m.terms; ++t) {
             if (m.a[t].mn_major != m.a[0].mn_major || m.b[t].mn_major != m.b[0].mn_major)
                 return fail(ctx, LTCA_ERR_INVALID, "gemm: the terms of a member share the operand forms");

@@ -44,7 +44,7 @@ struct GemmProblem {
 int gemm_sm100(ltca_ctx* ctx, const GemmProblem& gp);
 
 // Up to four products of the same shape in one launch, each of its own operand forms and number of summed terms, for every one
-// of `heads` (strides a_hs, b_hs, c_hs between them).  c_lo as in GemmProblem, for all members or for none.  Results need
+// of `heads` (strides a_hs, b_hs, c_hs between them).  c_lo as in GemmProblem.  Results need
 // 16-byte aligned rows (gemm_group_aligned).
 struct GemmGroup {
     struct Member {

@@ -881,7 +881,7 @@ size_t wide_extra(const TPlan& pl, int which) {
 // On products of the weights: what a forward keeps (x, the weights with the second terms of Wq and Wk, M, N, T, z, lse, scores,
 // probabilities) and what no later call needs (the other second terms).
 size_t composed_kept(const TPlan& pl) { return pl.xb + 5 * pl.w_in + pl.w_out + 2 * pl.me + 2 * pl.act + pl.lse + pl.mat32 + pl.mat16; }
-size_t composed_scratch(const TPlan& pl) { return pl.xb + pl.w_in + pl.w_out + 2 * pl.me + pl.act; }
+size_t composed_scratch(const TPlan& pl) { return pl.xb + pl.w_in + pl.w_out + pl.me + pl.act; }
 
 size_t tensor_workspace(const TPlan& pl, int which) {
     if (pl.composed) {
@@ -911,7 +911,7 @@ struct TBufs {
     void *xl, *wql, *wkl, *ql, *kl, *P;
     float* scores;
     // ... on products of the weights
-    void *wvl, *wol, *m, *ml, *n, *nl, *t, *tl, *z;
+    void *wvl, *wol, *m, *ml, *n, *t, *tl, *z;
 };
 
 // What both forms of the module on the written-out-score path have alike comes first.
@@ -1014,7 +1014,6 @@ int composed_forward_core(ltca_ctx* ctx, const ltca_tsa_params* t, const TPlan& 
     tb->wvl = r; r += pl.w_in;
     tb->wol = r; r += pl.w_out;
     tb->ml = r;  r += pl.me;
-    tb->nl = r;  r += pl.me;
     tb->tl = r;  r += pl.act;
     tb->rest = r;
     tb->q = tb->k = tb->v = tb->ctx = tb->ql = tb->kl = nullptr;
@@ -1064,7 +1063,7 @@ int composed_forward_core(ltca_ctx* ctx, const ltca_tsa_params* t, const TPlan& 
         n.a[1] = GemmOperand{tb->wv, HW, 0};  n.b[1] = GemmOperand{tb->wol, Ep, 1};
         n.a[2] = GemmOperand{tb->wvl, HW, 0}; n.b[2] = GemmOperand{tb->wo, Ep, 1};
         n.a_hs = E; n.b_hs = (int64_t)E * Ep;
-        n.c = tb->n; n.c_lo = tb->nl;
+        n.c = tb->n;
         m.ldc = n.ldc = HW;
         m.c_hs = n.c_hs = E;
         if ((rc = gemm_sm100_group(ctx, gg))) return rc;
