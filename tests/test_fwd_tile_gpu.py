@@ -101,6 +101,22 @@ def test_forward_tiles_with_a_mask(ctx, case, storage, D):
     assert ctx.device_status() == 0
 
 
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("storage", ["bf16", "f32"])
+def test_forward_tiles_in_groups_of_pairs(ctx, storage, D):
+    """K and V of 99 (batch, head) pairs, 50 MB in bf16, are dealt out in two groups, the last one smaller."""
+    B, H, Sq, Sk = 3, 33, 260, 131072 // D
+    dt = torch.bfloat16 if storage == "bf16" else torch.float32
+    q, k, v = (bf16_round(randn((B, H, n, D), 90 + i, 0.5)) for i, n in enumerate((Sq, Sk, Sk)))
+    tq, tk, tv = (torch.from_numpy(a).cuda().to(dt) for a in (q, k, v))
+    o, lse = ctx.attn_fwd(tq, tk, tv, causal=True, mode=_lib.MODE_BF16)
+    o_ref, lse_ref = oracle.attn_fwd(q, k, v, 1.0 / math.sqrt(D), True)
+    half = 2.0 ** -8 if storage == "bf16" else 0.0
+    err = np.abs(o.float().cpu().numpy() - o_ref)
+    assert (err <= 2e-3 + half * np.abs(o_ref)).all(), err.max()
+    assert max_abs(lse.cpu().numpy(), lse_ref) < 2e-3
+
+
 LIMIT_CASES = [
     # B, H, Sq, Sk, causal, lengths, mask
     (1, 1, 1, 1, False, False, False),          # fewer tiles than one CTA has teams

@@ -176,3 +176,38 @@ def test_kept_forward_is_read_in_the_form_it_was_written(case):
         assert torch.equal(a, r) and torch.equal(b, r)
     torch.cuda.synchronize()
     assert ctx.device_status() == 0 and other.device_status() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("case", [(4, 136, 136, 2), (16, 64, 256, 4)])
+def test_results_that_start_off_a_16_byte_boundary(case):
+    """Results that TMA cannot store or add to: a product of their own for each of the weights, and dx added to in place."""
+    import ctypes as C
+    import torch
+    import cuda_ltc_b200 as ltc
+    from cuda_ltc_b200 import _lib
+    B, S, E, H = case
+    ctx = ltc.Context(0)
+    g = torch.Generator(device="cuda").manual_seed(5)
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda")
+    lim = (3.0 / E) ** 0.5
+    x, dy = 0.5 * rnd(B * S, E), rnd(B * S, E)
+    w = [lim * 0.5 * rnd(E, H * E) for _ in range(3)] + [lim * 0.5 * rnd(H * E, E)]
+    want = ctx.tsa_bwd(x, *w, dy, B, S, H, E)
+    p = ctx._tsa_sizes(x, *w, B, S, H, E, _lib.MODE_AUTO, False)
+    p.time_major = 1
+    p.x, p.wq, p.wk, p.wv, p.wo, p.dy = (t.data_ptr() for t in (x, *w, dy))
+    got = [torch.full((t.numel() + 2,), float("nan"), device="cuda") for t in want]
+    for n, t in zip(("dx", "dwq", "dwk", "dwv", "dwo"), got):
+        setattr(p, n, t.data_ptr() + 4)
+    need = C.c_size_t(0)
+    ctx.check(ctx.lib.ltca_tsa_workspace_bytes(C.byref(p), 2, C.byref(need)))
+    ws = torch.empty(need.value, dtype=torch.uint8, device="cuda")
+    p.workspace, p.workspace_bytes = ws.data_ptr(), need.value
+    ctx.check(ctx.lib.ltca_tsa_bwd(ctx.handle, C.byref(p)))
+    torch.cuda.synchronize()
+    for a, r in zip(got, want):
+        # the same products; sums of fp32 in another order at most
+        assert rel_l2(a[1:-1].cpu().numpy(), r.flatten().cpu().numpy()) < 1e-6
+        assert torch.isnan(a[0]) and torch.isnan(a[-1])
+    assert ctx.device_status() == 0
