@@ -298,12 +298,15 @@ def other_configs(torch, ctx, peaks):
     kwr = dict(scale=1.0, causal=False, time_major=True, mode=_lib.MODE_AUTO)
     f_ms = _timed(torch, lambda: ctx.tsa_fwd(x, *wsr, wor, B, S, H, Wr, gamma=gamma, beta=beta, **kwr), n=10, flush=flush)
     b_ms = _timed(torch, lambda: ctx.tsa_bwd(x, *wsr, wor, dy, B, S, H, Wr, **kwr), n=10, flush=flush)
+    # two products with x, T = x M and z = x N, where q, k, v and the output projection would be four, and the products of
+    # the weights (M and N) behind them
     gemm_r = 2.0 * B * S * E * H * Wr
+    weights_r = 2.0 * E * E * H * Wr
     core_r = 4.0 * B * H * S * S * Wr
     out["config2_module_reference_form_head_width_512"] = {
         "fwd_us": f_ms * 1e3, "bwd_incl_recomputed_fwd_us": b_ms * 1e3,
-        "fwd_tflops": (4 * gemm_r + core_r) / f_ms / 1e9,
-        "path": "written-out scores, batched tcgen05 GEMMs, two-term Q/K operands"}
+        "fwd_tflops": (2 * gemm_r + 2 * weights_r + core_r) / f_ms / 1e9,
+        "path": "per-head products of the weights, written-out scores, batched tcgen05 GEMMs, two-term operands up to the scores"}
     del wsr, wor
     # config 5: attention core
     fl5 = flops_fwd(64, 8, 512, 64)
@@ -417,13 +420,18 @@ def module_measurement(args):
     rows = B * S * world
     gemm = 2.0 * rows * E * H * W                       # one projection
     core = 4.0 * B * world * H * S * S * W / (1 if args.reference_form else 2)
+    fwd_flops, bwd_flops = 4 * gemm + core, 11 * gemm + 3.5 * core
+    if args.reference_form:
+        # on per-head products of the weights: T, z, M and N forward; the same again, four gradients of rows and four of weights
+        weights = 2.0 * world * E * E * H * W
+        fwd_flops, bwd_flops = 2 * gemm + 2 * weights + core, 6 * gemm + 6 * weights + 2.5 * core
     print(json.dumps({"workload": f"TimeSelfAttention module, B=32 per GPU, S=256 E=512 H=8 W={W} "
                                   + ("scale 1 unmasked (reference form), AUTO mode" if args.reference_form else
                                      "causal, tensor-pipe mode") + "; weight gradients summed over the ranks",
                       "n_gpus": world,
                       "fwd_us": f_ms * 1e3, "bwd_incl_recompute_us": b_ms * 1e3,
-                      "fwd_tflops": (4 * gemm + core) / f_ms / 1e9,
-                      "bwd_tflops": (11 * gemm + 3.5 * core) / b_ms / 1e9,
+                      "fwd_tflops": fwd_flops / f_ms / 1e9,
+                      "bwd_tflops": bwd_flops / b_ms / 1e9,
                       "device_status": status}))
 
 

@@ -534,8 +534,8 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
 // leaves a tile's warps idle for about 1300 cycles while P is multiplied and the next scores are formed), and the tiles
 // are independent work: a causal tile of two key steps leaves after two and the next takes its place, and a call is
 // dealt out in pieces of 128 rows.  A persistent kernel with four tiles on one key stream, which this replaces, made the
-// early tiles of 512 causal rows wait for the late ones' keys: B64 H8 S512 causal 68 us against 49, B8 H16 S4096 causal
-// 440 against 392.  What it pays is a set-up per tile and a K/V read per tile from L2 (20 bytes per clock and SM).
+// early tiles of 512 causal rows wait for the late ones' keys: B64 H8 S512 causal 68 us against 46 now, B8 H16 S4096 causal
+// 440 against 365.  What it pays is a set-up per tile and a K/V read per tile from L2 (20 bytes per clock and SM).
 //   - warps 0-3 softmax, one row per thread, head_dim keys per step; tensor memory S [0, D), O [D, 2 D).  At head_dim 128 a
 //     thread so holds 128 scores in its 216 registers and two warps share a scheduler; two threads per row, 64 scores each,
 //     had four of them but met once a step to agree on the row's maximum (B8 H16 S4096 causal 568 us, one per row 525).
@@ -556,9 +556,9 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
 // SM that has room, so there one CTA per SM holds the same number of tiles side by side, a team of warps each with its own
 // ring, barriers and accumulators, and the teams take tiles from a counter until there are none left.  A tile's
 // arithmetic, and with it every bit of the result, is that of the plain form; a team waits for its slowest warp between
-// tiles and loads nothing of the next tile before that.  On 16 SMs B8 H16 S4096 causal takes 4.00 ms, 434 us scaled to 148,
-// where the plain form takes 396 there (four tiles that start together stay in step); on 132 SMs 516 us, B8 H16 S1024
-// causal 56, B64 H8 S512 causal 61.
+// tiles and loads nothing of the next tile before that.  On 16 SMs B8 H16 S4096 causal takes 3.72 ms, 402 us scaled to 148,
+// where the plain form takes 365 there (four tiles that start together stay in step); on 132 SMs 473 us, B8 H16 S1024
+// causal 43, B64 H8 S512 causal 56.
 // ---------------------------------------------------------------------------------------------
 template <int D, bool kSplitP, bool kMask>
 struct TileCfg {
@@ -1037,9 +1037,12 @@ int launch_fwd(ltca_ctx* ctx, const ltca_attn_params* p, const void* mask_words,
     a.status = ctx->d_status;
 
     // The one-tile kernel, except where head_dim is 64 and the call has so few tiles that two-tile CTAs run in one wave and
-    // keys enough that a tile's own step time decides: there two threads per row shorten the step (B=1 H=8 S=4096 causal
-    // 60 us against 65, B=4 H=16 Sq=512 Sk=4096 64 against 78; at S=512 the one-tile kernel is the faster one again, 11.2
-    // against 12.0 for B=4 H=8).  The device's SM count decides, not a limit set on the context: the choice, and with it
+    // keys enough that a tile's own step time decides: there two threads per row shorten the step (two-tile kernel against
+    // one-tile, us: bf16 B=1 H=8 S=4096 causal 60 and 61, B=4 H=16 Sq=512 Sk=4096 63 and 76, B=16 H=8 Sq=128 Sk=1024 15 and
+    // 17; at S=512 the one-tile kernel is the faster one, 10.4 for B=4 H=8).  The line is older than the one-tile kernel's
+    // hand-over of P in halves: with few pairs and long keys that kernel has since become the faster one for fp32 results (B=1
+    // H=8 S=4096 causal 91 and 85; but B=4 H=16 Sq=512 Sk=4096 119 and 131) and is 1 to 13 % faster at some bf16 shapes
+    // (B=2 H=8 S=1024 18.1 and 17.3, B=1 H=8 S=700 15.0 and 13.0; but S=2048 causal B=2 31.6 and 32.4).  The device's SM count decides, not a limit set on the context: the choice, and with it
     // the bits of the result, does not move with the launch width.
     const int64_t ctas2 = (int64_t)p->B * p->H * ((p->Sq + 2 * kBlockM - 1) / (2 * kBlockM));
     const int64_t sms = ctx->sm_device > 0 ? ctx->sm_device : kPlanSms;

@@ -7,7 +7,8 @@ the per-rank timings (maximum over ranks) and, for checks, of a few scalars.
 
 The whole module (projections around the core) shards by sequences with replicated weights:
 forward and the input gradient stay local, and only the weight gradients, which are sums over
-rows, need one sum over the ranks (``sum_weight_grads``).
+rows, need one sum over the ranks (``sum_weight_grads``).  The module's kernels and the order of its products follow the
+number of rows in a call, so a batch dealt out over another number of ranks has other bits, within the mode's accuracy.
 
 The reference is single-GPU (its only device selection is ``cudaSetDevice(0)`` in a test,
 src/ml/time_self_attention_test.cu:523); this module has no counterpart there.

@@ -229,6 +229,10 @@ int ltca_attn_decode_static(void* stream, const ltca_attn_params* p, char* err, 
  * wq, wk, wv : [E, H*W] row-major, y = x w.   wo : [H*W, E].   W = head_width:
  * E (reference-compatible, include/cuDNN_ops.h:166-169) or E/H (benchmark form).
  * Biases are optional (FlashAttention form, src/ml/flash_attention.cu:458-470).
+ *
+ * The bits of a result belong to the shape, rows included: the kernels, and for heads as wide as the model the order
+ * in which the products are formed (from 4 E rows on), follow it.  The same sequences in calls of other sizes, on
+ * other numbers of ranks or in a short last batch, differ within the mode's accuracy.
  */
 typedef struct {
     int32_t B, S, E, H;
