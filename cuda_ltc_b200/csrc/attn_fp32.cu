@@ -4,8 +4,8 @@
 //
 // Replaces flashAttentionKernel (reference src/ml/flash_attention.cu:18-272) on its own valid
 // domain (head_dim <= 16, one key tile) and extends it to a true online softmax for longer
-// sequences; the score tiles keep one query row inside a half-warp so that row maxima
-// and row sums are half-warp shuffle reductions.
+// sequences; the score tiles keep one query row inside sixteen lanes so that row maxima
+// and row sums are shuffle reductions.
 #include <math.h>
 
 #include <numeric>
@@ -154,8 +154,16 @@ __device__ __forceinline__ void load_padded(float* dst, const T* base, int64_t r
     }
 }
 
+// Lanes.  A 16-byte shared read takes two wavefronts where every lane shares its address with lane ^ 1 or lane ^ 2, and four
+// where the lanes that share one lie further apart (measured: 2.1 and 4.0 cycles an SM, however few addresses there are).  So
+// the two sides of every product below alternate at the lowest lane bits: bit 0 picks the row, bit 1 the column.
+// With the row at bit 4 and with it at bit 0, us: tiles of 16 rows, B4 H4 S512 D32 forward 40 and 30, backward 136 and 103; tiles
+// of 64 rows, B16 H8 S250 backward D16 92 and 83, D32 135 and 130.
+//
 // Thread layout of the score products: NT threads as (NT / 16) x 16.  Thread (ty, tx) owns columns tx + 16 j and rows
 // row_of(ty) + (NT / 16) i; the two rows that a warp holds per i lie four apart, which puts their words in different banks.
+__device__ __forceinline__ int score_tx() { return (threadIdx.x >> 1) & 15; }
+__device__ __forceinline__ int score_ty() { return 2 * (threadIdx.x >> 5) + (threadIdx.x & 1); }
 __device__ __forceinline__ int row_of(int ty) { return ((ty >> 1) & 3) + 4 * (ty & 1) + 8 * (ty >> 3); }
 
 // s[i][j] = A[row i] . B[col j] over DP features
@@ -196,8 +204,8 @@ struct AccLayout {
     int tx, ty;
     bool active;
     __device__ __forceinline__ AccLayout() {
-        tx = threadIdx.x % TX;
-        ty = threadIdx.x / TX;
+        tx = (threadIdx.x & 31) / 2 % TX;
+        ty = 32 / TX * (threadIdx.x / 32) + 2 * ((threadIdx.x & 31) / 2 / TX) + threadIdx.x % 2;
         active = ty < TY;
     }
 };
@@ -260,14 +268,15 @@ __device__ __forceinline__ uint32_t row_mask(const uint32_t* words, int tx) {
     for (int j = 0; j < CN; ++j) bits |= (words[j / 2] >> (tx + 16 * (j % 2)) & 1u) << j;
     return bits;
 }
-__device__ __forceinline__ float half_warp_max(float v) {
+// over a row's 16 threads (score_tx)
+__device__ __forceinline__ float row_max(float v) {
 #pragma unroll
-    for (int o = 8; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+    for (int o = 16; o > 1; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
     return v;
 }
-__device__ __forceinline__ float half_warp_sum(float v) {
+__device__ __forceinline__ float row_sum(float v) {
 #pragma unroll
-    for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    for (int o = 16; o > 1; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
 
@@ -289,7 +298,7 @@ __global__ void __launch_bounds__(NT, TM < 64 ? 4 : DP <= 32 ? 4 : DP <= 64 ? 3 
     float* row_scale = Ps + TM * LP;     // [TM]: what the accumulator is multiplied with (step), 1 / sum (end)
     const bool vec = a.vec != 0;
 
-    const int tx = threadIdx.x & 15, row0 = row_of(threadIdx.x >> 4);
+    const int tx = score_tx(), row0 = row_of(score_ty());
     const int q0 = blockIdx.x * TM;
     const int h = blockIdx.y, b = blockIdx.z;
     int kvlen = a.Sk;
@@ -375,7 +384,7 @@ __global__ void __launch_bounds__(NT, TM < 64 ? 4 : DP <= 32 ? 4 : DP <= 64 ? 3 
                 s[i][j] = v;
                 mt = fmaxf(mt, v);
             }
-            mt = half_warp_max(mt);
+            mt = row_max(mt);
             const float m_new = fmaxf(m_run[i], mt);
             const float m_safe = (m_new == kNegInf) ? 0.f : m_new;
             const float corr = (m_run[i] == kNegInf) ? 0.f : expf(m_run[i] - m_safe);
@@ -386,7 +395,7 @@ __global__ void __launch_bounds__(NT, TM < 64 ? 4 : DP <= 32 ? 4 : DP <= 64 ? 3 
                 Ps[r * LP + tx + 16 * j] = p;
                 rs += p;
             }
-            rs = half_warp_sum(rs);
+            rs = row_sum(rs);
             l_run[i] = l_run[i] * corr + rs;
             m_run[i] = m_new;
             if (tx == 0) row_scale[r] = corr;
@@ -513,7 +522,7 @@ __global__ void __launch_bounds__(NT, kCtas) attn_bwd_dq_fp32_kernel(const CoreA
     float* row_delta = Ss + TM * LP;
     const bool vec = a.vec != 0;
 
-    const int tx = threadIdx.x & 15, row0 = row_of(threadIdx.x >> 4);
+    const int tx = score_tx(), row0 = row_of(score_ty());
     const int q0 = blockIdx.x * TM;
     const int h = blockIdx.y, b = blockIdx.z;
     int kvlen = a.Sk;
@@ -646,7 +655,7 @@ __global__ void __launch_bounds__(NT, kCtas) attn_bwd_dkv_fp32_kernel(const Core
     float* row_delta = row_lse + QN;
     const bool vec = a.vec != 0;
 
-    const int tx = threadIdx.x & 15, row0 = row_of(threadIdx.x >> 4);
+    const int tx = score_tx(), row0 = row_of(score_ty());
     const int k0 = blockIdx.x * TK;
     const int h = blockIdx.y, b = blockIdx.z;
     int kvlen = a.Sk;

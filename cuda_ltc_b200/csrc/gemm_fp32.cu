@@ -111,7 +111,8 @@ __global__ void __launch_bounds__(NT) gemm_fp32_kernel(const __grid_constant__ G
     constexpr int KC = G::KC, RM = G::RM, CN = G::CN, kStages = G::kStages;
     constexpr int kA = G::template a_floats<TA>(), kB = G::template b_floats<TB>();
     extern __shared__ __align__(16) float sm[];
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    // the row at lane bit 0: both operands' 16-byte reads then meet their like at lane ^ 1 or ^ 2, two wavefronts instead of four
+    const int tx = (threadIdx.x >> 1) & 15, ty = 2 * (threadIdx.x >> 5) + (threadIdx.x & 1);
     const int slice = blockIdx.z % g.slices, first = g.sum ? 0 : blockIdx.z / g.slices;
     const int terms = g.sum ? g.n : 1;
     const int M = g.p[first].M, N = g.p[first].N, K = g.p[first].K;
@@ -222,7 +223,7 @@ constexpr int kSmallFloats = kSmallStages * 2 * 32 * (32 + kPad);
 template <bool TA, bool TB>
 __device__ __forceinline__ void small_product(const Gemm32Args& g, int tx0, int ty0, int z, float* sm) {
     constexpr int KC = kSmallK, KW = KC / kSmallWarps, LD = 32 + kPad, kTile = 32 * LD, S = kSmallStages;
-    const int warp = threadIdx.x >> 5, tx = threadIdx.x & 7, ty = (threadIdx.x >> 3) & 3;
+    const int warp = threadIdx.x >> 5, tx = (threadIdx.x >> 1) & 7, ty = (threadIdx.x & 1) + 2 * ((threadIdx.x >> 4) & 1);
     const int first = g.sum ? 0 : z, terms = g.sum ? g.n : 1;
     const int M = g.p[first].M, N = g.p[first].N, K = g.p[first].K;
     const int m0 = ty0 * 32, n0 = tx0 * 32;
