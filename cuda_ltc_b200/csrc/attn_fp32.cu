@@ -167,14 +167,14 @@ __device__ __forceinline__ int score_ty() { return 2 * (threadIdx.x >> 5) + (thr
 __device__ __forceinline__ int row_of(int ty) { return ((ty >> 1) & 3) + 4 * (ty & 1) + 8 * (ty >> 3); }
 
 // s[i][j] = A[row i] . B[col j] over DP features
-template <int DP, int NT, int RM, int CN>
+template <int DP, int NT, int RM, int CN, int kUnroll = 2>
 __device__ __forceinline__ void tile_dot(float (&s)[RM][CN], const float* A, const float* B, int row0, int tx) {
     constexpr int LD = DP + kPad, RS = NT / 16;
 #pragma unroll
     for (int i = 0; i < RM; ++i)
 #pragma unroll
         for (int j = 0; j < CN; ++j) s[i][j] = 0.f;
-#pragma unroll 2
+#pragma unroll kUnroll
     for (int d = 0; d < DP; d += 4) {
         float4 b[CN];
 #pragma unroll
@@ -315,35 +315,34 @@ __global__ void __launch_bounds__(NT, TM < 64 ? 4 : DP <= 32 ? 4 : DP <= 64 ? 3 
     load_padded<DP, KN, NT>(Vs, vb, a.vs.seq, 0, a.Sk, a.D, vec);
     cp_async_commit();
 
-    // Dense mask of this thread's scores: bit CN i + j for row i, column j.  The next step's values are read in two
-    // halves, one under each product, and packed behind it.
-    constexpr int RH = RM / 2;
-    static_assert(RM * CN <= 32 && RM % 2 == 0, "one word");
-    const float* mask = kMask ? a.keep_mask + ((int64_t)b * a.Sq + q0 + row0) * a.Sk + tx : nullptr;
-    float mv[RH][CN];
+    // Dense mask: every warp votes its share of the next step's words (32 keys of a row each) in two halves, one read under the
+    // value product, where the scores' registers are free, the other under the wait for the next keys.
+    constexpr int kWords2 = TM / (NT / 32);                               // words of half a warp's rows
+    uint32_t* mask_sm = reinterpret_cast<uint32_t*>(row_scale + TM);      // [TM][2]
+    const int lane = threadIdx.x & 31, mask_row = (threadIdx.x >> 5) * kWords2;
+    float mv[kWords2];
+    static_assert(kWords2 % 2 == 0, "whole rows");
     auto mask_read = [&](int half, int k) {
+        const int r0 = q0 + mask_row + half * (kWords2 / 2);
+        const float* p = a.keep_mask + ((int64_t)b * a.Sq + r0) * a.Sk + k + lane;
 #pragma unroll
-        for (int i = 0; i < RH; ++i)
-#pragma unroll
-            for (int j = 0; j < CN; ++j) {
-                const int r = RS * (half * RH + i);
-                mv[i][j] = (q0 + row0 + r < a.Sq && k + tx + 16 * j < k_end) ? __ldg(mask + (int64_t)r * a.Sk + k + 16 * j) : 0.f;
-            }
+        for (int w = 0; w < kWords2; w += 2, p += a.Sk) {
+            const bool row = r0 + w / 2 < a.Sq;
+            mv[w] = row && k + lane < k_end ? __ldg(p) : 0.f;
+            mv[w + 1] = row && k + 32 + lane < k_end ? __ldg(p + 32) : 0.f;
+        }
     };
-    auto mask_pack = [&](int half) {
-        uint32_t bits = 0;
+    auto mask_vote = [&](int half) {
 #pragma unroll
-        for (int i = 0; i < RH; ++i)
-#pragma unroll
-            for (int j = 0; j < CN; ++j) bits |= (mv[i][j] != 0.f ? 1u : 0u) << (CN * (half * RH + i) + j);
-        return bits;
+        for (int w = 0; w < kWords2; w += 2) {
+            const uint32_t x = __ballot_sync(0xffffffffu, mv[w] != 0.f), y = __ballot_sync(0xffffffffu, mv[w + 1] != 0.f);
+            if (lane == 0) *reinterpret_cast<uint2*>(mask_sm + 2 * mask_row + half * kWords2 + w) = make_uint2(x, y);
+        }
     };
-    uint32_t keep = ~0u;
     if (kMask) {
         mask_read(0, 0);
-        keep = mask_pack(0);
+        mask_vote(0);
         mask_read(1, 0);
-        keep |= mask_pack(1);
     }
 
     const Lt L;
@@ -358,13 +357,11 @@ __global__ void __launch_bounds__(NT, TM < 64 ? 4 : DP <= 32 ? 4 : DP <= 64 ? 3 
 
     for (int k0 = 0; k0 < k_end; k0 += KN) {
         const bool more = k0 + KN < k_end;
-        uint32_t keep_next = 0;
-        if (kMask && more) mask_read(0, k0 + KN);
         cp_async_wait<1>();
+        if (kMask) mask_vote(1);
         __syncthreads();
         float s[RM][CN];
-        tile_dot<DP, NT, RM, CN>(s, Qs, Ks, row0, tx);
-        if (kMask && more) keep_next = mask_pack(0);
+        tile_dot<DP, NT, RM, CN, TM == 64 && (kMask || DP >= 32) ? 1 : 2>(s, Qs, Ks, row0, tx);      // (two at a time spill there)
         const bool all_visible = k0 + KN <= kvlen && !kMask && (!a.causal || k0 + KN - 1 <= q0 + a.causal_off);
 #pragma unroll
         for (int i = 0; i < RM; ++i) {
@@ -373,7 +370,7 @@ __global__ void __launch_bounds__(NT, TM < 64 ? 4 : DP <= 32 ? 4 : DP <= 64 ? 3 
             if (!all_visible) {
                 const int last = a.causal ? min(kvlen - 1, q0 + r + a.causal_off) : kvlen - 1;
                 visible = row_limit<CN>(k0 + tx, last);
-                if (kMask) visible &= keep >> (CN * i);
+                if (kMask) visible &= row_mask<CN>(mask_sm + 2 * r, tx);
             }
             float mt = kNegInf;
 #pragma unroll
@@ -400,9 +397,9 @@ __global__ void __launch_bounds__(NT, TM < 64 ? 4 : DP <= 32 ? 4 : DP <= 64 ? 3 
             m_run[i] = m_new;
             if (tx == 0) row_scale[r] = corr;
         }
-        if (kMask && more) mask_read(1, k0 + KN);
         cp_async_wait<0>();
         __syncthreads();
+        if (kMask && more) mask_read(0, k0 + KN);
         if (more) load_padded<DP, KN, NT>(Ks, kb, a.ks.seq, k0 + KN, a.Sk, a.D, vec);
         cp_async_commit();
         if (L.active) {
@@ -415,7 +412,10 @@ __global__ void __launch_bounds__(NT, TM < 64 ? 4 : DP <= 32 ? 4 : DP <= 64 ? 3 
             }
             accumulate<DP, TM, NT>(acc, L, Ps, LP, Vs, min(KN, (k_end - k0 + 3) & ~3));
         }
-        if (kMask && more) keep = keep_next | mask_pack(1);
+        if (kMask && more) {
+            mask_vote(0);
+            mask_read(1, k0 + KN);
+        }
         __syncthreads();
         if (more) load_padded<DP, KN, NT>(Vs, vb, a.vs.seq, k0 + KN, a.Sk, a.D, vec);
         cp_async_commit();
@@ -809,7 +809,7 @@ int set_smem(ltca_ctx* ctx, K kern, size_t bytes, SmemOptIn& once) {
 template <typename T, int DP, int TM, int NT, bool kMask>
 int run_fwd(ltca_ctx* ctx, const CoreArgs& a) {
     static SmemOptIn once;
-    constexpr size_t smem = ((size_t)(TM + 128) * (DP + kPad) + TM * (64 + kPad) + TM) * sizeof(float);
+    constexpr size_t smem = ((size_t)(TM + 128) * (DP + kPad) + TM * (64 + kPad) + TM + (kMask ? 2 * TM : 0)) * sizeof(float);
     int rc = set_smem(ctx, attn_fwd_fp32_kernel<T, DP, TM, NT, kMask>, smem, once);
     if (rc) return rc;
     dim3 grid((a.Sq + TM - 1) / TM, a.H, a.B);
