@@ -8,8 +8,6 @@
 // and row sums are shuffle reductions.
 #include <math.h>
 
-#include <numeric>
-
 #include "attn_mask.cuh"
 #include "host_common.h"
 #include "sm100_ptx.cuh"
@@ -40,6 +38,8 @@ struct CoreArgs {
     const int32_t* kv_len;
     const uint32_t* mask_bits;  // backward: the dense mask packed, [B, Sq, mask_nw]; null: no room for it
     int mask_nw;
+    float* dq_part;             // one-pass backward: dQ of every key block, [key blocks][pairs of the launch][Sq][part_ld]
+    int part_ld, pair0, pairs;  // (batch, head) pairs of the launch: pair0 .. pair0 + pairs
     // dq kernel: dO is not there yet, it is dy Wo_h^T (see FromOutput); dO's rows are written for the dK/dV kernel
     const float *dy, *wo;
     int64_t dy_batch, dy_seq;
@@ -131,6 +131,7 @@ __device__ __forceinline__ bool key_visible(const CoreArgs& a, int b, int qi, in
 // fewer instructions, but a broadcast 16-byte read takes two wavefronts and the row state leaves two or three warps per
 // scheduler; the same times within 5 % (without the mask forward 41 against 44 us, backward 167 against 162).
 // ----------------------------------------------------------------------------------------------
+constexpr int kOnePassThreads64 = 256;     // threads of the one-pass backward's CTA at DP = 64
 constexpr int kPad = 4;      // floats added to a shared row: neighbouring rows' 16-byte pieces lie in different banks
 
 // Rows [r0, r0 + ROWS) into shared [ROWS][DP + kPad]; see load_tile.
@@ -507,9 +508,8 @@ __device__ __forceinline__ void form_dout(float* dst, const CoreArgs& a, int b, 
 
 // pass 1: delta = rowsum(dO o O), left for pass 2, and dQ.  One CTA per TM query rows, KN keys per step.
 // kForm: dO is formed here (a kernel of its own, since form_dout takes registers: without it twice as many CTAs fit on an SM).
-// kCtas: how many share an SM (their registers); four leave no registers for the rows' deltas.
-template <typename T, int DP, int TM, int KN, int NT, int kMask, bool kForm, int kCtas>
-__global__ void __launch_bounds__(NT, kCtas) attn_bwd_dq_fp32_kernel(const CoreArgs a) {
+template <typename T, int DP, int TM, int KN, int NT, int kMask, bool kForm>
+__global__ void __launch_bounds__(NT, NT == 128 ? 3 : 1) attn_bwd_dq_fp32_kernel(const CoreArgs a) {
     grid_dependency_wait();
     constexpr int LD = DP + kPad, LP = KN + kPad, RS = NT / 16, RM = TM / RS, CN = KN / 16, NW = KN / 32;
     using Lt = AccLayout<DP, TM, NT>;
@@ -568,7 +568,7 @@ __global__ void __launch_bounds__(NT, kCtas) attn_bwd_dq_fp32_kernel(const CoreA
         const int r = row0 + RS * i;
         const float l = q0 + r < a.Sq ? a.lse_in[stat0 + q0 + r] : kNegInf;
         lse[i] = l == kNegInf ? INFINITY : l;
-        if constexpr (kCtas < 4) dlt[i] = row_delta[r];
+        dlt[i] = row_delta[r];
     }
 #pragma unroll
     for (int i = 0; i < Lt::NR; ++i)
@@ -611,7 +611,7 @@ __global__ void __launch_bounds__(NT, kCtas) attn_bwd_dq_fp32_kernel(const CoreA
                 bool zero = !(visible >> j & 1u);
                 if (a.use_clamp && v >= a.clamp) { v = a.clamp; zero = true; }     // the gradient of a clamped score
                 const float p = expf(v - lse[i]);
-                Ss[r * LP + tx + 16 * j] = zero ? 0.f : p * (dp[i][j] - (kCtas < 4 ? dlt[i] : row_delta[r])) * a.scale;
+                Ss[r * LP + tx + 16 * j] = zero ? 0.f : p * (dp[i][j] - dlt[i]) * a.scale;
             }
         }
         __syncthreads();
@@ -639,8 +639,8 @@ __global__ void __launch_bounds__(NT, kCtas) attn_bwd_dq_fp32_kernel(const CoreA
 }
 
 // pass 2: dK and dV.  One CTA per TK keys, QN query rows per step; a thread accumulates NR neighbouring keys.
-template <typename T, int DP, int TK, int QN, int NT, int kMask, int kCtas>
-__global__ void __launch_bounds__(NT, kCtas) attn_bwd_dkv_fp32_kernel(const CoreArgs a) {
+template <typename T, int DP, int TK, int QN, int NT, int kMask>
+__global__ void __launch_bounds__(NT, TK < 64 || DP <= 32 ? 3 : DP <= 64 ? 2 : 1) attn_bwd_dkv_fp32_kernel(const CoreArgs a) {
     grid_dependency_wait();
     constexpr int LD = DP + kPad, LP = TK + kPad, RS = NT / 16, RM = QN / RS, CN = TK / 16, NW = (TK + 31) / 32;
     using Lt = AccLayout<DP, TK, NT>;
@@ -772,6 +772,250 @@ __global__ void __launch_bounds__(NT, kCtas) attn_bwd_dkv_fp32_kernel(const Core
     }
 }
 
+// ----------------------------------------------------------------------------------------------
+// one pass: dK, dV and dQ from one evaluation of the scores and of dP.  One CTA per 64 keys, 64 query rows per step.
+//
+// Five products a tile instead of the seven of the two kernels above.  dQ of a step is this CTA's 64 keys' share of it, written
+// out and added up by attn_bwd_dq_sum_kernel in the order of the keys; a call of 64 keys or fewer writes it where it belongs.
+// P and then dS go through the same shared memory: what a tile holds beside it (K, V, Q, dO) leaves room for four CTAs an SM
+// at head widths up to 32.  A thread reads its own probabilities back for dS, so they take no registers under dP's product.
+// Against the two kernels, us: B16 H8 S250 D32 130 -> 89, causal 109 -> 66, with a dense mask 156 -> 96; B32 H8 S256 D16 143 -> 94;
+// B8 H8 S512 D64 459 -> 323, causal 349 -> 175; one block of keys, B64 H8 S60 D32 43 -> 24.  256 threads at D = 64: 293 us for B32
+// H8 S256, with 128 (a larger block of scores each, half the warps) 318.  What bounds it: issue slots (about 6300 cycles a tile and
+// SM at D = 32) and shared-memory wavefronts (5000), at 16 warps an SM.
+// ----------------------------------------------------------------------------------------------
+template <typename T, int DP, int NT, bool kMask>
+__global__ void __launch_bounds__(NT, DP <= 32 ? 4 : 2) attn_bwd_fp32_kernel(const CoreArgs a) {
+    grid_dependency_wait();
+    constexpr int N = 64, LD = DP + kPad, LP = N + kPad, RS = NT / 16, RM = N / RS, CN = N / 16;
+    constexpr int kPer = NT / N, kOq = DP / (4 * kPer);       // delta: threads of a row, 16-byte pieces of each
+    using Lt = AccLayout<DP, N, NT>;
+    extern __shared__ __align__(16) float sm[];
+    float* Ks = sm;
+    float* Vs = Ks + N * LD;
+    float* Qs = Vs + N * LD;
+    float* Gs = Qs + N * LD;             // dO
+    float* Ps = Gs + N * LD;             // P, then dS
+    float* row_lse = Ps + N * LP;
+    float* row_delta = row_lse + N;
+    uint32_t* mask_sm = reinterpret_cast<uint32_t*>(row_delta + N);      // [N][2]
+    const bool vec = a.vec != 0;
+
+    const int tx = score_tx(), row0 = row_of(score_ty());
+    const int bh = a.pair0 + blockIdx.x, b = bh / a.H, h = bh % a.H;
+    const int k0 = blockIdx.y * N;
+    int kvlen = a.Sk;
+    if (a.kv_len) kvlen = min(max(a.kv_len[b], 0), a.Sk);
+
+    const T* qb = reinterpret_cast<const T*>(a.q) + b * a.qs.batch + h * a.qs.head;
+    const T* kb = reinterpret_cast<const T*>(a.k) + b * a.ks.batch + h * a.ks.head;
+    const T* vb = reinterpret_cast<const T*>(a.v) + b * a.vs.batch + h * a.vs.head;
+    const T* gb = reinterpret_cast<const T*>(a.dout) + b * a.dos.batch + h * a.dos.head;
+    const T* ob = reinterpret_cast<const T*>(a.o_in) + b * a.os.batch + h * a.os.head;
+    load_padded<DP, N, NT>(Ks, kb, a.ks.seq, k0, a.Sk, a.D, vec);
+    load_padded<DP, N, NT>(Vs, vb, a.vs.seq, k0, a.Sk, a.D, vec);
+
+    const Lt L;
+    f32x2 acck[Lt::NR][2 * Lt::CG], accv[Lt::NR][2 * Lt::CG];
+#pragma unroll
+    for (int i = 0; i < Lt::NR; ++i)
+#pragma unroll
+        for (int c = 0; c < 2 * Lt::CG; ++c) { acck[i][c] = 0ull; accv[i][c] = 0ull; }
+
+    const int64_t stat0 = (int64_t)bh * a.Sq;
+    // first query row that can see key k0 (causal): qi >= k0 - causal_off
+    const int q_begin = a.causal ? max(0, k0 - a.causal_off) / N * N : 0;
+    const int q_end = k0 < kvlen ? a.Sq : 0;
+    for (int q0 = q_begin; q0 < q_end; q0 += N) {
+        load_padded<DP, N, NT>(Qs, qb, a.qs.seq, q0, a.Sq, a.D, vec);
+        load_padded<DP, N, NT>(Gs, gb, a.dos.seq, q0, a.Sq, a.D, vec);
+        cp_async_commit();
+        const int dr = threadIdx.x / kPer, dc = 4 * (threadIdx.x % kPer);
+        float4 orow[kOq];
+#pragma unroll
+        for (int i = 0; i < kOq; ++i) {
+            const int c = dc + 4 * kPer * i;
+            orow[i] = q0 + dr < a.Sq ? row4(ob + (int64_t)(q0 + dr) * a.os.seq, c, a.D, vec) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        if (threadIdx.x < N) {
+            // rows without visible keys and rows beyond the tensor: lse = +inf, probabilities 0
+            const int qi = q0 + threadIdx.x;
+            const float l = qi < a.Sq ? a.lse_in[stat0 + qi] : kNegInf;
+            row_lse[threadIdx.x] = l == kNegInf ? INFINITY : l;
+        }
+        if (kMask && threadIdx.x < 2 * N) {
+            const int qi = q0 + threadIdx.x / 2, kw = k0 / 32 + threadIdx.x % 2;
+            mask_sm[threadIdx.x] = a.mask_bits ? mask_word<kWords>(a, b, qi, kw) : mask_word<kDense>(a, b, qi, kw);
+        }
+        cp_async_wait<0>();
+        __syncthreads();
+        {   // delta = rowsum(dO o O)
+            float4 e = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int i = 0; i < kOq; ++i) {
+                const float4 g = *reinterpret_cast<const float4*>(Gs + dr * LD + dc + 4 * kPer * i);
+                e.x = fmaf(orow[i].x, g.x, e.x); e.y = fmaf(orow[i].y, g.y, e.y);
+                e.z = fmaf(orow[i].z, g.z, e.z); e.w = fmaf(orow[i].w, g.w, e.w);
+            }
+            float d = (e.x + e.y) + (e.z + e.w);
+#pragma unroll
+            for (int o = kPer / 2; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+            if (threadIdx.x % kPer == 0) row_delta[dr] = d;
+        }
+        const bool all_visible = k0 + N <= kvlen && !kMask && (!a.causal || k0 + N - 1 <= q0 + a.causal_off);
+        uint32_t dead = 0;               // scores whose gradient is 0: hidden or clamped ones, bit CN i + j
+        {
+            float s[RM][CN];
+            tile_dot<DP, NT, RM, CN>(s, Qs, Ks, row0, tx);
+#pragma unroll
+            for (int i = 0; i < RM; ++i) {
+                const int r = row0 + RS * i;
+                const float lse = row_lse[r];
+                uint32_t visible = ~0u;
+                if (!all_visible) {
+                    const int last = a.causal ? min(kvlen - 1, q0 + r + a.causal_off) : kvlen - 1;
+                    visible = row_limit<CN>(k0 + tx, last);
+                    if (kMask) visible &= row_mask<CN>(mask_sm + 2 * r, tx);
+                }
+#pragma unroll
+                for (int j = 0; j < CN; ++j) {
+                    float v = s[i][j] * a.scale;
+                    bool hidden = !(visible >> j & 1u), zero = hidden;
+                    if (a.use_clamp && v >= a.clamp) { v = a.clamp; zero = true; }     // the gradient of a clamped score
+                    const float p = expf(v - lse);
+                    Ps[r * LP + tx + 16 * j] = hidden ? 0.f : p;
+                    dead |= (zero ? 1u : 0u) << (CN * i + j);
+                }
+            }
+        }
+        __syncthreads();
+        const int n = min(N, a.Sq - q0);
+        if (L.active) {
+#pragma unroll 4
+            for (int r = 0; r < n; ++r) {
+                float pp[Lt::NR];
+                ld_row<Lt::NR>(pp, Ps + r * LP + Lt::NR * L.ty);
+#pragma unroll
+                for (int c = 0; c < Lt::CG; ++c) {
+                    const ulonglong2 g = *reinterpret_cast<const ulonglong2*>(Gs + r * LD + 4 * L.tx + 64 * c);
+#pragma unroll
+                    for (int i = 0; i < Lt::NR; ++i) {
+                        const f32x2 pw = pair(pp[i], pp[i]);
+                        accv[i][2 * c] = fma2(pw, g.x, accv[i][2 * c]);
+                        accv[i][2 * c + 1] = fma2(pw, g.y, accv[i][2 * c + 1]);
+                    }
+                }
+            }
+        }
+        {
+            float dp[RM][CN];
+            tile_dot<DP, NT, RM, CN>(dp, Gs, Vs, row0, tx);
+            __syncthreads();
+#pragma unroll
+            for (int i = 0; i < RM; ++i) {
+                const int r = row0 + RS * i;
+                const float dlt = row_delta[r];
+#pragma unroll
+                for (int j = 0; j < CN; ++j) {
+                    float* x = Ps + r * LP + tx + 16 * j;
+                    *x = dead >> (CN * i + j) & 1u ? 0.f : *x * (dp[i][j] - dlt) * a.scale;
+                }
+            }
+        }
+        __syncthreads();
+        if (L.active) {
+#pragma unroll 4
+            for (int r = 0; r < n; ++r) {
+                float dd[Lt::NR];
+                ld_row<Lt::NR>(dd, Ps + r * LP + Lt::NR * L.ty);
+#pragma unroll
+                for (int c = 0; c < Lt::CG; ++c) {
+                    const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(Qs + r * LD + 4 * L.tx + 64 * c);
+#pragma unroll
+                    for (int i = 0; i < Lt::NR; ++i) {
+                        const f32x2 dw = pair(dd[i], dd[i]);
+                        acck[i][2 * c] = fma2(dw, q.x, acck[i][2 * c]);
+                        acck[i][2 * c + 1] = fma2(dw, q.y, acck[i][2 * c + 1]);
+                    }
+                }
+            }
+            f32x2 acc[Lt::NR][2 * Lt::CG];
+#pragma unroll
+            for (int i = 0; i < Lt::NR; ++i)
+#pragma unroll
+                for (int c = 0; c < 2 * Lt::CG; ++c) acc[i][c] = 0ull;
+            int k_end = kvlen;                                // no row of the tile sees a key beyond it
+            if (a.causal) k_end = min(k_end, min(q0 + N - 1, a.Sq - 1) + a.causal_off + 1);
+            accumulate<DP, N, NT>(acc, L, Ps, LP, Ks, min(N, (k_end - k0 + 3) & ~3));
+#pragma unroll
+            for (int i = 0; i < Lt::NR; ++i) {
+                const int qi = q0 + L.ty + Lt::TY * i;
+                if (qi >= a.Sq) continue;
+#pragma unroll
+                for (int c = 0; c < Lt::CG; ++c) {
+                    const int col = 4 * L.tx + 64 * c;
+                    const float2 x = halves(acc[i][2 * c]), y = halves(acc[i][2 * c + 1]);
+                    const float4 v = make_float4(x.x, x.y, y.x, y.y);
+                    if (a.dq_part) {
+                        if (col < a.part_ld)
+                            *reinterpret_cast<float4*>(a.dq_part + (((int64_t)blockIdx.y * a.pairs + blockIdx.x) * a.Sq + qi) * a.part_ld + col) = v;
+                    } else {
+                        T* dqb = reinterpret_cast<T*>(a.dq) + b * a.dqs.batch + h * a.dqs.head;
+                        store4(dqb + (int64_t)qi * a.dqs.seq, col, a.D, v, vec);
+                    }
+                }
+            }
+        }
+        __syncthreads();
+    }
+    cp_async_wait<0>();
+    if (!a.dq_part) {                    // rows that see none of the keys
+        T* dqb = reinterpret_cast<T*>(a.dq) + b * a.dqs.batch + h * a.dqs.head;
+        const int rows = q_end > 0 ? min(q_begin, a.Sq) : a.Sq;
+        for (int e = threadIdx.x; e < rows * (DP / 4); e += NT)
+            store4(dqb + (int64_t)(e / (DP / 4)) * a.dqs.seq, 4 * (e % (DP / 4)), a.D, make_float4(0.f, 0.f, 0.f, 0.f), vec);
+    }
+    if (!L.active) return;
+    T* dkb = reinterpret_cast<T*>(a.dk) + b * a.dks.batch + h * a.dks.head;
+    T* dvb = reinterpret_cast<T*>(a.dv) + b * a.dvs.batch + h * a.dvs.head;
+#pragma unroll
+    for (int i = 0; i < Lt::NR; ++i) {
+        const int kj = k0 + Lt::NR * L.ty + i;
+        if (kj >= a.Sk) continue;
+#pragma unroll
+        for (int c = 0; c < Lt::CG; ++c) {
+            const float2 x = halves(acck[i][2 * c]), y = halves(acck[i][2 * c + 1]);
+            const float2 u = halves(accv[i][2 * c]), w = halves(accv[i][2 * c + 1]);
+            store4(dkb + (int64_t)kj * a.dks.seq, 4 * L.tx + 64 * c, a.D, make_float4(x.x, x.y, y.x, y.y), vec);
+            store4(dvb + (int64_t)kj * a.dvs.seq, 4 * L.tx + 64 * c, a.D, make_float4(u.x, u.y, w.x, w.y), vec);
+        }
+    }
+}
+
+// dQ = the sum of the key blocks' shares, in the order of the keys; a block that no row of a 64-row tile sees left none.
+template <typename T>
+__global__ void __launch_bounds__(256) attn_bwd_dq_sum_kernel(const CoreArgs a) {
+    grid_dependency_wait();
+    const int quads = a.part_ld / 4;
+    const int64_t total = (int64_t)a.pairs * a.Sq * quads, step = total * 4;
+    for (int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x; e < total; e += (int64_t)gridDim.x * 256) {
+        const int64_t row = e / quads;
+        const int c = 4 * (int)(e - row * quads), qi = (int)(row % a.Sq), bh = a.pair0 + (int)(row / a.Sq);
+        const int b = bh / a.H, h = bh % a.H;
+        int keys = a.Sk;
+        if (a.kv_len) keys = min(max(a.kv_len[b], 0), a.Sk);
+        if (a.causal) keys = min(keys, qi / 64 * 64 + 64 + a.causal_off);
+        const float* src = a.dq_part + 4 * e;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+        for (int k = 0; k < keys; k += 64, src += step) {
+            const float4 x = *reinterpret_cast<const float4*>(src);
+            v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w;
+        }
+        store4(reinterpret_cast<T*>(a.dq) + b * a.dqs.batch + h * a.dqs.head + (int64_t)qi * a.dqs.seq, c, a.D, v, a.vec != 0);
+    }
+}
+
 CoreArgs make_args(const ltca_attn_params* p) {
     CoreArgs a;
     memset(&a, 0, sizeof(a));
@@ -817,36 +1061,32 @@ int run_fwd(ltca_ctx* ctx, const CoreArgs& a) {
     return LTCA_OK;
 }
 
-// Whether four CTAs of that much dynamic shared memory are resident on one SM at once.
-constexpr bool four_fit_sm(size_t smem) { return 4 * (smem + 1024) <= 228 * 1024; }
-
-template <typename T, int DP, int TM, int KN, int NT, int kMask, bool kForm = false, int kCtas = NT == 128 ? 3 : 1>
+template <typename T, int DP, int TM, int KN, int NT, int kMask, bool kForm = false>
 int run_dq(ltca_ctx* ctx, const CoreArgs& a) {
     static SmemOptIn once;
     constexpr size_t smem = ((size_t)(2 * TM + 2 * KN) * (DP + kPad) + TM * (KN + kPad) + TM) * sizeof(float);
-    static_assert(kCtas != 4 || four_fit_sm(smem), "four CTAs to an SM");
-    int rc = set_smem(ctx, attn_bwd_dq_fp32_kernel<T, DP, TM, KN, NT, kMask, kForm, kCtas>, smem, once);
+    int rc = set_smem(ctx, attn_bwd_dq_fp32_kernel<T, DP, TM, KN, NT, kMask, kForm>, smem, once);
     if (rc) return rc;
     dim3 grid((a.Sq + TM - 1) / TM, a.H, a.B);
-    LTCA_CUDA_OK(ctx, launch_dependent(attn_bwd_dq_fp32_kernel<T, DP, TM, KN, NT, kMask, kForm, kCtas>, grid, dim3(NT), smem, ctx->stream, a));
+    LTCA_CUDA_OK(ctx, launch_dependent(attn_bwd_dq_fp32_kernel<T, DP, TM, KN, NT, kMask, kForm>, grid, dim3(NT), smem, ctx->stream, a));
     return LTCA_OK;
 }
-template <typename T, int DP, int TK, int QN, int NT, int kMask, int kCtas = TK < 64 || DP <= 32 ? 3 : DP <= 64 ? 2 : 1>
+template <typename T, int DP, int TK, int QN, int NT, int kMask>
 int run_dkv(ltca_ctx* ctx, const CoreArgs& a) {
     static SmemOptIn once;
     constexpr size_t smem = ((size_t)(2 * TK + 2 * QN) * (DP + kPad) + 2 * QN * (TK + kPad) + 2 * QN) * sizeof(float);
-    static_assert(kCtas != 4 || four_fit_sm(smem), "four CTAs to an SM");
-    int rc = set_smem(ctx, attn_bwd_dkv_fp32_kernel<T, DP, TK, QN, NT, kMask, kCtas>, smem, once);
+    int rc = set_smem(ctx, attn_bwd_dkv_fp32_kernel<T, DP, TK, QN, NT, kMask>, smem, once);
     if (rc) return rc;
     dim3 grid((a.Sk + TK - 1) / TK, a.H, a.B);
-    LTCA_CUDA_OK(ctx, launch_dependent(attn_bwd_dkv_fp32_kernel<T, DP, TK, QN, NT, kMask, kCtas>, grid, dim3(NT), smem, ctx->stream, a));
+    LTCA_CUDA_OK(ctx, launch_dependent(attn_bwd_dkv_fp32_kernel<T, DP, TK, QN, NT, kMask>, grid, dim3(NT), smem, ctx->stream, a));
     return LTCA_OK;
 }
 
 // (None of these kernels lets the next one's CTAs be placed before it ends: released at the start, or when the tile loop is
 // done, they take whatever slots are left and sit unevenly on the SMs, 82 or 62 us instead of 57 for B16 H8 S100 D32.)
 // Tiles of 64 rows reuse what they load most; where they would leave SMs idle, tiles of 16 rows give four times the CTAs
-// and a quarter of the serial work.
+// and a quarter of the serial work.  The two-kernel backward's 64-row tiles are left for heads above 64 and for calls whose
+// workspace has no room for dQ's shares.
 template <typename T, int DP, int kMask>
 int run_small_dq(ltca_ctx* ctx, const CoreArgs& a) {
     if constexpr (sizeof(T) == 4 && DP <= 64) {
@@ -855,30 +1095,33 @@ int run_small_dq(ltca_ctx* ctx, const CoreArgs& a) {
     return run_dq<T, DP, 16, 32, 128, kMask>(ctx, a);
 }
 bool fills_sms(const ltca_ctx* ctx, int B, int H, int S) { return (int64_t)B * H * ((S + 63) / 64) >= ctx->sm_device; }
-// Whether the 64-row backward tiles of a narrow head go four to an SM, in 128 registers a thread, instead of three.  (Figures:
-// backward, us, three and four.)
-//   - Tiles of one length: where that saves a wave.  B16 H8 S250 D32 151 and 135, B32 H8 S512 D32 878 and 857, B64 H8 S64 D16
-//     47 and 33; without a wave saved B12 H8 S400 D32 275 and 291, with a dense mask at D16 215 and 223.  Two tiles to a causal
-//     pair count as one length: B32 H8 S128 causal D16 59 and 52, D32 74 and 69.
-//   - Longer causal rows: what three to an SM even out as they go, four to an SM start side by side, and an SM takes about every
-//     sm_device-th tile, which is a pair's same tile over and over where that number and the tiles of a pair have a divisor in
-//     common (B16 H8 S256 D16 87 and 91, D32 115 and 118; B8 H8 S512 D32 193 and 204).  So where they have none and more
-//     than a few tiles are left over by three (B14 H8 S320 D16 109 and 92, D32 149 and 138; B12 H8 S448 D32 227 and 221; four
-//     left over, B8 H8 S448, 153 and 161), or where an SM has more than five tiles (B24 H8 S256 D16 117 and 111, D32 157 and 157;
-//     B64 H8 S512 D16 784 and 729, D32 1090 and 1062).
-//   - Key lengths, each pair's own: from five tiles on at the narrowest heads (uniform lengths, B32 H8 S256 D16 129 and 111; B10
-//     H8 S384 D16 109 and 120); three at others (B32 H8 S256 D32 180 and 183).
-bool four_tiles(const ltca_ctx* ctx, const CoreArgs& a, bool narrowest) {
-    const int64_t sms = ctx->sm_device, per_pair = ((a.Sq < a.Sk ? a.Sq : a.Sk) + 63) / 64, n = (int64_t)a.B * a.H * per_pair;
-    const bool many = n > 5 * sms;
-    if (a.kv_len) return many && narrowest;
-    if (a.causal && per_pair > 2) return many || (5 * n > 16 * sms && std::gcd(per_pair, sms) == 1);
-    return (n + 4 * sms - 1) / (4 * sms) < (n + 3 * sms - 1) / (3 * sms);
+// The one-pass backward, in as many launches as the room for dQ's shares allows.
+template <typename T, int DP, bool kMask>
+int run_one_pass(ltca_ctx* ctx, CoreArgs a) {
+    static SmemOptIn once;
+    constexpr int NT = DP <= 32 ? 128 : kOnePassThreads64;
+    constexpr size_t smem = ((size_t)4 * 64 * (DP + kPad) + 64 * (64 + kPad) + 2 * 64 + (kMask ? 2 * 64 : 0)) * sizeof(float);
+    int rc = set_smem(ctx, attn_bwd_fp32_kernel<T, DP, NT, kMask>, smem, once);
+    if (rc) return rc;
+    const int all = a.B * a.H, most = a.pairs;
+    for (a.pair0 = 0; a.pair0 < all; a.pair0 += most) {
+        a.pairs = all - a.pair0 < most ? all - a.pair0 : most;
+        const dim3 grid(a.pairs, (a.Sk + 63) / 64);
+        LTCA_CUDA_OK(ctx, launch_dependent(attn_bwd_fp32_kernel<T, DP, NT, kMask>, grid, dim3(NT), smem, ctx->stream, a));
+        if (!a.dq_part) continue;
+        const int64_t blocks = ((int64_t)a.pairs * a.Sq * (a.part_ld / 4) + 255) / 256, limit = 16ll * ctx->sm_device;
+        const dim3 rg((unsigned)(blocks < limit ? blocks : limit));
+        LTCA_CUDA_OK(ctx, launch_dependent(attn_bwd_dq_sum_kernel<T>, rg, dim3(256), 0, ctx->stream, a));
+    }
+    return LTCA_OK;
 }
 template <typename T, int DP, bool kMask>
 int run_rows(ltca_ctx* ctx, const CoreArgs& a, bool bwd) {
     auto fills = [&](int S) { return fills_sms(ctx, a.B, a.H, S); };
     constexpr int NT = DP > 64 ? 256 : 128;         // at DP = 128 eight columns per thread need the wider CTA
+    if constexpr (DP <= 64) {
+        if (bwd && a.pairs) return run_one_pass<T, DP, kMask>(ctx, a);
+    }
     if (!bwd) return fills(a.Sq) ? run_fwd<T, DP, 64, NT, kMask>(ctx, a) : run_fwd<T, DP, 16, 128, kMask>(ctx, a);
     int rc;
     if constexpr (kMask) {
@@ -886,15 +1129,6 @@ int run_rows(ltca_ctx* ctx, const CoreArgs& a, bool bwd) {
         if (!a.mask_bits) return (rc = run_small_dq<T, DP, kDense>(ctx, a)) ? rc : run_dkv<T, DP, 16, 32, 128, kDense>(ctx, a);
     }
     constexpr int kM = kMask ? kWords : kNoMask;
-    // Four tiles to an SM for the narrowest heads (D16), and for dQ up to D32: the shared memory of four dK/dV tiles is more than
-    // an SM's there, and in 128 registers three of them are slower (B16 H8 S250 D32 139 us, in 168 136).  With a dense mask at
-    // D32 the words do not fit the registers either (B20 H16 S100 D24 120 and 132).
-    if constexpr (DP <= 16 || (DP <= 32 && kM == kNoMask)) {
-        if (four_tiles(ctx, a, DP <= 16)) {
-            if ((rc = run_dq<T, DP, 64, 64, NT, kM, false, 4>(ctx, a))) return rc;
-            return run_dkv<T, DP, 64, 64, NT, kM, DP <= 16 ? 4 : 3>(ctx, a);
-        }
-    }
     if ((rc = fills(a.Sq) ? run_dq<T, DP, 64, 64, NT, kM>(ctx, a) : run_small_dq<T, DP, kM>(ctx, a))) return rc;
     return fills(a.Sk) ? run_dkv<T, DP, 64, 64, NT, kM>(ctx, a) : run_dkv<T, DP, 16, 32, 128, kM>(ctx, a);
 }
@@ -1111,8 +1345,28 @@ int dispatch(ltca_ctx* ctx, const CoreArgs& a, bool bwd) {
 
 // delta, and the dense mask as bits (the kernels for head_dim up to 128)
 static size_t delta_bytes(const ltca_attn_params* p) { return align_up((size_t)p->B * p->H * p->Sq * sizeof(float), 256); }
+// dQ's shares in the one-pass backward, one per 64 keys: all pairs' up to kPartBytes, as many pairs' as fit in that beyond it
+// (several launches), none where one pair's take more.  Keys of one block need none.
+constexpr size_t kPartBytes = 512u << 20;
+struct OnePass {
+    int pairs = 0;       // (batch, head) pairs a launch; 0: not for the one-pass kernel
+    int ld = 0;
+    size_t bytes = 0;
+};
+static OnePass one_pass(const ltca_attn_params* p) {
+    OnePass o;
+    if (p->D > 64) return o;
+    const int64_t all = (int64_t)p->B * p->H, blocks = ((int64_t)p->Sk + 63) / 64;
+    o.ld = (p->D + 3) / 4 * 4;
+    const size_t one = (size_t)blocks * p->Sq * o.ld * sizeof(float);
+    if (blocks > 1 && one > kPartBytes) return o;
+    const int64_t fit = blocks > 1 ? (int64_t)(kPartBytes / one) : all;
+    o.pairs = (int)(fit < all ? fit : all);
+    o.bytes = blocks > 1 ? o.pairs * one : 0;
+    return o;
+}
 size_t attn_bwd_fp32_workspace(const ltca_attn_params* p) {
-    return delta_bytes(p) + (p->D <= 128 ? mask_words_bytes(p) : 0);
+    return delta_bytes(p) + (p->D <= 128 ? mask_words_bytes(p) + one_pass(p).bytes : 0);
 }
 
 int launch_attn_fwd_fp32(ltca_ctx* ctx, const ltca_attn_params* p) {
@@ -1140,8 +1394,18 @@ int launch_attn_bwd_fp32(ltca_ctx* ctx, const ltca_attn_params* p, const FromOut
         a.dy_batch = from->batch; a.dy_seq = from->seq;
     }
     if (p->D <= 128) {
+        // delta, dQ's shares, the mask's words; a workspace without room for the shares takes the two kernels, one without room for
+        // the words (sized without the mask) reads the mask as it is
+        const OnePass one = one_pass(p);
+        const bool room = one.pairs && !from && p->workspace_bytes >= delta_bytes(p) + one.bytes;
+        const size_t used = delta_bytes(p) + (room ? one.bytes : 0);
+        if (room && fills_sms(ctx, p->B, p->H, p->Sq < p->Sk ? p->Sq : p->Sk)) {
+            a.pairs = one.pairs;
+            a.part_ld = one.ld;
+            a.dq_part = one.bytes ? reinterpret_cast<float*>(reinterpret_cast<char*>(p->workspace) + delta_bytes(p)) : nullptr;
+        }
         const void* words = nullptr;
-        if (int rc = mask_words_of(ctx, p, delta_bytes(p), &words)) return rc;
+        if (int rc = mask_words_of(ctx, p, used, &words)) return rc;
         const MaskArgs m = mask_args(p, words);
         a.mask_bits = m.by_query;
         a.mask_nw = m.nk;
