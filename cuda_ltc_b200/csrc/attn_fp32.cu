@@ -40,7 +40,7 @@ struct CoreArgs {
     int mask_nw;
     float* dq_part;             // one-pass backward: dQ of every key block, [key blocks][pairs of the launch][Sq][part_ld]
     int part_ld, pair0, pairs;  // (batch, head) pairs of the launch: pair0 .. pair0 + pairs
-    // dq kernel: dO is not there yet, it is dy Wo_h^T (see FromOutput); dO's rows are written for the dK/dV kernel
+    // dO is not there yet, it is dy Wo_h^T (see FromOutput); the two-kernel backward's first kernel writes dO's rows for the second
     const float *dy, *wo;
     int64_t dy_batch, dy_seq;
     int E;
@@ -476,8 +476,8 @@ __global__ void attn_bwd_delta_kernel(const CoreArgs a) {
 // ----------------------------------------------------------------------------------------------
 // dst[r][c] = dO[r0 + r][c] = sum over e of dy[r0 + r][e] Wo[h D + c][e], e ascending as in the product that this replaces, also
 // written to dO's rows.  A thread keeps a row of Wo's head for its column c and goes down the tile's rows, whose dy its warp
-// reads at one address.
-template <int DP, int ROWS, int NT>
+// reads at one address.  kRows: dO's rows are written as well.
+template <int DP, int ROWS, int NT, bool kRows>
 __device__ __forceinline__ void form_dout(float* dst, const CoreArgs& a, int b, int h, int r0) {
     constexpr int LD = DP + kPad, RT = NT / DP, NR = ROWS / RT;
     const int c = threadIdx.x % DP, rt = threadIdx.x / DP;
@@ -502,7 +502,7 @@ __device__ __forceinline__ void form_dout(float* dst, const CoreArgs& a, int b, 
         const int r = rt + RT * i;
         const bool in = r0 + r < a.Sq && c < a.D;
         dst[r * LD + c] = in ? g[i] : 0.f;
-        if (in) out[(int64_t)(r0 + r) * a.dos.seq] = g[i];
+        if (kRows && in) out[(int64_t)(r0 + r) * a.dos.seq] = g[i];
     }
 }
 
@@ -538,7 +538,7 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 3 : 1) attn_bwd_dq_fp32_kernel
     load_padded<DP, KN, NT>(Ks, kb, a.ks.seq, 0, a.Sk, a.D, vec);
     load_padded<DP, KN, NT>(Vs, vb, a.vs.seq, 0, a.Sk, a.D, vec);
     cp_async_commit();
-    if constexpr (kForm) form_dout<DP, TM, NT>(Gs, a, b, h, q0);
+    if constexpr (kForm) form_dout<DP, TM, NT, true>(Gs, a, b, h, q0);
     cp_async_wait<0>();
     __syncthreads();
 
@@ -784,10 +784,10 @@ __global__ void __launch_bounds__(NT, TK < 64 || DP <= 32 ? 3 : DP <= 64 ? 2 : 1
 // H8 S256, with 128 (a larger block of scores each, half the warps) 318.  What bounds it: issue slots (about 6300 cycles a tile and
 // SM at D = 32) and shared-memory wavefronts (5000), at 16 warps an SM.
 // ----------------------------------------------------------------------------------------------
-template <typename T, int DP, int NT, bool kMask>
-__global__ void __launch_bounds__(NT, DP <= 32 ? 4 : 2) attn_bwd_fp32_kernel(const CoreArgs a) {
+template <typename T, int DP, int N, int NT, bool kMask, bool kForm>
+__global__ void __launch_bounds__(NT, kForm ? 256 / NT : DP <= 32 ? 4 : 2) attn_bwd_fp32_kernel(const CoreArgs a) {
     grid_dependency_wait();
-    constexpr int N = 64, LD = DP + kPad, LP = N + kPad, RS = NT / 16, RM = N / RS, CN = N / 16;
+    constexpr int LD = DP + kPad, LP = N + kPad, RS = NT / 16, RM = N / RS, CN = N / 16, NW = N / 32;
     constexpr int kPer = NT / N, kOq = DP / (4 * kPer);       // delta: threads of a row, 16-byte pieces of each
     using Lt = AccLayout<DP, N, NT>;
     extern __shared__ __align__(16) float sm[];
@@ -798,7 +798,7 @@ __global__ void __launch_bounds__(NT, DP <= 32 ? 4 : 2) attn_bwd_fp32_kernel(con
     float* Ps = Gs + N * LD;             // P, then dS
     float* row_lse = Ps + N * LP;
     float* row_delta = row_lse + N;
-    uint32_t* mask_sm = reinterpret_cast<uint32_t*>(row_delta + N);      // [N][2]
+    uint32_t* mask_sm = reinterpret_cast<uint32_t*>(row_delta + N);      // [N][NW]
     const bool vec = a.vec != 0;
 
     const int tx = score_tx(), row0 = row_of(score_ty());
@@ -828,7 +828,7 @@ __global__ void __launch_bounds__(NT, DP <= 32 ? 4 : 2) attn_bwd_fp32_kernel(con
     const int q_end = k0 < kvlen ? a.Sq : 0;
     for (int q0 = q_begin; q0 < q_end; q0 += N) {
         load_padded<DP, N, NT>(Qs, qb, a.qs.seq, q0, a.Sq, a.D, vec);
-        load_padded<DP, N, NT>(Gs, gb, a.dos.seq, q0, a.Sq, a.D, vec);
+        if constexpr (!kForm) load_padded<DP, N, NT>(Gs, gb, a.dos.seq, q0, a.Sq, a.D, vec);
         cp_async_commit();
         const int dr = threadIdx.x / kPer, dc = 4 * (threadIdx.x % kPer);
         float4 orow[kOq];
@@ -843,10 +843,11 @@ __global__ void __launch_bounds__(NT, DP <= 32 ? 4 : 2) attn_bwd_fp32_kernel(con
             const float l = qi < a.Sq ? a.lse_in[stat0 + qi] : kNegInf;
             row_lse[threadIdx.x] = l == kNegInf ? INFINITY : l;
         }
-        if (kMask && threadIdx.x < 2 * N) {
-            const int qi = q0 + threadIdx.x / 2, kw = k0 / 32 + threadIdx.x % 2;
+        if (kMask && threadIdx.x < NW * N) {
+            const int qi = q0 + threadIdx.x / NW, kw = k0 / 32 + threadIdx.x % NW;
             mask_sm[threadIdx.x] = a.mask_bits ? mask_word<kWords>(a, b, qi, kw) : mask_word<kDense>(a, b, qi, kw);
         }
+        if constexpr (kForm) form_dout<DP, N, NT, false>(Gs, a, b, h, q0);
         cp_async_wait<0>();
         __syncthreads();
         {   // delta = rowsum(dO o O)
@@ -875,7 +876,7 @@ __global__ void __launch_bounds__(NT, DP <= 32 ? 4 : 2) attn_bwd_fp32_kernel(con
                 if (!all_visible) {
                     const int last = a.causal ? min(kvlen - 1, q0 + r + a.causal_off) : kvlen - 1;
                     visible = row_limit<CN>(k0 + tx, last);
-                    if (kMask) visible &= row_mask<CN>(mask_sm + 2 * r, tx);
+                    if (kMask) visible &= row_mask<CN>(mask_sm + NW * r, tx);
                 }
 #pragma unroll
                 for (int j = 0; j < CN; ++j) {
@@ -1096,24 +1097,32 @@ int run_small_dq(ltca_ctx* ctx, const CoreArgs& a) {
 }
 bool fills_sms(const ltca_ctx* ctx, int B, int H, int S) { return (int64_t)B * H * ((S + 63) / 64) >= ctx->sm_device; }
 // The one-pass backward, in as many launches as the room for dQ's shares allows.
-template <typename T, int DP, bool kMask>
-int run_one_pass(ltca_ctx* ctx, CoreArgs a) {
+template <typename T, int DP, int N, int NT, bool kMask, bool kForm = false>
+int launch_one_pass(ltca_ctx* ctx, CoreArgs a) {
     static SmemOptIn once;
-    constexpr int NT = DP <= 32 ? 128 : kOnePassThreads64;
-    constexpr size_t smem = ((size_t)4 * 64 * (DP + kPad) + 64 * (64 + kPad) + 2 * 64 + (kMask ? 2 * 64 : 0)) * sizeof(float);
-    int rc = set_smem(ctx, attn_bwd_fp32_kernel<T, DP, NT, kMask>, smem, once);
+    constexpr size_t smem = ((size_t)4 * N * (DP + kPad) + N * (N + kPad) + 2 * N + (kMask ? N * N / 32 : 0)) * sizeof(float);
+    int rc = set_smem(ctx, attn_bwd_fp32_kernel<T, DP, N, NT, kMask, kForm>, smem, once);
     if (rc) return rc;
     const int all = a.B * a.H, most = a.pairs;
     for (a.pair0 = 0; a.pair0 < all; a.pair0 += most) {
         a.pairs = all - a.pair0 < most ? all - a.pair0 : most;
-        const dim3 grid(a.pairs, (a.Sk + 63) / 64);
-        LTCA_CUDA_OK(ctx, launch_dependent(attn_bwd_fp32_kernel<T, DP, NT, kMask>, grid, dim3(NT), smem, ctx->stream, a));
+        const dim3 grid(a.pairs, (a.Sk + N - 1) / N);
+        LTCA_CUDA_OK(ctx, launch_dependent(attn_bwd_fp32_kernel<T, DP, N, NT, kMask, kForm>, grid, dim3(NT), smem, ctx->stream, a));
         if (!a.dq_part) continue;
         const int64_t blocks = ((int64_t)a.pairs * a.Sq * (a.part_ld / 4) + 255) / 256, limit = 16ll * ctx->sm_device;
         const dim3 rg((unsigned)(blocks < limit ? blocks : limit));
         LTCA_CUDA_OK(ctx, launch_dependent(attn_bwd_dq_sum_kernel<T>, rg, dim3(256), 0, ctx->stream, a));
     }
     return LTCA_OK;
+}
+// Key blocks of 64, or of 32 where that holds all keys: a quarter of a tile's scores (B16 H8 S16: D16 6.7 -> 3.8 us, D32 9.1 -> 4.6).
+template <typename T, int DP, bool kMask>
+int run_one_pass(ltca_ctx* ctx, const CoreArgs& a) {
+    constexpr int NT = DP <= 32 ? 128 : kOnePassThreads64;
+    if constexpr (sizeof(T) == 4) {
+        if (a.dy) return launch_one_pass<T, DP, 32, 128, kMask, true>(ctx, a);
+    }
+    return a.Sk <= 32 ? launch_one_pass<T, DP, 32, 128, kMask>(ctx, a) : launch_one_pass<T, DP, 64, NT, kMask>(ctx, a);
 }
 template <typename T, int DP, bool kMask>
 int run_rows(ltca_ctx* ctx, const CoreArgs& a, bool bwd) {
@@ -1365,6 +1374,15 @@ static OnePass one_pass(const ltca_attn_params* p) {
     o.bytes = blocks > 1 ? o.pairs * one : 0;
     return o;
 }
+// Where one pass over the scores is the faster one.  A CTA walks all queries of its 64 keys: with few CTAs that chain is longer than
+// that of the two kernels' 16-row tiles.  (Backward, us, two kernels and one pass.)  One key block: always (B2 H4 S64 D32 11.4
+// and 10.9, B12 H8 S64 D64 22 and 14).  Otherwise from two thirds of a CTA per SM on (128 CTAs, B4 H4 S512: D16 67 and 56, D32
+// 103 and 77; 64 CTAs, B2 H4 S512 causal: D16 51 and 53, D32 69 and 73), above head width 32, where a tile has twice the warps, from
+// a third on (64 CTAs, B2 H4 S512 105 and 93; 28 CTAs, B1 H4 S400 70 and 80).
+static bool one_pass_pays(const ltca_ctx* ctx, const ltca_attn_params* p) {
+    const int64_t blocks = ((int64_t)p->Sk + 63) / 64, ctas = (int64_t)p->B * p->H * blocks;
+    return blocks == 1 || 3 * ctas >= (p->D > 32 ? 1 : 2) * (int64_t)ctx->sm_device;
+}
 size_t attn_bwd_fp32_workspace(const ltca_attn_params* p) {
     return delta_bytes(p) + (p->D <= 128 ? mask_words_bytes(p) + one_pass(p).bytes : 0);
 }
@@ -1378,7 +1396,7 @@ int launch_attn_fwd_fp32(ltca_ctx* ctx, const ltca_attn_params* p) {
 
 bool attn_bwd_fp32_forms_dout(const ltca_ctx* ctx, const ltca_attn_params* p, const FromOutput& f) {
     const auto al = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
-    return p->dtype == LTCA_F32 && p->D <= 64 && !fills_sms(ctx, p->B, p->H, p->Sq) && f.E <= kFormDoutMaxE && (f.E % 8) == 0 &&
+    return p->dtype == LTCA_F32 && p->D <= 64 && (p->Sk <= 32 || p->Sk > 64) && !fills_sms(ctx, p->B, p->H, p->Sq) && f.E <= kFormDoutMaxE && (f.E % 8) == 0 &&
            (int64_t)p->B * p->Sq <= kFormDoutRows && al(f.dy) && al(f.wo);
 }
 
@@ -1397,9 +1415,9 @@ int launch_attn_bwd_fp32(ltca_ctx* ctx, const ltca_attn_params* p, const FromOut
         // delta, dQ's shares, the mask's words; a workspace without room for the shares takes the two kernels, one without room for
         // the words (sized without the mask) reads the mask as it is
         const OnePass one = one_pass(p);
-        const bool room = one.pairs && !from && p->workspace_bytes >= delta_bytes(p) + one.bytes;
+        const bool room = one.pairs && (!from || p->Sk <= 32) && p->workspace_bytes >= delta_bytes(p) + one.bytes;
         const size_t used = delta_bytes(p) + (room ? one.bytes : 0);
-        if (room && fills_sms(ctx, p->B, p->H, p->Sq < p->Sk ? p->Sq : p->Sk)) {
+        if (room && one_pass_pays(ctx, p)) {
             a.pairs = one.pairs;
             a.part_ld = one.ld;
             a.dq_part = one.bytes ? reinterpret_cast<float*>(reinterpret_cast<char*>(p->workspace) + delta_bytes(p)) : nullptr;

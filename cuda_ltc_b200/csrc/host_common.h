@@ -203,11 +203,12 @@ bool attn_bwd_sm100_supported(const ltca_attn_params* p);
 size_t attn_bwd_sm100_workspace(const ltca_attn_params* p);
 int launch_attn_fwd_fp32(ltca_ctx* ctx, const ltca_attn_params* p);
 // The gradient at the attention's result as a module's backward has it: dO_h = dy Wo_h^T, dy rows of E floats at these strides, Wo
-// [H D, E].  Small calls leave that product to the dQ kernel, which writes dO for the dK/dV kernel: a launch less, backward of
-// B8 S32 E32 H4 26.6 -> 25.5 us, B8 S64 43.0 -> 41.0.  Only where the kernel has tiles of 16 rows: with 64 a thread's part of the
-// product is long and holds up the tile's scores (B32 S64 E64 H4 width 16: 41 -> 49 us).  And up to 512 rows: it gains a few
-// per cent a little beyond (B16 S64 E32 H2 38.3 -> 37.2, B64 S64 E16 H1 40.1 -> 37.8), less the more there is to compute (B32
-// S64 E32 H2 42.6 -> 42.0) and in the end nothing (B128 S64 E16 H1 82.1 -> 82.9).
+// [H D, E].  Small calls leave that product to the attention backward: a launch less.  Up to 32 keys the one-pass kernel forms dO
+// where it needs it (B8 S32 E32 H4: with its one launch for dQ, dK and dV 18.7 -> 15.4 us); beyond 64 keys the dQ kernel does and
+// writes it for the dK/dV kernel (B8 S128 E32 H4 43.8 us).  Between them the product stays a launch of its own, since a 64-row
+// tile's part of it is long and holds up the tile's scores (B4 S64 E64 H2 21.7 us formed, 19.8 with the launch).  And up to 512
+// rows: it gains a few per cent a little beyond (two kernels, B16 S64 E32 H2 38.3 -> 37.2, B64 S64 E16 H1 40.1 -> 37.8), less the
+// more there is to compute and in the end nothing (B128 S64 E16 H1 82.1 -> 82.9).
 struct FromOutput { const float *dy, *wo; int E; int64_t batch, seq; };
 constexpr int kFormDoutMaxE = 64, kFormDoutRows = 512;
 bool attn_bwd_exact(const ltca_attn_params* p);       // whether ltca_attn_bwd takes the exact kernels

@@ -103,3 +103,26 @@ def test_a_workspace_without_room_for_the_shares(ctx):
     ctx.check(ctx.lib.ltca_attn_bwd(ctx.handle, C.byref(p)))
     for name, x, ref, mag in zip(("dq", "dk", "dv"), got, want, mags):
         assert float((x.double() - ref).abs().max()) <= 2.0 ** -18 * mag, name
+
+
+@pytest.mark.parametrize("B,S,E,H,W", [(2, 32, 32, 4, 32), (3, 31, 24, 2, 30), (2, 5, 8, 2, 64), (2, 1, 16, 1, 9), (2, 33, 16, 2, 16)])
+def test_module_backward_that_forms_the_gradient_at_the_context(ctx, B, S, E, H, W):
+    """dO = dy Wo^T formed inside the attention backward (up to 32 keys; 33: a product of its own) gives the gradients of the
+    module in 64 bits."""
+    g = torch.Generator(device="cuda").manual_seed(8)
+    rand = lambda *s: torch.randn(s, generator=g, device="cuda")
+    x, dy = rand(B * S, E), rand(B * S, E)
+    w = [rand(E, H * W) / math.sqrt(E) for _ in range(3)] + [rand(H * W, E) / math.sqrt(H * W)]
+    sc = 1.0 / math.sqrt(W)
+    got = ctx.tsa_bwd(x, *w, dy, B, S, H, W, scale=sc, causal=True, time_major=False, mode=_lib.MODE_FP32)
+    xd, dyd = x.double(), dy.double()
+    leaves = [t.double().requires_grad_() for t in w]
+    heads = lambda t: t.view(B, S, H, W).transpose(1, 2)
+    q, k, v = (heads(xd @ t) for t in leaves[:3])
+    s = (q @ k.transpose(-1, -2) * sc).masked_fill(~torch.ones(S, S, dtype=torch.bool, device="cuda").tril(), -math.inf)
+    out = (torch.softmax(s, -1) @ v).transpose(1, 2).reshape(B * S, H * W) @ leaves[3]
+    want = torch.autograd.grad((out * dyd).sum(), leaves)
+    named = got if isinstance(got, dict) else dict(zip(("dx", "dwq", "dwk", "dwv", "dwo"), got))
+    for name, ref in zip(("dwq", "dwk", "dwv", "dwo"), want):
+        # chains of at most 64 + 96 + 64 fp32 terms of magnitude about 1
+        assert float((named[name].double() - ref).abs().max()) <= 2.0 ** -16 * float(ref.abs().max()) + 1e-6, name
