@@ -10,18 +10,18 @@
 // repeatability, src/ml/time_self_attention_test.cu:799-838):
 //   1. attn_bwd_stats_kernel: delta and lse * log2(e) into padded [B*H, Sq_pad] fp32 rows
 //      (padding and fully hidden rows get lse = +inf so that their P is exactly 0).
-//   2. attn_bwd_dq_sm100_kernel: one CTA per 256 query rows; Q and dO tiles stay in shared
-//      memory, K/V stream through a ring in 64-key steps.  Per step and 128-row tile:
+//   2. attn_bwd_dq_sm100_kernel: one CTA per 128 query rows; Q and dO stay in shared
+//      memory, K/V stream through a ring in 64-key steps.  Per step:
 //      S = Q K^T and dP = dO V^T into tensor memory, the elementwise warps (one query row per
-//      thread) turn them into dS (bf16, written back over S), and dQ += dS K takes dS from
+//      two threads) turn them into dS (bf16, two terms), and dQ += dS K takes dS from
 //      tensor memory and K as an MN-major operand from shared memory.
-//   3. attn_bwd_dkv_sm100_kernel: the transposed problem, one CTA per 256 keys; K and V tiles
+//   3. attn_bwd_dkv_sm100_kernel: the transposed problem, one CTA per 128 keys; K and V
 //      stay in shared memory, Q/dO (and the per-row statistics) stream in 64-query steps.
 //      S^T = K Q^T and dP^T = V dO^T put one KEY per tensor-memory lane, so P^T and dS^T are
 //      directly the A operands of dV += P^T dO and dK += dS^T Q.
-// Both main kernels share the forward's structure: warps 0-3 / 4-7 elementwise for tile 0 / 1,
-// warp 8 issues tcgen05.mma, warp 9 drives TMA; the two tiles are interleaved so one tile's
-// elementwise work overlaps the other's contractions.  Every wait is bounded.
+// (2 and 3 for fp32 results; bf16 results have kernels of their own further down.)  Warps 0-7 elementwise, warp 8
+// issues tcgen05.mma, warp 9 drives TMA; two CTAs share an SM, so one's elementwise work overlaps the
+// other's contractions.  Every wait is bounded.
 #include <type_traits>
 
 #include "host_common.h"
@@ -46,6 +46,16 @@ constexpr int kCtrlRegs = 56;        // kept by the TMA / MMA-issue warps
 constexpr int kMathRegs = 104;       // taken by the elementwise warps
 // setmaxnreg can only redistribute what the CTA was launched with; asking for more never returns
 static_assert(512 * kMathRegs + 128 * kCtrlRegs <= kThreads * kLaunchRegs, "register budget");
+// dQ and dK/dV for fp32 results: a CTA per 128-row tile, two to an SM, heaviest tiles first.  As one CTA with two neighbouring
+// tiles (the tensor memory and warps of both) a causal pair of tiles took the time of its longer one and a launch ended on whole
+// pairs; a tile of a CTA's own also hides its set-up and its result's store under the other's steps.  Backward, us: B32 H8 S256
+// causal 79 -> 75, B12 H8 S384 76 -> 48, B1 H16 S4096 causal 447 -> 258, B64 H8 S64 52 -> 37.
+constexpr int kTileThreads = 384;    // 8 elementwise warps + one warpgroup of control warps
+constexpr int kTileMmaWarp = 8, kTileTmaWarp = 9;
+constexpr uint32_t kTileTmemCols = 256;
+constexpr int kTileLaunchRegs = 80, kTileCtrlRegs = 48, kTileMathRegs = 96;
+static_assert(256 * kTileMathRegs + 128 * kTileCtrlRegs <= kTileThreads * kTileLaunchRegs, "register budget");
+static_assert(2 * kTileThreads * kTileLaunchRegs <= 65536, "two to an SM");
 constexpr int kBigTile = kTile * kD * 2;      // 16 KB
 constexpr int kSmallTile = kStep * kD * 2;    // 8 KB
 
@@ -153,25 +163,25 @@ __global__ void __launch_bounds__(8 * kStatsRows) attn_bwd_stats_kernel(const St
 // ---------------------------------------------------------------------------------------------
 struct DqSmem {
     static constexpr int kStages = 8;                         // ring of 8 KB K / V step tiles
-    static constexpr int kQOff = 0;                           // Q0, Q1
-    static constexpr int kDoOff = 2 * kBigTile;               // dO0, dO1
-    static constexpr int kRingOff = 4 * kBigTile;
+    static constexpr int kQOff = 0;
+    static constexpr int kDoOff = kBigTile;
+    static constexpr int kRingOff = 2 * kBigTile;
     static constexpr int kBarOff = kRingOff + kStages * kSmallTile;
-    // bars: qdo_full, ring_full[S], ring_empty[S], sdp_full[2], sdp_free[2], ds_full[2], dq_done[2], stagger
-    static constexpr int kNumBars = 1 + 2 * kStages + 9;
+    // bars: qdo_full, ring_full[S], ring_empty[S], sdp_full, sdp_free, ds_full, dq_done
+    static constexpr int kNumBars = 1 + 2 * kStages + 4;
     static constexpr int kMiscOff = kBarOff + kNumBars * 8;
     static constexpr int kDynBytes = kMiscOff + 16 + 1024;
 };
 
 struct DkvSmem {
-    static constexpr int kStages = 6;                         // ring of (Q_j, dO_j, lse2_j, delta_j)
+    static constexpr int kStages = 4;                         // ring of (Q_j, dO_j, lse2_j, delta_j)
     static constexpr int kStageBytes = 2 * kSmallTile + 1024; // stats padded to keep 1024-B alignment
-    static constexpr int kKOff = 0;                           // K0, K1
-    static constexpr int kVOff = 2 * kBigTile;                // V0, V1
-    static constexpr int kRingOff = 4 * kBigTile;
+    static constexpr int kKOff = 0;
+    static constexpr int kVOff = kBigTile;
+    static constexpr int kRingOff = 2 * kBigTile;
     static constexpr int kBarOff = kRingOff + kStages * kStageBytes;
-    // bars: kv_full, ring_full[S], ring_empty[S], sdp_full[2], pds_full[2], acc_done[2], stagger
-    static constexpr int kNumBars = 1 + 2 * kStages + 7;
+    // bars: kv_full, ring_full[S], ring_empty[S], sdp_full, pds_full, acc_done
+    static constexpr int kNumBars = 1 + 2 * kStages + 3;
     static constexpr int kMiscOff = kBarOff + kNumBars * 8;
     static constexpr int kDynBytes = kMiscOff + 16 + 1024;
 };
@@ -213,15 +223,14 @@ __device__ __forceinline__ void pack32(const uint32_t (&v)[32], uint32_t (&hi)[1
 
 // ---------------------------------------------------------------------------------------------
 // 2. dQ
-// tensor memory: tile t at t*192: S [0,64)  dP [64,128)  dQ [128,192);
-// dS (bf16) of tile t at 384 + t*32, its low-order term (kSplit) at 448 + t*32.
-// A query row belongs to two threads (warps w and w + 8), each owning 32 of the step's 64 keys.
+// tensor memory: S [0,64)  dP [64,128)  dQ [128,192)  dS (bf16) [192,224), its low-order term (kSplit) [224,256).
+// A query row belongs to two threads (warps w and w + 4), each owning 32 of the step's 64 keys.
 // ---------------------------------------------------------------------------------------------
 // kSplit (fp32 gradients out): dS is written as two bf16 terms and the dQ contraction runs once
 // per term, so that the 2^-9 rounding of a single bf16 dS does not dominate the error of an fp32
 // result.
 template <typename OutT, bool kSplit, bool kMask>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(kTileThreads, 2)
 attn_bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
                          const __grid_constant__ CUtensorMap tmap_do,
                          const __grid_constant__ CUtensorMap tmap_k,
@@ -235,49 +244,37 @@ attn_bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
     auto bar_qdo_full = [&]() { return bar_base; };
     auto bar_ring_full = [&](int s) { return bar_base + 8u * (1 + s); };
     auto bar_ring_empty = [&](int s) { return bar_base + 8u * (1 + L::kStages + s); };
-    auto bar_sdp_full = [&](int t) { return bar_base + 8u * (1 + 2 * L::kStages + t); };
-    auto bar_sdp_free = [&](int t) { return bar_base + 8u * (3 + 2 * L::kStages + t); };
-    auto bar_ds_full = [&](int t) { return bar_base + 8u * (5 + 2 * L::kStages + t); };
-    auto bar_dq_done = [&](int t) { return bar_base + 8u * (7 + 2 * L::kStages + t); };
-    auto bar_stagger = [&]() { return bar_base + 8u * (9 + 2 * L::kStages); };
+    auto bar_sdp_full = [&]() { return bar_base + 8u * (1 + 2 * L::kStages); };
+    auto bar_sdp_free = [&]() { return bar_base + 8u * (2 + 2 * L::kStages); };
+    auto bar_ds_full = [&]() { return bar_base + 8u * (3 + 2 * L::kStages); };
+    auto bar_dq_done = [&]() { return bar_base + 8u * (4 + 2 * L::kStages); };
     volatile uint32_t* misc = reinterpret_cast<volatile uint32_t*>(smem_gen + L::kMiscOff);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int m_block = gridDim.x - 1 - blockIdx.x;
-    const int h = blockIdx.y, b = blockIdx.z;
+    int rank, h, b;
+    sched_block(rank, h, b, kSchedGroup);
+    const int q0 = (gridDim.x - 1 - rank) * kTile;  // late queries see the most keys
 
     int kvlen = a.Sk;
     if (a.kv_len) {
         grid_dependency_wait();                // the lengths may come from the kernel before this one
         kvlen = min(max(a.kv_len[b], 0), a.Sk);
     }
-    int n_steps[2];
-#pragma unroll
-    for (int t = 0; t < 2; ++t) {
-        const int q0 = m_block * 2 * kTile + t * kTile;
-        int lim = 0;
-        if (q0 < a.Sq) {
-            lim = kvlen;
-            if (a.causal) lim = min(lim, min(q0 + kTile - 1, a.Sq - 1) + a.causal_off + 1);
-        }
-        n_steps[t] = lim > 0 ? (lim + kStep - 1) / kStep : 0;
-    }
-    const int n_max = max(n_steps[0], n_steps[1]);
+    int lim_all = kvlen;
+    if (a.causal) lim_all = min(lim_all, min(q0 + kTile - 1, a.Sq - 1) + a.causal_off + 1);
+    const int n = lim_all > 0 ? (lim_all + kStep - 1) / kStep : 0;
 
     if (threadIdx.x == 0) {
         mbar_init(bar_qdo_full(), 1);
-        for (int s = 0; s < L::kStages; ++s) { mbar_init(bar_ring_full(s), 1); mbar_init(bar_ring_empty(s), 2); }
-        for (int t = 0; t < 2; ++t) {
-            mbar_init(bar_sdp_full(t), 1);
-            mbar_init(bar_sdp_free(t), 8);         // one arrival per elementwise warp of the tile
-            mbar_init(bar_ds_full(t), 8);
-            mbar_init(bar_dq_done(t), 1);
-        }
-        mbar_init(bar_stagger(), 8);
+        for (int s = 0; s < L::kStages; ++s) { mbar_init(bar_ring_full(s), 1); mbar_init(bar_ring_empty(s), 1); }
+        mbar_init(bar_sdp_full(), 1);
+        mbar_init(bar_sdp_free(), 8);             // one arrival per elementwise warp
+        mbar_init(bar_ds_full(), 8);
+        mbar_init(bar_dq_done(), 1);
         misc[1] = 0u;
         mbar_fence_init();
     }
-    if (warp == kMmaWarp0) { tmem_alloc(smem_u32(const_cast<uint32_t*>(&misc[0])), kTmemCols); tmem_relinquish(); }
+    if (warp == kTileMmaWarp) { tmem_alloc(smem_u32(const_cast<uint32_t*>(&misc[0])), kTileTmemCols); tmem_relinquish(); }
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
@@ -289,18 +286,15 @@ attn_bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
     LTCA_TRACE_DECL(LTCA_TRACE_KERNEL == 1 && blockIdx.x == 0 && blockIdx.y == 5 && blockIdx.z == 0);
     LTCA_TRACE_EVT(0x01);
 
-    if (warp >= 16) {
-      reg_dealloc<kCtrlRegs>();
-      if (warp == kTmaWarp) {
-        if (lane == 0 && n_max > 0) {
-            mbar_arrive_expect_tx(bar_qdo_full(), 4u * kBigTile);
-            for (int t = 0; t < 2; ++t) {
-                const int q0 = m_block * 2 * kTile + t * kTile;
-                tma_load_4d(q_smem + t * kBigTile, &tmap_q, bar_qdo_full(), 0, q0, h, b);
-                tma_load_4d(do_smem + t * kBigTile, &tmap_do, bar_qdo_full(), 0, q0, h, b);
-            }
+    if (warp >= kTileMmaWarp) {
+      reg_dealloc<kTileCtrlRegs>();
+      if (warp == kTileTmaWarp) {
+        if (lane == 0 && n > 0) {
+            mbar_arrive_expect_tx(bar_qdo_full(), 2u * kBigTile);
+            tma_load_4d(q_smem, &tmap_q, bar_qdo_full(), 0, q0, h, b);
+            tma_load_4d(do_smem, &tmap_do, bar_qdo_full(), 0, q0, h, b);
             bool ok = true;
-            for (int j = 0; j < n_max && ok; ++j) {
+            for (int j = 0; j < n && ok; ++j) {
 #pragma unroll
                 for (int which = 0; which < 2; ++which) {          // 0: K_j, 1: V_j
                     const int item = 2 * j + which;
@@ -312,19 +306,17 @@ attn_bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
                 }
             }
         }
-      } else if (warp == kMmaWarp0 || warp == kMmaWarp0 + 1) {
-        const int t = warp - kMmaWarp0;            // this thread issues the contractions of tile t
-        if (lane == 0 && n_max > 0) {
-            const int n_t = n_steps[t];
+      } else if (warp == kTileMmaWarp) {
+        if (lane == 0 && n > 0) {
             constexpr uint32_t idesc_s = make_idesc_bf16(kTile, kStep, 0, 0);
             constexpr uint32_t idesc_dq = make_idesc_bf16(kTile, kD, 0, 1);
-            const uint64_t q_desc = make_smem_desc_sw128(q_smem + t * kBigTile, 16, 1024);
-            const uint64_t do_desc = make_smem_desc_sw128(do_smem + t * kBigTile, 16, 1024);
+            const uint64_t q_desc = make_smem_desc_sw128(q_smem, 16, 1024);
+            const uint64_t do_desc = make_smem_desc_sw128(do_smem, 16, 1024);
             const uint64_t ring_desc = make_smem_desc_sw128(ring_smem, 16, 1024);
             const uint64_t ring_desc_mn = make_smem_desc_sw128(ring_smem, 8192, 1024);
-            const uint32_t tb = tmem_base + t * 192;
-            const uint32_t ds_hi = tmem_base + 384 + t * 32, ds_lo = tmem_base + 448 + t * 32;
-            // S_t = Q_t K_j^T and dP_t = dO_t V_j^T
+            const uint32_t tb = tmem_base;
+            const uint32_t ds_hi = tmem_base + 192, ds_lo = tmem_base + 224;
+            // S = Q K_j^T and dP = dO V_j^T
             auto issue_sdp = [&](int slot_k, int slot_v) {
                 const uint64_t kd = ring_desc + (uint64_t)((slot_k * kSmallTile) >> 4);
                 const uint64_t vd = ring_desc + (uint64_t)((slot_v * kSmallTile) >> 4);
@@ -333,7 +325,7 @@ attn_bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
 #pragma unroll
                 for (int k = 0; k < kD / 16; ++k) mma_ss(tb + 64, do_desc + 2 * k, vd + 2 * k, idesc_s, k > 0);
             };
-            // dQ_t += dS_t K_j   (dS from tensor memory, K_j rows as the contraction index)
+            // dQ += dS K_j   (dS from tensor memory, K_j rows as the contraction index)
             auto issue_dq = [&](int slot_k, bool acc) {
                 const uint64_t kd = ring_desc_mn + (uint64_t)((slot_k * kSmallTile) >> 4);
 #pragma unroll
@@ -350,54 +342,51 @@ attn_bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
             ok = ok && mbar_wait(bar_ring_full(slot_of(1)), phase_of(1), wc, 0x52);
             if (ok) {
                 tc_fence_after_sync();
-                if (n_t > 0) { issue_sdp(slot_of(0), slot_of(1)); mma_commit(bar_sdp_full(t)); }
+                issue_sdp(slot_of(0), slot_of(1));
+                mma_commit(bar_sdp_full());
                 mma_commit(bar_ring_empty(slot_of(1)));            // V_0 is consumed
             }
-            for (int j = 0; j < n_max && ok; ++j) {
+            for (int j = 0; j < n && ok; ++j) {
                 const int item_k = 2 * j, item_k1 = 2 * j + 2, item_v1 = 2 * j + 3;
-                if (j + 1 < n_max) {
+                if (j + 1 < n) {
                     ok = mbar_wait(bar_ring_full(slot_of(item_k1)), phase_of(item_k1), wc, 0x53);
                     ok = ok && mbar_wait(bar_ring_full(slot_of(item_v1)), phase_of(item_v1), wc, 0x54);
-                    if (ok && j + 1 < n_t) {
+                    if (ok) {
                         // S and dP of step j are in registers: compute step j + 1 now
-                        ok = mbar_wait(bar_sdp_free(t), (uint32_t)(j & 1), wc, 0x5a + t);
+                        ok = mbar_wait(bar_sdp_free(), (uint32_t)(j & 1), wc, 0x5a);
                         if (!ok) break;
                         tc_fence_after_sync();
                         LTCA_TRACE_EVT(0x20 + (j << 8));
                         issue_sdp(slot_of(item_k1), slot_of(item_v1));
-                        mma_commit(bar_sdp_full(t));
+                        mma_commit(bar_sdp_full());
                         LTCA_TRACE_EVT(0x21 + (j << 8));
                     }
                     if (!ok) break;
                     mma_commit(bar_ring_empty(slot_of(item_v1)));
                 }
-                if (j < n_t) {
-                    ok = mbar_wait(bar_ds_full(t), (uint32_t)(j & 1), wc, 0x55 + t);
-                    if (!ok) break;
-                    tc_fence_after_sync();
-                    LTCA_TRACE_EVT(0x22 + (j << 8));
-                    issue_dq(slot_of(item_k), j > 0);
-                    mma_commit(bar_dq_done(t));
-                    LTCA_TRACE_EVT(0x23 + (j << 8));
-                }
+                ok = mbar_wait(bar_ds_full(), (uint32_t)(j & 1), wc, 0x55);
+                if (!ok) break;
+                tc_fence_after_sync();
+                LTCA_TRACE_EVT(0x22 + (j << 8));
+                issue_dq(slot_of(item_k), j > 0);
+                mma_commit(bar_dq_done());
+                LTCA_TRACE_EVT(0x23 + (j << 8));
                 mma_commit(bar_ring_empty(slot_of(item_k)));
             }
-            if (ok && n_t > 0) ok = mbar_wait(bar_dq_done(t), (uint32_t)((n_t - 1) & 1), wc, 0x58 + t);
+            if (ok) ok = mbar_wait(bar_dq_done(), (uint32_t)((n - 1) & 1), wc, 0x58);
         }
       }
     } else {
-        reg_alloc<kMathRegs>();
-        const int t = (warp >> 2) & 1, half = warp >> 3, wq = warp & 3;
+        reg_alloc<kTileMathRegs>();
+        const int half = warp >> 2, wq = warp & 3;
         const int row = wq * 32 + lane;
-        const int q0 = m_block * 2 * kTile + t * kTile;
         const int qi = q0 + row;
-        const int n_t = n_steps[t];
         const uint32_t lane_base = (uint32_t)(wq * 32) << 16;
-        const uint32_t tS = tmem_base + lane_base + t * 192 + half * 32;
+        const uint32_t tS = tmem_base + lane_base + half * 32;
         const uint32_t tDP = tS + 64;
-        const uint32_t tDQ = tmem_base + lane_base + t * 192 + 128 + half * 32;
-        const uint32_t tDS = tmem_base + lane_base + 384 + t * 32 + half * 16;
-        const uint32_t tDSlo = tDS + 64;
+        const uint32_t tDQ = tmem_base + lane_base + 128 + half * 32;
+        const uint32_t tDS = tmem_base + lane_base + 192 + half * 16;
+        const uint32_t tDSlo = tDS + 32;
         const float c2 = a.scale_log2;
         const bool general = kMask || (a.use_clamp != 0);
         const int64_t srow = ((int64_t)b * a.H + h) * a.Sq_pad + qi;      // qi < Sq_pad by construction
@@ -405,10 +394,10 @@ attn_bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
         const float dlt = a.delta[srow];
 
         bool ok = true;
-        for (int j = 0; j < n_t; ++j) {
+        for (int j = 0; j < n; ++j) {
             uint32_t keep = ~0u;
             if (kMask) keep = mask_bits_of_queries(a.mask, b, q0 + wq * 32, j * kStep + half * 32);
-            ok = mbar_wait_warp(bar_sdp_full(t), (uint32_t)(j & 1), wc, 0x60 + t);
+            ok = mbar_wait_warp(bar_sdp_full(), (uint32_t)(j & 1), wc, 0x60);
             if (!ok) break;
             tc_fence_after_sync();
             LTCA_TRACE_EVT(0x10 + (j << 8));
@@ -418,14 +407,8 @@ attn_bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
             tmem_wait_ld();
             tc_fence_before_sync();
             __syncwarp();
-            if (lane == 0) mbar_arrive(bar_sdp_free(t));
+            if (lane == 0) mbar_arrive(bar_sdp_free());
             LTCA_TRACE_EVT(0x11 + (j << 8));
-            // One-time delay of tile 1: from then on one tile's exponentials overlap the other
-            // tile's loads, stores and barrier traffic instead of all warps stalling together.
-            if (t == 1 && j == 0 && n_steps[0] > 0) {
-                ok = mbar_wait_warp(bar_stagger(), 0, wc, 0x66);
-                if (!ok) break;
-            }
             const int k0 = j * kStep;
             const bool edge = (k0 + kStep > kvlen) || (a.causal && (k0 + kStep - 1 > q0 + a.causal_off));
             // dS = P o (dP - delta), left in dp[]; the masked variant only runs on edge steps
@@ -461,14 +444,10 @@ attn_bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
             }
             uint32_t hi[16], lo[16];
             pack32<kSplit>(dp, hi, lo);
-            if (t == 0 && j == 0) {
-                __syncwarp();
-                if (lane == 0) mbar_arrive(bar_stagger());
-            }
             LTCA_TRACE_EVT(0x12 + (j << 8));
             if (j > 0) {
                 // the previous dS must have been consumed before it is overwritten
-                ok = mbar_wait_warp(bar_dq_done(t), (uint32_t)((j - 1) & 1), wc, 0x64 + t);
+                ok = mbar_wait_warp(bar_dq_done(), (uint32_t)((j - 1) & 1), wc, 0x64);
                 if (!ok) break;
             }
             tmem_st16(tDS, hi);
@@ -476,18 +455,18 @@ attn_bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
             tmem_wait_st();
             tc_fence_before_sync();
             __syncwarp();
-            if (lane == 0) mbar_arrive(bar_ds_full(t));
+            if (lane == 0) mbar_arrive(bar_ds_full());
             LTCA_TRACE_EVT(0x13 + (j << 8));
         }
-        if (ok && q0 < a.Sq) {
-            if (n_t > 0) {
-                ok = mbar_wait_warp(bar_dq_done(t), (uint32_t)((n_t - 1) & 1), wc, 0x62 + t);
+        if (ok) {
+            if (n > 0) {
+                ok = mbar_wait_warp(bar_dq_done(), (uint32_t)((n - 1) & 1), wc, 0x62);
                 tc_fence_after_sync();
             }
             OutT* drow = reinterpret_cast<OutT*>(a.dq) + b * a.dqs.batch + h * a.dqs.head +
                          (int64_t)qi * a.dqs.seq + half * 32;
             uint32_t o[32];
-            if (n_t > 0 && ok) { tmem_ld32(tDQ, o); tmem_wait_ld(); }
+            if (n > 0 && ok) { tmem_ld32(tDQ, o); tmem_wait_ld(); }
             else {
 #pragma unroll
                 for (int c = 0; c < 32; ++c) o[c] = 0u;
@@ -498,24 +477,24 @@ attn_bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
 
     tc_fence_before_sync();
     __syncthreads();
-    if (warp == kMmaWarp0) {
+    if (warp == kTileMmaWarp) {
         __syncwarp();
         if (misc[1]) __nanosleep(200000);
         tc_fence_after_sync();
-        tmem_dealloc(tmem_base, kTmemCols);
+        tmem_dealloc(tmem_base, kTileTmemCols);
     }
 }
 
 // ---------------------------------------------------------------------------------------------
 // 3. dK, dV (transposed problem: one KEY per tensor-memory lane)
-// tensor memory per tile t (base t*256): S^T [0,64) dP^T [64,128) dV [128,192) dK [192,256).
-// A key row belongs to two threads (warps w and w + 8); thread `half` owns query columns
+// tensor memory: S^T [0,64) dP^T [64,128) dV [128,192) dK [192,256).
+// A key row belongs to two threads (warps w and w + 4); thread `half` owns query columns
 // [32*half, 32*half + 32) of S^T and dP^T and writes its P^T / dS^T back INSIDE those columns
 // (bf16 pairs in the first 16, the kSplit low-order term in the next 16), so neither thread
 // ever overwrites scores the other has not read yet.
 // ---------------------------------------------------------------------------------------------
 template <typename OutT, bool kSplit, bool kMask>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(kTileThreads, 2)
 attn_bwd_dkv_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
                           const __grid_constant__ CUtensorMap tmap_do,
                           const __grid_constant__ CUtensorMap tmap_k,
@@ -529,15 +508,15 @@ attn_bwd_dkv_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
     auto bar_kv_full = [&]() { return bar_base; };
     auto bar_ring_full = [&](int s) { return bar_base + 8u * (1 + s); };
     auto bar_ring_empty = [&](int s) { return bar_base + 8u * (1 + L::kStages + s); };
-    auto bar_sdp_full = [&](int t) { return bar_base + 8u * (1 + 2 * L::kStages + t); };
-    auto bar_pds_full = [&](int t) { return bar_base + 8u * (3 + 2 * L::kStages + t); };
-    auto bar_acc_done = [&](int t) { return bar_base + 8u * (5 + 2 * L::kStages + t); };
-    auto bar_stagger = [&]() { return bar_base + 8u * (7 + 2 * L::kStages); };
+    auto bar_sdp_full = [&]() { return bar_base + 8u * (1 + 2 * L::kStages); };
+    auto bar_pds_full = [&]() { return bar_base + 8u * (2 + 2 * L::kStages); };
+    auto bar_acc_done = [&]() { return bar_base + 8u * (3 + 2 * L::kStages); };
     volatile uint32_t* misc = reinterpret_cast<volatile uint32_t*>(smem_gen + L::kMiscOff);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int n_block = blockIdx.x;                 // early key blocks carry the most causal work
-    const int h = blockIdx.y, b = blockIdx.z;
+    int rank, h, b;
+    sched_block(rank, h, b, kSchedGroup);
+    const int k0 = rank * kTile;                    // early keys are seen by the most queries
 
     int kvlen = a.Sk;
     if (a.kv_len) {
@@ -545,33 +524,19 @@ attn_bwd_dkv_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
         kvlen = min(max(a.kv_len[b], 0), a.Sk);
     }
     const int n_q = (a.Sq + kStep - 1) / kStep;     // query steps in total
-    int j_begin[2];                                 // first query step that can see the tile's keys
-    bool active[2];
-#pragma unroll
-    for (int t = 0; t < 2; ++t) {
-        const int k0 = n_block * 2 * kTile + t * kTile;
-        active[t] = (k0 < kvlen);
-        int jb = 0;
-        if (a.causal) jb = max(0, k0 - a.causal_off) / kStep;
-        j_begin[t] = jb;
-        if (jb >= n_q) active[t] = false;
-    }
-    const bool any_active = active[0] || active[1];
-    const int j_first = min(active[0] ? j_begin[0] : n_q, active[1] ? j_begin[1] : n_q);
+    const int j_first = a.causal ? max(0, k0 - a.causal_off) / kStep : 0;   // the first that can see the tile's keys
+    const bool active = k0 < kvlen && j_first < n_q;
 
     if (threadIdx.x == 0) {
         mbar_init(bar_kv_full(), 1);
-        for (int s = 0; s < L::kStages; ++s) { mbar_init(bar_ring_full(s), 1); mbar_init(bar_ring_empty(s), 2); }
-        for (int t = 0; t < 2; ++t) {
-            mbar_init(bar_sdp_full(t), 1);
-            mbar_init(bar_pds_full(t), 8);         // one arrival per elementwise warp of the tile
-            mbar_init(bar_acc_done(t), 1);
-        }
-        mbar_init(bar_stagger(), 8);
+        for (int s = 0; s < L::kStages; ++s) { mbar_init(bar_ring_full(s), 1); mbar_init(bar_ring_empty(s), 1); }
+        mbar_init(bar_sdp_full(), 1);
+        mbar_init(bar_pds_full(), 8);             // one arrival per elementwise warp
+        mbar_init(bar_acc_done(), 1);
         misc[1] = 0u;
         mbar_fence_init();
     }
-    if (warp == kMmaWarp0) { tmem_alloc(smem_u32(const_cast<uint32_t*>(&misc[0])), kTmemCols); tmem_relinquish(); }
+    if (warp == kTileMmaWarp) { tmem_alloc(smem_u32(const_cast<uint32_t*>(&misc[0])), kTileTmemCols); tmem_relinquish(); }
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
@@ -584,16 +549,13 @@ attn_bwd_dkv_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
     LTCA_TRACE_DECL(LTCA_TRACE_KERNEL == 2 && blockIdx.x == 0 && blockIdx.y == 5 && blockIdx.z == 0);
     LTCA_TRACE_EVT(0x01);
 
-    if (warp >= 16) {
-      reg_dealloc<kCtrlRegs>();
-      if (warp == kTmaWarp) {
-        if (lane == 0 && any_active) {
-            mbar_arrive_expect_tx(bar_kv_full(), 4u * kBigTile);
-            for (int t = 0; t < 2; ++t) {
-                const int k0 = n_block * 2 * kTile + t * kTile;
-                tma_load_4d(k_smem + t * kBigTile, &tmap_k, bar_kv_full(), 0, k0, h, b);
-                tma_load_4d(v_smem + t * kBigTile, &tmap_v, bar_kv_full(), 0, k0, h, b);
-            }
+    if (warp >= kTileMmaWarp) {
+      reg_dealloc<kTileCtrlRegs>();
+      if (warp == kTileTmaWarp) {
+        if (lane == 0 && active) {
+            mbar_arrive_expect_tx(bar_kv_full(), 2u * kBigTile);
+            tma_load_4d(k_smem, &tmap_k, bar_kv_full(), 0, k0, h, b);
+            tma_load_4d(v_smem, &tmap_v, bar_kv_full(), 0, k0, h, b);
             const float* lse2_row = a.lse2 + ((int64_t)b * a.H + h) * a.Sq_pad;
             const float* dlt_row = a.delta + ((int64_t)b * a.H + h) * a.Sq_pad;
             bool ok = true;
@@ -614,19 +576,16 @@ attn_bwd_dkv_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
                       "r"(bar_ring_full(slot_of(j))) : "memory");
             }
         }
-      } else if (warp == kMmaWarp0 || warp == kMmaWarp0 + 1) {
-        const int t = warp - kMmaWarp0;            // this thread issues the contractions of tile t
-        if (lane == 0 && any_active) {
+      } else if (warp == kTileMmaWarp) {
+        if (lane == 0 && active) {
             constexpr uint32_t idesc_s = make_idesc_bf16(kTile, kStep, 0, 0);
             constexpr uint32_t idesc_acc = make_idesc_bf16(kTile, kD, 0, 1);
-            const uint64_t k_desc = make_smem_desc_sw128(k_smem + t * kBigTile, 16, 1024);
-            const uint64_t v_desc = make_smem_desc_sw128(v_smem + t * kBigTile, 16, 1024);
+            const uint64_t k_desc = make_smem_desc_sw128(k_smem, 16, 1024);
+            const uint64_t v_desc = make_smem_desc_sw128(v_smem, 16, 1024);
             const uint64_t ring_desc = make_smem_desc_sw128(ring_smem, 16, 1024);
             const uint64_t ring_desc_mn = make_smem_desc_sw128(ring_smem, 8192, 1024);
-            const uint32_t tb = tmem_base + t * 256;
-            const bool act = active[t];
-            const int jb = j_begin[t];
-            // S^T_t = K_t Q_j^T and dP^T_t = V_t dO_j^T
+            const uint32_t tb = tmem_base;
+            // S^T = K Q_j^T and dP^T = V dO_j^T
             auto issue_sdp = [&](int slot) {
                 const uint64_t qd = ring_desc + (uint64_t)((slot * L::kStageBytes) >> 4);
                 const uint64_t gd = qd + (uint64_t)(kSmallTile >> 4);
@@ -635,7 +594,7 @@ attn_bwd_dkv_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
 #pragma unroll
                 for (int k = 0; k < kD / 16; ++k) mma_ss(tb + 64, v_desc + 2 * k, gd + 2 * k, idesc_s, k > 0);
             };
-            // dV_t += P^T_t dO_j and dK_t += dS^T_t Q_j   (query rows are the contraction index);
+            // dV += P^T dO_j and dK += dS^T Q_j   (query rows are the contraction index);
             // queries [0,32) sit in columns [0,16) of their region, queries [32,64) in [32,48)
             auto issue_acc = [&](int slot, bool acc) {
                 const uint64_t qd = ring_desc_mn + (uint64_t)((slot * L::kStageBytes) >> 4);
@@ -658,61 +617,53 @@ attn_bwd_dkv_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
                 }
             };
             bool ok = mbar_wait(bar_kv_full(), 0, wc, 0x80);
-            if (ok && j_first < n_q) {
-                ok = mbar_wait(bar_ring_full(slot_of(j_first)), phase_of(j_first), wc, 0x81);
-                if (ok && act && jb == j_first) {
-                    tc_fence_after_sync();
-                    issue_sdp(slot_of(j_first));
-                    mma_commit(bar_sdp_full(t));
-                }
+            ok = ok && mbar_wait(bar_ring_full(slot_of(j_first)), phase_of(j_first), wc, 0x81);
+            if (ok) {
+                tc_fence_after_sync();
+                issue_sdp(slot_of(j_first));
+                mma_commit(bar_sdp_full());
             }
             for (int j = j_first; j < n_q && ok; ++j) {
                 const bool have_next = (j + 1 < n_q);
                 if (have_next) ok = mbar_wait(bar_ring_full(slot_of(j + 1)), phase_of(j + 1), wc, 0x82);
+                ok = ok && mbar_wait(bar_pds_full(), (uint32_t)((j - j_first) & 1), wc, 0x83);
                 if (!ok) break;
-                if (act) {
-                    if (j >= jb) {
-                        ok = mbar_wait(bar_pds_full(t), (uint32_t)((j - jb) & 1), wc, 0x83 + t);
-                        if (!ok) break;
-                        tc_fence_after_sync();
-                        LTCA_TRACE_EVT(0x22 + (j << 8));
-                        issue_acc(slot_of(j), j > jb);
-                        mma_commit(bar_acc_done(t));
-                        LTCA_TRACE_EVT(0x23 + (j << 8));
-                    }
-                    if (have_next && j + 1 >= jb) {
-                        issue_sdp(slot_of(j + 1));
-                        mma_commit(bar_sdp_full(t));
-                        LTCA_TRACE_EVT(0x21 + (j << 8));
-                    }
-                }
+                tc_fence_after_sync();
+                LTCA_TRACE_EVT(0x22 + (j << 8));
+                issue_acc(slot_of(j), j > j_first);
+                mma_commit(bar_acc_done());
                 mma_commit(bar_ring_empty(slot_of(j)));
+                LTCA_TRACE_EVT(0x23 + (j << 8));
+                if (have_next) {
+                    issue_sdp(slot_of(j + 1));
+                    mma_commit(bar_sdp_full());
+                    LTCA_TRACE_EVT(0x21 + (j << 8));
+                }
             }
-            if (ok && act) ok = mbar_wait(bar_acc_done(t), (uint32_t)((n_q - 1 - jb) & 1), wc, 0x88 + t);
+            if (ok) ok = mbar_wait(bar_acc_done(), (uint32_t)((n_q - 1 - j_first) & 1), wc, 0x88);
         }
       }
     } else {
-        reg_alloc<kMathRegs>();
-        const int t = (warp >> 2) & 1, half = warp >> 3, wq = warp & 3;
+        reg_alloc<kTileMathRegs>();
+        const int half = warp >> 2, wq = warp & 3;
         const int row = wq * 32 + lane;
-        const int k0 = n_block * 2 * kTile + t * kTile;
         const int kj = k0 + row;                                   // this thread's key
         const uint32_t lane_base = (uint32_t)(wq * 32) << 16;
-        const uint32_t tS = tmem_base + lane_base + t * 256 + half * 32;
+        const uint32_t tS = tmem_base + lane_base + half * 32;
         const uint32_t tDP = tS + 64;
-        const uint32_t tDV = tmem_base + lane_base + t * 256 + 128 + half * 32;
+        const uint32_t tDV = tmem_base + lane_base + 128 + half * 32;
         const uint32_t tDK = tDV + 64;
         const float c2 = a.scale_log2;
         const bool general = kMask || (a.use_clamp != 0);
         const bool key_live = kj < kvlen;
 
         bool ok = true;
-        if (active[t]) {
-            for (int j = j_begin[t]; j < n_q; ++j) {
-                const int it = j - j_begin[t];
+        if (active) {
+            for (int j = j_first; j < n_q; ++j) {
+                const int it = j - j_first;
                 uint32_t keep = ~0u;
                 if (kMask) keep = mask_bits_of_key(a.mask, b, j * kStep + half * 32, kj);
-                ok = mbar_wait_warp(bar_sdp_full(t), (uint32_t)(it & 1), wc, 0x90 + t);
+                ok = mbar_wait_warp(bar_sdp_full(), (uint32_t)(it & 1), wc, 0x90);
                 if (!ok) break;
                 tc_fence_after_sync();
                 LTCA_TRACE_EVT(0x10 + (j << 8));
@@ -721,10 +672,6 @@ attn_bwd_dkv_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
                 tmem_ld32(tDP, dp);
                 tmem_wait_ld();
                 LTCA_TRACE_EVT(0x11 + (j << 8));
-                if (t == 1 && it == 0 && active[0] && j_begin[0] <= j_begin[1]) {
-                    ok = mbar_wait_warp(bar_stagger(), 0, wc, 0x96);
-                    if (!ok) break;
-                }
                 // lse2 and delta of this thread's 32 query columns (broadcast reads: every lane
                 // of the warp reads the same address)
                 const float4* st4 = reinterpret_cast<const float4*>(
@@ -794,10 +741,6 @@ attn_bwd_dkv_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
                 uint32_t pt[16], ptl[16], dst[16], dstl[16];
                 pack32<kSplit>(s, pt, ptl);
                 pack32<kSplit>(dp, dst, dstl);
-                if (t == 0 && it == 0) {
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(bar_stagger());
-                }
                 LTCA_TRACE_EVT(0x12 + (j << 8));
                 tmem_st16(tS, pt);
                 tmem_st16(tDP, dst);
@@ -808,14 +751,14 @@ attn_bwd_dkv_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
                 tmem_wait_st();
                 tc_fence_before_sync();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(bar_pds_full(t));
+                if (lane == 0) mbar_arrive(bar_pds_full());
                 LTCA_TRACE_EVT(0x13 + (j << 8));
             }
         }
         // epilogue: dV and scale * dK (zeros for tiles that no query can see)
-        if (ok && k0 < a.Sk) {
-            if (active[t]) {
-                ok = mbar_wait_warp(bar_acc_done(t), (uint32_t)((n_q - 1 - j_begin[t]) & 1), wc, 0x92 + t);
+        if (ok) {
+            if (active) {
+                ok = mbar_wait_warp(bar_acc_done(), (uint32_t)((n_q - 1 - j_first) & 1), wc, 0x92);
                 tc_fence_after_sync();
             }
             OutT* dkrow = reinterpret_cast<OutT*>(a.dk) + b * a.dks.batch + h * a.dks.head +
@@ -823,24 +766,24 @@ attn_bwd_dkv_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
             OutT* dvrow = reinterpret_cast<OutT*>(a.dv) + b * a.dvs.batch + h * a.dvs.head +
                           (int64_t)kj * a.dvs.seq + half * 32;
             uint32_t o[32];
-            if (active[t] && ok) { tmem_ld32(tDV, o); tmem_wait_ld(); }
+            if (active && ok) { tmem_ld32(tDV, o); tmem_wait_ld(); }
             else {
 #pragma unroll
                 for (int c = 0; c < 32; ++c) o[c] = 0u;
             }
             if (kj < a.Sk) store_row32<OutT>(dvrow, o, 1.0f);
-            if (active[t] && ok) { tmem_ld32(tDK, o); tmem_wait_ld(); }
+            if (active && ok) { tmem_ld32(tDK, o); tmem_wait_ld(); }
             if (kj < a.Sk) store_row32<OutT>(dkrow, o, a.scale);
         }
     }
 
     tc_fence_before_sync();
     __syncthreads();
-    if (warp == kMmaWarp0) {
+    if (warp == kTileMmaWarp) {
         __syncwarp();
         if (misc[1]) __nanosleep(200000);
         tc_fence_after_sync();
-        tmem_dealloc(tmem_base, kTmemCols);
+        tmem_dealloc(tmem_base, kTileTmemCols);
     }
 }
 
@@ -2412,12 +2355,13 @@ int launch_main(ltca_ctx* ctx, const ltca_attn_params* p, const void* mask_words
         static SmemOptIn opt_dq, opt_dkv;         // one pair per template instantiation
         LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(opt_dq, ctx->device, kdq, DqSmem::kDynBytes));
         LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(opt_dkv, ctx->device, kdkv, DkvSmem::kDynBytes));
-        dim3 gq((p->Sq + 2 * kTile - 1) / (2 * kTile), p->H, p->B);
-        LTCA_CUDA_OK(ctx, launch_dependent_if(small_attention_call(p), kdq, gq, dim3(kThreads), DqSmem::kDynBytes, ctx->stream, tq128, tdo128, tk64, tv64, a));
+        static_assert(2 * (DqSmem::kDynBytes + 1024) <= 228 * 1024 && 2 * (DkvSmem::kDynBytes + 1024) <= 228 * 1024, "two to an SM");
+        dim3 gq((p->Sq + kTile - 1) / kTile, p->H, p->B);
+        LTCA_CUDA_OK(ctx, launch_dependent_if(small_attention_call(p), kdq, gq, dim3(kTileThreads), DqSmem::kDynBytes, ctx->stream, tq128, tdo128, tk64, tv64, a));
         LTCA_LAUNCH_OK(ctx, "attn_bwd_dq_sm100_kernel");
         kernel_timing_mark(ctx, 2);
-        dim3 gk((p->Sk + 2 * kTile - 1) / (2 * kTile), p->H, p->B);
-        LTCA_CUDA_OK(ctx, launch_dependent_if(small_attention_call(p), kdkv, gk, dim3(kThreads), DkvSmem::kDynBytes, ctx->stream, tq64, tdo64, tk128, tv128, a));
+        dim3 gk((p->Sk + kTile - 1) / kTile, p->H, p->B);
+        LTCA_CUDA_OK(ctx, launch_dependent_if(small_attention_call(p), kdkv, gk, dim3(kTileThreads), DkvSmem::kDynBytes, ctx->stream, tq64, tdo64, tk128, tv128, a));
         LTCA_LAUNCH_OK(ctx, "attn_bwd_dkv_sm100_kernel");
     }
     kernel_timing_mark(ctx, 3);
