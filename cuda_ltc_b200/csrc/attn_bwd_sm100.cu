@@ -186,29 +186,23 @@ struct DkvSmem {
     static constexpr int kDynBytes = kMiscOff + 16 + 1024;
 };
 
-template <typename OutT>
-__device__ __forceinline__ void store_row32(OutT* dst, const uint32_t (&o)[32], float mul) {
-    if constexpr (sizeof(OutT) == 2) {
-        uint4* d = reinterpret_cast<uint4*>(dst);
+// Row `row` of a staged result box: 32 fp32 columns, 128 rows of 128 bytes, swizzled as the store's tensor map has it.  Stored
+// straight from registers, 16 bytes of 32 rows an instruction, the results held up the SM's shared memory: backward, us, stored
+// so and through TMA: B32 H8 S256 causal 75 -> 65, B64 H8 S200 131 -> 119, B4 H16 S1024 163 -> 152.
+__device__ __forceinline__ void stage_row32(uint8_t* box, int row, const uint32_t (&o)[32], float mul) {
 #pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            uint4 w;
-            w.x = pack_bf16x2(__uint_as_float(o[8 * v + 0]) * mul, __uint_as_float(o[8 * v + 1]) * mul);
-            w.y = pack_bf16x2(__uint_as_float(o[8 * v + 2]) * mul, __uint_as_float(o[8 * v + 3]) * mul);
-            w.z = pack_bf16x2(__uint_as_float(o[8 * v + 4]) * mul, __uint_as_float(o[8 * v + 5]) * mul);
-            w.w = pack_bf16x2(__uint_as_float(o[8 * v + 6]) * mul, __uint_as_float(o[8 * v + 7]) * mul);
-            d[v] = w;
-        }
-    } else {
-        float4* d = reinterpret_cast<float4*>(dst);
-#pragma unroll
-        for (int v = 0; v < 8; ++v)
-            d[v] = make_float4(__uint_as_float(o[4 * v + 0]) * mul, __uint_as_float(o[4 * v + 1]) * mul,
-                               __uint_as_float(o[4 * v + 2]) * mul, __uint_as_float(o[4 * v + 3]) * mul);
-    }
+    for (int v = 0; v < 8; ++v)
+        *reinterpret_cast<float4*>(box + row * 128 + ((v ^ (row & 7)) << 4)) =
+            make_float4(__uint_as_float(o[4 * v + 0]) * mul, __uint_as_float(o[4 * v + 1]) * mul,
+                        __uint_as_float(o[4 * v + 2]) * mul, __uint_as_float(o[4 * v + 3]) * mul);
+}
+// Behind the staging of a tile's result by all elementwise warps: its boxes may be stored.
+__device__ __forceinline__ void tile_staged() {
+    fence_proxy_async_smem();
+    asm volatile("bar.sync 1, 256;" ::: "memory");
 }
 
-// Packs 32 fp32 values into 16 bf16 pairs (and, for the split variants, the rounding residue).
+// Packs 32 fp32 values into 16 bf16 pairs (kSplit: and what their rounding left into 16 more).
 template <bool kSplit>
 __device__ __forceinline__ void pack32(const uint32_t (&v)[32], uint32_t (&hi)[16], uint32_t (&lo)[16]) {
 #pragma unroll
@@ -223,18 +217,18 @@ __device__ __forceinline__ void pack32(const uint32_t (&v)[32], uint32_t (&hi)[1
 
 // ---------------------------------------------------------------------------------------------
 // 2. dQ
-// tensor memory: S [0,64)  dP [64,128)  dQ [128,192)  dS (bf16) [192,224), its low-order term (kSplit) [224,256).
+// tensor memory: S [0,64)  dP [64,128)  dQ [128,192)  dS (bf16) [192,224), its low-order term [224,256).
 // A query row belongs to two threads (warps w and w + 4), each owning 32 of the step's 64 keys.
 // ---------------------------------------------------------------------------------------------
-// kSplit (fp32 gradients out): dS is written as two bf16 terms and the dQ contraction runs once
-// per term, so that the 2^-9 rounding of a single bf16 dS does not dominate the error of an fp32
-// result.
-template <typename OutT, bool kSplit, bool kMask>
+// dS is written as two bf16 terms and the dQ contraction runs once per term, so that the 2^-9 rounding of a single bf16 dS does
+// not dominate the error of an fp32 result.
+template <bool kMask>
 __global__ void __launch_bounds__(kTileThreads, 2)
 attn_bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
                          const __grid_constant__ CUtensorMap tmap_do,
                          const __grid_constant__ CUtensorMap tmap_k,
-                         const __grid_constant__ CUtensorMap tmap_v, const BwdArgs a) {
+                         const __grid_constant__ CUtensorMap tmap_v,
+                         const __grid_constant__ CUtensorMap tmap_dq, const BwdArgs a) {
     using L = DqSmem;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -331,11 +325,9 @@ attn_bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
 #pragma unroll
                 for (int k = 0; k < kStep / 16; ++k)
                     mma_ts(tb + 128, ds_hi + k * 8, kd + 128 * k, idesc_dq, (acc || k > 0) ? 1u : 0u);
-                if constexpr (kSplit) {
 #pragma unroll
-                    for (int k = 0; k < kStep / 16; ++k)
-                        mma_ts(tb + 128, ds_lo + k * 8, kd + 128 * k, idesc_dq, 1u);
-                }
+                for (int k = 0; k < kStep / 16; ++k)
+                    mma_ts(tb + 128, ds_lo + k * 8, kd + 128 * k, idesc_dq, 1u);
             };
             bool ok = mbar_wait(bar_qdo_full(), 0, wc, 0x50);
             ok = ok && mbar_wait(bar_ring_full(slot_of(0)), phase_of(0), wc, 0x51);
@@ -443,7 +435,7 @@ attn_bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
                 }
             }
             uint32_t hi[16], lo[16];
-            pack32<kSplit>(dp, hi, lo);
+            pack32<true>(dp, hi, lo);
             LTCA_TRACE_EVT(0x12 + (j << 8));
             if (j > 0) {
                 // the previous dS must have been consumed before it is overwritten
@@ -451,7 +443,7 @@ attn_bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
                 if (!ok) break;
             }
             tmem_st16(tDS, hi);
-            if constexpr (kSplit) tmem_st16(tDSlo, lo);
+            tmem_st16(tDSlo, lo);
             tmem_wait_st();
             tc_fence_before_sync();
             __syncwarp();
@@ -463,15 +455,20 @@ attn_bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
                 ok = mbar_wait_warp(bar_dq_done(), (uint32_t)((n - 1) & 1), wc, 0x62);
                 tc_fence_after_sync();
             }
-            OutT* drow = reinterpret_cast<OutT*>(a.dq) + b * a.dqs.batch + h * a.dqs.head +
-                         (int64_t)qi * a.dqs.seq + half * 32;
             uint32_t o[32];
             if (n > 0 && ok) { tmem_ld32(tDQ, o); tmem_wait_ld(); }
             else {
 #pragma unroll
                 for (int c = 0; c < 32; ++c) o[c] = 0u;
             }
-            if (qi < a.Sq) store_row32<OutT>(drow, o, a.scale);
+            stage_row32(smem_gen + half * kBigTile, row, o, a.scale);      // over Q and dO, which every product has read
+        }
+        tile_staged();
+        if (warp == 0 && lane == 0 && ok) {
+            tma_store_4d(&tmap_dq, smem_base, 0, q0, h, b);
+            tma_store_4d(&tmap_dq, smem_base + kBigTile, 32, q0, h, b);
+            tma_store_commit();
+            tma_store_wait_read<0>();
         }
     }
 
@@ -490,15 +487,17 @@ attn_bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
 // tensor memory: S^T [0,64) dP^T [64,128) dV [128,192) dK [192,256).
 // A key row belongs to two threads (warps w and w + 4); thread `half` owns query columns
 // [32*half, 32*half + 32) of S^T and dP^T and writes its P^T / dS^T back INSIDE those columns
-// (bf16 pairs in the first 16, the kSplit low-order term in the next 16), so neither thread
+// (bf16 pairs in the first 16, their low-order term in the next 16), so neither thread
 // ever overwrites scores the other has not read yet.
 // ---------------------------------------------------------------------------------------------
-template <typename OutT, bool kSplit, bool kMask>
+template <bool kMask>
 __global__ void __launch_bounds__(kTileThreads, 2)
 attn_bwd_dkv_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
                           const __grid_constant__ CUtensorMap tmap_do,
                           const __grid_constant__ CUtensorMap tmap_k,
-                          const __grid_constant__ CUtensorMap tmap_v, const BwdArgs a) {
+                          const __grid_constant__ CUtensorMap tmap_v,
+                          const __grid_constant__ CUtensorMap tmap_dk,
+                          const __grid_constant__ CUtensorMap tmap_dv, const BwdArgs a) {
     using L = DkvSmem;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -607,14 +606,12 @@ attn_bwd_dkv_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
                 for (int k = 0; k < kStep / 16; ++k)
                     mma_ts(tb + 192, tb + 64 + (k / 2) * 32 + (k % 2) * 8, qd + 128 * k, idesc_acc,
                            (acc || k > 0) ? 1u : 0u);
-                if constexpr (kSplit) {
 #pragma unroll
-                    for (int k = 0; k < kStep / 16; ++k)
-                        mma_ts(tb + 128, tb + 16 + (k / 2) * 32 + (k % 2) * 8, gd + 128 * k, idesc_acc, 1u);
+                for (int k = 0; k < kStep / 16; ++k)
+                    mma_ts(tb + 128, tb + 16 + (k / 2) * 32 + (k % 2) * 8, gd + 128 * k, idesc_acc, 1u);
 #pragma unroll
-                    for (int k = 0; k < kStep / 16; ++k)
-                        mma_ts(tb + 192, tb + 80 + (k / 2) * 32 + (k % 2) * 8, qd + 128 * k, idesc_acc, 1u);
-                }
+                for (int k = 0; k < kStep / 16; ++k)
+                    mma_ts(tb + 192, tb + 80 + (k / 2) * 32 + (k % 2) * 8, qd + 128 * k, idesc_acc, 1u);
             };
             bool ok = mbar_wait(bar_kv_full(), 0, wc, 0x80);
             ok = ok && mbar_wait(bar_ring_full(slot_of(j_first)), phase_of(j_first), wc, 0x81);
@@ -739,15 +736,13 @@ attn_bwd_dkv_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
                     }
                 }
                 uint32_t pt[16], ptl[16], dst[16], dstl[16];
-                pack32<kSplit>(s, pt, ptl);
-                pack32<kSplit>(dp, dst, dstl);
+                pack32<true>(s, pt, ptl);
+                pack32<true>(dp, dst, dstl);
                 LTCA_TRACE_EVT(0x12 + (j << 8));
                 tmem_st16(tS, pt);
                 tmem_st16(tDP, dst);
-                if constexpr (kSplit) {
-                    tmem_st16(tS + 16, ptl);
-                    tmem_st16(tDP + 16, dstl);
-                }
+                tmem_st16(tS + 16, ptl);
+                tmem_st16(tDP + 16, dstl);
                 tmem_wait_st();
                 tc_fence_before_sync();
                 __syncwarp();
@@ -761,19 +756,25 @@ attn_bwd_dkv_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
                 ok = mbar_wait_warp(bar_acc_done(), (uint32_t)((n_q - 1 - j_first) & 1), wc, 0x92);
                 tc_fence_after_sync();
             }
-            OutT* dkrow = reinterpret_cast<OutT*>(a.dk) + b * a.dks.batch + h * a.dks.head +
-                          (int64_t)kj * a.dks.seq + half * 32;
-            OutT* dvrow = reinterpret_cast<OutT*>(a.dv) + b * a.dvs.batch + h * a.dvs.head +
-                          (int64_t)kj * a.dvs.seq + half * 32;
             uint32_t o[32];
             if (active && ok) { tmem_ld32(tDV, o); tmem_wait_ld(); }
             else {
 #pragma unroll
                 for (int c = 0; c < 32; ++c) o[c] = 0u;
             }
-            if (kj < a.Sk) store_row32<OutT>(dvrow, o, 1.0f);
+            stage_row32(smem_gen + half * kBigTile, row, o, 1.0f);         // over K and V, and dK over the ring: all have been read
             if (active && ok) { tmem_ld32(tDK, o); tmem_wait_ld(); }
-            if (kj < a.Sk) store_row32<OutT>(dkrow, o, a.scale);
+            stage_row32(smem_gen + L::kRingOff + half * kBigTile, row, o, a.scale);
+        }
+        tile_staged();
+        if (warp == 0 && lane == 0 && ok) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                tma_store_4d(&tmap_dv, smem_base + i * kBigTile, 32 * i, k0, h, b);
+                tma_store_4d(&tmap_dk, smem_base + L::kRingOff + i * kBigTile, 32 * i, k0, h, b);
+            }
+            tma_store_commit();
+            tma_store_wait_read<0>();
         }
     }
 
@@ -2350,18 +2351,22 @@ int launch_main(ltca_ctx* ctx, const ltca_attn_params* p, const void* mask_words
             LTCA_LAUNCH_OK(ctx, "attn_bwd_dkv4_sm100_kernel");
         }
     } else {
-        auto kdq = attn_bwd_dq_sm100_kernel<OutT, sizeof(OutT) == 4, kMask>;
-        auto kdkv = attn_bwd_dkv_sm100_kernel<OutT, sizeof(OutT) == 4, kMask>;
+        auto kdq = attn_bwd_dq_sm100_kernel<kMask>;
+        auto kdkv = attn_bwd_dkv_sm100_kernel<kMask>;
+        CUtensorMap tdq, tdk, tdv;
+        if ((rc = make_tmap_bhsd(ctx, &tdq, p->dq, 4, p->B, p->H, p->Sq, kD, p->dq_strides, 32, kTile))) return rc;
+        if ((rc = make_tmap_bhsd(ctx, &tdk, p->dk, 4, p->B, p->H, p->Sk, kD, p->dk_strides, 32, kTile))) return rc;
+        if ((rc = make_tmap_bhsd(ctx, &tdv, p->dv, 4, p->B, p->H, p->Sk, kD, p->dv_strides, 32, kTile))) return rc;
         static SmemOptIn opt_dq, opt_dkv;         // one pair per template instantiation
         LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(opt_dq, ctx->device, kdq, DqSmem::kDynBytes));
         LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(opt_dkv, ctx->device, kdkv, DkvSmem::kDynBytes));
         static_assert(2 * (DqSmem::kDynBytes + 1024) <= 228 * 1024 && 2 * (DkvSmem::kDynBytes + 1024) <= 228 * 1024, "two to an SM");
         dim3 gq((p->Sq + kTile - 1) / kTile, p->H, p->B);
-        LTCA_CUDA_OK(ctx, launch_dependent_if(small_attention_call(p), kdq, gq, dim3(kTileThreads), DqSmem::kDynBytes, ctx->stream, tq128, tdo128, tk64, tv64, a));
+        LTCA_CUDA_OK(ctx, launch_dependent_if(small_attention_call(p), kdq, gq, dim3(kTileThreads), DqSmem::kDynBytes, ctx->stream, tq128, tdo128, tk64, tv64, tdq, a));
         LTCA_LAUNCH_OK(ctx, "attn_bwd_dq_sm100_kernel");
         kernel_timing_mark(ctx, 2);
         dim3 gk((p->Sk + kTile - 1) / kTile, p->H, p->B);
-        LTCA_CUDA_OK(ctx, launch_dependent_if(small_attention_call(p), kdkv, gk, dim3(kTileThreads), DkvSmem::kDynBytes, ctx->stream, tq64, tdo64, tk128, tv128, a));
+        LTCA_CUDA_OK(ctx, launch_dependent_if(small_attention_call(p), kdkv, gk, dim3(kTileThreads), DkvSmem::kDynBytes, ctx->stream, tq64, tdo64, tk128, tv128, tdk, tdv, a));
         LTCA_LAUNCH_OK(ctx, "attn_bwd_dkv_sm100_kernel");
     }
     kernel_timing_mark(ctx, 3);
