@@ -6,22 +6,21 @@
 // The reference reaches this arithmetic through cudnnMultiHeadAttnBackwardData
 // (reference src/ml/cuDNN_ops.cu:240-337); its FlashAttention class has no backward.
 //
-// Three launches, no atomics (two runs give identical bits; the reference's tests pin backward
+// No atomics on a result but in the one-kernel form below (two runs give identical bits; the reference's tests pin backward
 // repeatability, src/ml/time_self_attention_test.cu:799-838):
 //   1. attn_bwd_stats_kernel: delta and lse * log2(e) into padded [B*H, Sq_pad] fp32 rows
 //      (padding and fully hidden rows get lse = +inf so that their P is exactly 0).
-//   2. attn_bwd_dq_sm100_kernel: one CTA per 128 query rows; Q and dO stay in shared
-//      memory, K/V stream through a ring in 64-key steps.  Per step:
-//      S = Q K^T and dP = dO V^T into tensor memory, the elementwise warps (one query row per
-//      two threads) turn them into dS (bf16, two terms), and dQ += dS K takes dS from
-//      tensor memory and K as an MN-major operand from shared memory.
-//   3. attn_bwd_dkv_sm100_kernel: the transposed problem, one CTA per 128 keys; K and V
-//      stay in shared memory, Q/dO (and the per-row statistics) stream in 64-query steps.
+//   2. attn_bwd_dkv_sm100_kernel, a CTA per 128-row tile, of two kinds:
+//      dK/dV, 128 keys: K and V stay in shared memory, Q/dO (and the per-row statistics) stream in 64-query steps.
 //      S^T = K Q^T and dP^T = V dO^T put one KEY per tensor-memory lane, so P^T and dS^T are
 //      directly the A operands of dV += P^T dO and dK += dS^T Q.
-// (2 and 3 for fp32 results; bf16 results have kernels of their own further down.)  Warps 0-7 elementwise, warp 8
-// issues tcgen05.mma, warp 9 drives TMA; two CTAs share an SM, so one's elementwise work overlaps the
-// other's contractions.  Every wait is bounded.
+//      dQ, 128 queries: Q and dO stay in shared memory, K/V stream through a ring in 64-key steps.  Per step:
+//      S = Q K^T and dP = dO V^T into tensor memory, the elementwise warps (one query row per
+//      two threads) turn them into dS (bf16), and dQ += dS K takes dS from
+//      tensor memory and K as an MN-major operand from shared memory.
+//      Warps 0-7 elementwise, warp 8 issues tcgen05.mma, warp 9 drives TMA; two CTAs share an SM, so one's
+//      elementwise work overlaps the other's contractions.  Every wait is bounded.
+// Long sequences with bf16 results have persistent kernels of their own further down (bwd_in_tiles).
 #include <type_traits>
 
 #include "host_common.h"
@@ -46,10 +45,11 @@ constexpr int kCtrlRegs = 56;        // kept by the TMA / MMA-issue warps
 constexpr int kMathRegs = 104;       // taken by the elementwise warps
 // setmaxnreg can only redistribute what the CTA was launched with; asking for more never returns
 static_assert(512 * kMathRegs + 128 * kCtrlRegs <= kThreads * kLaunchRegs, "register budget");
-// dQ and dK/dV for fp32 results: a CTA per 128-row tile, two to an SM, heaviest tiles first.  As one CTA with two neighbouring
-// tiles (the tensor memory and warps of both) a causal pair of tiles took the time of its longer one and a launch ended on whole
-// pairs; a tile of a CTA's own also hides its set-up and its result's store under the other's steps.  Backward, us: B32 H8 S256
-// causal 79 -> 75, B12 H8 S384 76 -> 48, B1 H16 S4096 causal 447 -> 258, B64 H8 S64 52 -> 37.
+// A CTA per 128-row tile, two to an SM, heaviest tiles first.  As one CTA with two neighbouring tiles (the tensor memory and warps of
+// both) a causal pair of tiles took the time of its longer one and a launch ended on whole pairs; a tile of a CTA's own also hides
+// its set-up and its result's store under the other's steps.  Backward with fp32 results, us: B32 H8 S256 causal 79 -> 75,
+// B12 H8 S384 76 -> 48, B1 H16 S4096 causal 447 -> 258, B64 H8 S64 52 -> 37.  dQ's tiles and dK/dV's in one launch instead of two:
+// B32 H8 S256 causal 65 -> 59, B1 H8 S300 25 -> 16, B4 H16 S1024 causal 121 -> 101, B2 H2 S2048 98 -> 64.
 constexpr int kTileThreads = 384;    // 8 elementwise warps + one warpgroup of control warps
 constexpr int kTileMmaWarp = 8, kTileTmaWarp = 9;
 constexpr uint32_t kTileTmemCols = 256;
@@ -59,6 +59,8 @@ static_assert(2 * kTileThreads * kTileLaunchRegs <= 65536, "two to an SM");
 constexpr int kBigTile = kTile * kD * 2;      // 16 KB
 constexpr int kSmallTile = kStep * kD * 2;    // 8 KB
 
+// The operands in tiles of 128 rows and of 64, and the results.
+struct BwdMaps { CUtensorMap q128, do128, k128, v128, q64, do64, k64, v64, dq, dk, dv; };
 struct BwdArgs {
     int B, H, Sq, Sk, Sq_pad;
     int causal, causal_off;
@@ -186,15 +188,30 @@ struct DkvSmem {
     static constexpr int kDynBytes = kMiscOff + 16 + 1024;
 };
 
-// Row `row` of a staged result box: 32 fp32 columns, 128 rows of 128 bytes, swizzled as the store's tensor map has it.  Stored
-// straight from registers, 16 bytes of 32 rows an instruction, the results held up the SM's shared memory: backward, us, stored
-// so and through TMA: B32 H8 S256 causal 75 -> 65, B64 H8 S200 131 -> 119, B4 H16 S1024 163 -> 152.
-__device__ __forceinline__ void stage_row32(uint8_t* box, int row, const uint32_t (&o)[32], float mul) {
+// Half a row (32 columns) of a staged result: boxes of 128 rows of 128 bytes, swizzled as the store's tensor map has it, one box of
+// all columns in bf16, a box a half in fp32.  Stored straight from registers, 16 bytes of 32 rows an instruction, the results held
+// up the SM's shared memory: backward with fp32 results, us, stored so and through TMA: B32 H8 S256 causal 75 -> 65, B64 H8 S200
+// 131 -> 119, B4 H16 S1024 163 -> 152.
+template <typename OutT>
+__device__ __forceinline__ void stage_half(uint8_t* tile, int half, int row, const uint32_t (&o)[32], float mul) {
+    auto f = [&](int i) { return __uint_as_float(o[i]) * mul; };
+    if constexpr (sizeof(OutT) == 4) {
 #pragma unroll
-    for (int v = 0; v < 8; ++v)
-        *reinterpret_cast<float4*>(box + row * 128 + ((v ^ (row & 7)) << 4)) =
-            make_float4(__uint_as_float(o[4 * v + 0]) * mul, __uint_as_float(o[4 * v + 1]) * mul,
-                        __uint_as_float(o[4 * v + 2]) * mul, __uint_as_float(o[4 * v + 3]) * mul);
+        for (int v = 0; v < 8; ++v)
+            *reinterpret_cast<float4*>(tile + half * kBigTile + row * 128 + ((v ^ (row & 7)) << 4)) =
+                make_float4(f(4 * v), f(4 * v + 1), f(4 * v + 2), f(4 * v + 3));
+    } else {
+#pragma unroll
+        for (int v = 0; v < 4; ++v)
+            *reinterpret_cast<uint4*>(tile + row * 128 + (((4 * half + v) ^ (row & 7)) << 4)) =
+                make_uint4(pack_bf16x2(f(8 * v), f(8 * v + 1)), pack_bf16x2(f(8 * v + 2), f(8 * v + 3)),
+                           pack_bf16x2(f(8 * v + 4), f(8 * v + 5)), pack_bf16x2(f(8 * v + 6), f(8 * v + 7)));
+    }
+}
+template <typename OutT>
+__device__ __forceinline__ void store_tile(const CUtensorMap* map, uint32_t tile, int row0, int h, int b) {
+    tma_store_4d(map, tile, 0, row0, h, b);
+    if constexpr (sizeof(OutT) == 4) tma_store_4d(map, tile + kBigTile, 32, row0, h, b);
 }
 // Behind the staging of a tile's result by all elementwise warps: its boxes may be stored.
 __device__ __forceinline__ void tile_staged() {
@@ -222,14 +239,10 @@ __device__ __forceinline__ void pack32(const uint32_t (&v)[32], uint32_t (&hi)[1
 // ---------------------------------------------------------------------------------------------
 // dS is written as two bf16 terms and the dQ contraction runs once per term, so that the 2^-9 rounding of a single bf16 dS does
 // not dominate the error of an fp32 result.
-template <bool kMask>
-__global__ void __launch_bounds__(kTileThreads, 2)
-attn_bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
-                         const __grid_constant__ CUtensorMap tmap_do,
-                         const __grid_constant__ CUtensorMap tmap_k,
-                         const __grid_constant__ CUtensorMap tmap_v,
-                         const __grid_constant__ CUtensorMap tmap_dq, const BwdArgs a) {
+template <typename OutT, bool kMask, typename Wait>
+__device__ __forceinline__ void dq_tile(const BwdMaps& m, const BwdArgs& a, int q0, int h, int b, const Wait& wait) {
     using L = DqSmem;
+    constexpr bool kSplit = sizeof(OutT) == 4;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -245,13 +258,9 @@ attn_bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
     volatile uint32_t* misc = reinterpret_cast<volatile uint32_t*>(smem_gen + L::kMiscOff);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    int rank, h, b;
-    sched_block(rank, h, b, kSchedGroup);
-    const int q0 = (gridDim.x - 1 - rank) * kTile;  // late queries see the most keys
-
     int kvlen = a.Sk;
     if (a.kv_len) {
-        grid_dependency_wait();                // the lengths may come from the kernel before this one
+        wait();                // the lengths may come from the kernel before this one
         kvlen = min(max(a.kv_len[b], 0), a.Sk);
     }
     int lim_all = kvlen;
@@ -274,7 +283,7 @@ attn_bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
     tc_fence_after_sync();
     const uint32_t tmem_base = misc[0];
     const WaitCtx wc{&misc[1], a.status};
-    grid_dependency_wait();                    // the operands are complete once the kernel before this one has ended
+    wait();                    // the operands are complete once the kernel before this one has ended
     auto slot_of = [&](int item) { return item % L::kStages; };
     auto phase_of = [&](int item) { return (uint32_t)((item / L::kStages) & 1); };
     LTCA_TRACE_DECL(LTCA_TRACE_KERNEL == 1 && blockIdx.x == 0 && blockIdx.y == 5 && blockIdx.z == 0);
@@ -285,8 +294,8 @@ attn_bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
       if (warp == kTileTmaWarp) {
         if (lane == 0 && n > 0) {
             mbar_arrive_expect_tx(bar_qdo_full(), 2u * kBigTile);
-            tma_load_4d(q_smem, &tmap_q, bar_qdo_full(), 0, q0, h, b);
-            tma_load_4d(do_smem, &tmap_do, bar_qdo_full(), 0, q0, h, b);
+            tma_load_4d(q_smem, &m.q128, bar_qdo_full(), 0, q0, h, b);
+            tma_load_4d(do_smem, &m.do128, bar_qdo_full(), 0, q0, h, b);
             bool ok = true;
             for (int j = 0; j < n && ok; ++j) {
 #pragma unroll
@@ -295,7 +304,7 @@ attn_bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
                     ok = ok && mbar_wait(bar_ring_empty(slot_of(item)), phase_of(item) ^ 1u, wc, 0x40 + which);
                     if (!ok) break;
                     mbar_arrive_expect_tx(bar_ring_full(slot_of(item)), (uint32_t)kSmallTile);
-                    tma_load_4d(ring_smem + slot_of(item) * kSmallTile, which == 0 ? &tmap_k : &tmap_v,
+                    tma_load_4d(ring_smem + slot_of(item) * kSmallTile, which == 0 ? &m.k64 : &m.v64,
                                 bar_ring_full(slot_of(item)), 0, j * kStep, h, b);
                 }
             }
@@ -325,9 +334,11 @@ attn_bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
 #pragma unroll
                 for (int k = 0; k < kStep / 16; ++k)
                     mma_ts(tb + 128, ds_hi + k * 8, kd + 128 * k, idesc_dq, (acc || k > 0) ? 1u : 0u);
+                if constexpr (kSplit) {
 #pragma unroll
-                for (int k = 0; k < kStep / 16; ++k)
-                    mma_ts(tb + 128, ds_lo + k * 8, kd + 128 * k, idesc_dq, 1u);
+                    for (int k = 0; k < kStep / 16; ++k)
+                        mma_ts(tb + 128, ds_lo + k * 8, kd + 128 * k, idesc_dq, 1u);
+                }
             };
             bool ok = mbar_wait(bar_qdo_full(), 0, wc, 0x50);
             ok = ok && mbar_wait(bar_ring_full(slot_of(0)), phase_of(0), wc, 0x51);
@@ -435,7 +446,7 @@ attn_bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
                 }
             }
             uint32_t hi[16], lo[16];
-            pack32<true>(dp, hi, lo);
+            pack32<kSplit>(dp, hi, lo);
             LTCA_TRACE_EVT(0x12 + (j << 8));
             if (j > 0) {
                 // the previous dS must have been consumed before it is overwritten
@@ -443,7 +454,7 @@ attn_bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
                 if (!ok) break;
             }
             tmem_st16(tDS, hi);
-            tmem_st16(tDSlo, lo);
+            if constexpr (kSplit) tmem_st16(tDSlo, lo);
             tmem_wait_st();
             tc_fence_before_sync();
             __syncwarp();
@@ -461,12 +472,11 @@ attn_bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
 #pragma unroll
                 for (int c = 0; c < 32; ++c) o[c] = 0u;
             }
-            stage_row32(smem_gen + half * kBigTile, row, o, a.scale);      // over Q and dO, which every product has read
+            stage_half<OutT>(smem_gen, half, row, o, a.scale);             // over Q and dO, which every product has read
         }
         tile_staged();
         if (warp == 0 && lane == 0 && ok) {
-            tma_store_4d(&tmap_dq, smem_base, 0, q0, h, b);
-            tma_store_4d(&tmap_dq, smem_base + kBigTile, 32, q0, h, b);
+            store_tile<OutT>(&m.dq, smem_base, q0, h, b);
             tma_store_commit();
             tma_store_wait_read<0>();
         }
@@ -490,15 +500,10 @@ attn_bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
 // (bf16 pairs in the first 16, their low-order term in the next 16), so neither thread
 // ever overwrites scores the other has not read yet.
 // ---------------------------------------------------------------------------------------------
-template <bool kMask>
-__global__ void __launch_bounds__(kTileThreads, 2)
-attn_bwd_dkv_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
-                          const __grid_constant__ CUtensorMap tmap_do,
-                          const __grid_constant__ CUtensorMap tmap_k,
-                          const __grid_constant__ CUtensorMap tmap_v,
-                          const __grid_constant__ CUtensorMap tmap_dk,
-                          const __grid_constant__ CUtensorMap tmap_dv, const BwdArgs a) {
+template <typename OutT, bool kMask, typename Wait>
+__device__ __forceinline__ void dkv_tile(const BwdMaps& m, const BwdArgs& a, int k0, int h, int b, const Wait& wait) {
     using L = DkvSmem;
+    constexpr bool kSplit = sizeof(OutT) == 4;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -513,13 +518,9 @@ attn_bwd_dkv_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
     volatile uint32_t* misc = reinterpret_cast<volatile uint32_t*>(smem_gen + L::kMiscOff);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    int rank, h, b;
-    sched_block(rank, h, b, kSchedGroup);
-    const int k0 = rank * kTile;                    // early keys are seen by the most queries
-
     int kvlen = a.Sk;
     if (a.kv_len) {
-        grid_dependency_wait();                // the lengths may come from the kernel before this one
+        wait();                // the lengths may come from the kernel before this one
         kvlen = min(max(a.kv_len[b], 0), a.Sk);
     }
     const int n_q = (a.Sq + kStep - 1) / kStep;     // query steps in total
@@ -541,7 +542,7 @@ attn_bwd_dkv_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
     tc_fence_after_sync();
     const uint32_t tmem_base = misc[0];
     const WaitCtx wc{&misc[1], a.status};
-    grid_dependency_wait();                    // the operands are complete once the kernel before this one has ended
+    wait();                    // the operands are complete once the kernel before this one has ended
     // ring items are numbered from the first streamed step of this CTA
     auto slot_of = [&](int j) { return (j - j_first) % L::kStages; };
     auto phase_of = [&](int j) { return (uint32_t)(((j - j_first) / L::kStages) & 1); };
@@ -553,8 +554,8 @@ attn_bwd_dkv_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
       if (warp == kTileTmaWarp) {
         if (lane == 0 && active) {
             mbar_arrive_expect_tx(bar_kv_full(), 2u * kBigTile);
-            tma_load_4d(k_smem, &tmap_k, bar_kv_full(), 0, k0, h, b);
-            tma_load_4d(v_smem, &tmap_v, bar_kv_full(), 0, k0, h, b);
+            tma_load_4d(k_smem, &m.k128, bar_kv_full(), 0, k0, h, b);
+            tma_load_4d(v_smem, &m.v128, bar_kv_full(), 0, k0, h, b);
             const float* lse2_row = a.lse2 + ((int64_t)b * a.H + h) * a.Sq_pad;
             const float* dlt_row = a.delta + ((int64_t)b * a.H + h) * a.Sq_pad;
             bool ok = true;
@@ -563,8 +564,8 @@ attn_bwd_dkv_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
                 if (!ok) break;
                 const uint32_t st = ring_smem + slot_of(j) * L::kStageBytes;
                 mbar_arrive_expect_tx(bar_ring_full(slot_of(j)), 2u * kSmallTile + 512u);
-                tma_load_4d(st, &tmap_q, bar_ring_full(slot_of(j)), 0, j * kStep, h, b);
-                tma_load_4d(st + kSmallTile, &tmap_do, bar_ring_full(slot_of(j)), 0, j * kStep, h, b);
+                tma_load_4d(st, &m.q64, bar_ring_full(slot_of(j)), 0, j * kStep, h, b);
+                tma_load_4d(st + kSmallTile, &m.do64, bar_ring_full(slot_of(j)), 0, j * kStep, h, b);
                 asm volatile(
                     "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], 256, [%2];"
                     ::"r"(st + 2 * kSmallTile), "l"(reinterpret_cast<uint64_t>(lse2_row + j * kStep)),
@@ -606,12 +607,14 @@ attn_bwd_dkv_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
                 for (int k = 0; k < kStep / 16; ++k)
                     mma_ts(tb + 192, tb + 64 + (k / 2) * 32 + (k % 2) * 8, qd + 128 * k, idesc_acc,
                            (acc || k > 0) ? 1u : 0u);
+                if constexpr (kSplit) {
 #pragma unroll
-                for (int k = 0; k < kStep / 16; ++k)
-                    mma_ts(tb + 128, tb + 16 + (k / 2) * 32 + (k % 2) * 8, gd + 128 * k, idesc_acc, 1u);
+                    for (int k = 0; k < kStep / 16; ++k)
+                        mma_ts(tb + 128, tb + 16 + (k / 2) * 32 + (k % 2) * 8, gd + 128 * k, idesc_acc, 1u);
 #pragma unroll
-                for (int k = 0; k < kStep / 16; ++k)
-                    mma_ts(tb + 192, tb + 80 + (k / 2) * 32 + (k % 2) * 8, qd + 128 * k, idesc_acc, 1u);
+                    for (int k = 0; k < kStep / 16; ++k)
+                        mma_ts(tb + 192, tb + 80 + (k / 2) * 32 + (k % 2) * 8, qd + 128 * k, idesc_acc, 1u);
+                }
             };
             bool ok = mbar_wait(bar_kv_full(), 0, wc, 0x80);
             ok = ok && mbar_wait(bar_ring_full(slot_of(j_first)), phase_of(j_first), wc, 0x81);
@@ -736,13 +739,15 @@ attn_bwd_dkv_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
                     }
                 }
                 uint32_t pt[16], ptl[16], dst[16], dstl[16];
-                pack32<true>(s, pt, ptl);
-                pack32<true>(dp, dst, dstl);
+                pack32<kSplit>(s, pt, ptl);
+                pack32<kSplit>(dp, dst, dstl);
                 LTCA_TRACE_EVT(0x12 + (j << 8));
                 tmem_st16(tS, pt);
                 tmem_st16(tDP, dst);
-                tmem_st16(tS + 16, ptl);
-                tmem_st16(tDP + 16, dstl);
+                if constexpr (kSplit) {
+                    tmem_st16(tS + 16, ptl);
+                    tmem_st16(tDP + 16, dstl);
+                }
                 tmem_wait_st();
                 tc_fence_before_sync();
                 __syncwarp();
@@ -762,17 +767,14 @@ attn_bwd_dkv_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
 #pragma unroll
                 for (int c = 0; c < 32; ++c) o[c] = 0u;
             }
-            stage_row32(smem_gen + half * kBigTile, row, o, 1.0f);         // over K and V, and dK over the ring: all have been read
+            stage_half<OutT>(smem_gen, half, row, o, 1.0f);                // over K and V, and dK over the ring: all have been read
             if (active && ok) { tmem_ld32(tDK, o); tmem_wait_ld(); }
-            stage_row32(smem_gen + L::kRingOff + half * kBigTile, row, o, a.scale);
+            stage_half<OutT>(smem_gen + L::kRingOff, half, row, o, a.scale);
         }
         tile_staged();
         if (warp == 0 && lane == 0 && ok) {
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                tma_store_4d(&tmap_dv, smem_base + i * kBigTile, 32 * i, k0, h, b);
-                tma_store_4d(&tmap_dk, smem_base + L::kRingOff + i * kBigTile, 32 * i, k0, h, b);
-            }
+            store_tile<OutT>(&m.dv, smem_base, k0, h, b);
+            store_tile<OutT>(&m.dk, smem_base + L::kRingOff, k0, h, b);
             tma_store_commit();
             tma_store_wait_read<0>();
         }
@@ -785,6 +787,23 @@ attn_bwd_dkv_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
         if (misc[1]) __nanosleep(200000);
         tc_fence_after_sync();
         tmem_dealloc(tmem_base, kTileTmemCols);
+    }
+}
+
+// dK/dV's tiles and dQ's in one launch, dK/dV's (the longer ones) first, each heaviest first.
+template <typename OutT, bool kMask>
+__global__ void __launch_bounds__(kTileThreads, 2)
+attn_bwd_dkv_sm100_kernel(const __grid_constant__ BwdMaps m, const __grid_constant__ BwdArgs a, const __grid_constant__ ItemGrid keys,
+                          const __grid_constant__ ItemGrid queries) {
+    const auto wait = [] { grid_dependency_wait(); };
+    int rank, h, b;
+    const int item = (int)blockIdx.x - keys.n_items;
+    if (item < 0) {
+        sched_item(keys, blockIdx.x, rank, h, b);
+        dkv_tile<OutT, kMask>(m, a, rank * kTile, h, b, wait);                         // early keys are seen by the most queries
+    } else {
+        sched_item(queries, item, rank, h, b);
+        dq_tile<OutT, kMask>(m, a, (queries.nblk - 1 - rank) * kTile, h, b, wait);     // late queries see the most keys
     }
 }
 
@@ -2244,24 +2263,45 @@ size_t dq_acc_bytes(const ltca_attn_params* p) {
     return align_up((size_t)p->B * p->H * sq_pad * kD * sizeof(float), 256);
 }
 
-// The fused kernel serves bf16 storage unless the caller asks for bit-reproducible dQ.  (At 512 queries and fewer
-// the two paths are within 5 % of each other, in the fused kernel's favour when the inputs come from HBM.)
+// The fused kernel serves bf16 storage unless the caller asks for bit-reproducible dQ, or the call is short (bwd_in_tiles): its
+// accumulator is part of the workspace in either case.
 bool use_fused(const ltca_attn_params* p) { return p->dtype == LTCA_BF16 && !p->bwd_deterministic; }
+
+// bf16 results: where a CTA per tile, dQ's and dK/dV's in one launch, beats the persistent kernels, whose steps are twice as long but
+// which have one CTA an SM and a launch each.  (Backward, us, persistent and tiles; S the longer of both lengths, tiles those of
+// queries and keys.)
+//   - Bit-reproducible (the same bits either way): up to 768 (B16 H4 S200 22.0 and 13.2, B64 H8 S512 causal 178 and 167, B64 H8 S640
+//     309 and 311), and up to 2048 while there are few (1536 tiles, B16 H4 S1536 201 and 197; 2048 tiles, B16 H8 S1024 175 and
+//     180; B4 H4 S4096 causal 161 and 168).
+//   - Otherwise against the one-kernel form, which evaluates the scores once: few tiles (512, B32 H4 S256 26 and 21, B16 H4 S512 32.3
+//     and 31.2; B32 H4 S512 55 and 58; at 128 B2 H4 S1024 25.9 and 25.5, B4 H4 S1024 27.7 and 29.8), up to 128 any number (B64 H16
+//     S128 67 and 58; B64 H8 S256 73 and 74), causal up to 384 (B64 H8 S384 122 and 117; B32 H8 S512 83 and 86), never with a
+//     mask (B8 H8 S500 47 and 53).
+// A limit on the context's SMs keeps to the persistent kernels, which obey it.
+bool bwd_in_tiles(const ltca_ctx* ctx, const ltca_attn_params* p) {
+    if (ctx->sm_count < ctx->sm_device) return false;
+    const int S = p->Sq > p->Sk ? p->Sq : p->Sk;
+    const int64_t tiles = (int64_t)p->B * p->H * ((p->Sq + kTile - 1) / kTile + (p->Sk + kTile - 1) / kTile);
+    if (p->bwd_deterministic) return S <= 768 || (S <= 2048 && tiles <= 1536);
+    if (p->keep_mask) return false;
+    return S <= 128 || (S <= 384 && p->causal) || (S <= 640 && tiles <= 512) || (S <= 1024 && tiles <= 128);
+}
 
 template <typename OutT, bool kMask>
 int launch_main(ltca_ctx* ctx, const ltca_attn_params* p, const void* mask_words, const void* q, const void* k, const void* v,
                 const void* dout, const ltca_strides& qs, const ltca_strides& ks, const ltca_strides& vs,
                 const ltca_strides& dos, const float* lse2, const float* delta, float* dq_acc) {
-    CUtensorMap tq128, tdo128, tk64, tv64, tq64, tdo64, tk128, tv128;
+    BwdMaps m;
     int rc;
-    if ((rc = make_tmap_bhsd(ctx, &tq128, q, 2, p->B, p->H, p->Sq, kD, qs, 64, kTile))) return rc;
-    if ((rc = make_tmap_bhsd(ctx, &tdo128, dout, 2, p->B, p->H, p->Sq, kD, dos, 64, kTile))) return rc;
-    if ((rc = make_tmap_bhsd(ctx, &tk64, k, 2, p->B, p->H, p->Sk, kD, ks, 64, kStep))) return rc;
-    if ((rc = make_tmap_bhsd(ctx, &tv64, v, 2, p->B, p->H, p->Sk, kD, vs, 64, kStep))) return rc;
-    if ((rc = make_tmap_bhsd(ctx, &tq64, q, 2, p->B, p->H, p->Sq, kD, qs, 64, kStep))) return rc;
-    if ((rc = make_tmap_bhsd(ctx, &tdo64, dout, 2, p->B, p->H, p->Sq, kD, dos, 64, kStep))) return rc;
-    if ((rc = make_tmap_bhsd(ctx, &tk128, k, 2, p->B, p->H, p->Sk, kD, ks, 64, kTile))) return rc;
-    if ((rc = make_tmap_bhsd(ctx, &tv128, v, 2, p->B, p->H, p->Sk, kD, vs, 64, kTile))) return rc;
+    if ((rc = make_tmap_bhsd(ctx, &m.q128, q, 2, p->B, p->H, p->Sq, kD, qs, 64, kTile))) return rc;
+    if ((rc = make_tmap_bhsd(ctx, &m.do128, dout, 2, p->B, p->H, p->Sq, kD, dos, 64, kTile))) return rc;
+    if ((rc = make_tmap_bhsd(ctx, &m.k128, k, 2, p->B, p->H, p->Sk, kD, ks, 64, kTile))) return rc;
+    if ((rc = make_tmap_bhsd(ctx, &m.v128, v, 2, p->B, p->H, p->Sk, kD, vs, 64, kTile))) return rc;
+    constexpr int es = sizeof(OutT), cols = 128 / es;       // of a result's box
+    if (es == 4 || !dq_acc)
+        if ((rc = make_tmap_bhsd(ctx, &m.dq, p->dq, es, p->B, p->H, p->Sq, kD, p->dq_strides, cols, kTile))) return rc;
+    if ((rc = make_tmap_bhsd(ctx, &m.dk, p->dk, es, p->B, p->H, p->Sk, kD, p->dk_strides, cols, kTile))) return rc;
+    if ((rc = make_tmap_bhsd(ctx, &m.dv, p->dv, es, p->B, p->H, p->Sk, kD, p->dv_strides, cols, kTile))) return rc;
 
     BwdArgs a;
     memset(&a, 0, sizeof(a));
@@ -2282,7 +2322,7 @@ int launch_main(ltca_ctx* ctx, const ltca_attn_params* p, const void* mask_words
     a.status = ctx->d_status;
 
     if constexpr (sizeof(OutT) == 2) {
-        if (dq_acc) {
+        if (dq_acc) {                             // not in tiles
             static SmemOptIn opt_fused;
             LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(opt_fused, ctx->device, attn_bwd_fused_sm100_kernel<kMask>,
                                                   FusedSmem::kDynBytes));
@@ -2294,13 +2334,11 @@ int launch_main(ltca_ctx* ctx, const ltca_attn_params* p, const void* mask_words
             ig.n_items = ig.nblk * ig.BH;
             ig.counters = ctx->d_sched + 4;             // ints 4,5: shared with the dK/dV kernel (never both in one call)
             const int n_cta = ig.n_items < ctx->sm_count ? ig.n_items : ctx->sm_count;
-            CUtensorMap tdk, tdv, tacc;
-            if ((rc = make_tmap_bhsd(ctx, &tdk, p->dk, 2, p->B, p->H, p->Sk, kD, p->dk_strides, 64, kTile))) return rc;
-            if ((rc = make_tmap_bhsd(ctx, &tdv, p->dv, 2, p->B, p->H, p->Sk, kD, p->dv_strides, 64, kTile))) return rc;
+            CUtensorMap tacc;
             const ltca_strides accs{(int64_t)p->H * a.Sq_pad * kD, (int64_t)a.Sq_pad * kD, kD};
             if ((rc = make_tmap_bhsd(ctx, &tacc, dq_acc, 4, p->B, p->H, a.Sq_pad, kD, accs, 32, kTile))) return rc;
             LTCA_CUDA_OK(ctx, launch_dependent_if(small_attention_call(p), attn_bwd_fused_sm100_kernel<kMask>, dim3(n_cta), dim3(kThreads), FusedSmem::kDynBytes,
-                                               ctx->stream, tq128, tdo128, tk128, tv128, tdk, tdv, tacc, a, ig));
+                                               ctx->stream, m.q128, m.do128, m.k128, m.v128, m.dk, m.dv, tacc, a, ig));
             LTCA_LAUNCH_OK(ctx, "attn_bwd_fused_sm100_kernel");
             kernel_timing_mark(ctx, 2);
             const int64_t rows = (int64_t)p->B * p->H * p->Sq;
@@ -2311,6 +2349,32 @@ int launch_main(ltca_ctx* ctx, const ltca_attn_params* p, const void* mask_words
             kernel_timing_mark(ctx, 3);
             return LTCA_OK;
         }
+    }
+    if (sizeof(OutT) == 4 || bwd_in_tiles(ctx, p)) {
+        if ((rc = make_tmap_bhsd(ctx, &m.q64, q, 2, p->B, p->H, p->Sq, kD, qs, 64, kStep))) return rc;
+        if ((rc = make_tmap_bhsd(ctx, &m.do64, dout, 2, p->B, p->H, p->Sq, kD, dos, 64, kStep))) return rc;
+        if ((rc = make_tmap_bhsd(ctx, &m.k64, k, 2, p->B, p->H, p->Sk, kD, ks, 64, kStep))) return rc;
+        if ((rc = make_tmap_bhsd(ctx, &m.v64, v, 2, p->B, p->H, p->Sk, kD, vs, 64, kStep))) return rc;
+        static SmemOptIn opt_tiles;               // one per template instantiation
+        constexpr int smem = DqSmem::kDynBytes > DkvSmem::kDynBytes ? DqSmem::kDynBytes : DkvSmem::kDynBytes;
+        static_assert(2 * (smem + 1024) <= 228 * 1024, "two to an SM");
+        auto kern = attn_bwd_dkv_sm100_kernel<OutT, kMask>;
+        LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(opt_tiles, ctx->device, kern, smem));
+        ItemGrid keys, queries;
+        keys.group = queries.group = kSchedGroup;
+        keys.H = queries.H = p->H;
+        keys.BH = queries.BH = p->H * p->B;
+        keys.counters = queries.counters = nullptr;
+        keys.nblk = (p->Sk + kTile - 1) / kTile;
+        queries.nblk = (p->Sq + kTile - 1) / kTile;
+        keys.n_items = keys.nblk * keys.BH;
+        queries.n_items = queries.nblk * queries.BH;
+        const dim3 grid((unsigned)keys.n_items + (unsigned)queries.n_items);
+        LTCA_CUDA_OK(ctx, launch_dependent_if(small_attention_call(p), kern, grid, dim3(kTileThreads), smem, ctx->stream, m, a, keys, queries));
+        LTCA_LAUNCH_OK(ctx, "attn_bwd_dkv_sm100_kernel");
+        kernel_timing_mark(ctx, 2);
+        kernel_timing_mark(ctx, 3);
+        return LTCA_OK;
     }
     if constexpr (sizeof(OutT) == 2) {
         {
@@ -2324,10 +2388,8 @@ int launch_main(ltca_ctx* ctx, const ltca_attn_params* p, const void* mask_words
             ig.n_items = ig.nblk * ig.BH;
             ig.counters = ctx->d_sched + 2;             // ints 2,3: the dQ kernel's item counters
             const int n_cta = ig.n_items < ctx->sm_count ? ig.n_items : ctx->sm_count;
-            CUtensorMap tdq;
-            if ((rc = make_tmap_bhsd(ctx, &tdq, p->dq, 2, p->B, p->H, p->Sq, kD, p->dq_strides, 64, kTile))) return rc;
             LTCA_CUDA_OK(ctx, launch_dependent_if(small_attention_call(p), attn_bwd_dq4_sm100_kernel<kMask>, dim3(n_cta), dim3(kThreads), Dq4Smem::kDynBytes,
-                                               ctx->stream, tq128, tdo128, tk128, tv128, tdq, a, ig));
+                                               ctx->stream, m.q128, m.do128, m.k128, m.v128, m.dq, a, ig));
             LTCA_LAUNCH_OK(ctx, "attn_bwd_dq4_sm100_kernel");
         }
         kernel_timing_mark(ctx, 2);
@@ -2343,31 +2405,10 @@ int launch_main(ltca_ctx* ctx, const ltca_attn_params* p, const void* mask_words
             ig.n_items = ig.nblk * ig.BH;
             ig.counters = ctx->d_sched + 4;             // ints 4,5: the dK/dV kernel's item counters
             const int n_cta = ig.n_items < ctx->sm_count ? ig.n_items : ctx->sm_count;
-            CUtensorMap tdk, tdv;
-            if ((rc = make_tmap_bhsd(ctx, &tdk, p->dk, 2, p->B, p->H, p->Sk, kD, p->dk_strides, 64, kTile))) return rc;
-            if ((rc = make_tmap_bhsd(ctx, &tdv, p->dv, 2, p->B, p->H, p->Sk, kD, p->dv_strides, 64, kTile))) return rc;
             LTCA_CUDA_OK(ctx, launch_dependent_if(small_attention_call(p), attn_bwd_dkv4_sm100_kernel<kMask>, dim3(n_cta), dim3(kThreads), Dkv4Smem::kDynBytes,
-                                               ctx->stream, tq128, tdo128, tk128, tv128, tdk, tdv, a, ig));
+                                               ctx->stream, m.q128, m.do128, m.k128, m.v128, m.dk, m.dv, a, ig));
             LTCA_LAUNCH_OK(ctx, "attn_bwd_dkv4_sm100_kernel");
         }
-    } else {
-        auto kdq = attn_bwd_dq_sm100_kernel<kMask>;
-        auto kdkv = attn_bwd_dkv_sm100_kernel<kMask>;
-        CUtensorMap tdq, tdk, tdv;
-        if ((rc = make_tmap_bhsd(ctx, &tdq, p->dq, 4, p->B, p->H, p->Sq, kD, p->dq_strides, 32, kTile))) return rc;
-        if ((rc = make_tmap_bhsd(ctx, &tdk, p->dk, 4, p->B, p->H, p->Sk, kD, p->dk_strides, 32, kTile))) return rc;
-        if ((rc = make_tmap_bhsd(ctx, &tdv, p->dv, 4, p->B, p->H, p->Sk, kD, p->dv_strides, 32, kTile))) return rc;
-        static SmemOptIn opt_dq, opt_dkv;         // one pair per template instantiation
-        LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(opt_dq, ctx->device, kdq, DqSmem::kDynBytes));
-        LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(opt_dkv, ctx->device, kdkv, DkvSmem::kDynBytes));
-        static_assert(2 * (DqSmem::kDynBytes + 1024) <= 228 * 1024 && 2 * (DkvSmem::kDynBytes + 1024) <= 228 * 1024, "two to an SM");
-        dim3 gq((p->Sq + kTile - 1) / kTile, p->H, p->B);
-        LTCA_CUDA_OK(ctx, launch_dependent_if(small_attention_call(p), kdq, gq, dim3(kTileThreads), DqSmem::kDynBytes, ctx->stream, tq128, tdo128, tk64, tv64, tdq, a));
-        LTCA_LAUNCH_OK(ctx, "attn_bwd_dq_sm100_kernel");
-        kernel_timing_mark(ctx, 2);
-        dim3 gk((p->Sk + kTile - 1) / kTile, p->H, p->B);
-        LTCA_CUDA_OK(ctx, launch_dependent_if(small_attention_call(p), kdkv, gk, dim3(kTileThreads), DkvSmem::kDynBytes, ctx->stream, tq64, tdo64, tk128, tv128, tdk, tdv, a));
-        LTCA_LAUNCH_OK(ctx, "attn_bwd_dkv_sm100_kernel");
     }
     kernel_timing_mark(ctx, 3);
     return LTCA_OK;
@@ -2408,7 +2449,10 @@ int launch_attn_bwd_sm100(ltca_ctx* ctx, const ltca_attn_params* p) {
     float* lse2 = reinterpret_cast<float*>(w);  w += stats_bytes(p);
     float* delta = reinterpret_cast<float*>(w); w += stats_bytes(p);
     float* dq_acc = nullptr;
-    if (use_fused(p)) { dq_acc = reinterpret_cast<float*>(w); w += dq_acc_bytes(p); }
+    if (use_fused(p)) {
+        if (!bwd_in_tiles(ctx, p)) dq_acc = reinterpret_cast<float*>(w);
+        w += dq_acc_bytes(p);
+    }
 
     StatsArgs s;
     s.B = p->B; s.H = p->H; s.Sq = p->Sq; s.Sq_pad = (int)align_up((size_t)p->Sq, 256);
