@@ -70,18 +70,21 @@ struct GemmCfg {
 };
 
 struct GemmMaps { CUtensorMap a[kMaxGemmProblems], b[kMaxGemmProblems], c[kMaxGemmProblems]; };
-// A group's: up to three terms each, second terms of the results behind the first.
+// A group's: up to three terms a member (twelve in all), second terms of the results behind the first.
+constexpr int kMaxGroupPairs = 12;
 struct GemmGroupMaps {
-    CUtensorMap a[3 * kMaxGemmProblems], b[3 * kMaxGemmProblems], c[2 * kMaxGemmProblems];
-    int first[kMaxGemmProblems + 1];   // a member's pairs
-    int form[kMaxGemmProblems];        // ... operand forms (bit 0: A stored [K, M], bit 1: B stored [K, N]), and whether its
+    CUtensorMap a[kMaxGroupPairs], b[kMaxGroupPairs], c[2 * kMaxGemmGroup];
+    int first[kMaxGemmGroup + 1];      // a member's pairs
+    int form[kMaxGemmGroup];           // ... operand forms (bit 0: A stored [K, M], bit 1: B stored [K, N]), and whether its
                                        // result has a second term (bit 2; where any has one)
+    int M[kMaxGemmGroup], N[kMaxGemmGroup], K[kMaxGemmGroup], ksplit[kMaxGemmGroup], tiles_x[kMaxGemmGroup], tiles_y[kMaxGemmGroup];
+    int tile0[kMaxGemmGroup + 1];      // ... tiles: members one after the other
 };
 
 struct GemmKArgs {
     int M, N, K;
     int n_sum, ksplit;
-    int tiles_x, tiles_y, tiles_z;   // N tiles, M tiles, problems x K slices
+    int tiles_x, tiles_y, tiles_z;   // N tiles, M tiles, problems x K slices (a group: all tiles, 1, 1)
     int batch_h, batch_b;            // independent products of the same shape (slowest index of the tile list)
     int sum_h;                       // heads whose products one tile sums up
     int a_head, b_head;              // 0: the heads share the operand
@@ -101,32 +104,47 @@ struct GemmKArgs {
 // One tile of the work list of a CTA.
 struct GemmTile {
     int m0, n0, problem, slice, kb_begin, kb_end, pair_begin, n_pairs, n_iters;
+    int M, N, ksplit;                // of its problem
     int bh, bb;                      // batch entry
 };
 template <int kBN, int kTileM, typename Maps>
 __device__ __forceinline__ GemmTile gemm_tile(const Maps& maps, const GemmKArgs& g, int sum_h, int linear, int rank) {
     GemmTile t;
-    const int x = linear % g.tiles_x;
-    const int yz = linear / g.tiles_x;
-    const int y = yz % g.tiles_y, zw = yz / g.tiles_y;
-    const int z = zw % g.tiles_z, w = zw / g.tiles_z;
-    t.bh = w % g.batch_h;
-    t.bb = w / g.batch_h;
+    int K, tiles_x, tiles_y;
+    if constexpr (std::is_same<Maps, GemmGroupMaps>::value) {
+        t.problem = 0;
+        while (linear >= maps.tile0[t.problem + 1]) ++t.problem;
+        linear -= maps.tile0[t.problem];
+        t.M = maps.M[t.problem]; t.N = maps.N[t.problem]; K = maps.K[t.problem]; t.ksplit = maps.ksplit[t.problem];
+        tiles_x = maps.tiles_x[t.problem]; tiles_y = maps.tiles_y[t.problem];
+    } else {
+        t.M = g.M; t.N = g.N; K = g.K; t.ksplit = g.ksplit;
+        tiles_x = g.tiles_x; tiles_y = g.tiles_y;
+    }
+    const int x = linear % tiles_x;
+    const int yz = linear / tiles_x;
+    const int y = yz % tiles_y, zw = yz / tiles_y;
     t.n0 = x * kBN;
     t.m0 = y * kTileM + rank * kBM;
-    t.problem = z / g.ksplit;
-    t.slice = z % g.ksplit;
-    const int nkb = (g.K + kBK - 1) / kBK;
-    const int per = (nkb + g.ksplit - 1) / g.ksplit;
-    t.kb_begin = min(t.slice * per, nkb);
-    t.kb_end = min(t.kb_begin + per, nkb);
     if constexpr (std::is_same<Maps, GemmGroupMaps>::value) {
+        t.slice = zw % t.ksplit;
+        t.bh = zw / t.ksplit;
+        t.bb = 0;
         t.pair_begin = maps.first[t.problem];
         t.n_pairs = maps.first[t.problem + 1] - t.pair_begin;
     } else {
+        const int z = zw % g.tiles_z, w = zw / g.tiles_z;
+        t.bh = w % g.batch_h;
+        t.bb = w / g.batch_h;
+        t.problem = z / g.ksplit;
+        t.slice = z % g.ksplit;
         t.pair_begin = g.n_sum > 1 ? 0 : t.problem;
         t.n_pairs = g.n_sum > 1 ? g.n_sum : 1;
     }
+    const int nkb = (K + kBK - 1) / kBK;
+    const int per = (nkb + t.ksplit - 1) / t.ksplit;
+    t.kb_begin = min(t.slice * per, nkb);
+    t.kb_end = min(t.kb_begin + per, nkb);
     t.n_iters = t.n_pairs * sum_h * (t.kb_end - t.kb_begin);
     return t;
 }
@@ -171,7 +189,9 @@ gemm_bf16_sm100_kernel(const __grid_constant__ typename std::conditional<kKind =
     volatile uint32_t* misc = reinterpret_cast<volatile uint32_t*>(smem_gen + L::kMiscOff);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int n_tiles = g.tiles_x * g.tiles_y * g.tiles_z * g.batch_h * g.batch_b;
+    int n_tiles;
+    if constexpr (kKind == kGroup) n_tiles = g.tiles_x;
+    else n_tiles = g.tiles_x * g.tiles_y * g.tiles_z * g.batch_h * g.batch_b;
     const int rank = kPair ? (int)cluster_rank() : 0;             // rank 0 issues the pair's MMAs
     LTCA_TRACE_DECL(blockIdx.x == 5 && g.tiles_z == LTCA_TRACE_GEMM_Z);
     LTCA_TRACE_EVT(0x01);
@@ -318,7 +338,7 @@ gemm_bf16_sm100_kernel(const __grid_constant__ typename std::conditional<kKind =
                 ++na;
             }
             const uint32_t tacc = tmem_base + (uint32_t)kBN * buf + ((uint32_t)(qd * 32) << 16);
-            const float* bias = (g.ksplit == 1) ? g.bias[t.problem] : nullptr;
+            const float* bias = kKind != kGroup && g.ksplit == 1 ? g.bias[t.problem] : nullptr;
             if (g.tma_store) {
                 // The tile leaves box by box: 128 rows of 128 bytes (64 bf16 or 32 fp32 columns) go to shared memory
                 // in the layout of a 128-byte swizzled TMA box and one thread stores the box; the tensor map clips
@@ -367,7 +387,7 @@ gemm_bf16_sm100_kernel(const __grid_constant__ typename std::conditional<kKind =
                 float* bias_s = reinterpret_cast<float*>(smem_gen + L::kBiasOff);
                 if (bias) {
                     // (the last reads of the tile before lie before that tile's last barrier)
-                    for (int c = row; c < kBN; c += 128) bias_s[c] = t.n0 + c < g.N ? __ldg(bias + t.n0 + c) : 0.f;
+                    for (int c = row; c < kBN; c += 128) bias_s[c] = t.n0 + c < t.N ? __ldg(bias + t.n0 + c) : 0.f;
                     asm volatile("bar.sync 1, 128;" ::: "memory");
                 }
                 auto add_bias = [&](int gn0, uint32_t (&v)[32]) {
@@ -404,13 +424,13 @@ gemm_bf16_sm100_kernel(const __grid_constant__ typename std::conditional<kKind =
                     asm volatile("bar.sync 1, 128;" ::: "memory");    // the four epilogue warps have staged their rows
                     if (warp == 2 && lane == 0) {
                         // (partial tiles are one [problem][slice][M][N] tensor)
-                        const CUtensorMap* tc = &maps.c[g.ksplit > 1 ? 0 : t.problem];
-                        if (gn0 < g.N && t.m0 < g.M) {
+                        const CUtensorMap* tc = &maps.c[kKind != kGroup && g.ksplit > 1 ? 0 : t.problem];
+                        if (gn0 < t.N && t.m0 < t.M) {
                             if (add_to_c) tma_reduce_add_4d(tc, stage_addr + hb * (kBM * 128), gn0, t.m0, t.bh, t.bb);
-                            else tma_store_4d(tc, stage_addr + hb * (kBM * 128), gn0, t.m0, g.ksplit > 1 ? t.slice : t.bh,
-                                              g.ksplit > 1 ? t.problem : t.bb);
+                            else tma_store_4d(tc, stage_addr + hb * (kBM * 128), gn0, t.m0, t.ksplit > 1 ? t.slice : t.bh,
+                                              t.ksplit > 1 ? (kKind == kGroup ? 0 : t.problem) : t.bb);
                             if (g.c_lo && has_second_term(maps, t.problem))
-                                tma_store_4d(&maps.c[kKind == kGroup ? kMaxGemmProblems + t.problem : 1], stage_addr + (hb + 1) * (kBM * 128), gn0, t.m0, t.bh, t.bb);
+                                tma_store_4d(&maps.c[kKind == kGroup ? kMaxGemmGroup + t.problem : 1], stage_addr + (hb + 1) * (kBM * 128), gn0, t.m0, t.bh, t.bb);
                         }
                         tma_store_commit();
                         // the box that the next piece takes has been read
@@ -739,21 +759,21 @@ int gemm_sm100(ltca_ctx* ctx, const GemmProblem& gp) {
         launch = kind == kTilePair ? launch_gemm<256, true, kHeads> : kind == kTile256 ? launch_gemm<256, false, kHeads> : launch_gemm<128, false, kHeads>;
     rc = launch(ctx, maps, g, amn, bmn, n_tiles, sms);
     if (rc) return rc;
-    if (g.ksplit > 1) {
-        const int64_t mn = (int64_t)gp.M * gp.N;
-        float* c[kMaxGemmProblems];
-        bool vec = (mn & 3) == 0 && (reinterpret_cast<uintptr_t>(gp.partial) & 15) == 0 && mn / 4 * gp.n_problems >= (int64_t)kPlanSms * 1024;
-        for (int i = 0; i < kMaxGemmProblems; ++i) {
-            c[i] = reinterpret_cast<float*>(gp.c[i < gp.n_problems ? i : 0]);
-            vec = vec && (reinterpret_cast<uintptr_t>(c[i]) & 15) == 0;
-        }
-        const int64_t per = vec ? 1024 : 256;
-        const dim3 rg((unsigned)((mn + per - 1) / per), gp.n_problems);
-        auto kern = vec ? gemm_splitk_reduce_kernel<4> : gemm_splitk_reduce_kernel<1>;
-        LTCA_CUDA_OK(ctx, launch_dependent(kern, rg, dim3(256), 0, ctx->stream,
-                                           (const float*)gp.partial, c[0], c[1], c[2], c[3], mn, g.ksplit, ctx->run_if));
-        LTCA_LAUNCH_OK(ctx, "gemm_splitk_reduce_kernel");
+    return g.ksplit > 1 ? sum_splits(ctx, gp.partial, gp.c, gp.n_problems, (int64_t)gp.M * gp.N, g.ksplit) : LTCA_OK;
+}
+
+int sum_splits(ltca_ctx* ctx, const float* partial, void* const* dst, int n, int64_t mn, int ksplit) {
+    float* c[kMaxGemmProblems];
+    bool vec = (mn & 3) == 0 && (reinterpret_cast<uintptr_t>(partial) & 15) == 0 && mn / 4 * n >= (int64_t)kPlanSms * 1024;
+    for (int i = 0; i < kMaxGemmProblems; ++i) {
+        c[i] = reinterpret_cast<float*>(dst[i < n ? i : 0]);
+        vec = vec && (reinterpret_cast<uintptr_t>(c[i]) & 15) == 0;
     }
+    const int64_t per = vec ? 1024 : 256;
+    const dim3 rg((unsigned)((mn + per - 1) / per), n);
+    auto kern = vec ? gemm_splitk_reduce_kernel<4> : gemm_splitk_reduce_kernel<1>;
+    LTCA_CUDA_OK(ctx, launch_dependent(kern, rg, dim3(256), 0, ctx->stream, partial, c[0], c[1], c[2], c[3], mn, ksplit, ctx->run_if));
+    LTCA_LAUNCH_OK(ctx, "gemm_splitk_reduce_kernel");
     return LTCA_OK;
 }
 
@@ -761,6 +781,7 @@ bool gemm_group_aligned(const GemmGroup& gg) {
     const int ces = gg.out_bf16 ? 2 : 4;
     for (int i = 0; i < gg.n; ++i) {
         const GemmGroup::Member& m = gg.m[i];
+        if (m.ksplit > 1 && ((m.N & 3) || gg.heads > 1 || gg.out_bf16)) return false;
         if (((m.ldc * ces) & 15) || (gg.heads > 1 && ((m.c_hs * ces) & 15)) || (reinterpret_cast<uintptr_t>(m.c) & 15) ||
             (reinterpret_cast<uintptr_t>(m.c_lo) & 15))
             return false;
@@ -781,13 +802,12 @@ static int launch_group(ltca_ctx* ctx, const GemmGroupMaps& m, const GemmKArgs& 
 }
 
 int gemm_sm100_group(ltca_ctx* ctx, const GemmGroup& gg) {
-    if (gg.M < 1 || gg.N < 1 || gg.K < 1 || gg.heads < 1 || gg.n < 1 || gg.n > kMaxGemmProblems || !gemm_group_aligned(gg))
-        return fail(ctx, LTCA_ERR_INVALID, "gemm: between 1 and 4 members with 16-byte aligned results");
+    if (gg.heads < 1 || gg.n < 1 || gg.n > kMaxGemmGroup || !gemm_group_aligned(gg))
+        return fail(ctx, LTCA_ERR_INVALID, "gemm: between 1 and %d members with 16-byte aligned results", kMaxGemmGroup);
     GemmGroupMaps maps;
     GemmKArgs g;
     memset(&maps, 0, sizeof(maps));
     memset(&g, 0, sizeof(g));
-    g.M = gg.M; g.N = gg.N; g.K = gg.K;
     g.n_sum = 1; g.ksplit = 1; g.sum_h = 1;
     g.batch_h = gg.heads; g.batch_b = 1;
     g.a_head = g.b_head = 1;
@@ -797,10 +817,16 @@ int gemm_sm100_group(ltca_ctx* ctx, const GemmGroup& gg) {
         if (gg.m[i].c_lo) g.c_lo = gg.m[i].c_lo;       // (whether any is there: the stores go by the members' tensor maps)
     g.status = ctx->d_status;
     g.run_if = ctx->run_if;
+    const int sms = ctx->sm_count > 0 ? ctx->sm_count : kPlanSms;
+    bool wide = false;
+    for (int i = 0; i < gg.n; ++i) wide = wide || gg.m[i].N > 128;
+    wide = wide && !gemm_group_one_wave(ctx, gg);      // (pick_tile's rule, for all members alike)
+    int64_t n_tiles = 0;
     int rc;
     for (int i = 0; i < gg.n; ++i) {
         const GemmGroup::Member& m = gg.m[i];
-        if (m.terms < 1 || m.terms > 3 || (m.c_lo && !gg.out_bf16))
+        if (m.M < 1 || m.N < 1 || m.K < 1 || m.ksplit < 1) return fail(ctx, LTCA_ERR_INVALID, "gemm: empty member");
+        if (m.terms < 1 || m.terms > 3 || maps.first[i] + m.terms > kMaxGroupPairs || (m.c_lo && !gg.out_bf16))
             return fail(ctx, LTCA_ERR_INVALID, "gemm: a member has one to three terms, and a second term of its result in bf16 only");
         const int64_t as[2] = {m.a_hs, 0}, bs[2] = {m.b_hs, 0};
         maps.first[i + 1] = maps.first[i] + m.terms;
@@ -808,24 +834,30 @@ int gemm_sm100_group(ltca_ctx* ctx, const GemmGroup& gg) {
         for (int t = 0; t < m.terms; ++t) {
             if (m.a[t].mn_major != m.a[0].mn_major || m.b[t].mn_major != m.b[0].mn_major)
                 return fail(ctx, LTCA_ERR_INVALID, "gemm: the terms of a member share the operand forms");
-            if ((rc = make_operand_map(ctx, &maps.a[maps.first[i] + t], m.a[t], gg.M, gg.K, gg.heads, 1, as, false))) return rc;
-            if ((rc = make_operand_map(ctx, &maps.b[maps.first[i] + t], m.b[t], gg.N, gg.K, gg.heads, 1, bs, false))) return rc;
+            if ((rc = make_operand_map(ctx, &maps.a[maps.first[i] + t], m.a[t], m.M, m.K, gg.heads, 1, as, false))) return rc;
+            if ((rc = make_operand_map(ctx, &maps.b[maps.first[i] + t], m.b[t], m.N, m.K, gg.heads, 1, bs, false))) return rc;
         }
-        const ltca_strides cs{0, m.c_hs, m.ldc};
+        const bool split = m.ksplit > 1;               // the slices stand where the heads' results do
+        const ltca_strides cs{0, split ? (int64_t)m.M * m.N : m.c_hs, split ? m.N : m.ldc};
         for (int l = 0; l < (m.c_lo ? 2 : 1); ++l)
-            if ((rc = make_tmap_bhsd(ctx, &maps.c[l * kMaxGemmProblems + i], l ? m.c_lo : m.c, gg.out_bf16 ? 2 : 4, 1, gg.heads, gg.M, gg.N, cs,
-                                     gg.out_bf16 ? 64 : 32, kBM))) return rc;
-        g.C[i] = m.c;
+            if ((rc = make_tmap_bhsd(ctx, &maps.c[l * kMaxGemmGroup + i], l ? m.c_lo : m.c, gg.out_bf16 ? 2 : 4, 1, split ? m.ksplit : gg.heads,
+                                     m.M, m.N, cs, gg.out_bf16 ? 64 : 32, kBM))) return rc;
+        maps.M[i] = m.M; maps.N[i] = m.N; maps.K[i] = m.K; maps.ksplit[i] = m.ksplit;
+        maps.tiles_x[i] = (m.N + (wide ? 255 : 127)) / (wide ? 256 : 128);
+        maps.tiles_y[i] = (m.M + kBM - 1) / kBM;
+        n_tiles += (int64_t)maps.tiles_x[i] * maps.tiles_y[i] * m.ksplit * gg.heads;
+        if (n_tiles > 0x7fffffff) return fail(ctx, LTCA_ERR_UNSUPPORTED, "gemm: too many tiles");
+        maps.tile0[i + 1] = (int)n_tiles;
     }
-    const int sms = ctx->sm_count > 0 ? ctx->sm_count : kPlanSms;
-    const int64_t z = (int64_t)gg.n * gg.heads;
-    const bool wide = pick_tile(gg.M, gg.N, 0, z, sms) != kTile128;    // (0: no pairs)
-    g.tiles_x = (gg.N + (wide ? 255 : 127)) / (wide ? 256 : 128);
-    g.tiles_y = (gg.M + kBM - 1) / kBM;
-    g.tiles_z = gg.n;
-    const int64_t n_tiles = g.tiles_x * (g.tiles_y * z);
-    if (n_tiles > 0x7fffffff) return fail(ctx, LTCA_ERR_UNSUPPORTED, "gemm: too many tiles");
+    g.tiles_x = (int)n_tiles; g.tiles_y = g.tiles_z = 1;
     return wide ? launch_group<256>(ctx, maps, g, n_tiles, sms) : launch_group<128>(ctx, maps, g, n_tiles, sms);
+}
+
+bool gemm_group_one_wave(const ltca_ctx* ctx, const GemmGroup& gg) {
+    int64_t n = 0;
+    for (int i = 0; i < gg.n; ++i)
+        n += (int64_t)((gg.m[i].M + 127) / 128) * ((gg.m[i].N + 127) / 128) * gg.m[i].ksplit * gg.heads;
+    return n <= (ctx->sm_count > 0 ? ctx->sm_count : kPlanSms);
 }
 
 int convert_rows_bf16(ltca_ctx* ctx, const float* src, int64_t ld_src, void* dst, int64_t ld_dst, int64_t rows,

@@ -43,22 +43,29 @@ struct GemmProblem {
 
 int gemm_sm100(ltca_ctx* ctx, const GemmProblem& gp);
 
-// Up to four products of the same shape in one launch, each of its own operand forms and number of summed terms, for every one
-// of `heads` (strides a_hs, b_hs, c_hs between them).  c_lo as in GemmProblem.  Results need
-// 16-byte aligned rows (gemm_group_aligned).
+// Up to five products in one launch, each of its own shape, operand forms and number of summed terms, for every one
+// of `heads` (strides a_hs, b_hs, c_hs between them).  c_lo as in GemmProblem.  Results need 16-byte aligned rows
+// (gemm_group_aligned).  ksplit > 1 (one head, fp32 results, rows of N): `c` takes the slices, [ksplit][M][N], for sum_splits.
+constexpr int kMaxGemmGroup = 5;
 struct GemmGroup {
     struct Member {
+        int M = 0, N = 0, K = 0, ksplit = 1;
         int terms = 1;
         GemmOperand a[3] = {}, b[3] = {};
         int64_t a_hs = 0, b_hs = 0, c_hs = 0, ldc = 0;
         void* c = nullptr;
         void* c_lo = nullptr;
     };
-    int M = 0, N = 0, K = 0, heads = 1, n = 0, out_bf16 = 0;
-    Member m[kMaxGemmProblems];
+    int heads = 1, n = 0, out_bf16 = 0;
+    Member m[kMaxGemmGroup];
 };
+// Whether all its tiles fit beside one another on the SMs as 128 x 128 ones: then a launch of its own for each of its members
+// would leave SMs idle.
+bool gemm_group_one_wave(const ltca_ctx* ctx, const GemmGroup& gg);
 bool gemm_group_aligned(const GemmGroup& gg);
 int gemm_sm100_group(ltca_ctx* ctx, const GemmGroup& gg);
+// dst[i][e] = sum over s < ksplit of partial[i][s][e], e < mn, in slice order.
+int sum_splits(ltca_ctx* ctx, const float* partial, void* const* dst, int n, int64_t mn, int ksplit);
 int gemm_sm100_pick_ksplit(int M, int N, int K, int n_problems, int sm_count);
 size_t gemm_sm100_partial_bytes(int M, int N, int n_problems, int ksplit);
 // dst[r, c] = bf16(src[r, c]) for a [rows, cols] block with row pitches ld_src / ld_dst (elements).
