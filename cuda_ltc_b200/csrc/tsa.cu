@@ -156,7 +156,7 @@ __device__ __forceinline__ void layer_norm_row(const float* __restrict__ y, cons
     for (int i = lane; i < E; i += 32)
         put1(out, row, i, fmaf((value(i) - mean) * inv_std, gamma ? gamma[i] : 1.f, beta ? beta[i] : 0.f));
 }
-__device__ __forceinline__ bool aligned16(const void* a, const void* b, const void* c, const void* d, const void* e) {
+__host__ __device__ __forceinline__ bool aligned16(const void* a, const void* b, const void* c, const void* d, const void* e) {
     return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c) |
              reinterpret_cast<uintptr_t>(d) | reinterpret_cast<uintptr_t>(e)) & 15) == 0;
 }
@@ -519,6 +519,18 @@ struct ColSum {
     int64_t rows;
     int n, max_cols;
     float* partial;                     // [n][kColChunks][max_cols]
+    // What module_tail also does where `tail` says that one follows: the slices of split products (sum_splits) ...
+    bool tail;
+    const float* split;
+    float* split_dst[kMaxGemmProblems];
+    int64_t split_mn;
+    int splits, split_n;
+    // ... and the LayerNorm's backward, whose products' column sums go to ln_partial, [chunks of ln_rows rows][2][E]
+    const float *ln_g, *ln_x, *ln_gamma, *ln_res;
+    float *ln_dx, *ln_partial, *ln_dgamma, *ln_dbeta;
+    int E, ln_rows, ln_chunks;
+    int ln_blocks, col_blocks;          // blocks of the launch; the slices' come behind them
+    float eps;
     void add(const void* s, bool is_bf16, int64_t pitch, int c, float* d) {
         if (!d) return;
         src[n] = s; dst[n] = d; ld[n] = pitch; cols[n] = c; bf16[n] = is_bf16 ? 1 : 0;
@@ -535,23 +547,32 @@ __device__ __forceinline__ float column_chunk(const T* src, int64_t ld, int64_t 
     for (int64_t r = r0; r < r1; ++r) acc += ld_f(src + r * ld);
     return acc;
 }
+__device__ __forceinline__ void column_partial(const ColSum& a, int j, int chunk, int c) {
+    const int64_t per = (a.rows + kColChunks - 1) / kColChunks;
+    const int64_t r0 = chunk * per, r1 = r0 + per < a.rows ? r0 + per : a.rows;
+    a.partial[((int64_t)j * kColChunks + chunk) * a.max_cols + c] =
+        a.bf16[j] ? column_chunk(static_cast<const __nv_bfloat16*>(a.src[j]) + c, a.ld[j], r0, r1)
+                  : column_chunk(static_cast<const float*>(a.src[j]) + c, a.ld[j], r0, r1);
+}
+__device__ __forceinline__ void column_final(const ColSum& a, int j, int c) {
+    a.dst[j][c] = column_chunk(a.partial + (int64_t)j * kColChunks * a.max_cols + c, a.max_cols, 0, kColChunks);
+}
 __global__ void __launch_bounds__(128) column_sum_partial_kernel(const __grid_constant__ ColSum a) {
     grid_dependency_wait();
     const int j = blockIdx.z, c = blockIdx.x * 128 + threadIdx.x;
-    if (c >= a.cols[j]) return;
-    const int64_t per = (a.rows + kColChunks - 1) / kColChunks;
-    const int64_t r0 = blockIdx.y * per, r1 = r0 + per < a.rows ? r0 + per : a.rows;
-    a.partial[((int64_t)j * kColChunks + blockIdx.y) * a.max_cols + c] =
-        a.bf16[j] ? column_chunk(static_cast<const __nv_bfloat16*>(a.src[j]) + c, a.ld[j], r0, r1)
-                  : column_chunk(static_cast<const float*>(a.src[j]) + c, a.ld[j], r0, r1);
+    if (c < a.cols[j]) column_partial(a, j, blockIdx.y, c);
 }
 __global__ void __launch_bounds__(128) column_sum_final_kernel(const __grid_constant__ ColSum a) {
     grid_dependency_wait();
     const int j = blockIdx.y, c = blockIdx.x * 128 + threadIdx.x;
-    if (c >= a.cols[j]) return;
-    a.dst[j][c] = column_chunk(a.partial + (int64_t)j * kColChunks * a.max_cols + c, a.max_cols, 0, kColChunks);
+    if (c < a.cols[j]) column_final(a, j, c);
 }
 int column_sums(ltca_ctx* ctx, ColSum a, int64_t rows, float* scratch) {
+    if (a.split_n) {
+        void* dst[kMaxGemmProblems];
+        for (int i = 0; i < a.split_n; ++i) dst[i] = a.split_dst[i];
+        if (int rc = sum_splits(ctx, a.split, dst, a.split_n, a.split_mn, a.splits)) return rc;
+    }
     if (a.n == 0) return LTCA_OK;
     a.rows = rows;
     a.partial = scratch;
@@ -560,9 +581,182 @@ int column_sums(ltca_ctx* ctx, ColSum a, int64_t rows, float* scratch) {
     LTCA_CUDA_OK(ctx, launch_dependent(column_sum_final_kernel, dim3(bx, a.n), dim3(128), 0, ctx->stream, a));
     return LTCA_OK;
 }
+
+// The end of the FlashAttention form's backward: LayerNorm backward, the column sums' first stage and the sums over split products'
+// slices need nothing of one another, so they share a launch, and the second stage of all column sums follows.  As launches of
+// their own they were five of 3 to 5 us each: backward B16 S200 E256 H4 72.5 -> 70.2, B32 S300 147 -> 137.  dgamma and dbeta are summed where their products are
+// formed, a warp its rows, the warps of a block in order, then the blocks: the products are neither written nor read.
+// kN4 = E / 128, or 0 for rows of up to 128 columns.
+constexpr int kTailThreads = 256, kTailWarps = kTailThreads / 32, kMaxLnChunks = 256, kLnParts = 4;
+template <int kN4>
+__device__ __forceinline__ void tail_layer_norm(const ColSum& a, float (*sm)[kTailThreads / 32][kN4 > 0 ? 128 * kN4 : 128]) {
+    constexpr int kC = kN4 > 0 ? 4 * kN4 : 4;              // columns of a lane
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, E = a.E;
+    const int64_t r0 = (int64_t)blockIdx.x * a.ln_rows, r1 = r0 + a.ln_rows < a.rows ? r0 + a.ln_rows : a.rows;
+    // element e of this lane: column 4 (lane + 32 (e / 4)) + e % 4 in 16-byte pieces, lane + 32 e otherwise
+    auto col = [&](int e) { return kN4 > 0 ? 4 * (lane + 32 * (e / 4)) + e % 4 : lane + 32 * e; };
+    auto read = [&](const float* p, float (&v)[kC]) {
+        if constexpr (kN4 > 0) {
+#pragma unroll
+            for (int e = 0; e < kC; e += 4) {
+                const float4 x = ldg4(p, lane + 8 * e);
+                v[e] = x.x; v[e + 1] = x.y; v[e + 2] = x.z; v[e + 3] = x.w;
+            }
+        } else {
+#pragma unroll
+            for (int e = 0; e < kC; ++e) v[e] = col(e) < E ? __ldg(p + col(e)) : 0.f;
+        }
+    };
+    float gm[kC], dg[kC], db[kC];
+    read(a.ln_gamma, gm);
+#pragma unroll
+    for (int e = 0; e < kC; ++e) dg[e] = db[e] = 0.f;
+    for (int64_t row = r0 + warp; row < r1; row += kTailWarps) {
+        float xh[kC], gv[kC], rs[kC];
+        read(a.ln_x + row * E, xh);
+        read(a.ln_g + row * E, gv);
+#pragma unroll
+        for (int e = 0; e < kC; ++e) rs[e] = 0.f;
+        if (a.ln_dx && a.ln_res) read(a.ln_res + row * E, rs);
+        float s0 = 0.f;
+#pragma unroll
+        for (int e = 0; e < kC; e += 4) s0 += (xh[e] + xh[e + 1]) + (xh[e + 2] + xh[e + 3]);
+        const float mean = warp_total(s0) / E;
+        float s1 = 0.f;
+#pragma unroll
+        for (int e = 0; e < kC; ++e) {
+            xh[e] = kN4 > 0 || col(e) < E ? xh[e] - mean : 0.f;
+            s1 = fmaf(xh[e], xh[e], s1);
+        }
+        const float inv_std = rsqrtf(warp_total(s1) / E + a.eps);
+        float a1 = 0.f, a2 = 0.f;
+#pragma unroll
+        for (int e = 0; e < kC; ++e) {
+            xh[e] *= inv_std;
+            dg[e] = fmaf(gv[e], xh[e], dg[e]);
+            db[e] += gv[e];
+            gv[e] *= gm[e];
+            a1 += gv[e];
+            a2 = fmaf(gv[e], xh[e], a2);
+        }
+        if (!a.ln_dx) continue;
+        const float m1 = warp_total(a1) / E, m2 = warp_total(a2) / E;
+        float* dx = a.ln_dx + row * E;
+#pragma unroll
+        for (int e = 0; e < kC; ++e) rs[e] += inv_std * (gv[e] - m1 - xh[e] * m2);
+        if constexpr (kN4 > 0) {
+#pragma unroll
+            for (int e = 0; e < kC; e += 4) reinterpret_cast<float4*>(dx)[lane + 8 * e] = make_float4(rs[e], rs[e + 1], rs[e + 2], rs[e + 3]);
+        } else {
+#pragma unroll
+            for (int e = 0; e < kC; ++e)
+                if (col(e) < E) dx[col(e)] = rs[e];
+        }
+    }
+    if (!a.ln_partial) return;
+#pragma unroll
+    for (int e = 0; e < kC; ++e) {
+        sm[0][warp][col(e)] = dg[e];
+        sm[1][warp][col(e)] = db[e];
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < 2 * E; i += kTailThreads) {
+        const int k = i / E, c = i - k * E;
+        float v = 0.f;
+#pragma unroll
+        for (int w = 0; w < kTailWarps; ++w) v += sm[k][w][c];
+        a.ln_partial[((int64_t)blockIdx.x * 2 + k) * E + c] = v;
+    }
+}
+template <int kN4>
+__global__ void __launch_bounds__(kTailThreads) module_tail_kernel(const __grid_constant__ ColSum a) {
+    grid_dependency_wait();
+    extern __shared__ __align__(16) float tail_sm[];
+    int block = blockIdx.x;
+    if (block < a.ln_blocks) {
+        tail_layer_norm<kN4>(a, reinterpret_cast<float (*)[kTailWarps][kN4 > 0 ? 128 * kN4 : 128]>(tail_sm));
+        return;
+    }
+    block -= a.ln_blocks;
+    if (block < a.col_blocks) {                        // two runs of 128 columns of a chunk a block, chunks fastest
+        const int u = 2 * block + (threadIdx.x >> 7), per_job = kColChunks * ((a.max_cols + 127) / 128);
+        const int j = u / per_job, chunk = u % per_job % kColChunks, c = u % per_job / kColChunks * 128 + (threadIdx.x & 127);
+        if (j < a.n && c < a.cols[j]) column_partial(a, j, chunk, c);
+        return;
+    }
+    block -= a.col_blocks;                             // a slice sum as gemm_splitk_reduce_kernel has it
+    const int per = (int)((a.split_mn + kTailThreads - 1) / kTailThreads);
+    const int p = block / per;
+    const int64_t i = (int64_t)(block - p * per) * kTailThreads + threadIdx.x;
+    if (i >= a.split_mn) return;
+    const float* src = a.split + (int64_t)p * a.splits * a.split_mn + i;
+    float acc = 0.f;
+    for (int s = 0; s < a.splits; s += 4) {
+        float v[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[e] = s + e < a.splits ? __ldg(src + (int64_t)(s + e) * a.split_mn) : 0.f;
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            if (s + e < a.splits) acc += v[e];
+    }
+    a.split_dst[p][i] = acc;
+}
+// Second stage: jobs as in column_sum_final_kernel, then dgamma and dbeta (32 columns a block, the blocks' sums in four parts).
+__global__ void __launch_bounds__(128) module_tail_final_kernel(const __grid_constant__ ColSum a) {
+    grid_dependency_wait();
+    const int j = blockIdx.y;
+    if (j < a.n) {
+        const int c = blockIdx.x * 128 + threadIdx.x;
+        if (c < a.cols[j]) column_final(a, j, c);
+        return;
+    }
+    __shared__ float part[kLnParts][32];
+    const int k = j - a.n, c = blockIdx.x * 32 + (threadIdx.x & 31), p = threadIdx.x >> 5;
+    float* dst = k == 0 ? a.ln_dgamma : a.ln_dbeta;
+    if (!dst || blockIdx.x * 32 >= a.E) return;
+    const int per = (a.ln_chunks + kLnParts - 1) / kLnParts, c0 = p * per, c1 = min(c0 + per, a.ln_chunks);
+    part[p][threadIdx.x & 31] = c < a.E ? column_chunk(a.ln_partial + (int64_t)k * a.E + c, 2 * (int64_t)a.E, c0, c1) : 0.f;
+    __syncthreads();
+    if (p == 0 && c < a.E) dst[c] = ((part[0][threadIdx.x] + part[1][threadIdx.x]) + part[2][threadIdx.x]) + part[3][threadIdx.x];
+}
+// Row widths that the tail's LayerNorm takes.
+bool tail_width(int E) { return row_pieces(E) > 0 || E <= 128; }
+// `scratch` as for column_sums.  Pointers of the LayerNorm have been checked (16 bytes, where row_pieces(E) > 0).
+int module_tail(ltca_ctx* ctx, ColSum a, int64_t rows, float* scratch) {
+    a.rows = rows;
+    a.partial = scratch;
+    int64_t per = (rows + kMaxLnChunks - 1) / kMaxLnChunks;
+    per = (per + kTailWarps - 1) / kTailWarps * kTailWarps;            // whole rounds of the warps
+    a.ln_rows = (int)per;
+    a.ln_chunks = a.ln_blocks = (int)((rows + per - 1) / per);
+    a.ln_partial = a.ln_dgamma || a.ln_dbeta ? scratch + (int64_t)a.n * kColChunks * a.max_cols : nullptr;
+    a.col_blocks = (a.n * kColChunks * ((a.max_cols + 127) / 128) + 1) / 2;
+    const int64_t blocks = a.ln_blocks + a.col_blocks + a.split_n * ((a.split_mn + kTailThreads - 1) / kTailThreads);
+    auto kern = module_tail_kernel<0>;
+    switch (row_pieces(a.E)) {
+        case 1: kern = module_tail_kernel<1>; break;
+        case 2: kern = module_tail_kernel<2>; break;
+        case 3: kern = module_tail_kernel<3>; break;
+        case 4: kern = module_tail_kernel<4>; break;
+        case 5: kern = module_tail_kernel<5>; break;
+        case 6: kern = module_tail_kernel<6>; break;
+        case 7: kern = module_tail_kernel<7>; break;
+        case 8: kern = module_tail_kernel<8>; break;
+    }
+    const size_t smem = (size_t)2 * kTailWarps * (a.E < 128 ? 128 : a.E) * sizeof(float);
+    static SmemOptIn once[9];
+    if (smem > 48 * 1024) LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(once[row_pieces(a.E)], ctx->device, kern, (int)smem));
+    LTCA_CUDA_OK(ctx, launch_dependent(kern, dim3((unsigned)blocks), dim3(kTailThreads), smem, ctx->stream, a));
+    const int ln_jobs = a.ln_partial ? 2 : 0;
+    if (a.n + ln_jobs == 0) return LTCA_OK;
+    const unsigned bx = (unsigned)((a.max_cols + 127) / 128), lx = ln_jobs ? (unsigned)((a.E + 31) / 32) : 0;
+    LTCA_CUDA_OK(ctx, launch_dependent(module_tail_final_kernel, dim3(bx > lx ? bx : lx, a.n + ln_jobs), dim3(128), 0, ctx->stream, a));
+    return LTCA_OK;
+}
+// Four jobs' chunks and the LayerNorm's, or six jobs' chunks.
 size_t colsum_scratch_bytes(const ltca_tsa_params* t) {
     const int hw = t->H * t->head_width;
-    return align_up((size_t)kMaxColJobs * kColChunks * (hw > t->E ? hw : t->E) * sizeof(float), 256);
+    return align_up((size_t)((kMaxColJobs - 2) * kColChunks + 2 * kMaxLnChunks) * (hw > t->E ? hw : t->E) * sizeof(float), 256);
 }
 
 // `xo` receives LayerNorm(x) (or x), `go` the gradient behind the dropout (null outputs: no such part); w: matrices to
@@ -1418,7 +1612,7 @@ int tensor_forward(ltca_ctx* ctx, const ltca_tsa_params* t, const ltca_tsa_param
 // tensor_backward on q, k, v and ctx.  `w`: the workspace behind `g`.  In parts only on the written-out-score path, from a kept forward and
 // with dy's bf16 copy in its place.
 int projected_backward(ltca_ctx* ctx, const ltca_tsa_params* t, const ltca_tsa_params& layout, const TPlan& pl, const BwdBufs& g, char* w,
-                       BwdPart part, bool want_dx, bool want_dw, const ltca_tsa_params* outer, float* outer_g) {
+                       BwdPart part, bool want_dx, bool want_dw, ColSum* sums, const ltca_tsa_params* outer, float* outer_g) {
     void *dyb = g.dyb, *dctx = g.dctx, *dq = g.dq, *dk = g.dk, *dv = g.dv;
     int rc;
     float* partial = reinterpret_cast<float*>(w); w += pl.partial;
@@ -1489,6 +1683,12 @@ int projected_backward(ltca_ctx* ctx, const ltca_tsa_params* t, const ltca_tsa_p
         }
         if (gemm_group_one_wave(ctx, gg) && gemm_group_aligned(gg)) {
             if ((rc = gemm_sm100_group(ctx, gg)) || pl.ks_in == 1) return rc;
+            if (sums->tail) {
+                sums->split = partial;
+                for (int i = 0; i < 4; ++i) sums->split_dst[i] = dst[i];
+                sums->split_mn = mn; sums->splits = pl.ks_in; sums->split_n = 4;
+                return LTCA_OK;
+            }
             return sum_splits(ctx, partial, reinterpret_cast<void**>(dst), 4, mn, pl.ks_in);
         }
     }
@@ -1588,7 +1788,7 @@ int tensor_backward(ltca_ctx* ctx, const ltca_tsa_params* t, bool want_dx, bool 
             }
             ctx->run_if.word = reinterpret_cast<const uint32_t*>(t->saved);
             ctx->run_if.value = kKeptProjections;
-            if ((rc = projected_backward(ctx, t, layout, pl[0], g, w, part, want_dx, want_dw, outer, outer_g))) return rc;
+            if ((rc = projected_backward(ctx, t, layout, pl[0], g, w, part, want_dx, want_dw, sums, outer, outer_g))) return rc;
             ctx->run_if.value = kKeptComposed;
             if ((rc = composed_backward(ctx, t, pl[1], g, w, part, want_dx, want_dw))) return rc;
         }
@@ -1596,7 +1796,7 @@ int tensor_backward(ltca_ctx* ctx, const ltca_tsa_params* t, bool want_dx, bool 
     } else if (composed) {
         if ((rc = composed_backward(ctx, t, pl[1], g, w, kWhole, want_dx, want_dw))) return rc;
     } else {
-        if ((rc = projected_backward(ctx, t, layout, pl[0], g, w, kWhole, want_dx, want_dw, outer, outer_g))) return rc;
+        if ((rc = projected_backward(ctx, t, layout, pl[0], g, w, kWhole, want_dx, want_dw, sums, outer, outer_g))) return rc;
     }
     if (want_dw) {
         // bias gradients (FlashAttention form): column sums of the projection outputs' gradients
@@ -1762,6 +1962,8 @@ static int prenorm_backward(ltca_ctx* ctx, const ltca_tsa_params* t, bool want_d
     c.workspace_bytes = t->workspace_bytes - 3 * act;
     ColSum sums;
     memset(&sums, 0, sizeof(sums));
+    const bool vec = row_pieces(t->E) == 0 || aligned16(dxin, t->x, t->ln_gamma, g, t->dx);
+    sums.tail = need_dxin && t->use_layer_norm && tail_width(t->E) && vec;
     if ((rc = tsa_backward(ctx, &c, need_dxin, want_dw, &sums, fused ? t : nullptr, drops ? gbuf : nullptr))) return rc;
     if (need_dxin && !t->use_layer_norm) {
         if (want_dx && t->use_residual) {
@@ -1769,6 +1971,15 @@ static int prenorm_backward(ltca_ctx* ctx, const ltca_tsa_params* t, bool want_d
         } else if (want_dx) {
             LTCA_CUDA_OK(ctx, cudaMemcpyAsync(t->dx, dxin, (size_t)n * sizeof(float), cudaMemcpyDeviceToDevice, ctx->stream));
         }
+    } else if (sums.tail) {
+        sums.ln_g = dxin; sums.ln_x = t->x; sums.ln_gamma = t->ln_gamma;
+        sums.ln_res = want_dx && t->use_residual ? g : nullptr;
+        sums.ln_dx = want_dx ? t->dx : nullptr;
+        sums.ln_dgamma = want_ln_params ? t->dgamma : nullptr;
+        sums.ln_dbeta = want_ln_params ? t->dbeta : nullptr;
+        sums.E = t->E;
+        sums.eps = 1e-5f;
+        return module_tail(ctx, sums, rows, colsum_scratch);
     } else if (need_dxin) {
         // LayerNorm(x) is no longer needed: its buffer takes dxin * xhat, whose column sums are dgamma
         float* prod = (want_ln_params && t->dgamma) ? xin : nullptr;
