@@ -90,6 +90,11 @@ struct StatsArgs {
     float *lse2, *delta;
     float* dq_acc;           // optional: fp32 [B*H, Sq_pad, 64] accumulator of the fused kernel, cleared here
     uint4* dout_bf16;        // fp32 storage: dO rounded to bf16, [B*H, Sq, 64], for the contractions
+    // ... and Q, K and V likewise, by the blocks behind the statistics': tensor j's from pack0[j] on
+    const float* src[3];
+    ltca_strides src_st[3];
+    uint4* dst[3];
+    unsigned S[3], stat_blocks, pack0[4];
 };
 
 __device__ __forceinline__ void load8(const __nv_bfloat16* p, float (&f)[8]) {
@@ -112,9 +117,37 @@ __device__ __forceinline__ void load8(const float* p, float (&f)[8]) {
 // is a multiple of 256), so the pair comes from two 32-bit divisions by block (inside a step at B8 H16 S4096 46.3 us, with a
 // row's place from 64-bit divisions per thread 47.4).  More rows per thread were slower.
 constexpr int kStatsRows = 32;
+// kPackRounds rows of 64 floats to bf16 per eight lanes, their loads in flight together.  In the statistics' launch, of which they
+// need nothing: a launch of their own was 1 to 2 us of a backward (B32 H8 S256 65.1 -> 63.3, B2 H4 S100 11.0 -> 9.7).
+constexpr unsigned kPackRounds = 4, kPackRows = kPackRounds * kStatsRows;
+__device__ __forceinline__ void pack_rows(const StatsArgs& a, unsigned block) {
+    const int j = block < a.pack0[1] ? 0 : block < a.pack0[2] ? 1 : 2;
+    const unsigned S = a.S[j], rows = (unsigned)(a.B * a.H) * S, row0 = (block - a.pack0[j]) * kPackRows + (threadIdx.x >> 3), sub = threadIdx.x & 7;
+    float f[kPackRounds][8];
+#pragma unroll
+    for (unsigned c = 0; c < kPackRounds; ++c) {
+        const unsigned row = row0 + c * kStatsRows;
+        if (row >= rows) break;
+        const unsigned bh = row / S, s = row - bh * S, b = bh / (unsigned)a.H, h = bh - b * (unsigned)a.H;
+        load8(a.src[j] + b * a.src_st[j].batch + h * a.src_st[j].head + s * a.src_st[j].seq + 8 * sub, f[c]);
+    }
+#pragma unroll
+    for (unsigned c = 0; c < kPackRounds; ++c) {
+        const unsigned row = row0 + c * kStatsRows;
+        if (row >= rows) break;
+        a.dst[j][(uint64_t)row * 8 + sub] = make_uint4(pack_bf16x2(f[c][0], f[c][1]), pack_bf16x2(f[c][2], f[c][3]),
+                                                       pack_bf16x2(f[c][4], f[c][5]), pack_bf16x2(f[c][6], f[c][7]));
+    }
+}
 template <typename T>
 __global__ void __launch_bounds__(8 * kStatsRows) attn_bwd_stats_kernel(const StatsArgs a) {
     grid_dependency_wait();
+    if constexpr (sizeof(T) == 4) {
+        if (blockIdx.x >= a.stat_blocks) {
+            pack_rows(a, blockIdx.x - a.stat_blocks);
+            return;
+        }
+    }
     const unsigned per_pair = (unsigned)a.Sq_pad / kStatsRows, bh = blockIdx.x / per_pair;
     const unsigned b = bh / (unsigned)a.H, h = bh - b * (unsigned)a.H;
     const int qi = (int)(blockIdx.x - bh * per_pair) * kStatsRows + (threadIdx.x >> 3), sub = threadIdx.x & 7;
@@ -2455,27 +2488,38 @@ int launch_attn_bwd_sm100(ltca_ctx* ctx, const ltca_attn_params* p) {
     }
 
     StatsArgs s;
+    memset(&s, 0, sizeof(s));
     s.B = p->B; s.H = p->H; s.Sq = p->Sq; s.Sq_pad = (int)align_up((size_t)p->Sq, 256);
     s.o = p->o; s.dout = p->dout; s.os = p->o_strides; s.dos = p->do_strides;
     s.lse = p->lse; s.lse2 = lse2; s.delta = delta; s.dq_acc = dq_acc;
     // fp32 storage: bf16 copies of the four operands (dO's comes with the statistics), fp32 gradients out
     void *qb = w, *kb = w + pq, *vb = w + pq + pk, *gb = w + pq + 2 * pk;
     s.dout_bf16 = reinterpret_cast<uint4*>(gb);
-    const unsigned blocks = (unsigned)((int64_t)p->B * p->H * (s.Sq_pad / kStatsRows));
+    s.stat_blocks = (unsigned)((int64_t)p->B * p->H * (s.Sq_pad / kStatsRows));
     kernel_timing_mark(ctx, 0);
-    if (p->dtype == LTCA_BF16)
-        LTCA_CUDA_OK(ctx, launch_dependent_if(small_attention_call(p), attn_bwd_stats_kernel<__nv_bfloat16>, dim3(blocks), dim3(8 * kStatsRows), 0, ctx->stream, s));
-    else
-        LTCA_CUDA_OK(ctx, launch_dependent_if(small_attention_call(p), attn_bwd_stats_kernel<float>, dim3(blocks), dim3(8 * kStatsRows), 0, ctx->stream, s));
-    LTCA_LAUNCH_OK(ctx, "attn_bwd_stats_kernel");
-    if (p->dtype == LTCA_BF16) kernel_timing_mark(ctx, 1);
-
-    if (p->dtype == LTCA_BF16)
+    if (p->dtype == LTCA_BF16) {
+        LTCA_CUDA_OK(ctx, launch_dependent_if(small_attention_call(p), attn_bwd_stats_kernel<__nv_bfloat16>, dim3(s.stat_blocks), dim3(8 * kStatsRows), 0, ctx->stream, s));
+        LTCA_LAUNCH_OK(ctx, "attn_bwd_stats_kernel");
+        kernel_timing_mark(ctx, 1);
         return (p->keep_mask ? launch_main<__nv_bfloat16, true> : launch_main<__nv_bfloat16, false>)(
             ctx, p, words, p->q, p->k, p->v, p->dout, p->q_strides, p->k_strides, p->v_strides, p->do_strides, lse2, delta, dq_acc);
+    }
 
     const PackJob jobs[3] = {{p->q, p->q_strides, qb, p->Sq}, {p->k, p->k_strides, kb, p->Sk}, {p->v, p->v_strides, vb, p->Sk}};
-    if (int rc = pack_many_to_bf16(ctx, jobs, 3, p->B, p->H, kD)) return rc;
+    int64_t blocks = s.stat_blocks;
+    for (int j = 0; j < 3; ++j) {
+        if (bad16(jobs[j].src, jobs[j].st)) return fail(ctx, LTCA_ERR_INVALID, "fp32 tensors need 16-byte aligned rows for the tensor-pipe modes");
+        s.src[j] = reinterpret_cast<const float*>(jobs[j].src);
+        s.src_st[j] = jobs[j].st;
+        s.dst[j] = reinterpret_cast<uint4*>(jobs[j].dst);
+        s.S[j] = (unsigned)jobs[j].S;
+        const int64_t rows = (int64_t)p->B * p->H * jobs[j].S;
+        blocks += (rows + kPackRows - 1) / kPackRows;
+        if (rows > 0xffffffffll - kPackRows || blocks > 0x7fffffffll) return fail(ctx, LTCA_ERR_INVALID, "pack: tensor too large");
+        s.pack0[j + 1] = (unsigned)(blocks - s.stat_blocks);
+    }
+    LTCA_CUDA_OK(ctx, launch_dependent_if(small_attention_call(p), attn_bwd_stats_kernel<float>, dim3((unsigned)blocks), dim3(8 * kStatsRows), 0, ctx->stream, s));
+    LTCA_LAUNCH_OK(ctx, "attn_bwd_stats_kernel");
     kernel_timing_mark(ctx, 1);
     ltca_strides cq{(int64_t)p->H * p->Sq * kD, (int64_t)p->Sq * kD, kD};
     ltca_strides ck{(int64_t)p->H * p->Sk * kD, (int64_t)p->Sk * kD, kD};

@@ -20,7 +20,7 @@ def test_steps_and_rescales(ctx, Sk, masked):
     # the last key of every second step is far above the rest for rows 5, 37 and 129 alone
     q[..., 0], k[..., 0] = 0.0, 0.0
     q[:, :, [5, 37, 129], 0] = 8.0
-    peaks = torch.arange(63, Sk, 128, device="cuda")
+    peaks = torch.arange(63, max(Sk, 63), 128, device="cuda")
     k[:, :, peaks, 0] = 20.0 + 10.0 * torch.arange(len(peaks), device="cuda")
     q, k, v = (t.bfloat16() for t in (q, k, v))
     m = (torch.rand((B, Sq, Sk), generator=g, device="cuda") > 0.3).float() if masked else None
