@@ -784,7 +784,7 @@ __global__ void __launch_bounds__(NT, TK < 64 || DP <= 32 ? 3 : DP <= 64 ? 2 : 1
 // H8 S256, with 128 (a larger block of scores each, half the warps) 318.  What bounds it: issue slots (about 6300 cycles a tile and
 // SM at D = 32) and shared-memory wavefronts (5000), at 16 warps an SM.
 // ----------------------------------------------------------------------------------------------
-template <typename T, int DP, int N, int NT, bool kMask, bool kForm>
+template <typename T, int DP, int N, int NT, int kMask, bool kForm>
 __global__ void __launch_bounds__(NT, kForm ? 256 / NT : DP <= 32 ? 4 : 2) attn_bwd_fp32_kernel(const CoreArgs a) {
     grid_dependency_wait();
     constexpr int LD = DP + kPad, LP = N + kPad, RS = NT / 16, RM = N / RS, CN = N / 16, NW = N / 32;
@@ -843,12 +843,31 @@ __global__ void __launch_bounds__(NT, kForm ? 256 / NT : DP <= 32 ? 4 : 2) attn_
             const float l = qi < a.Sq ? a.lse_in[stat0 + qi] : kNegInf;
             row_lse[threadIdx.x] = l == kNegInf ? INFINITY : l;
         }
-        if (kMask && threadIdx.x < NW * N) {
-            const int qi = q0 + threadIdx.x / NW, kw = k0 / 32 + threadIdx.x % NW;
-            mask_sm[threadIdx.x] = a.mask_bits ? mask_word<kWords>(a, b, qi, kw) : mask_word<kDense>(a, b, qi, kw);
+        // dense mask: as words where there are any, else every warp votes the words (32 keys of a row each) of its share of the
+        // rows.  The words cost a launch, the votes 2 to 7 % of a step: up to two steps a CTA go without (backward, us, words and
+        // votes: B8 H8 S32 D32 8.9 and 5.7, B16 H4 S100 D32 26.5 and 25.3, B16 H8 S250 D32 95.2 and 94.4, B12 H8 S400 D32 203 and 217).
+        constexpr int kRows = N / (NT / 32);
+        float mv[kRows * NW];
+        const int lane = threadIdx.x & 31, mask_row = (threadIdx.x >> 5) * kRows;
+        if constexpr (kMask == kDense) {
+            const float* p = a.keep_mask + ((int64_t)b * a.Sq + q0 + mask_row) * a.Sk + k0 + lane;
+#pragma unroll
+            for (int r = 0; r < kRows; ++r, p += a.Sk)
+#pragma unroll
+                for (int w = 0; w < NW; ++w)
+                    mv[r * NW + w] = q0 + mask_row + r < a.Sq && k0 + 32 * w + lane < a.Sk ? __ldg(p + 32 * w) : 0.f;
+        } else if constexpr (kMask == kWords) {
+            if (threadIdx.x < NW * N) mask_sm[threadIdx.x] = mask_word<kWords>(a, b, q0 + threadIdx.x / NW, k0 / 32 + threadIdx.x % NW);
         }
         if constexpr (kForm) form_dout<DP, N, NT, false>(Gs, a, b, h, q0);
         cp_async_wait<0>();
+        if constexpr (kMask == kDense) {
+#pragma unroll
+            for (int w = 0; w < kRows * NW; ++w) {
+                const uint32_t bits = __ballot_sync(0xffffffffu, mv[w] != 0.f);
+                if (lane == 0) mask_sm[mask_row * NW + w] = bits;
+            }
+        }
         __syncthreads();
         {   // delta = rowsum(dO o O)
             float4 e = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -1097,7 +1116,7 @@ int run_small_dq(ltca_ctx* ctx, const CoreArgs& a) {
 }
 bool fills_sms(const ltca_ctx* ctx, int B, int H, int S) { return (int64_t)B * H * ((S + 63) / 64) >= ctx->sm_device; }
 // The one-pass backward, in as many launches as the room for dQ's shares allows.
-template <typename T, int DP, int N, int NT, bool kMask, bool kForm = false>
+template <typename T, int DP, int N, int NT, int kMask, bool kForm = false>
 int launch_one_pass(ltca_ctx* ctx, CoreArgs a) {
     static SmemOptIn once;
     constexpr size_t smem = ((size_t)4 * N * (DP + kPad) + N * (N + kPad) + 2 * N + (kMask ? N * N / 32 : 0)) * sizeof(float);
@@ -1118,11 +1137,13 @@ int launch_one_pass(ltca_ctx* ctx, CoreArgs a) {
 // Key blocks of 64, or of 32 where that holds all keys: a quarter of a tile's scores (B16 H8 S16: D16 6.7 -> 3.8 us, D32 9.1 -> 4.6).
 template <typename T, int DP, bool kMask>
 int run_one_pass(ltca_ctx* ctx, const CoreArgs& a) {
-    constexpr int NT = DP <= 32 ? 128 : kOnePassThreads64;
+    constexpr int NT = DP <= 32 ? 128 : kOnePassThreads64, kM = kMask ? kDense : kNoMask;
     if constexpr (sizeof(T) == 4) {
-        if (a.dy) return launch_one_pass<T, DP, 32, 128, kMask, true>(ctx, a);
+        if (a.dy) return launch_one_pass<T, DP, 32, 128, kM, true>(ctx, a);
     }
-    return a.Sk <= 32 ? launch_one_pass<T, DP, 32, 128, kMask>(ctx, a) : launch_one_pass<T, DP, 64, NT, kMask>(ctx, a);
+    if (a.Sk <= 32) return launch_one_pass<T, DP, 32, 128, kM>(ctx, a);
+    if (kMask && a.mask_bits) return launch_one_pass<T, DP, 64, NT, kWords>(ctx, a);
+    return launch_one_pass<T, DP, 64, NT, kM>(ctx, a);
 }
 template <typename T, int DP, bool kMask>
 int run_rows(ltca_ctx* ctx, const CoreArgs& a, bool bwd) {
@@ -1368,7 +1389,7 @@ static OnePass one_pass(const ltca_attn_params* p) {
     const int64_t all = (int64_t)p->B * p->H, blocks = ((int64_t)p->Sk + 63) / 64;
     o.ld = (p->D + 3) / 4 * 4;
     const size_t one = (size_t)blocks * p->Sq * o.ld * sizeof(float);
-    if (blocks > 1 && one > kPartBytes) return o;
+    if (blocks > 65535 || (blocks > 1 && one > kPartBytes)) return o;
     const int64_t fit = blocks > 1 ? (int64_t)(kPartBytes / one) : all;
     o.pairs = (int)(fit < all ? fit : all);
     o.bytes = blocks > 1 ? o.pairs * one : 0;
@@ -1412,18 +1433,19 @@ int launch_attn_bwd_fp32(ltca_ctx* ctx, const ltca_attn_params* p, const FromOut
         a.dy_batch = from->batch; a.dy_seq = from->seq;
     }
     if (p->D <= 128) {
-        // delta, dQ's shares, the mask's words; a workspace without room for the shares takes the two kernels, one without room for
-        // the words (sized without the mask) reads the mask as it is
+        // delta, dQ's shares, the mask's words (not in a workspace sized without the mask); without room for the shares the two
+        // kernels run
         const OnePass one = one_pass(p);
-        const bool room = one.pairs && (!from || p->Sk <= 32) && p->workspace_bytes >= delta_bytes(p) + one.bytes;
-        const size_t used = delta_bytes(p) + (room ? one.bytes : 0);
-        if (room && one_pass_pays(ctx, p)) {
+        const bool once = one.pairs && (!from || p->Sk <= 32) && p->workspace_bytes >= delta_bytes(p) + one.bytes && one_pass_pays(ctx, p);
+        if (once) {
             a.pairs = one.pairs;
             a.part_ld = one.ld;
             a.dq_part = one.bytes ? reinterpret_cast<float*>(reinterpret_cast<char*>(p->workspace) + delta_bytes(p)) : nullptr;
         }
         const void* words = nullptr;
-        if (int rc = mask_words_of(ctx, p, used, &words)) return rc;
+        if (!once || p->Sk > 128) {
+            if (int rc = mask_words_of(ctx, p, delta_bytes(p) + (once ? one.bytes : 0), &words)) return rc;
+        }
         const MaskArgs m = mask_args(p, words);
         a.mask_bits = m.by_query;
         a.mask_nw = m.nk;
