@@ -91,8 +91,8 @@ __device__ __forceinline__ void store4(T* row, int d, int D, float4 v, bool vec)
     }
 }
 
-// How the backward kernels meet a dense mask: not at all, as packed words, or (a workspace sized without the mask has no room
-// for the words) as it is.
+// How the backward kernels meet a dense mask: not at all, as packed words, or as it is (a workspace sized without the mask has no
+// room for the words; short one-pass calls).
 constexpr int kNoMask = 0, kWords = 1, kDense = 2;
 // Word w of query qi's row: bit c = key 32 w + c is kept; 0 beyond the tensor.
 template <int kMask>

@@ -162,8 +162,8 @@ __device__ __forceinline__ bool is_mn(const Maps& maps, int problem, int bit) {
 // tensor memory, convert it and hand it to the TMA store, the MMA thread is already accumulating tile i+1 and
 // the producer is loading tile i+2's operands.
 // kKind: kHeads has operands that heads share, sums over heads and results that are added to C (the plain kernel is free of
-// them: they cost it 0.1 us a launch); the members of a kGroup differ in their operand forms (kAMn, kBMn do not count) and
-// their number of terms.  Four weight gradients of 8 x 512 x 512 x 512 with three and two terms: 55 us as four launches, 31 as
+// them: they cost it 0.1 us a launch); the members of a kGroup differ in shape, split of K, operand forms (kAMn, kBMn do
+// not count) and number of terms.  Four weight gradients of 8 x 512 x 512 x 512 with three and two terms: 55 us as four launches, 31 as
 // one.
 enum GemmKind { kPlain, kHeads, kGroup };
 template <bool kAMn, bool kBMn, int kBN, bool kPair, int kKind>
