@@ -536,15 +536,9 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
 // dealt out in pieces of 128 rows.  A persistent kernel with four tiles on one key stream, which this replaces, made the
 // early tiles of 512 causal rows wait for the late ones' keys: B64 H8 S512 causal 68 us against 46 now, B8 H16 S4096 causal
 // 440 against 365.  What it pays is a set-up per tile and a K/V read per tile from L2 (20 bytes per clock and SM).
-//   - warps 0-3 softmax, one row per thread.  Head_dim 64: 64 keys per step, tensor memory S [0, 64), O [64, 128).
-//   - head_dim 128, bf16 results: 64 keys per step and two score buffers, S0 [0, 64), S1 [64, 128), O [128, 256), so that a step's
-//     scores are formed under the softmax of the step before; its P V waits for nothing else.  A rescale, rare, first waits for
-//     the products before it.  The ring's four slots of 64 keys go in the order of use (K0 K1 V0 K2 V1 ...), two steps ahead.
-//     With one buffer and 128 keys per step (two slots of 128) a tile's softmax and its products took turns, as far as the SM's
-//     other tile did not fill the gaps: B4 H16 S1500 85 us and 78, causal 49.5 and 46.3, B8 H16 S4096 985 and 936, B1 H8 S700 13.9 and
-//     11.9, B64 H8 S256 37.7 and 35.5 (B16 H8 S256 causal 8.3 and 8.7).  K and V in the order K0 V0 K1 V1 gained half of it.  An
-//     earlier form had two threads per row, who met once a step to agree on the row's maximum (B8 H16 S4096 causal 568 us, one per
-//     row 525).
+//   - warps 0-3 softmax, one row per thread, head_dim keys per step; tensor memory S [0, D), O [D, 2 D).  At head_dim 128 a
+//     thread so holds 128 scores in its 216 registers and two warps share a scheduler; two threads per row, 64 scores each,
+//     had four of them but met once a step to agree on the row's maximum (B8 H16 S4096 causal 568 us, one per row 525).
 //     fp32 results at head_dim 128 have two threads per row (warps 0-7), which share the work of P's second term, and the
 //     halves of P below are one thread's each (B8 H16 S2048 causal 325 -> 319 us).  Not with a mask, whose words no longer fit
 //     their 104 registers: what is spilled goes out to L2, since the tiles leave an SM next to no L1 (masked B64 H8 S200 126 us
@@ -568,26 +562,23 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
 // ---------------------------------------------------------------------------------------------
 template <int D, bool kSplitP, bool kMask>
 struct TileCfg {
-    static constexpr bool kDouble = D == 128 && !kSplitP;          // two score buffers (above)
-    static constexpr int kBN = kDouble ? 64 : D;                   // keys per step
+    static constexpr int kBN = D;                                  // keys per step
     static constexpr int kRowSplit = D == 128 && kSplitP && !kMask ? 2 : 1;    // threads per row
     static constexpr int kCols = kBN / kRowSplit;                  // score columns of a thread
     static constexpr int kMathWarps = 4 * kRowSplit;
     static constexpr int kThreads = 32 * (kMathWarps + 4);
     static constexpr int kCtas = D == 64 ? 4 : 2;                  // per SM
     static constexpr int kLaunchRegs = 65536 / (kCtas * kThreads) / 8 * 8;
-    static constexpr int kMathRegs = D == 64 || kRowSplit > 1 ? 104 : 216, kCtrlRegs = D == 64 ? 24 : kRowSplit > 1 ? 32 : 40;
+    static constexpr int kMathRegs = kCols == 64 ? 104 : 216, kCtrlRegs = D == 64 ? 24 : kCols == 64 ? 32 : 40;
     static_assert(32 * kMathWarps * kMathRegs + 128 * kCtrlRegs <= kThreads * kLaunchRegs, "register budget");
     static constexpr int kBlocks = D / 64;                         // 128-byte column blocks of a row
     static constexpr int kQBytes = kBlockM * D * 2;
     static constexpr int kKvBytes = kBN * D * 2;
-    static constexpr int kStages = kBN == 64 ? 4 : 2;              // ring slots: K0 V0 K1 V1 ...
+    static constexpr int kStages = D == 64 ? 4 : 2;                // ring slots: K0 V0 K1 V1 ...
     static constexpr int kRingOff = kQBytes;
     static constexpr int kXchgOff = kRingOff + kStages * kKvBytes; // row maxima [2 buffers][2 halves][128], row sums [2][128]
     static constexpr int kBarOff = kXchgOff + (kRowSplit > 1 ? 3 * 2 * kBlockM * 4 : 0);
-    // q_full, kv_full[], kv_empty[], s_full[2 buffers], p_full[2 buffers][2 halves], staged, pair[4]
-    static constexpr int kNumBars = 1 + 2 * kStages + 2 + 4 + 1 + 4;
-    static constexpr int kOCol = kDouble ? 128 : kBN;              // tensor memory: the score buffer(s), O
+    static constexpr int kNumBars = 1 + 2 * kStages + 4 + 4;       // q_full, kv_full[], kv_empty[], s_full, p_full[2], staged, pair[4]
     static constexpr int kMiscOff = kBarOff + kNumBars * 8;        // tmem base, abort flag, a team's next tile
     static constexpr int kDynBytes = kMiscOff + 32 + 1024;
     static_assert(kCtas * (kDynBytes + 1024) <= 228 * 1024, "shared memory");
@@ -616,8 +607,8 @@ attn_fwd_tile_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
     const uint32_t bar_base = smem_base + L::kBarOff;
     auto bar_kv_full = [&](int s) { return bar_base + 8u * (1 + s); };
     auto bar_kv_empty = [&](int s) { return bar_base + 8u * (1 + L::kStages + s); };
-    const uint32_t bar_q_full = bar_base, bar_s_full = bar_base + 8u * (1 + 2 * L::kStages), bar_p_full = bar_s_full + 16,
-                   bar_staged = bar_s_full + 48, bar_pair0 = bar_s_full + 56;
+    const uint32_t bar_q_full = bar_base, bar_s_full = bar_base + 8u * (1 + 2 * L::kStages), bar_p_full = bar_s_full + 8,
+                   bar_staged = bar_s_full + 24, bar_pair0 = bar_s_full + 32;
     volatile uint32_t* misc = reinterpret_cast<volatile uint32_t*>(smem_gen + L::kMiscOff);
     volatile uint32_t* misc_cta = reinterpret_cast<volatile uint32_t*>(smem_raw + (smem_cta - smem_u32(smem_raw)) + L::kMiscOff);
     const int warp = kTeams > 1 ? __shfl_sync(0xffffffffu, tid >> 5, 0) : tid >> 5, lane = tid & 31;
@@ -626,11 +617,6 @@ attn_fwd_tile_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
         mbar_init(bar_q_full, 1);
         for (int s = 0; s < L::kStages; ++s) { mbar_init(bar_kv_full(s), 1); mbar_init(bar_kv_empty(s), 1); }
         mbar_init(bar_s_full, 1);
-        if (L::kDouble) {
-            mbar_init(bar_s_full + 8u, 1);
-            mbar_init(bar_p_full + 16u, 4);
-            mbar_init(bar_p_full + 24u, 4);
-        }
         mbar_init(bar_p_full, L::kMathWarps);  // the first half of P, and O at its scale in all columns
         mbar_init(bar_p_full + 8u, 4);
         mbar_init(bar_staged, L::kMathWarps);
@@ -710,98 +696,55 @@ attn_fwd_tile_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
                     ok = mbar_wait(bar_kv_empty(s), phase_of(e0 + e) ^ 1u, wc, 0x50);
                     if (!ok) break;
                     mbar_arrive_expect_tx(bar_kv_full(s), (uint32_t)L::kKvBytes);
-                    bool is_v = (e & 1) != 0;
-                    int step = e >> 1;
-                    if constexpr (L::kDouble) {                        // K0 K1 V0 K2 V1 K3 ... (entry_k, entry_v)
-                        is_v = e == 2 * n_t - 1 || (e > 0 && !(e & 1));
-                        step = is_v ? (e == 2 * n_t - 1 ? n_t - 1 : e / 2 - 1) : (e + 1) / 2;
-                    }
                     for (int kb = 0; kb < L::kBlocks; ++kb)
-                        tma_load_4d(ring + s * L::kKvBytes + kb * (kBN * 128), is_v ? &tmap_v : &tmap_k, bar_kv_full(s), kb * 64,
-                                    step * kBN, h, b);
+                        tma_load_4d(ring + s * L::kKvBytes + kb * (kBN * 128), (e & 1) ? &tmap_v : &tmap_k, bar_kv_full(s), kb * 64,
+                                    (e >> 1) * kBN, h, b);
                 }
             } else if (warp == kMmaWarp && lane == 0 && n_t > 0) {
                 constexpr uint32_t idesc_qk = make_idesc_bf16(kBlockM, kBN, 0, 0);
                 constexpr uint32_t idesc_pv = make_idesc_bf16(kBlockM, D, 0, 1);
                 const uint32_t q_lo = smem_desc_lo(smem_base, 16), k_lo = smem_desc_lo(ring, 16), v_lo = smem_desc_lo(ring, kBN * 128);
-                auto issue_qk = [&](int s, int buf) {
+                auto issue_qk = [&](int s) {
     #pragma unroll
                     for (int k = 0; k < D / 16; ++k)
-                        mma_ss_lo(tmem_base + 64 * buf, q_lo + (k / 4) * (kBlockM * 8) + (k % 4) * 2,
+                        mma_ss_lo(tmem_base, q_lo + (k / 4) * (kBlockM * 8) + (k % 4) * 2,
                                   k_lo + ((s * L::kKvBytes) >> 4) + (k / 4) * (kBN * 8) + (k % 4) * 2, idesc_qk, k > 0 ? 1u : 0u);
                 };
-                auto issue_pv = [&](int s, int part, bool first, int buf) {     // one half of the step's keys
+                auto issue_pv = [&](int s, int part, bool first) {     // one half of the step's keys
                     constexpr int kSteps = kBN / 32;
                     const uint32_t vd = v_lo + ((s * L::kKvBytes) >> 4);
     #pragma unroll
                     for (int t = 0; t < (kSplitP ? 2 : 1); ++t)
     #pragma unroll
                         for (int k = 0; k < kSteps; ++k)
-                            mma_ts_lo(tmem_base + L::kOCol, tmem_base + 64 * buf + (kBN / 2) * t + (part * kSteps + k) * 8, vd + 128 * (part * kSteps + k),
+                            mma_ts_lo(tmem_base + kBN, tmem_base + (kBN / 2) * t + (part * kSteps + k) * 8, vd + 128 * (part * kSteps + k),
                                       idesc_pv, (!first || t > 0 || k > 0) ? 1u : 0u);
                 };
                 bool ok = mbar_wait(bar_q_full, (uint32_t)(tiles & 1), wc, 0x51) && mbar_wait(bar_kv_full(slot_of(e0)), phase_of(e0), wc, 0x52);
                 if (ok) {
                     tc_fence_after_sync();
-                    issue_qk(slot_of(e0), 0);
+                    issue_qk(slot_of(e0));
                     mma_commit(bar_kv_empty(slot_of(e0)));
                     mma_commit(bar_s_full);
                 }
-                if constexpr (L::kDouble) {
-                    // Score buffer j & 1 belongs to step j: S, then P, until P V has read it, and S of step j + 2.  Its barrier completes
-                    // with step j's scores and then once more behind step j's P V, whether or not scores follow.
-                    // The ring goes in the order of use, K0 K1 V0 K2 V1 ...: a step's K and V are asked for two steps ahead.
-                    auto entry_k = [&](int j) { return j < 2 ? j : 2 * j - 1; };
-                    auto entry_v = [&](int j) { return min(2 * j + 2, 2 * n_t - 1); };
-                    if (ok && n_t > 1) {
-                        ok = mbar_wait(bar_kv_full(slot_of(1)), phase_of(1), wc, 0x54);
-                        if (ok) {
-                            tc_fence_after_sync();
-                            issue_qk(slot_of(1), 1);
-                            mma_commit(bar_kv_empty(slot_of(1)));
-                        }
-                    }
-                    if (ok) mma_commit(bar_s_full + 8u);
-                    for (int j = 0; j < n_t && ok; ++j) {
-                        const int e_v = entry_v(j), e_k = entry_k(j + 2), buf = j & 1;
-                        ok = mbar_wait(bar_kv_full(slot_of(e_v)), phase_of(e_v), wc, 0x53);
-                        for (int part = 0; part < 2 && ok; ++part) {
-                            ok = mbar_wait(bar_p_full + 16u * buf + 8u * part, (uint32_t)((j >> 1) & 1), wc, 0x55);
-                            if (!ok) break;
-                            tc_fence_after_sync();
-                            issue_pv(slot_of(e_v), part, j == 0 && part == 0, buf);
-                        }
+                for (int j = 0; j < n_t && ok; ++j) {
+                    const int e_v = e0 + 2 * j + 1, e_k = e0 + 2 * j + 2;
+                    const bool more = j + 1 < n_t;
+                    ok = mbar_wait(bar_kv_full(slot_of(e_v)), phase_of(e_v), wc, 0x53);
+                    if (more) ok = ok && mbar_wait(bar_kv_full(slot_of(e_k)), phase_of(e_k), wc, 0x54);
+                    for (int part = 0; part < 2 && ok; ++part) {
+                        ok = mbar_wait(bar_p_full + 8u * part, (uint32_t)((steps + j) & 1), wc, 0x55);
                         if (!ok) break;
-                        mma_commit(bar_kv_empty(slot_of(e_v)));
-                        if (j + 2 < n_t) {
-                            ok = mbar_wait(bar_kv_full(slot_of(e_k)), phase_of(e_k), wc, 0x54);
-                            if (!ok) break;
-                            tc_fence_after_sync();
-                            issue_qk(slot_of(e_k), buf);
-                            mma_commit(bar_kv_empty(slot_of(e_k)));
-                        }
-                        mma_commit(bar_s_full + 8u * buf);
+                        tc_fence_after_sync();
+                        issue_pv(slot_of(e_v), part, j == 0 && part == 0);
                     }
-                } else {
-                    for (int j = 0; j < n_t && ok; ++j) {
-                        const int e_v = e0 + 2 * j + 1, e_k = e0 + 2 * j + 2;
-                        const bool more = j + 1 < n_t;
-                        ok = mbar_wait(bar_kv_full(slot_of(e_v)), phase_of(e_v), wc, 0x53);
-                        if (more) ok = ok && mbar_wait(bar_kv_full(slot_of(e_k)), phase_of(e_k), wc, 0x54);
-                        for (int part = 0; part < 2 && ok; ++part) {
-                            ok = mbar_wait(bar_p_full + 8u * part, (uint32_t)((steps + j) & 1), wc, 0x55);
-                            if (!ok) break;
-                            tc_fence_after_sync();
-                            issue_pv(slot_of(e_v), part, j == 0 && part == 0, 0);
-                        }
-                        if (!ok) break;
-                        mma_commit(bar_kv_empty(slot_of(e_v)));
-                        if (more) {
-                            issue_qk(slot_of(e_k), 0);
-                            mma_commit(bar_kv_empty(slot_of(e_k)));
-                        }
-                        mma_commit(bar_s_full);                            // S of step j + 1 ready, O holds steps 0 .. j
-                }
+                    if (!ok) break;
+                    mma_commit(bar_kv_empty(slot_of(e_v)));
+                    if (more) {
+                        issue_qk(slot_of(e_k));
+                        mma_commit(bar_kv_empty(slot_of(e_k)));
+                    }
+                    mma_commit(bar_s_full);                            // S of step j + 1 ready, O holds steps 0 .. j
                 }
             }
         } while (kTeams > 1);
@@ -810,7 +753,7 @@ attn_fwd_tile_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
         const int wq = warp & 3, half = kRS > 1 ? warp >> 2 : 0;
         const int row = wq * 32 + lane;
         const uint32_t lane_base = (uint32_t)(wq * 32) << 16;
-        const uint32_t tS = tmem_base + lane_base + half * kC, tO = tmem_base + lane_base + L::kOCol + half * (D / kRS);
+        const uint32_t tS = tmem_base + lane_base + half * kC, tO = tmem_base + lane_base + kBN + half * (D / kRS);
         const uint32_t tP = tmem_base + lane_base + half * (kC / 2), tPlo = tP + kBN / 2;
         float* xchg = reinterpret_cast<float*>(smem_gen + L::kXchgOff);
         auto xslot = [&](int buf, int hf) { return xchg + (buf * 2 + hf) * kBlockM + row; };
@@ -843,13 +786,12 @@ attn_fwd_tile_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
     #pragma unroll
                 for (int w = 0; w < kC / 32; ++w)
                     keep[w] = kMask ? mask_bits_of_queries(a.mask, b, q0 + wq * 32, j * kBN + half * kC + 32 * w) : ~0u;
-                const uint32_t buf = L::kDouble ? j & 1 : 0;
-                ok = mbar_wait_warp(bar_s_full + 8u * buf, (uint32_t)((L::kDouble ? j >> 1 : s_full0 + j) & 1), wc, 0x56);
+                ok = mbar_wait_warp(bar_s_full, (uint32_t)((s_full0 + j) & 1), wc, 0x56);
                 if (!ok) break;
                 tc_fence_after_sync();
                 uint32_t su[kC];
     #pragma unroll
-                for (int c = 0; c < kC; c += 32) tmem_ld32(tS + 64 * buf + c, reinterpret_cast<uint32_t(&)[32]>(su[c]));
+                for (int c = 0; c < kC; c += 32) tmem_ld32(tS + c, reinterpret_cast<uint32_t(&)[32]>(su[c]));
                 tmem_wait_ld();
     #pragma unroll
                 for (int c = 0; c < kC; c += 32) tmem_ld_fence(reinterpret_cast<uint32_t(&)[32]>(su[c]));
@@ -896,11 +838,6 @@ attn_fwd_tile_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
                     need = true;
                 }
                 if (j > 0 && __any_sync(0xffffffffu, need)) {
-                    if constexpr (L::kDouble) {            // O holds steps 0 .. j - 1 once the other buffer's barrier says so
-                        ok = mbar_wait_warp(bar_s_full + 8u * (buf ^ 1), (uint32_t)(((j + 1) >> 1) & 1), wc, 0x5a);
-                        if (!ok) break;
-                        tc_fence_after_sync();
-                    }
     #pragma unroll 1
                     for (int c0 = 0; c0 < D / kRS; c0 += 16) {
                         uint32_t o[16];
@@ -944,14 +881,14 @@ attn_fwd_tile_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
                             lo[cc / 2 + 1] = pack_bf16x2(p2 - __uint_as_float(h23 << 16), p3 - __uint_as_float(h23 & 0xffff0000u));
                         }
                     }
-                    tmem_st16(tP + 64 * buf + ch * 16, hi);            // P over S (all of S is in registers)
+                    tmem_st16(tP + ch * 16, hi);                       // P over S (all of S is in registers)
                     if constexpr (kSplitP) tmem_st16(tPlo + ch * 16, lo);
                     constexpr int kHalf = kBN / 64;                    // pieces in one half of the step's keys
                     if (ch % kHalf == kHalf - 1) {                     // their contraction may begin
                         tmem_wait_st();
                         tc_fence_before_sync();
                         __syncwarp();
-                        if (lane == 0) mbar_arrive(bar_p_full + 16u * buf + 8u * (half + ch / kHalf));
+                        if (lane == 0) mbar_arrive(bar_p_full + 8u * (half + ch / kHalf));
                     }
                 }
                 const float2 s01 = halves(sum01), s23 = halves(sum23);
@@ -966,8 +903,7 @@ attn_fwd_tile_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
                     ok = ok && meet();
                     if (ok) l_run += *xslot(2, half ^ 1);
                 }
-                if constexpr (L::kDouble) ok = ok && mbar_wait_warp(bar_s_full + 8u * ((n_t - 1) & 1), (uint32_t)(((n_t + 1) >> 1) & 1), wc, 0x57);
-                else ok = ok && mbar_wait_warp(bar_s_full, (uint32_t)((s_full0 + n_t) & 1), wc, 0x57);
+                ok = ok && mbar_wait_warp(bar_s_full, (uint32_t)((s_full0 + n_t) & 1), wc, 0x57);
                 tc_fence_after_sync();
                 float inv = 0.f, lse = neg_inf();
                 if (l_run > 0.f) {

@@ -1,4 +1,4 @@
-"""The head_dim 128 forward with two score buffers: one to six key steps of 64, whole and cut, where single rows (and so single
+"""The head_dim 128 forward with bf16 results: one to three key steps of 128, whole and cut, where single rows (and so single
 warps) rescale at single steps and the others never do.  Against PyTorch in 64 bits."""
 import math
 
@@ -17,7 +17,7 @@ def test_steps_and_rescales(ctx, Sk, masked):
     g = torch.Generator(device="cuda").manual_seed(13)
     rand = lambda n: torch.randn((B, H, n, D), generator=g, device="cuda") * 0.5
     q, k, v = rand(Sq), rand(Sk), rand(Sk)
-    # the last key of every second step is far above the rest for rows 5, 37 and 129 alone
+    # the last key of each step's first half is far above the rest for rows 5, 37 and 129 alone
     q[..., 0], k[..., 0] = 0.0, 0.0
     q[:, :, [5, 37, 129], 0] = 8.0
     peaks = torch.arange(63, max(Sk, 63), 128, device="cuda")
