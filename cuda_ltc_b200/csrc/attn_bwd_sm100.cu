@@ -71,10 +71,12 @@ struct BwdArgs {
     const float* delta;              // [B*H, Sq_pad]
     void *dq, *dk, *dv;
     ltca_strides dqs, dks, dvs;
+    int plain;                       // kPlainDq ...: results whose strides a tensor map does not take
     MaskArgs mask;
     const int32_t* kv_len;
     uint32_t* status;
 };
+constexpr int kPlainDq = 1, kPlainDk = 2, kPlainDv = 4;
 
 __device__ __forceinline__ float neg_inf() { return __int_as_float(0xff800000); }
 __device__ __forceinline__ float pos_inf() { return __int_as_float(0x7f800000); }
@@ -245,6 +247,17 @@ template <typename OutT>
 __device__ __forceinline__ void store_tile(const CUtensorMap* map, uint32_t tile, int row0, int h, int b) {
     tma_store_4d(map, tile, 0, row0, h, b);
     if constexpr (sizeof(OutT) == 4) tma_store_4d(map, tile + kBigTile, 32, row0, h, b);
+}
+// The same from all elementwise threads, for strides of any sign (fp32 results: others are refused those strides).
+__device__ __forceinline__ void copy_tile(void* dst, const ltca_strides& st, const uint8_t* tile, int row0, int rows, int h, int b) {
+    float* base = reinterpret_cast<float*>(dst) + b * st.batch + h * st.head;
+#pragma unroll 1
+    for (int e = threadIdx.x; e < kTile * (kD / 4); e += 256) {
+        const int r = e / (kD / 4), half = e / 8 % 2, v = e % 8;
+        if (row0 + r < rows)
+            *reinterpret_cast<float4*>(base + (row0 + r) * st.seq + 32 * half + 4 * v) =
+                *reinterpret_cast<const float4*>(tile + half * kBigTile + r * 128 + ((v ^ (r & 7)) << 4));
+    }
 }
 // Behind the staging of a tile's result by all elementwise warps: its boxes may be stored.
 __device__ __forceinline__ void tile_staged() {
@@ -508,7 +521,9 @@ __device__ __forceinline__ void dq_tile(const BwdMaps& m, const BwdArgs& a, int 
             stage_half<OutT>(smem_gen, half, row, o, a.scale);             // over Q and dO, which every product has read
         }
         tile_staged();
-        if (warp == 0 && lane == 0 && ok) {
+        if (kSplit && a.plain & kPlainDq) {
+            if (ok) copy_tile(a.dq, a.dqs, smem_gen, q0, a.Sq, h, b);
+        } else if (warp == 0 && lane == 0 && ok) {
             store_tile<OutT>(&m.dq, smem_base, q0, h, b);
             tma_store_commit();
             tma_store_wait_read<0>();
@@ -805,9 +820,13 @@ __device__ __forceinline__ void dkv_tile(const BwdMaps& m, const BwdArgs& a, int
             stage_half<OutT>(smem_gen + L::kRingOff, half, row, o, a.scale);
         }
         tile_staged();
+        if (kSplit && a.plain && ok) {
+            if (a.plain & kPlainDv) copy_tile(a.dv, a.dvs, smem_gen, k0, a.Sk, h, b);
+            if (a.plain & kPlainDk) copy_tile(a.dk, a.dks, smem_gen + L::kRingOff, k0, a.Sk, h, b);
+        }
         if (warp == 0 && lane == 0 && ok) {
-            store_tile<OutT>(&m.dv, smem_base, k0, h, b);
-            store_tile<OutT>(&m.dk, smem_base + L::kRingOff, k0, h, b);
+            if (!(kSplit && a.plain & kPlainDv)) store_tile<OutT>(&m.dv, smem_base, k0, h, b);
+            if (!(kSplit && a.plain & kPlainDk)) store_tile<OutT>(&m.dk, smem_base + L::kRingOff, k0, h, b);
             tma_store_commit();
             tma_store_wait_read<0>();
         }
@@ -2300,6 +2319,12 @@ size_t dq_acc_bytes(const ltca_attn_params* p) {
 // accumulator is part of the workspace in either case.
 bool use_fused(const ltca_attn_params* p) { return p->dtype == LTCA_BF16 && !p->bwd_deterministic; }
 
+// Whether a tensor map takes a result's strides: forward ones.  (make_tmap_bhsd puts a stride of its own in the place of 0.)
+bool tma_strides(const ltca_strides& s, int B, int H) {
+    constexpr int64_t kMost = 1ll << 37;                    // 2^40 bytes is the map's limit
+    return s.seq > 0 && s.seq < kMost && (H == 1 || (s.head > 0 && s.head < kMost)) && (B == 1 || (s.batch > 0 && s.batch < kMost));
+}
+
 // bf16 results: where a CTA per tile, dQ's and dK/dV's in one launch, beats the persistent kernels, whose steps are twice as long but
 // which have one CTA an SM and a launch each.  (Backward, us, persistent and tiles; S the longer of both lengths, tiles those of
 // queries and keys.)
@@ -2316,7 +2341,7 @@ bool bwd_in_tiles(const ltca_ctx* ctx, const ltca_attn_params* p) {
     const int S = p->Sq > p->Sk ? p->Sq : p->Sk;
     const int64_t tiles = (int64_t)p->B * p->H * ((p->Sq + kTile - 1) / kTile + (p->Sk + kTile - 1) / kTile);
     if (p->bwd_deterministic) return S <= 768 || (S <= 2048 && tiles <= 1536);
-    if (p->keep_mask) return false;
+    if (p->keep_mask || !tma_strides(p->dq_strides, p->B, p->H)) return false;     // (the one-kernel form's dQ takes any strides)
     return S <= 128 || (S <= 384 && p->causal) || (S <= 640 && tiles <= 512) || (S <= 1024 && tiles <= 128);
 }
 
@@ -2331,10 +2356,12 @@ int launch_main(ltca_ctx* ctx, const ltca_attn_params* p, const void* mask_words
     if ((rc = make_tmap_bhsd(ctx, &m.k128, k, 2, p->B, p->H, p->Sk, kD, ks, 64, kTile))) return rc;
     if ((rc = make_tmap_bhsd(ctx, &m.v128, v, 2, p->B, p->H, p->Sk, kD, vs, 64, kTile))) return rc;
     constexpr int es = sizeof(OutT), cols = 128 / es;       // of a result's box
-    if (es == 4 || !dq_acc)
+    auto plain = [&](const ltca_strides& st) { return es == 4 && !tma_strides(st, p->B, p->H); };
+    const int plain_results = (plain(p->dq_strides) ? kPlainDq : 0) | (plain(p->dk_strides) ? kPlainDk : 0) | (plain(p->dv_strides) ? kPlainDv : 0);
+    if (!(plain_results & kPlainDq) && (es == 4 || !dq_acc))
         if ((rc = make_tmap_bhsd(ctx, &m.dq, p->dq, es, p->B, p->H, p->Sq, kD, p->dq_strides, cols, kTile))) return rc;
-    if ((rc = make_tmap_bhsd(ctx, &m.dk, p->dk, es, p->B, p->H, p->Sk, kD, p->dk_strides, cols, kTile))) return rc;
-    if ((rc = make_tmap_bhsd(ctx, &m.dv, p->dv, es, p->B, p->H, p->Sk, kD, p->dv_strides, cols, kTile))) return rc;
+    if (!(plain_results & kPlainDk) && (rc = make_tmap_bhsd(ctx, &m.dk, p->dk, es, p->B, p->H, p->Sk, kD, p->dk_strides, cols, kTile))) return rc;
+    if (!(plain_results & kPlainDv) && (rc = make_tmap_bhsd(ctx, &m.dv, p->dv, es, p->B, p->H, p->Sk, kD, p->dv_strides, cols, kTile))) return rc;
 
     BwdArgs a;
     memset(&a, 0, sizeof(a));
@@ -2350,6 +2377,7 @@ int launch_main(ltca_ctx* ctx, const ltca_attn_params* p, const void* mask_words
     a.lse2 = lse2; a.delta = delta;
     a.dq = p->dq; a.dk = p->dk; a.dv = p->dv;
     a.dqs = p->dq_strides; a.dks = p->dk_strides; a.dvs = p->dv_strides;
+    a.plain = plain_results;
     a.mask = mask_args(p, mask_words);
     a.kv_len = p->kv_len;
     a.status = ctx->d_status;
