@@ -1375,37 +1375,53 @@ int dispatch(ltca_ctx* ctx, const CoreArgs& a, bool bwd) {
 
 // delta, and the dense mask as bits (the kernels for head_dim up to 128)
 static size_t delta_bytes(const ltca_attn_params* p) { return align_up((size_t)p->B * p->H * p->Sq * sizeof(float), 256); }
-// dQ's shares in the one-pass backward, one per 64 keys: all pairs' up to kPartBytes, as many pairs' as fit in that beyond it
-// (several launches), none where one pair's take more.  Keys of one block need none.
+// The one-pass backward: how many (batch, head) pairs a launch takes, and the room for their shares of dQ, one per 64 keys (none where
+// there is one block of keys).  kPartBytes and the room there is bound it: beyond them several launches.
 constexpr size_t kPartBytes = 512u << 20;
 struct OnePass {
-    int pairs = 0;       // (batch, head) pairs a launch; 0: not for the one-pass kernel
-    int ld = 0;
+    int pairs = 0, ld = 0;        // 0: the two kernels
     size_t bytes = 0;
 };
-static OnePass one_pass(const ltca_attn_params* p) {
+// Where one pass over the scores is the faster one.  (Backward, us, two kernels and one pass.)
+//   - One key block: always (B2 H4 S64 D32 11.4 and 10.9, B12 H8 S64 D64 22 and 14).
+//   - A CTA walks all queries of its 64 keys: with few CTAs that chain is longer than that of the two kernels' 16-row tiles.  From two
+//     thirds of a CTA per SM on (128 CTAs, B4 H4 S512: D16 67 and 56, D32 103 and 77; 64 CTAs, B2 H4 S512 causal: D16 51 and 53, D32
+//     69 and 73), above head width 32, where a tile has twice the warps, from a third on (64 CTAs, B2 H4 S512 105 and 93; 28 CTAs,
+//     B1 H4 S400 70 and 80).
+//   - Several launches drain one by one, and a causal one lasts as long as the chain of the first keys, twice the mean.  Where a launch
+//     has on average 0.6 of the CTAs that are resident at once; causal 0.6 in two launches, a tenth more for each further one, 0.9 in
+//     the end.  Full, D64 S8192 13 pairs 0.80 of them 20270 and 16750, S10000 0.53 29170 and 39880; D32 S6000 8 pairs 0.64 3920 and
+//     3140, S10000 0.53 9730 and 10320.  Causal, two launches: D32 S6000 0.64 2510 and 2170, S8192 5 pairs 0.54 2740 and 2750; four:
+//     S8192 8 pairs in two of 0.86 4300 and 3340, 13 in four of 0.70 6040 and 6180; seven: D64 S8192 0.80 11200 and 12210; one pair a
+//     launch, D32 S12000 0.32 8240 and 14320.
+static OnePass one_pass(const ltca_attn_params* p, int sms, size_t room) {
     OnePass o;
-    if (p->D > 64) return o;
     const int64_t all = (int64_t)p->B * p->H, blocks = ((int64_t)p->Sk + 63) / 64;
+    if (p->D > 64 || p->B > 65535 || p->H > 65535 || all > 0x7fffffff || blocks > 65535) return o;     // (B, H: as the two kernels' grids)
     o.ld = (p->D + 3) / 4 * 4;
+    if (blocks == 1) {
+        o.pairs = (int)all;
+        return o;
+    }
     const size_t one = (size_t)blocks * p->Sq * o.ld * sizeof(float);
-    if (blocks > 65535 || (blocks > 1 && one > kPartBytes)) return o;
-    const int64_t fit = blocks > 1 ? (int64_t)(kPartBytes / one) : all;
-    o.pairs = (int)(fit < all ? fit : all);
-    o.bytes = blocks > 1 ? o.pairs * one : 0;
+    const int64_t fit = (int64_t)((room < kPartBytes ? room : kPartBytes) / one);
+    if (fit == 0) return o;
+    const int64_t launches = (all + fit - 1) / fit, slots = (p->D > 32 ? 2 : 4) * (int64_t)sms;      // slots: CTAs resident at once
+    // As many pairs a launch as there is room for, or as many in each where that takes less time: waves of CTAs, causal the chain (D32
+    // 8 pairs S6000 7 + 1 3395 us, 4 + 4 3140; D16 S10000 5 + 3 5000, 4 + 4 5480).
+    auto time = [&](int64_t n) { return p->causal ? (n * blocks > 2 * slots ? n * blocks : 2 * slots) : (n * blocks + slots - 1) / slots; };
+    auto total = [&](int64_t n) { return (launches - 1) * time(n) + time(all - (launches - 1) * n); };
+    int64_t pairs = (all + launches - 1) / launches;
+    if (launches > 1 && total(pairs) >= total(fit)) pairs = fit;
+    if (3 * pairs * blocks < (p->D > 32 ? 1 : 2) * (int64_t)sms) return o;
+    const int64_t tenths = p->causal && launches > 2 ? (launches < 5 ? 4 + launches : 9) : 6;
+    if (launches > 1 && 10 * all * blocks < tenths * launches * slots) return o;
+    o.pairs = (int)pairs;
+    o.bytes = pairs * one;
     return o;
 }
-// Where one pass over the scores is the faster one.  A CTA walks all queries of its 64 keys: with few CTAs that chain is longer than
-// that of the two kernels' 16-row tiles.  (Backward, us, two kernels and one pass.)  One key block: always (B2 H4 S64 D32 11.4
-// and 10.9, B12 H8 S64 D64 22 and 14).  Otherwise from two thirds of a CTA per SM on (128 CTAs, B4 H4 S512: D16 67 and 56, D32
-// 103 and 77; 64 CTAs, B2 H4 S512 causal: D16 51 and 53, D32 69 and 73), above head width 32, where a tile has twice the warps, from
-// a third on (64 CTAs, B2 H4 S512 105 and 93; 28 CTAs, B1 H4 S400 70 and 80).
-static bool one_pass_pays(const ltca_ctx* ctx, const ltca_attn_params* p) {
-    const int64_t blocks = ((int64_t)p->Sk + 63) / 64, ctas = (int64_t)p->B * p->H * blocks;
-    return blocks == 1 || 3 * ctas >= (p->D > 32 ? 1 : 2) * (int64_t)ctx->sm_device;
-}
 size_t attn_bwd_fp32_workspace(const ltca_attn_params* p) {
-    return delta_bytes(p) + (p->D <= 128 ? mask_words_bytes(p) + one_pass(p).bytes : 0);
+    return delta_bytes(p) + (p->D <= 128 ? mask_words_bytes(p) + one_pass(p, kPlanSms, kPartBytes).bytes : 0);
 }
 
 int launch_attn_fwd_fp32(ltca_ctx* ctx, const ltca_attn_params* p) {
@@ -1435,8 +1451,8 @@ int launch_attn_bwd_fp32(ltca_ctx* ctx, const ltca_attn_params* p, const FromOut
     if (p->D <= 128) {
         // delta, dQ's shares, the mask's words (not in a workspace sized without the mask); without room for the shares the two
         // kernels run
-        const OnePass one = one_pass(p);
-        const bool once = one.pairs && (!from || p->Sk <= 32) && p->workspace_bytes >= delta_bytes(p) + one.bytes && one_pass_pays(ctx, p);
+        const OnePass one = !from || p->Sk <= 32 ? one_pass(p, ctx->sm_device, p->workspace_bytes - delta_bytes(p)) : OnePass();
+        const bool once = one.pairs > 0;
         if (once) {
             a.pairs = one.pairs;
             a.part_ld = one.ld;
