@@ -1420,8 +1420,8 @@ static OnePass one_pass(const ltca_attn_params* p, int sms, size_t room) {
     o.bytes = pairs * one;
     return o;
 }
-size_t attn_bwd_fp32_workspace(const ltca_attn_params* p) {
-    return delta_bytes(p) + (p->D <= 128 ? mask_words_bytes(p) + one_pass(p, kPlanSms, kPartBytes).bytes : 0);
+size_t attn_bwd_fp32_workspace(const ltca_attn_params* p, bool shares) {
+    return delta_bytes(p) + (p->D <= 128 ? mask_words_bytes(p) + (shares ? one_pass(p, kPlanSms, kPartBytes).bytes : 0) : 0);
 }
 
 int launch_attn_fwd_fp32(ltca_ctx* ctx, const ltca_attn_params* p) {

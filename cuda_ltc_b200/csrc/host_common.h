@@ -214,7 +214,8 @@ constexpr int kFormDoutMaxE = 64, kFormDoutRows = 512;
 bool attn_bwd_exact(const ltca_attn_params* p);       // whether ltca_attn_bwd takes the exact kernels
 bool attn_bwd_fp32_forms_dout(const ltca_ctx* ctx, const ltca_attn_params* p, const FromOutput& f);
 int launch_attn_bwd_fp32(ltca_ctx* ctx, const ltca_attn_params* p, const FromOutput* from = nullptr);
-size_t attn_bwd_fp32_workspace(const ltca_attn_params* p);
+// `shares`: with room for dQ's shares in the one-pass kernel, without which the two kernels run
+size_t attn_bwd_fp32_workspace(const ltca_attn_params* p, bool shares = true);
 int launch_attn_decode(ltca_ctx* ctx, const ltca_attn_params* p);
 size_t attn_decode_workspace(const ltca_attn_params* p);
 

@@ -815,6 +815,8 @@ struct Plan {
     size_t y;            // bytes of one [rows, E] buffer
     size_t attn_fwd, attn_bwd;
 };
+// Whether a call's workspace has the room that ltca_tsa_workspace_bytes asks for, or lacks the exact backward's shares of dQ.
+enum Room { kLeastRoom, kFullRoom };
 
 void fill_attn(const ltca_tsa_params* t, ltca_attn_params* a) {
     memset(a, 0, sizeof(*a));
@@ -838,7 +840,7 @@ void fill_attn(const ltca_tsa_params* t, ltca_attn_params* a) {
     a->bwd_deterministic = 1;
 }
 
-int make_plan(const ltca_tsa_params* t, Plan* pl) {
+int make_plan(const ltca_tsa_params* t, Plan* pl, Room room = kFullRoom) {
     pl->rows = (int64_t)t->B * t->S;
     pl->HW = t->H * t->head_width;
     pl->buf = align_up((size_t)pl->rows * pl->HW * sizeof(float), 256);
@@ -849,6 +851,10 @@ int make_plan(const ltca_tsa_params* t, Plan* pl) {
     // pointers only need to be non-null for the size queries
     int rc = ltca_attn_workspace_bytes(&a, 0, &pl->attn_fwd);
     if (rc) return rc;
+    if (room == kLeastRoom && attn_bwd_exact(&a)) {
+        pl->attn_bwd = attn_bwd_fp32_workspace(&a, false);
+        return LTCA_OK;
+    }
     return ltca_attn_workspace_bytes(&a, 1, &pl->attn_bwd);
 }
 
@@ -1155,12 +1161,21 @@ void fill_composed(const ltca_tsa_params* t, const TPlan& pl, const TBufs& tb, W
 // The attention scratch (TBufs::rest) of a call whose buffers start at w; not on the written-out-score path.
 char* scratch_of(const ltca_tsa_params* t, const TPlan& pl, char* w) { return t->saved ? w : w + tensor_saved_bytes(pl); }
 
-// The call as its workspace is laid out.  Packed mask words are part of what ltca_tsa_workspace_bytes asks for, but a
-// workspace that was sized without the mask is laid out without them: the attention kernels then read the dense values.
-ltca_tsa_params laid_out(const ltca_tsa_params* t, int which) {
+int workspace_bytes(const ltca_tsa_params* t, int which, Room room, size_t* bytes_out);
+// The call as its workspace is laid out.  Packed mask words and the exact backward's shares of dQ are part of what
+// ltca_tsa_workspace_bytes asks for, but a workspace that was sized without the mask is laid out without the words (the attention
+// kernels then read the dense values), and one that has no room for the shares without those.
+ltca_tsa_params laid_out(const ltca_tsa_params* t, int which, Room* room = nullptr) {
     ltca_tsa_params l = *t;
-    size_t need = 0;
-    if (l.keep_mask && (ltca_tsa_workspace_bytes(&l, which, &need) || l.workspace_bytes < need)) l.keep_mask = nullptr;
+    if (!room && !t->keep_mask) return l;
+    for (Room r : {kFullRoom, kLeastRoom}) {
+        if (room) *room = r;
+        for (const float* mask : {t->keep_mask, (const float*)nullptr}) {
+            size_t need = 0;
+            l.keep_mask = mask;
+            if (!workspace_bytes(&l, which, r, &need) && l.workspace_bytes >= need) return l;
+        }
+    }
     return l;
 }
 
@@ -1808,21 +1823,14 @@ int tensor_backward(ltca_ctx* ctx, const ltca_tsa_params* t, bool want_dx, bool 
     return LTCA_OK;
 }
 
-}  // namespace
-}  // namespace ltca
-
-using namespace ltca;
-
-extern "C" {
-
 // Workspace of the TimeSelfAttention form (no input LayerNorm, no dropout), without the column-sum scratch.
-static int inner_workspace(const ltca_tsa_params* t, int which, size_t* bytes_out) {
+int inner_workspace(const ltca_tsa_params* t, int which, Room room, size_t* bytes_out) {
     if (use_tensor(t, which != 0 || keeps_for_backward(t))) {
         return planned_bytes(t, which != 0 || keeps_for_backward(t), [&](const TPlan& tp) { return tensor_workspace(tp, which); },
                              bytes_out);
     }
     Plan pl;
-    int rc = make_plan(t, &pl);
+    int rc = make_plan(t, &pl, room);
     if (rc) return rc;
     size_t n = 4 * pl.buf + pl.lse;                       // q, k, v, ctx, lse
     if (which == 0) {
@@ -1837,7 +1845,7 @@ static int inner_workspace(const ltca_tsa_params* t, int which, size_t* bytes_ou
 }
 
 // The module without the FlashAttention-form steps: what the pre_norm wrappers run in the middle.
-static ltca_tsa_params core_form(const ltca_tsa_params* t) {
+ltca_tsa_params core_form(const ltca_tsa_params* t) {
     ltca_tsa_params c = *t;
     c.pre_norm = 0;
     c.use_residual = 0;
@@ -1847,9 +1855,31 @@ static ltca_tsa_params core_form(const ltca_tsa_params* t) {
     c.dbeta = nullptr;
     return c;
 }
-static size_t act_bytes(const ltca_tsa_params* t) {
+size_t act_bytes(const ltca_tsa_params* t) {
     return align_up((size_t)t->B * t->S * t->E * sizeof(float), 256);
 }
+
+int workspace_bytes(const ltca_tsa_params* t, int which, Room room, size_t* bytes_out) {
+    size_t n = 0;
+    int rc;
+    if (t->pre_norm) {
+        const ltca_tsa_params c = core_form(t);
+        if ((rc = inner_workspace(&c, which, room, &n))) return rc;
+        n += (which == 0 ? 1 : 3) * act_bytes(t);         // LayerNorm(x); backward: + masked dy, gradient at LayerNorm(x)
+    } else if ((rc = inner_workspace(t, which, room, &n))) {
+        return rc;
+    }
+    if (which != 0) n += colsum_scratch_bytes(t);
+    *bytes_out = n;
+    return LTCA_OK;
+}
+
+}  // namespace
+}  // namespace ltca
+
+using namespace ltca;
+
+extern "C" {
 
 int ltca_tsa_saved_bytes(const ltca_tsa_params* t, size_t* bytes_out) {
     if (!t || !bytes_out) return LTCA_ERR_INVALID;
@@ -1880,18 +1910,7 @@ int ltca_tsa_weight_cache_bytes(const ltca_tsa_params* t, size_t* bytes_out) {
 
 int ltca_tsa_workspace_bytes(const ltca_tsa_params* t, int which, size_t* bytes_out) {
     if (!t || !bytes_out || which < 0 || which > 3) return LTCA_ERR_INVALID;
-    size_t n = 0;
-    int rc;
-    if (t->pre_norm) {
-        const ltca_tsa_params c = core_form(t);
-        if ((rc = inner_workspace(&c, which, &n))) return rc;
-        n += (which == 0 ? 1 : 3) * act_bytes(t);         // LayerNorm(x); backward: + masked dy, gradient at LayerNorm(x)
-    } else if ((rc = inner_workspace(t, which, &n))) {
-        return rc;
-    }
-    if (which != 0) n += colsum_scratch_bytes(t);
-    *bytes_out = n;
-    return LTCA_OK;
+    return workspace_bytes(t, which, kFullRoom, bytes_out);
 }
 
 static int tsa_forward(ltca_ctx* ctx, const ltca_tsa_params* t, const ltca_tsa_params* outer, bool fused);
@@ -1931,8 +1950,9 @@ static int prenorm_forward(ltca_ctx* ctx, const ltca_tsa_params* t) {
 // FlashAttention form, backward (an extension: the reference class has no backward pass).
 static int prenorm_backward(ltca_ctx* ctx, const ltca_tsa_params* t, bool want_dx, bool want_dw) {
     size_t need = 0;
-    const ltca_tsa_params layout = laid_out(t, 1);
-    int rc = ltca_tsa_workspace_bytes(&layout, 1, &need);
+    Room room;
+    const ltca_tsa_params layout = laid_out(t, 1, &room);
+    int rc = workspace_bytes(&layout, 1, room, &need);
     if (rc) return rc;
     if (!t->workspace || t->workspace_bytes < need)
         return fail(ctx, LTCA_ERR_WORKSPACE, "backward needs %zu bytes of workspace", need);
@@ -2053,8 +2073,9 @@ static int tsa_backward(ltca_ctx* ctx, const ltca_tsa_params* t, bool want_dx, b
         return fail(ctx, LTCA_ERR_INVALID, "dropout_prob must be in [0, 1)");
     if (t->pre_norm) return prenorm_backward(ctx, t, want_dx, want_dw);
     size_t need = 0;
-    const ltca_tsa_params layout = laid_out(t, 1);
-    ltca_tsa_workspace_bytes(&layout, 1, &need);
+    Room room;
+    const ltca_tsa_params layout = laid_out(t, 1, &room);
+    workspace_bytes(&layout, 1, room, &need);
     if (!t->workspace || t->workspace_bytes < need)
         return fail(ctx, LTCA_ERR_WORKSPACE, "backward needs %zu bytes of workspace", need);
     float* colsum_scratch =
@@ -2067,7 +2088,7 @@ static int tsa_backward(ltca_ctx* ctx, const ltca_tsa_params* t, bool want_dx, b
         return column_sums(ctx, own, (int64_t)t->B * t->S, colsum_scratch);
     }
     Plan pl;
-    if ((rc = make_plan(&layout, &pl))) return rc;
+    if ((rc = make_plan(&layout, &pl, room))) return rc;
     char* w = reinterpret_cast<char*>(t->workspace);
     float* dctx = reinterpret_cast<float*>(w); w += pl.buf;
     float* dq = reinterpret_cast<float*>(w);   w += pl.buf;

@@ -168,8 +168,12 @@ int ltca_ctx_set_sm_limit(ltca_ctx* ctx, int32_t n_sms);
 /* ---- attention core --------------------------------------------------------------------- */
 
 /* Scratch needed by ltca_attn_fwd (backward = 0) or ltca_attn_bwd (backward = 1).  With keep_mask set the answer holds
- * room for the mask packed into bits; a call whose workspace was sized without the mask runs too, on the mask as it is
- * (the same for the module's entry points below). */
+ * room for the mask packed into bits; a call whose workspace was sized without the mask runs too, on the mask as it is.
+ * For the exact backward (LTCA_MODE_FP32, and LTCA_MODE_AUTO where that is what it means) of head widths up to 64 and more
+ * than 64 keys the answer holds up to 512 MB for the key blocks' shares of dQ, where the kernel that needs them is the faster
+ * one.  A call with less room runs too, down to B H Sq floats: in several launches with the same bits, or on two kernels
+ * whose sums have another order.  (Both hold for the module's entry points below, which take the two kernels where there is
+ * not all of that room.) */
 int ltca_attn_workspace_bytes(const ltca_attn_params* p, int backward, size_t* bytes_out);
 
 /* 1 if the tensor-pipe (tcgen05) kernels cover this problem, 0 if it runs on the fp32 path. */

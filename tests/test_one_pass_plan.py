@@ -85,3 +85,55 @@ def test_less_room_takes_more_launches(ctx, causal, masked):
     for a, b in zip(run(delta + one), want):
         assert float((a.double() - b.double()).norm()) <= 1e-5 * float(b.double().norm())
     assert ctx.device_status() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("pre_norm", [0, 1])
+@pytest.mark.parametrize("masked", [False, True])
+def test_module_without_room_for_the_shares(ctx, pre_norm, masked):
+    B, S, H, W = 20, 130, 8, 16
+    E = H * W
+    g = torch.Generator(device="cuda").manual_seed(16)
+    rand = lambda *s: torch.randn(s, generator=g, device="cuda")
+    x, dy, gamma, beta = rand(B * S, E), rand(B * S, E), 1.0 + 0.1 * rand(E), 0.1 * rand(E)
+    w = [rand(E, E) / math.sqrt(E) for _ in range(4)]
+    m = (torch.rand((B, S, S), generator=g, device="cuda") > 0.3).float() if masked else None
+    if m is not None:
+        m.diagonal(dim1=1, dim2=2).fill_(1.0)
+    names = ["dx", "dwq", "dwk", "dwv", "dwo", *(["dbq", "dbk", "dbv", "dbo", "dgamma", "dbeta"] if pre_norm else [])]
+    p = _lib.TsaParams()
+    p.B, p.S, p.E, p.H, p.head_width, p.scale, p.mode = B, S, E, H, W, W ** -0.5, _lib.MODE_FP32
+    p.use_residual = p.use_layer_norm = 1
+    p.pre_norm = pre_norm
+    p.x, p.dy, p.ln_gamma, p.ln_beta = (t.data_ptr() for t in (x, dy, gamma, beta))
+    for name, t in zip(("wq", "wk", "wv", "wo"), w):
+        setattr(p, name, t.data_ptr())
+    p.keep_mask = m.data_ptr() if masked else None
+    need = C.c_size_t(0)
+    ctx.check(ctx.lib.ltca_tsa_workspace_bytes(C.byref(p), 3, C.byref(need)))
+    shares = B * H * _one(S, S, W)
+    words = (S + 31) // 32 * S * B * 4
+
+    def run(nbytes):
+        ws = torch.full((max(nbytes, 256) + 4096,), 0x55, dtype=torch.uint8, device="cuda")
+        p.workspace, p.workspace_bytes = ws.data_ptr(), nbytes
+        got = {n: torch.full_like(t, math.nan) for n, t in zip(names, [x, *w, *([gamma] * 6)])}
+        for n, t in got.items():
+            setattr(p, n, t.data_ptr())
+        rc = ctx.lib.ltca_tsa_bwd(ctx.handle, C.byref(p))
+        assert bool((ws[nbytes:] == 0x55).all())          # nothing beyond what was given
+        return rc, got
+
+    rc, want = run(need.value)
+    assert rc == 0
+    for room in (need.value - 256, need.value - shares):
+        rc, got = run(room)
+        assert rc == 0, ctx.lib.ltca_last_error(ctx.handle)
+        for n in names:
+            # sums of fp32 terms in another order, three products in a row; dbk's terms, as large as those of dk, sum up to 0 (a shift of
+            # all keys moves no softmax): 2^-24 sqrt(rows) of the rows' norm
+            scale = max(float(want[o].double().norm()) for o in (("dbk", "dbv") if n == "dbk" else (n,)))
+            assert float((got[n].double() - want[n].double()).norm()) <= 2e-5 * scale, n
+    rc, _ = run(need.value - shares - (2 * words if masked else 0) - 256)
+    assert rc == -4                                       # LTCA_ERR_WORKSPACE
+    assert ctx.device_status() == 0
