@@ -2325,6 +2325,25 @@ bool tma_strides(const ltca_strides& s, int B, int H) {
     return s.seq > 0 && s.seq < kMost && (H == 1 || (s.head > 0 && s.head < kMost)) && (B == 1 || (s.batch > 0 && s.batch < kMost));
 }
 
+// Whether a result lies over an operand (gradients in place).  The tiles of dQ and those of dK and dV run side by side and read all
+// four operands, so neither may write over one; in the persistent kernels dK and dV may take the places of K and V, and in the
+// one-kernel form, whose dQ is written by the launch behind it, dQ that of Q or dO.
+bool in_place(const ltca_attn_params* p) {
+    const int es = elem_size(p->dtype);
+    struct Range { const char *begin, *end; };
+    auto range = [&](const void* t, const ltca_strides& st, int S) {
+        int64_t lo = 0, hi = kD;
+        for (int64_t last : {(p->B - 1) * st.batch, (p->H - 1) * st.head, (S - 1) * st.seq}) (last < 0 ? lo : hi) += last;
+        return Range{reinterpret_cast<const char*>(t) + lo * es, reinterpret_cast<const char*>(t) + hi * es};
+    };
+    const Range in[] = {range(p->q, p->q_strides, p->Sq), range(p->k, p->k_strides, p->Sk), range(p->v, p->v_strides, p->Sk),
+                        range(p->dout, p->do_strides, p->Sq)};
+    for (const Range& r : {range(p->dq, p->dq_strides, p->Sq), range(p->dk, p->dk_strides, p->Sk), range(p->dv, p->dv_strides, p->Sk)})
+        for (const Range& i : in)
+            if (r.begin < i.end && i.begin < r.end) return true;
+    return false;
+}
+
 // bf16 results: where a CTA per tile, dQ's and dK/dV's in one launch, beats the persistent kernels, whose steps are twice as long but
 // which have one CTA an SM and a launch each.  (Backward, us, persistent and tiles; S the longer of both lengths, tiles those of
 // queries and keys.)
@@ -2337,7 +2356,7 @@ bool tma_strides(const ltca_strides& s, int B, int H) {
 //     mask (B8 H8 S500 47 and 53).
 // A limit on the context's SMs keeps to the persistent kernels, which obey it.
 bool bwd_in_tiles(const ltca_ctx* ctx, const ltca_attn_params* p) {
-    if (ctx->sm_count < ctx->sm_device) return false;
+    if (ctx->sm_count < ctx->sm_device || in_place(p)) return false;
     const int S = p->Sq > p->Sk ? p->Sq : p->Sk;
     const int64_t tiles = (int64_t)p->B * p->H * ((p->Sq + kTile - 1) / kTile + (p->Sk + kTile - 1) / kTile);
     if (p->bwd_deterministic) return S <= 768 || (S <= 2048 && tiles <= 1536);
