@@ -285,7 +285,7 @@ __device__ __forceinline__ void pack32(const uint32_t (&v)[32], uint32_t (&hi)[1
 // ---------------------------------------------------------------------------------------------
 // dS is written as two bf16 terms and the dQ contraction runs once per term, so that the 2^-9 rounding of a single bf16 dS does
 // not dominate the error of an fp32 result.
-template <typename OutT, bool kMask, typename Wait>
+template <typename OutT, bool kMask, bool kPlain, typename Wait>
 __device__ __forceinline__ void dq_tile(const BwdMaps& m, const BwdArgs& a, int q0, int h, int b, const Wait& wait) {
     using L = DqSmem;
     constexpr bool kSplit = sizeof(OutT) == 4;
@@ -521,7 +521,7 @@ __device__ __forceinline__ void dq_tile(const BwdMaps& m, const BwdArgs& a, int 
             stage_half<OutT>(smem_gen, half, row, o, a.scale);             // over Q and dO, which every product has read
         }
         tile_staged();
-        if (kSplit && a.plain & kPlainDq) {
+        if (kPlain && a.plain & kPlainDq) {
             if (ok) copy_tile(a.dq, a.dqs, smem_gen, q0, a.Sq, h, b);
         } else if (warp == 0 && lane == 0 && ok) {
             store_tile<OutT>(&m.dq, smem_base, q0, h, b);
@@ -548,7 +548,7 @@ __device__ __forceinline__ void dq_tile(const BwdMaps& m, const BwdArgs& a, int 
 // (bf16 pairs in the first 16, their low-order term in the next 16), so neither thread
 // ever overwrites scores the other has not read yet.
 // ---------------------------------------------------------------------------------------------
-template <typename OutT, bool kMask, typename Wait>
+template <typename OutT, bool kMask, bool kPlain, typename Wait>
 __device__ __forceinline__ void dkv_tile(const BwdMaps& m, const BwdArgs& a, int k0, int h, int b, const Wait& wait) {
     using L = DkvSmem;
     constexpr bool kSplit = sizeof(OutT) == 4;
@@ -820,13 +820,13 @@ __device__ __forceinline__ void dkv_tile(const BwdMaps& m, const BwdArgs& a, int
             stage_half<OutT>(smem_gen + L::kRingOff, half, row, o, a.scale);
         }
         tile_staged();
-        if (kSplit && a.plain && ok) {
+        if (kPlain && ok) {
             if (a.plain & kPlainDv) copy_tile(a.dv, a.dvs, smem_gen, k0, a.Sk, h, b);
             if (a.plain & kPlainDk) copy_tile(a.dk, a.dks, smem_gen + L::kRingOff, k0, a.Sk, h, b);
         }
         if (warp == 0 && lane == 0 && ok) {
-            if (!(kSplit && a.plain & kPlainDv)) store_tile<OutT>(&m.dv, smem_base, k0, h, b);
-            if (!(kSplit && a.plain & kPlainDk)) store_tile<OutT>(&m.dk, smem_base + L::kRingOff, k0, h, b);
+            if (!(kPlain && a.plain & kPlainDv)) store_tile<OutT>(&m.dv, smem_base, k0, h, b);
+            if (!(kPlain && a.plain & kPlainDk)) store_tile<OutT>(&m.dk, smem_base + L::kRingOff, k0, h, b);
             tma_store_commit();
             tma_store_wait_read<0>();
         }
@@ -842,8 +842,9 @@ __device__ __forceinline__ void dkv_tile(const BwdMaps& m, const BwdArgs& a, int
     }
 }
 
-// dK/dV's tiles and dQ's in one launch, dK/dV's (the longer ones) first, each heaviest first.
-template <typename OutT, bool kMask>
+// dK/dV's tiles and dQ's in one launch, dK/dV's (the longer ones) first, each heaviest first.  kPlain: with results of BwdArgs::plain
+// (as a branch of the one kernel the step B32 H8 S256 took 81.1 us and not 80.9).
+template <typename OutT, bool kMask, bool kPlain>
 __global__ void __launch_bounds__(kTileThreads, 2)
 attn_bwd_dkv_sm100_kernel(const __grid_constant__ BwdMaps m, const __grid_constant__ BwdArgs a, const __grid_constant__ ItemGrid keys,
                           const __grid_constant__ ItemGrid queries) {
@@ -852,10 +853,10 @@ attn_bwd_dkv_sm100_kernel(const __grid_constant__ BwdMaps m, const __grid_consta
     const int item = (int)blockIdx.x - keys.n_items;
     if (item < 0) {
         sched_item(keys, blockIdx.x, rank, h, b);
-        dkv_tile<OutT, kMask>(m, a, rank * kTile, h, b, wait);                         // early keys are seen by the most queries
+        dkv_tile<OutT, kMask, kPlain>(m, a, rank * kTile, h, b, wait);                       // early keys are seen by the most queries
     } else {
         sched_item(queries, item, rank, h, b);
-        dq_tile<OutT, kMask>(m, a, (queries.nblk - 1 - rank) * kTile, h, b, wait);     // late queries see the most keys
+        dq_tile<OutT, kMask, kPlain>(m, a, (queries.nblk - 1 - rank) * kTile, h, b, wait);   // late queries see the most keys
     }
 }
 
@@ -2435,11 +2436,11 @@ int launch_main(ltca_ctx* ctx, const ltca_attn_params* p, const void* mask_words
         if ((rc = make_tmap_bhsd(ctx, &m.do64, dout, 2, p->B, p->H, p->Sq, kD, dos, 64, kStep))) return rc;
         if ((rc = make_tmap_bhsd(ctx, &m.k64, k, 2, p->B, p->H, p->Sk, kD, ks, 64, kStep))) return rc;
         if ((rc = make_tmap_bhsd(ctx, &m.v64, v, 2, p->B, p->H, p->Sk, kD, vs, 64, kStep))) return rc;
-        static SmemOptIn opt_tiles;               // one per template instantiation
+        static SmemOptIn opt_tiles, opt_plain;    // one per template instantiation
         constexpr int smem = DqSmem::kDynBytes > DkvSmem::kDynBytes ? DqSmem::kDynBytes : DkvSmem::kDynBytes;
         static_assert(2 * (smem + 1024) <= 228 * 1024, "two to an SM");
-        auto kern = attn_bwd_dkv_sm100_kernel<OutT, kMask>;
-        LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(opt_tiles, ctx->device, kern, smem));
+        auto kern = plain_results ? attn_bwd_dkv_sm100_kernel<OutT, kMask, es == 4> : attn_bwd_dkv_sm100_kernel<OutT, kMask, false>;
+        LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(plain_results ? opt_plain : opt_tiles, ctx->device, kern, smem));
         ItemGrid keys, queries;
         keys.group = queries.group = kSchedGroup;
         keys.H = queries.H = p->H;
