@@ -75,7 +75,8 @@ class Context:
         self.check(self.lib.ltca_ctx_enable_kernel_timing(self.handle, int(enable)))
 
     def last_bwd_kernel_ms(self):
-        """(statistics, dQ kernel, dK/dV kernel) durations in ms of the last timed backward."""
+        """Durations in ms of the last timed backward: (statistics, dQ kernel, dK/dV kernel); (statistics, fused kernel, dQ's
+        conversion) for the fused form; (statistics, tiles of dQ, dK and dV, 0) where one launch forms all three."""
         ms = (C.c_float * 3)()
         self.check(self.lib.ltca_ctx_last_bwd_kernel_ms(self.handle, ms))
         return tuple(float(x) for x in ms)

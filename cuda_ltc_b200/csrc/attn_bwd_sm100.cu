@@ -2455,6 +2455,7 @@ int launch_main(ltca_ctx* ctx, const ltca_attn_params* p, const void* mask_words
         LTCA_LAUNCH_OK(ctx, "attn_bwd_dkv_sm100_kernel");
         kernel_timing_mark(ctx, 2);
         kernel_timing_mark(ctx, 3);
+        ctx->kev_one_launch = true;
         return LTCA_OK;
     }
     if constexpr (sizeof(OutT) == 2) {
@@ -2545,6 +2546,7 @@ int launch_attn_bwd_sm100(ltca_ctx* ctx, const ltca_attn_params* p) {
     s.dout_bf16 = reinterpret_cast<uint4*>(gb);
     s.stat_blocks = (unsigned)((int64_t)p->B * p->H * (s.Sq_pad / kStatsRows));
     kernel_timing_mark(ctx, 0);
+    ctx->kev_one_launch = false;
     if (p->dtype == LTCA_BF16) {
         LTCA_CUDA_OK(ctx, launch_dependent_if(small_attention_call(p), attn_bwd_stats_kernel<__nv_bfloat16>, dim3(s.stat_blocks), dim3(8 * kStatsRows), 0, ctx->stream, s));
         LTCA_LAUNCH_OK(ctx, "attn_bwd_stats_kernel");

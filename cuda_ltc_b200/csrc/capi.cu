@@ -473,6 +473,7 @@ int ltca_ctx_last_bwd_kernel_ms(ltca_ctx* ctx, float* ms_out) {
         return fail(ctx, LTCA_ERR_INVALID, "no timed tensor-pipe backward has run on this context");
     LTCA_CUDA_OK(ctx, cudaEventSynchronize(ctx->kev[3]));
     for (int i = 0; i < 3; ++i) LTCA_CUDA_OK(ctx, cudaEventElapsedTime(&ms_out[i], ctx->kev[i], ctx->kev[i + 1]));
+    if (ctx->kev_one_launch) ms_out[2] = 0.f;            // (the time between the two last events)
     return LTCA_OK;
 }
 

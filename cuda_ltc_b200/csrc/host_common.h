@@ -48,6 +48,7 @@ struct ltca_ctx {
     bool time_kernels = false;
     cudaEvent_t kev[4] = {nullptr, nullptr, nullptr, nullptr};
     int kev_recorded = 0;
+    bool kev_one_launch = false;      // the last timed backward's dQ, dK and dV came from one launch
 };
 
 namespace ltca {
