@@ -332,7 +332,7 @@ __device__ __forceinline__ void dq_tile(const BwdMaps& m, const BwdArgs& a, int 
     wait();                    // the operands are complete once the kernel before this one has ended
     auto slot_of = [&](int item) { return item % L::kStages; };
     auto phase_of = [&](int item) { return (uint32_t)((item / L::kStages) & 1); };
-    LTCA_TRACE_DECL(LTCA_TRACE_KERNEL == 1 && blockIdx.x == 0 && blockIdx.y == 5 && blockIdx.z == 0);
+    LTCA_TRACE_DECL(LTCA_TRACE_KERNEL == 1 && q0 + kTile >= a.Sq && h == 5 && b == 0);
     LTCA_TRACE_EVT(0x01);
 
     if (warp >= kTileMmaWarp) {
@@ -594,7 +594,7 @@ __device__ __forceinline__ void dkv_tile(const BwdMaps& m, const BwdArgs& a, int
     // ring items are numbered from the first streamed step of this CTA
     auto slot_of = [&](int j) { return (j - j_first) % L::kStages; };
     auto phase_of = [&](int j) { return (uint32_t)(((j - j_first) / L::kStages) & 1); };
-    LTCA_TRACE_DECL(LTCA_TRACE_KERNEL == 2 && blockIdx.x == 0 && blockIdx.y == 5 && blockIdx.z == 0);
+    LTCA_TRACE_DECL(LTCA_TRACE_KERNEL == 2 && k0 == 0 && h == 5 && b == 0);
     LTCA_TRACE_EVT(0x01);
 
     if (warp >= kTileMmaWarp) {
@@ -2459,38 +2459,30 @@ int launch_main(ltca_ctx* ctx, const ltca_attn_params* p, const void* mask_words
         return LTCA_OK;
     }
     if constexpr (sizeof(OutT) == 2) {
-        {
-            static SmemOptIn opt_dq4;
-            LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(opt_dq4, ctx->device, attn_bwd_dq4_sm100_kernel<kMask>, Dq4Smem::kDynBytes));
+        // item counters: ints 2,3 the dQ kernel's, 4,5 the dK/dV kernel's
+        auto items = [&](int S, int counter) {
             ItemGrid ig;
             ig.group = kSchedGroup;
-            ig.nblk = (p->Sq + kTile - 1) / kTile;
+            ig.nblk = (S + kTile - 1) / kTile;
             ig.H = p->H;
             ig.BH = p->H * p->B;
             ig.n_items = ig.nblk * ig.BH;
-            ig.counters = ctx->d_sched + 2;             // ints 2,3: the dQ kernel's item counters
-            const int n_cta = ig.n_items < ctx->sm_count ? ig.n_items : ctx->sm_count;
-            LTCA_CUDA_OK(ctx, launch_dependent_if(small_attention_call(p), attn_bwd_dq4_sm100_kernel<kMask>, dim3(n_cta), dim3(kThreads), Dq4Smem::kDynBytes,
-                                               ctx->stream, m.q128, m.do128, m.k128, m.v128, m.dq, a, ig));
-            LTCA_LAUNCH_OK(ctx, "attn_bwd_dq4_sm100_kernel");
-        }
+            ig.counters = ctx->d_sched + counter;
+            return ig;
+        };
+        auto ctas = [&](const ItemGrid& ig) { return dim3(ig.n_items < ctx->sm_count ? ig.n_items : ctx->sm_count); };
+        static SmemOptIn opt_dq4, opt_dkv4;
+        LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(opt_dq4, ctx->device, attn_bwd_dq4_sm100_kernel<kMask>, Dq4Smem::kDynBytes));
+        const ItemGrid queries = items(p->Sq, 2), keys = items(p->Sk, 4);
+        const dim3 gq = ctas(queries), gk = ctas(keys);
+        LTCA_CUDA_OK(ctx, launch_dependent_if(small_attention_call(p), attn_bwd_dq4_sm100_kernel<kMask>, gq, dim3(kThreads), Dq4Smem::kDynBytes,
+                                           ctx->stream, m.q128, m.do128, m.k128, m.v128, m.dq, a, queries));
+        LTCA_LAUNCH_OK(ctx, "attn_bwd_dq4_sm100_kernel");
         kernel_timing_mark(ctx, 2);
-        {
-            static SmemOptIn opt_dkv4;
-            LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(opt_dkv4, ctx->device, attn_bwd_dkv4_sm100_kernel<kMask>,
-                                                  Dkv4Smem::kDynBytes));
-            ItemGrid ig;
-            ig.group = kSchedGroup;
-            ig.nblk = (p->Sk + kTile - 1) / kTile;
-            ig.H = p->H;
-            ig.BH = p->H * p->B;
-            ig.n_items = ig.nblk * ig.BH;
-            ig.counters = ctx->d_sched + 4;             // ints 4,5: the dK/dV kernel's item counters
-            const int n_cta = ig.n_items < ctx->sm_count ? ig.n_items : ctx->sm_count;
-            LTCA_CUDA_OK(ctx, launch_dependent_if(small_attention_call(p), attn_bwd_dkv4_sm100_kernel<kMask>, dim3(n_cta), dim3(kThreads), Dkv4Smem::kDynBytes,
-                                               ctx->stream, m.q128, m.do128, m.k128, m.v128, m.dk, m.dv, a, ig));
-            LTCA_LAUNCH_OK(ctx, "attn_bwd_dkv4_sm100_kernel");
-        }
+        LTCA_CUDA_OK(ctx, opt_in_dynamic_smem(opt_dkv4, ctx->device, attn_bwd_dkv4_sm100_kernel<kMask>, Dkv4Smem::kDynBytes));
+        LTCA_CUDA_OK(ctx, launch_dependent_if(small_attention_call(p), attn_bwd_dkv4_sm100_kernel<kMask>, gk, dim3(kThreads), Dkv4Smem::kDynBytes,
+                                           ctx->stream, m.q128, m.do128, m.k128, m.v128, m.dk, m.dv, a, keys));
+        LTCA_LAUNCH_OK(ctx, "attn_bwd_dkv4_sm100_kernel");
     }
     kernel_timing_mark(ctx, 3);
     return LTCA_OK;

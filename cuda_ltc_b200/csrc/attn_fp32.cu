@@ -1,6 +1,6 @@
 // fp32 attention: the exact arithmetic mode (fp32 FMA, accurate expf) and the path for every
 // shape the tensor-pipe kernels do not take (any head_dim up to 512, dense keep-masks, tiny
-// sequences).  Forward and backward (two passes, no atomics, bit-reproducible).
+// sequences).  Forward and backward (one pass over the scores or two, no atomics, bit-reproducible).
 //
 // Replaces flashAttentionKernel (reference src/ml/flash_attention.cu:18-272) on its own valid
 // domain (head_dim <= 16, one key tile) and extends it to a true online softmax for longer
@@ -1108,8 +1108,8 @@ int run_dkv(ltca_ctx* ctx, const CoreArgs& a) {
 // (None of these kernels lets the next one's CTAs be placed before it ends: released at the start, or when the tile loop is
 // done, they take whatever slots are left and sit unevenly on the SMs, 82 or 62 us instead of 57 for B16 H8 S100 D32.)
 // Tiles of 64 rows reuse what they load most; where they would leave SMs idle, tiles of 16 rows give four times the CTAs
-// and a quarter of the serial work.  The two-kernel backward's 64-row tiles are left for heads above 64 and for calls whose
-// workspace has no room for dQ's shares.
+// and a quarter of the serial work.  The two-kernel backward is left for heads above 64 and where one_pass says so: few CTAs of 64
+// keys (16-row tiles, of dQ 64-row ones where many queries meet few keys) and calls without room for dQ's shares (64-row tiles).
 template <typename T, int DP, int kMask>
 int run_small_dq(ltca_ctx* ctx, const CoreArgs& a) {
     if constexpr (sizeof(T) == 4 && DP <= 64) {

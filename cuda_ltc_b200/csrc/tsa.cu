@@ -568,11 +568,6 @@ __global__ void __launch_bounds__(128) column_sum_final_kernel(const __grid_cons
     if (c < a.cols[j]) column_final(a, j, c);
 }
 int column_sums(ltca_ctx* ctx, ColSum a, int64_t rows, float* scratch) {
-    if (a.split_n) {
-        void* dst[kMaxGemmProblems];
-        for (int i = 0; i < a.split_n; ++i) dst[i] = a.split_dst[i];
-        if (int rc = sum_splits(ctx, a.split, dst, a.split_n, a.split_mn, a.splits)) return rc;
-    }
     if (a.n == 0) return LTCA_OK;
     a.rows = rows;
     a.partial = scratch;
@@ -1430,8 +1425,10 @@ int composed_backward(ltca_ctx* ctx, const ltca_tsa_params* t, const TPlan& pl, 
         if (gemm_group_aligned(gg)) {
             if ((rc = gemm_sm100_group(ctx, gg))) return rc;
         } else {
-            for (const GemmGroup::Member& m : gg.m)
-                if (&m < gg.m + gg.n && (rc = per_head(ctx, t, E, m.terms, m.a, m.a_hs, m.b, m.b_hs, m.c, m.ldc, m.c_hs, 0))) return rc;
+            for (int i = 0; i < gg.n; ++i) {
+                const GemmGroup::Member& m = gg.m[i];
+                if ((rc = per_head(ctx, t, E, m.terms, m.a, m.a_hs, m.b, m.b_hs, m.c, m.ldc, m.c_hs, 0))) return rc;
+            }
         }
     }
     if (t->dbq || t->dbk || t->dbv) {
@@ -1677,7 +1674,7 @@ int projected_backward(ltca_ctx* ctx, const ltca_tsa_params* t, const ltca_tsa_p
         GemmGroup gg;
         gg.n = 5;
         const void* wsrc[3] = {tb.wq, tb.wk, tb.wv};
-        float* dst[4] = {t->dwq, t->dwk, t->dwv, t->dwo};
+        void* dst[4] = {t->dwq, t->dwk, t->dwv, t->dwo};
         GemmGroup::Member& x = gg.m[4];
         x.M = rows; x.N = E; x.K = HW;
         x.terms = 3;
@@ -1700,11 +1697,11 @@ int projected_backward(ltca_ctx* ctx, const ltca_tsa_params* t, const ltca_tsa_p
             if ((rc = gemm_sm100_group(ctx, gg)) || pl.ks_in == 1) return rc;
             if (sums->tail) {
                 sums->split = partial;
-                for (int i = 0; i < 4; ++i) sums->split_dst[i] = dst[i];
+                for (int i = 0; i < 4; ++i) sums->split_dst[i] = static_cast<float*>(dst[i]);
                 sums->split_mn = mn; sums->splits = pl.ks_in; sums->split_n = 4;
                 return LTCA_OK;
             }
-            return sum_splits(ctx, partial, reinterpret_cast<void**>(dst), 4, mn, pl.ks_in);
+            return sum_splits(ctx, partial, dst, 4, mn, pl.ks_in);
         }
     }
     if (want_dx) {
