@@ -500,11 +500,12 @@ def test_sm_limit_changes_the_launch_width_not_the_results(ctx):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("deterministic", [False, True])
-def test_backward_with_runs_of_empty_work_items(ctx, deterministic):
+@pytest.mark.parametrize("deterministic,persistent", [(False, True), (True, False), (True, True)])
+def test_backward_with_runs_of_empty_work_items(ctx, deterministic, persistent):
     """More work items than SMs, most of them without work (short key lengths in four of five batch entries, and
     more queries than keys under a causal mask): the persistent backward kernels skip long runs of empty items
-    behind an item with work, whose last accumulation must not wait for the next item with work."""
+    behind an item with work, whose last accumulation must not wait for the next item with work.  (880 tiles of up to
+    2048 positions: bit-reproducible calls run in tiles, except under a limit on the SMs; others take the fused kernel.)"""
     B, H, Sq, Sk, D = 5, 11, 1062, 865, 64
     q, k, v, do = make_case(B, H, Sq, Sk, D, 610, 0.5)
     qr, kr, vr, dor = bf16_round(q), bf16_round(k), bf16_round(v), bf16_round(do)
@@ -515,8 +516,13 @@ def test_backward_with_runs_of_empty_work_items(ctx, deterministic):
     tq, tk, tv, tdo = (dev(x, torch.bfloat16) for x in (q, k, v, do))
     dL = torch.from_numpy(L).cuda()
     o, lse = ctx.attn_fwd(tq, tk, tv, scale=sc, causal=True, kv_len=dL, mode=_lib.MODE_BF16)
-    grads = ctx.attn_bwd(tq, tk, tv, o, lse, tdo, scale=sc, causal=True, kv_len=dL, mode=_lib.MODE_BF16,
-                         deterministic=deterministic)
+    try:
+        if persistent:
+            ctx.set_sm_limit(ctx.sm_count() - 1)
+        grads = ctx.attn_bwd(tq, tk, tv, o, lse, tdo, scale=sc, causal=True, kv_len=dL, mode=_lib.MODE_BF16,
+                             deterministic=deterministic)
+    finally:
+        ctx.set_sm_limit(0)
     torch.cuda.synchronize()
     assert ctx.device_status() == 0
     # (bf16 storage: the stored result carries one more rounding, as in test_tensor_pipe_backward)

@@ -47,7 +47,9 @@ def test_masked_forward_and_backward(ctx, shape, storage):
         assert torch.equal(o, o2) and torch.equal(lse, lse2)
 
 
-@pytest.mark.parametrize("shape", [(2, 2, 1, 1, 16), (1, 3, 31, 33, 32), (2, 80, 70, 97, 64), (1, 2, 129, 65, 128)])
+@pytest.mark.parametrize("shape", [(2, 2, 1, 1, 16), (1, 3, 31, 33, 32), (2, 80, 70, 97, 64), (1, 2, 129, 65, 128),
+                                   # one pass over more than two key blocks: by words, and without room for them on the mask as it is
+                                   (3, 40, 70, 161, 32), (2, 40, 130, 257, 16), (3, 20, 65, 190, 64)])
 @pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
 def test_exact_backward_in_a_workspace_sized_without_the_mask(ctx, shape, dt):
     B, H, Sq, Sk, D = shape

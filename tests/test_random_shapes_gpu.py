@@ -22,7 +22,8 @@ def _dev(a, dtype=None):
 
 
 def test_streaming_kernels_random_shapes(ctx):
-    """Head width 64, bf16 storage: forward, the fused backward and the two-kernel backward."""
+    """Head width 64, bf16 storage: forward, and the backward in tiles, by the fused kernel and by the two persistent
+    kernels, which short calls too take under a limit on the SMs."""
     import torch
     from cuda_ltc_b200 import _lib
     rng = np.random.default_rng(101)
@@ -43,12 +44,16 @@ def test_streaming_kernels_random_shapes(ctx):
         o, lse = ctx.attn_fwd(tq, tk, tv, **kw)
         what = (B, H, Sq, Sk, causal, L is not None)
         assert np.abs(o.float().cpu().numpy() - o_ref).max() < 1.2e-2, what
-        for det in (False, True):
-            grads = ctx.attn_bwd(tq, tk, tv, o, lse, tdo, deterministic=det, **kw)
+        for det, limit in ((False, 0), (True, 0), (False, ctx.sm_count() - 1), (True, ctx.sm_count() - 1)):
+            try:
+                ctx.set_sm_limit(limit)
+                grads = ctx.attn_bwd(tq, tk, tv, o, lse, tdo, deterministic=det, **kw)
+            finally:
+                ctx.set_sm_limit(0)
             torch.cuda.synchronize()
             assert ctx.device_status() == 0, what
             for g, r in zip(grads, ref):
-                assert np.abs(g.float().cpu().numpy() - r).max() <= 1.2e-2 * max(1.0, np.abs(r).max()), (what, det)
+                assert np.abs(g.float().cpu().numpy() - r).max() <= 1.2e-2 * max(1.0, np.abs(r).max()), (what, det, limit)
         done += 1
 
 
@@ -79,12 +84,16 @@ def test_streaming_kernels_random_shapes_many_pairs(ctx):
         o, lse = ctx.attn_fwd(tq, tk, tv, **kw)
         what = (B, H, Sq, Sk, causal, None if L is None else L.tolist(), str(dt))
         assert np.abs(o.float().cpu().numpy() - o_ref).max() < 1.2e-2, what
-        for det in (False, True):
-            grads = ctx.attn_bwd(tq, tk, tv, o, lse, tdo, deterministic=det, **kw)
+        for det, limit in ((False, 0), (True, 0), (False, ctx.sm_count() - 1), (True, ctx.sm_count() - 1)):
+            try:
+                ctx.set_sm_limit(limit)
+                grads = ctx.attn_bwd(tq, tk, tv, o, lse, tdo, deterministic=det, **kw)
+            finally:
+                ctx.set_sm_limit(0)
             torch.cuda.synchronize()
             assert ctx.device_status() == 0, what
             for g, r in zip(grads, ref):
-                assert np.abs(g.float().cpu().numpy() - r).max() <= 1.2e-2 * max(1.0, np.abs(r).max()), (what, det)
+                assert np.abs(g.float().cpu().numpy() - r).max() <= 1.2e-2 * max(1.0, np.abs(r).max()), (what, det, limit)
         done += 1
 
 
