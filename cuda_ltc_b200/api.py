@@ -175,8 +175,8 @@ class Context:
     def attn_bwd(self, q, k, v, o, lse, dout, scale=None, causal=False, keep_mask=None,
                  kv_len=None, score_clamp=0.0, mode=_lib.MODE_AUTO, dq=None, dk=None, dv=None,
                  deterministic=False):
-        """dq, dk, dv.  ``deterministic=True`` asks for bit-identical results from run to run (bf16 storage on the
-        tensor pipe otherwise takes the fused kernel, whose dq can differ between runs by fp32 rounding)."""
+        """dq, dk, dv.  ``deterministic=True`` asks for bit-identical results from run to run (long bf16 calls on the
+        tensor pipe otherwise take the fused kernel, whose dq can differ between runs by fp32 rounding)."""
         return self._host.attn_bwd(q, k, v, o, lse, dout, scale, causal, keep_mask, kv_len, score_clamp, mode, dq, dk, dv,
                                    deterministic)
 

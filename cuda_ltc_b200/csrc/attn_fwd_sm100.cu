@@ -539,6 +539,9 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q,
 //   - warps 0-3 softmax, one row per thread, head_dim keys per step; tensor memory S [0, D), O [D, 2 D).  At head_dim 128 a
 //     thread so holds 128 scores in its 216 registers and two warps share a scheduler; two threads per row, 64 scores each,
 //     had four of them but met once a step to agree on the row's maximum (B8 H16 S4096 causal 568 us, one per row 525).
+//     Two score buffers and 64 keys a step there overlap a step's products with the softmax before it (ragged causal B4 H16 S1500
+//     40.5 -> 37.0 us), but take P relative to a maximum over half as many keys: the error against 64 bits grows by 1 % at inputs
+//     of unit variance, and B16 H8 S256 causal takes 8.5 us and not 8.2.
 //     fp32 results at head_dim 128 have two threads per row (warps 0-7), which share the work of P's second term, and the
 //     halves of P below are one thread's each (B8 H16 S2048 causal 325 -> 319 us).  Not with a mask, whose words no longer fit
 //     their 104 registers: what is spilled goes out to L2, since the tiles leave an SM next to no L1 (masked B64 H8 S200 126 us
