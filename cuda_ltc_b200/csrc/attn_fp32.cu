@@ -1386,11 +1386,15 @@ struct OnePass {
     size_t bytes = 0;
 };
 // Where one pass over the scores is the faster one.  (Backward, us, two kernels and one pass.)
-//   - One key block: always (B2 H4 S64 D32 11.4 and 10.9, B12 H8 S64 D64 22 and 14).
-//   - A CTA walks all queries of its 64 keys: with few CTAs that chain is longer than that of the two kernels' 16-row tiles.  From two
-//     thirds of a CTA per SM on (128 CTAs, B4 H4 S512: D16 67 and 56, D32 103 and 77; 64 CTAs, B2 H4 S512 causal: D16 51 and 53, D32
-//     69 and 73), above head width 32, where a tile has twice the warps, from a third on (64 CTAs, B2 H4 S512 105 and 93; 28 CTAs,
-//     B1 H4 S400 70 and 80).
+//   - A CTA walks all queries of its 64 keys: with few CTAs that chain is longer than that of the two kernels, which deal the
+//     queries out.  From two thirds of a CTA per SM on (128 CTAs, B4 H4 S512: D16 67 and 56, D32 103 and 77; 64 CTAs, B2 H4 S512 causal:
+//     D16 51 and 53, D32 69 and 73).  Above head width 32, where a tile has twice the warps, from a third on (64 CTAs, B2 H4 S512 105
+//     and 93; 28 CTAs, B1 H4 S400 70 and 80), with more than 512 queries and more than there are keys from 0.55 (16 pairs, 64 CTAs, 3000
+//     queries over 256 keys 7 % slower; 24 pairs 15 % faster).
+//   - One key block writes dQ where it belongs, which saves a launch.  Up to 64 queries, one or two steps, always (B2 H4 S64 D32 11.4 and
+//     10.9), but for blocks of 64 keys at head widths 17 to 32 (32 queries, 50 keys: 5 % slower).  Up to 512 queries from a third of
+//     a CTA per SM on (64 pairs, 512 queries, 50 keys: D16 0.88 of the time, D32 0.95, D64 0.87; 32 pairs 1.27, 1.43, 1.27), beyond them, and
+//     for blocks of 32 keys above head width 32, from 0.55 (1000 queries, 50 keys, D32: 64 pairs 1.06, 88 pairs 0.87).
 //   - Several launches drain one by one, and a causal one lasts as long as the chain of the first keys, twice the mean.  Where a launch
 //     has on average 0.6 of the CTAs that are resident at once; causal 0.6 in two launches, a tenth more for each further one, 0.9 in
 //     the end.  Full, D64 S8192 13 pairs 0.80 of them 20270 and 16750, S10000 0.53 29170 and 39880; D32 S6000 8 pairs 0.64 3920 and
@@ -1402,21 +1406,28 @@ static OnePass one_pass(const ltca_attn_params* p, int sms, size_t room) {
     const int64_t all = (int64_t)p->B * p->H, blocks = ((int64_t)p->Sk + 63) / 64;
     if (p->D > 64 || p->B > 65535 || p->H > 65535 || all > 0x7fffffff || blocks > 65535) return o;     // (B, H: as the two kernels' grids)
     o.ld = (p->D + 3) / 4 * 4;
-    if (blocks == 1) {
-        o.pairs = (int)all;
+    const bool single = blocks == 1, narrow = p->D <= 32;
+    const int tile = p->Sk <= 32 ? 32 : 64, unseeing = p->causal && p->Sq > p->Sk ? (p->Sq - p->Sk) / tile * tile : 0;
+    const int rows = p->Sq - unseeing;                                     // less whole tiles of queries that see no key
+    int need = 66;                                                         // CTAs, in hundredths of the SMs
+    if (single ? rows <= 512 && (narrow || p->Sk > 32) : !narrow && (rows <= 512 || rows <= p->Sk)) need = 33;
+    else if (single || !narrow) need = 55;
+    if (single && rows <= 64 && (rows > 32 || p->Sk <= 32 || p->D <= 16 || !narrow)) need = 0;
+    if (single) {
+        if (100 * all >= need * (int64_t)sms) o.pairs = (int)all;
         return o;
     }
     const size_t one = (size_t)blocks * p->Sq * o.ld * sizeof(float);
     const int64_t fit = (int64_t)((room < kPartBytes ? room : kPartBytes) / one);
     if (fit == 0) return o;
-    const int64_t launches = (all + fit - 1) / fit, slots = (p->D > 32 ? 2 : 4) * (int64_t)sms;      // slots: CTAs resident at once
+    const int64_t launches = (all + fit - 1) / fit, slots = (narrow ? 4 : 2) * (int64_t)sms;      // slots: CTAs resident at once
     // As many pairs a launch as there is room for, or as many in each where that takes less time: waves of CTAs, causal the chain (D32
     // 8 pairs S6000 7 + 1 3395 us, 4 + 4 3140; D16 S10000 5 + 3 5000, 4 + 4 5480).
     auto time = [&](int64_t n) { return p->causal ? (n * blocks > 2 * slots ? n * blocks : 2 * slots) : (n * blocks + slots - 1) / slots; };
     auto total = [&](int64_t n) { return (launches - 1) * time(n) + time(all - (launches - 1) * n); };
     int64_t pairs = (all + launches - 1) / launches;
     if (launches > 1 && total(pairs) >= total(fit)) pairs = fit;
-    if (3 * pairs * blocks < (p->D > 32 ? 1 : 2) * (int64_t)sms) return o;
+    if (100 * pairs * blocks < need * (int64_t)sms) return o;
     const int64_t tenths = p->causal && launches > 2 ? (launches < 5 ? 4 + launches : 9) : 6;
     if (launches > 1 && 10 * all * blocks < tenths * launches * slots) return o;
     o.pairs = (int)pairs;

@@ -32,6 +32,10 @@ def _one(Sq, Sk, D):
     (64, 8, 64, 64, 32, False, 0),             # one block of keys: dQ is written where it belongs
     (4, 4, 512, 512, 32, False, 16),           # 128 CTAs on 148 SMs
     (1, 1, 2048, 2048, 64, False, 0),          # 32 CTAs: the two kernels
+    (1, 28, 3000, 128, 64, False, 0),          # 56 CTAs that walk 3000 queries: the two kernels, which deal them out
+    (1, 28, 3000, 128, 64, True, 28),          # ... of which the last 128 see a key
+    (1, 28, 300, 128, 64, False, 28),
+    (1, 42, 3000, 128, 64, False, 42),         # 84 CTAs
     (1, 1, 4096, 4096, 32, False, 0),
     (64, 8, 512, 512, 64, False, 512),         # all pairs at once, the most room there is
     (1, 8, 6000, 6000, 32, False, 4),          # seven pairs fit: two launches of four, a wave each, not 1.1 waves and the rest
