@@ -316,16 +316,18 @@ __global__ void __launch_bounds__(NT, TM < 64 ? 4 : DP <= 32 ? 4 : DP <= 64 ? 3 
     load_padded<DP, KN, NT>(Vs, vb, a.vs.seq, 0, a.Sk, a.D, vec);
     cp_async_commit();
 
-    // Dense mask: every warp votes its share of the next step's words (32 keys of a row each) in two halves, one read under the score
-    // product, the other under the value product.  (The first half under the value product and the second behind it, whose latency
-    // then lies bare: B64 H8 S128 D32 44.9 us, so 43.2; B16 H8 S250 D32 47.1 and 45.8, D64 83.7 and 83.3, B24 H8 S200 D64 106.1 and 107.0.
-    // Both halves under the value product: spills at D32, 4 % slower.)
+    // Dense mask: every warp votes its share of the next step's words (32 keys of a row each) in two halves.  64-row tiles of heads up to
+    // 32 (kEarly) read one under the score product and the other under the value product, into one of two sets of words; others the
+    // first under the value product and the second behind it, under the wait for the next keys.  (us, late and early: B64 H8 S128 D32
+    // 44.9 and 43.2, B16 H8 S250 D32 47.1 and 45.7, D16 33.8 and 33.3, D64 83.7 and 83.3, B24 H8 S200 D64 105.9 and 106.7, B2 H4 S200 D64
+    // in 16-row tiles 13.0 and 13.3.  Both halves under the value product: spills at D32, 4 % slower.)
+    constexpr bool kEarly = TM == 64 && DP <= 32;
     constexpr int kWords2 = TM / (NT / 32);                               // words of half a warp's rows
-    uint32_t* mask_sm = reinterpret_cast<uint32_t*>(row_scale + TM);      // [2 steps][TM][2]
+    uint32_t* mask_sm = reinterpret_cast<uint32_t*>(row_scale + TM);      // [TM][2], kEarly: of two steps
     const int lane = threadIdx.x & 31, mask_row = (threadIdx.x >> 5) * kWords2;
     float mv[kWords2];
     static_assert(kWords2 % 2 == 0, "whole rows");
-    auto mask_read = [&](int half, int k) {
+    auto mask_read = [&](float (&mv)[kWords2], int half, int k) {
         const int r0 = q0 + mask_row + half * (kWords2 / 2);
         const float* p = a.keep_mask + ((int64_t)b * a.Sq + r0) * a.Sk + k + lane;
 #pragma unroll
@@ -335,7 +337,7 @@ __global__ void __launch_bounds__(NT, TM < 64 ? 4 : DP <= 32 ? 4 : DP <= 64 ? 3 
             mv[w + 1] = row && k + 32 + lane < k_end ? __ldg(p + 32) : 0.f;
         }
     };
-    auto mask_vote = [&](uint32_t* words, int half) {
+    auto mask_vote = [&](const float (&mv)[kWords2], uint32_t* words, int half) {
 #pragma unroll
         for (int w = 0; w < kWords2; w += 2) {
             const uint32_t x = __ballot_sync(0xffffffffu, mv[w] != 0.f), y = __ballot_sync(0xffffffffu, mv[w + 1] != 0.f);
@@ -343,10 +345,11 @@ __global__ void __launch_bounds__(NT, TM < 64 ? 4 : DP <= 32 ? 4 : DP <= 64 ? 3 
         }
     };
     if (kMask) {
-        mask_read(0, 0);
-        mask_vote(mask_sm, 0);
-        mask_read(1, 0);
-        mask_vote(mask_sm, 1);
+        float first[kWords2];                                             // the first step's halves in flight together
+        mask_read(first, 0, 0);
+        mask_read(mv, 1, 0);
+        mask_vote(first, mask_sm, 0);
+        if (kEarly) mask_vote(mv, mask_sm, 1);
     }
 
     const Lt L;
@@ -361,14 +364,15 @@ __global__ void __launch_bounds__(NT, TM < 64 ? 4 : DP <= 32 ? 4 : DP <= 64 ? 3 
 
     for (int k0 = 0; k0 < k_end; k0 += KN) {
         const bool more = k0 + KN < k_end;
-        const uint32_t* mask_now = mask_sm + (k0 / KN & 1) * (2 * TM);
-        uint32_t* mask_next = mask_sm + ((k0 / KN + 1) & 1) * (2 * TM);
-        if (kMask && more) mask_read(0, k0 + KN);
+        uint32_t* mask_now = mask_sm + (kEarly ? (k0 / KN & 1) * (2 * TM) : 0);
+        uint32_t* mask_next = mask_sm + (kEarly ? ((k0 / KN + 1) & 1) * (2 * TM) : 0);
+        if (kMask && kEarly && more) mask_read(mv, 0, k0 + KN);
         cp_async_wait<1>();
+        if (kMask && !kEarly) mask_vote(mv, mask_now, 1);
         __syncthreads();
         float s[RM][CN];
         tile_dot<DP, NT, RM, CN, TM == 64 && (kMask || DP >= 32) ? 1 : 2>(s, Qs, Ks, row0, tx);      // (two at a time spill there)
-        if (kMask && more) mask_vote(mask_next, 0);
+        if (kMask && kEarly && more) mask_vote(mv, mask_next, 0);
         const bool all_visible = k0 + KN <= kvlen && !kMask && (!a.causal || k0 + KN - 1 <= q0 + a.causal_off);
 #pragma unroll
         for (int i = 0; i < RM; ++i) {
@@ -404,9 +408,10 @@ __global__ void __launch_bounds__(NT, TM < 64 ? 4 : DP <= 32 ? 4 : DP <= 64 ? 3 
             m_run[i] = m_new;
             if (tx == 0) row_scale[r] = corr;
         }
-        if (kMask && more) mask_read(1, k0 + KN);
+        if (kMask && kEarly && more) mask_read(mv, 1, k0 + KN);
         cp_async_wait<0>();
         __syncthreads();
+        if (kMask && !kEarly && more) mask_read(mv, 0, k0 + KN);
         if (more) load_padded<DP, KN, NT>(Ks, kb, a.ks.seq, k0 + KN, a.Sk, a.D, vec);
         cp_async_commit();
         if (L.active) {
@@ -419,7 +424,11 @@ __global__ void __launch_bounds__(NT, TM < 64 ? 4 : DP <= 32 ? 4 : DP <= 64 ? 3 
             }
             accumulate<DP, TM, NT>(acc, L, Ps, LP, Vs, min(KN, (k_end - k0 + 3) & ~3));
         }
-        if (kMask && more) mask_vote(mask_next, 1);
+        if (kMask && kEarly && more) mask_vote(mv, mask_next, 1);
+        if (kMask && !kEarly && more) {
+            mask_vote(mv, mask_next, 0);
+            mask_read(mv, 1, k0 + KN);
+        }
         __syncthreads();
         if (more) load_padded<DP, KN, NT>(Vs, vb, a.vs.seq, k0 + KN, a.Sk, a.D, vec);
         cp_async_commit();
@@ -1076,7 +1085,7 @@ int set_smem(ltca_ctx* ctx, K kern, size_t bytes, SmemOptIn& once) {
 template <typename T, int DP, int TM, int NT, bool kMask>
 int run_fwd(ltca_ctx* ctx, const CoreArgs& a) {
     static SmemOptIn once;
-    constexpr size_t smem = ((size_t)(TM + 128) * (DP + kPad) + TM * (64 + kPad) + TM + (kMask ? 4 * TM : 0)) * sizeof(float);
+    constexpr size_t smem = ((size_t)(TM + 128) * (DP + kPad) + TM * (64 + kPad) + TM + (kMask ? (TM == 64 && DP <= 32 ? 4 : 2) * TM : 0)) * sizeof(float);
     int rc = set_smem(ctx, attn_fwd_fp32_kernel<T, DP, TM, NT, kMask>, smem, once);
     if (rc) return rc;
     dim3 grid((a.Sq + TM - 1) / TM, a.H, a.B);
