@@ -1160,19 +1160,25 @@ int workspace_bytes(const ltca_tsa_params* t, int which, Room room, size_t* byte
 // The call as its workspace is laid out.  Packed mask words and the exact backward's shares of dQ are part of what
 // ltca_tsa_workspace_bytes asks for, but a workspace that was sized without the mask is laid out without the words (the attention
 // kernels then read the dense values), and one that has no room for the shares without those.
-ltca_tsa_params laid_out(const ltca_tsa_params* t, int which, Room* room = nullptr) {
-    ltca_tsa_params l = *t;
-    if (!room && !t->keep_mask) return l;
-    for (Room r : {kFullRoom, kLeastRoom}) {
-        if (room) *room = r;
-        for (const float* mask : {t->keep_mask, (const float*)nullptr}) {
-            size_t need = 0;
-            l.keep_mask = mask;
-            if (!workspace_bytes(&l, which, r, &need) && l.workspace_bytes >= need) return l;
+struct Layout {
+    ltca_tsa_params t;
+    Room room;
+    size_t need;                   // what it takes: more than there is where no layout fits
+    int rc;
+};
+Layout lay_out(const ltca_tsa_params* t, int which) {
+    Layout l{*t, kFullRoom, 0, LTCA_OK};
+    for (Room room : {kFullRoom, kLeastRoom}) {
+        l.room = room;
+        for (int masked = t->keep_mask ? 1 : 0; masked >= 0; --masked) {
+            l.t.keep_mask = masked ? t->keep_mask : nullptr;
+            l.rc = workspace_bytes(&l.t, which, room, &l.need);
+            if (!l.rc && t->workspace_bytes >= l.need) return l;
         }
     }
     return l;
 }
+ltca_tsa_params laid_out(const ltca_tsa_params* t, int which) { return t->keep_mask ? lay_out(t, which).t : *t; }
 
 // What a module call tells its kernels through the context, taken back when the call returns.
 struct CallHints {
@@ -1946,10 +1952,9 @@ static int prenorm_forward(ltca_ctx* ctx, const ltca_tsa_params* t) {
 
 // FlashAttention form, backward (an extension: the reference class has no backward pass).
 static int prenorm_backward(ltca_ctx* ctx, const ltca_tsa_params* t, bool want_dx, bool want_dw) {
-    size_t need = 0;
-    Room room;
-    const ltca_tsa_params layout = laid_out(t, 1, &room);
-    int rc = workspace_bytes(&layout, 1, room, &need);
+    const Layout layout = lay_out(t, 1);
+    const size_t need = layout.need;
+    int rc = layout.rc;
     if (rc) return rc;
     if (!t->workspace || t->workspace_bytes < need)
         return fail(ctx, LTCA_ERR_WORKSPACE, "backward needs %zu bytes of workspace", need);
@@ -2069,10 +2074,8 @@ static int tsa_backward(ltca_ctx* ctx, const ltca_tsa_params* t, bool want_dx, b
     if (t->dropout_prob < 0.f || t->dropout_prob >= 1.f)
         return fail(ctx, LTCA_ERR_INVALID, "dropout_prob must be in [0, 1)");
     if (t->pre_norm) return prenorm_backward(ctx, t, want_dx, want_dw);
-    size_t need = 0;
-    Room room;
-    const ltca_tsa_params layout = laid_out(t, 1, &room);
-    workspace_bytes(&layout, 1, room, &need);
+    const Layout layout = lay_out(t, 1);
+    const size_t need = layout.need;
     if (!t->workspace || t->workspace_bytes < need)
         return fail(ctx, LTCA_ERR_WORKSPACE, "backward needs %zu bytes of workspace", need);
     float* colsum_scratch =
@@ -2085,7 +2088,7 @@ static int tsa_backward(ltca_ctx* ctx, const ltca_tsa_params* t, bool want_dx, b
         return column_sums(ctx, own, (int64_t)t->B * t->S, colsum_scratch);
     }
     Plan pl;
-    if ((rc = make_plan(&layout, &pl, room))) return rc;
+    if ((rc = make_plan(&layout.t, &pl, layout.room))) return rc;
     char* w = reinterpret_cast<char*>(t->workspace);
     float* dctx = reinterpret_cast<float*>(w); w += pl.buf;
     float* dq = reinterpret_cast<float*>(w);   w += pl.buf;
