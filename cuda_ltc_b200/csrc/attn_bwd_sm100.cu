@@ -842,7 +842,7 @@ __device__ __forceinline__ void dkv_tile(const BwdMaps& m, const BwdArgs& a, int
     }
 }
 
-// dK/dV's tiles and dQ's in one launch, dK/dV's (the longer ones) first, each heaviest first.  kPlain: with results of BwdArgs::plain
+// dK/dV's tiles and dQ's in one launch, dK/dV's (the longer ones where the lengths are alike) first, each heaviest first.  kPlain: with results of BwdArgs::plain
 // (as a branch of the one kernel the step B32 H8 S256 took 81.1 us and not 80.9).
 template <typename OutT, bool kMask, bool kPlain>
 __global__ void __launch_bounds__(kTileThreads, 2)
@@ -2355,20 +2355,34 @@ bool in_place(const ltca_attn_params* p) {
 //     and 31.2; B32 H4 S512 55 and 58; at 128 B2 H4 S1024 25.9 and 25.5, B4 H4 S1024 27.7 and 29.8), up to 128 any number (B64 H16
 //     S128 67 and 58; B64 H8 S256 73 and 74), causal up to 384 (B64 H8 S384 122 and 117; B32 H8 S512 83 and 86), never with a
 //     mask (B8 H8 S500 47 and 53).
+//   - A tile walks the other side's whole length in steps of 64, the persistent kernels in steps of 128, and the one-kernel form has no tile
+//     that walks the keys.  So few queries over more than 576 keys stay with that form (8 pairs, 128 queries: 640 keys 12.9 and 13.4, 1024
+//     13.1 and 18.4; 384 queries 800 keys 16.6 and 15.5, 1024 17.1 and 18.5).  The persistent pair keeps more than 1024 queries that all see
+//     far fewer keys, in one wave (8 pairs, 2000 queries: 128 keys 37.5 and 45.0, 1024 45.4 and 49.3, 2000 79 and 76), and more than
+//     1024 keys of 257 to 2/7 as many queries that see all, in more than two waves, where dQ's long tiles come last (32 pairs, 2000 keys: 512
+//     queries 61 and 68, 640 85 and 75).
 // A limit on the context's SMs keeps to the persistent kernels, which obey it.
 bool bwd_in_tiles(const ltca_ctx* ctx, const ltca_attn_params* p) {
-    if (ctx->sm_count < ctx->sm_device || in_place(p)) return false;
+    if (ctx->sm_count < ctx->sm_device) return false;
     const int S = p->Sq > p->Sk ? p->Sq : p->Sk;
     const int64_t tiles = (int64_t)p->B * p->H * ((p->Sq + kTile - 1) / kTile + (p->Sk + kTile - 1) / kTile);
-    if (p->bwd_deterministic) return S <= 768 || (S <= 2048 && tiles <= 1536);
-    if (p->keep_mask || !tma_strides(p->dq_strides, p->B, p->H)) return false;     // (the one-kernel form's dQ takes any strides)
-    return S <= 128 || (S <= 384 && p->causal) || (S <= 640 && tiles <= 512) || (S <= 1024 && tiles <= 128);
+    bool pays;
+    if (p->bwd_deterministic) {
+        const bool few_keys = !p->causal && p->Sq > 1024 && 2 * (int64_t)p->Sq > 3 * (int64_t)p->Sk && tiles <= 2 * ctx->sm_device;
+        const bool few_queries = !p->causal && p->Sk > 1024 && p->Sq > 256 && 2 * (int64_t)p->Sk > 7 * (int64_t)p->Sq && tiles > 4 * ctx->sm_device;
+        pays = S <= 768 || (S <= 2048 && tiles <= 1536 && !few_keys && !few_queries);
+    } else {
+        const bool few_queries = tiles <= 128 && (p->Sk > 640 ? 5 * (int64_t)p->Sq < 2 * (int64_t)p->Sk : p->Sk > 576 && p->Sq <= kTile);
+        pays = S <= 128 || (S <= 384 && p->causal) || (((S <= 640 && tiles <= 512) || (S <= 1024 && tiles <= 128)) && !few_queries);
+        pays = pays && !p->keep_mask && tma_strides(p->dq_strides, p->B, p->H);       // (the one-kernel form's dQ takes any strides)
+    }
+    return pays && !in_place(p);
 }
 
 template <typename OutT, bool kMask>
 int launch_main(ltca_ctx* ctx, const ltca_attn_params* p, const void* mask_words, const void* q, const void* k, const void* v,
                 const void* dout, const ltca_strides& qs, const ltca_strides& ks, const ltca_strides& vs,
-                const ltca_strides& dos, const float* lse2, const float* delta, float* dq_acc) {
+                const ltca_strides& dos, const float* lse2, const float* delta, float* dq_acc, bool tiles) {
     BwdMaps m;
     int rc;
     if ((rc = make_tmap_bhsd(ctx, &m.q128, q, 2, p->B, p->H, p->Sq, kD, qs, 64, kTile))) return rc;
@@ -2431,7 +2445,7 @@ int launch_main(ltca_ctx* ctx, const ltca_attn_params* p, const void* mask_words
             return LTCA_OK;
         }
     }
-    if (sizeof(OutT) == 4 || bwd_in_tiles(ctx, p)) {
+    if (tiles) {
         if ((rc = make_tmap_bhsd(ctx, &m.q64, q, 2, p->B, p->H, p->Sq, kD, qs, 64, kStep))) return rc;
         if ((rc = make_tmap_bhsd(ctx, &m.do64, dout, 2, p->B, p->H, p->Sq, kD, dos, 64, kStep))) return rc;
         if ((rc = make_tmap_bhsd(ctx, &m.k64, k, 2, p->B, p->H, p->Sk, kD, ks, 64, kStep))) return rc;
@@ -2523,8 +2537,9 @@ int launch_attn_bwd_sm100(ltca_ctx* ctx, const ltca_attn_params* p) {
     float* lse2 = reinterpret_cast<float*>(w);  w += stats_bytes(p);
     float* delta = reinterpret_cast<float*>(w); w += stats_bytes(p);
     float* dq_acc = nullptr;
+    const bool tiles = p->dtype == LTCA_F32 || bwd_in_tiles(ctx, p);
     if (use_fused(p)) {
-        if (!bwd_in_tiles(ctx, p)) dq_acc = reinterpret_cast<float*>(w);
+        if (!tiles) dq_acc = reinterpret_cast<float*>(w);
         w += dq_acc_bytes(p);
     }
 
@@ -2544,7 +2559,7 @@ int launch_attn_bwd_sm100(ltca_ctx* ctx, const ltca_attn_params* p) {
         LTCA_LAUNCH_OK(ctx, "attn_bwd_stats_kernel");
         kernel_timing_mark(ctx, 1);
         return (p->keep_mask ? launch_main<__nv_bfloat16, true> : launch_main<__nv_bfloat16, false>)(
-            ctx, p, words, p->q, p->k, p->v, p->dout, p->q_strides, p->k_strides, p->v_strides, p->do_strides, lse2, delta, dq_acc);
+            ctx, p, words, p->q, p->k, p->v, p->dout, p->q_strides, p->k_strides, p->v_strides, p->do_strides, lse2, delta, dq_acc, tiles);
     }
 
     const PackJob jobs[3] = {{p->q, p->q_strides, qb, p->Sq}, {p->k, p->k_strides, kb, p->Sk}, {p->v, p->v_strides, vb, p->Sk}};
@@ -2566,7 +2581,7 @@ int launch_attn_bwd_sm100(ltca_ctx* ctx, const ltca_attn_params* p) {
     ltca_strides cq{(int64_t)p->H * p->Sq * kD, (int64_t)p->Sq * kD, kD};
     ltca_strides ck{(int64_t)p->H * p->Sk * kD, (int64_t)p->Sk * kD, kD};
     return (p->keep_mask ? launch_main<float, true> : launch_main<float, false>)(ctx, p, words, qb, kb, vb, gb, cq, ck, ck, cq, lse2,
-                                                                                 delta, nullptr);
+                                                                                 delta, nullptr, tiles);
 }
 
 }  // namespace ltca

@@ -71,3 +71,20 @@ def test_backward_in_tiles(ctx, case, storage):
     for a, b in zip(grads, persistent):
         assert torch.equal(a, b)
     assert ctx.device_status() == 0
+
+
+# (few queries over many keys and the other way round, on both sides of the lines that keep such calls on the one-kernel form or
+# the persistent pair)
+@pytest.mark.parametrize("B,H,Sq,Sk,causal", [(1, 2, 100, 576, False), (1, 2, 100, 600, False), (1, 3, 128, 1024, True), (1, 2, 410, 1024, False),
+                                              (1, 2, 409, 1024, False), (2, 2, 1100, 100, False), (2, 2, 1100, 800, True), (4, 8, 300, 1060, False)])
+@pytest.mark.parametrize("det", [False, True])
+def test_unequal_lengths(ctx, B, H, Sq, Sk, causal, det):
+    g = torch.Generator(device="cuda").manual_seed(19)
+    rand = lambda n: (torch.randn((B, H, n, 64), generator=g, device="cuda") * 0.5).bfloat16()
+    q, k, v, do = rand(Sq), rand(Sk), rand(Sk), rand(Sq)
+    o, lse = ctx.attn_fwd(q, k, v, causal=causal, mode=_lib.MODE_BF16)
+    grads = ctx.attn_bwd(q, k, v, o, lse, do, causal=causal, deterministic=det, mode=_lib.MODE_BF16)
+    for name, got, ref in zip(("dq", "dk", "dv"), grads, _reference(q, k, v, do, causal, None, None, 0.0)):
+        err = (got.double() - ref).abs()         # as above
+        assert bool((err <= 2e-3 * max(1.0, float(ref.abs().max())) + 2.0 ** -8 * ref.abs()).all()), (name, float(err.max()))
+    assert ctx.device_status() == 0
