@@ -1394,16 +1394,20 @@ struct OnePass {
     int pairs = 0, ld = 0;        // 0: the two kernels
     size_t bytes = 0;
 };
-// Where one pass over the scores is the faster one.  (Backward, us, two kernels and one pass.)
-//   - A CTA walks all queries of its 64 keys: with few CTAs that chain is longer than that of the two kernels, which deal the
-//     queries out.  From two thirds of a CTA per SM on (128 CTAs, B4 H4 S512: D16 67 and 56, D32 103 and 77; 64 CTAs, B2 H4 S512 causal:
-//     D16 51 and 53, D32 69 and 73).  Above head width 32, where a tile has twice the warps, from a third on (64 CTAs, B2 H4 S512 105
-//     and 93; 28 CTAs, B1 H4 S400 70 and 80), with more than 512 queries and more than there are keys from 0.55 (16 pairs, 64 CTAs, 3000
-//     queries over 256 keys 7 % slower; 24 pairs 15 % faster).
-//   - One key block writes dQ where it belongs, which saves a launch.  Up to 64 queries, one or two steps, always (B2 H4 S64 D32 11.4 and
-//     10.9), but for blocks of 64 keys at head widths 17 to 32 (32 queries, 50 keys: 5 % slower).  Up to 512 queries from a third of
-//     a CTA per SM on (64 pairs, 512 queries, 50 keys: D16 0.88 of the time, D32 0.95, D64 0.87; 32 pairs 1.27, 1.43, 1.27), beyond them, and
-//     for blocks of 32 keys above head width 32, from 0.55 (1000 queries, 50 keys, D32: 64 pairs 1.06, 88 pairs 0.87).
+// Where one pass over the scores is the faster one.  A CTA walks all queries of its 64 keys, which the two kernels deal out; with few
+// CTAs that chain is the longer one.  (Of a CTA per SM; the time in units of the two kernels', or us of either.)
+//   - One key block writes dQ where it belongs, which saves a launch (and the mask's words another).  Up to 64 queries, one or two steps,
+//     always (B2 H4 S64 D32 11.4 and 10.9 us; at worst 32 queries, 64 keys, D32 1.07); to 128 where blocks of 32 keys gain as much or most
+//     queries see no key.  Up to 512 queries from 0.35 (50 keys, 512 queries: 56 pairs D16 0.90, D64 0.89; 44 pairs D16 1.15), to 256 from
+//     0.25 where the two kernels' dQ goes to 64-row tiles (20 keys, 256 queries, D16: 36 pairs 1.14, 40 pairs 0.81), beyond from 0.42, in
+//     blocks of 64 keys up to head width 32 from 0.54 (1024 queries: 80 pairs D16 0.94, 64 pairs D64 0.87).  A tenth more for blocks of 64
+//     keys at head widths 17 to 32 (0.05 to 0.1 slower than at others throughout), 0.15 for causal calls with dQ in 16-row tiles, which skip
+//     more (B26 H2, 93 queries, 46 keys, D8 1.15).
+//   - Several blocks: a CTA for each SM, or two thirds, above head width 32, where a tile has twice the warps, one third (128 CTAs, B4 H4
+//     S512: D16 67 and 56 us, D32 103 and 77; 64 CTAs, B2 H4 S512 D64 105 and 93; 28 CTAs, B1 H4 S400 D64 70 and 80); there with more
+//     than 512 queries and more than there are keys 0.54 (256 keys, 3000 queries: 16 pairs 1.07, 24 pairs 0.85).  Three quarters of that
+//     in keys, since a last block may hold few.  Causal calls with dQ in 16-row tiles: in keys 0.75, above head width 32 0.37 (S256 D16
+//     100 CTAs 1.00, 128 0.93; D64 40 CTAs 1.02, 64 0.91; S65, two blocks, D32 128 CTAs 1.25), unless a mask's words even that out.
 //   - Several launches drain one by one, and a causal one lasts as long as the chain of the first keys, twice the mean.  Where a launch
 //     has on average 0.6 of the CTAs that are resident at once; causal 0.6 in two launches, a tenth more for each further one, 0.9 in
 //     the end.  Full, D64 S8192 13 pairs 0.80 of them 20270 and 16750, S10000 0.53 29170 and 39880; D32 S6000 8 pairs 0.64 3920 and
@@ -1415,14 +1419,15 @@ static OnePass one_pass(const ltca_attn_params* p, int sms, size_t room) {
     const int64_t all = (int64_t)p->B * p->H, blocks = ((int64_t)p->Sk + 63) / 64;
     if (p->D > 64 || p->B > 65535 || p->H > 65535 || all > 0x7fffffff || blocks > 65535) return o;     // (B, H: as the two kernels' grids)
     o.ld = (p->D + 3) / 4 * 4;
-    const bool single = blocks == 1, narrow = p->D <= 32;
-    const int tile = p->Sk <= 32 ? 32 : 64, unseeing = p->causal && p->Sq > p->Sk ? (p->Sq - p->Sk) / tile * tile : 0;
+    const bool narrow = p->D <= 32, small = p->Sk <= 32;                   // small: blocks of 32 keys
+    const int unseeing = p->causal && p->Sq > p->Sk ? (p->Sq - p->Sk) / (small ? 32 : 64) * (small ? 32 : 64) : 0;
     const int rows = p->Sq - unseeing;                                     // less whole tiles of queries that see no key
-    int need = 66;                                                         // CTAs, in hundredths of the SMs
-    if (single ? rows <= 512 && (narrow || p->Sk > 32) : !narrow && (rows <= 512 || rows <= p->Sk)) need = 33;
-    else if (single || !narrow) need = 55;
-    if (single && rows <= 64 && (rows > 32 || p->Sk <= 32 || p->D <= 16 || !narrow)) need = 0;
-    if (single) {
+    const bool dq64 = all * (((int64_t)p->Sq + 63) / 64) >= sms;           // the two kernels' dQ in 64-row tiles
+    if (blocks == 1) {
+        int need = rows > 512 ? (narrow && !small ? 54 : 42) : rows <= 256 && dq64 ? 25 : 35;
+        if (narrow && p->D > 16 && !small) need += 10;
+        if (p->causal && !dq64) need += 15;
+        if (rows <= 64 || (rows <= 128 && ((small && (p->D <= 16 || p->keep_mask)) || (unseeing && dq64)))) need = 0;
         if (100 * all >= need * (int64_t)sms) o.pairs = (int)all;
         return o;
     }
@@ -1436,7 +1441,11 @@ static OnePass one_pass(const ltca_attn_params* p, int sms, size_t room) {
     auto total = [&](int64_t n) { return (launches - 1) * time(n) + time(all - (launches - 1) * n); };
     int64_t pairs = (all + launches - 1) / launches;
     if (launches > 1 && total(pairs) >= total(fit)) pairs = fit;
-    if (100 * pairs * blocks < need * (int64_t)sms) return o;
+    if (pairs * blocks < sms) {
+        const bool skips = p->causal && rows > 64 && !dq64 && !p->keep_mask;
+        const int need = skips ? (narrow ? 100 : 49) : narrow ? 66 : rows <= 512 || rows <= p->Sk ? 33 : 54;      // in keys three quarters
+        if ((!skips && 100 * pairs * blocks < need * (int64_t)sms) || 400 * pairs * p->Sk < 3 * need * 64 * (int64_t)sms) return o;
+    }
     const int64_t tenths = p->causal && launches > 2 ? (launches < 5 ? 4 + launches : 9) : 6;
     if (launches > 1 && 10 * all * blocks < tenths * launches * slots) return o;
     o.pairs = (int)pairs;
