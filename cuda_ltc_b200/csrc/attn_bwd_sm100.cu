@@ -2357,23 +2357,34 @@ bool in_place(const ltca_attn_params* p) {
 //     mask (B8 H8 S500 47 and 53).
 //   - A tile walks the other side's whole length in steps of 64, the persistent kernels in steps of 128, and the one-kernel form has no tile
 //     that walks the keys.  So few queries over more than 576 keys stay with that form (8 pairs, 128 queries: 640 keys 12.9 and 13.4, 1024
-//     13.1 and 18.4; 384 queries 800 keys 16.6 and 15.5, 1024 17.1 and 18.5).  The persistent pair keeps more than 1024 queries that all see
+//     13.1 and 18.4; 384 queries 800 keys 16.6 and 15.5, 1024 17.1 and 18.5), and so do more than 900 queries over a third as many keys
+//     (2 pairs, 64 keys: 900 queries 1.00 of the time, 1000 1.05).  The persistent pair keeps more than 1024 queries that all see
 //     far fewer keys, in one wave (8 pairs, 2000 queries: 128 keys 37.5 and 45.0, 1024 45.4 and 49.3, 2000 79 and 76), and more than
 //     1024 keys of 257 to 2/7 as many queries that see all, in more than two waves, where dQ's long tiles come last (32 pairs, 2000 keys: 512
-//     queries 61 and 68, 640 85 and 75).
+//     queries 61 and 68, 640 85 and 75).  With a mask, whose words cost a step of 64 as much as one of 128, it keeps causal calls of more
+//     than 900 on both sides (16 pairs S900 1.06 of its time in tiles, S1500 1.22; 32 pairs, 167 queries 1149 keys 0.88), of more than 640
+//     while its two kernels are three waves at most and half full (16 pairs S800 1.03, 32 pairs S900 0.99), and others of more than 900
+//     over more than 300 in up to six waves that are three quarters full (16 pairs S1000 1.07, S1280, whose waves are half full, 0.86;
+//     8 pairs S2048 1.20, 4 pairs 0.85; 64 pairs, 2 queries 1910 keys 0.91).
 // A limit on the context's SMs keeps to the persistent kernels, which obey it.
 bool bwd_in_tiles(const ltca_ctx* ctx, const ltca_attn_params* p) {
     if (ctx->sm_count < ctx->sm_device) return false;
     const int S = p->Sq > p->Sk ? p->Sq : p->Sk;
-    const int64_t tiles = (int64_t)p->B * p->H * ((p->Sq + kTile - 1) / kTile + (p->Sk + kTile - 1) / kTile);
+    const int64_t pairs = (int64_t)p->B * p->H, tq = pairs * ((p->Sq + kTile - 1) / kTile), tk = pairs * ((p->Sk + kTile - 1) / kTile);
+    const int64_t tiles = tq + tk;
     bool pays;
     if (p->bwd_deterministic) {
         const bool few_keys = !p->causal && p->Sq > 1024 && 2 * (int64_t)p->Sq > 3 * (int64_t)p->Sk && tiles <= 2 * ctx->sm_device;
         const bool few_queries = !p->causal && p->Sk > 1024 && p->Sq > 256 && 2 * (int64_t)p->Sk > 7 * (int64_t)p->Sq && tiles > 4 * ctx->sm_device;
-        pays = S <= 768 || (S <= 2048 && tiles <= 1536 && !few_keys && !few_queries);
+        const int shorter = p->Sq < p->Sk ? p->Sq : p->Sk;
+        const int64_t sms = ctx->sm_device, waves = (tq + sms - 1) / sms + (tk + sms - 1) / sms;      // of the persistent pair
+        const bool masked = p->keep_mask && (p->causal ? shorter > 900 || (shorter > 640 && waves <= 3 && 2 * tiles > waves * sms)
+                                                       : S > 900 && shorter > 300 && waves <= 6 && 4 * tiles > 3 * waves * sms);
+        pays = S <= 768 || (S <= 2048 && tiles <= 1536 && !few_keys && !few_queries && !masked);
     } else {
         const bool few_queries = tiles <= 128 && (p->Sk > 640 ? 5 * (int64_t)p->Sq < 2 * (int64_t)p->Sk : p->Sk > 576 && p->Sq <= kTile);
-        pays = S <= 128 || (S <= 384 && p->causal) || (((S <= 640 && tiles <= 512) || (S <= 1024 && tiles <= 128)) && !few_queries);
+        const bool few_keys = !p->causal && p->Sq > 900 && 3 * (int64_t)p->Sk <= p->Sq;
+        pays = S <= 128 || (S <= 384 && p->causal) || (((S <= 640 && tiles <= 512) || (S <= 1024 && tiles <= 128)) && !few_queries && !few_keys);
         pays = pays && !p->keep_mask && tma_strides(p->dq_strides, p->B, p->H);       // (the one-kernel form's dQ takes any strides)
     }
     return pays && !in_place(p);
